@@ -148,33 +148,35 @@ NodeP make_result(nrs_ctx* ctx, const std::vector<size_t>& shape, std::vector<No
 
 // Stages NHWC planes of an NCHW tensor [n,c,h,w] at `src` into fresh pool blocks and registers
 // them with the context under `src`.  Returns false (nothing allocated) when the tensor-core
-// convolutions would not take this tensor (FP32 mode, channel count not a multiple of 32).
+// convolutions would not take this tensor (FP32 mode).
 static bool stage_planes(nrs_ctx* ctx, const float* src, const std::vector<size_t>& shape, float** hi, float** lo) {
   *hi = *lo = nullptr;
-  if (ctx->math_mode == NRS_MATH_FP32 || shape.size() != 4 || shape[1] % 32 != 0 || shape[0] == 0) return false;
+  if (ctx->math_mode == NRS_MATH_FP32 || shape.size() != 4 || shape[0] == 0) return false;
   if (!tc::tensor_map_encoder()) return false;
   if (ctx->plane_hints.count(src)) return false;   // already there (the tensor feeds two convolutions)
   const bool split = ctx->math_mode == NRS_MATH_3XTF32;
   const size_t n = shape[0], c = shape[1], hw = shape[2] * shape[3];
-  *hi = dalloc(ctx, n * c * hw);
-  if (split) *lo = dalloc(ctx, n * c * hw);
-  check(ctx, nrs_tc_stage(ctx, src, *hi, *lo, (int)hw, (int)c, (int)c, (int)n, c * hw, c * hw, true));
+  const size_t floats = n * hw * nrs_plane_ld((int)c);
+  *hi = dalloc(ctx, floats);
+  if (split) *lo = dalloc(ctx, floats);
+  check(ctx, nrs_tc_stage_image(ctx, src, *hi, *lo, (int)n, (int)c, (int)hw));
   ctx->plane_hints[src] = NrsPlanes{*hi, *lo, split ? 1 : 0};
   return true;
 }
 
-// Row planes of a 2-D tensor [rows][cols] (cols a multiple of 32) for the tensor-core GEMMs: the layout
-// is the tensor's own, so the same planes serve it as the A operand of x@W and, read along the rows, as
+// Row planes of a 2-D tensor [rows][cols] for the tensor-core GEMMs: the layout is the tensor's own (rows
+// padded to 32 bytes), so the same planes serve it as the A operand of x@W and, read along the rows, as
 // an operand of the weight gradient x^T dz.  Stages them into fresh pool blocks and registers them with
 // the context under `src`; false (nothing allocated) when a tensor-core GEMM would not read them.
 static bool stage_planes_2d(nrs_ctx* ctx, const float* src, size_t rows, size_t cols, float** hi, float** lo) {
   *hi = *lo = nullptr;
-  if (ctx->math_mode == NRS_MATH_FP32 || cols % 32 != 0 || rows == 0 || rows > 2147483647u || cols > 2147483647u) return false;
+  if (ctx->math_mode == NRS_MATH_FP32 || rows == 0 || rows > 2147483647u || cols > 2147483647u) return false;
   if (!tc::tensor_map_encoder() || ctx->plane_hints.count(src)) return false;
   const bool split = ctx->math_mode == NRS_MATH_3XTF32;
-  *hi = dalloc(ctx, rows * cols);
-  if (split) *lo = dalloc(ctx, rows * cols);
-  check(ctx, nrs_tc_stage(ctx, src, *hi, *lo, (int)rows, (int)cols, (int)cols, 1, 0, 0, false));
+  const int ld = nrs_plane_ld((int)cols);
+  *hi = dalloc(ctx, rows * ld);
+  if (split) *lo = dalloc(ctx, rows * ld);
+  check(ctx, nrs_tc_stage(ctx, src, *hi, *lo, (int)rows, (int)cols, ld, 1, 0, 0, false));
   NrsPlanes pl{*hi, *lo, split ? 1 : 0};
   pl.rows = (int)rows;
   pl.cols = (int)cols;
@@ -644,22 +646,23 @@ NodeP conv2d_act(const NodeP& x, const NodeP& w, const NodeP& b, size_t stride, 
   const int oh = (h + 2 * (int)pad - kh) / (int)stride + 1, ow = (wd + 2 * (int)pad - kw) / (int)stride + 1;
   NodeP out = make_out(ctx, {(size_t)n, (size_t)co, (size_t)oh, (size_t)ow}, {x, w, b});
   // The input's NHWC planes serve this forward pass and, later, the weight gradient.
-  if (stride == 1 && !x->planes_hi && co % 32 == 0 && w->requires_grad) {
+  const bool patches = nrs_conv_uses_patches(ci, kh, kw);
+  if (!patches && !x->planes_hi && w->requires_grad && planes_possible(ctx)) {
     float *phi = nullptr, *plo = nullptr;
     if (stage_planes(ctx, x->data, x->shape, &phi, &plo)) { x->planes_hi = phi; x->planes_lo = plo; }
   }
-  // Image layer in a TF32 mode: forward and weight gradient both run on the tensor cores over the
+  // Few input channels in a TF32 mode: forward and weight gradient both run on the tensor cores over the
   // input's patch planes; make them once.
-  if ((ci == 1 || ci == 3) && kh == 3 && kw == 3 && stride == 1 && co % 32 == 0 && !x->patches_hi && planes_possible(ctx) &&
-      (size_t)n * oh * ow >= 4096 && !ctx->patch_hints.count(x->data)) {
-    const size_t floats = (size_t)n * oh * ow * 32;
+  if (patches && w->requires_grad && !x->patches_hi && planes_possible(ctx) && (long)n * oh * ow >= kNrsPatchMinPixels &&
+      !ctx->patch_hints.count(x->data)) {
+    const size_t floats = (size_t)n * oh * ow * nrs_plane_ld(ci * kh * kw);
     float* phi = dalloc(ctx, floats);
     float* plo = ctx->math_mode == NRS_MATH_3XTF32 ? dalloc(ctx, floats) : nullptr;
-    const int st = nrs_smallc_patch_planes(ctx, x->data, phi, plo, n, ci, h, wd, (int)pad);
+    const int st = nrs_patch_planes(ctx, x->data, phi, plo, n, ci, h, wd, kh, kw, (int)stride, (int)pad);
     if (st == NRS_OK) {
       x->patches_hi = phi;
       x->patches_lo = plo;
-      ctx->patch_hints[x->data] = NrsPlanes{phi, plo, (plo ? 1 : 0) | ((int)pad << 8)};
+      ctx->patch_hints[x->data] = NrsPatchPlanes{phi, plo, kh, kw, (int)stride, (int)pad};
     } else {
       nrs_free(ctx, phi);
       if (plo) nrs_free(ctx, plo);
@@ -698,18 +701,18 @@ NodeP conv2d_act(const NodeP& x, const NodeP& w, const NodeP& b, size_t stride, 
   Node* self = out.get();
   const int s = (int)stride, p = (int)pad;
   out->relu_folded = act == NRS_ACT_RELU;
-  // (an image layer with 1 or 3 input channels takes dy planes too: its weight gradient runs on the
-  // tensor cores over patch planes)
-  const bool image_layer = (ci == 1 || ci == 3) && kh == 3 && kw == 3;
-  out->wants_grad_planes = act == NRS_ACT_RELU && s == 1 && (ci % 32 == 0 || image_layer) && co % 32 == 0;
-  out->backward_fn = [self, x, w, b, n, ci, h, wd, co, kh, kw, s, p, act, image_layer]() {
+  // every tensor-core backward pass reads dy planes (the producers of a gradient write them with a pixel stride
+  // of the channel count: whole groups of eight only)
+  const bool dy_planes = s <= 8 && !(patches && (long)n * oh * ow < kNrsPatchMinPixels);
+  out->wants_grad_planes = act == NRS_ACT_RELU && dy_planes && co % 8 == 0;
+  out->backward_fn = [self, x, w, b, n, ci, h, wd, co, kh, kw, s, p, act, dy_planes]() {
     nrs_ctx* ctx = self->ctx;
     const float* dy = grad_in(self);
     float* masked = nullptr;
     float *dhi = nullptr, *dlo = nullptr;
     bool staged = false;
     // Do the tensor-core data / weight gradients want NHWC planes of dy?
-    const bool want_planes = s == 1 && (ci % 32 == 0 || image_layer) && co % 32 == 0 && planes_possible(ctx);
+    const bool want_planes = dy_planes && planes_possible(ctx);
     if (self->grad_premasked) {
       // The consumer (a max-pool's backward pass or a convolution's data-gradient epilogue) already
       // folded the ReLU mask into this gradient, and may have left its planes.
@@ -719,7 +722,7 @@ NodeP conv2d_act(const NodeP& x, const NodeP& w, const NodeP& b, size_t stride, 
       }
     } else if (act == NRS_ACT_RELU) {  // y > 0 exactly where the pre-activation was > 0
       masked = dalloc(ctx, self->len());
-      if (want_planes) {   // mask and stage in one pass
+      if (want_planes && co % 8 == 0) {   // mask and stage in one pass
         const bool split = ctx->math_mode == NRS_MATH_3XTF32;
         dhi = dalloc(ctx, self->len());
         if (split) dlo = dalloc(ctx, self->len());
@@ -729,6 +732,7 @@ NodeP conv2d_act(const NodeP& x, const NodeP& w, const NodeP& b, size_t stride, 
         staged = true;
       } else {
         check(ctx, nrs_relu_bwd(ctx, self->data, dy, masked, self->len(), 0));
+        if (want_planes) staged = stage_planes(ctx, masked, self->shape, &dhi, &dlo);
       }
       dy = masked;
     } else if (want_planes) {
@@ -769,7 +773,7 @@ NodeP maxpool2d(const NodeP& x, size_t kernel, size_t stride, bool emit_planes) 
   check(ctx, nrs_alloc(ctx, out->len() * sizeof(int32_t), 0, &am));
   out->saved.push_back(am);
   bool done = false;
-  if (emit_planes && k == 2 && s == 2 && c % 32 == 0 && planes_possible(ctx)) {
+  if (emit_planes && k == 2 && s == 2 && c % 8 == 0 && planes_possible(ctx)) {
     // a tensor-core convolution reads the result next: write its operand planes in the same pass
     float* phi = dalloc(ctx, out->len());
     float* plo = ctx->math_mode == NRS_MATH_3XTF32 ? dalloc(ctx, out->len()) : nullptr;

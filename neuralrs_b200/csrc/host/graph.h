@@ -53,7 +53,7 @@ struct Node {
   // by the forward pass and the weight gradient (registered with the context while alive).
   float* planes_hi = nullptr;
   float* planes_lo = nullptr;
-  // For an image tensor (1 or 3 channels) read by a 3x3 layer: its patch planes, shared by that
+  // For an image tensor of few channels: its patch planes for the layer that read it first, shared by that
   // layer's forward pass and weight gradient (registered with the context while alive).
   float* patches_hi = nullptr;
   float* patches_lo = nullptr;

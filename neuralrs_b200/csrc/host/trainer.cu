@@ -238,7 +238,7 @@ NodeP forward(nrs_trainer* t, const NodeP& x, const int32_t* ids_dev, size_t bat
         // The layer list shows what reads this output: if it is a stride-1 convolution, its
         // NHWC operand planes are written by this layer's kernel.
         const size_t nx = li + (relu_next ? 2 : 1);
-        const bool conv_reads = nx < t->layers.size() && t->layers[nx].kind == NRS_LAYER_CONV && t->layers[nx].d == 1;
+        const bool conv_reads = nx < t->layers.size() && t->layers[nx].kind == NRS_LAYER_CONV && t->layers[nx].d <= 8;
         h = nrs::cuda::conv2d_act(h, t->params[pi], t->params[pi + 1], (size_t)l.d, (size_t)l.e,
                                   relu_next ? NRS_ACT_RELU : NRS_ACT_NONE, conv_reads);
         pi += 2;
@@ -280,7 +280,7 @@ NodeP forward(nrs_trainer* t, const NodeP& x, const int32_t* ids_dev, size_t bat
       case NRS_LAYER_RELU: h = nrs::cuda::relu(h); break;
       case NRS_LAYER_GELU: h = nrs::cuda::gelu(h); break;
       case NRS_LAYER_MAXPOOL: {
-        const bool conv_reads = li + 1 < t->layers.size() && t->layers[li + 1].kind == NRS_LAYER_CONV && t->layers[li + 1].d == 1;
+        const bool conv_reads = li + 1 < t->layers.size() && t->layers[li + 1].kind == NRS_LAYER_CONV && t->layers[li + 1].d <= 8;
         h = nrs::cuda::maxpool2d(h, (size_t)l.a, (size_t)l.b, conv_reads);
         break;
       }
@@ -318,9 +318,12 @@ void stage_weights(nrs_trainer* t) {
     for (const nrs_layer_spec& l : t->layers) {
       switch (l.kind) {
         case NRS_LAYER_CONV:
-          if (l.d == 1 && l.a % 32 == 0 && l.b % 32 == 0) {
+          if (l.d <= 8) {
             const NodeP& w = t->params[pi];
-            d.push_back(NrsWeightDesc{w->data, NRS_WF_CONV_FWD, 0, 0, l.b, l.a, l.c * l.c});
+            if (nrs_conv_uses_patches(l.a, l.c, l.c))   // a 1x1 layer over the values of a patch
+              d.push_back(NrsWeightDesc{w->data, NRS_WF_CONV_FWD, 0, 0, l.b, l.a * l.c * l.c, 1});
+            else
+              d.push_back(NrsWeightDesc{w->data, NRS_WF_CONV_FWD, 0, 0, l.b, l.a, l.c * l.c});
             if (!first_contraction) d.push_back(NrsWeightDesc{w->data, NRS_WF_CONV_DGRAD, 0, 0, l.b, l.a, l.c * l.c});
           }
           first_contraction = false;

@@ -45,6 +45,23 @@ struct NrsPlanes {
   int rows = 0, cols = 0;
 };
 
+// Patch planes of an image tensor [n][ci][h][w]: for every output pixel of a convolution the ci*kh*kw input values
+// under it, [n*oh*ow][nrs_plane_ld(ci*kh*kw)].
+struct NrsPatchPlanes {
+  float* hi;
+  float* lo;
+  int kh, kw, stride, pad;
+};
+// Layers that run on patches: with fewer than 8 input channels a 32-channel K-block per tap would be mostly padding
+// (a factor of 4 and more), while all taps together fill a few blocks (up to 128 values, at most 1 KB per pixel).
+// (Images of a few hundred pixels in all take the direct kernels of conv_smallc.cu where those apply: fewer launches.)
+constexpr long kNrsPatchMinPixels = 1024;
+inline bool nrs_conv_uses_patches(int ci, int kh, int kw) { return ci < 8 && kh * kw > 1 && ci * kh * kw <= 128; }
+
+// Floats between two pixels of a tensor's NHWC planes: its channels rounded up to whole 32-byte sectors (TMA wants
+// 16-byte strides; with 112-byte rows, 27 values padded to 28, a convolution over them ran 41 us instead of 28).
+constexpr inline int nrs_plane_ld(int channels) { return (channels + 7) & ~7; }
+
 // Extra work a convolution kernel can fold into the epilogue that writes `out` (keyed by the
 // output pointer in nrs_ctx::out_extras).  A kernel that honours the request erases the entry;
 // an entry still present after the call means the caller has to do the work itself.
@@ -128,10 +145,9 @@ struct nrs_ctx {
   std::map<const void*, NrsPlanes> owned_planes;   // nrs_planes_cache: planes the context itself allocated
   std::map<const void*, NrsOutExtras> out_extras;
   std::map<const void*, NrsColsumRequest> colsum_requests;
-  // Patch planes ([pixels][32], see conv_smallc.cu) of an image tensor, keyed by its device pointer:
-  // the host graph makes them once per step for the image layer's forward pass and weight gradient
-  // (`split`: bit 0 = residual plane present, bits 8.. = the padding they were made for).
-  std::map<const void*, NrsPlanes> patch_hints;
+  // Patch planes (see conv_patch.cu) of a tensor with few channels, keyed by its device pointer: the host graph
+  // makes them once per step for the layer's forward pass and weight gradient.
+  std::map<const void*, NrsPatchPlanes> patch_hints;
   NrsWeightSet weight_set;
   // Set by a caller that has just issued a kernel whose output the NEXT tensor-core weight-gradient launch
   // does not read (see NRS_PDL_PROLOGUE): that launch may overlap it.  Consumed by the launch.
@@ -192,6 +208,7 @@ extern "C" int nrs_layernorm_bwd_planes(nrs_ctx* ctx, const float* g, const floa
 // TF32 planes of a batch of [rows][K] matrices (tc_stage.cu); see tc_mainloop.cuh for the layouts.
 int nrs_tc_stage(nrs_ctx* ctx, const float* src, float* hi, float* lo, int rows, int K, int ldk, int batch,
                  size_t src_bstride, size_t dst_bstride, bool src_k_by_rows);
+int nrs_tc_stage_image(nrs_ctx* ctx, const float* src, float* hi, float* lo, int n, int c, int hw);
 // Counter window of a per-sample draw of `count` elements (count = samples * per-sample) in blocks of four:
 // first block to use and by how many blocks the stream advances.  Falls back to the plain stream (this
 // process's own draws) when no shard is set, the call is not per-sample, or the shard does not start on a
@@ -351,8 +368,13 @@ int nrs_tc_attention_fwd(nrs_ctx* ctx, const float* q, const float* k, const flo
 int nrs_tc_attention_bwd(nrs_ctx* ctx, const float* q, const float* k, const float* v, const float* probs, const float* dout,
                          float* dq, float* dk, float* dv, int batch, int seq, int heads, int d_head, int acc_q, int acc_k,
                          int acc_v);
-// Patch planes of x[n,ci,h,w] for a 3x3 / pad `pad` image layer (ci = 1 or 3): hi/lo [n*oh*ow][32].
-int nrs_smallc_patch_planes(nrs_ctx* ctx, const float* x, float* hi, float* lo, int n, int ci, int h, int wd, int pad);
+// Tensor-core convolution through patch planes (conv_patch.cu); NRS_ERR_UNSUPPORTED (no error text) for layers that
+// do not use patches.
+int nrs_patch_planes(nrs_ctx* ctx, const float* x, float* hi, float* lo, int n, int ci, int h, int wd, int kh, int kw, int stride, int pad);
+int nrs_patch_conv_fwd(nrs_ctx* ctx, const float* x, const float* w, const float* b, float* y, int n, int ci, int h, int wd, int co,
+                       int kh, int kw, int stride, int pad, int act);
+int nrs_patch_conv_wgrad(nrs_ctx* ctx, const float* x, const float* dy, float* dw, int n, int ci, int h, int wd, int co, int kh, int kw,
+                         int stride, int pad, int accumulate);
 // Direct FFMA kernels for 3x3 stride-1 layers over 1 or 3 input channels (conv_smallc.cu).
 int nrs_smallc_conv_fwd(nrs_ctx* ctx, const float* x, const float* w, const float* b, float* y, int n, int ci, int h,
                         int wd, int co, int kh, int kw, int stride, int pad, int act);

@@ -6,8 +6,8 @@
 // dense/batched GEMM in all transpositions and convolution forward, data
 // gradient and weight gradient read straight from the NCHW tensors.  It is the
 // exact-f32 path: NRS_MATH_FP32 always runs it, and the tensor-core modes run
-// it for shapes the tcgen05 kernels do not cover (tiny channel counts, strides,
-// ragged tiles).  Long-K problems (weight gradients) are split along K into a
+// it for shapes the tcgen05 kernels do not cover (products of a few dozen rows,
+// strides above 8).  Long-K problems (weight gradients) are split along K into a
 // workspace and reduced in a fixed order, so results are run-to-run
 // deterministic.
 //
@@ -352,6 +352,13 @@ int thin_gemm(nrs_ctx* ctx, int ta, int tb, int m, int n, int k, const float* a,
   return NRS_OK;
 }
 
+// Whether an image layer tries the direct FFMA kernels first: always in FP32 mode, and in the TF32 modes for images
+// of a few hundred pixels in all, where one launch beats patches, weight planes and a tile pipeline.
+bool conv_runs_direct(const nrs_ctx* ctx, int n, int ci, int kh, int kw, int h, int wd, int stride, int pad) {
+  const long pixels = (long)n * ((h + 2 * pad - kh) / stride + 1) * ((wd + 2 * pad - kw) / stride + 1);
+  return ctx->math_mode == NRS_MATH_FP32 || (nrs_conv_uses_patches(ci, kh, kw) && pixels < kNrsPatchMinPixels);
+}
+
 int check_conv_dims(nrs_ctx* ctx, const char* who, int n, int ci, int h, int wd, int co, int kh, int kw,
                     int stride, int pad) {
   NRS_REQUIRE(ctx, n >= 0 && ci > 0 && h > 0 && wd > 0 && co > 0 && kh > 0 && kw > 0, NRS_ERR_SHAPE,
@@ -430,10 +437,15 @@ int nrs_conv2d_fwd(nrs_ctx* ctx, const float* x, const float* w, const float* b,
   NRS_REQUIRE(ctx, x && w && y, NRS_ERR_ARG, "nrs_conv2d_fwd: null tensor");
   NrsProfScope prof(ctx, NRS_PROF_CONV_FWD,
                     2.0 * n * co * ((h + 2 * pad - kh) / stride + 1) * ((wd + 2 * pad - kw) / stride + 1) * ci * kh * kw);
-  st = nrs_smallc_conv_fwd(ctx, x, w, b, y, n, ci, h, wd, co, kh, kw, stride, pad, act);
-  if (st != NRS_ERR_UNSUPPORTED) return st;
+  // TF32 modes: the tensor cores, whatever the channel counts and the stride (patches below 8 input channels); see the
+  // comment at conv_runs_direct for the two exceptions.  FP32 mode: the FFMA kernels.
+  if (conv_runs_direct(ctx, n, ci, kh, kw, h, wd, stride, pad)) {
+    st = nrs_smallc_conv_fwd(ctx, x, w, b, y, n, ci, h, wd, co, kh, kw, stride, pad, act);
+    if (st != NRS_ERR_UNSUPPORTED) return st;
+  }
   if (ctx->math_mode != NRS_MATH_FP32) {
-    st = nrs_tc_conv_fwd(ctx, x, w, b, y, n, ci, h, wd, co, kh, kw, stride, pad, act);
+    st = nrs_patch_conv_fwd(ctx, x, w, b, y, n, ci, h, wd, co, kh, kw, stride, pad, act);
+    if (st == NRS_ERR_UNSUPPORTED) st = nrs_tc_conv_fwd(ctx, x, w, b, y, n, ci, h, wd, co, kh, kw, stride, pad, act);
     if (st != NRS_ERR_UNSUPPORTED) return st;
   }
   NrsConvFpropProb p;
@@ -496,7 +508,11 @@ int nrs_conv2d_bwd(nrs_ctx* ctx, const float* x, const float* w, const float* dy
   if (dw) {
     NrsProfScope prof(ctx, NRS_PROF_CONV_WGRAD, conv_flop);
     NrsIndependentNext overlap(ctx, wgrad_may_overlap);
-    st = nrs_smallc_conv_wgrad(ctx, x, dy, dw, n, ci, h, wd, co, kh, kw, stride, pad, accumulate);
+    st = NRS_ERR_UNSUPPORTED;
+    if (conv_runs_direct(ctx, n, ci, kh, kw, h, wd, stride, pad))
+      st = nrs_smallc_conv_wgrad(ctx, x, dy, dw, n, ci, h, wd, co, kh, kw, stride, pad, accumulate);
+    if (st == NRS_ERR_UNSUPPORTED && ctx->math_mode != NRS_MATH_FP32)
+      st = nrs_patch_conv_wgrad(ctx, x, dy, dw, n, ci, h, wd, co, kh, kw, stride, pad, accumulate);
     if (st == NRS_ERR_UNSUPPORTED && ctx->math_mode != NRS_MATH_FP32)
       st = nrs_tc_conv_wgrad_rows(ctx, x, dy, dw, n, ci, h, wd, co, kh, kw, stride, pad, accumulate);
     if (st == NRS_ERR_UNSUPPORTED && ctx->math_mode != NRS_MATH_FP32)
@@ -535,14 +551,15 @@ int nrs_planes_cache(nrs_ctx* ctx, const float* t, int n, int c, int h, int w) {
   NRS_REQUIRE(ctx, n >= 0 && c > 0 && h > 0 && w > 0, NRS_ERR_SHAPE, "nrs_planes_cache: bad shape [%d,%d,%d,%d]", n, c, h, w);
   int st = nrs_planes_drop(ctx, t);   // the contents may have changed since an earlier call
   if (st != NRS_OK) return st;
-  if (ctx->math_mode == NRS_MATH_FP32 || c % 32 != 0 || n == 0 || !tc::tensor_map_encoder()) return NRS_OK;
+  if (ctx->math_mode == NRS_MATH_FP32 || n == 0 || !tc::tensor_map_encoder()) return NRS_OK;
+  if (c < 8) return NRS_OK;                        // such layers read patches (nrs_conv_uses_patches)
   if (ctx->plane_hints.count(t)) return NRS_OK;   // someone else (the node graph) already keeps planes of it
   const bool split = ctx->math_mode == NRS_MATH_3XTF32;
-  const size_t hw = (size_t)h * w, floats = (size_t)n * c * hw;
+  const size_t hw = (size_t)h * w, floats = (size_t)n * nrs_plane_ld(c) * hw;
   void *hi = nullptr, *lo = nullptr;
   st = nrs_alloc(ctx, floats * sizeof(float), 0, &hi);
   if (st == NRS_OK && split) st = nrs_alloc(ctx, floats * sizeof(float), 0, &lo);
-  if (st == NRS_OK) st = nrs_tc_stage(ctx, t, (float*)hi, (float*)lo, (int)hw, c, c, n, (size_t)c * hw, (size_t)c * hw, true);
+  if (st == NRS_OK) st = nrs_tc_stage_image(ctx, t, (float*)hi, (float*)lo, n, c, (int)hw);
   if (st != NRS_OK) {
     if (hi) nrs_free(ctx, hi);
     if (lo) nrs_free(ctx, lo);

@@ -215,15 +215,17 @@ inline PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 }
 
 // f32 tensor of `rank` dims (dim[0] innermost, contiguous), strides in BYTES for dims 1..rank-1
-// (multiples of 16), box extents per dim (box[0]*4 must be 128 for the 128-byte swizzle).
+// (multiples of 16), box extents per dim (box[0]*4 must be 128 for the 128-byte swizzle).  `step` (optional):
+// every step[i]-th element is taken along dim i >= 1 (a strided convolution's pixels); box[i] counts the elements
+// that land in shared memory, and box[i] * step[i] may not exceed 256.
 inline bool encode_tmap_f32(CUtensorMap* out, const void* base, int rank, const uint64_t* dim, const uint64_t* stride_bytes,
-                            const uint32_t* box, bool atom32 = false) {
+                            const uint32_t* box, bool atom32 = false, const uint32_t* step = nullptr) {
   auto enc = tensor_map_encoder();
   if (!enc) return false;
   cuuint64_t gdim[5];
   cuuint64_t gstr[4];
   cuuint32_t bx[5], es[5];
-  for (int i = 0; i < rank; ++i) { gdim[i] = dim[i]; bx[i] = box[i]; es[i] = 1; }
+  for (int i = 0; i < rank; ++i) { gdim[i] = dim[i]; es[i] = step ? step[i] : 1; bx[i] = box[i] * es[i]; }
   for (int i = 0; i + 1 < rank; ++i) gstr[i] = stride_bytes[i];
   const CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, (cuuint32_t)rank, const_cast<void*>(base), gdim, gstr, bx, es,
                          CU_TENSOR_MAP_INTERLEAVE_NONE, atom32 ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B,

@@ -6,19 +6,24 @@
 // reduction runs over (tap, 32-channel block).  For every tap the A slice is ONE
 // 4-D TMA box {32 channels, Wt, Ht, Nt} whose spatial origin is shifted by the
 // tap offset; rows or columns that fall outside the image are zero-filled by TMA,
-// which is exactly the zero padding.  (The shift lands on the W/H coordinates;
-// the innermost, 16-byte-aligned coordinate is the channel block.)  The B slice
-// is a plain 2-D box of the re-laid-out weights [out_ch][(tap, in_ch)].
+// which is exactly the zero padding, and so are the channels beyond the last one of
+// a ragged channel block.  (The shift lands on the W/H coordinates; the innermost,
+// 16-byte-aligned coordinate is the channel block.)  The B slice is a plain 2-D box
+// of the re-laid-out weights [out_ch][(tap, in_ch padded to 32)].
 //
-//   forward        y[n,co,oy,ox]  = act(b[co] + sum x[n,ci,oy+i-p,ox+j-p] w[co,ci,i,j])
-//   data gradient  dx[n,ci,y,x] (+)= sum dy[n,co,y-i+p,x-j+p] w[co,ci,i,j]
+//   forward        y[n,co,oy,ox]  = act(b[co] + sum x[n,ci,oy*s+i-p,ox*s+j-p] w[co,ci,i,j])
+//   data gradient  dx[n,ci,y,x] (+)= sum dy[n,co,(y+p-i)/s,(x+p-j)/s] w[co,ci,i,j]
 // are the same kernel with the tap sign flipped and the roles of the channel
-// counts exchanged.  The epilogue writes NCHW directly: for a fixed channel the 32
-// lanes of a warp hold 32 consecutive pixels, so every store is a full 128-byte line.
+// counts exchanged.  A stride s makes the forward box take every s-th pixel (the
+// tensor map's element strides).  The data gradient of a strided layer falls into
+// s*s independent stride-1 problems, one per residue of (y+p, x+p) modulo s: each
+// reads the taps of its own residue only (no multiplication by the zeros between
+// the pixels of dy) and writes every s-th pixel of dx.  The epilogue writes NCHW
+// directly: for a fixed channel the 32 lanes of a warp hold 32 consecutive pixels,
+// so every store of a stride-1 problem is a full 128-byte line.
 //
-// Stride-1 convolutions with channel counts that are multiples of 32 run here;
-// everything else (first layers with 1 or 3 channels, strides) runs on the FFMA
-// implicit-GEMM kernel.
+// Measured (x[64,48,57,57] -> 80 channels, 3x3, stride 2, 3xTF32): forward 220 us as an FFMA implicit GEMM, 61 here;
+// data gradient 1706 us (three quarters of its products were with zeros), 97 in its four residues.
 //
 // Reference counterparts: conv2d_im2col + matmul_nn + conv2d_col2out (forward),
 // conv2d_out2mm + matmul_tn + conv2d_col2im (data gradient) — src/cuda/nn/conv.rs:27-149,
@@ -28,10 +33,15 @@
 namespace {
 
 struct ConvPolicy {
-  int Wt, Ht, Nt, tiles_y;
-  int out_h, out_w, n_img, n_ch_out;
-  int cblocks, kw_taps;
+  int Wt, Ht, Nt, tiles_x, tiles_y;   // pixel tile in the space of (u, v), the pixels this launch computes
+  int sub_h, sub_w;                   // extents of that space
+  int out_h, out_w;                   // the tensor written: pixel (u, v) is (u*out_step + out_y0, v*out_step + out_x0)
+  int out_step, out_y0, out_x0;
+  int n_img, n_ch_out;
+  int cblocks, tap_cols;              // 32-channel blocks per tap; taps per kernel row that take part
+  int in_step;                        // pixels of the activation per step of (u, v)
   int sgn, base_y, base_x;
+  int w_tap0, w_tap_row, w_tap_col;   // weight tap of (0, 0), and its steps along both tap axes
   float* out;
   const float* bias;
   int act, accumulate;
@@ -45,21 +55,59 @@ struct ConvPolicy {
   float* colsum_partial;
 
   __device__ __forceinline__ uint32_t a_slice_bytes() const { return slice_bytes; }
-  __device__ __forceinline__ void load_a(void* dst, const CUtensorMap* tm, uint64_t* bar, int kb, int tile_m, int) const {
-    const int tap = kb / cblocks, cb = kb - tap * cblocks;
-    const int i = tap / kw_taps, j = tap - i * kw_taps;
-    const int n0 = (tile_m / tiles_y) * Nt, y0 = (tile_m % tiles_y) * Ht;
-    tc::tma_load_4d(dst, tm, bar, cb * 32, sgn * j + base_x, y0 + sgn * i + base_y, n0);
+  __device__ __forceinline__ void origin(int tile_m, int* x0, int* y0, int* n0) const {
+    const int tx = tile_m % tiles_x, t = tile_m / tiles_x;
+    *x0 = tx * Wt;
+    *y0 = (t % tiles_y) * Ht;
+    *n0 = (t / tiles_y) * Nt;
+  }
+  // Position of a K-slice: tap (i, j), channel block cb; the box origin of tap (i, j) and the weight column.
+  struct Cursor { int b_col, cb, i, j, x, y, n, x_first; };
+  __device__ __forceinline__ Cursor cursor(int tile_m, int, int kb) const {
+    Cursor c;
+    const int tap = kb / cblocks;
+    c.cb = kb - tap * cblocks;
+    c.i = tap / tap_cols;
+    c.j = tap - c.i * tap_cols;
+    int x0, y0;
+    origin(tile_m, &x0, &y0, &c.n);
+    c.x_first = x0 * in_step + base_x;
+    c.x = c.x_first + sgn * c.j;
+    c.y = y0 * in_step + base_y + sgn * c.i;
+    c.b_col = weight_column(c);
+    return c;
+  }
+  __device__ __forceinline__ int weight_column(const Cursor& c) const {
+    return ((w_tap0 + c.i * w_tap_row + c.j * w_tap_col) * cblocks + c.cb) * 32;
+  }
+  __device__ __forceinline__ void advance(Cursor& c) const {
+    c.b_col += 32;
+    if (++c.cb < cblocks) return;
+    c.cb = 0;
+    c.x += sgn;
+    if (++c.j == tap_cols) {
+      c.j = 0;
+      c.x = c.x_first;
+      c.y += sgn;
+      ++c.i;
+    }
+    c.b_col = weight_column(c);
+  }
+  __device__ __forceinline__ void load_a(void* dst, const CUtensorMap* tm, uint64_t* bar, const Cursor& c) const {
+    tc::tma_load_4d(dst, tm, bar, c.cb * 32, c.x, c.y, c.n);
   }
   // NCHW offset of channel 0 of the pixel behind accumulator row `row`, and the pixel's linear index.
   __device__ __forceinline__ bool locate(int tile_m, int row, size_t* nchw_off, size_t* pixel) const {
     if (row >= Wt * Ht * Nt) return false;
-    const int xt = row % Wt, t = row / Wt;
-    const int yt = t % Ht, nt = t / Ht;
-    const int n = (tile_m / tiles_y) * Nt + nt, y = (tile_m % tiles_y) * Ht + yt;
-    if (n >= n_img || y >= out_h) return false;
-    *nchw_off = (size_t)n * n_ch_out * out_h * out_w + (size_t)y * out_w + xt;
-    *pixel = ((size_t)n * out_h + y) * out_w + xt;
+    int x0, y0, n0;
+    origin(tile_m, &x0, &y0, &n0);
+    const int t = row / Wt;
+    const int nt = t / Ht;
+    const int v = x0 + row - t * Wt, u = y0 + t - nt * Ht, n = n0 + nt;
+    if (n >= n_img || u >= sub_h || v >= sub_w) return false;
+    const int y = u * out_step + out_y0, x = v * out_step + out_x0;
+    *nchw_off = (size_t)n * n_ch_out * out_h * out_w + (size_t)y * out_w + x;
+    *pixel = ((size_t)n * out_h + y) * out_w + x;
     return true;
   }
   __device__ __forceinline__ void store(int tile_m, int, int row, int ch, float v) const {
@@ -81,30 +129,42 @@ struct ConvPolicy {
   __device__ __forceinline__ float* colsum_row(int tile_m, int q) const {
     return colsum_partial ? colsum_partial + ((size_t)tile_m * 4 + q) * n_ch_out : nullptr;
   }
-  // TMA-store origin (x, y, image) of tile_m's pixel box in the NHWC planes.
-  __device__ __forceinline__ void out_origin(int tile_m, int* x0, int* y0, int* n0) const {
-    *x0 = 0;
-    *y0 = (tile_m % tiles_y) * Ht;
-    *n0 = (tile_m / tiles_y) * Nt;
+  // An accumulator row: does it hold a pixel, the NCHW offset of that pixel in channel 0, and the origin of its tile's
+  // box (x, y, image), which is where the TMA store of the tile's planes goes (out_step == 1).
+  struct Row { bool live; size_t off; int x0, y0, n0; };
+  __device__ __forceinline__ Row row(int tile_m, int, int r) const {
+    Row w;
+    size_t pixel;
+    w.off = 0;
+    w.live = locate(tile_m, r, &w.off, &pixel);
+    origin(tile_m, &w.x0, &w.y0, &w.n0);
+    return w;
   }
-  // One accumulator row, 32 consecutive channels [nb, nb+32): bias, activation, accumulate, mask,
-  // NCHW store; the finished values come back in v (zeros for rows outside the tensor) so the
+  // One accumulator row, channels [nb, nb+32) as far as they exist: bias, activation, accumulate, mask,
+  // NCHW store; the finished values come back in v (zeros for rows and channels outside the tensor) so the
   // caller can emit them as planes.  Loads are issued in batches ahead of the stores.
-  __device__ __forceinline__ void epilogue(int tile_m, int, int row, int nb, int, const uint32_t (&r)[32], float (&v)[32]) const {
-    size_t off, pixel;
-    const bool live = nb < n_ch_out && locate(tile_m, row, &off, &pixel);   // channel counts are multiples of 32
-    if (!live) {
+  __device__ __forceinline__ void epilogue(const Row& rw, int nb, const uint32_t (&r)[32], float (&v)[32]) const {
+    if (!rw.live) {
 #pragma unroll
       for (int j = 0; j < 32; ++j) v[j] = 0.0f;
       return;
     }
+    // Whole channel blocks take their own instantiation: with per-channel conditions the loads of a block no longer
+    // issue together (measured on the 64-channel data gradient with mask and planes: 58 -> 217 us).
+    if (n_ch_out - nb >= 32) finish<true>(rw.off, nb, r, v);
+    else finish<false>(rw.off, nb, r, v);
+  }
+  template <bool FULL>
+  __device__ __forceinline__ void finish(size_t off, int nb, const uint32_t (&r)[32], float (&v)[32]) const {
     const size_t plane = (size_t)out_h * out_w;
     float* dst = out + off + (size_t)nb * plane;
+    const int nch = FULL ? 32 : n_ch_out - nb;   // channels of this block that exist
 #pragma unroll
-    for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
+    for (int j = 0; j < 32; ++j) v[j] = (FULL || j < nch) ? __uint_as_float(r[j]) : 0.0f;
     if (bias) {
 #pragma unroll
-      for (int j = 0; j < 32; ++j) v[j] += __ldg(bias + nb + j);
+      for (int j = 0; j < 32; ++j)
+        if (FULL || j < nch) v[j] += __ldg(bias + nb + j);
     }
     if (act != NRS_ACT_NONE) {
 #pragma unroll
@@ -113,11 +173,11 @@ struct ConvPolicy {
     if (accumulate) {
       float o[32];
 #pragma unroll
-      for (int j = 0; j < 32; ++j) o[j] = dst[(size_t)j * plane];
+      for (int j = 0; j < 32; ++j) o[j] = (FULL || j < nch) ? dst[(size_t)j * plane] : 0.0f;
 #pragma unroll
       for (int j = 0; j < 32; ++j) v[j] += o[j];
     }
-    if (mask_src) {
+    if (FULL && mask_src) {   // a mask is taken for whole channel blocks only
       const float* m = mask_src + off + (size_t)nb * plane;
       float mv[32];
 #pragma unroll
@@ -126,21 +186,33 @@ struct ConvPolicy {
       for (int j = 0; j < 32; ++j) v[j] = mv[j] > 0.0f ? v[j] : 0.0f;
     }
 #pragma unroll
-    for (int j = 0; j < 32; ++j) dst[(size_t)j * plane] = v[j];
+    for (int j = 0; j < 32; ++j)
+      if (FULL || j < nch) dst[(size_t)j * plane] = v[j];
   }
 };
 
+// One axis of a (sub-)problem: `len` output pixels at positions u*step + first, `taps` kernel taps tap0,
+// tap0 + tap_step, ..., and the activation coordinate of tap t for pixel u: u * in_step + base + sgn * t.
+struct ConvAxis {
+  int len, step, first;
+  int taps, tap0, tap_step;
+  int in_step, base;
+};
+
 struct ConvPlan {
-  // activation read by the A operand: [n_img][a_h][a_w][a_ch] NHWC planes, staged from NCHW `act_src`
+  // activation read by the A operand: [n_img][a_h][a_w] pixels of a_ch channels, NHWC planes (pixel stride
+  // nrs_plane_ld(a_ch) floats) staged from NCHW `act_src`
   const float* act_src;
   int n_img, a_ch, a_h, a_w;
   // weights and which re-layout
   const float* w;
   int co, ci, kh, kw, for_dgrad;
+  void *w_hi, *w_lo;   // its planes once staged (the residues of a strided data gradient share them)
   // output NCHW [n_img][n_ch_out][out_h][out_w]
   float* out;
   int n_ch_out, out_h, out_w;
-  int sgn, base;
+  int sgn;
+  ConvAxis ay, ax;
   const float* bias;
   int act, accumulate;
 };
@@ -148,17 +220,19 @@ struct ConvPlan {
 template <int BN, int NPLANES>
 int run_conv(nrs_ctx* ctx, const ConvPlan& p, const float* a_hi, const float* a_lo, const float* w_hi, const float* w_lo,
              const ConvPolicy& pol, int tiles_m, int* splits_out) {
-  const int taps = p.kh * p.kw;
-  const int kdim = taps * p.a_ch;
+  const int a_ld = nrs_plane_ld(p.a_ch);
+  const int kdim = p.kh * p.kw * pol.cblocks * 32;
   CUtensorMap ta_hi, ta_lo, tb_hi, tb_lo;
   const uint64_t adim[4] = {(uint64_t)p.a_ch, (uint64_t)p.a_w, (uint64_t)p.a_h, (uint64_t)p.n_img};
-  const uint64_t astr[3] = {(uint64_t)p.a_ch * 4, (uint64_t)p.a_w * p.a_ch * 4, (uint64_t)p.a_h * p.a_w * p.a_ch * 4};
+  const uint64_t astr[3] = {(uint64_t)a_ld * 4, (uint64_t)p.a_w * a_ld * 4, (uint64_t)p.a_h * p.a_w * a_ld * 4};
   const uint32_t abox[4] = {32, (uint32_t)pol.Wt, (uint32_t)pol.Ht, (uint32_t)pol.Nt};
+  const uint32_t astep[4] = {1, (uint32_t)pol.in_step, (uint32_t)pol.in_step, 1};
   const uint64_t bdim[3] = {(uint64_t)kdim, (uint64_t)p.n_ch_out, 1};
   const uint64_t bstr[2] = {(uint64_t)kdim * 4, (uint64_t)kdim * p.n_ch_out * 4};
   const uint32_t bbox[3] = {32, (uint32_t)BN, 1};
-  bool ok = tc::encode_tmap_f32(&ta_hi, a_hi, 4, adim, astr, abox) && tc::encode_tmap_f32(&tb_hi, w_hi, 3, bdim, bstr, bbox);
-  if (NPLANES == 2) ok = ok && tc::encode_tmap_f32(&ta_lo, a_lo, 4, adim, astr, abox) && tc::encode_tmap_f32(&tb_lo, w_lo, 3, bdim, bstr, bbox);
+  bool ok = tc::encode_tmap_f32(&ta_hi, a_hi, 4, adim, astr, abox, false, astep) && tc::encode_tmap_f32(&tb_hi, w_hi, 3, bdim, bstr, bbox);
+  if (NPLANES == 2)
+    ok = ok && tc::encode_tmap_f32(&ta_lo, a_lo, 4, adim, astr, abox, false, astep) && tc::encode_tmap_f32(&tb_lo, w_lo, 3, bdim, bstr, bbox);
   else { ta_lo = ta_hi; tb_lo = tb_hi; }
   // Output planes (optional): the same box geometry as an activation load, in output space.
   CUtensorMap to_hi, to_lo;
@@ -169,107 +243,150 @@ int run_conv(nrs_ctx* ctx, const ConvPlan& p, const float* a_hi, const float* a_
     if (pol.out_lo) ok = ok && tc::encode_tmap_f32(&to_lo, pol.out_lo, 4, odim, ostr, abox);
   }
   NRS_REQUIRE(ctx, ok, NRS_ERR_CUDA, "tc_conv: cuTensorMapEncodeTiled failed");
-  return tc::launch<BN, NPLANES, ConvPolicy>(ctx, ta_hi, ta_lo, tb_hi, tb_lo, pol, tiles_m, p.n_ch_out, 1, taps * (p.a_ch / 32),
-                                             pol.out_hi ? &to_hi : nullptr, pol.out_lo ? &to_lo : nullptr, splits_out);
+  return tc::launch<BN, NPLANES, ConvPolicy>(ctx, ta_hi, ta_lo, tb_hi, tb_lo, pol, tiles_m, p.n_ch_out, 1,
+                                             p.ay.taps * p.ax.taps * pol.cblocks, pol.out_hi ? &to_hi : nullptr,
+                                             pol.out_lo ? &to_lo : nullptr, splits_out);
 }
 
-int conv_common(nrs_ctx* ctx, const ConvPlan& p) {
-  if (!tc::tensor_map_encoder()) return NRS_ERR_UNSUPPORTED;
-  if (p.a_ch % 32 != 0 || p.n_ch_out % 32 != 0 || p.out_w > 128 || p.out_w < 1) return NRS_ERR_UNSUPPORTED;
-  if (p.a_w > 256 * 1024 || p.n_img < 1) return NRS_ERR_UNSUPPORTED;
-  const bool split = ctx->math_mode == NRS_MATH_3XTF32;
-
-  // tile geometry in output space
-  ConvPolicy pol{};
-  pol.Wt = p.out_w;
-  pol.Ht = 128 / pol.Wt;
-  if (pol.Ht > p.out_h) pol.Ht = p.out_h;
-  pol.Nt = 1;
-  if (pol.Ht == p.out_h) {
-    pol.Nt = 128 / (pol.Wt * pol.Ht);
-    if (pol.Nt > p.n_img) pol.Nt = p.n_img;
-    if (pol.Nt < 1) pol.Nt = 1;
+// Pixel tile: the Wt x Ht x Nt box of at most 128 pixels (a box side times the activation step may not exceed
+// TMA's 256) that covers the output in the fewest tiles; among equals the widest, whose stores have the longest runs.
+void plan_pixel_tile(const ConvPlan& p, ConvPolicy* pol) {
+  const int lim = 256 / p.ax.in_step < tc::BM ? 256 / p.ax.in_step : tc::BM;
+  const int lim_y = 256 / p.ay.in_step;
+  long best = -1;
+  for (int tx = (p.ax.len + lim - 1) / lim, end = tx + 3; tx < end && tx <= p.ax.len; ++tx) {
+    const int Wt = (p.ax.len + tx - 1) / tx;
+    int Ht = tc::BM / Wt;
+    if (Ht > p.ay.len) Ht = p.ay.len;
+    if (Ht > lim_y) Ht = lim_y;
+    int Nt = 1;
+    if (Ht == p.ay.len && Wt == p.ax.len) {
+      Nt = tc::BM / (Wt * Ht);
+      if (Nt > p.n_img) Nt = p.n_img;
+    }
+    const int nx = (p.ax.len + Wt - 1) / Wt, ny = (p.ay.len + Ht - 1) / Ht;
+    const long tiles = (long)nx * ny * ((p.n_img + Nt - 1) / Nt);
+    if (best < 0 || tiles < best) {
+      best = tiles;
+      pol->Wt = Wt; pol->Ht = Ht; pol->Nt = Nt; pol->tiles_x = nx; pol->tiles_y = ny;
+    }
   }
-  // keep every TMA box inside the tensor's extents (only the origin may leave it)
-  if (pol.Wt > p.a_w || pol.Ht > p.a_h || pol.Nt > p.n_img) return NRS_ERR_UNSUPPORTED;
-  pol.tiles_y = (p.out_h + pol.Ht - 1) / pol.Ht;
-  const long tiles_m = (long)((p.n_img + pol.Nt - 1) / pol.Nt) * pol.tiles_y;
+}
+
+// Column tile.  Clocks of one 32-element K-block of a tile, from in-kernel measurements of the issuing thread
+// (4 K-steps of 8): 128 columns 1060, 64 columns 832, 32 columns 690, and about as many again per tile for the
+// accumulator's way out.  The width with the least (waves of the grid) x (clocks per tile) is taken: wide tiles for
+// large outputs, narrower ones where they fill SMs that would idle or where a ragged channel count would pad.
+int plan_column_tile(const nrs_ctx* ctx, long tiles_m, int n_ch_out, int kblocks) {
+  const int width[3] = {128, 64, 32}, kb_clk[3] = {1060, 832, 690}, tile_clk[3] = {2600, 1700, 1300};
+  int best = 128;
+  double best_t = -1.0;
+  for (int i = 0; i < 3; ++i) {
+    if (width[i] > 32 && width[i] / 2 >= n_ch_out) continue;   // half of the tile or more would be padding
+    const long tiles = tiles_m * ((n_ch_out + width[i] - 1) / width[i]);
+    const double waves = (double)((tiles + ctx->sm_count - 1) / ctx->sm_count);
+    const double t = waves * ((double)kblocks * kb_clk[i] + tile_clk[i]);
+    if (best_t < 0.0 || t < best_t) { best_t = t; best = width[i]; }
+  }
+  return best;
+}
+
+int conv_common(nrs_ctx* ctx, ConvPlan& p) {
+  if (p.ax.len < 1 || p.ay.len < 1 || p.ax.taps < 1 || p.ay.taps < 1) return NRS_OK;
+  const bool split = ctx->math_mode == NRS_MATH_3XTF32;
+  ConvPolicy pol{};
+  plan_pixel_tile(p, &pol);
+  const long tiles_m = (long)((p.n_img + pol.Nt - 1) / pol.Nt) * pol.tiles_y * pol.tiles_x;
   if (tiles_m > 2147483647L) return NRS_ERR_UNSUPPORTED;
+  pol.sub_h = p.ay.len; pol.sub_w = p.ax.len;
   pol.out_h = p.out_h; pol.out_w = p.out_w; pol.n_img = p.n_img; pol.n_ch_out = p.n_ch_out;
-  pol.cblocks = p.a_ch / 32; pol.kw_taps = p.kw;
-  pol.sgn = p.sgn; pol.base_y = p.base; pol.base_x = p.base;
+  pol.out_step = p.ay.step; pol.out_y0 = p.ay.first; pol.out_x0 = p.ax.first;
+  pol.cblocks = (p.a_ch + 31) / 32; pol.tap_cols = p.ax.taps;
+  pol.in_step = p.ay.in_step;
+  pol.sgn = p.sgn; pol.base_y = p.ay.base; pol.base_x = p.ax.base;
+  pol.w_tap0 = p.ay.tap0 * p.kw + p.ax.tap0; pol.w_tap_row = p.ay.tap_step * p.kw; pol.w_tap_col = p.ax.tap_step;
   pol.out = p.out; pol.bias = p.bias; pol.act = p.act; pol.accumulate = p.accumulate;
   pol.slice_bytes = (uint32_t)(pol.Wt * pol.Ht * pol.Nt) * 128u;
-  auto extras = ctx->out_extras.find(p.out);
+  // Requests of the caller are honoured where this launch writes every pixel of the output (planes: whole
+  // 32-channel blocks); the caller finds the others still registered and does the work itself.
+  const bool whole = pol.out_step == 1 && p.n_ch_out % 32 == 0;
+  auto extras = whole ? ctx->out_extras.find(p.out) : ctx->out_extras.end();
   if (extras != ctx->out_extras.end()) {
     const NrsOutExtras& e = extras->second;
-    if (e.relu_mask_src && p.accumulate) return NRS_ERR_UNSUPPORTED;   // the mask would hit the old content too
-    if (e.lo && !split) return NRS_ERR_UNSUPPORTED;
-    pol.mask_src = e.relu_mask_src; pol.out_hi = e.hi; pol.out_lo = e.lo;
+    if ((e.relu_mask_src && p.accumulate) ||   // the mask would hit the old content too
+        (e.lo && !split)) {
+      extras = ctx->out_extras.end();
+    } else {
+      pol.mask_src = e.relu_mask_src; pol.out_hi = e.hi; pol.out_lo = e.lo;
+    }
   }
   auto colsum = ctx->colsum_requests.find(p.out);
-  if (colsum != ctx->colsum_requests.end() && !p.accumulate && tiles_m * 4 <= colsum->second.cap_rows)
+  if (whole && colsum != ctx->colsum_requests.end() && !p.accumulate && tiles_m * 4 <= colsum->second.cap_rows)
     pol.colsum_partial = colsum->second.partial;
 
   // stage the activation: per image [C][H*W] -> [H*W][C] planes
-  const size_t a_plane = (size_t)p.n_img * p.a_h * p.a_w * p.a_ch;
-  const size_t w_plane = (size_t)p.co * p.ci * p.kh * p.kw;
-  void *a_hi = nullptr, *a_lo = nullptr, *w_hi = nullptr, *w_lo = nullptr;
+  void *a_hi = nullptr, *a_lo = nullptr;
   int st = NRS_OK;
   const NrsPlanes* ready = nrs_planes_find(ctx, p.act_src, split);
   if (ready) {
     a_hi = ready->hi;
     a_lo = ready->lo;
   } else {
+    const size_t a_plane = (size_t)p.n_img * p.a_h * p.a_w * nrs_plane_ld(p.a_ch);
     st = nrs_ws_slot(ctx, NRS_WS_A_HI, a_plane * sizeof(float), &a_hi);
     if (st == NRS_OK && split) st = nrs_ws_slot(ctx, NRS_WS_A_LO, a_plane * sizeof(float), &a_lo);
-    if (st != NRS_OK) return st;
-    const size_t img = (size_t)p.a_h * p.a_w * p.a_ch;
-    st = nrs_tc_stage(ctx, p.act_src, (float*)a_hi, (float*)a_lo, p.a_h * p.a_w, p.a_ch, p.a_ch, p.n_img, img, img, true);
+    if (st == NRS_OK) st = nrs_tc_stage_image(ctx, p.act_src, (float*)a_hi, (float*)a_lo, p.n_img, p.a_ch, p.a_h * p.a_w);
     if (st != NRS_OK) return st;
   }
   const NrsWeightPlanes* wp = nrs_weight_planes_find(ctx, p.w, p.for_dgrad ? NRS_WF_CONV_DGRAD : NRS_WF_CONV_FWD);
-  if (wp && wp->co == p.co && wp->ci == p.ci && wp->taps == p.kh * p.kw) {   // staged ahead with the rest of the model's weights
-    w_hi = wp->hi;
-    w_lo = wp->lo;
+  if (p.w_hi) {
+  } else if (wp && wp->co == p.co && wp->ci == p.ci && wp->taps == p.kh * p.kw) {   // staged ahead with the rest of the model's weights
+    p.w_hi = wp->hi;
+    p.w_lo = wp->lo;
   } else {
+    void *w_hi = nullptr, *w_lo = nullptr;
+    const size_t w_plane = (size_t)p.n_ch_out * p.kh * p.kw * pol.cblocks * 32;
     st = nrs_ws_slot(ctx, NRS_WS_B_HI, w_plane * sizeof(float), &w_hi);
     if (st == NRS_OK && split) st = nrs_ws_slot(ctx, NRS_WS_B_LO, w_plane * sizeof(float), &w_lo);
     if (st != NRS_OK) return st;
     st = nrs_tc_stage_conv_weight(ctx, p.w, (float*)w_hi, (float*)w_lo, p.co, p.ci, p.kh, p.kw, p.for_dgrad);
     if (st != NRS_OK) return st;
+    p.w_hi = w_hi;
+    p.w_lo = w_lo;
   }
 
-  int bn = p.n_ch_out % 128 == 0 ? 128 : (p.n_ch_out % 64 == 0 ? 64 : 32);
-  // Few tiles (small batches): 64-column tiles before a K-split, whose second pass costs more than the narrower
-  // tile loses and cannot produce the per-tile channel sums — taken while 128-wide tiles would leave more than a
-  // third of the SMs without one.
-  if (bn == 128 && (long)tiles_m * (p.n_ch_out / 128) * 3 < 2L * ctx->sm_count) bn = 64;
   if (extras != ctx->out_extras.end()) ctx->out_extras.erase(extras);   // honoured from here on
   int splits = 0;
 #define NRS_RUN(BN_)                                                                                                     \
-  st = split ? run_conv<BN_, 2>(ctx, p, (const float*)a_hi, (const float*)a_lo, (const float*)w_hi, (const float*)w_lo, pol, (int)tiles_m, &splits) \
-             : run_conv<BN_, 1>(ctx, p, (const float*)a_hi, nullptr, (const float*)w_hi, nullptr, pol, (int)tiles_m, &splits)
-  if (bn == 128) { NRS_RUN(128); }
-  else if (bn == 64) { NRS_RUN(64); }
-  else { NRS_RUN(32); }
+  st = split ? run_conv<BN_, 2>(ctx, p, (const float*)a_hi, (const float*)a_lo, (const float*)p.w_hi, (const float*)p.w_lo, pol, (int)tiles_m, &splits) \
+             : run_conv<BN_, 1>(ctx, p, (const float*)a_hi, nullptr, (const float*)p.w_hi, nullptr, pol, (int)tiles_m, &splits)
+  switch (plan_column_tile(ctx, tiles_m, p.n_ch_out, p.ay.taps * p.ax.taps * pol.cblocks)) {
+    case 128: NRS_RUN(128); break;
+    case 64: NRS_RUN(64); break;
+    default: NRS_RUN(32); break;
+  }
 #undef NRS_RUN
   // channel sums come from the direct epilogue only (a K-split stores through the reduce kernel)
   if (st == NRS_OK && pol.colsum_partial && splits == 1) colsum->second.rows = (int)tiles_m * 4;
   return st;
 }
 
+// Strides beyond TMA's element-stride limit keep the FFMA kernels.
+bool tensor_core_conv(int stride) { return tc::tensor_map_encoder() && stride <= 8; }
+
 }  // namespace
 
 // y = act(conv(x, w) + b); NRS_ERR_UNSUPPORTED when the shape is outside this kernel's range.
 int nrs_tc_conv_fwd(nrs_ctx* ctx, const float* x, const float* w, const float* b, float* y, int n, int ci, int h,
                     int wd, int co, int kh, int kw, int stride, int pad, int act) {
-  if (stride != 1) return NRS_ERR_UNSUPPORTED;
+  if (!tensor_core_conv(stride)) return NRS_ERR_UNSUPPORTED;
   ConvPlan p{};
   p.act_src = x; p.n_img = n; p.a_ch = ci; p.a_h = h; p.a_w = wd;
   p.w = w; p.co = co; p.ci = ci; p.kh = kh; p.kw = kw; p.for_dgrad = 0;
-  p.out = y; p.n_ch_out = co; p.out_h = h + 2 * pad - kh + 1; p.out_w = wd + 2 * pad - kw + 1;
-  p.sgn = 1; p.base = -pad;
+  p.out = y; p.n_ch_out = co; p.out_h = (h + 2 * pad - kh) / stride + 1; p.out_w = (wd + 2 * pad - kw) / stride + 1;
+  p.sgn = 1;
+  p.ay = ConvAxis{p.out_h, 1, 0, kh, 0, 1, stride, -pad};
+  p.ax = ConvAxis{p.out_w, 1, 0, kw, 0, 1, stride, -pad};
   p.bias = b; p.act = act; p.accumulate = 0;
   return conv_common(ctx, p);
 }
@@ -277,12 +394,43 @@ int nrs_tc_conv_fwd(nrs_ctx* ctx, const float* x, const float* w, const float* b
 // dx (+)= conv_transpose(dy, w)
 int nrs_tc_conv_dgrad(nrs_ctx* ctx, const float* w, const float* dy, float* dx, int n, int ci, int h, int wd, int co,
                       int kh, int kw, int stride, int pad, int accumulate) {
-  if (stride != 1) return NRS_ERR_UNSUPPORTED;
+  if (!tensor_core_conv(stride)) return NRS_ERR_UNSUPPORTED;
   ConvPlan p{};
-  p.act_src = dy; p.n_img = n; p.a_ch = co; p.a_h = h + 2 * pad - kh + 1; p.a_w = wd + 2 * pad - kw + 1;
+  p.act_src = dy; p.n_img = n; p.a_ch = co; p.a_h = (h + 2 * pad - kh) / stride + 1; p.a_w = (wd + 2 * pad - kw) / stride + 1;
   p.w = w; p.co = co; p.ci = ci; p.kh = kh; p.kw = kw; p.for_dgrad = 1;
   p.out = dx; p.n_ch_out = ci; p.out_h = h; p.out_w = wd;
-  p.sgn = -1; p.base = pad;
+  p.sgn = -1;
   p.bias = nullptr; p.act = NRS_ACT_NONE; p.accumulate = accumulate;
-  return conv_common(ctx, p);
+  // Residue r = (y + pad) % stride: its pixels are y = u*stride + first, its taps r, r + stride, ..., and tap t of
+  // them reads dy row u + (first + pad - r)/stride - t.
+  auto axis = [&](int r, int extent, int k) {
+    const int first = ((r - pad) % stride + stride) % stride;
+    return ConvAxis{first < extent ? (extent - first + stride - 1) / stride : 0, stride, first,
+                    r < k ? (k - r + stride - 1) / stride : 0, r, stride, 1, (first + pad - r) / stride};
+  };
+  if (stride > kh || stride > kw) {   // some residues meet no tap: their pixels receive no gradient
+    if (!accumulate) NRS_CUDA(ctx, cudaMemsetAsync(dx, 0, (size_t)n * ci * h * wd * sizeof(float), ctx->stream));
+  }
+  // the residues share dy's planes: staged once here unless the caller left them with the context
+  const bool split = ctx->math_mode == NRS_MATH_3XTF32;
+  bool lent = false;
+  if (stride > 1 && !nrs_planes_find(ctx, dy, split)) {
+    void *hi = nullptr, *lo = nullptr;
+    const size_t plane = (size_t)n * p.a_h * p.a_w * nrs_plane_ld(co);
+    int st = nrs_ws_slot(ctx, NRS_WS_A_HI, plane * sizeof(float), &hi);
+    if (st == NRS_OK && split) st = nrs_ws_slot(ctx, NRS_WS_A_LO, plane * sizeof(float), &lo);
+    if (st == NRS_OK) st = nrs_tc_stage_image(ctx, dy, (float*)hi, (float*)lo, n, co, p.a_h * p.a_w);
+    if (st != NRS_OK) return st;
+    ctx->plane_hints[dy] = NrsPlanes{(float*)hi, (float*)lo, split ? 1 : 0};
+    lent = true;
+  }
+  int st = NRS_OK;
+  for (int ry = 0; ry < stride && st == NRS_OK; ++ry)
+    for (int rx = 0; rx < stride && st == NRS_OK; ++rx) {
+      p.ay = axis(ry, h, kh);
+      p.ax = axis(rx, wd, kw);
+      st = conv_common(ctx, p);
+    }
+  if (lent) ctx->plane_hints.erase(dy);
+  return st;
 }

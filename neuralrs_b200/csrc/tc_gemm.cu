@@ -27,8 +27,11 @@ struct GemmPolicy {
   static constexpr bool kCanEmit = false;
 
   __device__ __forceinline__ uint32_t a_slice_bytes() const { return tc::BM * tc::BK * 4; }
-  __device__ __forceinline__ void load_a(void* dst, const CUtensorMap* tm, uint64_t* bar, int kb, int tile_m, int batch) const {
-    tc::tma_load_3d(dst, tm, bar, kb * tc::BK, tile_m * tc::BM, batch);
+  struct Cursor { int b_col, row, batch; };
+  __device__ __forceinline__ Cursor cursor(int tile_m, int batch, int kb) const { return Cursor{kb * tc::BK, tile_m * tc::BM, batch}; }
+  __device__ __forceinline__ void advance(Cursor& c) const { c.b_col += tc::BK; }
+  __device__ __forceinline__ void load_a(void* dst, const CUtensorMap* tm, uint64_t* bar, const Cursor& c) const {
+    tc::tma_load_3d(dst, tm, bar, c.b_col, c.row, c.batch);
   }
   __device__ __forceinline__ void store(int tile_m, int batch, int row, int n, float v) const {
     const int m = tile_m * tc::BM + row;
@@ -40,11 +43,16 @@ struct GemmPolicy {
     if (beta != 0.0f) v += beta * *dst;
     *dst = v;
   }
+  struct Row { bool live; size_t off; };   // an accumulator row: is there one in C, and where
+  __device__ __forceinline__ Row row(int tile_m, int batch, int r) const {
+    const int m = tile_m * tc::BM + r;
+    return Row{m < M, (size_t)batch * batch_stride + (size_t)m * N};
+  }
   // 32 consecutive columns [nb, nb+32) of one accumulator row.
-  __device__ __forceinline__ void epilogue(int tile_m, int batch, int row, int nb, int ncols, const uint32_t (&r)[32]) const {
-    const int m = tile_m * tc::BM + row;
-    if (m >= M || nb >= N) return;
-    float* crow = C + (size_t)batch * batch_stride + (size_t)m * N;
+  __device__ __forceinline__ void epilogue(const Row& rw, int nb, int ncols, const uint32_t (&r)[32]) const {
+    if (!rw.live || nb >= N) return;
+    float* crow = C + rw.off;
+    float* prow = pre + rw.off;
     if (vec_ok && ncols == 32 && nb + 32 <= N) {
 #pragma unroll
       for (int j = 0; j < 32; j += 4) {
@@ -54,7 +62,7 @@ struct GemmPolicy {
           const float4 bv = *reinterpret_cast<const float4*>(bias + nb + j);
           v.x += bv.x; v.y += bv.y; v.z += bv.z; v.w += bv.w;
         }
-        if (pre) *reinterpret_cast<float4*>(pre + (size_t)batch * batch_stride + (size_t)m * N + nb + j) = v;
+        if (pre) *reinterpret_cast<float4*>(prow + nb + j) = v;
         v.x = nrs_apply_act(v.x, act); v.y = nrs_apply_act(v.y, act);
         v.z = nrs_apply_act(v.z, act); v.w = nrs_apply_act(v.w, act);
         float4* dst = reinterpret_cast<float4*>(crow + nb + j);
@@ -71,7 +79,7 @@ struct GemmPolicy {
         if (j < ncols && n < N) {
           float v = __uint_as_float(r[j]);
           if (bias) v += bias[n];
-          if (pre) pre[(size_t)batch * batch_stride + (size_t)m * N + n] = v;
+          if (pre) prow[n] = v;
           v = nrs_apply_act(v, act);
           if (beta != 0.0f) v += beta * crow[n];
           crow[n] = v;
@@ -92,21 +100,22 @@ struct Operand {
 // Brings one operand into K-major planes.  stored_kmajor: memory is [rows][K]; else [K][rows].
 int prepare_operand(nrs_ctx* ctx, const float* src, int rows, int K, int batch, bool stored_kmajor, bool split,
                     int ws_hi, int ws_lo, Operand* out, bool is_weight) {
+  const int ldk = nrs_plane_ld(K);   // TMA zero-fills what a K-block reads beyond K
   if (batch == 1) {
-    const int ldk = (K + 31) / 32 * 32;
     // a weight staged ahead with the rest of the model's (weight_set.cu) ...
     if (is_weight) {
       const NrsWeightPlanes* wp = nrs_weight_planes_find(ctx, src, stored_kmajor ? NRS_WF_LINEAR_ROWS : NRS_WF_LINEAR_T);
       if (wp && wp->rows == rows && wp->K == K) {
-        *out = Operand{wp->hi, wp->lo, ldk, ldk, (size_t)rows * ldk};
+        const int ldw = (K + 31) / 32 * 32;
+        *out = Operand{wp->hi, wp->lo, ldw, ldw, (size_t)rows * ldw};
         return NRS_OK;
       }
     }
     // ... or an activation whose [rows][K] planes its producer or an earlier consumer left with the context
-    if (stored_kmajor && K == ldk) {
+    if (stored_kmajor) {
       const NrsPlanes* ready = nrs_planes_find(ctx, src, split);
       if (ready && ready->rows == rows && ready->cols == K) {
-        *out = Operand{ready->hi, ready->lo, ldk, ldk, (size_t)rows * ldk};
+        *out = Operand{ready->hi, ready->lo, ldk, K, (size_t)rows * ldk};
         return NRS_OK;
       }
     }
@@ -116,7 +125,6 @@ int prepare_operand(nrs_ctx* ctx, const float* src, int rows, int K, int batch, 
     *out = Operand{src, nullptr, K, K, (size_t)rows * K};
     return NRS_OK;
   }
-  const int ldk = (K + 31) / 32 * 32;
   const size_t plane = (size_t)rows * ldk;
   void *phi = nullptr, *plo = nullptr;
   int st = nrs_ws_slot(ctx, ws_hi, plane * batch * sizeof(float), &phi);
@@ -127,7 +135,7 @@ int prepare_operand(nrs_ctx* ctx, const float* src, int rows, int K, int batch, 
   }
   st = nrs_tc_stage(ctx, src, (float*)phi, (float*)plo, rows, K, ldk, batch, (size_t)rows * K, plane, !stored_kmajor);
   if (st != NRS_OK) return st;
-  *out = Operand{(const float*)phi, (const float*)plo, ldk, ldk, plane};
+  *out = Operand{(const float*)phi, (const float*)plo, ldk, K, plane};
   return NRS_OK;
 }
 

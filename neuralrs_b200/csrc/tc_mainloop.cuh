@@ -150,18 +150,22 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
         const int kb_begin = split * sp.kb_per_split;
         const int kb_end = min(sp.kb_total, kb_begin + sp.kb_per_split);
         const int n0 = tile_n * BN;
+        // Where the K-slices of this tile lie, stepped along instead of recomputed (the divisions of a recomputation per
+        // slice and plane made the one producing thread the bottleneck: 58 -> 72 us on a 64-channel convolution).
+        typename Policy::Cursor cur = pol.cursor(tile_m, batch, kb_begin);
         for (int kb = kb_begin; kb < kb_end; ++kb, ++it) {
           const int s = it % L::kStages;
           const uint32_t ph = (it / L::kStages) & 1u;
           if (!mbar_wait(&empty_bar[s], ph ^ 1u)) { atomicExch(err_flag, kErrProducerWait); ok = false; break; }
           uint8_t* st = smem + s * L::kStage;
           mbar_expect_tx(&full_bar[s], stage_bytes);
-          pol.load_a(st, &tm_a_hi, &full_bar[s], kb, tile_m, batch);
-          tma_load_3d(st + L::kATile, &tm_b_hi, &full_bar[s], kb * BK, n0, batch);
+          pol.load_a(st, &tm_a_hi, &full_bar[s], cur);
+          tma_load_3d(st + L::kATile, &tm_b_hi, &full_bar[s], cur.b_col, n0, batch);
           if (NPLANES == 2) {
-            tma_load_3d(st + L::kATile + L::kBTile, &tm_b_lo, &full_bar[s], kb * BK, n0, batch);
-            pol.load_a(st + L::kATile + 2 * L::kBTile, &tm_a_lo, &full_bar[s], kb, tile_m, batch);
+            tma_load_3d(st + L::kATile + L::kBTile, &tm_b_lo, &full_bar[s], cur.b_col, n0, batch);
+            pol.load_a(st + L::kATile + 2 * L::kBTile, &tm_a_lo, &full_bar[s], cur);
           }
+          pol.advance(cur);
         }
       }
       if (!ok) {
@@ -228,6 +232,7 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
       const int batch = z / sp.splits, split = z - batch * sp.splits;
       const int n0 = tile_n * BN;
       const uint32_t buf = local & 1u, use = local >> 1;
+      const typename Policy::Row rw = pol.row(tile_m, batch, row);   // index arithmetic under the main loop
       if (!mbar_wait(&acc_full[buf], use & 1u)) {
         if (lane == 0) atomicExch(err_flag, kErrEpilogueWait);
         break;
@@ -253,7 +258,8 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
           __syncwarp();
           if (lane == 0) mbar_arrive(&acc_empty[buf]);
         }
-        const int ncols = (BN - c * 32) < 32 ? (BN - c * 32) : 32;
+        if (n0 + c * 32 >= sp.n_total) continue;   // padding columns of a ragged last tile
+        [[maybe_unused]] const int ncols = (BN - c * 32) < 32 ? (BN - c * 32) : 32;
         if (sp.splits > 1) {
           float* dst = sp.partial + (((size_t)split * sp.batches + batch) * sp.rows_total + (size_t)tile_m * BM + row) * sp.n_total;
 #pragma unroll
@@ -263,7 +269,7 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
           }
         } else if constexpr (Policy::kCanEmit) {
           float v[32];
-          pol.epilogue(tile_m, batch, row, n0 + c * 32, ncols, r, v);
+          pol.epilogue(rw, n0 + c * 32, r, v);
           if (float* cs = pol.colsum_row(tile_m, q)) {
             // Sum over this warp's 32 rows, one channel per lane: a 32 x 32 transpose-reduce in 31
             // shuffles (each stage halves the values a lane holds; fixed order, deterministic).
@@ -304,15 +310,13 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
             mbar_arrive(&emit_bar[1]);
             if (emit_issuer) {
               if (!mbar_wait(&emit_bar[1], ph)) { atomicExch(err_flag, kErrEpilogueWait); ok = false; break; }
-              int c1, c2, c3;
-              pol.out_origin(tile_m, &c1, &c2, &c3);
-              tma_store_4d(&tm_out_hi, emit_tile, n0 + c * 32, c1, c2, c3);
-              if (NPLANES == 2 && emit == 2) tma_store_4d(&tm_out_lo, emit_tile + BM * 128, n0 + c * 32, c1, c2, c3);
+              tma_store_4d(&tm_out_hi, emit_tile, n0 + c * 32, rw.x0, rw.y0, rw.n0);
+              if (NPLANES == 2 && emit == 2) tma_store_4d(&tm_out_lo, emit_tile + BM * 128, n0 + c * 32, rw.x0, rw.y0, rw.n0);
               bulk_commit();
             }
           }
         } else {
-          pol.epilogue(tile_m, batch, row, n0 + c * 32, ncols, r);
+          pol.epilogue(rw, n0 + c * 32, ncols, r);
         }
       }
     }
@@ -434,10 +438,12 @@ int launch(nrs_ctx* ctx, const CUtensorMap& ta_hi, const CUtensorMap& ta_lo, con
 }  // namespace tc
 
 // Operand staging (tc_stage.cu).  Planes are [batch][rows][ldk] f32 with ldk a multiple of
-// 32 and zeros beyond K; `lo == nullptr` means no split (hi = the values themselves).
+// 8 and zeros beyond K; `lo == nullptr` means no split (hi = the values themselves).
 // src_k_by_rows: the source is stored [K][rows] (transposed) instead of [rows][K].
 int nrs_tc_stage(nrs_ctx* ctx, const float* src, float* hi, float* lo, int rows, int K, int ldk, int batch,
                  size_t src_bstride, size_t dst_bstride, bool src_k_by_rows);
+// NHWC planes of an NCHW tensor [n][c][hw], pixel stride nrs_plane_ld(c) floats (zeros between c and there).
+int nrs_tc_stage_image(nrs_ctx* ctx, const float* src, float* hi, float* lo, int n, int c, int hw);
 // Masked gradient staging (see stage_masked_kernel): mode 0 = ReLU mask of dy[n,c,h,w] by y;
 // mode 1 = gradient of a k x k / stride-k max-pool (g[n,c,h/k,w/k], argmax) followed by the ReLU
 // mask, taken from the pooled output y[n,c,h/k,w/k].  nchw_out and the planes are each optional
@@ -452,8 +458,8 @@ int nrs_tc_stage_masked(nrs_ctx* ctx, int mode, const float* g, const float* y, 
 int nrs_tc_pool2_fwd_planes(nrs_ctx* ctx, const float* x, float* y, int32_t* argmax, float* hi, float* lo, int n, int c,
                             int h, int w);
 inline size_t nrs_stage_masked_partial_rows(int n, int h, int w) { return ((size_t)n * (h / 2) * (w / 2) + 31) / 32; }
-// Conv weights w[co][ci][kh][kw] -> K-major planes.
-//  for_dgrad == 0: out[co][(i*kw + j)*ci_n + ci]   (forward B operand)
-//  for_dgrad == 1: out[ci][(i*kw + j)*co_n + co]   (data-gradient B operand)
+// Conv weights w[co][ci][kh][kw] -> K-major planes; the channels of a tap are padded with zeros to a multiple of 32.
+//  for_dgrad == 0: out[co][(i*kw + j)*ceil32(ci) + ci]   (forward B operand)
+//  for_dgrad == 1: out[ci][(i*kw + j)*ceil32(co) + co]   (data-gradient B operand)
 int nrs_tc_stage_conv_weight(nrs_ctx* ctx, const float* w, float* hi, float* lo, int co, int ci, int kh, int kw,
                              int for_dgrad);

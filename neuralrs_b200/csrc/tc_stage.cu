@@ -1,5 +1,5 @@
 // Operand staging for the tensor-core kernels: one memory-bound pass that brings an
-// operand into the K-major, 32-float-aligned form TMA wants and, for 3xTF32,
+// operand into the K-major form with 16-byte aligned rows that TMA wants and, for 3xTF32,
 // splits it into a TF32 high plane (round-to-nearest) and an f32 residual plane
 // (x - hi, exact).  Without the split the single plane is still rounded to nearest
 // TF32: the tensor core truncates its inputs, and truncation's systematic bias
@@ -63,8 +63,8 @@ stage_transpose_kernel(const float* __restrict__ src, float* __restrict__ hi, fl
   }
   __syncthreads();
   for (int i = ty; i < 32; i += 8) {
-    const int r = r0 + i, k = k0 + tx;  // k < ldk always: ldk is a multiple of 32
-    if (r < rows) {
+    const int r = r0 + i, k = k0 + tx;
+    if (r < rows && k < ldk) {
       const float v = tile[tx][i];
       if (SPLIT) {
         const float h = tc::tf32_rn(v);
@@ -77,27 +77,56 @@ stage_transpose_kernel(const float* __restrict__ src, float* __restrict__ hi, fl
   }
 }
 
+// NCHW [n][c][hw] -> NHWC planes [n][hw][ld].  A block takes 32 channels x 128 pixels of an image: 16 independent
+// 128-byte row segments in flight per warp on the way in, full 128-byte lines (32 channels of a pixel, 128-bit
+// stores) on the way out.  HBM-bound: 4 B read and 4 or 8 B written per element.
+constexpr int kStagePx = 128;
+template <bool SPLIT>
+__global__ void __launch_bounds__(256)
+stage_image_kernel(const float* __restrict__ src, float* __restrict__ hi, float* __restrict__ lo, int c_n, int hw, int ld) {
+  NRS_PDL_PROLOGUE();
+  __shared__ float tile[32][kStagePx + 1];
+  const int p0 = blockIdx.x * kStagePx, c0 = blockIdx.y * 32;
+  const size_t img = blockIdx.z;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float v[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {   // warp w: channels w, w+8, ...; four pixel segments each
+    const int c = c0 + warp + 8 * (i >> 2), px = p0 + (i & 3) * 32 + lane;
+    v[i] = (c < c_n && px < hw) ? src[(img * c_n + c) * hw + px] : 0.0f;
+  }
+#pragma unroll
+  for (int i = 0; i < 16; ++i) tile[warp + 8 * (i >> 2)][(i & 3) * 32 + lane] = v[i];
+  __syncthreads();
+  const int cq = (threadIdx.x & 7) * 4;
+  if (c0 + cq >= ld) return;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int pl = k * 32 + (threadIdx.x >> 3);
+    if (p0 + pl >= hw) break;
+    const float4 f = make_float4(tile[cq][pl], tile[cq + 1][pl], tile[cq + 2][pl], tile[cq + 3][pl]);
+    const float4 h = make_float4(tc::tf32_rn(f.x), tc::tf32_rn(f.y), tc::tf32_rn(f.z), tc::tf32_rn(f.w));
+    const size_t o = (img * hw + p0 + pl) * ld + c0 + cq;
+    *reinterpret_cast<float4*>(hi + o) = h;
+    if (SPLIT) *reinterpret_cast<float4*>(lo + o) = make_float4(f.x - h.x, f.y - h.y, f.z - h.z, f.w - h.w);
+  }
+}
+
 template <bool SPLIT>
 __global__ void __launch_bounds__(256)
 stage_conv_weight_kernel(const float* __restrict__ w, float* __restrict__ hi, float* __restrict__ lo, int co_n, int ci_n,
                          int kh, int kw, int for_dgrad) {
   NRS_PDL_PROLOGUE();
-  const size_t total = (size_t)co_n * ci_n * kh * kw;
+  const int taps = kh * kw, rows = for_dgrad ? ci_n : co_n, inner = for_dgrad ? co_n : ci_n, ld = (inner + 31) / 32 * 32;
+  const size_t total = (size_t)rows * ld * taps;
   const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= total) return;
-  // idx enumerates the OUTPUT so writes are coalesced.
-  const int taps = kh * kw;
-  int co, ci, t;
-  if (!for_dgrad) {            // out[co][t*ci_n + ci]
-    ci = (int)(idx % ci_n);
-    t = (int)((idx / ci_n) % taps);
-    co = (int)(idx / ((size_t)ci_n * taps));
-  } else {                     // out[ci][t*co_n + co]
-    co = (int)(idx % co_n);
-    t = (int)((idx / co_n) % taps);
-    ci = (int)(idx / ((size_t)co_n * taps));
-  }
-  const float v = w[((size_t)co * ci_n + ci) * taps + t];
+  // idx enumerates the OUTPUT [row][t*ld + k] so writes are coalesced.
+  const int k = (int)(idx % ld);
+  const int t = (int)((idx / ld) % taps);
+  const int row = (int)(idx / ((size_t)ld * taps));
+  const int co = for_dgrad ? k : row, ci = for_dgrad ? row : k;
+  const float v = k < inner ? w[((size_t)co * ci_n + ci) * taps + t] : 0.0f;
   if (SPLIT) {
     const float h = tc::tf32_rn(v);
     hi[idx] = h;
@@ -340,7 +369,7 @@ int nrs_tc_stage(nrs_ctx* ctx, const float* src, float* hi, float* lo, int rows,
     if (lo) NRS_PDL_LAUNCH((stage_rows_kernel<true>), grid, 256, 0, ctx->stream, src, hi, lo, rows, K, ldk, src_bstride, dst_bstride);
     else NRS_PDL_LAUNCH((stage_rows_kernel<false>), grid, 256, 0, ctx->stream, src, hi, nullptr, rows, K, ldk, src_bstride, dst_bstride);
   } else {
-    dim3 grid((unsigned)((rows + 31) / 32), (unsigned)(ldk / 32), (unsigned)batch);
+    dim3 grid((unsigned)((rows + 31) / 32), (unsigned)((ldk + 31) / 32), (unsigned)batch);
     if (grid.y > 65535 || grid.z > 65535) return NRS_ERR_UNSUPPORTED;
     if (lo) NRS_PDL_LAUNCH((stage_transpose_kernel<true>), grid, 256, 0, ctx->stream, src, hi, lo, rows, K, ldk, src_bstride, dst_bstride);
     else NRS_PDL_LAUNCH((stage_transpose_kernel<false>), grid, 256, 0, ctx->stream, src, hi, nullptr, rows, K, ldk, src_bstride, dst_bstride);
@@ -349,9 +378,21 @@ int nrs_tc_stage(nrs_ctx* ctx, const float* src, float* hi, float* lo, int rows,
   return NRS_OK;
 }
 
+int nrs_tc_stage_image(nrs_ctx* ctx, const float* src, float* hi, float* lo, int n, int c, int hw) {
+  if (n <= 0 || c <= 0 || hw <= 0) return NRS_OK;
+  const int ld = nrs_plane_ld(c);
+  if (hw == 1) return nrs_tc_stage(ctx, src, hi, lo, n, c, ld, 1, 0, 0, false);   // already pixel-major: split only
+  dim3 grid((unsigned)((hw + kStagePx - 1) / kStagePx), (unsigned)((ld + 31) / 32), (unsigned)n);
+  if (grid.y > 65535 || grid.z > 65535) return NRS_ERR_UNSUPPORTED;
+  if (lo) NRS_PDL_LAUNCH((stage_image_kernel<true>), grid, 256, 0, ctx->stream, src, hi, lo, c, hw, ld);
+  else NRS_PDL_LAUNCH((stage_image_kernel<false>), grid, 256, 0, ctx->stream, src, hi, nullptr, c, hw, ld);
+  NRS_LAUNCHED(ctx);
+  return NRS_OK;
+}
+
 int nrs_tc_stage_conv_weight(nrs_ctx* ctx, const float* w, float* hi, float* lo, int co, int ci, int kh, int kw,
                              int for_dgrad) {
-  const size_t total = (size_t)co * ci * kh * kw;
+  const size_t total = (size_t)(for_dgrad ? ci : co) * (((for_dgrad ? co : ci) + 31) / 32 * 32) * kh * kw;
   if (total == 0) return NRS_OK;
   if (lo) NRS_PDL_LAUNCH((stage_conv_weight_kernel<true>), nrs_blocks(total, 256), 256, 0, ctx->stream, w, hi, lo, co, ci, kh, kw, for_dgrad);
   else NRS_PDL_LAUNCH((stage_conv_weight_kernel<false>), nrs_blocks(total, 256), 256, 0, ctx->stream, w, hi, nullptr, co, ci, kh, kw, for_dgrad);

@@ -11,7 +11,11 @@
 // (4 pixels x 128 B per swizzle group), which TMA produces with
 // CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B.  A K-step of 8 pixels is two groups (SBO =
 // 512 B apart); 32-channel blocks sit LBO bytes apart.  The x operand of
-// tap (i,j) is the same box shifted by (i-p, j-p) with TMA zero fill as padding.
+// tap (i,j) is the same box shifted by (i-p, j-p) with TMA zero fill as padding; a stride s
+// makes it take every s-th pixel (the tensor map's element strides).  A box may reach beyond
+// the image: dy is zero there, so those pixels add nothing, and rows of any width are cut into
+// boxes of a multiple of 8 pixels.  Channel counts that are no multiple of 32 are fetched one
+// 32-channel block at a time, with zeros beyond the last channel.
 //
 // The reduction is long (batch x H x W pixels) and the output tiny, so pixels
 // are split across CTAs; each CTA writes its partial tile and a second kernel
@@ -36,14 +40,15 @@ struct WgradParams {
   int kp;                         // pixels per tile = Wt*Ht*Nt (multiple of 8)
   int n_tiles;                    // pixel tiles in all
   int tiles_per_split;
-  int co, ci, kh, kw, pad;
+  int co, ci, kh, kw, pad, stride;
   int taps_per_group, n_groups;   // taps handled by one CTA
-  int cblocks;                    // ci / 32
-  int a_box_blocks;               // 32-channel blocks of dy one box brings (min(4, co/32))
+  int cblocks;                    // ceil(ci / 32)
+  int a_box_blocks;               // 32-channel blocks of dy one box brings (min(4, ceil(co/32)))
+  int ragged_a, ragged_x;         // channel count no multiple of 32: one 4-D box per block instead of one 5-D box for all
   int m_blocks;                   // ceil(co / 128)
   float* partial;                 // [split][m_block][group][col_block][128][group_cols]
-  int group_cols;                 // taps_per_group * ci (1x1 with more than 256 input channels: 256)
-  int col_blocks;                 // 1x1 only: column blocks of 256 input channels, each its own CTA
+  int group_cols;                 // taps_per_group * cblocks * 32 (more than 256 input channels: 256)
+  int col_blocks;                 // more than 256 input channels: column blocks of 256, each its own CTA
   int independent;                // reads nothing the kernel launched just before it wrote (NRS_PDL_PROLOGUE)
   float* direct;                  // 1x1, one split, no accumulation: the tile is the result; written straight to dw[co][ci]
 };
@@ -104,8 +109,8 @@ tc_wgrad_kernel(const __grid_constant__ CUtensorMap tm_dy_hi, const __grid_const
       // planes x (1 + taps) TMA instructions instead of one per block.
       // (a ragged last column block still receives a full box: TMA zero-fills the blocks beyond the tensor)
       const uint32_t tx = NPLANES * (uint32_t)(p.a_box_blocks + ntaps * (p.col_blocks > 1 ? 8 : p.cblocks)) * blk_bytes;
-      int tap_i[9], tap_j[9];
-      for (int t = 0; t < ntaps && t < 9; ++t) { tap_i[t] = (tap0 + t) / p.kw; tap_j[t] = (tap0 + t) - tap_i[t] * p.kw; }
+      const int i_first = tap0 / p.kw, j_first = tap0 - i_first * p.kw;
+      const int x_blocks = p.col_blocks > 1 ? 8 : p.cblocks;
       int issued = 0;
       bool ok = true;
       for (int it = 0; it < ntiles; ++it, ++issued) {
@@ -123,10 +128,23 @@ tc_wgrad_kernel(const __grid_constant__ CUtensorMap tm_dy_hi, const __grid_const
           const CUtensorMap* txm = pl == 0 ? &tm_x_hi : &tm_x_lo;
           uint8_t* a_dst = st + pl * (a_bytes + b_bytes);
           uint8_t* b_dst = a_dst + a_bytes;
-          tc::tma_load_5d(a_dst, tdy, &full_bar[s], 0, x0, y0, n0, mb * kABlocks);
-          for (int t = 0; t < ntaps; ++t)
-            tc::tma_load_5d(b_dst + (size_t)t * p.cblocks * blk_bytes, txm, &full_bar[s], 0, x0 + tap_j[t] - p.pad,
-                            y0 + tap_i[t] - p.pad, n0, cbk * 8);
+          if (p.ragged_a) {
+            for (int b = 0; b < p.a_box_blocks; ++b)
+              tc::tma_load_4d(a_dst + b * blk_bytes, tdy, &full_bar[s], (mb * kABlocks + b) * 32, x0, y0, n0);
+          } else {
+            tc::tma_load_5d(a_dst, tdy, &full_bar[s], 0, x0, y0, n0, mb * kABlocks);
+          }
+          int ti = i_first, tj = j_first;
+          for (int t = 0; t < ntaps; ++t) {
+            const int xx = x0 * p.stride + tj - p.pad, xy = y0 * p.stride + ti - p.pad;
+            uint8_t* dst = b_dst + (size_t)t * p.cblocks * blk_bytes;
+            if (p.ragged_x) {
+              for (int b = 0; b < x_blocks; ++b) tc::tma_load_4d(dst + b * blk_bytes, txm, &full_bar[s], (cbk * 8 + b) * 32, xx, xy, n0);
+            } else {
+              tc::tma_load_5d(dst, txm, &full_bar[s], 0, xx, xy, n0, cbk * 8);
+            }
+            if (++tj == p.kw) { tj = 0; ++ti; }
+          }
         }
       }
       if (!ok) {
@@ -177,7 +195,7 @@ tc_wgrad_kernel(const __grid_constant__ CUtensorMap tm_dy_hi, const __grid_const
     if (ok) {
       tc::tc_fence_after_sync();
       const int row = q * 32 + lane;
-      const int live_cols = p.col_blocks > 1 ? cblocks * 32 : ntaps * p.ci;
+      const int live_cols = p.col_blocks > 1 ? cblocks * 32 : ntaps * p.cblocks * 32;
       float* dst = p.direct ? p.direct + (size_t)(mb * 128 + row) * p.ci + (size_t)cbk * 256
                             : p.partial + (((((size_t)split * p.m_blocks + mb) * p.n_groups + grp) * p.col_blocks + cbk) * 128 + row) *
                                               p.group_cols;
@@ -207,7 +225,7 @@ tc_wgrad_kernel(const __grid_constant__ CUtensorMap tm_dy_hi, const __grid_const
   }
 }
 
-// dw[co][ci][tap] (+)= sum over splits of partial[split][mb][grp][row][t*ci + c].  A block is
+// dw[co][ci][tap] (+)= sum over splits of partial[split][mb][grp][row][t*cblocks*32 + c].  A block is
 // (kReduceThreads / lanes) outputs x `lanes` split lanes: lane y sums splits y, y+lanes, ... and the lanes are
 // combined in lane order through shared memory, so the order of the additions is fixed (bit-reproducible)
 // while the loads of one output are spread over `lanes` threads instead of one serial chain.
@@ -218,7 +236,7 @@ tc_wgrad_reduce_kernel(const WgradParams p, int splits, int lanes, float* __rest
   const int per_block = kReduceThreads / lanes;   // output quads of this block
   const int lane = threadIdx.x / per_block, slot = threadIdx.x - lane * per_block;
   const int taps = p.kh * p.kw;
-  const int cq = p.ci / 4;                        // a thread owns four consecutive input channels (ci % 32 == 0)
+  const int cq = (p.ci + 3) / 4;                  // a thread owns four consecutive input channels (padded in the partials)
   const size_t total = (size_t)p.co * cq * taps;
   const size_t idx = (size_t)blockIdx.x * per_block + slot;
   const bool live = idx < total;
@@ -230,7 +248,7 @@ tc_wgrad_reduce_kernel(const WgradParams p, int splits, int lanes, float* __rest
   const int grp = tap / p.taps_per_group, t = tap - grp * p.taps_per_group;
   const size_t tile = (size_t)128 * p.group_cols;
   const int cbk = p.col_blocks > 1 ? c / 256 : 0;
-  const size_t col = p.col_blocks > 1 ? (size_t)(c - cbk * 256) : (size_t)t * p.ci + c;
+  const size_t col = p.col_blocks > 1 ? (size_t)(c - cbk * 256) : (size_t)t * p.cblocks * 32 + c;
   const size_t off = ((((size_t)mb * p.n_groups + grp) * p.col_blocks + cbk) * 128 + row) * p.group_cols + col;
   const size_t split_stride = (size_t)p.m_blocks * p.n_groups * p.col_blocks * tile;
   float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -251,7 +269,36 @@ tc_wgrad_reduce_kernel(const WgradParams p, int splits, int lanes, float* __rest
   float* dst = dw + ((size_t)co * p.ci + c) * taps + tap;
   const float r[4] = {s.x, s.y, s.z, s.w};
 #pragma unroll
-  for (int k = 0; k < 4; ++k) dst[(size_t)k * taps] = accumulate ? dst[(size_t)k * taps] + r[k] : r[k];
+  for (int k = 0; k < 4; ++k)
+    if (c + k < p.ci) dst[(size_t)k * taps] = accumulate ? dst[(size_t)k * taps] + r[k] : r[k];
+}
+
+// Pixel tile = one TMA box {32 channels, Wt, Ht, Nt} of kp = Wt*Ht*Nt pixels, a multiple of 8 (a K-step) up to 64.
+// Boxes of whole rows, or of a multiple of 8 pixels of a row; the one that walks the fewest pixels, padding included,
+// is taken, where every tile costs about 6 pixels' worth of ring bookkeeping (measured: 16-pixel tiles with a deeper
+// ring are slower, the single producer thread becomes TMA-issue bound) and a ring of fewer than three slots a few
+// percent.  A box may reach past the last image too (a few 1x1 "images").
+void plan_pixel_box(WgradParams* p, int n, int oh, int ow, size_t bytes_per_pixel) {
+  double best = -1.0;
+  for (int c = 0; c <= 8; ++c) {
+    const int Wt = c == 0 ? ow : 8 * c;
+    if (Wt > 64 || Wt * p->stride > 256 || (c > 0 && Wt - ow >= 8)) continue;
+    for (int Ht = 1; Ht <= oh && Wt * Ht <= 64 && Ht * p->stride <= 256; ++Ht) {
+      const bool whole = Ht == oh && Wt >= ow;
+      for (int Nt = 1; Nt <= (whole ? n + 7 : 1) && Wt * Ht * Nt <= 64; ++Nt) {
+        const int kp = Wt * Ht * Nt;
+        if (kp % 8 != 0) continue;
+        const int stages = (int)((200 * 1024) / (bytes_per_pixel * kp));
+        if (stages < 2) continue;
+        const long tiles = (long)((ow + Wt - 1) / Wt) * ((oh + Ht - 1) / Ht) * ((n + Nt - 1) / Nt);
+        const double cost = (double)tiles * (kp + 6) * (stages < 3 ? 1.06 : 1.0);
+        if (best < 0.0 || cost < best) {
+          best = cost;
+          p->Wt = Wt; p->Ht = Ht; p->Nt = Nt; p->kp = kp;
+        }
+      }
+    }
+  }
 }
 
 }  // namespace
@@ -277,48 +324,38 @@ int launch_wgrad(nrs_ctx* ctx, const CUtensorMap* maps, const WgradParams& p, in
 int nrs_tc_conv_wgrad(nrs_ctx* ctx, const float* x, const float* dy, float* dw, int n, int ci, int h, int wd, int co,
                       int kh, int kw, int stride, int pad, int accumulate) {
   if (!tc::tensor_map_encoder()) return NRS_ERR_UNSUPPORTED;
-  if (stride != 1 || ci % 32 != 0 || co % 32 != 0 || n < 1) return NRS_ERR_UNSUPPORTED;
-  if (ci > kMaxN && !(kh == 1 && kw == 1)) return NRS_ERR_UNSUPPORTED;   // wide layers: 1x1 only (column blocks)
-  const int oh = h + 2 * pad - kh + 1, ow = wd + 2 * pad - kw + 1;
-  if (ow > wd || oh > h || ow < 1 || oh < 1 || ow > 64) return NRS_ERR_UNSUPPORTED;
+  if (n < 1 || stride > 8) return NRS_ERR_UNSUPPORTED;
+  const int oh = (h + 2 * pad - kh) / stride + 1, ow = (wd + 2 * pad - kw) / stride + 1;
+  if (ow < 1 || oh < 1) return NRS_ERR_UNSUPPORTED;
   const bool split3 = ctx->math_mode == NRS_MATH_3XTF32;
   const int planes = split3 ? 2 : 1;
 
-  // Pixel tile = one TMA box {32 channels, Wt, Ht, Nt} of about 32 pixels.  (Measured: 16-pixel
-  // tiles with a deeper ring are slower — the single producer thread becomes TMA-issue bound.)
-  const int target = 32;
   WgradParams p{};
-  p.Wt = ow;
-  if (ow > target && ow % target == 0) p.Wt = target;
-  p.tiles_x = ow / p.Wt;
-  p.Ht = target / p.Wt > 1 ? target / p.Wt : 1;
-  if (p.Ht > oh) p.Ht = oh;
-  while ((p.Wt * p.Ht) % 8 != 0 && p.Ht < oh) ++p.Ht;
-  p.Nt = 1;
-  if (p.Ht == oh && p.Wt * p.Ht < target) {
-    p.Nt = target / (p.Wt * p.Ht);
-    if (p.Nt > n) p.Nt = n;
-  }
-  p.kp = p.Wt * p.Ht * p.Nt;
-  if (p.kp % 8 != 0 || p.kp > 64) return NRS_ERR_UNSUPPORTED;
-  p.tiles_y = (oh + p.Ht - 1) / p.Ht;
-  p.n_tiles = ((n + p.Nt - 1) / p.Nt) * p.tiles_y * p.tiles_x;
-  p.co = co; p.ci = ci; p.kh = kh; p.kw = kw; p.pad = pad;
-  p.cblocks = ci / 32;
+  p.co = co; p.ci = ci; p.kh = kh; p.kw = kw; p.pad = pad; p.stride = stride;
+  p.cblocks = (ci + 31) / 32;
+  p.ragged_a = co % 32 != 0;
+  p.ragged_x = ci % 32 != 0;
   p.m_blocks = (co + 127) / 128;
   const int taps = kh * kw;
-  int tpg = ci <= kMaxN ? kMaxN / ci : 1;
+  int tpg = p.cblocks * 32 <= kMaxN ? kMaxN / (p.cblocks * 32) : 1;
   if (tpg > taps) tpg = taps;
   p.n_groups = (taps + tpg - 1) / tpg;
   p.taps_per_group = (taps + p.n_groups - 1) / p.n_groups;
-  p.group_cols = p.taps_per_group * ci;
+  p.group_cols = p.taps_per_group * p.cblocks * 32;
   p.col_blocks = 1;
-  if (ci > kMaxN) {                 // 1x1: the input channels are cut into column blocks of 256, one CTA each
+  if (p.cblocks * 32 > kMaxN) {     // the input channels are cut into column blocks of 256, one CTA each
     p.col_blocks = (ci + kMaxN - 1) / kMaxN;
-    p.n_groups = 1;
+    p.n_groups = taps;
     p.taps_per_group = 1;
     p.group_cols = kMaxN;
   }
+  plan_pixel_box(&p, n, oh, ow, (size_t)planes * (kABlocks + p.group_cols / 32) * 128);
+  if (p.kp == 0) return NRS_ERR_UNSUPPORTED;
+  p.tiles_x = (ow + p.Wt - 1) / p.Wt;
+  p.tiles_y = (oh + p.Ht - 1) / p.Ht;
+  const long n_tiles = (long)((n + p.Nt - 1) / p.Nt) * p.tiles_y * p.tiles_x;
+  if (n_tiles > 2147483647L) return NRS_ERR_UNSUPPORTED;
+  p.n_tiles = (int)n_tiles;
 
   // ring depth from the shared-memory budget
   const size_t stage_bytes = (size_t)planes * (kABlocks + p.group_cols / 32) * p.kp * 128;
@@ -340,14 +377,14 @@ int nrs_tc_conv_wgrad(nrs_ctx* ctx, const float* x, const float* dy, float* dw, 
   if (splits > 65535) return NRS_ERR_UNSUPPORTED;
 
   // workspaces: NHWC planes of dy and x, and the partial tiles
-  const size_t dy_plane = (size_t)n * oh * ow * co, x_plane = (size_t)n * h * wd * ci;
+  const int dy_ld = nrs_plane_ld(co), x_ld = nrs_plane_ld(ci);
+  const size_t dy_plane = (size_t)n * oh * ow * dy_ld, x_plane = (size_t)n * h * wd * x_ld;
   const size_t partial_floats = (size_t)splits * p.m_blocks * p.n_groups * p.col_blocks * 128 * p.group_cols;
   void *dy_hi = nullptr, *dy_lo = nullptr, *x_hi = nullptr, *x_lo = nullptr, *part = nullptr;
   bool may_overlap = ctx->independent_next;   // withdrawn below if this call stages an operand itself
   int st = nrs_ws_slot(ctx, NRS_WS_WGRAD_PARTIAL, partial_floats * sizeof(float), &part);
   if (st != NRS_OK) return st;
   p.partial = (float*)part;
-  const size_t dy_img = (size_t)oh * ow * co, x_img = (size_t)h * wd * ci;
   if (const NrsPlanes* ready = nrs_planes_find(ctx, dy, split3)) {
     dy_hi = ready->hi;
     dy_lo = ready->lo;
@@ -355,9 +392,7 @@ int nrs_tc_conv_wgrad(nrs_ctx* ctx, const float* x, const float* dy, float* dw, 
     may_overlap = false;
     st = nrs_ws_slot(ctx, NRS_WS_A_HI, dy_plane * sizeof(float), &dy_hi);
     if (st == NRS_OK && split3) st = nrs_ws_slot(ctx, NRS_WS_A_LO, dy_plane * sizeof(float), &dy_lo);
-    if (st == NRS_OK)   // a [n, c, 1, 1] tensor is already pixel-major: split only
-      st = oh * ow == 1 ? nrs_tc_stage(ctx, dy, (float*)dy_hi, (float*)dy_lo, n, co, co, 1, 0, 0, false)
-                        : nrs_tc_stage(ctx, dy, (float*)dy_hi, (float*)dy_lo, oh * ow, co, co, n, dy_img, dy_img, true);
+    if (st == NRS_OK) st = nrs_tc_stage_image(ctx, dy, (float*)dy_hi, (float*)dy_lo, n, co, oh * ow);
     if (st != NRS_OK) return st;
   }
   if (const NrsPlanes* ready = nrs_planes_find(ctx, x, split3)) {
@@ -367,28 +402,31 @@ int nrs_tc_conv_wgrad(nrs_ctx* ctx, const float* x, const float* dy, float* dw, 
     may_overlap = false;
     st = nrs_ws_slot(ctx, NRS_WS_B_HI, x_plane * sizeof(float), &x_hi);
     if (st == NRS_OK && split3) st = nrs_ws_slot(ctx, NRS_WS_B_LO, x_plane * sizeof(float), &x_lo);
-    if (st == NRS_OK)
-      st = h * wd == 1 ? nrs_tc_stage(ctx, x, (float*)x_hi, (float*)x_lo, n, ci, ci, 1, 0, 0, false)
-                       : nrs_tc_stage(ctx, x, (float*)x_hi, (float*)x_lo, h * wd, ci, ci, n, x_img, x_img, true);
+    if (st == NRS_OK) st = nrs_tc_stage_image(ctx, x, (float*)x_hi, (float*)x_lo, n, ci, h * wd);
     if (st != NRS_OK) return st;
   }
 
+  // Planes viewed as [channel block][n][h][w][32 channels], the block index outermost, so that one box brings all
+  // blocks; with a ragged channel count as [n][h][w][channels], one block per box.
   CUtensorMap maps[4];
-  p.a_box_blocks = co / 32 < kABlocks ? co / 32 : kABlocks;
-  // planes viewed as [channel block][n][h][w][32 channels]: the block index is the outermost dimension
-  const uint64_t ddim[5] = {32, (uint64_t)ow, (uint64_t)oh, (uint64_t)n, (uint64_t)(co / 32)};
-  const uint64_t dstr[4] = {(uint64_t)co * 4, (uint64_t)ow * co * 4, (uint64_t)oh * ow * co * 4, 128};
-  const uint64_t xdim[5] = {32, (uint64_t)wd, (uint64_t)h, (uint64_t)n, (uint64_t)(ci / 32)};
-  const uint64_t xstr[4] = {(uint64_t)ci * 4, (uint64_t)wd * ci * 4, (uint64_t)h * wd * ci * 4, 128};
-  const uint32_t dbox[5] = {32, (uint32_t)p.Wt, (uint32_t)p.Ht, (uint32_t)p.Nt, (uint32_t)p.a_box_blocks};
-  const uint32_t xbox[5] = {32, (uint32_t)p.Wt, (uint32_t)p.Ht, (uint32_t)p.Nt, (uint32_t)(p.col_blocks > 1 ? 8 : p.cblocks)};
-  bool ok = tc::encode_tmap_f32(&maps[0], dy_hi, 5, ddim, dstr, dbox, true) && tc::encode_tmap_f32(&maps[2], x_hi, 5, xdim, xstr, xbox, true);
-  if (split3) ok = ok && tc::encode_tmap_f32(&maps[1], dy_lo, 5, ddim, dstr, dbox, true) && tc::encode_tmap_f32(&maps[3], x_lo, 5, xdim, xstr, xbox, true);
+  p.a_box_blocks = (co + 31) / 32 < kABlocks ? (co + 31) / 32 : kABlocks;
+  auto encode = [&](CUtensorMap* m, void* base, bool ragged, int c, int ld, int img_h, int img_w, int step, int blocks) {
+    const uint64_t dim[5] = {(uint64_t)(ragged ? c : 32), (uint64_t)img_w, (uint64_t)img_h, (uint64_t)n, (uint64_t)(c / 32)};
+    const uint64_t str[4] = {(uint64_t)ld * 4, (uint64_t)img_w * ld * 4, (uint64_t)img_h * img_w * ld * 4, 128};
+    const uint32_t box[5] = {32, (uint32_t)p.Wt, (uint32_t)p.Ht, (uint32_t)p.Nt, (uint32_t)blocks};
+    const uint32_t es[5] = {1, (uint32_t)step, (uint32_t)step, 1, 1};
+    return tc::encode_tmap_f32(m, base, ragged ? 4 : 5, dim, str, box, true, es);
+  };
+  const int x_blocks = p.col_blocks > 1 ? 8 : p.cblocks;
+  bool ok = encode(&maps[0], dy_hi, p.ragged_a, co, dy_ld, oh, ow, 1, p.a_box_blocks) &&
+            encode(&maps[2], x_hi, p.ragged_x, ci, x_ld, h, wd, stride, x_blocks);
+  if (split3) ok = ok && encode(&maps[1], dy_lo, p.ragged_a, co, dy_ld, oh, ow, 1, p.a_box_blocks) &&
+                   encode(&maps[3], x_lo, p.ragged_x, ci, x_ld, h, wd, stride, x_blocks);
   else { maps[1] = maps[0]; maps[3] = maps[2]; }
   NRS_REQUIRE(ctx, ok, NRS_ERR_CUDA, "tc_wgrad: cuTensorMapEncodeTiled failed");
   p.independent = may_overlap ? 1 : 0;
   // a single split of a 1x1 "convolution" (A^T B) that overwrites its output needs no second pass
-  p.direct = (splits == 1 && taps == 1 && !accumulate && (reinterpret_cast<uintptr_t>(dw) & 15) == 0) ? dw : nullptr;
+  p.direct = (splits == 1 && taps == 1 && ci % 32 == 0 && !accumulate && (reinterpret_cast<uintptr_t>(dw) & 15) == 0) ? dw : nullptr;
 
 #define NRS_WG(PL)                                                                     \
   switch (stages) {                                                                    \
@@ -402,9 +440,9 @@ int nrs_tc_conv_wgrad(nrs_ctx* ctx, const float* x, const float* dy, float* dw, 
 #undef NRS_WG
   if (st != NRS_OK) return st;
   if (p.direct) return NRS_OK;
-  const size_t total = (size_t)co * ci * taps;
+  const size_t total = (size_t)co * ((ci + 3) / 4) * taps;
   const int lanes = reduce_lanes(splits);
-  NRS_PDL_LAUNCH(tc_wgrad_reduce_kernel, nrs_blocks(total / 4, kReduceThreads / lanes), kReduceThreads, 0, ctx->stream, p, splits, lanes, dw,
+  NRS_PDL_LAUNCH(tc_wgrad_reduce_kernel, nrs_blocks(total, kReduceThreads / lanes), kReduceThreads, 0, ctx->stream, p, splits, lanes, dw,
                  accumulate);
   NRS_LAUNCHED(ctx);
   return NRS_OK;
@@ -414,9 +452,9 @@ int nrs_tc_conv_wgrad(nrs_ctx* ctx, const float* x, const float* dy, float* dw, 
 // the reduction index k is the slow index of both operands, which is what the weight-gradient kernel above
 // consumes (a 1x1 convolution over k "pixels": rows = A's columns, columns = B's columns).  The weight
 // gradient of a Linear layer, dW = x^T dz, is this product on the activations' own row-major planes.
-// NRS_ERR_UNSUPPORTED (no error text) unless m and n are multiples of 32 and k of 8.
+// NRS_ERR_UNSUPPORTED (no error text) for products too thin for a 128-row tile.
 int nrs_tc_gemm_tn(nrs_ctx* ctx, int m, int n, int k, const float* a, const float* b, float* c, int accumulate) {
-  if (m % 32 != 0 || n % 32 != 0 || k < 8 || (k < 32 && k % 8 != 0)) return NRS_ERR_UNSUPPORTED;
+  if (m < 32 || n < 32 || k < 8) return NRS_ERR_UNSUPPORTED;
   // Outputs of up to 4 M elements (the Linear layers of the CNN and transformer configurations).  Larger ones
   // (4096 x 4096 hidden layers) stay on the persistent GEMM kernel: its rastered tiles reuse operands through L2,
   // and the transposes it needs are small beside such a product.

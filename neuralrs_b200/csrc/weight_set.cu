@@ -64,27 +64,24 @@ weight_stage_batch_kernel(const WeightJob* __restrict__ jobs, int n_jobs, unsign
       if (r < j.rows) put(j.hi, j.lo, (size_t)r * j.ldk + k0 + tx, tile[tx][i]);
     }
   } else {
-    // convolution weights w[co][ci][tap]: forward out[co][tap*ci_n + ci], data gradient out[ci][tap*co_n + co]
-    const size_t total = (size_t)j.co * j.ci * j.taps;
+    // convolution weights w[co][ci][tap]: forward out[co][tap*ld + ci], data gradient out[ci][tap*ld + co], where ld
+    // is the inner channel count padded with zeros to a multiple of 32
+    const bool fwd = j.form == NRS_WF_CONV_FWD;
+    const int inner = fwd ? j.ci : j.co, ld = (inner + 31) / 32 * 32;
+    const size_t total = (size_t)(fwd ? j.co : j.ci) * ld * j.taps;
     const size_t idx = (size_t)blk * 256 + threadIdx.x;
     if (idx >= total) return;
-    int co, ci, t;
-    if (j.form == NRS_WF_CONV_FWD) {
-      ci = (int)(idx % j.ci);
-      t = (int)((idx / j.ci) % j.taps);
-      co = (int)(idx / ((size_t)j.ci * j.taps));
-    } else {
-      co = (int)(idx % j.co);
-      t = (int)((idx / j.co) % j.taps);
-      ci = (int)(idx / ((size_t)j.co * j.taps));
-    }
-    put(j.hi, j.lo, idx, j.src[((size_t)co * j.ci + ci) * j.taps + t]);
+    const int k = (int)(idx % ld);
+    const int t = (int)((idx / ld) % j.taps);
+    const int row = (int)(idx / ((size_t)ld * j.taps));
+    const int co = fwd ? row : k, ci = fwd ? k : row;
+    put(j.hi, j.lo, idx, k < inner ? j.src[((size_t)co * j.ci + ci) * j.taps + t] : 0.0f);
   }
 }
 
 size_t plane_floats(const NrsWeightDesc& d) {
   if (d.form == NRS_WF_LINEAR_ROWS || d.form == NRS_WF_LINEAR_T) return (size_t)d.rows * ((d.K + 31) / 32 * 32);
-  return (size_t)d.co * d.ci * d.taps;
+  return d.form == NRS_WF_CONV_FWD ? (size_t)d.co * ((d.ci + 31) / 32 * 32) * d.taps : (size_t)d.ci * ((d.co + 31) / 32 * 32) * d.taps;
 }
 
 }  // namespace
@@ -128,7 +125,7 @@ int nrs_weight_set_build(nrs_ctx* ctx, const NrsWeightDesc* descs, int count) {
     j.first_block = block;
     if (d.form == NRS_WF_LINEAR_ROWS) block += (unsigned)(((size_t)d.rows * (j.ldk / 4) + 255) / 256);
     else if (d.form == NRS_WF_LINEAR_T) block += (unsigned)(((d.rows + 31) / 32) * (j.ldk / 32));
-    else block += (unsigned)(((size_t)d.co * d.ci * d.taps + 255) / 256);
+    else block += (unsigned)((plane_floats(d) + 255) / 256);
     jobs.push_back(j);
     ws.job_src.push_back(d.w);
     ws.job_first.push_back(j.first_block);
