@@ -6,6 +6,7 @@
 // re-read from L1), forward and backward share one pass, and the batch mean is
 // reduced on the device in a fixed order.
 #include "nrs_internal.h"
+#include "row_pipe.cuh"
 
 namespace {
 
@@ -19,6 +20,83 @@ __device__ __forceinline__ float warp_sum(float v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
+
+// Batch mean without a second launch: wsum[0..n) (shared memory, one sum per warp or team) -> block, in order ->
+// block_partial[block]; the block that arrives last folds the partials in block order (lane l takes l, l+32, ..., then
+// a butterfly), so the order of the additions is fixed whichever block that is.
+__device__ __forceinline__ void fold_batch_loss(const float* wsum, int n, float* block_partial, unsigned* ticket, float* loss_dev,
+                                                float inv_div) {
+  __shared__ bool last;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    float s = 0.0f;
+    for (int w = 0; w < n; ++w) s += wsum[w];
+    block_partial[blockIdx.x] = s;
+    __threadfence();
+    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last || threadIdx.x >= 32) return;
+  __threadfence();
+  float s = 0.0f;
+  for (unsigned i = threadIdx.x; i < gridDim.x; i += 32) s += __ldcg(block_partial + i);
+  s = warp_sum(s);
+  if (threadIdx.x == 0) {
+    loss_dev[0] = s * inv_div;
+    *ticket = 0;
+  }
+}
+
+// Large batches and odd widths (row_pipe.cuh): logits in the first buffer, the one-hot row (when there is one) in the
+// second; the gradient replaces the logits.
+struct CeOp {
+  const int32_t* labels;
+  float *row_loss, *block_partial, *loss_dev;
+  unsigned* ticket;
+  float inv_div;
+  int has_target;
+  template <int NPL> struct State { float loss; };
+  template <class C, class S> __device__ __forceinline__ void start(const C&, S& s) const { s.loss = 0.0f; }
+  template <int NPL, int VEC, class C, class S>
+  __device__ __forceinline__ void row(const rowpipe::Team& tm, const C& c, S& s, float* buf0, float* buf1, int r) const {
+    float x[NPL], t[NPL], mx = -INFINITY;
+    c.load(buf0, x, -INFINITY);
+    if (has_target) {
+      c.load(buf1, t);
+    } else {
+      const int label = labels[r];
+#pragma unroll
+      for (int i = 0; i < NPL; ++i) t[i] = c.first(i / VEC) + i % VEC == label ? 1.0f : 0.0f;
+    }
+    float v[3] = {0.0f, 0.0f, 0.0f};   // sum exp(x - max), sum t*x, sum t
+#pragma unroll
+    for (int i = 0; i < NPL; ++i)
+      if (c.live(i / VEC)) {
+        mx = fmaxf(mx, x[i]);
+        v[1] += t[i] * x[i];
+        v[2] += t[i];
+      }
+    mx = tm.max(mx);
+#pragma unroll
+    for (int i = 0; i < NPL; ++i)
+      if (c.live(i / VEC)) { x[i] = expf(x[i] - mx); v[0] += x[i]; }
+    tm.sum(v);
+    const float lse = logf(v[0]) + mx, inv_se = 1.0f / v[0];
+#pragma unroll
+    for (int i = 0; i < NPL; ++i) x[i] = (x[i] * inv_se - t[i]) * inv_div;
+    c.store(buf0, x);
+    const float rl = lse * v[2] - v[1];
+    if (row_loss && tm.warp == 0 && tm.lane == 0) row_loss[r] = rl;
+    s.loss += rl;
+  }
+  template <int NPL, int VEC, class C, class S>
+  __device__ __forceinline__ void finish(const rowpipe::Team& tm, const C&, S& s, float* smem, int team, int teams) const {
+    if (!loss_dev) return;
+    if (tm.warp == 0 && tm.lane == 0) smem[team] = s.loss;
+    fold_batch_loss(smem, teams, block_partial, ticket, loss_dev, inv_div);
+  }
+  static size_t finish_bytes(int teams, int) { return (size_t)teams * sizeof(float); }
+};
 
 // One warp per row.  row_loss (optional) gets -sum_c t*(x - lse); grad (optional)
 // gets (softmax - t) * inv_div.  Scalar path (any width / alignment).
@@ -136,30 +214,9 @@ ce_rows_vec_kernel(const float* __restrict__ logits, const float* __restrict__ t
     warp_loss += rl;
   }
   if (!loss_dev) return;
-  // Batch mean without a second launch: warps -> block (warp order) -> block_partial[block]; the block that
-  // arrives last folds the partials in block order (lane l takes l, l+32, ..., then a butterfly), so the order
-  // of the additions is fixed whichever block that is.
   __shared__ float wsum[32];
-  __shared__ bool last;
   if (lane == 0) wsum[threadIdx.x >> 5] = warp_loss;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float s = 0.0f;
-    for (int w = 0; w < warps_per_block; ++w) s += wsum[w];
-    block_partial[blockIdx.x] = s;
-    __threadfence();
-    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
-  }
-  __syncthreads();
-  if (!last || threadIdx.x >= 32) return;
-  __threadfence();
-  float s = 0.0f;
-  for (unsigned i = lane; i < gridDim.x; i += 32) s += __ldcg(block_partial + i);
-  s = warp_sum(s);
-  if (lane == 0) {
-    loss_dev[0] = s * inv_div;
-    *ticket = 0;
-  }
+  fold_batch_loss(wsum, warps_per_block, block_partial, ticket, loss_dev, inv_div);
 }
 
 // loss_dev[0] = (sum_b row_loss[b]) * inv_div, one block, fixed summation tree.
@@ -198,6 +255,23 @@ int run_ce(nrs_ctx* ctx, const char* who, const float* logits, const float* targ
   }
   NRS_REQUIRE(ctx, logits && (target || labels), NRS_ERR_ARG, "%s: null tensor", who);
   const float inv_div = 1.0f / (float)divisor;
+  if (rowpipe::applies(batch, classes, classes % 4 == 0 && classes <= 1024, {logits, target, grad})) {
+    rowpipe::Params p{};
+    p.in[0] = logits; p.in[1] = target;
+    p.n_in = p.n_buf = target ? 2 : 1;
+    p.out[0] = grad;
+    p.rows = batch; p.f = classes;
+    CeOp op{labels, row_loss, nullptr, loss_dev, nullptr, inv_div, target != nullptr};
+    if (loss_dev) {
+      void* ws = nullptr;
+      int st = nrs_workspace(ctx, (size_t)ctx->sm_count * sizeof(float), &ws);
+      if (st == NRS_OK) st = nrs_fold_ticket(ctx, &op.ticket);
+      if (st != NRS_OK) return st;
+      op.block_partial = (float*)ws;
+    }
+    const int st = rowpipe::launch(ctx, p, op);
+    if (st != NRS_ERR_UNSUPPORTED) return st;
+  }
   int blocks = (batch + 7) / 8;
   if (blocks > ctx->sm_count * 8) blocks = ctx->sm_count * 8;
   // wide rows: one resident wave (three blocks of 80 registers per SM) of warps that walk several rows each,

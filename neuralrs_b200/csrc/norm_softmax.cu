@@ -13,9 +13,158 @@
 // softmax_forward / softmax_backward (src/cuda/graph/softmax.rs:12-35); CPU
 // semantics src/nn/normalization.rs:38-103, src/autograd/graph/softmax.rs:23-60.
 #include "nrs_internal.h"
+#include "row_pipe.cuh"
 #include "tc_common.cuh"
 
 namespace {
+
+// ------------------------------------------------------------------ large tensors and odd widths (row_pipe.cuh)
+struct NoState {};
+
+// x = a (+ b); xhat replaces a, y = gamma*xhat + beta goes to the second buffer.
+struct LnFwdOp {
+  const float *gamma, *beta;
+  float* istd_out;
+  float eps;
+  int has_b;
+  template <int NPL> struct State { float gamma[NPL], beta[NPL]; };   // the lane's columns, for all rows it meets
+  template <class C, class S> __device__ __forceinline__ void start(const C& c, S& s) const {
+    c.load(gamma, s.gamma);
+    c.load(beta, s.beta);
+  }
+  template <int NPL, int VEC, class C, class S>
+  __device__ __forceinline__ void row(const rowpipe::Team& tm, const C& c, S& s, float* buf0, float* buf1, int r) const {
+    float v[NPL], t[1] = {0.0f};
+    c.load(buf0, v);
+    if (has_b) {
+      float w[NPL];
+      c.load(buf1, w);
+#pragma unroll
+      for (int i = 0; i < NPL; ++i) v[i] += w[i];
+    }
+#pragma unroll
+    for (int i = 0; i < NPL; ++i) t[0] += v[i];
+    tm.sum(t);
+    const float mean = t[0] / (float)c.f;
+    t[0] = 0.0f;
+#pragma unroll
+    for (int i = 0; i < NPL; ++i) {
+      v[i] -= mean;
+      if (c.live(i / VEC)) t[0] += v[i] * v[i];
+    }
+    tm.sum(t);
+    const float istd = 1.0f / sqrtf(t[0] / (float)c.f + eps);
+    if (istd_out && tm.warp == 0 && tm.lane == 0) istd_out[r] = istd;
+#pragma unroll
+    for (int i = 0; i < NPL; ++i) v[i] *= istd;
+    c.store(buf0, v);
+#pragma unroll
+    for (int i = 0; i < NPL; ++i) v[i] = s.gamma[i] * v[i] + s.beta[i];
+    c.store(buf1, v);
+  }
+  template <int NPL, int VEC, class C, class S>
+  __device__ void finish(const rowpipe::Team&, const C&, S&, float*, int, int) const {}
+  static size_t finish_bytes(int, int) { return 0; }
+};
+
+// g in the first buffer, xhat in the second; the input gradient replaces g.  With `partial` every lane also keeps the
+// column sums of g*xhat and g over all rows it meets; they are folded team by team into partial[block][2][f].
+struct LnBwdOp {
+  const float *istd, *gamma;
+  float* partial;
+  int want_dx;
+  template <int NPL> struct State { float pg[NPL], pb[NPL], gamma[NPL]; };
+  template <class C, class S> __device__ __forceinline__ void start(const C& c, S& s) const {
+    c.load(gamma, s.gamma);
+#pragma unroll
+    for (int i = 0; i < (int)(sizeof(s.pg) / sizeof(float)); ++i) s.pg[i] = s.pb[i] = 0.0f;
+  }
+  template <int NPL, int VEC, class C, class S>
+  __device__ __forceinline__ void row(const rowpipe::Team& tm, const C& c, S& s, float* buf0, float* buf1, int r) const {
+    const float is = want_dx ? __ldg(istd + r) : 0.0f;   // on its way while the row is reduced
+    float g[NPL], xh[NPL];
+    c.load(buf0, g);
+    c.load(buf1, xh);
+    if (partial) {
+#pragma unroll
+      for (int i = 0; i < NPL; ++i) { s.pg[i] += g[i] * xh[i]; s.pb[i] += g[i]; }
+    }
+    if (!want_dx) return;
+    float t[2] = {0.0f, 0.0f};
+#pragma unroll
+    for (int i = 0; i < NPL; ++i) {
+      g[i] *= s.gamma[i];
+      t[0] += g[i];
+      t[1] += g[i] * xh[i];
+    }
+    tm.sum(t);
+    const float s1 = t[0] / (float)c.f, s2 = t[1] / (float)c.f;
+#pragma unroll
+    for (int i = 0; i < NPL; ++i) g[i] = is * (g[i] - s1 - xh[i] * s2);
+    c.store(buf0, g);
+  }
+  template <int NPL, int VEC, class C, class S>
+  __device__ __forceinline__ void finish(const rowpipe::Team&, const C& c, S& s, float* smem, int team, int teams) const {
+    if (!partial) return;
+    float* mine = smem + (size_t)team * 2 * c.f;
+#pragma unroll
+    for (int k = 0; k < NPL; ++k) {
+      const int col = c.first(k / VEC) + k % VEC;
+      if (col < c.f) { mine[col] = s.pg[k]; mine[c.f + col] = s.pb[k]; }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < 2 * c.f; i += blockDim.x) {
+      float t = 0.0f;
+      for (int w = 0; w < teams; ++w) t += smem[(size_t)w * 2 * c.f + i];
+      partial[(size_t)blockIdx.x * 2 * c.f + i] = t;
+    }
+  }
+  static size_t finish_bytes(int teams, int f) { return (size_t)teams * 2 * f * sizeof(float); }
+};
+
+struct SoftmaxFwdOp {
+  template <int NPL> using State = NoState;
+  template <class C, class S> __device__ void start(const C&, S&) const {}
+  template <int NPL, int VEC, class C, class S>
+  __device__ __forceinline__ void row(const rowpipe::Team& tm, const C& c, S&, float* buf0, float*, int) const {
+    float v[NPL], mx = -INFINITY, t[1] = {0.0f};
+    c.load(buf0, v, -INFINITY);
+#pragma unroll
+    for (int i = 0; i < NPL; ++i) mx = fmaxf(mx, v[i]);
+    mx = tm.max(mx);
+#pragma unroll
+    for (int i = 0; i < NPL; ++i)
+      if (c.live(i / VEC)) { v[i] = expf(v[i] - mx); t[0] += v[i]; }
+    tm.sum(t);
+#pragma unroll
+    for (int i = 0; i < NPL; ++i) v[i] = v[i] / t[0];
+    c.store(buf0, v);
+  }
+  template <int NPL, int VEC, class C, class S>
+  __device__ void finish(const rowpipe::Team&, const C&, S&, float*, int, int) const {}
+  static size_t finish_bytes(int, int) { return 0; }
+};
+
+// y in the first buffer, g in the second; the gradient replaces y.
+struct SoftmaxBwdOp {
+  template <int NPL> using State = NoState;
+  template <class C, class S> __device__ void start(const C&, S&) const {}
+  template <int NPL, int VEC, class C, class S>
+  __device__ __forceinline__ void row(const rowpipe::Team& tm, const C& c, S&, float* buf0, float* buf1, int) const {
+    float y[NPL], g[NPL], t[1] = {0.0f};
+    c.load(buf0, y);
+    c.load(buf1, g);
+#pragma unroll
+    for (int i = 0; i < NPL; ++i) t[0] += y[i] * g[i];
+    tm.sum(t);
+#pragma unroll
+    for (int i = 0; i < NPL; ++i) y[i] *= g[i] - t[0];
+    c.store(buf0, y);
+  }
+  template <int NPL, int VEC, class C, class S>
+  __device__ void finish(const rowpipe::Team&, const C&, S&, float*, int, int) const {}
+  static size_t finish_bytes(int, int) { return 0; }
+};
 
 // The TF32 operand planes of a value that the next tensor-core GEMM will read (rows x f, the tensor's own
 // layout): written by the producing kernel so that no separate staging pass reads the tensor again.
@@ -430,6 +579,15 @@ int layernorm_fwd(nrs_ctx* ctx, const char* who, const float* a, const float* b,
   if (rows == 0) return NRS_OK;
   NRS_REQUIRE(ctx, a && gamma && beta && y, NRS_ERR_ARG, "%s: null tensor", who);
   const int vpl = vec_vpl(f, {a, b, gamma, beta, y, xhat, y_hi, y_lo});
+  if (!(y_hi && vpl) && rowpipe::applies(rows, f, vpl != 0, {a, b, gamma, beta, y, xhat})) {
+    rowpipe::Params p{};
+    p.in[0] = a; p.in[1] = b; p.n_in = b ? 2 : 1; p.n_buf = 2;
+    p.out[0] = xhat; p.out_buf[0] = 0;
+    p.out[1] = y; p.out_buf[1] = 1;
+    p.rows = rows; p.f = f;
+    const int st = rowpipe::launch(ctx, p, LnFwdOp{gamma, beta, istd, eps, b != nullptr});
+    if (st != NRS_ERR_UNSUPPORTED) return st;
+  }
   if (vpl) {
     if (y_hi)
       NRS_DISPATCH_VPL(vpl, NRS_PDL_LAUNCH((ln_fwd_vec_kernel<V, true>), row_grid(ctx, rows), kRowThreads, 0, ctx->stream, a, b, gamma,
@@ -462,6 +620,29 @@ int layernorm_bwd(nrs_ctx* ctx, const char* who, const float* g, const float* xh
   NRS_REQUIRE(ctx, g && xhat && istd && gamma, NRS_ERR_ARG, "%s: null tensor", who);
   if (!dx && !dgamma) return NRS_OK;
   const int vpl = vec_vpl(f, {g, xhat, gamma, dx, dx2, d_hi, d_lo});
+  if (!(d_hi && vpl) && rowpipe::applies(rows, f, vpl != 0, {g, xhat, gamma, dx, dx2})) {
+    rowpipe::Params p{};
+    p.in[0] = g; p.in[1] = xhat; p.n_in = p.n_buf = 2;
+    p.out[0] = dx; p.out_add[0] = acc1;
+    p.out[1] = dx2; p.out_add[1] = acc2;
+    p.rows = rows; p.f = f;
+    float* partial = nullptr;
+    if (dgamma) {
+      void* ws = nullptr;
+      const int st = nrs_workspace(ctx, (size_t)ctx->sm_count * 2 * f * sizeof(float), &ws);
+      if (st != NRS_OK) return st;
+      partial = (float*)ws;
+    }
+    int blocks = 0;
+    const int st = rowpipe::launch(ctx, p, LnBwdOp{istd, gamma, partial, dx != nullptr}, &blocks);
+    if (st != NRS_ERR_UNSUPPORTED) {
+      if (st != NRS_OK || !dgamma) return st;
+      NRS_PDL_LAUNCH(ln_param_fold_kernel, nrs_blocks(2 * (size_t)f, 32), 256, 0, ctx->stream, (const float*)partial, dgamma, dbeta, f,
+                     blocks, accumulate_params);
+      NRS_LAUNCHED(ctx);
+      return NRS_OK;
+    }
+  }
   if (vpl) {
     // one pass over g and xhat for everything; the block size keeps the per-warp column partials within 32 KB
     int warps = 8;
@@ -576,6 +757,16 @@ int nrs_softmax_fwd(nrs_ctx* ctx, const float* x, float* y, int rows, int width)
   if (rows == 0) return NRS_OK;
   NRS_REQUIRE(ctx, x && y, NRS_ERR_ARG, "nrs_softmax_fwd: null tensor");
   const int vpl = vec_vpl(width, {x, y});
+  // (widths the vector kernel takes stay there at every size: bound by its exponentials and divisions, not by HBM, it
+  // does better with a full SM of warps: [16384][1000] 24 us against 54)
+  if (!vpl && rowpipe::applies(rows, width, false, {x, y})) {
+    rowpipe::Params p{};
+    p.in[0] = x; p.n_in = p.n_buf = 1;
+    p.out[0] = y;
+    p.rows = rows; p.f = width;
+    const int st = rowpipe::launch(ctx, p, SoftmaxFwdOp{});
+    if (st != NRS_ERR_UNSUPPORTED) return st;
+  }
   if (vpl) {
     NRS_DISPATCH_VPL(vpl, NRS_PDL_LAUNCH(softmax_fwd_vec_kernel<V>, row_grid(ctx, rows), kRowThreads, 0, ctx->stream, x, y, rows, width));
   } else {
@@ -591,6 +782,14 @@ int nrs_softmax_bwd(nrs_ctx* ctx, const float* y, const float* g, float* dx, int
   if (rows == 0) return NRS_OK;
   NRS_REQUIRE(ctx, y && g && dx, NRS_ERR_ARG, "nrs_softmax_bwd: null tensor");
   const int vpl = vec_vpl(width, {y, g, dx});
+  if (rowpipe::applies(rows, width, vpl != 0, {y, g, dx})) {
+    rowpipe::Params p{};
+    p.in[0] = y; p.in[1] = g; p.n_in = p.n_buf = 2;
+    p.out[0] = dx; p.out_add[0] = accumulate;
+    p.rows = rows; p.f = width;
+    const int st = rowpipe::launch(ctx, p, SoftmaxBwdOp{});
+    if (st != NRS_ERR_UNSUPPORTED) return st;
+  }
   if (vpl) {
     NRS_DISPATCH_VPL(vpl, NRS_PDL_LAUNCH(softmax_bwd_vec_kernel<V>, row_grid(ctx, rows), kRowThreads, 0, ctx->stream, y, g, dx, rows,
                                          width, accumulate));

@@ -1,0 +1,49 @@
+"""The shared-memory row pipeline of the row-wise operators: sizes where it takes over, odd widths, groups of rows with
+a ragged last copy, rows spread over several warps, one row, and the widest row it takes; against the f64 oracle."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from .conftest import rel_l2
+from .gpu_util import Dev, call
+
+pytestmark = pytest.mark.gpu
+F = C.c_float
+SHAPES = [(1, 17), (3, 1), (9001, 17), (1031, 515), (2100, 256), (700, 1000), (257, 2050), (130, 4097), (3, 8192), (2, 8193), (5, 6)]
+
+
+@pytest.mark.parametrize("rows,f", SHAPES)
+def test_row_pipeline(gpu_ctx, oracle64, rows, f):
+    rng = np.random.default_rng(rows + f)
+    a, b, g = (rng.normal(size=(rows, f)).astype(np.float32) for _ in range(3))
+    gamma, beta = rng.normal(size=f).astype(np.float32), rng.normal(size=f).astype(np.float32)
+    labels = rng.integers(0, f, rows).astype(np.int32)
+    t = np.zeros((rows, f), np.float32)
+    t[np.arange(rows), labels] = 1.0
+    x = (a + b).astype(np.float32)
+    ad, bd, gd, gm, bt, td, lb = (Dev(gpu_ctx, v) for v in (a, b, g, gamma, beta, t, labels))
+    y, xh, o1 = (Dev(gpu_ctx, shape=(rows, f)) for _ in range(3))
+    ist, dg, db, loss = Dev(gpu_ctx, shape=(rows,)), Dev(gpu_ctx, shape=(f,)), Dev(gpu_ctx, shape=(f,)), Dev(gpu_ctx, shape=(1,))
+    if f > 1:   # one feature has no variance
+        yr, xhr, isr = oracle64.layernorm_fwd(x, gamma, beta, 1e-5)
+        call(gpu_ctx, "nrs_layernorm_residual_fwd", ad, bd, gm, bt, y, xh, ist, rows, f, F(1e-5))
+        assert np.abs(y.get() - yr).max() <= 2e-4 and np.abs(xh.get() - xhr).max() <= 2e-4
+        dxr, dgr, dbr = oracle64.layernorm_bwd(g, xhr, isr, gamma)
+        o2 = Dev(gpu_ctx, np.ones_like(a))
+        call(gpu_ctx, "nrs_layernorm_residual_bwd", gd, xh, ist, gm, o1, o2, dg, db, rows, f, 0, 1, 0)
+        assert rel_l2(o1.get(), dxr) <= 2e-5 and rel_l2(o2.get() - 1.0, dxr) <= 4e-5
+        assert rel_l2(dg.get(), dgr) <= 1e-5 and rel_l2(db.get(), dbr) <= 1e-5
+    xd = Dev(gpu_ctx, x)
+    pr = oracle64.softmax_fwd(x)
+    call(gpu_ctx, "nrs_softmax_fwd", xd, y, rows, f)
+    assert rel_l2(y.get(), pr) <= 1e-6
+    sr = pr * (g - (pr * g).sum(1, keepdims=True))
+    for k in (1, 2):
+        call(gpu_ctx, "nrs_softmax_bwd", y, gd, o1, rows, f, k - 1)
+        assert np.linalg.norm(o1.get() - k * sr) <= 1e-5 * np.linalg.norm(pr * g)
+    ref_loss = -np.log(pr[np.arange(rows), labels]).mean()
+    for name, target in (("nrs_ce_fwd_bwd", td), ("nrs_ce_fwd_bwd_indexed", lb)):
+        call(gpu_ctx, name, xd, target, loss, o1, rows, f, rows)
+        assert abs(loss.get()[0] - ref_loss) <= 1e-5 * max(1.0, abs(ref_loss))
+        assert np.linalg.norm(o1.get() - (pr - t) / rows) <= 2e-6 * np.linalg.norm(t) / rows
