@@ -65,12 +65,7 @@ struct FReluBwd {  // a = x, b = g
 template <bool Acc>
 struct FGeluBwd {
   __device__ float operator()(float xi, float g, float o) const {
-    const float c = 0.7978845608f;
-    const float inner = c * (xi + 0.044715f * xi * xi * xi);
-    const float t = tanhf(inner);
-    const float dinner = c * (1.0f + 3.0f * 0.044715f * xi * xi);
-    const float dgelu = 0.5f * (1.0f + t) + 0.5f * xi * (1.0f - t * t) * dinner;
-    return (Acc ? o : 0.0f) + g * dgelu;
+    return (Acc ? o : 0.0f) + g * nrs_gelu_d(xi);
   }
 };
 template <bool Acc>

@@ -99,6 +99,15 @@ struct GradTarget {
 static GradTarget grad_target(const NodeP& n) {
   Node* r = grad_root(n.get());
   if (!r->grad) r->grad = dalloc(r->ctx, r->len());
+  if (r->gz_valid) {   // another share arrives: what was derived from the first one is stale
+    r->gz_valid = false;
+    nrs_free(r->ctx, r->gplanes_hi);
+    if (r->gplanes_lo) nrs_free(r->ctx, r->gplanes_lo);
+    r->gplanes_hi = r->gplanes_lo = nullptr;
+    nrs_free(r->ctx, r->gchan_partial);
+    r->gchan_partial = nullptr;
+    r->gchan_rows = 0;
+  }
   if (r->grad_premasked) {
     // A second consumer adds an unmasked share: drop the claim (and the now stale planes); the
     // ReLU mask is a 0/1 factor, so masking the sum later leaves the first share unchanged.
@@ -1096,7 +1105,42 @@ NodeP dropout2d(const NodeP& x, float p, bool training, const NodeP& mask) {
   return dropout_nd(x, p, training, mask, true, "cuda dropout2d");
 }
 
-NodeP linear_act(const NodeP& x, const NodeP& w, const NodeP& b, int act) {
+// dX = dz W^T of a Linear layer.  Where x is the output of another Linear layer with a fused activation and this is
+// the first share of its gradient, the epilogue also multiplies by that activation's derivative and leaves the planes
+// and column sums of the product, which is all that layer's backward pass reads (three passes over the tensor less).
+static void linear_input_grad(nrs_ctx* ctx, const NodeP& x, const NodeP& w, const float* dz, int m, int k, int n) {
+  const bool fold = x->fold_act != NRS_ACT_NONE && !x->view_of && !x->grad_valid && !x->gplanes_hi && planes_possible(ctx) &&
+                    nrs_gemm_on_tensor_cores(ctx, m, k, n);
+  GradTarget t = grad_target(x);
+  if (fold) {
+    NrsGemmExtras e;
+    e.dact = x->fold_act;
+    e.dact_src = x->fold_src;
+    e.hi = dalloc(ctx, x->len());
+    if (ctx->math_mode == NRS_MATH_3XTF32) e.lo = dalloc(ctx, x->len());
+    e.colsum_cap = (m + 127) / 128 * 4;
+    e.colsum = dalloc(ctx, (size_t)e.colsum_cap * k);
+    const int st = nrs_gemm_extras(ctx, 0, 1, m, k, n, dz, w->data, t.ptr, nullptr, NRS_ACT_NONE, 0.0f, &e);
+    if (st == NRS_OK && e.honoured && e.colsum_rows > 0) {
+      x->gplanes_hi = e.hi;
+      x->gplanes_lo = e.lo;
+      x->gchan_partial = e.colsum;
+      x->gchan_rows = e.colsum_rows;
+      x->gz_valid = true;
+      return;
+    }
+    nrs_free(ctx, e.hi);
+    if (e.lo) nrs_free(ctx, e.lo);
+    nrs_free(ctx, e.colsum);
+    if (st == NRS_OK) return;   // the gradient itself is there
+    if (st != NRS_ERR_UNSUPPORTED) check(ctx, st);
+  }
+  check(ctx, nrs_gemm(ctx, 0, 1, m, k, n, dz, w->data, t.ptr, nullptr, NRS_ACT_NONE, t.accumulate ? 1.0f : 0.0f));
+}
+
+// emit_planes: the caller knows that a tensor-core GEMM reads the result (always assumed of a GELU layer, which has
+// no other use in the models of this API): its epilogue writes the result's operand planes.
+NodeP linear_act(const NodeP& x, const NodeP& w, const NodeP& b, int act, bool emit_planes) {
   require_gpu(x, "cuda linear: input");
   require_gpu(w, "cuda linear: weights");
   require_gpu(b, "cuda linear: bias");
@@ -1112,38 +1156,65 @@ NodeP linear_act(const NodeP& x, const NodeP& w, const NodeP& b, int act) {
   if (act == NRS_ACT_GELU) {
     pre = dalloc(ctx, out->len());
     out->saved.push_back(pre);
-    // one kernel writes the pre-activation (GELU's derivative reads it) and the activation
-    const int st = nrs_linear_act_pre(ctx, m, n, k, x->data, w->data, b->data, NRS_ACT_GELU, out->data, pre);
-    if (st == NRS_ERR_UNSUPPORTED) {
-      check(ctx, nrs_gemm(ctx, 0, 0, m, n, k, x->data, w->data, pre, b->data, NRS_ACT_NONE, 0.0f));
-      check(ctx, nrs_gelu_fwd(ctx, pre, out->data, out->len()));
-    } else {
-      check(ctx, st);
-    }
+  }
+  NrsGemmExtras e;
+  e.pre = pre;
+  if (tensor_cores && w->requires_grad && n % 8 == 0 && (emit_planes || act == NRS_ACT_GELU) && !ctx->plane_hints.count(out->data)) {
+    e.hi = dalloc(ctx, out->len());
+    if (ctx->math_mode == NRS_MATH_3XTF32) e.lo = dalloc(ctx, out->len());
+  }
+  const int st = pre || e.hi ? nrs_gemm_extras(ctx, 0, 0, m, n, k, x->data, w->data, out->data, b->data, act, 0.0f, &e) : NRS_ERR_UNSUPPORTED;
+  if (st == NRS_OK && e.hi) {
+    out->planes_hi = e.hi;
+    out->planes_lo = e.lo;
+    NrsPlanes pl{e.hi, e.lo, e.lo ? 1 : 0};
+    pl.rows = m;
+    pl.cols = n;
+    ctx->plane_hints[out->data] = pl;
+  } else if (e.hi) {
+    nrs_free(ctx, e.hi);
+    if (e.lo) nrs_free(ctx, e.lo);
+  }
+  if (st == NRS_ERR_UNSUPPORTED) {
+    check(ctx, nrs_gemm(ctx, 0, 0, m, n, k, x->data, w->data, pre ? pre : out->data, b->data, pre ? NRS_ACT_NONE : act, 0.0f));
+    if (pre) check(ctx, nrs_gelu_fwd(ctx, pre, out->data, out->len()));
   } else {
-    check(ctx, nrs_gemm(ctx, 0, 0, m, n, k, x->data, w->data, out->data, b->data, act, 0.0f));
+    check(ctx, st);
   }
   Node* self = out.get();
+  if (act != NRS_ACT_NONE && tensor_cores && n % 8 == 0 && w->requires_grad && b->requires_grad && nrs_gemm_tn_reads_planes(k, n)) {
+    out->fold_act = act;
+    out->fold_src = act == NRS_ACT_GELU ? pre : out->data;
+  }
   out->backward_fn = [self, x, w, b, pre, act, m, k, n, tensor_cores]() {
     nrs_ctx* ctx = self->ctx;
-    const float* dz = grad_in(self);
+    const bool from_planes = self->gz_valid;
+    const float* dz = from_planes ? self->gplanes_hi : grad_in(self);
+    if (from_planes) {   // the reader of this layer's output left the planes and column sums of dz
+      NrsPlanes pl{self->gplanes_hi, self->gplanes_lo, self->gplanes_lo ? 1 : 0};
+      pl.rows = m;
+      pl.cols = n;
+      ctx->plane_hints[dz] = pl;
+    }
+    struct Forget {
+      nrs_ctx* c; const float* key;
+      ~Forget() { if (key) c->plane_hints.erase(key); }
+    } forget{ctx, from_planes ? dz : nullptr};
     float* tmp = nullptr;
-    if (act != NRS_ACT_NONE) {
+    if (act != NRS_ACT_NONE && !from_planes) {
       tmp = dalloc(ctx, self->len());
       if (act == NRS_ACT_RELU) check(ctx, nrs_relu_bwd(ctx, self->data, dz, tmp, self->len(), 0));
       else check(ctx, nrs_gelu_bwd(ctx, pre, dz, tmp, self->len(), 0));
       dz = tmp;
     }
     // dz feeds both dW = x^T dz and dX = dz W^T: its planes are made once
-    GradPlanes dz_planes(ctx, dz, (size_t)m, (size_t)n, tensor_cores && w->requires_grad && x->requires_grad);
+    GradPlanes dz_planes(ctx, dz, (size_t)m, (size_t)n, !from_planes && tensor_cores && w->requires_grad && x->requires_grad);
     if (b->requires_grad) {
       GradTarget t = grad_target(b);
-      check(ctx, nrs_sum_axis0(ctx, dz, t.ptr, m, n, t.accumulate));
+      if (from_planes) check(ctx, nrs_sum_axis0(ctx, self->gchan_partial, t.ptr, self->gchan_rows, n, t.accumulate));
+      else check(ctx, nrs_sum_axis0(ctx, dz, t.ptr, m, n, t.accumulate));
     }
-    if (x->requires_grad) {
-      GradTarget t = grad_target(x);
-      check(ctx, nrs_gemm(ctx, 0, 1, m, k, n, dz, w->data, t.ptr, nullptr, NRS_ACT_NONE, t.accumulate ? 1.0f : 0.0f));
-    }
+    if (x->requires_grad) linear_input_grad(ctx, x, w, dz, m, k, n);
     if (w->requires_grad) {   // after dX: it reads nothing dX wrote, so it may start under dX's tail
       GradTarget t = grad_target(w);
       NrsIndependentNext overlap(ctx, x->requires_grad);

@@ -68,6 +68,14 @@ struct Node {
   float* gchan_partial = nullptr;
   int gchan_rows = 0;
 
+  // Set on the output of a Linear layer with a fused activation whose backward pass can start from planes: the
+  // activation and what its derivative is taken from (RELU: the output, GELU: the pre-activation).  The Linear layer
+  // that reads the output may then leave, beside the gradient itself, the planes (gplanes_*) and column sums
+  // (gchan_*) of that gradient times the derivative (gz_valid).
+  int fold_act = 0;
+  const float* fold_src = nullptr;
+  bool gz_valid = false;
+
   size_t len() const;
   bool on_gpu() const { return data != nullptr; }
   ~Node();
@@ -149,7 +157,7 @@ NodeP dropout2d(const NodeP& x, float p, bool training, const NodeP& mask = null
 // Fused variants with no counterpart op in the reference: one kernel for
 // x@W + b followed by an activation, and conv + bias + activation.  Backward is
 // the composition of the unfused backward passes.
-NodeP linear_act(const NodeP& x, const NodeP& w, const NodeP& b, int act);
+NodeP linear_act(const NodeP& x, const NodeP& w, const NodeP& b, int act, bool emit_planes = false);
 // emit_planes: the caller knows a tensor-core convolution reads the result next, so the kernel
 // also writes the result's NHWC operand planes (a hint; ignored where it does not apply).
 NodeP conv2d_act(const NodeP& x, const NodeP& w, const NodeP& b, size_t stride, size_t pad, int act,

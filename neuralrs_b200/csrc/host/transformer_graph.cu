@@ -230,7 +230,7 @@ static NodeP block_body(const TransformerBlock& b, const NodeP& x, bool final_no
   NodeP flat = reshape(x1, {batch * seq, d});
   NodeP h, ff;
   if (b.fused_epilogues) {
-    h = linear_act(flat, b.ff1.weights, b.ff1.bias, b.act);
+    h = linear_act(flat, b.ff1.weights, b.ff1.bias, b.act, true);
     ff = linear_act(h, b.ff2.weights, b.ff2.bias, NRS_ACT_NONE);
   } else {
     h = b.ff1.forward(flat);

@@ -50,6 +50,14 @@ NRS_HD float nrs_gelu_f(float xi) {
   const float inner = 0.7978845608f * (xi + 0.044715f * xi * xi * xi);
   return 0.5f * xi * (1.0f + tanhf(inner));
 }
+// Derivative of nrs_gelu_f (gelu_grad, src/cuda/graph/gelu.rs:20-32).
+NRS_HD float nrs_gelu_d(float xi) {
+  const float c = 0.7978845608f;
+  const float inner = c * (xi + 0.044715f * xi * xi * xi);
+  const float t = tanhf(inner);
+  const float dinner = c * (1.0f + 3.0f * 0.044715f * xi * xi);
+  return 0.5f * (1.0f + t) + 0.5f * xi * (1.0f - t * t) * dinner;
+}
 NRS_HD float nrs_apply_act(float v, int act) {
   if (act == 1) return v > 0.0f ? v : 0.0f;
   if (act == 2) return nrs_gelu_f(v);

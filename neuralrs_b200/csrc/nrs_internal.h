@@ -343,13 +343,27 @@ static inline unsigned nrs_blocks(size_t work, unsigned per_block) {
 // Tensor-core contraction entry points (tc_gemm.cu / tc_conv.cu).  Each returns
 // NRS_ERR_UNSUPPORTED (without setting an error text) when the shape is outside
 // what the tcgen05 kernels cover, and the caller then runs the FFMA kernels.
-// pre_out (optional, [batch][m][n]): the value before the activation, written by the same epilogue.
+// What else the epilogue of a tensor-core GEMM may write or take part in (all optional).
+struct NrsGemmExtras {
+  float* pre = nullptr;        // [batch][m][n]: the value before the activation (what GELU's derivative needs)
+  // The result times the derivative of the activation that produced the operand it is the gradient of: `dact` is
+  // NRS_ACT_RELU (dact_src = that activation's output) or NRS_ACT_GELU (dact_src = its pre-activation), [m][n].  c keeps
+  // the value without the factor; planes and column sums are of the value with it.
+  int dact = NRS_ACT_NONE;
+  const float* dact_src = nullptr;
+  float* hi = nullptr;         // TF32 planes [m][n] for the GEMM that reads the result next (n a multiple of 8)
+  float* lo = nullptr;
+  float* colsum = nullptr;     // [colsum_cap][n] partial column sums
+  int colsum_cap = 0;
+  int colsum_rows = 0;         // out: rows of it written (0: none, the caller sums the columns itself)
+  bool skip_c = false;         // c is not written (its planes are all that is read)
+  bool honoured = false;       // out: the tensor-core kernel ran and did all of the above (but colsum: see colsum_rows)
+};
 int nrs_tc_gemm(nrs_ctx* ctx, int trans_a, int trans_b, int batch, int m, int n, int k,
-                const float* a, const float* b, float* c, const float* bias, int act, float beta, float* pre_out = nullptr);
-// c = act(a[m,k] . w[k,n] + bias) and pre = a . w + bias from one tensor-core kernel; NRS_ERR_UNSUPPORTED (no
-// error text) when the product would not run there.
-int nrs_linear_act_pre(nrs_ctx* ctx, int m, int n, int k, const float* a, const float* w, const float* bias, int act, float* c,
-                       float* pre);
+                const float* a, const float* b, float* c, const float* bias, int act, float beta, NrsGemmExtras* extras = nullptr);
+// nrs_gemm with extras; NRS_ERR_UNSUPPORTED (no error text) when the product would not run on the tensor cores.
+int nrs_gemm_extras(nrs_ctx* ctx, int trans_a, int trans_b, int m, int n, int k, const float* a, const float* b, float* c,
+                    const float* bias, int act, float beta, NrsGemmExtras* extras);
 int nrs_tc_conv_fwd(nrs_ctx* ctx, const float* x, const float* w, const float* b, float* y, int n, int ci, int h,
                     int wd, int co, int kh, int kw, int stride, int pad, int act);
 int nrs_tc_conv_dgrad(nrs_ctx* ctx, const float* w, const float* dy, float* dx, int n, int ci, int h, int wd, int co,
@@ -357,6 +371,9 @@ int nrs_tc_conv_dgrad(nrs_ctx* ctx, const float* w, const float* dy, float* dx, 
 int nrs_tc_conv_wgrad(nrs_ctx* ctx, const float* x, const float* dy, float* dw, int n, int ci, int h, int wd, int co,
                       int kh, int kw, int stride, int pad, int accumulate);
 bool nrs_gemm_on_tensor_cores(const nrs_ctx* ctx, int m, int n, int k);
+// Whether nrs_gemm's A^T B [m,n] runs on row planes of A and B (never on the f32 tensors): then a caller may hand it
+// planes without the tensor behind them.
+inline bool nrs_gemm_tn_reads_planes(int m, int n) { return m >= 32 && n >= 32 && ((long)m * n <= (4L << 20) || (m % 32 == 0 && n % 32 == 0 && m >= 64)); }
 // C[m,n] (+)= A^T B, A stored [k][m], B stored [k][n], on the weight-gradient kernel (no transposes).
 int nrs_tc_gemm_tn(nrs_ctx* ctx, int m, int n, int k, const float* a, const float* b, float* c, int accumulate);
 // Row-streaming variant for 3x3 / stride 1 / pad 1 (tc_wgrad_rows.cu); tried first.

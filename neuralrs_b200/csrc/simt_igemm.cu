@@ -382,11 +382,11 @@ bool nrs_gemm_on_tensor_cores(const nrs_ctx* ctx, int m, int n, int k) {
          tc::tensor_map_encoder() != nullptr;
 }
 
-int nrs_linear_act_pre(nrs_ctx* ctx, int m, int n, int k, const float* a, const float* w, const float* bias, int act, float* c,
-                       float* pre) {
+int nrs_gemm_extras(nrs_ctx* ctx, int trans_a, int trans_b, int m, int n, int k, const float* a, const float* b, float* c,
+                    const float* bias, int act, float beta, NrsGemmExtras* extras) {
   if (!nrs_gemm_on_tensor_cores(ctx, m, n, k)) return NRS_ERR_UNSUPPORTED;
   NrsProfScope prof(ctx, NRS_PROF_GEMM, 2.0 * m * n * k);
-  return nrs_tc_gemm(ctx, 0, 0, 1, m, n, k, a, w, c, bias, act, 0.0f, pre);
+  return nrs_tc_gemm(ctx, trans_a, trans_b, 1, m, n, k, a, b, c, bias, act, beta, extras);
 }
 
 extern "C" {
@@ -402,7 +402,7 @@ int nrs_gemm(nrs_ctx* ctx, int trans_a, int trans_b, int m, int n, int k, const 
   NrsProfScope prof(ctx, NRS_PROF_GEMM, 2.0 * m * n * k);
   if (k > 0 && thin_gemm_applies(m, n, k)) return thin_gemm(ctx, trans_a, trans_b, m, n, k, a, b, c, bias, act, beta);
   if (ctx->math_mode != NRS_MATH_FP32 && k > 0) {
-    if (trans_a && !trans_b && !bias && act == NRS_ACT_NONE && m >= 64) {   // A^T B: both operands read as stored
+    if (trans_a && !trans_b && !bias && act == NRS_ACT_NONE) {   // A^T B: both operands read as stored
       const int st = nrs_tc_gemm_tn(ctx, m, n, k, a, b, c, beta != 0.0f);
       if (st != NRS_ERR_UNSUPPORTED) return st;
     }

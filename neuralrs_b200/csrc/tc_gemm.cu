@@ -15,6 +15,10 @@
 
 namespace {
 
+// MN: both operands are stored with the reduction index slow ([k][m] and [k][n], the planes of activations and of
+// incoming gradients as they are): the slices arrive as 32-element column blocks, MN-major (see tc_wgrad.cu), and
+// nothing is transposed.
+template <bool MN>
 struct GemmPolicy {
   float* C;
   const float* bias;
@@ -22,69 +26,109 @@ struct GemmPolicy {
   float beta;
   int M, N;
   size_t batch_stride;
-  bool vec_ok;
-  float* pre;   // optional second output: the value before the activation (what GELU's derivative needs)
+  bool vec_ok;                 // rows of every output and epilogue input start on 16 bytes
+  NrsGemmExtras x;
+  // Several B matrices side by side ([Wq|Wk|Wv]): columns n0 of matrix n0 / seg_n, or reduction indices k of matrix
+  // k / seg_k; 0 = one matrix.  The matrices are the batches of B's tensor map.
+  int seg_n, seg_k;
   static constexpr bool kCanEmit = false;
+  static constexpr bool kMnMajor = MN;
+  static constexpr int kEpiWarps = 8;   // the epilogue is latency (TMEM, loads, tanh), not registers: two warps per lane quarter
 
   __device__ __forceinline__ uint32_t a_slice_bytes() const { return tc::BM * tc::BK * 4; }
   struct Cursor { int b_col, row, batch; };
   __device__ __forceinline__ Cursor cursor(int tile_m, int batch, int kb) const { return Cursor{kb * tc::BK, tile_m * tc::BM, batch}; }
   __device__ __forceinline__ void advance(Cursor& c) const { c.b_col += tc::BK; }
   __device__ __forceinline__ void load_a(void* dst, const CUtensorMap* tm, uint64_t* bar, const Cursor& c) const {
-    tc::tma_load_3d(dst, tm, bar, c.b_col, c.row, c.batch);
+    if (MN) tc::tma_load_3d(dst, tm, bar, 0, c.b_col, c.row / 32);
+    else tc::tma_load_3d(dst, tm, bar, c.b_col, c.row, c.batch);
   }
+  __device__ __forceinline__ void b_origin(const Cursor& c, int n0, int batch, int* b0, int* b1, int* b2) const {
+    if (MN) { *b0 = 0; *b1 = c.b_col; *b2 = n0 / 32; return; }
+    *b0 = c.b_col; *b1 = n0; *b2 = batch;
+    if (seg_n) { *b2 = n0 / seg_n; *b1 = n0 - *b2 * seg_n; }
+    if (seg_k) { *b2 = c.b_col / seg_k; *b0 = c.b_col - *b2 * seg_k; }
+  }
+  __device__ __forceinline__ float dact(float src) const { return x.dact == NRS_ACT_RELU ? (src > 0.0f ? 1.0f : 0.0f) : nrs_gelu_d(src); }
+  // One element, from the pass that sums a K-split.
   __device__ __forceinline__ void store(int tile_m, int batch, int row, int n, float v) const {
     const int m = tile_m * tc::BM + row;
     if (m >= M || n >= N) return;
-    float* dst = C + (size_t)batch * batch_stride + (size_t)m * N + n;
+    const size_t at = (size_t)batch * batch_stride + (size_t)m * N + n;
     if (bias) v += bias[n];
-    if (pre) pre[(size_t)batch * batch_stride + (size_t)m * N + n] = v;
+    if (x.pre) x.pre[at] = v;
     v = nrs_apply_act(v, act);
-    if (beta != 0.0f) v += beta * *dst;
-    *dst = v;
+    if (beta != 0.0f) v += beta * C[at];
+    if (!x.skip_c) C[at] = v;
+    if (!x.hi) return;
+    if (x.dact != NRS_ACT_NONE) v *= dact(x.dact_src[at]);
+    const float h = tc::tf32_rn(v);
+    x.hi[at] = h;
+    if (x.lo) x.lo[at] = v - h;
   }
-  struct Row { bool live; size_t off; };   // an accumulator row: is there one in C, and where
-  __device__ __forceinline__ Row row(int tile_m, int batch, int r) const {
-    const int m = tile_m * tc::BM + r;
-    return Row{m < M, (size_t)batch * batch_stride + (size_t)m * N};
-  }
-  // 32 consecutive columns [nb, nb+32) of one accumulator row.
-  __device__ __forceinline__ void epilogue(const Row& rw, int nb, int ncols, const uint32_t (&r)[32]) const {
-    if (!rw.live || nb >= N) return;
-    float* crow = C + rw.off;
-    float* prow = pre + rw.off;
-    if (vec_ok && ncols == 32 && nb + 32 <= N) {
+  __device__ __forceinline__ int row(int, int, int) const { return 0; }
+  // Eight row segments of a warp's 32 x 32 block: row r0 + 4*i of the tile, columns n..n+3 (see tc::rows_to_lines).
+  __device__ __forceinline__ void epilogue(int tile_m, int batch, int r0, int n, float4 (&v)[8]) const {
+    const int m0 = tile_m * tc::BM + r0, nn = N - n;   // nn: how many of the four columns exist (four or more: all)
+    const size_t at0 = (size_t)batch * batch_stride + (size_t)m0 * N + n, step = (size_t)4 * N;
+    if (bias) {
+      const float4 b = tc::load_guarded(bias + n, nn, vec_ok);
 #pragma unroll
-      for (int j = 0; j < 32; j += 4) {
-        float4 v = make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]), __uint_as_float(r[j + 2]),
-                               __uint_as_float(r[j + 3]));
-        if (bias) {
-          const float4 bv = *reinterpret_cast<const float4*>(bias + nb + j);
-          v.x += bv.x; v.y += bv.y; v.z += bv.z; v.w += bv.w;
-        }
-        if (pre) *reinterpret_cast<float4*>(prow + nb + j) = v;
-        v.x = nrs_apply_act(v.x, act); v.y = nrs_apply_act(v.y, act);
-        v.z = nrs_apply_act(v.z, act); v.w = nrs_apply_act(v.w, act);
-        float4* dst = reinterpret_cast<float4*>(crow + nb + j);
-        if (beta != 0.0f) {
-          const float4 o = *dst;
-          v.x += beta * o.x; v.y += beta * o.y; v.z += beta * o.z; v.w += beta * o.w;
-        }
-        *dst = v;
-      }
-    } else {
+      for (int i = 0; i < 8; ++i) { v[i].x += b.x; v[i].y += b.y; v[i].z += b.z; v[i].w += b.w; }
+    }
+    if (x.pre) {
 #pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        const int n = nb + j;
-        if (j < ncols && n < N) {
-          float v = __uint_as_float(r[j]);
-          if (bias) v += bias[n];
-          if (pre) prow[n] = v;
-          v = nrs_apply_act(v, act);
-          if (beta != 0.0f) v += beta * crow[n];
-          crow[n] = v;
-        }
+      for (int i = 0; i < 8; ++i)
+        if (m0 + 4 * i < M) tc::store_guarded(x.pre + at0 + i * step, v[i], nn, vec_ok);
+    }
+    if (act != NRS_ACT_NONE) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        v[i].x = nrs_apply_act(v[i].x, act); v[i].y = nrs_apply_act(v[i].y, act);
+        v[i].z = nrs_apply_act(v[i].z, act); v[i].w = nrs_apply_act(v[i].w, act);
       }
+    }
+    if (beta != 0.0f) {
+      float4 o[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        o[i] = m0 + 4 * i < M ? tc::load_guarded(C + at0 + i * step, nn, vec_ok) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) { v[i].x += beta * o[i].x; v[i].y += beta * o[i].y; v[i].z += beta * o[i].z; v[i].w += beta * o[i].w; }
+    }
+    if (!x.skip_c) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (m0 + 4 * i < M) tc::store_guarded(C + at0 + i * step, v[i], nn, vec_ok);
+    }
+    if (x.dact != NRS_ACT_NONE) {
+      float4 s[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        s[i] = m0 + 4 * i < M ? tc::load_guarded(x.dact_src + at0 + i * step, nn, vec_ok) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) { v[i].x *= dact(s[i].x); v[i].y *= dact(s[i].y); v[i].z *= dact(s[i].z); v[i].w *= dact(s[i].w); }
+    }
+    if (x.hi) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        if (m0 + 4 * i >= M) continue;
+        const float4 h = make_float4(tc::tf32_rn(v[i].x), tc::tf32_rn(v[i].y), tc::tf32_rn(v[i].z), tc::tf32_rn(v[i].w));
+        tc::store_guarded(x.hi + at0 + i * step, h, nn, vec_ok);
+        if (x.lo) tc::store_guarded(x.lo + at0 + i * step, make_float4(v[i].x - h.x, v[i].y - h.y, v[i].z - h.z, v[i].w - h.w), nn, vec_ok);
+      }
+    }
+    if (x.colsum) {   // sum over the warp's 32 rows, in a fixed order; lanes 0..7 write four columns each
+      float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (m0 + 4 * i < M) { s.x += v[i].x; s.y += v[i].y; s.z += v[i].z; s.w += v[i].w; }
+#pragma unroll
+      for (int d = 8; d <= 16; d <<= 1) {
+        s.x += __shfl_xor_sync(0xffffffffu, s.x, d); s.y += __shfl_xor_sync(0xffffffffu, s.y, d);
+        s.z += __shfl_xor_sync(0xffffffffu, s.z, d); s.w += __shfl_xor_sync(0xffffffffu, s.w, d);
+      }
+      if ((threadIdx.x & 31) < 8) tc::store_guarded(x.colsum + ((size_t)tile_m * 4 + (r0 >> 5)) * N + n, s, nn, vec_ok);
     }
   }
 };
@@ -97,9 +141,10 @@ struct Operand {
   size_t bstride;  // floats between batches
 };
 
-// Brings one operand into K-major planes.  stored_kmajor: memory is [rows][K]; else [K][rows].
+// Brings one operand into K-major planes.  stored_kmajor: memory is [rows][K]; else [K][rows].  in_place: plain TF32
+// may read a suitable source as it is (the tensor core truncates it); otherwise it is rounded into a plane.
 int prepare_operand(nrs_ctx* ctx, const float* src, int rows, int K, int batch, bool stored_kmajor, bool split,
-                    int ws_hi, int ws_lo, Operand* out, bool is_weight) {
+                    int ws_hi, int ws_lo, Operand* out, bool is_weight, bool in_place = true) {
   const int ldk = nrs_plane_ld(K);   // TMA zero-fills what a K-block reads beyond K
   if (batch == 1) {
     // a weight staged ahead with the rest of the model's (weight_set.cu) ...
@@ -120,7 +165,7 @@ int prepare_operand(nrs_ctx* ctx, const float* src, int rows, int K, int batch, 
       }
     }
   }
-  const bool direct = !split && stored_kmajor && (K % 4 == 0) && ((reinterpret_cast<uintptr_t>(src) & 15) == 0);
+  const bool direct = in_place && !split && stored_kmajor && (K % 4 == 0) && ((reinterpret_cast<uintptr_t>(src) & 15) == 0);
   if (direct) {
     *out = Operand{src, nullptr, K, K, (size_t)rows * K};
     return NRS_OK;
@@ -145,16 +190,64 @@ bool make_operand_map(CUtensorMap* tm, const float* base, const Operand& op, int
   const uint32_t box[3] = {(uint32_t)tc::BK, (uint32_t)box_rows, 1};
   return tc::encode_tmap_f32(tm, base, 3, dim, str, box);
 }
+// An operand stored [k][rows]: [row block][k][32 rows], one box = a K-slice of box_rows / 32 blocks.
+bool make_mn_operand_map(CUtensorMap* tm, const float* base, const Operand& op, int rows, int k, int box_rows) {
+  const uint64_t dim[3] = {32, (uint64_t)k, (uint64_t)(rows / 32)};
+  const uint64_t str[2] = {(uint64_t)op.ld * 4, 128};
+  const uint32_t box[3] = {32, (uint32_t)tc::BK, (uint32_t)(box_rows / 32)};
+  return tc::encode_tmap_f32(tm, base, 3, dim, str, box, true);
+}
 
-template <int BN, int NPLANES>
-int run(nrs_ctx* ctx, const Operand& A, const Operand& B, int batch, int m, int n, int k, const GemmPolicy& pol) {
+template <int BN, int NPLANES, bool MN>
+int run(nrs_ctx* ctx, const Operand& A, const Operand& B, int batch, int b_rows, int b_batch, int m, int n, int k,
+        const GemmPolicy<MN>& pol, int* splits) {
   CUtensorMap ta_hi, ta_lo, tb_hi, tb_lo;
-  bool ok = make_operand_map(&ta_hi, A.hi, A, m, batch, tc::BM) && make_operand_map(&tb_hi, B.hi, B, n, batch, BN);
-  if (NPLANES == 2) ok = ok && make_operand_map(&ta_lo, A.lo, A, m, batch, tc::BM) && make_operand_map(&tb_lo, B.lo, B, n, batch, BN);
+  auto map_a = [&](CUtensorMap* t, const float* p) { return MN ? make_mn_operand_map(t, p, A, m, k, tc::BM) : make_operand_map(t, p, A, m, batch, tc::BM); };
+  auto map_b = [&](CUtensorMap* t, const float* p) { return MN ? make_mn_operand_map(t, p, B, n, k, BN) : make_operand_map(t, p, B, b_rows, b_batch, BN); };
+  bool ok = map_a(&ta_hi, A.hi) && map_b(&tb_hi, B.hi);
+  if (NPLANES == 2) ok = ok && map_a(&ta_lo, A.lo) && map_b(&tb_lo, B.lo);
   else { ta_lo = ta_hi; tb_lo = tb_hi; }
   NRS_REQUIRE(ctx, ok, NRS_ERR_CUDA, "tc_gemm: cuTensorMapEncodeTiled failed (m=%d n=%d k=%d)", m, n, k);
-  return tc::launch<BN, NPLANES, GemmPolicy>(ctx, ta_hi, ta_lo, tb_hi, tb_lo, pol, (m + tc::BM - 1) / tc::BM, n, batch,
-                                             (k + tc::BK - 1) / tc::BK);
+  return tc::launch<BN, NPLANES, GemmPolicy<MN>>(ctx, ta_hi, ta_lo, tb_hi, tb_lo, pol, (m + tc::BM - 1) / tc::BM, n, batch,
+                                                 (k + tc::BK - 1) / tc::BK, nullptr, nullptr, splits);
+}
+
+// Tile width: 128 columns is the efficient shape, but a product with few tiles leaves most SMs idle and
+// a K-split needs a second pass, so narrower tiles are taken until about two thirds of the SMs have one.
+// `limit`: widest tile allowed (segmented B: the segment must be whole tiles).
+int column_tile(const nrs_ctx* ctx, int m, int n, int batch, int limit = 128) {
+  const long tiles_m = (m + tc::BM - 1) / tc::BM;
+  auto tiles = [&](int bn) { return tiles_m * ((n + bn - 1) / bn) * batch; };
+  const long want = (long)ctx->sm_count * 2 / 3;
+  int bn = n <= 32 ? 32 : n <= 64 ? 64 : 128;
+  if (bn > limit) bn = limit;
+  if (bn == 128 && tiles(128) < want) bn = 64;
+  if (bn == 64 && n > 32 && tiles(64) < want) bn = 32;
+  return bn;
+}
+
+template <bool MN>
+int dispatch(nrs_ctx* ctx, int bn, bool split, const Operand& A, const Operand& B, int batch, int b_rows, int b_batch, int m, int n,
+             int k, GemmPolicy<MN>& pol, NrsGemmExtras* extras) {
+  auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+  pol.vec_ok = n % 4 == 0 && ((size_t)m * n) % 4 == 0 && aligned(pol.C) && aligned(pol.bias);
+  if (extras) {
+    pol.x = *extras;
+    pol.vec_ok = pol.vec_ok && aligned(extras->pre) && aligned(extras->dact_src);
+    if (extras->colsum && (m + tc::BM - 1) / tc::BM * 4 > extras->colsum_cap) pol.x.colsum = nullptr;
+  }
+  int st, splits = 1;
+#define NRS_RUN_GEMM(BN_) (split ? run<BN_, 2, MN>(ctx, A, B, batch, b_rows, b_batch, m, n, k, pol, &splits) \
+                                 : run<BN_, 1, MN>(ctx, A, B, batch, b_rows, b_batch, m, n, k, pol, &splits))
+  if (bn == 128) st = NRS_RUN_GEMM(128);
+  else if (bn == 64) st = NRS_RUN_GEMM(64);
+  else st = NRS_RUN_GEMM(32);
+#undef NRS_RUN_GEMM
+  if (extras && st == NRS_OK) {
+    extras->honoured = true;
+    extras->colsum_rows = pol.x.colsum && splits == 1 ? (m + tc::BM - 1) / tc::BM * 4 : 0;   // a K-split's second pass makes none
+  }
+  return st;
 }
 
 }  // namespace
@@ -252,35 +345,29 @@ extern "C" int nrs_measure_tf32_umma_peak(nrs_ctx* ctx, double* tflops_out) {
 }
 
 int nrs_tc_gemm(nrs_ctx* ctx, int trans_a, int trans_b, int batch, int m, int n, int k, const float* a, const float* b,
-                float* c, const float* bias, int act, float beta, float* pre_out) {
+                float* c, const float* bias, int act, float beta, NrsGemmExtras* extras) {
   if (!tc::tensor_map_encoder()) return NRS_ERR_UNSUPPORTED;
   // Small or skinny problems stay on the FFMA kernel: a 128-row tile would be mostly padding.
   if (m < 64 || n < 32 || k < 32) return NRS_ERR_UNSUPPORTED;
   if (batch > 65535) return NRS_ERR_UNSUPPORTED;
-  // Batched operands read in place need 16-byte aligned batch strides.
   const bool split = ctx->math_mode == NRS_MATH_3XTF32;
   Operand A, B;
-  int st = prepare_operand(ctx, a, m, k, batch, /*stored_kmajor=*/!trans_a, split, NRS_WS_A_HI, NRS_WS_A_LO, &A, false);
+  int st;
+  if (trans_a && !trans_b && batch == 1 && m % 32 == 0 && n % 32 == 0) {   // A^T B on the operands' own rows
+    st = prepare_operand(ctx, a, k, m, 1, true, split, NRS_WS_A_HI, NRS_WS_A_LO, &A, false, false);
+    if (st == NRS_OK) st = prepare_operand(ctx, b, k, n, 1, true, split, NRS_WS_B_HI, NRS_WS_B_LO, &B, false, false);
+    if (st != NRS_OK) return st;
+    GemmPolicy<true> pol{c, bias, act, beta, m, n, (size_t)m * n, false, {}, 0, 0};
+    return dispatch<true>(ctx, column_tile(ctx, m, n, 1), split, A, B, 1, n, 1, m, n, k, pol, extras);
+  }
+  st = prepare_operand(ctx, a, m, k, batch, /*stored_kmajor=*/!trans_a, split, NRS_WS_A_HI, NRS_WS_A_LO, &A, false);
   if (st != NRS_OK) return st;
   st = prepare_operand(ctx, b, n, k, batch, /*stored_kmajor=*/trans_b != 0, split, NRS_WS_B_HI, NRS_WS_B_LO, &B, true);
   if (st != NRS_OK) return st;
+  // Batched operands read in place need 16-byte aligned batch strides.
   if (batch > 1 && ((A.bstride % 4) || (B.bstride % 4))) return NRS_ERR_UNSUPPORTED;
-  GemmPolicy pol{c, bias, act, beta, m, n, (size_t)m * n, false, pre_out};
-  pol.vec_ok = (n % 4 == 0) && ((reinterpret_cast<uintptr_t>(c) & 15) == 0) && (((size_t)m * n) % 4 == 0) &&
-               ((reinterpret_cast<uintptr_t>(bias) & 15) == 0) && ((reinterpret_cast<uintptr_t>(pre_out) & 15) == 0);
-  // Tile width: 128 columns is the efficient shape, but a product with few tiles leaves most SMs idle and
-  // a K-split needs a second pass, so narrower tiles are taken until about two thirds of the SMs have one.
-  const long tiles_m = (m + tc::BM - 1) / tc::BM;
-  auto tiles = [&](int bn) { return tiles_m * ((n + bn - 1) / bn) * batch; };
-  const long want = (long)ctx->sm_count * 2 / 3;
-  int bn = n <= 32 ? 32 : n <= 64 ? 64 : 128;
-  if (bn == 128 && tiles(128) < want) bn = 64;
-  if (bn == 64 && n > 32 && tiles(64) < want) bn = 32;
-#define NRS_RUN_GEMM(BN_) (split ? run<BN_, 2>(ctx, A, B, batch, m, n, k, pol) : run<BN_, 1>(ctx, A, B, batch, m, n, k, pol))
-  if (bn == 128) return NRS_RUN_GEMM(128);
-  if (bn == 64) return NRS_RUN_GEMM(64);
-  return NRS_RUN_GEMM(32);
-#undef NRS_RUN_GEMM
+  GemmPolicy<false> pol{c, bias, act, beta, m, n, (size_t)m * n, false, {}, 0, 0};
+  return dispatch<false>(ctx, column_tile(ctx, m, n, batch), split, A, B, batch, n, batch, m, n, k, pol, extras);
 }
 
 extern "C" int nrs_has_tensor_core_path(void) { return 1; }

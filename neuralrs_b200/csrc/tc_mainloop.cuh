@@ -9,7 +9,8 @@
 //              the ring runs ahead across tile boundaries
 //   warp 1     TMEM allocation; one thread issues the UMMAs (M=128, K=8) and commits
 //              ring slots back to the producer, then the accumulator to the epilogue
-//   warps 2-5  epilogue: tcgen05.ld (thread = accumulator row), policy-defined store
+//   warps 2..  epilogue (4 or 8 warps, the policy's choice): tcgen05.ld (thread = accumulator row),
+//              policy-defined store
 // TMEM holds two accumulators, so the epilogue of tile i runs under the main loop of
 // tile i+1.
 // A Policy supplies how an A slice is fetched (dense rows for GEMM, a shifted
@@ -42,7 +43,6 @@
 namespace tc {
 
 constexpr int BM = 128, BK = 32;   // BK f32 = 128 bytes = one swizzle row
-constexpr int kThreads = 192;
 constexpr int kMaxChainK = 4096;   // longest single accumulation chain in 3xTF32 mode
 constexpr int kGroupM = 16;        // row tiles per raster group (see TileMap)
 
@@ -89,12 +89,47 @@ struct TileMap {
   }
 };
 
-// Shared memory of the plane-emission staging tile: one [128 rows][128 B] tile per plane.
+// Shared memory of the epilogue: the plane-emission staging tile, one [128 rows][128 B] tile per plane, or (row-major
+// results) a 32 x 32 transpose tile per warp.
 template <int NPLANES, class Policy>
-__host__ __device__ constexpr int emit_bytes() { return Policy::kCanEmit ? NPLANES * BM * 128 : 0; }
+__host__ __device__ constexpr int emit_bytes() { return Policy::kCanEmit ? NPLANES * BM * 128 : Policy::kEpiWarps * 4096; }
+template <class Policy>
+__host__ __device__ constexpr int threads() { return 64 + 32 * Policy::kEpiWarps; }
+
+// Four consecutive values of which `n` (or more: all) exist; `vec`: dst is 16-byte aligned when all four do.
+__device__ __forceinline__ void store_guarded(float* dst, float4 v, int n, bool vec) {
+  if (vec && n >= 4) { *reinterpret_cast<float4*>(dst) = v; return; }
+  if (n > 0) dst[0] = v.x;
+  if (n > 1) dst[1] = v.y;
+  if (n > 2) dst[2] = v.z;
+  if (n > 3) dst[3] = v.w;
+}
+__device__ __forceinline__ float4 load_guarded(const float* src, int n, bool vec) {
+  if (vec && n >= 4) return *reinterpret_cast<const float4*>(src);
+  return make_float4(n > 0 ? src[0] : 0.0f, n > 1 ? src[1] : 0.0f, n > 2 ? src[2] : 0.0f, n > 3 ? src[3] : 0.0f);
+}
+
+// A warp's 32 rows x 32 columns, one row per lane, turned into eight float4s per lane that lie along the rows: lane l
+// gets row 4*i + l/8, columns 4*(l%8)..+3 in v[i].  A global access of the warp then covers four full 128-byte lines
+// instead of 16 bytes in each of 32 (which took the store unit 32 cycles an instruction: 2 us per 128 x 128 tile and
+// output).  The tile is 32 rows of 128 bytes with the 16-byte chunks XORed by row % 8: conflict-free both ways.
+__device__ __forceinline__ void rows_to_lines(float* tile, int lane, const uint32_t (&r)[32], float4 (&v)[8]) {
+  float4* t4 = reinterpret_cast<float4*>(tile);
+  __syncwarp();   // the previous block's values have been read
+#pragma unroll
+  for (int g = 0; g < 8; ++g)
+    t4[lane * 8 + (g ^ (lane & 7))] = make_float4(__uint_as_float(r[4 * g]), __uint_as_float(r[4 * g + 1]), __uint_as_float(r[4 * g + 2]),
+                                                  __uint_as_float(r[4 * g + 3]));
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int row = 4 * i + (lane >> 3);
+    v[i] = t4[row * 8 + ((lane & 7) ^ (row & 7))];
+  }
+}
 
 template <int BN, int NPLANES, class Policy>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(threads<Policy>(), 1)
 tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ CUtensorMap tm_a_lo,
           const __grid_constant__ CUtensorMap tm_b_hi, const __grid_constant__ CUtensorMap tm_b_lo,
           const __grid_constant__ CUtensorMap tm_out_hi, const __grid_constant__ CUtensorMap tm_out_lo,
@@ -121,7 +156,7 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
     if (emit >= 1) prefetch_tmap(&tm_out_hi);
     if (emit == 2) prefetch_tmap(&tm_out_lo);
     for (int s = 0; s < L::kStages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-    for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 4); mbar_init(&emit_bar[b], 128); }
+    for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], Policy::kEpiWarps); mbar_init(&emit_bar[b], 128); }
     fence_barrier_init();
   }
   if (warp == 1) {
@@ -160,9 +195,11 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
           uint8_t* st = smem + s * L::kStage;
           mbar_expect_tx(&full_bar[s], stage_bytes);
           pol.load_a(st, &tm_a_hi, &full_bar[s], cur);
-          tma_load_3d(st + L::kATile, &tm_b_hi, &full_bar[s], cur.b_col, n0, batch);
+          int b0, b1, b2;
+          pol.b_origin(cur, n0, batch, &b0, &b1, &b2);
+          tma_load_3d(st + L::kATile, &tm_b_hi, &full_bar[s], b0, b1, b2);
           if (NPLANES == 2) {
-            tma_load_3d(st + L::kATile + L::kBTile, &tm_b_lo, &full_bar[s], cur.b_col, n0, batch);
+            tma_load_3d(st + L::kATile + L::kBTile, &tm_b_lo, &full_bar[s], b0, b1, b2);
             pol.load_a(st + L::kATile + 2 * L::kBTile, &tm_a_lo, &full_bar[s], cur);
           }
           pol.advance(cur);
@@ -180,8 +217,14 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
   } else if (warp == 1) {
     if (lane == 0) {
       // ---------------- UMMA issuer
-      constexpr uint32_t idesc_wide = make_idesc_tf32(BM, NPLANES * BN, false, false);
-      constexpr uint32_t idesc_half = make_idesc_tf32(BM, BN, false, false);
+      constexpr bool kMN = Policy::kMnMajor;
+      constexpr uint32_t idesc_wide = make_idesc_tf32(BM, NPLANES * BN, kMN, kMN);
+      constexpr uint32_t idesc_half = make_idesc_tf32(BM, BN, kMN, kMN);
+      // K-major: 8 elements of K are 32 bytes inside the swizzle row.  MN-major: 32-column blocks of [32 k][128 B], so
+      // a K-step is 1024 bytes and blocks are 4096 apart (the blocks of B_lo follow those of B_hi).
+      auto desc = [](uint32_t addr, int k) {
+        return kMN ? make_smem_desc_sw128_32b(addr + (uint32_t)k * 1024u, BK * 128, 512) : make_smem_desc_sw128(addr + (uint32_t)k * 32u, 16, 1024);
+      };
       uint32_t it = 0, local = 0;
       bool ok = true;
       for (long t = blockIdx.x; t < tmap.total && ok; t += gridDim.x, ++local) {
@@ -205,13 +248,10 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
           const uint32_t a_lo = b_hi + 2 * L::kBTile;
 #pragma unroll
           for (int k = 0; k < BK / 8; ++k) {
-            const uint32_t koff = k * 32;  // 8 f32 along K inside the 128-byte swizzle row
-            const uint64_t da_hi = make_smem_desc_sw128(a_hi + koff, 16, 1024);
-            const uint64_t db_hi = make_smem_desc_sw128(b_hi + koff, 16, 1024);
+            const uint64_t da_hi = desc(a_hi, k), db_hi = desc(b_hi, k);
             umma_tf32(d, da_hi, db_hi, idesc_wide, (i | k) != 0);   // hi*hi | hi*lo
             if (NPLANES == 2) {
-              const uint64_t da_lo = make_smem_desc_sw128(a_lo + koff, 16, 1024);
-              umma_tf32(d, da_lo, db_hi, idesc_half, 1);             // + lo*hi
+              umma_tf32(d, desc(a_lo, k), db_hi, idesc_half, 1);             // + lo*hi
             }
           }
           umma_commit(&empty_bar[s]);  // slot reusable once these UMMAs have read it
@@ -232,15 +272,22 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
       const int batch = z / sp.splits, split = z - batch * sp.splits;
       const int n0 = tile_n * BN;
       const uint32_t buf = local & 1u, use = local >> 1;
-      const typename Policy::Row rw = pol.row(tile_m, batch, row);   // index arithmetic under the main loop
+      [[maybe_unused]] const auto rw = pol.row(tile_m, batch, row);   // index arithmetic under the main loop
       if (!mbar_wait(&acc_full[buf], use & 1u)) {
         if (lane == 0) atomicExch(err_flag, kErrEpilogueWait);
         break;
       }
       tc_fence_after_sync();
+      if (BN == 32 && warp >= 6) {   // one column block only: the second warp of a quarter just hands the accumulator back
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&acc_empty[buf]);
+        continue;
+      }
       const uint32_t acc = tmem_base + buf * (uint32_t)L::kAccCols + ((uint32_t)(q * 32) << 16);
+      // two warps of a lane quarter take alternate 32-column blocks
+      constexpr int kBlocks = BN / 32, kStep = Policy::kEpiWarps / 4;
 #pragma unroll 1
-      for (int c = 0; c < (BN + 31) / 32; ++c) {
+      for (int c = kStep == 1 ? 0 : (warp - 2) >> 2; c < kBlocks; c += kStep) {
         uint32_t r[32];
         tmem_ld_32x32(acc + (uint32_t)(c * 32), r);
         if (NPLANES == 2) {
@@ -252,22 +299,32 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
         } else {
           tmem_ld_wait();
         }
-        if (c == (BN + 31) / 32 - 1) {
+        if (c + kStep >= kBlocks) {
           // Everything this warp needs is in registers: hand the accumulator back.
           tc_fence_before_sync();
           __syncwarp();
           if (lane == 0) mbar_arrive(&acc_empty[buf]);
         }
         if (n0 + c * 32 >= sp.n_total) continue;   // padding columns of a ragged last tile
-        [[maybe_unused]] const int ncols = (BN - c * 32) < 32 ? (BN - c * 32) : 32;
-        if (sp.splits > 1) {
+        if constexpr (!Policy::kCanEmit) {
+          float4 v[8];
+          rows_to_lines(reinterpret_cast<float*>(emit_tile) + (warp - 2) * 1024, lane, r, v);
+          const int r0 = q * 32 + (lane >> 3), n = n0 + c * 32 + (lane & 7) * 4;
+          if (sp.splits > 1) {
+            float* dst = sp.partial + (((size_t)split * sp.batches + batch) * sp.rows_total + (size_t)tile_m * BM + r0) * sp.n_total + n;
+#pragma unroll
+            for (int i = 0; i < 8; ++i, dst += (size_t)4 * sp.n_total) store_guarded(dst, v[i], sp.n_total - n, sp.n_total % 4 == 0);
+          } else {
+            pol.epilogue(tile_m, batch, r0, n, v);
+          }
+        } else if (sp.splits > 1) {
           float* dst = sp.partial + (((size_t)split * sp.batches + batch) * sp.rows_total + (size_t)tile_m * BM + row) * sp.n_total;
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
             const int n = n0 + c * 32 + j;
-            if (c * 32 + j < BN && n < sp.n_total) dst[n] = __uint_as_float(r[j]);
+            if (n < sp.n_total) dst[n] = __uint_as_float(r[j]);
           }
-        } else if constexpr (Policy::kCanEmit) {
+        } else {
           float v[32];
           pol.epilogue(rw, n0 + c * 32, r, v);
           if (float* cs = pol.colsum_row(tile_m, q)) {
@@ -315,8 +372,6 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
               bulk_commit();
             }
           }
-        } else {
-          pol.epilogue(rw, n0 + c * 32, ncols, r);
         }
       }
     }
@@ -424,7 +479,7 @@ int launch(nrs_ctx* ctx, const CUtensorMap& ta_hi, const CUtensorMap& ta_lo, con
   const unsigned grid = (unsigned)(tmap.total < ctx->sm_count ? tmap.total : ctx->sm_count);
   // Planes can only be emitted by the direct epilogue; with a K-split the policy's store() writes them.
   const int emit = (Policy::kCanEmit && out_hi && sp.splits == 1) ? (out_lo && NPLANES == 2 ? 2 : 1) : 0;
-  NRS_PDL_LAUNCH((tc_kernel<BN, NPLANES, Policy>), grid, kThreads, kSmem, ctx->stream, ta_hi, ta_lo, tb_hi, tb_lo,
+  NRS_PDL_LAUNCH((tc_kernel<BN, NPLANES, Policy>), grid, threads<Policy>(), kSmem, ctx->stream, ta_hi, ta_lo, tb_hi, tb_lo,
                  out_hi ? *out_hi : ta_hi, out_lo ? *out_lo : ta_hi, pol, sp, tmap, emit, err);
   NRS_LAUNCHED(ctx);
   if (sp.splits > 1) {
