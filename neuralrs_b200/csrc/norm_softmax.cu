@@ -579,7 +579,7 @@ int layernorm_fwd(nrs_ctx* ctx, const char* who, const float* a, const float* b,
   if (rows == 0) return NRS_OK;
   NRS_REQUIRE(ctx, a && gamma && beta && y, NRS_ERR_ARG, "%s: null tensor", who);
   const int vpl = vec_vpl(f, {a, b, gamma, beta, y, xhat, y_hi, y_lo});
-  if (!(y_hi && vpl) && rowpipe::applies(rows, f, vpl != 0, {a, b, gamma, beta, y, xhat})) {
+  if (!(y_hi && vpl) && rowpipe::applies(rows, f, vpl != 0, 1u << 20, {a, b, gamma, beta, y, xhat})) {
     rowpipe::Params p{};
     p.in[0] = a; p.in[1] = b; p.n_in = b ? 2 : 1; p.n_buf = 2;
     p.out[0] = xhat; p.out_buf[0] = 0;
@@ -620,7 +620,7 @@ int layernorm_bwd(nrs_ctx* ctx, const char* who, const float* g, const float* xh
   NRS_REQUIRE(ctx, g && xhat && istd && gamma, NRS_ERR_ARG, "%s: null tensor", who);
   if (!dx && !dgamma) return NRS_OK;
   const int vpl = vec_vpl(f, {g, xhat, gamma, dx, dx2, d_hi, d_lo});
-  if (!(d_hi && vpl) && rowpipe::applies(rows, f, vpl != 0, {g, xhat, gamma, dx, dx2})) {
+  if (!(d_hi && vpl) && rowpipe::applies(rows, f, vpl != 0, 1u << 20, {g, xhat, gamma, dx, dx2})) {
     rowpipe::Params p{};
     p.in[0] = g; p.in[1] = xhat; p.n_in = p.n_buf = 2;
     p.out[0] = dx; p.out_add[0] = acc1;
@@ -759,7 +759,7 @@ int nrs_softmax_fwd(nrs_ctx* ctx, const float* x, float* y, int rows, int width)
   const int vpl = vec_vpl(width, {x, y});
   // (widths the vector kernel takes stay there at every size: bound by its exponentials and divisions, not by HBM, it
   // does better with a full SM of warps: [16384][1000] 24 us against 54)
-  if (!vpl && rowpipe::applies(rows, width, false, {x, y})) {
+  if (!vpl && rowpipe::applies(rows, width, false, 0, {x, y})) {
     rowpipe::Params p{};
     p.in[0] = x; p.n_in = p.n_buf = 1;
     p.out[0] = y;
@@ -782,7 +782,7 @@ int nrs_softmax_bwd(nrs_ctx* ctx, const float* y, const float* g, float* dx, int
   if (rows == 0) return NRS_OK;
   NRS_REQUIRE(ctx, y && g && dx, NRS_ERR_ARG, "nrs_softmax_bwd: null tensor");
   const int vpl = vec_vpl(width, {y, g, dx});
-  if (rowpipe::applies(rows, width, vpl != 0, {y, g, dx})) {
+  if (rowpipe::applies(rows, width, vpl != 0, 1u << 20, {y, g, dx})) {
     rowpipe::Params p{};
     p.in[0] = y; p.in[1] = g; p.n_in = p.n_buf = 2;
     p.out[0] = dx; p.out_add[0] = accumulate;

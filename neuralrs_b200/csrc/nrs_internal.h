@@ -373,7 +373,7 @@ int nrs_tc_conv_wgrad(nrs_ctx* ctx, const float* x, const float* dy, float* dw, 
 bool nrs_gemm_on_tensor_cores(const nrs_ctx* ctx, int m, int n, int k);
 // Whether nrs_gemm's A^T B [m,n] runs on row planes of A and B (never on the f32 tensors): then a caller may hand it
 // planes without the tensor behind them.
-inline bool nrs_gemm_tn_reads_planes(int m, int n) { return m >= 32 && n >= 32 && ((long)m * n <= (4L << 20) || (m % 32 == 0 && n % 32 == 0 && m >= 64)); }
+inline bool nrs_gemm_tn_reads_planes(int m, int n) { return m >= 32 && n >= 32 && ((long)m * n <= (4L << 20) || (m % 32 == 0 && n % 32 == 0)); }
 // C[m,n] (+)= A^T B, A stored [k][m], B stored [k][n], on the weight-gradient kernel (no transposes).
 int nrs_tc_gemm_tn(nrs_ctx* ctx, int m, int n, int k, const float* a, const float* b, float* c, int accumulate);
 // Row-streaming variant for 3x3 / stride 1 / pad 1 (tc_wgrad_rows.cu); tried first.

@@ -209,13 +209,13 @@ row_pipe_kernel(const Params p, const Op op, int* __restrict__ err_flag) {
 }
 
 // Whether a tensor set takes this path: 16-byte aligned bases, rows of at most 8192 columns (one slot of two
-// buffers is then 64 KB), and either at least a megabyte per tensor (below that the register kernels' shorter
-// prologue wins) or a width the vector kernels do not take.
-inline bool applies(int rows, int f, bool vector_kernel_exists, std::initializer_list<const void*> ptrs) {
+// buffers is then 64 KB), and enough elements: `vector_from` where a register kernel takes the width (the operator's
+// own crossover), 128 K where only the scalar loops do (below, their shorter prologue wins: [64][10] 4 us against 20).
+inline bool applies(int rows, int f, bool vector_kernel_exists, size_t vector_from, std::initializer_list<const void*> ptrs) {
   if (f > 8192 || rows < 1) return false;
   for (const void* q : ptrs)
     if (reinterpret_cast<uintptr_t>(q) & 15) return false;
-  return !vector_kernel_exists || (size_t)rows * f >= (1u << 19);
+  return (size_t)rows * f >= (vector_kernel_exists ? vector_from : (size_t)1 << 17);
 }
 
 template <int NPL, int VEC, class Op>

@@ -327,8 +327,106 @@ thin_n_cols_kernel(const float* __restrict__ a, const float* __restrict__ b, flo
   }
 }
 
+// m < 16, A row-major, B as stored ([k][n]): a few requests through a Linear layer.  Bound by reading B once, so a block
+// takes 32 columns of a K-split, its 8 warps every eighth row of B (full lines, several in flight), A's rows come from
+// shared memory, and enough splits run to cover the SMs.  The warps are added in order, the splits by the last block of
+// a column group to arrive, in split order (fixed order of additions, no second launch).  [1,3136] x [3136,128]: the
+// 128 x 128 tile took 30 us in two launches, this 6.
+constexpr int kThinM = 15, kThinMChunk = 512;
+template <int MT>
+__global__ void __launch_bounds__(256)
+thin_m_kernel(const float* __restrict__ a, const float* __restrict__ b, float* c, const float* __restrict__ bias, int m, int n, int k,
+              int act, float beta, int k_per, float* partial, unsigned* tickets) {
+  NRS_PDL_PROLOGUE();
+  __shared__ float as[MT][kThinMChunk];
+  __shared__ float sums[8][MT][32];
+  __shared__ bool last;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int col = blockIdx.x * 32 + lane, split = blockIdx.y, splits = gridDim.y;
+  const int k0 = split * k_per, k1 = min(k, k0 + k_per);
+  float acc[MT];
+#pragma unroll
+  for (int i = 0; i < MT; ++i) acc[i] = 0.0f;
+  for (int i = threadIdx.x; i < MT * (k1 - k0); i += blockDim.x) {
+    const int r = i / (k1 - k0), kk = i - r * (k1 - k0);
+    as[r][kk] = r < m ? a[(size_t)r * k + k0 + kk] : 0.0f;
+  }
+  __syncthreads();
+  if (col < n) {
+#pragma unroll 8
+    for (int kk = k0 + warp; kk < k1; kk += 8) {
+      const float w = b[(size_t)kk * n + col];
+#pragma unroll
+      for (int i = 0; i < MT; ++i) acc[i] = fmaf(as[i][kk - k0], w, acc[i]);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < MT; ++i) sums[warp][i][lane] = acc[i];
+  __syncthreads();
+  auto finish = [&](int row, int cc, float v) {
+    if (bias) v += bias[cc];
+    v = nrs_apply_act(v, act);
+    float* dst = c + (size_t)row * n + cc;
+    if (beta != 0.0f) v += beta * *dst;
+    *dst = v;
+  };
+  for (int o = threadIdx.x; o < m * 32; o += blockDim.x) {
+    const int r = o >> 5, cl = o & 31, cc = blockIdx.x * 32 + cl;
+    if (cc >= n) continue;
+    float v = 0.0f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) v += sums[w][r][cl];
+    if (splits == 1) finish(r, cc, v);
+    else partial[((size_t)split * m + r) * n + cc] = v;
+  }
+  if (splits == 1) return;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(&tickets[blockIdx.x], 1u) == (unsigned)splits - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  for (int o = threadIdx.x; o < m * 32; o += blockDim.x) {
+    const int r = o >> 5, cc = blockIdx.x * 32 + (o & 31);
+    if (cc >= n) continue;
+    float v = 0.0f;
+#pragma unroll 8
+    for (int z = 0; z < splits; ++z) v += __ldcg(partial + ((size_t)z * m + r) * n + cc);
+    finish(r, cc, v);
+  }
+  if (threadIdx.x == 0) tickets[blockIdx.x] = 0;
+}
+
+int thin_m_gemm(nrs_ctx* ctx, int m, int n, int k, const float* a, const float* b, float* c, const float* bias, int act, float beta) {
+  const int cols = (n + 31) / 32;
+  if (m > kThinM || n <= kThinN || k < 64 || cols >= kNrsFoldTickets) return NRS_ERR_UNSUPPORTED;
+  int splits = (2 * ctx->sm_count + cols - 1) / cols;
+  if (splits > k / 32) splits = k / 32;                                     // at least four rows of B per warp
+  if (splits < (k + kThinMChunk - 1) / kThinMChunk) splits = (k + kThinMChunk - 1) / kThinMChunk;
+  if (splits > 65535) return NRS_ERR_UNSUPPORTED;
+  const int k_per = (k + splits - 1) / splits;
+  splits = (k + k_per - 1) / k_per;
+  float* partial = nullptr;
+  unsigned* tickets = nullptr;
+  if (splits > 1) {
+    void* ws = nullptr;
+    int st = nrs_workspace(ctx, (size_t)splits * m * n * sizeof(float), &ws);
+    if (st == NRS_OK) st = nrs_fold_ticket(ctx, &tickets);
+    if (st != NRS_OK) return st;
+    partial = (float*)ws;
+    tickets += 1;   // slot 0 serves kernels with one counter
+  }
+  const dim3 grid((unsigned)cols, (unsigned)splits);
+  if (m == 1) NRS_PDL_LAUNCH((thin_m_kernel<1>), grid, 256, 0, ctx->stream, a, b, c, bias, m, n, k, act, beta, k_per, partial, tickets);
+  else if (m <= 4) NRS_PDL_LAUNCH((thin_m_kernel<4>), grid, 256, 0, ctx->stream, a, b, c, bias, m, n, k, act, beta, k_per, partial, tickets);
+  else if (m <= 8) NRS_PDL_LAUNCH((thin_m_kernel<8>), grid, 256, 0, ctx->stream, a, b, c, bias, m, n, k, act, beta, k_per, partial, tickets);
+  else NRS_PDL_LAUNCH((thin_m_kernel<15>), grid, 256, 0, ctx->stream, a, b, c, bias, m, n, k, act, beta, k_per, partial, tickets);
+  NRS_LAUNCHED(ctx);
+  return NRS_OK;
+}
+
 bool thin_gemm_applies(int m, int n, int k) {
-  return (n <= kThinN || k <= 16) && (double)m * n * k <= 6.4e7 && (long)m * n >= 1024;
+  return (n <= kThinN || k <= 16) && (double)m * n * k <= 6.4e7;
 }
 
 int thin_gemm(nrs_ctx* ctx, int ta, int tb, int m, int n, int k, const float* a, const float* b, float* c,
@@ -378,7 +476,7 @@ int check_conv_dims(nrs_ctx* ctx, const char* who, int n, int ci, int h, int wd,
 
 // True when nrs_gemm would run an [m,k] x [k,n] product (any transposes) on the tensor-core kernels.
 bool nrs_gemm_on_tensor_cores(const nrs_ctx* ctx, int m, int n, int k) {
-  return ctx->math_mode != NRS_MATH_FP32 && k >= 32 && m >= 64 && n >= 32 && !thin_gemm_applies(m, n, k) &&
+  return ctx->math_mode != NRS_MATH_FP32 && k >= 32 && m >= 16 && n >= 32 && !thin_gemm_applies(m, n, k) &&
          tc::tensor_map_encoder() != nullptr;
 }
 
@@ -401,6 +499,10 @@ int nrs_gemm(nrs_ctx* ctx, int trans_a, int trans_b, int m, int n, int k, const 
   NRS_REQUIRE(ctx, c && (k == 0 || (a && b)), NRS_ERR_ARG, "nrs_gemm: null operand");
   NrsProfScope prof(ctx, NRS_PROF_GEMM, 2.0 * m * n * k);
   if (k > 0 && thin_gemm_applies(m, n, k)) return thin_gemm(ctx, trans_a, trans_b, m, n, k, a, b, c, bias, act, beta);
+  if (!trans_a && !trans_b) {
+    const int st = thin_m_gemm(ctx, m, n, k, a, b, c, bias, act, beta);
+    if (st != NRS_ERR_UNSUPPORTED) return st;
+  }
   if (ctx->math_mode != NRS_MATH_FP32 && k > 0) {
     if (trans_a && !trans_b && !bias && act == NRS_ACT_NONE) {   // A^T B: both operands read as stored
       const int st = nrs_tc_gemm_tn(ctx, m, n, k, a, b, c, beta != 0.0f);

@@ -347,8 +347,8 @@ extern "C" int nrs_measure_tf32_umma_peak(nrs_ctx* ctx, double* tflops_out) {
 int nrs_tc_gemm(nrs_ctx* ctx, int trans_a, int trans_b, int batch, int m, int n, int k, const float* a, const float* b,
                 float* c, const float* bias, int act, float beta, NrsGemmExtras* extras) {
   if (!tc::tensor_map_encoder()) return NRS_ERR_UNSUPPORTED;
-  // Small or skinny problems stay on the FFMA kernel: a 128-row tile would be mostly padding.
-  if (m < 64 || n < 32 || k < 32) return NRS_ERR_UNSUPPORTED;
+  // Fewer rows than a UMMA's smallest useful share of a 128-row tile stay on the FFMA kernels.
+  if (m < 16 || n < 32 || k < 32) return NRS_ERR_UNSUPPORTED;
   if (batch > 65535) return NRS_ERR_UNSUPPORTED;
   const bool split = ctx->math_mode == NRS_MATH_3XTF32;
   Operand A, B;

@@ -405,13 +405,16 @@ tc_splitk_reduce_kernel(const Policy pol, const SplitInfo sp) {
 
 // Chooses the K-split: enough CTAs to fill the GPU, and no accumulation chain longer
 // than kMaxChainK elements when `limit_chain`.
-inline void plan_split(const nrs_ctx* ctx, long tiles, int kb_total, bool limit_chain, int* splits, int* kb_per_split) {
+inline void plan_split(const nrs_ctx* ctx, long tiles, long out_elems, int kb_total, bool limit_chain, int* splits, int* kb_per_split) {
   int s = 1;
   // (More than half a wave of tiles runs unsplit: the second pass over the partial tiles costs more
   // than the idle SMs.)
   if (2 * tiles <= ctx->sm_count && kb_total >= 32) {
     s = (int)(ctx->sm_count / tiles);
-    if (s > kb_total / 16) s = kb_total / 16;   // a split shorter than 16 K-blocks is all prologue and second pass
+    // a split shorter than 16 K-blocks is all prologue and second pass, except where the output is so small (a Linear
+    // layer at a batch of a few dozen) that the second pass is nothing: there down to 4
+    const int shortest = out_elems <= (1 << 15) ? 4 : 16;
+    if (s > kb_total / shortest) s = kb_total / shortest;
   }
   if (limit_chain) {
     const int need = (kb_total * BK + kMaxChainK - 1) / kMaxChainK;
@@ -459,7 +462,7 @@ int launch(nrs_ctx* ctx, const CUtensorMap& ta_hi, const CUtensorMap& ta_lo, con
   NRS_ENSURE_SMEM(ctx, attr, (tc_kernel<BN, NPLANES, Policy>), kSmem);
   const int tiles_n = (n_total + BN - 1) / BN;
   SplitInfo sp{};
-  plan_split(ctx, (long)tiles_m * tiles_n * batches, kb_total, NPLANES == 2, &sp.splits, &sp.kb_per_split);
+  plan_split(ctx, (long)tiles_m * tiles_n * batches, (long)tiles_m * BM * n_total * batches, kb_total, NPLANES == 2, &sp.splits, &sp.kb_per_split);
   sp.kb_total = kb_total;
   sp.batches = batches;
   sp.n_total = n_total;

@@ -10,7 +10,7 @@ from .gpu_util import Dev, call
 
 pytestmark = pytest.mark.gpu
 F = C.c_float
-SHAPES = [(1, 17), (3, 1), (9001, 17), (1031, 515), (2100, 256), (700, 1000), (257, 2050), (130, 4097), (3, 8192), (2, 8193), (5, 6)]
+SHAPES = [(3, 17), (9001, 17), (1031, 515), (4100, 256), (1060, 1000), (257, 2050), (130, 4097), (17, 8192), (17, 8193), (70001, 2), (8400, 1000)]
 
 
 @pytest.mark.parametrize("rows,f", SHAPES)
