@@ -1,6 +1,7 @@
 // Context lifecycle, device memory pool and host<->device copies.
 // Stands in for the reference's global backend and residency helpers
 // (src/cuda/backend.rs:19-32, src/cuda/runtime.rs:39-124).
+#include "fold.h"
 #include "nrs_internal.h"
 
 #include <algorithm>
@@ -330,6 +331,7 @@ int nrs_destroy(nrs_ctx* ctx) {
   for (int i = 0; i < NRS_WS_COUNT; ++i) if (ctx->ws_slot[i]) cudaFree(ctx->ws_slot[i]);
   if (ctx->err_host) cudaFreeHost((void*)ctx->err_host);
   nrs_bounce_free(ctx);
+  nrs_folds_free(ctx);
   if (ctx->fold_ticket) cudaFree(ctx->fold_ticket);
   for (auto& r : ctx->prof_records) { cudaEventDestroy(r.start); cudaEventDestroy(r.stop); }
   for (auto& e : ctx->prof_free_events) cudaEventDestroy(e);

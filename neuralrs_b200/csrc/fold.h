@@ -1,0 +1,18 @@
+// Second stages of split reductions, run one by one or collected into one launch (fold.cu).
+#pragma once
+
+#include "nrs_internal.h"
+
+// While on, submitted folds wait for nrs_folds_flush (a backward pass's end) or nrs_folds_settle.
+void nrs_folds_begin(nrs_ctx* ctx);
+int nrs_folds_flush(nrs_ctx* ctx);
+void nrs_folds_end(nrs_ctx* ctx);    // leaves the collecting mode; what is still queued is dropped (a failed pass)
+void nrs_folds_free(nrs_ctx* ctx);
+// Runs what is queued if it writes `dst`: called by whoever is about to read or add to a gradient.
+int nrs_folds_settle(nrs_ctx* ctx, const float* dst);
+// Memory for a fold's partial sums that lives until the fold has run; outside of the collecting mode the given
+// workspace slot (-1: the context's workspace).
+int nrs_fold_partial(nrs_ctx* ctx, int ws_slot, size_t bytes, float** out);
+int nrs_fold_submit(nrs_ctx* ctx, NrsFoldJob job);
+// dst[c] (+)= sum over rows of src[r*stride + c]; src must stay as it is until the fold has run.
+int nrs_fold_columns(nrs_ctx* ctx, const float* src, float* dst, int rows, int cols, int stride, int accumulate);

@@ -1,6 +1,7 @@
 // Define-by-run graph over the C ABI: Node, the resident operators with their
 // backward closures, backward_graph and AdamW.  See graph.h for what it mirrors.
 #include "host/graph.h"
+#include "fold.h"
 #include "nrs_internal.h"
 #include "tc_mainloop.cuh"
 
@@ -99,6 +100,7 @@ struct GradTarget {
 static GradTarget grad_target(const NodeP& n) {
   Node* r = grad_root(n.get());
   if (!r->grad) r->grad = dalloc(r->ctx, r->len());
+  check(r->ctx, nrs_folds_settle(r->ctx, r->grad));   // an earlier share may still wait in the fold queue
   if (r->gz_valid) {   // another share arrives: what was derived from the first one is stale
     r->gz_valid = false;
     nrs_free(r->ctx, r->gplanes_hi);
@@ -124,6 +126,7 @@ static GradTarget grad_target(const NodeP& n) {
 static const float* grad_in(Node* n) {
   Node* r = grad_root(n);
   if (!r->grad) r->grad = dalloc(r->ctx, r->len());
+  check(r->ctx, nrs_folds_settle(r->ctx, r->grad));
   if (!r->grad_valid) {
     check(r->ctx, nrs_memset_zero(r->ctx, r->grad, r->len() * sizeof(float)));
     r->grad_valid = true;
@@ -632,7 +635,7 @@ static void conv_backward(Node* self, const NodeP& x, const NodeP& w, const Node
   if (b->requires_grad) {
     GradTarget t = grad_target(b);
     if (self->grad_premasked && self->gchan_partial && self->gchan_rows > 0)   // the producer of dy left channel sums
-      check(ctx, nrs_sum_axis0(ctx, self->gchan_partial, t.ptr, self->gchan_rows, co, t.accumulate));
+      check(ctx, nrs_fold_columns(ctx, self->gchan_partial, t.ptr, self->gchan_rows, co, co, t.accumulate));
     else
       check(ctx, nrs_conv2d_bwd(ctx, x->data, w->data, dy, nullptr, nullptr, t.ptr, n, ci, h, wd, co, kh, kw, stride,
                                 pad, t.accumulate));
@@ -1211,7 +1214,7 @@ NodeP linear_act(const NodeP& x, const NodeP& w, const NodeP& b, int act, bool e
     GradPlanes dz_planes(ctx, dz, (size_t)m, (size_t)n, !from_planes && tensor_cores && w->requires_grad && x->requires_grad);
     if (b->requires_grad) {
       GradTarget t = grad_target(b);
-      if (from_planes) check(ctx, nrs_sum_axis0(ctx, self->gchan_partial, t.ptr, self->gchan_rows, n, t.accumulate));
+      if (from_planes) check(ctx, nrs_fold_columns(ctx, self->gchan_partial, t.ptr, self->gchan_rows, n, n, t.accumulate));
       else check(ctx, nrs_sum_axis0(ctx, dz, t.ptr, m, n, t.accumulate));
     }
     if (x->requires_grad) linear_input_grad(ctx, x, w, dz, m, k, n);
@@ -1477,8 +1480,16 @@ void backward_graph(const NodeP& root) {
   std::vector<NodeP> topo;
   std::unordered_set<const Node*> seen;
   build_topo(root, seen, topo);
+  // Nothing in here reads a parameter's gradient: the second stages of their reductions run together at the end (the
+  // nodes of `topo`, which hold some of the partial sums, are alive until then).
+  struct Collect {
+    nrs_ctx* ctx;
+    explicit Collect(nrs_ctx* c) : ctx(c) { nrs_folds_begin(c); }
+    ~Collect() { nrs_folds_end(ctx); }
+  } collect(root->ctx);
   for (auto it = topo.rbegin(); it != topo.rend(); ++it)
     if ((*it)->backward_fn) (*it)->backward_fn();
+  check(root->ctx, nrs_folds_flush(root->ctx));
 }
 
 }  // namespace nrs

@@ -12,6 +12,7 @@
 // Reference: ln_forward / ln_reduce / ln_dx (src/cuda/nn/normalization.rs:14-78),
 // softmax_forward / softmax_backward (src/cuda/graph/softmax.rs:12-35); CPU
 // semantics src/nn/normalization.rs:38-103, src/autograd/graph/softmax.rs:23-60.
+#include "fold.h"
 #include "nrs_internal.h"
 #include "row_pipe.cuh"
 #include "tc_common.cuh"
@@ -412,37 +413,6 @@ ln_param_kernel(const float* __restrict__ g, const float* __restrict__ xhat, flo
     partial[((size_t)split * 2 + 1) * f + c] = tb;
   }
 }
-// partial[part][2][f] folded over the parts: a block owns 32 of the 2f columns; its eight warps each
-// sum every eighth part (128-byte row segments, coalesced), and the eight sums are combined in warp
-// order — a fixed order of additions whatever the launch shape.
-__global__ void __launch_bounds__(256)
-ln_param_fold_kernel(const float* __restrict__ partial, float* dgamma, float* dbeta, int f, int parts, int accumulate) {
-  NRS_PDL_PROLOGUE();
-  __shared__ float sm[8][33];
-  const int lane = threadIdx.x & 31, wrp = threadIdx.x >> 5;
-  const int c = blockIdx.x * 32 + lane;          // column of the [2f]-wide partial rows
-  float t = 0.0f;
-  if (c < 2 * f) {
-    // four loads in flight per thread; the additions keep the order s = wrp, wrp + 8, ...
-    const size_t step = (size_t)8 * 2 * f;
-    const float* src = partial + (size_t)wrp * 2 * f + c;
-    int s = wrp;
-    for (; s + 24 < parts; s += 32, src += 4 * step) {
-      const float v0 = src[0], v1 = src[step], v2 = src[2 * step], v3 = src[3 * step];
-      t += v0; t += v1; t += v2; t += v3;
-    }
-    for (; s < parts; s += 8, src += step) t += *src;
-  }
-  sm[wrp][lane] = t;
-  __syncthreads();
-  if (wrp != 0 || c >= 2 * f) return;
-  float sum = 0.0f;
-#pragma unroll
-  for (int w = 0; w < 8; ++w) sum += sm[w][lane];
-  float* dst = c < f ? dgamma + c : dbeta + (c - f);
-  *dst = accumulate ? *dst + sum : sum;
-}
-
 // ------------------------------------------------------------------ softmax
 template <int VPL>
 __global__ void __launch_bounds__(kRowThreads)
@@ -603,6 +573,12 @@ int layernorm_fwd(nrs_ctx* ctx, const char* who, const float* a, const float* b,
   return NRS_OK;
 }
 
+// partial[part][2][f] -> dgamma, dbeta.
+int fold_params(nrs_ctx* ctx, const float* partial, float* dgamma, float* dbeta, int f, int parts, int accumulate) {
+  const int st = nrs_fold_columns(ctx, partial, dgamma, parts, f, 2 * f, accumulate);
+  return st != NRS_OK ? st : nrs_fold_columns(ctx, partial + f, dbeta, parts, f, 2 * f, accumulate);
+}
+
 int layernorm_bwd(nrs_ctx* ctx, const char* who, const float* g, const float* xhat, const float* istd, const float* gamma,
                   float* dx, float* dx2, float* dgamma, float* dbeta, int rows, int f, int acc1, int acc2, int accumulate_params,
                   float* d_hi = nullptr, float* d_lo = nullptr, int* emitted = nullptr) {
@@ -628,19 +604,14 @@ int layernorm_bwd(nrs_ctx* ctx, const char* who, const float* g, const float* xh
     p.rows = rows; p.f = f;
     float* partial = nullptr;
     if (dgamma) {
-      void* ws = nullptr;
-      const int st = nrs_workspace(ctx, (size_t)ctx->sm_count * 2 * f * sizeof(float), &ws);
+      const int st = nrs_fold_partial(ctx, -1, (size_t)ctx->sm_count * 2 * f * sizeof(float), &partial);
       if (st != NRS_OK) return st;
-      partial = (float*)ws;
     }
     int blocks = 0;
     const int st = rowpipe::launch(ctx, p, LnBwdOp{istd, gamma, partial, dx != nullptr}, &blocks);
     if (st != NRS_ERR_UNSUPPORTED) {
       if (st != NRS_OK || !dgamma) return st;
-      NRS_PDL_LAUNCH(ln_param_fold_kernel, nrs_blocks(2 * (size_t)f, 32), 256, 0, ctx->stream, (const float*)partial, dgamma, dbeta, f,
-                     blocks, accumulate_params);
-      NRS_LAUNCHED(ctx);
-      return NRS_OK;
+      return fold_params(ctx, partial, dgamma, dbeta, f, blocks, accumulate_params);
     }
   }
   if (vpl) {
@@ -651,10 +622,8 @@ int layernorm_bwd(nrs_ctx* ctx, const char* who, const float* g, const float* xh
     if (dgamma && blocks > 4 * ctx->sm_count) blocks = 4 * ctx->sm_count;   // one resident wave of longer-lived blocks: fewer partial rows to fold
     float* partial = nullptr;
     if (dgamma) {
-      void* ws = nullptr;
-      const int st = nrs_workspace(ctx, (size_t)blocks * 2 * f * sizeof(float), &ws);
+      const int st = nrs_fold_partial(ctx, -1, (size_t)blocks * 2 * f * sizeof(float), &partial);
       if (st != NRS_OK) return st;
-      partial = (float*)ws;
     }
     const size_t smem = dgamma ? (size_t)warps * 2 * f * sizeof(float) : 0;
     if (dx && d_hi)
@@ -665,12 +634,7 @@ int layernorm_bwd(nrs_ctx* ctx, const char* who, const float* g, const float* xh
                                            dx2, partial, rows, f, acc1, acc2, (float*)nullptr, (float*)nullptr));
     if (emitted && dx && d_hi) *emitted = 1;
     NRS_LAUNCHED(ctx);
-    if (dgamma) {
-      NRS_PDL_LAUNCH(ln_param_fold_kernel, nrs_blocks(2 * (size_t)f, 32), 256, 0, ctx->stream, (const float*)partial, dgamma, dbeta, f,
-                     blocks, accumulate_params);
-      NRS_LAUNCHED(ctx);
-    }
-    return NRS_OK;
+    return dgamma ? fold_params(ctx, partial, dgamma, dbeta, f, blocks, accumulate_params) : NRS_OK;
   }
   if (dx) {
     NRS_PDL_LAUNCH(ln_dx_kernel, row_grid(ctx, rows), kRowThreads, 0, ctx->stream, g, xhat, istd, gamma, dx, dx2, rows, f, acc1, acc2);
@@ -682,14 +646,12 @@ int layernorm_bwd(nrs_ctx* ctx, const char* who, const float* g, const float* xh
     if (splits > rows / 32) splits = rows / 32;
     if (splits < 1) splits = 1;
     if (splits > 65535) splits = 65535;
-    void* ws = nullptr;
-    const int st = nrs_workspace(ctx, (size_t)splits * 2 * f * sizeof(float), &ws);
+    float* ws = nullptr;
+    const int st = nrs_fold_partial(ctx, -1, (size_t)splits * 2 * f * sizeof(float), &ws);
     if (st != NRS_OK) return st;
-    NRS_PDL_LAUNCH(ln_param_kernel, dim3(col_blocks, splits), 256, 0, ctx->stream, g, xhat, (float*)ws, rows, f, splits);
+    NRS_PDL_LAUNCH(ln_param_kernel, dim3(col_blocks, splits), 256, 0, ctx->stream, g, xhat, ws, rows, f, splits);
     NRS_LAUNCHED(ctx);
-    NRS_PDL_LAUNCH(ln_param_fold_kernel, nrs_blocks(2 * (size_t)f, 32), 256, 0, ctx->stream, (const float*)ws, dgamma, dbeta, f, splits,
-                   accumulate_params);
-    NRS_LAUNCHED(ctx);
+    return fold_params(ctx, ws, dgamma, dbeta, f, splits, accumulate_params);
   }
   return NRS_OK;
 }

@@ -121,6 +121,32 @@ struct NrsStatSync {
   void* user = nullptr;
 };
 
+// One fold (fold.cu).  Kinds: column sums; the partial tiles of the general and of the row-streaming weight gradient.
+enum { NRS_FOLD_COLUMNS = 0, NRS_FOLD_WGRAD = 1, NRS_FOLD_WGRAD_ROWS = 2 };
+struct NrsFoldJob {
+  const float* src;
+  float* dst;
+  float* scratch;          // columns with several row splits: [splits][cols]
+  unsigned* tickets;
+  unsigned first_block;
+  int kind, accumulate, splits, lanes;
+  union { int rows; int co; };
+  union { int cols; int ci; };
+  union { int stride; int taps; };
+  // weight gradients: the partial tiles' layout (see the kernels)
+  int taps_per_group, n_groups, col_blocks, cblocks, group_cols;
+  int chunk, n_chunks, jtypes, a_blocks, pack;
+  int out_cols;            // general kernel, 1x1: the columns are several [co][out_cols] matrices side by side (0: one)
+  size_t split_stride;     // floats between two splits
+};
+struct NrsFolds {
+  bool active = false;
+  std::vector<NrsFoldJob> jobs;
+  unsigned tickets_used = 1;
+  std::vector<std::pair<void*, size_t>> chunks;   // memory for partial sums that wait
+  size_t chunk = 0, used = 0;
+};
+
 struct nrs_ctx {
   int device = 0;
   cudaStream_t own_stream = nullptr;
@@ -157,6 +183,7 @@ struct nrs_ctx {
   // does not read (see NRS_PDL_PROLOGUE): that launch may overlap it.  Consumed by the launch.
   bool independent_next = false;
   NrsStatSync stat_sync;
+  NrsFolds folds;
   // Counter-based generator state of the dropout masks (dropout.cu): seed, and the next unused counter block.
   uint64_t rng_seed = 0, rng_offset = 0;
   // A process that works on samples [shard_begin, shard_begin + shard_local) of a batch of shard_global
@@ -194,7 +221,7 @@ int nrs_fail(nrs_ctx* ctx, int code, const char* fmt, ...);
 int nrs_workspace(nrs_ctx* ctx, size_t bytes, void** out);
 // (the weight-gradient kernels keep their split partials in a slot of their own: they may run while the
 // data gradient's K-split is still being folded out of NRS_WS_PARTIAL)
-enum { NRS_WS_A_HI = 0, NRS_WS_A_LO = 1, NRS_WS_B_HI = 2, NRS_WS_B_LO = 3, NRS_WS_PARTIAL = 4, NRS_WS_WGRAD_PARTIAL = 5, NRS_WS_COUNT = 8 };
+enum { NRS_WS_A_HI = 0, NRS_WS_A_LO = 1, NRS_WS_B_HI = 2, NRS_WS_B_LO = 3, NRS_WS_PARTIAL = 4, NRS_WS_WGRAD_PARTIAL = 5, NRS_WS_FOLD = 6, NRS_WS_COUNT = 8 };
 int nrs_ws_slot(nrs_ctx* ctx, int slot, size_t bytes, void** out);
 int nrs_err_flag(nrs_ctx* ctx, int** out);
 // Zero-initialised device counters (kNrsFoldTickets of them) for "the last block to arrive folds the partials"
@@ -335,9 +362,8 @@ inline cudaError_t nrs_pdl_launch(void (*kernel)(P...), dim3 grid, dim3 block, s
 #define NRS_PDL_LAUNCH(kernel, grid, block, smem, stream, ...) \
   (void)nrs_pdl_launch(kernel, dim3(grid), dim3(block), (size_t)(smem), stream, __VA_ARGS__)
 
-// Split reduces of the weight-gradient kernels: threads per block, and how many of them share one output
-// (each summing every lanes-th split) for a given number of splits.
-constexpr int kReduceThreads = 256;
+// How many threads share one output of a weight gradient's split reduce (each summing every lanes-th split) for a
+// given number of splits.
 static inline int reduce_lanes(int splits) { return splits >= 32 ? 8 : splits >= 16 ? 4 : splits >= 8 ? 2 : 1; }
 
 static inline unsigned nrs_blocks(size_t work, unsigned per_block) {

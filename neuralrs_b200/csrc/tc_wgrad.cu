@@ -27,6 +27,7 @@
 //
 // Replaces conv2d_im2col + conv2d_out2mm + matmul_nt_splitk (src/cuda/nn/conv.rs:
 // 298-320).
+#include "fold.h"
 #include "tc_mainloop.cuh"
 
 namespace {
@@ -225,54 +226,6 @@ tc_wgrad_kernel(const __grid_constant__ CUtensorMap tm_dy_hi, const __grid_const
   }
 }
 
-// dw[co][ci][tap] (+)= sum over splits of partial[split][mb][grp][row][t*cblocks*32 + c].  A block is
-// (kReduceThreads / lanes) outputs x `lanes` split lanes: lane y sums splits y, y+lanes, ... and the lanes are
-// combined in lane order through shared memory, so the order of the additions is fixed (bit-reproducible)
-// while the loads of one output are spread over `lanes` threads instead of one serial chain.
-__global__ void __launch_bounds__(kReduceThreads)
-tc_wgrad_reduce_kernel(const WgradParams p, int splits, int lanes, float* __restrict__ dw, int accumulate) {
-  NRS_PDL_PROLOGUE();
-  __shared__ float4 lane_sum[kReduceThreads];
-  const int per_block = kReduceThreads / lanes;   // output quads of this block
-  const int lane = threadIdx.x / per_block, slot = threadIdx.x - lane * per_block;
-  const int taps = p.kh * p.kw;
-  const int cq = (p.ci + 3) / 4;                  // a thread owns four consecutive input channels (padded in the partials)
-  const size_t total = (size_t)p.co * cq * taps;
-  const size_t idx = (size_t)blockIdx.x * per_block + slot;
-  const bool live = idx < total;
-  // idx enumerates (co, tap, ci/4) so that reads of the partials are coalesced 128-bit loads along ci
-  const int c = (int)(idx % cq) * 4;
-  const int tap = (int)((idx / cq) % taps);
-  const int co = (int)(idx / ((size_t)cq * taps));
-  const int mb = co / 128, row = co - mb * 128;
-  const int grp = tap / p.taps_per_group, t = tap - grp * p.taps_per_group;
-  const size_t tile = (size_t)128 * p.group_cols;
-  const int cbk = p.col_blocks > 1 ? c / 256 : 0;
-  const size_t col = p.col_blocks > 1 ? (size_t)(c - cbk * 256) : (size_t)t * p.cblocks * 32 + c;
-  const size_t off = ((((size_t)mb * p.n_groups + grp) * p.col_blocks + cbk) * 128 + row) * p.group_cols + col;
-  const size_t split_stride = (size_t)p.m_blocks * p.n_groups * p.col_blocks * tile;
-  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (live) {
-#pragma unroll 4
-    for (int z = lane; z < splits; z += lanes) {
-      const float4 v = *reinterpret_cast<const float4*>(p.partial + (size_t)z * split_stride + off);
-      s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
-    }
-  }
-  lane_sum[threadIdx.x] = s;
-  __syncthreads();
-  if (lane != 0 || !live) return;
-  for (int l = 1; l < lanes; ++l) {
-    const float4 v = lane_sum[l * per_block + slot];
-    s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
-  }
-  float* dst = dw + ((size_t)co * p.ci + c) * taps + tap;
-  const float r[4] = {s.x, s.y, s.z, s.w};
-#pragma unroll
-  for (int k = 0; k < 4; ++k)
-    if (c + k < p.ci) dst[(size_t)k * taps] = accumulate ? dst[(size_t)k * taps] + r[k] : r[k];
-}
-
 // Pixel tile = one TMA box {32 channels, Wt, Ht, Nt} of kp = Wt*Ht*Nt pixels, a multiple of 8 (a K-step) up to 64.
 // Boxes of whole rows, or of a multiple of 8 pixels of a row; the one that walks the fewest pixels, padding included,
 // is taken, where every tile costs about 6 pixels' worth of ring bookkeeping (measured: 16-pixel tiles with a deeper
@@ -380,11 +333,12 @@ int nrs_tc_conv_wgrad(nrs_ctx* ctx, const float* x, const float* dy, float* dw, 
   const int dy_ld = nrs_plane_ld(co), x_ld = nrs_plane_ld(ci);
   const size_t dy_plane = (size_t)n * oh * ow * dy_ld, x_plane = (size_t)n * h * wd * x_ld;
   const size_t partial_floats = (size_t)splits * p.m_blocks * p.n_groups * p.col_blocks * 128 * p.group_cols;
-  void *dy_hi = nullptr, *dy_lo = nullptr, *x_hi = nullptr, *x_lo = nullptr, *part = nullptr;
-  bool may_overlap = ctx->independent_next;   // withdrawn below if this call stages an operand itself
-  int st = nrs_ws_slot(ctx, NRS_WS_WGRAD_PARTIAL, partial_floats * sizeof(float), &part);
+  void *dy_hi = nullptr, *dy_lo = nullptr, *x_hi = nullptr, *x_lo = nullptr;
+  // a single split of a 1x1 "convolution" (A^T B) that overwrites its output needs no second pass
+  p.direct = (splits == 1 && taps == 1 && ci % 32 == 0 && !accumulate && (reinterpret_cast<uintptr_t>(dw) & 15) == 0) ? dw : nullptr;
+  int st = p.direct ? NRS_OK : nrs_fold_partial(ctx, NRS_WS_WGRAD_PARTIAL, partial_floats * sizeof(float), &p.partial);
   if (st != NRS_OK) return st;
-  p.partial = (float*)part;
+  bool may_overlap = ctx->independent_next;   // withdrawn below if this call stages an operand itself
   if (const NrsPlanes* ready = nrs_planes_find(ctx, dy, split3)) {
     dy_hi = ready->hi;
     dy_lo = ready->lo;
@@ -425,8 +379,6 @@ int nrs_tc_conv_wgrad(nrs_ctx* ctx, const float* x, const float* dy, float* dw, 
   else { maps[1] = maps[0]; maps[3] = maps[2]; }
   NRS_REQUIRE(ctx, ok, NRS_ERR_CUDA, "tc_wgrad: cuTensorMapEncodeTiled failed");
   p.independent = may_overlap ? 1 : 0;
-  // a single split of a 1x1 "convolution" (A^T B) that overwrites its output needs no second pass
-  p.direct = (splits == 1 && taps == 1 && ci % 32 == 0 && !accumulate && (reinterpret_cast<uintptr_t>(dw) & 15) == 0) ? dw : nullptr;
 
 #define NRS_WG(PL)                                                                     \
   switch (stages) {                                                                    \
@@ -440,12 +392,16 @@ int nrs_tc_conv_wgrad(nrs_ctx* ctx, const float* x, const float* dy, float* dw, 
 #undef NRS_WG
   if (st != NRS_OK) return st;
   if (p.direct) return NRS_OK;
-  const size_t total = (size_t)co * ((ci + 3) / 4) * taps;
-  const int lanes = reduce_lanes(splits);
-  NRS_PDL_LAUNCH(tc_wgrad_reduce_kernel, nrs_blocks(total, kReduceThreads / lanes), kReduceThreads, 0, ctx->stream, p, splits, lanes, dw,
-                 accumulate);
-  NRS_LAUNCHED(ctx);
-  return NRS_OK;
+  // dw[co][ci][tap] (+)= sum over splits of partial[split][mb][grp][col block][row][t*cblocks*32 + c]
+  NrsFoldJob j{};
+  j.kind = NRS_FOLD_WGRAD;
+  j.src = p.partial; j.dst = dw;
+  j.accumulate = accumulate; j.splits = splits; j.lanes = reduce_lanes(splits);
+  j.co = co; j.ci = ci; j.taps = taps;
+  j.taps_per_group = p.taps_per_group; j.n_groups = p.n_groups; j.col_blocks = p.col_blocks; j.cblocks = p.cblocks;
+  j.group_cols = p.group_cols;
+  j.split_stride = (size_t)p.m_blocks * p.n_groups * p.col_blocks * 128 * p.group_cols;
+  return nrs_fold_submit(ctx, j);
 }
 
 // C[m,n] (+)= A^T B for A stored [k][m] and B stored [k][n] (both row-major) without transposing either:

@@ -34,6 +34,7 @@
 //
 // Replaces conv2d_im2col + conv2d_out2mm + matmul_nt_splitk (src/cuda/nn/conv.rs:
 // 298-320) for the shapes it covers; everything else takes tc_wgrad.cu.
+#include "fold.h"
 #include "tc_mainloop.cuh"
 
 namespace {
@@ -281,57 +282,6 @@ tc_wgrad_rows_kernel(const __grid_constant__ CUtensorMap tm_dy_hi, const __grid_
   }
 }
 
-// dw[co][ci][i][j] (+)= sum over splits of the partial accumulators.  A block is
-// (kReduceThreads / lanes) outputs x `lanes` split lanes: lane y sums splits y, y+lanes, ... and the lanes are
-// combined in lane order through shared memory: a fixed order of additions (bit-reproducible) without one
-// serial load chain per output.
-__global__ void __launch_bounds__(kReduceThreads)
-tc_wgrad_rows_reduce_kernel(const RowParams p, int splits, int ctas, int lanes, float* __restrict__ dw, int accumulate) {
-  NRS_PDL_PROLOGUE();
-  __shared__ float4 lane_sum[kReduceThreads];
-  const int per_block = kReduceThreads / lanes;   // output quads of this block
-  const int lane = threadIdx.x / per_block, slot = threadIdx.x - lane * per_block;
-  const int cq = p.ci / 4;                        // a thread owns four consecutive input channels (ci % 32 == 0)
-  const size_t total = (size_t)p.co * 9 * cq;
-  const size_t idx = (size_t)blockIdx.x * per_block + slot;
-  const bool live = idx < total;
-  // idx enumerates (co, j, i, ci/4): consecutive threads read consecutive 128-bit groups of partial columns
-  const int ci = (int)(idx % cq) * 4;
-  const int i = (int)((idx / cq) % 3);
-  const int j = (int)((idx / ((size_t)cq * 3)) % 3);
-  const int co = (int)(idx / ((size_t)cq * 9));
-  int mb = co / 128, row = co - mb * 128, jk = j;
-  if (p.pack) {   // tap 1 -> kind 0 rows [0,h); tap 0 -> kind 0 rows [h,2h); tap 2 -> kind 1 rows [0,h)
-    mb = 0;
-    jk = j == 2 ? 1 : 0;
-    row = co + (j == 0 ? 32 * p.a_blocks : 0);
-  }
-  const int cc = ci / p.chunk, c = ci - cc * p.chunk;
-  const int cta = (mb * p.jtypes + jk) * p.n_chunks + cc;
-  const size_t cols = (size_t)kTaps * p.chunk;
-  const size_t off = ((size_t)cta * 128 + row) * cols + (size_t)i * p.chunk + c;
-  const size_t split_stride = (size_t)ctas * 128 * cols;
-  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (live) {
-#pragma unroll 4
-    for (int z = lane; z < splits; z += lanes) {
-      const float4 v = *reinterpret_cast<const float4*>(p.partial + (size_t)z * split_stride + off);
-      s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
-    }
-  }
-  lane_sum[threadIdx.x] = s;
-  __syncthreads();
-  if (lane != 0 || !live) return;
-  for (int l = 1; l < lanes; ++l) {
-    const float4 v = lane_sum[l * per_block + slot];
-    s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
-  }
-  float* dst = dw + (((size_t)co * p.ci + ci) * 3 + i) * 3 + j;
-  const float r[4] = {s.x, s.y, s.z, s.w};
-#pragma unroll
-  for (int k = 0; k < 4; ++k) dst[(size_t)k * 9] = accumulate ? dst[(size_t)k * 9] + r[k] : r[k];
-}
-
 template <int NPLANES, int KS>
 int launch_rows(nrs_ctx* ctx, const CUtensorMap* maps, const RowParams& p, int ctas, int splits, size_t smem_bytes) {
   static NrsSmemAttr attr;
@@ -396,11 +346,10 @@ int nrs_tc_conv_wgrad_rows(nrs_ctx* ctx, const float* x, const float* dy, float*
   // workspaces: NHWC planes of dy and x (or the caller's registered planes), and the partial tiles
   const size_t dy_plane = (size_t)n * h * wd * co, x_plane = (size_t)n * h * wd * ci;
   const size_t partial_floats = (size_t)splits * ctas * 128 * kTaps * p.chunk;
-  void *dy_hi = nullptr, *dy_lo = nullptr, *x_hi = nullptr, *x_lo = nullptr, *part = nullptr;
-  bool may_overlap = ctx->independent_next;   // withdrawn below if this call stages an operand itself
-  int st = nrs_ws_slot(ctx, NRS_WS_WGRAD_PARTIAL, partial_floats * sizeof(float), &part);
+  void *dy_hi = nullptr, *dy_lo = nullptr, *x_hi = nullptr, *x_lo = nullptr;
+  int st = nrs_fold_partial(ctx, NRS_WS_WGRAD_PARTIAL, partial_floats * sizeof(float), &p.partial);
   if (st != NRS_OK) return st;
-  p.partial = (float*)part;
+  bool may_overlap = ctx->independent_next;   // withdrawn below if this call stages an operand itself
   const size_t dy_img = (size_t)h * wd * co, x_img = (size_t)h * wd * ci;
   if (const NrsPlanes* ready = nrs_planes_find(ctx, dy, split3)) {
     dy_hi = ready->hi;
@@ -443,10 +392,13 @@ int nrs_tc_conv_wgrad_rows(nrs_ctx* ctx, const float* x, const float* dy, float*
     default: st = split3 ? launch_rows<2, 8>(ctx, maps, p, ctas, splits, smem_bytes) : launch_rows<1, 8>(ctx, maps, p, ctas, splits, smem_bytes); break;
   }
   if (st != NRS_OK) return st;
-  const size_t total = (size_t)co * ci * 9;
-  const int lanes = reduce_lanes(splits);
-  NRS_PDL_LAUNCH(tc_wgrad_rows_reduce_kernel, nrs_blocks(total / 4, kReduceThreads / lanes), kReduceThreads, 0, ctx->stream, p, splits,
-                 ctas, lanes, dw, accumulate);
-  NRS_LAUNCHED(ctx);
-  return NRS_OK;
+  // dw[co][ci][i][j] (+)= sum over splits of the partial accumulators
+  NrsFoldJob jb{};
+  jb.kind = NRS_FOLD_WGRAD_ROWS;
+  jb.src = p.partial; jb.dst = dw;
+  jb.accumulate = accumulate; jb.splits = splits; jb.lanes = reduce_lanes(splits);
+  jb.co = co; jb.ci = ci; jb.taps = 9;
+  jb.chunk = p.chunk; jb.n_chunks = p.n_chunks; jb.jtypes = p.jtypes; jb.a_blocks = p.a_blocks; jb.pack = p.pack;
+  jb.split_stride = (size_t)ctas * 128 * kTaps * p.chunk;
+  return nrs_fold_submit(ctx, jb);
 }
