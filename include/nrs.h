@@ -122,6 +122,11 @@ int nrs_free(nrs_ctx* ctx, void* dptr);
 int nrs_memset_zero(nrs_ctx* ctx, void* dptr, size_t bytes);
 int nrs_h2d(nrs_ctx* ctx, void* dst_dev, const void* src_host, size_t bytes);
 int nrs_d2h(nrs_ctx* ctx, void* dst_host, const void* src_dev, size_t bytes); /* waits */
+/* Pinned (page-locked) host memory for read-backs and staging: nrs_d2h into it runs at
+ * the bus rate, three times that of pageable memory.  Needs no context; expensive to
+ * obtain, so keep and reuse blocks.  No reference counterpart. */
+int nrs_host_alloc(size_t bytes, void** out);
+int nrs_host_free(void* ptr);
 int nrs_d2d(nrs_ctx* ctx, void* dst_dev, const void* src_dev, size_t bytes);
 int nrs_sync(nrs_ctx* ctx);
 

@@ -4,10 +4,7 @@
 #include "fold.h"
 #include "nrs_internal.h"
 
-#include <algorithm>
-#include <atomic>
 #include <cstring>
-#include <thread>
 
 static thread_local std::string g_no_ctx_error;
 
@@ -134,98 +131,22 @@ NrsProfScope::~NrsProfScope() {
   if (cudaEventRecord(rec.stop, ctx->stream) == cudaSuccess) ctx->prof_records.push_back(rec);
 }
 
-// Device -> pageable host memory through pinned slots of the context's own: one copy and one wait for small reads; for
-// larger ones the bus fills one slot while host threads empty the others (a single thread moves some 17 GB/s into
-// fresh pages, the bus 52).  8 MB into a new numpy array: 0.54 ms as one cudaMemcpyAsync, 0.2 here.
+// Device -> host: small reads into pageable memory go through a pinned slot of the context's own (one copy, one wait,
+// one memcpy: 64 KB 23 -> 15 us); larger ones, and pinned destinations (nrs_host_alloc), are one asynchronous copy.
 namespace {
-constexpr size_t kBounceSlot = 512 * 1024;
-constexpr int kBounceSlots = 4;
-
-int bounce_ready(nrs_ctx* ctx) {
-  if (ctx->bounce) return NRS_OK;
-  void* h = nullptr;
-  NRS_CUDA(ctx, cudaHostAlloc(&h, kBounceSlot * kBounceSlots, cudaHostAllocPortable));
-  ctx->bounce = h;
-  for (int i = 0; i < kBounceSlots; ++i) NRS_CUDA(ctx, cudaEventCreateWithFlags(&ctx->bounce_ev[i], cudaEventDisableTiming));
-  return NRS_OK;
-}
-}  // namespace
-
-static void nrs_bounce_free(nrs_ctx* ctx) {
-  for (cudaEvent_t& e : ctx->bounce_ev)
-    if (e) cudaEventDestroy(e);
-  if (ctx->bounce) cudaFreeHost(ctx->bounce);
-  ctx->bounce = nullptr;
+constexpr size_t kBounceBytes = 256 * 1024;
 }
 
 static int nrs_bounce_d2h(nrs_ctx* ctx, void* dst, const void* src, size_t bytes) {
-  cudaPointerAttributes attr;
-  if (cudaPointerGetAttributes(&attr, dst) == cudaSuccess && attr.type == cudaMemoryTypeHost) {   // pinned already
+  if (bytes > kBounceBytes) {
     NRS_CUDA(ctx, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
     NRS_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     return NRS_OK;
   }
-  (void)cudaGetLastError();
-  int st = bounce_ready(ctx);
-  if (st != NRS_OK) return st;
-  uint8_t* ring = (uint8_t*)ctx->bounce;
-  if (bytes <= kBounceSlot) {
-    NRS_CUDA(ctx, cudaMemcpyAsync(ring, src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
-    NRS_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    std::memcpy(dst, ring, bytes);
-    return NRS_OK;
-  }
-  // Chunk i goes through slot i % kBounceSlots and is emptied by worker i % kBounceSlots (this thread is worker 0); a
-  // worker that has emptied its slot says so, and this thread then queues the slot's next chunk.
-  const size_t chunks = (bytes + kBounceSlot - 1) / kBounceSlot;
-  std::atomic<int> failed{0};
-  std::atomic<size_t> filled[kBounceSlots], emptied[kBounceSlots];
-  for (int s = 0; s < kBounceSlots; ++s) { filled[s] = 0; emptied[s] = 0; }
-  auto queue = [&](size_t i) -> cudaError_t {
-    const size_t n = std::min(kBounceSlot, bytes - i * kBounceSlot);
-    const int s = (int)(i % kBounceSlots);
-    cudaError_t e = cudaMemcpyAsync(ring + s * kBounceSlot, (const uint8_t*)src + i * kBounceSlot, n, cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess) e = cudaEventRecord(ctx->bounce_ev[s], ctx->stream);
-    filled[s].fetch_add(1, std::memory_order_release);
-    return e;
-  };
-  cudaError_t err = cudaSuccess;
-  for (size_t i = 0; i < chunks && i < (size_t)kBounceSlots && err == cudaSuccess; ++i) err = queue(i);
-  auto drain = [&](int s, size_t i) {   // empties chunk i out of slot s once its copy has landed
-    if (cudaEventSynchronize(ctx->bounce_ev[s]) != cudaSuccess) { failed = 1; return; }
-    std::memcpy((uint8_t*)dst + i * kBounceSlot, ring + s * kBounceSlot, std::min(kBounceSlot, bytes - i * kBounceSlot));
-    emptied[s].fetch_add(1, std::memory_order_release);
-  };
-  const int workers = (int)std::min<size_t>(kBounceSlots, chunks);
-  std::thread helper[kBounceSlots];
-  for (int s = 1; s < workers; ++s)
-    helper[s] = std::thread([&, s] {
-      cudaSetDevice(ctx->device);
-      size_t turn = 0;
-      for (size_t i = s; i < chunks && !failed; i += kBounceSlots, ++turn) {
-        while (filled[s].load(std::memory_order_acquire) <= turn && !failed) std::this_thread::yield();
-        if (!failed) drain(s, i);
-      }
-    });
-  size_t next = std::min<size_t>(kBounceSlots, chunks), mine = 0;
-  while (err == cudaSuccess && !failed && (next < chunks || mine < chunks)) {
-    const int s = (int)(next % kBounceSlots);
-    if (next < chunks && emptied[s].load(std::memory_order_acquire) == next / kBounceSlots) {
-      err = queue(next++);
-    } else if (mine < chunks && mine < next) {
-      drain(0, mine);
-      mine += kBounceSlots;
-    } else {
-      std::this_thread::yield();
-    }
-  }
-  if (err != cudaSuccess) failed = 1;
-  for (int s = 1; s < workers; ++s) helper[s].join();
-  if (failed) {
-    cudaStreamSynchronize(ctx->stream);   // nothing may still write into the slots
-    return nrs_fail(ctx, NRS_ERR_CUDA, "nrs_d2h: a chunk's copy failed: %s", cudaGetErrorString(err != cudaSuccess ? err : cudaGetLastError()));
-  }
+  if (!ctx->bounce) NRS_CUDA(ctx, cudaHostAlloc(&ctx->bounce, kBounceBytes, cudaHostAllocPortable));
+  NRS_CUDA(ctx, cudaMemcpyAsync(ctx->bounce, src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
   NRS_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  std::memcpy(dst, ctx->bounce, bytes);
   return NRS_OK;
 }
 
@@ -330,7 +251,7 @@ int nrs_destroy(nrs_ctx* ctx) {
   if (ctx->workspace) cudaFree(ctx->workspace);
   for (int i = 0; i < NRS_WS_COUNT; ++i) if (ctx->ws_slot[i]) cudaFree(ctx->ws_slot[i]);
   if (ctx->err_host) cudaFreeHost((void*)ctx->err_host);
-  nrs_bounce_free(ctx);
+  if (ctx->bounce) cudaFreeHost(ctx->bounce);
   nrs_folds_free(ctx);
   if (ctx->fold_ticket) cudaFree(ctx->fold_ticket);
   for (auto& r : ctx->prof_records) { cudaEventDestroy(r.start); cudaEventDestroy(r.stop); }
@@ -430,6 +351,25 @@ int nrs_d2h(nrs_ctx* ctx, void* dst_host, const void* src_dev, size_t bytes) {
     NRS_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   }
   return nrs_check_device_error(ctx);
+}
+
+int nrs_host_alloc(size_t bytes, void** out) {
+  if (!out) return nrs_fail(nullptr, NRS_ERR_ARG, "nrs_host_alloc: null out pointer");
+  *out = nullptr;
+  if (cudaHostAlloc(out, bytes ? bytes : 1, cudaHostAllocPortable) != cudaSuccess) {
+    (void)cudaGetLastError();
+    *out = nullptr;
+    return nrs_fail(nullptr, NRS_ERR_ALLOC, "nrs_host_alloc: no pinned memory for %zu bytes", bytes);
+  }
+  return NRS_OK;
+}
+
+int nrs_host_free(void* ptr) {
+  if (ptr && cudaFreeHost(ptr) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return nrs_fail(nullptr, NRS_ERR_ARG, "nrs_host_free: not a pinned block of nrs_host_alloc");
+  }
+  return NRS_OK;
 }
 
 int nrs_d2d(nrs_ctx* ctx, void* dst_dev, const void* src_dev, size_t bytes) {

@@ -242,11 +242,9 @@ void to_cuda(const NodeP& n) {
   r->grad_valid = false;
 }
 
-std::vector<float> to_host(const NodeP& n) {
+void to_host(const NodeP& n, float* host_out) {
   require_gpu(n, "to_host: node");
-  std::vector<float> out(n->len());
-  check(n->ctx, nrs_d2h(n->ctx, out.data(), n->data, out.size() * sizeof(float)));
-  return out;
+  check(n->ctx, nrs_d2h(n->ctx, host_out, n->data, n->len() * sizeof(float)));
 }
 
 void set_grad(const NodeP& n, const float* host) {
@@ -258,12 +256,11 @@ void set_grad(const NodeP& n, const float* host) {
   r->grad_valid = true;
 }
 
-std::vector<float> read_grad(const NodeP& n) {
+void read_grad(const NodeP& n, float* host_out) {
   require_gpu(n, "read_grad: node");
   Node* r = grad_root(n.get());
-  std::vector<float> out(r->len(), 0.0f);
-  if (r->grad && r->grad_valid) check(n->ctx, nrs_d2h(n->ctx, out.data(), r->grad, out.size() * sizeof(float)));
-  return out;
+  if (r->grad && r->grad_valid) check(n->ctx, nrs_d2h(n->ctx, host_out, r->grad, r->len() * sizeof(float)));
+  else std::memset(host_out, 0, r->len() * sizeof(float));
 }
 
 void zero_grad(const std::vector<NodeP>& params) {

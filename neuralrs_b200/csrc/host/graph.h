@@ -111,9 +111,9 @@ namespace cuda {
 
 // ---- runtime (src/cuda/runtime.rs:39-124)
 void to_cuda(const NodeP& n);
-std::vector<float> to_host(const NodeP& n);
+void to_host(const NodeP& n, float* host_out);     // len() floats; waits
 void set_grad(const NodeP& n, const float* host);
-std::vector<float> read_grad(const NodeP& n);
+void read_grad(const NodeP& n, float* host_out);   // zeros where nothing wrote it; waits
 void zero_grad(const std::vector<NodeP>& params);
 void synchronize(nrs_ctx* ctx);
 // Re-homes resident parameters into one FlatStore (values are preserved).

@@ -130,8 +130,7 @@ int nrs_to_host(nrs_node* n, float* host_out) {
   NODE_OK(n);
   if (!host_out && n->p->len()) return nrs_fail(ctx_of(n), NRS_ERR_ARG, "nrs_to_host: null output");
   return guarded(ctx_of(n), [&] {
-    auto v = nrs::cuda::to_host(n->p);
-    std::memcpy(host_out, v.data(), v.size() * sizeof(float));
+    nrs::cuda::to_host(n->p, host_out);
   });
 }
 
@@ -145,8 +144,7 @@ int nrs_read_grad(nrs_node* n, float* host_out) {
   NODE_OK(n);
   if (!host_out && n->p->len()) return nrs_fail(ctx_of(n), NRS_ERR_ARG, "nrs_read_grad: null output");
   return guarded(ctx_of(n), [&] {
-    auto v = nrs::cuda::read_grad(n->p);
-    std::memcpy(host_out, v.data(), v.size() * sizeof(float));
+    nrs::cuda::read_grad(n->p, host_out);
   });
 }
 

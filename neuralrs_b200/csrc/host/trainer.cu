@@ -827,8 +827,7 @@ int nrs_trainer_get_grad(nrs_trainer* t, int i, float* host_out) {
   if (!t) return nrs_fail(nullptr, NRS_ERR_ARG, "nrs_trainer_get_grad: null handle");
   NRS_REQUIRE(t->ctx, host_out && i >= 0 && i < (int)t->params.size(), NRS_ERR_ARG, "nrs_trainer_get_grad: bad index or null output");
   return guarded(t->ctx, [&] {
-    auto v = nrs::cuda::read_grad(t->params[i]);
-    std::memcpy(host_out, v.data(), v.size() * sizeof(float));
+    nrs::cuda::read_grad(t->params[i], host_out);
   });
 }
 

@@ -165,9 +165,7 @@ struct nrs_ctx {
   // Device word the tensor-core kernels set when a bounded wait runs out; read at sync points.
   int* err_flag = nullptr;
   volatile int* err_host = nullptr;  // the same word as the host sees it (mapped memory)
-  // Pinned slots for read-backs into pageable memory (ctx.cu), made on first use.
-  void* bounce = nullptr;
-  cudaEvent_t bounce_ev[4] = {nullptr, nullptr, nullptr, nullptr};
+  void* bounce = nullptr;            // pinned slot for small read-backs into pageable memory, made on first use
   unsigned* fold_ticket = nullptr;   // arrival counter of kernels whose last block folds the blocks' partial sums
   // Planes registered for a source tensor (keyed by its device pointer); the conv kernels
   // use them instead of staging again.  Whoever registers keeps both alive and unregisters.
