@@ -227,6 +227,9 @@ static bool planes_possible(nrs_ctx* ctx) {
   return ctx->math_mode != NRS_MATH_FP32 && tc::tensor_map_encoder();
 }
 
+void cache_row_planes(const NodeP& x, size_t rows, size_t cols) { cache_planes_2d(x, rows, cols); }
+bool operand_planes_possible(nrs_ctx* ctx) { return planes_possible(ctx); }
+
 namespace cuda {
 
 // ------------------------------------------------------------------ runtime
@@ -323,8 +326,29 @@ NodeP matmul(const NodeP& a, const NodeP& b) {
     const float* dc = grad_in(self);
     GradPlanes dc_planes(ctx, dc, (size_t)m, (size_t)n, tensor_cores && a->requires_grad && b->requires_grad);
     if (a->requires_grad) {
+      const bool emit = a->row_planes_wanted && tensor_cores && k % 8 == 0 && !a->view_of && !a->grad_valid && !a->gplanes_hi;
       GradTarget t = grad_target(a);  // dA (+)= dC . B^T
-      check(ctx, nrs_gemm(ctx, 0, 1, m, k, n, dc, b->data, t.ptr, nullptr, NRS_ACT_NONE, t.accumulate ? 1.0f : 0.0f));
+      int st = NRS_ERR_UNSUPPORTED;
+      if (emit && !ctx->plane_hints.count(t.ptr)) {
+        NrsGemmExtras e;
+        e.hi = dalloc(ctx, a->len());
+        if (ctx->math_mode == NRS_MATH_3XTF32) e.lo = dalloc(ctx, a->len());
+        st = nrs_gemm_extras(ctx, 0, 1, m, k, n, dc, b->data, t.ptr, nullptr, NRS_ACT_NONE, 0.0f, &e);
+        if (st == NRS_OK) {
+          a->gplanes_hi = e.hi;
+          a->gplanes_lo = e.lo;
+          NrsPlanes pl{e.hi, e.lo, e.lo ? 1 : 0};
+          pl.rows = m;
+          pl.cols = k;
+          ctx->plane_hints[t.ptr] = pl;
+        } else {
+          nrs_free(ctx, e.hi);
+          if (e.lo) nrs_free(ctx, e.lo);
+        }
+      }
+      if (st == NRS_ERR_UNSUPPORTED)
+        st = nrs_gemm(ctx, 0, 1, m, k, n, dc, b->data, t.ptr, nullptr, NRS_ACT_NONE, t.accumulate ? 1.0f : 0.0f);
+      check(ctx, st);
     }
     if (b->requires_grad) {
       GradTarget t = grad_target(b);  // dB (+)= A^T . dC: reads nothing dA wrote, so it may start under dA's tail

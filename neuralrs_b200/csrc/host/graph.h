@@ -76,6 +76,10 @@ struct Node {
   const float* fold_src = nullptr;
   bool gz_valid = false;
 
+  // Set on a [rows, cols] result whose backward pass reads its incoming gradient as row planes only: the matmul that
+  // consumes it lets its input-gradient kernel write them (gplanes_*, registered under the gradient's address).
+  bool row_planes_wanted = false;
+
   size_t len() const;
   bool on_gpu() const { return data != nullptr; }
   ~Node();
@@ -106,6 +110,8 @@ struct GradSlot {
 GradSlot grad_slot(const NodeP& n);   // marks the gradient as written
 const float* grad_view(Node* n);      // a node's own incoming gradient (zeros if nothing wrote it)
 NodeP make_result(nrs_ctx* ctx, const std::vector<size_t>& shape, std::vector<NodeP> parents);
+void cache_row_planes(const NodeP& x, size_t rows, size_t cols);   // TF32 row planes of x's data, kept with the node
+bool operand_planes_possible(nrs_ctx* ctx);                        // a TF32 math mode on a device with TMA
 
 namespace cuda {
 

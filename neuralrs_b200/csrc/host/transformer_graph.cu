@@ -7,6 +7,8 @@
 #include <cmath>
 #include <cstring>
 
+#include "attention_planes.h"
+#include "fold.h"
 #include "host/graph.h"
 
 namespace nrs {
@@ -203,10 +205,127 @@ static NodeP permute_heads(const NodeP& x, size_t batch, size_t seq, size_t head
   return out;
 }
 
+// Projections and attention core over operand planes (attention_planes.cu) as one node: x [tokens, d] -> [tokens, d], the
+// heads' results side by side.  One product makes Q, K and V, one sums the three shares of x's gradient, one makes the
+// three weight gradients.
+static NodeP planes_attention(const MultiHeadAttention& m, const NodeP& x, size_t batch, size_t seq) {
+  nrs_ctx* ctx = x->ctx;
+  const size_t tokens = batch * seq, d = m.d_model, heads = m.num_heads, d_head = d / heads;
+  const bool split = ctx->math_mode == NRS_MATH_3XTF32;
+  const NodeP wq = m.w_q, wk = m.w_k, wv = m.w_v;
+  NodeP out = make_result(ctx, {tokens, d}, {x, wq, wk, wv});
+  auto block = [ctx](size_t floats) {
+    void* p = nullptr;
+    check(ctx, nrs_alloc(ctx, floats * sizeof(float), 0, &p));
+    return (float*)p;
+  };
+  auto saved = [&](size_t floats) {
+    float* p = block(floats);
+    out->saved.push_back(p);
+    return p;
+  };
+  cache_row_planes(x, tokens, d);   // read again by the weight gradients
+  NrsGemmExtras e;
+  e.skip_c = true;
+  e.hi = saved(tokens * 3 * d);
+  e.lo = split ? saved(tokens * 3 * d) : nullptr;
+  const float* w[3] = {wq->data, wk->data, wv->data};
+  check(ctx, nrs_tc_gemm_weights(ctx, 0, 3, (int)tokens, (int)d, (int)d, x->data, w, nullptr, 0.0f, &e));
+  const size_t square = batch * heads * seq * (size_t)nrs_plane_ld((int)seq);
+  NrsMhaPlanes a{};
+  a.batch = (int)batch; a.seq = (int)seq; a.heads = (int)heads; a.d_head = (int)d_head; a.causal = m.causal ? 1 : 0;
+  a.qkv_hi = e.hi; a.qkv_lo = e.lo; a.qkv_ld = (int)(3 * d);
+  a.p_hi = saved(square);
+  a.p_lo = split ? saved(square) : nullptr;
+  a.out = out->data;
+  a.out_hi = block(tokens * d);
+  a.out_lo = split ? block(tokens * d) : nullptr;
+  out->planes_hi = a.out_hi;        // the output projection reads them (and its weight gradient)
+  out->planes_lo = a.out_lo;
+  NrsPlanes pl{a.out_hi, a.out_lo, split ? 1 : 0};
+  pl.rows = (int)tokens;
+  pl.cols = (int)d;
+  ctx->plane_hints[out->data] = pl;
+  a.scores = block(square);
+  const int st = nrs_mha_planes_fwd(ctx, a);
+  nrs_free(ctx, a.scores);
+  check(ctx, st);
+  out->row_planes_wanted = true;
+  Node* self = out.get();
+  out->backward_fn = [self, x, wq, wk, wv, a, tokens, d, square, split, block]() mutable {
+    nrs_ctx* ctx = self->ctx;
+    const float* g = grad_view(self);
+    // the gradient's row planes: left by the output projection's input-gradient kernel, else staged here
+    float *ghi = self->gplanes_hi, *glo = self->gplanes_lo;
+    if (!ghi) {
+      ghi = block(tokens * d);
+      glo = split ? block(tokens * d) : nullptr;
+      check(ctx, nrs_tc_stage(ctx, g, ghi, glo, (int)tokens, (int)d, (int)d, 1, 0, 0, false));
+    } else {
+      ctx->plane_hints.erase(g);
+      self->gplanes_hi = self->gplanes_lo = nullptr;
+    }
+    a.dout_hi = ghi; a.dout_lo = glo;
+    a.scores = block(square);
+    a.ds_hi = block(square);
+    a.ds_lo = split ? block(square) : nullptr;
+    a.dqkv_hi = block(tokens * 3 * d);
+    a.dqkv_lo = split ? block(tokens * 3 * d) : nullptr;
+    struct Release {
+      nrs_ctx* c; std::vector<float*> p; const float* key;
+      ~Release() {
+        if (key) c->plane_hints.erase(key);
+        for (float* q : p) if (q) nrs_free(c, q);
+      }
+    } release{ctx, {ghi, glo, a.scores, a.ds_hi, a.ds_lo, a.dqkv_hi, a.dqkv_lo}, nullptr};
+    check(ctx, nrs_mha_planes_bwd(ctx, a));
+    NrsPlanes pl{a.dqkv_hi, a.dqkv_lo, split ? 1 : 0};
+    pl.rows = (int)tokens;
+    pl.cols = (int)(3 * d);
+    ctx->plane_hints[a.dqkv_hi] = pl;
+    release.key = a.dqkv_hi;
+    if (x->requires_grad) {
+      GradSlot t = grad_slot(x);
+      const float* w[3] = {wq->data, wk->data, wv->data};
+      check(ctx, nrs_tc_gemm_weights(ctx, 1, 3, (int)tokens, (int)d, (int)d, a.dqkv_hi, w, t.ptr, t.accumulate ? 1.0f : 0.0f, nullptr));
+    }
+    GradSlot s[3] = {grad_slot(wq), grad_slot(wk), grad_slot(wv)};
+    const size_t dd = d * d;
+    const bool side_by_side = s[1].ptr == s[0].ptr + dd && s[2].ptr == s[0].ptr + 2 * dd && s[0].accumulate == s[1].accumulate &&
+                              s[0].accumulate == s[2].accumulate;   // a trainer's flat block: one write for all three
+    float* dst = side_by_side ? s[0].ptr : block(3 * dd);
+    NrsIndependentNext overlap(ctx, x->requires_grad);   // reads nothing that dX wrote
+    check(ctx, nrs_tc_conv_wgrad(ctx, a.dqkv_hi, x->data, dst, (int)tokens, (int)(3 * d), 1, 1, (int)d, 1, 1, 1, 0,
+                                 side_by_side ? s[0].accumulate : 0, (int)d));
+    if (!side_by_side) {
+      release.p.push_back(dst);
+      check(ctx, nrs_folds_flush(ctx));
+      for (int i = 0; i < 3; ++i)
+        check(ctx, s[i].accumulate ? nrs_accumulate(ctx, s[i].ptr, dst + i * dd, dd)
+                                   : nrs_d2d(ctx, s[i].ptr, dst + i * dd, dd * sizeof(float)));
+    }
+  };
+  return out;
+}
+
+// Which form attention takes in a TF32 mode.  (The kernels of attention_tc.cu stay for nrs_attention_fwd / _bwd, whose
+// callers hold q, k, v as separate f32 tensors.)
+static bool planes_attention_applies(const MultiHeadAttention& m, const NodeP& x, size_t batch, size_t seq) {
+  const size_t d = m.d_model, tokens = batch * seq;
+  if (!operand_planes_possible(x->ctx) || d % 32 != 0 || tokens < 16 || tokens > 2147483647u / 3 / d) return false;
+  for (const NodeP& w : {m.w_q, m.w_k, m.w_v})
+    if (!w || !w->on_gpu() || !w->requires_grad || w->view_of || w->shape.size() != 2 || w->shape[0] != d || w->shape[1] != d) return false;
+  return nrs_mha_planes_applies(x->ctx, (int)seq, (int)(d / m.num_heads));
+}
+
 NodeP MultiHeadAttention::forward_batch(const NodeP& x) const {
   if (!x || x->shape.size() != 3) fail(NRS_ERR_SHAPE, "cuda mha: input must be [batch, seq, d_model]");
   const size_t batch = x->shape[0], seq = x->shape[1], d = x->shape[2];
   if (d != d_model || num_heads == 0 || d_model % num_heads != 0) fail(NRS_ERR_SHAPE, "cuda mha: d_model / num_heads mismatch");
+  if (x->on_gpu() && planes_attention_applies(*this, x, batch, seq)) {
+    NodeP flat = reshape(x, {batch * seq, d});
+    return reshape(matmul(planes_attention(*this, flat, batch, seq), w_o), {batch, seq, d});
+  }
   auto proj = [&](const NodeP& w) { return reshape(matmul(reshape(x, {batch * seq, d}), w), {batch, seq, d}); };
   NodeP q = proj(w_q), k = proj(w_k), v = proj(w_v);
   // The reference slices the heads out column by column, runs attention_batch per head and

@@ -389,6 +389,9 @@ struct NrsGemmExtras {
 };
 int nrs_tc_gemm(nrs_ctx* ctx, int trans_a, int trans_b, int batch, int m, int n, int k,
                 const float* a, const float* b, float* c, const float* bias, int act, float beta, NrsGemmExtras* extras = nullptr);
+// x times several weights of one shape in one product (tc_gemm.cu); NRS_ERR_UNSUPPORTED (no error text) outside its range.
+int nrs_tc_gemm_weights(nrs_ctx* ctx, int reduce, int count, int m, int n, int k, const float* x, const float* const* w, float* c,
+                        float beta, NrsGemmExtras* extras);
 // nrs_gemm with extras; NRS_ERR_UNSUPPORTED (no error text) when the product would not run on the tensor cores.
 int nrs_gemm_extras(nrs_ctx* ctx, int trans_a, int trans_b, int m, int n, int k, const float* a, const float* b, float* c,
                     const float* bias, int act, float beta, NrsGemmExtras* extras);
@@ -396,8 +399,9 @@ int nrs_tc_conv_fwd(nrs_ctx* ctx, const float* x, const float* w, const float* b
                     int wd, int co, int kh, int kw, int stride, int pad, int act);
 int nrs_tc_conv_dgrad(nrs_ctx* ctx, const float* w, const float* dy, float* dx, int n, int ci, int h, int wd, int co,
                       int kh, int kw, int stride, int pad, int accumulate);
+// out_cols (1x1 only): the ci columns are matrices of out_cols columns side by side, written one behind the other.
 int nrs_tc_conv_wgrad(nrs_ctx* ctx, const float* x, const float* dy, float* dw, int n, int ci, int h, int wd, int co,
-                      int kh, int kw, int stride, int pad, int accumulate);
+                      int kh, int kw, int stride, int pad, int accumulate, int out_cols = 0);
 bool nrs_gemm_on_tensor_cores(const nrs_ctx* ctx, int m, int n, int k);
 // Whether nrs_gemm's A^T B [m,n] runs on row planes of A and B (never on the f32 tensors): then a caller may hand it
 // planes without the tensor behind them.

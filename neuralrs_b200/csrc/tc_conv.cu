@@ -93,8 +93,9 @@ struct ConvPolicy {
     }
     c.b_col = weight_column(c);
   }
-  __device__ __forceinline__ void b_origin(const Cursor& c, int n0, int batch, int* b0, int* b1, int* b2) const {
-    *b0 = c.b_col; *b1 = n0; *b2 = batch;
+  template <int BN>
+  __device__ __forceinline__ void load_b(void* dst, const CUtensorMap* tm, uint64_t* bar, const Cursor& c, int n0) const {
+    tc::tma_load_3d(dst, tm, bar, c.b_col, n0, 0);
   }
   __device__ __forceinline__ void load_a(void* dst, const CUtensorMap* tm, uint64_t* bar, const Cursor& c) const {
     tc::tma_load_4d(dst, tm, bar, c.cb * 32, c.x, c.y, c.n);
@@ -129,7 +130,9 @@ struct ConvPolicy {
     }
   }
   static constexpr bool kCanEmit = true;
-  static constexpr bool kMnMajor = false;
+  static constexpr bool kAMnMajor = false, kBMnMajor = false;
+  static constexpr bool kMaySplit = true;
+  __device__ __forceinline__ bool clip(int, int, int, int*, int*) const { return true; }
   static constexpr int kEpiWarps = 4;   // 250 registers per thread: no room for more
   __device__ __forceinline__ float* colsum_row(int tile_m, int q) const {
     return colsum_partial ? colsum_partial + ((size_t)tile_m * 4 + q) * n_ch_out : nullptr;

@@ -32,7 +32,9 @@ struct GemmPolicy {
   // k / seg_k; 0 = one matrix.  The matrices are the batches of B's tensor map.
   int seg_n, seg_k;
   static constexpr bool kCanEmit = false;
-  static constexpr bool kMnMajor = MN;
+  static constexpr bool kAMnMajor = MN, kBMnMajor = MN;
+  static constexpr bool kMaySplit = true;
+  __device__ __forceinline__ bool clip(int, int, int, int*, int*) const { return true; }
   static constexpr int kEpiWarps = 8;   // the epilogue is latency (TMEM, loads, tanh), not registers: two warps per lane quarter
 
   __device__ __forceinline__ uint32_t a_slice_bytes() const { return tc::BM * tc::BK * 4; }
@@ -43,11 +45,13 @@ struct GemmPolicy {
     if (MN) tc::tma_load_3d(dst, tm, bar, 0, c.b_col, c.row / 32);
     else tc::tma_load_3d(dst, tm, bar, c.b_col, c.row, c.batch);
   }
-  __device__ __forceinline__ void b_origin(const Cursor& c, int n0, int batch, int* b0, int* b1, int* b2) const {
-    if (MN) { *b0 = 0; *b1 = c.b_col; *b2 = n0 / 32; return; }
-    *b0 = c.b_col; *b1 = n0; *b2 = batch;
-    if (seg_n) { *b2 = n0 / seg_n; *b1 = n0 - *b2 * seg_n; }
-    if (seg_k) { *b2 = c.b_col / seg_k; *b0 = c.b_col - *b2 * seg_k; }
+  template <int BN>
+  __device__ __forceinline__ void load_b(void* dst, const CUtensorMap* tm, uint64_t* bar, const Cursor& c, int n0) const {
+    if (MN) { tc::tma_load_3d(dst, tm, bar, 0, c.b_col, n0 / 32); return; }
+    int b0 = c.b_col, b1 = n0, b2 = c.batch;
+    if (seg_n) { b2 = n0 / seg_n; b1 = n0 - b2 * seg_n; }
+    if (seg_k) { b2 = c.b_col / seg_k; b0 = c.b_col - b2 * seg_k; }
+    tc::tma_load_3d(dst, tm, bar, b0, b1, b2);
   }
   __device__ __forceinline__ float dact(float src) const { return x.dact == NRS_ACT_RELU ? (src > 0.0f ? 1.0f : 0.0f) : nrs_gelu_d(src); }
   // One element, from the pass that sums a K-split.
@@ -368,6 +372,47 @@ int nrs_tc_gemm(nrs_ctx* ctx, int trans_a, int trans_b, int batch, int m, int n,
   if (batch > 1 && ((A.bstride % 4) || (B.bstride % 4))) return NRS_ERR_UNSUPPORTED;
   GemmPolicy<false> pol{c, bias, act, beta, m, n, (size_t)m * n, false, {}, 0, 0};
   return dispatch<false>(ctx, column_tile(ctx, m, n, batch), split, A, B, batch, n, batch, m, n, k, pol, extras);
+}
+
+// x[m,k] times several weight matrices w[i] of one shape, in one product.  `reduce` == 0: c[m, count*n] = x . [w0|w1|..]
+// (w[i]: [k][n] as stored).  `reduce` != 0: c[m,n] (+)= sum_i x_i . w[i]^T with x = [x_0|x_1|..] of `count` blocks of
+// `n_i` columns, w[i]: [n][n_i].  The weights' planes come from the context's weight set when they lie there at equal
+// distances (a trainer's), else they are staged side by side.
+int nrs_tc_gemm_weights(nrs_ctx* ctx, int reduce, int count, int m, int n, int k, const float* x, const float* const* w, float* c,
+                        float beta, NrsGemmExtras* extras) {
+  if (ctx->math_mode == NRS_MATH_FP32 || !tc::tensor_map_encoder() || m < 16 || n < 32 || k < 32) return NRS_ERR_UNSUPPORTED;
+  const bool split = ctx->math_mode == NRS_MATH_3XTF32;
+  const int form = reduce ? NRS_WF_LINEAR_ROWS : NRS_WF_LINEAR_T;
+  if (!reduce && n % 32 != 0) return NRS_ERR_UNSUPPORTED;   // a column tile belongs to one matrix
+  if (reduce && k % 32 != 0) return NRS_ERR_UNSUPPORTED;    // and so does a K-slice
+  Operand A, B{};
+  int st = prepare_operand(ctx, x, m, reduce ? count * k : k, 1, true, split, NRS_WS_A_HI, NRS_WS_A_LO, &A, false);
+  if (st != NRS_OK) return st;
+  bool found = true;
+  for (int i = 0; i < count && found; ++i) {
+    const NrsWeightPlanes* wp = nrs_weight_planes_find(ctx, w[i], form);
+    found = wp && wp->rows == n && wp->K == k;
+    if (!found) break;
+    if (i == 0) { B.hi = wp->hi; B.lo = wp->lo; B.ld = (k + 31) / 32 * 32; B.kdim = B.ld; }
+    else if (i == 1) { found = wp->hi > B.hi; B.bstride = (size_t)(wp->hi - B.hi); }
+    found = found && wp->hi == B.hi + (size_t)i * B.bstride && (!split || wp->lo == B.lo + (size_t)i * B.bstride);
+  }
+  if (!found) {
+    const int ld = nrs_plane_ld(k);
+    const size_t plane = (size_t)n * ld;
+    void *hi = nullptr, *lo = nullptr;
+    st = nrs_ws_slot(ctx, NRS_WS_B_HI, plane * count * sizeof(float), &hi);
+    if (st == NRS_OK && split) st = nrs_ws_slot(ctx, NRS_WS_B_LO, plane * count * sizeof(float), &lo);
+    for (int i = 0; i < count && st == NRS_OK; ++i)
+      st = nrs_tc_stage(ctx, w[i], (float*)hi + i * plane, split ? (float*)lo + i * plane : nullptr, n, k, ld, 1, 0, 0, !reduce);
+    if (st != NRS_OK) return st;
+    B = Operand{(const float*)hi, (const float*)lo, ld, k, plane};
+  }
+  const int cols = reduce ? n : count * n, kk = reduce ? count * k : k;
+  GemmPolicy<false> pol{c, nullptr, NRS_ACT_NONE, beta, m, cols, (size_t)m * cols, false, {}, reduce ? 0 : n, reduce ? k : 0};
+  const int limit = reduce ? 128 : n % 128 == 0 ? 128 : n % 64 == 0 ? 64 : 32;
+  NrsProfScope prof(ctx, NRS_PROF_GEMM, 2.0 * m * cols * kk);
+  return dispatch<false>(ctx, column_tile(ctx, m, cols, 1, limit), split, A, B, 1, n, count, m, cols, kk, pol, extras);
 }
 
 extern "C" int nrs_has_tensor_core_path(void) { return 1; }

@@ -14,7 +14,8 @@
 // TMEM holds two accumulators, so the epilogue of tile i runs under the main loop of
 // tile i+1.
 // A Policy supplies how an A slice is fetched (dense rows for GEMM, a shifted
-// NHWC window for convolution) and what the epilogue does with a row of results.
+// NHWC window for convolution), which K-slices of a tile count and whether the tile
+// exists at all (clip: triangular products), and what the epilogue does with a row of results.
 // A policy with kCanEmit may also hand the finished values back: the epilogue warps then
 // write them as TF32 high / residual planes ([row][32 columns], 128-byte swizzle) into a
 // staging tile and one thread sends each tile to global memory with a TMA store — the
@@ -182,8 +183,9 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
         int tile_m, tile_n, z;
         tmap.decode(t, &tile_m, &tile_n, &z);
         const int batch = z / sp.splits, split = z - batch * sp.splits;
-        const int kb_begin = split * sp.kb_per_split;
-        const int kb_end = min(sp.kb_total, kb_begin + sp.kb_per_split);
+        int kb_begin = split * sp.kb_per_split;
+        int kb_end = min(sp.kb_total, kb_begin + sp.kb_per_split);
+        if (!pol.clip(tile_m, tile_n, BN, &kb_begin, &kb_end)) continue;
         const int n0 = tile_n * BN;
         // Where the K-slices of this tile lie, stepped along instead of recomputed (the divisions of a recomputation per
         // slice and plane made the one producing thread the bottleneck: 58 -> 72 us on a 64-channel convolution).
@@ -195,11 +197,9 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
           uint8_t* st = smem + s * L::kStage;
           mbar_expect_tx(&full_bar[s], stage_bytes);
           pol.load_a(st, &tm_a_hi, &full_bar[s], cur);
-          int b0, b1, b2;
-          pol.b_origin(cur, n0, batch, &b0, &b1, &b2);
-          tma_load_3d(st + L::kATile, &tm_b_hi, &full_bar[s], b0, b1, b2);
+          pol.template load_b<BN>(st + L::kATile, &tm_b_hi, &full_bar[s], cur, n0);
           if (NPLANES == 2) {
-            tma_load_3d(st + L::kATile + L::kBTile, &tm_b_lo, &full_bar[s], b0, b1, b2);
+            pol.template load_b<BN>(st + L::kATile + L::kBTile, &tm_b_lo, &full_bar[s], cur, n0);
             pol.load_a(st + L::kATile + 2 * L::kBTile, &tm_a_lo, &full_bar[s], cur);
           }
           pol.advance(cur);
@@ -217,23 +217,25 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
   } else if (warp == 1) {
     if (lane == 0) {
       // ---------------- UMMA issuer
-      constexpr bool kMN = Policy::kMnMajor;
-      constexpr uint32_t idesc_wide = make_idesc_tf32(BM, NPLANES * BN, kMN, kMN);
-      constexpr uint32_t idesc_half = make_idesc_tf32(BM, BN, kMN, kMN);
+      constexpr bool kAMn = Policy::kAMnMajor, kBMn = Policy::kBMnMajor;
+      constexpr uint32_t idesc_wide = make_idesc_tf32(BM, NPLANES * BN, kAMn, kBMn);
+      constexpr uint32_t idesc_half = make_idesc_tf32(BM, BN, kAMn, kBMn);
       // K-major: 8 elements of K are 32 bytes inside the swizzle row.  MN-major: 32-column blocks of [32 k][128 B], so
       // a K-step is 1024 bytes and blocks are 4096 apart (the blocks of B_lo follow those of B_hi).
-      auto desc = [](uint32_t addr, int k) {
-        return kMN ? make_smem_desc_sw128_32b(addr + (uint32_t)k * 1024u, BK * 128, 512) : make_smem_desc_sw128(addr + (uint32_t)k * 32u, 16, 1024);
+      auto desc = [](bool mn, uint32_t addr, int k) {
+        return mn ? make_smem_desc_sw128_32b(addr + (uint32_t)k * 1024u, BK * 128, 512) : make_smem_desc_sw128(addr + (uint32_t)k * 32u, 16, 1024);
       };
       uint32_t it = 0, local = 0;
       bool ok = true;
-      for (long t = blockIdx.x; t < tmap.total && ok; t += gridDim.x, ++local) {
+      for (long t = blockIdx.x; t < tmap.total && ok; t += gridDim.x) {
         int tile_m, tile_n, z;
         tmap.decode(t, &tile_m, &tile_n, &z);
         const int split = z % sp.splits;
-        const int kb_begin = split * sp.kb_per_split;
-        const int nkb = min(sp.kb_total, kb_begin + sp.kb_per_split) - kb_begin;   // >= 1 by construction
+        int kb_begin = split * sp.kb_per_split, kb_end = min(sp.kb_total, kb_begin + sp.kb_per_split);
+        if (!pol.clip(tile_m, tile_n, BN, &kb_begin, &kb_end)) continue;
+        const int nkb = kb_end - kb_begin;   // >= 1 by construction
         const uint32_t buf = local & 1u, use = local >> 1;
+        ++local;
         if (!mbar_wait(&acc_empty[buf], (use & 1u) ^ 1u)) { atomicExch(err_flag, kErrMmaWait); break; }
         tc_fence_after_sync();
         const uint32_t d = tmem_base + buf * (uint32_t)L::kAccCols;
@@ -248,10 +250,10 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
           const uint32_t a_lo = b_hi + 2 * L::kBTile;
 #pragma unroll
           for (int k = 0; k < BK / 8; ++k) {
-            const uint64_t da_hi = desc(a_hi, k), db_hi = desc(b_hi, k);
+            const uint64_t da_hi = desc(kAMn, a_hi, k), db_hi = desc(kBMn, b_hi, k);
             umma_tf32(d, da_hi, db_hi, idesc_wide, (i | k) != 0);   // hi*hi | hi*lo
             if (NPLANES == 2) {
-              umma_tf32(d, desc(a_lo, k), db_hi, idesc_half, 1);             // + lo*hi
+              umma_tf32(d, desc(kAMn, a_lo, k), db_hi, idesc_half, 1);             // + lo*hi
             }
           }
           umma_commit(&empty_bar[s]);  // slot reusable once these UMMAs have read it
@@ -266,12 +268,15 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
     const bool emit_issuer = warp == 2 && lane == 0;
     uint32_t local = 0, emitted = 0;
     bool ok = true;
-    for (long t = blockIdx.x; t < tmap.total && ok; t += gridDim.x, ++local) {
+    for (long t = blockIdx.x; t < tmap.total && ok; t += gridDim.x) {
       int tile_m, tile_n, z;
       tmap.decode(t, &tile_m, &tile_n, &z);
       const int batch = z / sp.splits, split = z - batch * sp.splits;
+      int kb_begin = split * sp.kb_per_split, kb_end = min(sp.kb_total, kb_begin + sp.kb_per_split);
+      if (!pol.clip(tile_m, tile_n, BN, &kb_begin, &kb_end)) continue;   // the same verdict in all three roles
       const int n0 = tile_n * BN;
       const uint32_t buf = local & 1u, use = local >> 1;
+      ++local;
       [[maybe_unused]] const auto rw = pol.row(tile_m, batch, row);   // index arithmetic under the main loop
       if (!mbar_wait(&acc_full[buf], use & 1u)) {
         if (lane == 0) atomicExch(err_flag, kErrEpilogueWait);
@@ -462,7 +467,12 @@ int launch(nrs_ctx* ctx, const CUtensorMap& ta_hi, const CUtensorMap& ta_lo, con
   NRS_ENSURE_SMEM(ctx, attr, (tc_kernel<BN, NPLANES, Policy>), kSmem);
   const int tiles_n = (n_total + BN - 1) / BN;
   SplitInfo sp{};
-  plan_split(ctx, (long)tiles_m * tiles_n * batches, (long)tiles_m * BM * n_total * batches, kb_total, NPLANES == 2, &sp.splits, &sp.kb_per_split);
+  if (Policy::kMaySplit) {
+    plan_split(ctx, (long)tiles_m * tiles_n * batches, (long)tiles_m * BM * n_total * batches, kb_total, NPLANES == 2, &sp.splits, &sp.kb_per_split);
+  } else {   // tiles whose K ranges differ
+    sp.splits = 1;
+    sp.kb_per_split = kb_total;
+  }
   sp.kb_total = kb_total;
   sp.batches = batches;
   sp.n_total = n_total;

@@ -275,7 +275,7 @@ int launch_wgrad(nrs_ctx* ctx, const CUtensorMap* maps, const WgradParams& p, in
 }  // namespace
 
 int nrs_tc_conv_wgrad(nrs_ctx* ctx, const float* x, const float* dy, float* dw, int n, int ci, int h, int wd, int co,
-                      int kh, int kw, int stride, int pad, int accumulate) {
+                      int kh, int kw, int stride, int pad, int accumulate, int out_cols) {
   if (!tc::tensor_map_encoder()) return NRS_ERR_UNSUPPORTED;
   if (n < 1 || stride > 8) return NRS_ERR_UNSUPPORTED;
   const int oh = (h + 2 * pad - kh) / stride + 1, ow = (wd + 2 * pad - kw) / stride + 1;
@@ -335,7 +335,7 @@ int nrs_tc_conv_wgrad(nrs_ctx* ctx, const float* x, const float* dy, float* dw, 
   const size_t partial_floats = (size_t)splits * p.m_blocks * p.n_groups * p.col_blocks * 128 * p.group_cols;
   void *dy_hi = nullptr, *dy_lo = nullptr, *x_hi = nullptr, *x_lo = nullptr;
   // a single split of a 1x1 "convolution" (A^T B) that overwrites its output needs no second pass
-  p.direct = (splits == 1 && taps == 1 && ci % 32 == 0 && !accumulate && (reinterpret_cast<uintptr_t>(dw) & 15) == 0) ? dw : nullptr;
+  p.direct = (splits == 1 && taps == 1 && ci % 32 == 0 && !accumulate && !out_cols && (reinterpret_cast<uintptr_t>(dw) & 15) == 0) ? dw : nullptr;
   int st = p.direct ? NRS_OK : nrs_fold_partial(ctx, NRS_WS_WGRAD_PARTIAL, partial_floats * sizeof(float), &p.partial);
   if (st != NRS_OK) return st;
   bool may_overlap = ctx->independent_next;   // withdrawn below if this call stages an operand itself
@@ -400,6 +400,7 @@ int nrs_tc_conv_wgrad(nrs_ctx* ctx, const float* x, const float* dy, float* dw, 
   j.co = co; j.ci = ci; j.taps = taps;
   j.taps_per_group = p.taps_per_group; j.n_groups = p.n_groups; j.col_blocks = p.col_blocks; j.cblocks = p.cblocks;
   j.group_cols = p.group_cols;
+  j.out_cols = out_cols;
   j.split_stride = (size_t)p.m_blocks * p.n_groups * p.col_blocks * 128 * p.group_cols;
   return nrs_fold_submit(ctx, j);
 }
