@@ -61,21 +61,22 @@ struct HeadPolicy {
     return Cursor{kb * tc::BK, tile_m * tc::BM, batch - b * heads, b};
   }
   __device__ __forceinline__ void advance(Cursor& c) const { c.k += tc::BK; }
-  __device__ __forceinline__ void load_a(void* dst, const CUtensorMap* tm, uint64_t* bar, const Cursor& c) const {
+  template <bool PAIR>
+  __device__ __forceinline__ void load_a(void* dst, const CUtensorMap* tm, uint32_t bar, const Cursor& c) const {
     if (AMN) {
 #pragma unroll
-      for (int i = 0; i < tc::BM / 32; ++i) tc::tma_load_4d((uint8_t*)dst + i * 4096, tm, bar, c.row + 32 * i, c.k, c.h, c.b);
+      for (int i = 0; i < tc::BM / 32; ++i) tc::tma_load_4d_to<PAIR>((uint8_t*)dst + i * 4096, tm, bar, c.row + 32 * i, c.k, c.h, c.b);
     } else {
-      tc::tma_load_4d(dst, tm, bar, c.k, c.row, c.h, c.b);
+      tc::tma_load_4d_to<PAIR>(dst, tm, bar, c.k, c.row, c.h, c.b);
     }
   }
-  template <int BN>
-  __device__ __forceinline__ void load_b(void* dst, const CUtensorMap* tm, uint64_t* bar, const Cursor& c, int n0) const {
+  template <int BN, bool PAIR>
+  __device__ __forceinline__ void load_b(void* dst, const CUtensorMap* tm, uint32_t bar, const Cursor& c, int n0) const {
     if (BMN) {
 #pragma unroll
-      for (int i = 0; i < BN / 32; ++i) tc::tma_load_4d((uint8_t*)dst + i * 4096, tm, bar, n0 + 32 * i, c.k, c.h, c.b);
+      for (int i = 0; i < BN / 32; ++i) tc::tma_load_4d_to<PAIR>((uint8_t*)dst + i * 4096, tm, bar, n0 + 32 * i, c.k, c.h, c.b);
     } else {
-      tc::tma_load_4d(dst, tm, bar, c.k, n0, c.h, c.b);
+      tc::tma_load_4d_to<PAIR>(dst, tm, bar, c.k, n0, c.h, c.b);
     }
   }
   __device__ __forceinline__ int row(int, int, int) const { return 0; }
@@ -112,7 +113,7 @@ int run(nrs_ctx* ctx, const HeadMat& A, const HeadMat& B, const HeadPolicy<AMN, 
   if (NPLANES == 2) ok = ok && head_map(&a_lo, A.lo, A, pol.heads, batch, AMN, tc::BM) && head_map(&b_lo, B.lo, B, pol.heads, batch, BMN, BN);
   else { a_lo = a_hi; b_lo = b_hi; }
   NRS_REQUIRE(ctx, ok, NRS_ERR_CUDA, "attention: cuTensorMapEncodeTiled failed");
-  return tc::launch<BN, NPLANES, HeadPolicy<AMN, BMN>>(ctx, a_hi, a_lo, b_hi, b_lo, pol, (pol.M + tc::BM - 1) / tc::BM, pol.N,
+  return tc::launch<BN, NPLANES, false, HeadPolicy<AMN, BMN>>(ctx, a_hi, a_lo, b_hi, b_lo, pol, (pol.M + tc::BM - 1) / tc::BM, pol.N,
                                                        batch * pol.heads, (k + tc::BK - 1) / tc::BK);
 }
 

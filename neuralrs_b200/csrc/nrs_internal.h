@@ -342,18 +342,26 @@ inline bool nrs_smem_attr_update(NrsSmemAttr& a, int device, size_t bytes) {
   do { NRS_PDL_WAIT(); NRS_PDL_TRIGGER(); } while (0)
 
 template <class... P, class... A>
-inline cudaError_t nrs_pdl_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+inline cudaError_t nrs_pdl_launch_cluster(unsigned cluster, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                          A&&... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
+  cudaLaunchAttribute attr[2] = {};
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+template <class... P, class... A>
+inline cudaError_t nrs_pdl_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+  return nrs_pdl_launch_cluster(1, kernel, grid, block, smem, stream, static_cast<A&&>(args)...);
 }
 // kernel<<<grid, block, smem, stream>>>(args...) as a programmatic dependent launch.  The kernel
 // expression goes in parentheses when its template arguments contain commas.

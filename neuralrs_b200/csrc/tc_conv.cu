@@ -93,12 +93,13 @@ struct ConvPolicy {
     }
     c.b_col = weight_column(c);
   }
-  template <int BN>
-  __device__ __forceinline__ void load_b(void* dst, const CUtensorMap* tm, uint64_t* bar, const Cursor& c, int n0) const {
-    tc::tma_load_3d(dst, tm, bar, c.b_col, n0, 0);
+  template <int BN, bool PAIR>
+  __device__ __forceinline__ void load_b(void* dst, const CUtensorMap* tm, uint32_t bar, const Cursor& c, int n0) const {
+    tc::tma_load_3d_to<PAIR>(dst, tm, bar, c.b_col, n0, 0);
   }
-  __device__ __forceinline__ void load_a(void* dst, const CUtensorMap* tm, uint64_t* bar, const Cursor& c) const {
-    tc::tma_load_4d(dst, tm, bar, c.cb * 32, c.x, c.y, c.n);
+  template <bool PAIR>
+  __device__ __forceinline__ void load_a(void* dst, const CUtensorMap* tm, uint32_t bar, const Cursor& c) const {
+    tc::tma_load_4d_to<PAIR>(dst, tm, bar, c.cb * 32, c.x, c.y, c.n);
   }
   // NCHW offset of channel 0 of the pixel behind accumulator row `row`, and the pixel's linear index.
   __device__ __forceinline__ bool locate(int tile_m, int row, size_t* nchw_off, size_t* pixel) const {
@@ -225,7 +226,7 @@ struct ConvPlan {
   int act, accumulate;
 };
 
-template <int BN, int NPLANES>
+template <int BN, int NPLANES, bool PAIR>
 int run_conv(nrs_ctx* ctx, const ConvPlan& p, const float* a_hi, const float* a_lo, const float* w_hi, const float* w_lo,
              const ConvPolicy& pol, int tiles_m, int* splits_out) {
   const int a_ld = nrs_plane_ld(p.a_ch);
@@ -237,7 +238,7 @@ int run_conv(nrs_ctx* ctx, const ConvPlan& p, const float* a_hi, const float* a_
   const uint32_t astep[4] = {1, (uint32_t)pol.in_step, (uint32_t)pol.in_step, 1};
   const uint64_t bdim[3] = {(uint64_t)kdim, (uint64_t)p.n_ch_out, 1};
   const uint64_t bstr[2] = {(uint64_t)kdim * 4, (uint64_t)kdim * p.n_ch_out * 4};
-  const uint32_t bbox[3] = {32, (uint32_t)BN, 1};
+  const uint32_t bbox[3] = {32, (uint32_t)(PAIR ? BN / 2 : BN), 1};
   bool ok = tc::encode_tmap_f32(&ta_hi, a_hi, 4, adim, astr, abox, false, astep) && tc::encode_tmap_f32(&tb_hi, w_hi, 3, bdim, bstr, bbox);
   if (NPLANES == 2)
     ok = ok && tc::encode_tmap_f32(&ta_lo, a_lo, 4, adim, astr, abox, false, astep) && tc::encode_tmap_f32(&tb_lo, w_lo, 3, bdim, bstr, bbox);
@@ -251,7 +252,7 @@ int run_conv(nrs_ctx* ctx, const ConvPlan& p, const float* a_hi, const float* a_
     if (pol.out_lo) ok = ok && tc::encode_tmap_f32(&to_lo, pol.out_lo, 4, odim, ostr, abox);
   }
   NRS_REQUIRE(ctx, ok, NRS_ERR_CUDA, "tc_conv: cuTensorMapEncodeTiled failed");
-  return tc::launch<BN, NPLANES, ConvPolicy>(ctx, ta_hi, ta_lo, tb_hi, tb_lo, pol, tiles_m, p.n_ch_out, 1,
+  return tc::launch<BN, NPLANES, PAIR, ConvPolicy>(ctx, ta_hi, ta_lo, tb_hi, tb_lo, pol, tiles_m, p.n_ch_out, 1,
                                              p.ay.taps * p.ax.taps * pol.cblocks, pol.out_hi ? &to_hi : nullptr,
                                              pol.out_lo ? &to_lo : nullptr, splits_out);
 }
@@ -279,24 +280,6 @@ void plan_pixel_tile(const ConvPlan& p, ConvPolicy* pol) {
       pol->Wt = Wt; pol->Ht = Ht; pol->Nt = Nt; pol->tiles_x = nx; pol->tiles_y = ny;
     }
   }
-}
-
-// Column tile.  Clocks of one 32-element K-block of a tile, from in-kernel measurements of the issuing thread
-// (4 K-steps of 8): 128 columns 1060, 64 columns 832, 32 columns 690, and about as many again per tile for the
-// accumulator's way out.  The width with the least (waves of the grid) x (clocks per tile) is taken: wide tiles for
-// large outputs, narrower ones where they fill SMs that would idle or where a ragged channel count would pad.
-int plan_column_tile(const nrs_ctx* ctx, long tiles_m, int n_ch_out, int kblocks) {
-  const int width[3] = {128, 64, 32}, kb_clk[3] = {1060, 832, 690}, tile_clk[3] = {2600, 1700, 1300};
-  int best = 128;
-  double best_t = -1.0;
-  for (int i = 0; i < 3; ++i) {
-    if (width[i] > 32 && width[i] / 2 >= n_ch_out) continue;   // half of the tile or more would be padding
-    const long tiles = tiles_m * ((n_ch_out + width[i] - 1) / width[i]);
-    const double waves = (double)((tiles + ctx->sm_count - 1) / ctx->sm_count);
-    const double t = waves * ((double)kblocks * kb_clk[i] + tile_clk[i]);
-    if (best_t < 0.0 || t < best_t) { best_t = t; best = width[i]; }
-  }
-  return best;
 }
 
 int conv_common(nrs_ctx* ctx, ConvPlan& p) {
@@ -365,14 +348,14 @@ int conv_common(nrs_ctx* ctx, ConvPlan& p) {
 
   if (extras != ctx->out_extras.end()) ctx->out_extras.erase(extras);   // honoured from here on
   int splits = 0;
-#define NRS_RUN(BN_)                                                                                                     \
-  st = split ? run_conv<BN_, 2>(ctx, p, (const float*)a_hi, (const float*)a_lo, (const float*)p.w_hi, (const float*)p.w_lo, pol, (int)tiles_m, &splits) \
-             : run_conv<BN_, 1>(ctx, p, (const float*)a_hi, nullptr, (const float*)p.w_hi, nullptr, pol, (int)tiles_m, &splits)
-  switch (plan_column_tile(ctx, tiles_m, p.n_ch_out, p.ay.taps * p.ax.taps * pol.cblocks)) {
-    case 128: NRS_RUN(128); break;
-    case 64: NRS_RUN(64); break;
-    default: NRS_RUN(32); break;
-  }
+  const tc::TilePlan tile = tc::plan_tile(ctx, tiles_m, p.n_ch_out, 1, p.ay.taps * p.ax.taps * pol.cblocks, split);
+#define NRS_RUN(BN_, PAIR_)                                                                                              \
+  st = split ? run_conv<BN_, 2, PAIR_>(ctx, p, (const float*)a_hi, (const float*)a_lo, (const float*)p.w_hi, (const float*)p.w_lo, pol, (int)tiles_m, &splits) \
+             : run_conv<BN_, 1, PAIR_>(ctx, p, (const float*)a_hi, nullptr, (const float*)p.w_hi, nullptr, pol, (int)tiles_m, &splits)
+  if (tile.pair) { if (tile.bn == 128) NRS_RUN(128, true); else NRS_RUN(64, true); }
+  else if (tile.bn == 128) NRS_RUN(128, false);
+  else if (tile.bn == 64) NRS_RUN(64, false);
+  else NRS_RUN(32, false);
 #undef NRS_RUN
   // channel sums come from the direct epilogue only (a K-split stores through the reduce kernel)
   if (st == NRS_OK && pol.colsum_partial && splits == 1) colsum->second.rows = (int)tiles_m * 4;

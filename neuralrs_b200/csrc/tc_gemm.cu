@@ -41,17 +41,18 @@ struct GemmPolicy {
   struct Cursor { int b_col, row, batch; };
   __device__ __forceinline__ Cursor cursor(int tile_m, int batch, int kb) const { return Cursor{kb * tc::BK, tile_m * tc::BM, batch}; }
   __device__ __forceinline__ void advance(Cursor& c) const { c.b_col += tc::BK; }
-  __device__ __forceinline__ void load_a(void* dst, const CUtensorMap* tm, uint64_t* bar, const Cursor& c) const {
-    if (MN) tc::tma_load_3d(dst, tm, bar, 0, c.b_col, c.row / 32);
-    else tc::tma_load_3d(dst, tm, bar, c.b_col, c.row, c.batch);
+  template <bool PAIR>
+  __device__ __forceinline__ void load_a(void* dst, const CUtensorMap* tm, uint32_t bar, const Cursor& c) const {
+    if (MN) tc::tma_load_3d_to<PAIR>(dst, tm, bar, 0, c.b_col, c.row / 32);
+    else tc::tma_load_3d_to<PAIR>(dst, tm, bar, c.b_col, c.row, c.batch);
   }
-  template <int BN>
-  __device__ __forceinline__ void load_b(void* dst, const CUtensorMap* tm, uint64_t* bar, const Cursor& c, int n0) const {
-    if (MN) { tc::tma_load_3d(dst, tm, bar, 0, c.b_col, n0 / 32); return; }
+  template <int BN, bool PAIR>
+  __device__ __forceinline__ void load_b(void* dst, const CUtensorMap* tm, uint32_t bar, const Cursor& c, int n0) const {
+    if (MN) { tc::tma_load_3d_to<PAIR>(dst, tm, bar, 0, c.b_col, n0 / 32); return; }
     int b0 = c.b_col, b1 = n0, b2 = c.batch;
     if (seg_n) { b2 = n0 / seg_n; b1 = n0 - b2 * seg_n; }
     if (seg_k) { b2 = c.b_col / seg_k; b0 = c.b_col - b2 * seg_k; }
-    tc::tma_load_3d(dst, tm, bar, b0, b1, b2);
+    tc::tma_load_3d_to<PAIR>(dst, tm, bar, b0, b1, b2);
   }
   __device__ __forceinline__ float dact(float src) const { return x.dact == NRS_ACT_RELU ? (src > 0.0f ? 1.0f : 0.0f) : nrs_gelu_d(src); }
   // One element, from the pass that sums a K-split.
@@ -202,36 +203,28 @@ bool make_mn_operand_map(CUtensorMap* tm, const float* base, const Operand& op, 
   return tc::encode_tmap_f32(tm, base, 3, dim, str, box, true);
 }
 
-template <int BN, int NPLANES, bool MN>
+template <int BN, int NPLANES, bool PAIR, bool MN>
 int run(nrs_ctx* ctx, const Operand& A, const Operand& B, int batch, int b_rows, int b_batch, int m, int n, int k,
         const GemmPolicy<MN>& pol, int* splits) {
+  constexpr int kBRows = PAIR ? BN / 2 : BN;   // rows of B that one CTA brings
   CUtensorMap ta_hi, ta_lo, tb_hi, tb_lo;
   auto map_a = [&](CUtensorMap* t, const float* p) { return MN ? make_mn_operand_map(t, p, A, m, k, tc::BM) : make_operand_map(t, p, A, m, batch, tc::BM); };
-  auto map_b = [&](CUtensorMap* t, const float* p) { return MN ? make_mn_operand_map(t, p, B, n, k, BN) : make_operand_map(t, p, B, b_rows, b_batch, BN); };
+  auto map_b = [&](CUtensorMap* t, const float* p) { return MN ? make_mn_operand_map(t, p, B, n, k, kBRows) : make_operand_map(t, p, B, b_rows, b_batch, kBRows); };
   bool ok = map_a(&ta_hi, A.hi) && map_b(&tb_hi, B.hi);
   if (NPLANES == 2) ok = ok && map_a(&ta_lo, A.lo) && map_b(&tb_lo, B.lo);
   else { ta_lo = ta_hi; tb_lo = tb_hi; }
   NRS_REQUIRE(ctx, ok, NRS_ERR_CUDA, "tc_gemm: cuTensorMapEncodeTiled failed (m=%d n=%d k=%d)", m, n, k);
-  return tc::launch<BN, NPLANES, GemmPolicy<MN>>(ctx, ta_hi, ta_lo, tb_hi, tb_lo, pol, (m + tc::BM - 1) / tc::BM, n, batch,
+  return tc::launch<BN, NPLANES, PAIR, GemmPolicy<MN>>(ctx, ta_hi, ta_lo, tb_hi, tb_lo, pol, (m + tc::BM - 1) / tc::BM, n, batch,
                                                  (k + tc::BK - 1) / tc::BK, nullptr, nullptr, splits);
 }
 
-// Tile width: 128 columns is the efficient shape, but a product with few tiles leaves most SMs idle and
-// a K-split needs a second pass, so narrower tiles are taken until about two thirds of the SMs have one.
 // `limit`: widest tile allowed (segmented B: the segment must be whole tiles).
-int column_tile(const nrs_ctx* ctx, int m, int n, int batch, int limit = 128) {
-  const long tiles_m = (m + tc::BM - 1) / tc::BM;
-  auto tiles = [&](int bn) { return tiles_m * ((n + bn - 1) / bn) * batch; };
-  const long want = (long)ctx->sm_count * 2 / 3;
-  int bn = n <= 32 ? 32 : n <= 64 ? 64 : 128;
-  if (bn > limit) bn = limit;
-  if (bn == 128 && tiles(128) < want) bn = 64;
-  if (bn == 64 && n > 32 && tiles(64) < want) bn = 32;
-  return bn;
+tc::TilePlan tile_of(const nrs_ctx* ctx, int m, int n, int batch, int k, bool split, int limit = 128) {
+  return tc::plan_tile(ctx, (m + tc::BM - 1) / tc::BM, n, batch, (k + tc::BK - 1) / tc::BK, split, limit);
 }
 
 template <bool MN>
-int dispatch(nrs_ctx* ctx, int bn, bool split, const Operand& A, const Operand& B, int batch, int b_rows, int b_batch, int m, int n,
+int dispatch(nrs_ctx* ctx, tc::TilePlan tile, bool split, const Operand& A, const Operand& B, int batch, int b_rows, int b_batch, int m, int n,
              int k, GemmPolicy<MN>& pol, NrsGemmExtras* extras) {
   auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
   pol.vec_ok = n % 4 == 0 && ((size_t)m * n) % 4 == 0 && aligned(pol.C) && aligned(pol.bias);
@@ -241,11 +234,12 @@ int dispatch(nrs_ctx* ctx, int bn, bool split, const Operand& A, const Operand& 
     if (extras->colsum && (m + tc::BM - 1) / tc::BM * 4 > extras->colsum_cap) pol.x.colsum = nullptr;
   }
   int st, splits = 1;
-#define NRS_RUN_GEMM(BN_) (split ? run<BN_, 2, MN>(ctx, A, B, batch, b_rows, b_batch, m, n, k, pol, &splits) \
-                                 : run<BN_, 1, MN>(ctx, A, B, batch, b_rows, b_batch, m, n, k, pol, &splits))
-  if (bn == 128) st = NRS_RUN_GEMM(128);
-  else if (bn == 64) st = NRS_RUN_GEMM(64);
-  else st = NRS_RUN_GEMM(32);
+#define NRS_RUN_GEMM(BN_, PAIR_) (split ? run<BN_, 2, PAIR_, MN>(ctx, A, B, batch, b_rows, b_batch, m, n, k, pol, &splits) \
+                                        : run<BN_, 1, PAIR_, MN>(ctx, A, B, batch, b_rows, b_batch, m, n, k, pol, &splits))
+  if (tile.pair) st = tile.bn == 128 ? NRS_RUN_GEMM(128, true) : NRS_RUN_GEMM(64, true);
+  else if (tile.bn == 128) st = NRS_RUN_GEMM(128, false);
+  else if (tile.bn == 64) st = NRS_RUN_GEMM(64, false);
+  else st = NRS_RUN_GEMM(32, false);
 #undef NRS_RUN_GEMM
   if (extras && st == NRS_OK) {
     extras->honoured = true;
@@ -362,7 +356,7 @@ int nrs_tc_gemm(nrs_ctx* ctx, int trans_a, int trans_b, int batch, int m, int n,
     if (st == NRS_OK) st = prepare_operand(ctx, b, k, n, 1, true, split, NRS_WS_B_HI, NRS_WS_B_LO, &B, false, false);
     if (st != NRS_OK) return st;
     GemmPolicy<true> pol{c, bias, act, beta, m, n, (size_t)m * n, false, {}, 0, 0};
-    return dispatch<true>(ctx, column_tile(ctx, m, n, 1), split, A, B, 1, n, 1, m, n, k, pol, extras);
+    return dispatch<true>(ctx, tile_of(ctx, m, n, 1, k, split), split, A, B, 1, n, 1, m, n, k, pol, extras);
   }
   st = prepare_operand(ctx, a, m, k, batch, /*stored_kmajor=*/!trans_a, split, NRS_WS_A_HI, NRS_WS_A_LO, &A, false);
   if (st != NRS_OK) return st;
@@ -371,7 +365,7 @@ int nrs_tc_gemm(nrs_ctx* ctx, int trans_a, int trans_b, int batch, int m, int n,
   // Batched operands read in place need 16-byte aligned batch strides.
   if (batch > 1 && ((A.bstride % 4) || (B.bstride % 4))) return NRS_ERR_UNSUPPORTED;
   GemmPolicy<false> pol{c, bias, act, beta, m, n, (size_t)m * n, false, {}, 0, 0};
-  return dispatch<false>(ctx, column_tile(ctx, m, n, batch), split, A, B, batch, n, batch, m, n, k, pol, extras);
+  return dispatch<false>(ctx, tile_of(ctx, m, n, batch, k, split), split, A, B, batch, n, batch, m, n, k, pol, extras);
 }
 
 // x[m,k] times several weight matrices w[i] of one shape, in one product.  `reduce` == 0: c[m, count*n] = x . [w0|w1|..]
@@ -412,7 +406,7 @@ int nrs_tc_gemm_weights(nrs_ctx* ctx, int reduce, int count, int m, int n, int k
   GemmPolicy<false> pol{c, nullptr, NRS_ACT_NONE, beta, m, cols, (size_t)m * cols, false, {}, reduce ? 0 : n, reduce ? k : 0};
   const int limit = reduce ? 128 : n % 128 == 0 ? 128 : n % 64 == 0 ? 64 : 32;
   NrsProfScope prof(ctx, NRS_PROF_GEMM, 2.0 * m * cols * kk);
-  return dispatch<false>(ctx, column_tile(ctx, m, cols, 1, limit), split, A, B, 1, n, count, m, cols, kk, pol, extras);
+  return dispatch<false>(ctx, tile_of(ctx, m, cols, 1, kk, split, limit), split, A, B, 1, n, count, m, cols, kk, pol, extras);
 }
 
 extern "C" int nrs_has_tensor_core_path(void) { return 1; }

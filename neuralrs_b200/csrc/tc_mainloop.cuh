@@ -3,11 +3,11 @@
 // memory, fed by TMA, consumed by tcgen05.mma kind::tf32.
 //
 // Persistent CTAs (one per SM) walk a list of output tiles (row tile, column tile,
-// batch x K-split).  Six warps, fixed roles:
-//   warp 0     TMA producer (one thread): per K-slice, one mbarrier-tracked ring
+// batch x K-split).  Six or ten warps, fixed roles:
+//   warp 0     TMA producer: per K-slice, one mbarrier-tracked ring
 //              slot holding the A and B slices (and their residual planes for 3xTF32);
 //              the ring runs ahead across tile boundaries
-//   warp 1     TMEM allocation; one thread issues the UMMAs (M=128, K=8) and commits
+//   warp 1     TMEM allocation; issues the UMMAs (M=128, K=8) and commits
 //              ring slots back to the producer, then the accumulator to the epilogue
 //   warps 2..  epilogue (4 or 8 warps, the policy's choice): tcgen05.ld (thread = accumulator row),
 //              policy-defined store
@@ -27,6 +27,16 @@
 // [0,BN), hi*lo in [BN,2BN)) and a second of width BN adds A_lo.B_hi onto the first half;
 // the epilogue sums the halves.  Against three UMMAs of width BN this reads a quarter
 // less shared memory per K-step, which is what bounds the narrow (BN = 64) tiles.
+//
+// What bounds a tile: with 128 columns in 3xTF32 the tensor pipe (768 clocks of UMMA per K-slice), with fewer the reads of
+// A from shared memory and the way of the operand planes through L2 (48 KB per K-slice of a 128 x 64 tile).  With PAIR the
+// two CTAs of a cluster work on two row tiles of one column tile: each brings its own A rows and half of the B rows, and
+// one warp issues UMMAs of 256 rows that read B from both (cta_group::2), which halves B's share of that traffic.  The
+// ring, the accumulators and the epilogue stay per CTA.  Clocks per K-slice (3xTF32 GEMM; TF32): single 128 columns
+// 905; 428, 64 columns 660; 369, pairs 820; 345 and 565; 317.  (With one thread per role, see elect_one: 960; 630 and 863;
+// 620, bound by the issuing thread, so that narrower tiles and pairs gained nothing.)  A 64-channel 3x3 layer on 100
+// images of 32 x 32: 59 -> 43 us.
+//
 // The tensor core's f32 accumulation is not round-to-nearest; its error grows
 // linearly with the length of one accumulation chain (about 7e-9 relative per K
 // element), so callers keep a chain at or below kMaxChainK by splitting K across
@@ -47,10 +57,10 @@ constexpr int BM = 128, BK = 32;   // BK f32 = 128 bytes = one swizzle row
 constexpr int kMaxChainK = 4096;   // longest single accumulation chain in 3xTF32 mode
 constexpr int kGroupM = 16;        // row tiles per raster group (see TileMap)
 
-template <int BN, int NPLANES, int EMIT_BYTES = 0>
+template <int BN, int NPLANES, int EMIT_BYTES, bool PAIR>
 struct SmemLayout {
   static constexpr int kATile = BM * BK * 4;   // 16 KB
-  static constexpr int kBTile = BN * BK * 4;
+  static constexpr int kBTile = BN / (PAIR ? 2 : 1) * BK * 4;   // this CTA's rows of B
   static constexpr int kStage = NPLANES * (kATile + kBTile);   // [A_hi][B_hi][B_lo][A_lo]
   static constexpr int kExtra = EMIT_BYTES /*plane staging tile*/ + 1024 /*align*/ + 256 /*barriers*/;
   static constexpr int kRing = 227 * 1024 - kExtra;
@@ -129,7 +139,7 @@ __device__ __forceinline__ void rows_to_lines(float* tile, int lane, const uint3
   }
 }
 
-template <int BN, int NPLANES, class Policy>
+template <int BN, int NPLANES, class Policy, bool PAIR>
 __global__ void __launch_bounds__(threads<Policy>(), 1)
 tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ CUtensorMap tm_a_lo,
           const __grid_constant__ CUtensorMap tm_b_hi, const __grid_constant__ CUtensorMap tm_b_lo,
@@ -137,7 +147,7 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
           const Policy pol, const SplitInfo sp, const TileMap tmap, const int emit /*planes to emit: 0, 1 or 2*/,
           int* __restrict__ err_flag) {
   constexpr int kEmitBytes = emit_bytes<NPLANES, Policy>();
-  using L = SmemLayout<BN, NPLANES, kEmitBytes>;
+  using L = SmemLayout<BN, NPLANES, kEmitBytes, PAIR>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint8_t* emit_tile = smem + L::kStages * L::kStage;   // [planes][128 rows][128 B], 1024-byte aligned
@@ -148,7 +158,10 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
   uint64_t* emit_bar = acc_empty + 2;            // [2] staging tile free / staging tile written
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(emit_bar + 2);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = (int)uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
+  // A pair walks the tile list together: its CTA of rank r takes row tile 2*i + r of every pair of row tiles i.
+  const int rank = PAIR ? (int)cluster_rank() : 0;
+  const long t_first = PAIR ? blockIdx.x / 2 : blockIdx.x, t_step = PAIR ? gridDim.x / 2 : gridDim.x;
 
   if (warp == 0 && lane == 0) {
     prefetch_tmap(&tm_a_hi);
@@ -157,77 +170,91 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
     if (emit >= 1) prefetch_tmap(&tm_out_hi);
     if (emit == 2) prefetch_tmap(&tm_out_lo);
     for (int s = 0; s < L::kStages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-    for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], Policy::kEpiWarps); mbar_init(&emit_bar[b], 128); }
+    for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], Policy::kEpiWarps * (PAIR ? 2 : 1)); mbar_init(&emit_bar[b], 128); }
     fence_barrier_init();
   }
   if (warp == 1) {
-    tmem_alloc(tmem_slot, L::kTmemCols);
-    tmem_relinquish();
+    tmem_alloc<PAIR>(tmem_slot, L::kTmemCols);
+    tmem_relinquish<PAIR>();
   }
   tc_fence_before_sync();
-  __syncthreads();
+  if constexpr (PAIR) cluster_sync(); else __syncthreads();
   tc_fence_after_sync();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = uniform(*tmem_slot);
   // Everything above (barriers, tensor memory, descriptor prefetch) may overlap the tail of the kernel
   // before this one in the stream; from here on its results are needed.
   NRS_PDL_WAIT();
   NRS_PDL_TRIGGER();   // the next kernel may be scheduled as this grid's SMs free up
 
   if (warp == 0) {
-    if (lane == 0) {
-      // ---------------- TMA producer
-      const uint32_t stage_bytes = (uint32_t)NPLANES * (pol.a_slice_bytes() + (uint32_t)L::kBTile);
-      uint32_t it = 0;   // ring position, runs on across tiles
-      bool ok = true;
-      for (long t = blockIdx.x; t < tmap.total && ok; t += gridDim.x) {
-        int tile_m, tile_n, z;
-        tmap.decode(t, &tile_m, &tile_n, &z);
-        const int batch = z / sp.splits, split = z - batch * sp.splits;
-        int kb_begin = split * sp.kb_per_split;
-        int kb_end = min(sp.kb_total, kb_begin + sp.kb_per_split);
-        if (!pol.clip(tile_m, tile_n, BN, &kb_begin, &kb_end)) continue;
-        const int n0 = tile_n * BN;
-        // Where the K-slices of this tile lie, stepped along instead of recomputed (the divisions of a recomputation per
-        // slice and plane made the one producing thread the bottleneck: 58 -> 72 us on a 64-channel convolution).
-        typename Policy::Cursor cur = pol.cursor(tile_m, batch, kb_begin);
-        for (int kb = kb_begin; kb < kb_end; ++kb, ++it) {
-          const int s = it % L::kStages;
-          const uint32_t ph = (it / L::kStages) & 1u;
-          if (!mbar_wait(&empty_bar[s], ph ^ 1u)) { atomicExch(err_flag, kErrProducerWait); ok = false; break; }
-          uint8_t* st = smem + s * L::kStage;
-          mbar_expect_tx(&full_bar[s], stage_bytes);
-          pol.load_a(st, &tm_a_hi, &full_bar[s], cur);
-          pol.template load_b<BN>(st + L::kATile, &tm_b_hi, &full_bar[s], cur, n0);
+    // ---------------- TMA producer
+    // Both CTAs of a pair count their bytes on the barrier of rank 0, which expects the sum.
+    const uint32_t stage_bytes = (uint32_t)(PAIR ? 2 : 1) * NPLANES * (pol.a_slice_bytes() + (uint32_t)L::kBTile);
+    uint32_t s = 0, ph = 0, issued = 0;   // ring slot, its use's parity, slices so far: run on across tiles
+    bool ok = true;
+    for (long t = t_first; t < tmap.total && ok; t += t_step) {
+      int tile_m, tile_n, z;
+      tmap.decode(t, &tile_m, &tile_n, &z);
+      if (PAIR) tile_m = 2 * tile_m + rank;   // beyond the last row tile: TMA fills zeros
+      const int batch = z / sp.splits, split = z - batch * sp.splits;
+      int kb_begin = split * sp.kb_per_split;
+      int kb_end = min(sp.kb_total, kb_begin + sp.kb_per_split);
+      if (!pol.clip(tile_m, tile_n, BN, &kb_begin, &kb_end)) continue;
+      const int n0 = tile_n * BN + (PAIR ? rank * (BN / 2) : 0);
+      // Where the K-slices of this tile lie, stepped along instead of recomputed (the divisions of a recomputation per
+      // slice and plane made the producer the bottleneck: 58 -> 72 us on a 64-channel convolution).
+      typename Policy::Cursor cur = pol.cursor(tile_m, batch, kb_begin);
+      for (int kb = kb_begin; kb < kb_end; ++kb) {
+        if (!mbar_wait_warp(&empty_bar[s], ph ^ 1u)) { ok = false; break; }
+        uint8_t* st = smem + s * L::kStage;
+        uint32_t bar;
+        if constexpr (PAIR) bar = cluster_addr(&full_bar[s], 0); else bar = smem_u32(&full_bar[s]);
+        if (elect_one()) {
+          if (rank == 0) mbar_expect_tx(&full_bar[s], stage_bytes);
+          pol.template load_a<PAIR>(st, &tm_a_hi, bar, cur);
+          pol.template load_b<BN, PAIR>(st + L::kATile, &tm_b_hi, bar, cur, n0);
           if (NPLANES == 2) {
-            pol.template load_b<BN>(st + L::kATile + L::kBTile, &tm_b_lo, &full_bar[s], cur, n0);
-            pol.load_a(st + L::kATile + 2 * L::kBTile, &tm_a_lo, &full_bar[s], cur);
+            pol.template load_b<BN, PAIR>(st + L::kATile + L::kBTile, &tm_b_lo, bar, cur, n0);
+            pol.template load_a<PAIR>(st + L::kATile + 2 * L::kBTile, &tm_a_lo, bar, cur);
           }
-          pol.advance(cur);
         }
+        __syncwarp();
+        pol.advance(cur);
+        ++issued;
+        if (++s == (uint32_t)L::kStages) { s = 0; ph ^= 1u; }
       }
-      if (!ok) {
-        // Loads already issued still land in this CTA's shared memory: wait for them
-        // (bounded) before the CTA may retire.
-        for (uint32_t j = (it > (uint32_t)L::kStages ? it - L::kStages : 0); j < it; ++j) {
-          const int s = j % L::kStages;
-          if (!mbar_wait(&full_bar[s], (j / L::kStages) & 1u)) { atomicExch(err_flag, kErrDrainWait); break; }
+    }
+    if (!ok) {
+      if (lane == 0) atomicExch(err_flag, kErrProducerWait);
+      // Loads already issued still land in this CTA's shared memory: wait for them
+      // (bounded) before the CTA may retire.  (Rank 1 of a pair has no barrier of its own to ask; its last load was
+      // issued a full wait limit, a second, ago.)
+      if (rank == 0) for (uint32_t j = (issued > (uint32_t)L::kStages ? issued - L::kStages : 0); j < issued; ++j) {
+        const int sj = j % L::kStages;
+        if (!mbar_wait_warp(&full_bar[sj], (j / L::kStages) & 1u)) {
+          if (lane == 0) atomicExch(err_flag, kErrDrainWait);
+          break;
         }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (rank == 0) {
       // ---------------- UMMA issuer
       constexpr bool kAMn = Policy::kAMnMajor, kBMn = Policy::kBMnMajor;
-      constexpr uint32_t idesc_wide = make_idesc_tf32(BM, NPLANES * BN, kAMn, kBMn);
-      constexpr uint32_t idesc_half = make_idesc_tf32(BM, BN, kAMn, kBMn);
+      constexpr int kRows = PAIR ? 2 * BM : BM;
+      constexpr uint32_t idesc_wide = make_idesc_tf32(kRows, NPLANES * BN, kAMn, kBMn);
+      constexpr uint32_t idesc_half = make_idesc_tf32(kRows, BN, kAMn, kBMn);
+      // A pair's wide product reads [B_hi half ; B_lo half] from each CTA, so its columns are hh0 hl0 hh1 hl1 (h: half of
+      // the tile's columns, 0 and 1).  The narrow one (lh0 lh1) is added to hl0 hh1, one half further on.
+      constexpr uint32_t kNarrow = PAIR ? BN / 2 : 0;
       // K-major: 8 elements of K are 32 bytes inside the swizzle row.  MN-major: 32-column blocks of [32 k][128 B], so
       // a K-step is 1024 bytes and blocks are 4096 apart (the blocks of B_lo follow those of B_hi).
       auto desc = [](bool mn, uint32_t addr, int k) {
         return mn ? make_smem_desc_sw128_32b(addr + (uint32_t)k * 1024u, BK * 128, 512) : make_smem_desc_sw128(addr + (uint32_t)k * 32u, 16, 1024);
       };
-      uint32_t it = 0, local = 0;
+      uint32_t s = 0, ph = 0, local = 0;
       bool ok = true;
-      for (long t = blockIdx.x; t < tmap.total && ok; t += gridDim.x) {
+      for (long t = t_first; t < tmap.total && ok; t += t_step) {
         int tile_m, tile_n, z;
         tmap.decode(t, &tile_m, &tile_n, &z);
         const int split = z % sp.splits;
@@ -236,30 +263,32 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
         const int nkb = kb_end - kb_begin;   // >= 1 by construction
         const uint32_t buf = local & 1u, use = local >> 1;
         ++local;
-        if (!mbar_wait(&acc_empty[buf], (use & 1u) ^ 1u)) { atomicExch(err_flag, kErrMmaWait); break; }
+        if (!(PAIR ? mbar_wait_warp_cluster(&acc_empty[buf], (use & 1u) ^ 1u) : mbar_wait_warp(&acc_empty[buf], (use & 1u) ^ 1u))) { ok = false; break; }
         tc_fence_after_sync();
         const uint32_t d = tmem_base + buf * (uint32_t)L::kAccCols;
-        for (int i = 0; i < nkb; ++i, ++it) {
-          const int s = it % L::kStages;
-          const uint32_t ph = (it / L::kStages) & 1u;
+        for (int i = 0; i < nkb; ++i) {
           // (No tcgen05 fence here: the mbarrier's complete_tx orders the TMA writes before the
           // UMMAs, and a fence would make the issuing thread wait out the UMMAs in flight.)
-          if (!mbar_wait(&full_bar[s], ph)) { atomicExch(err_flag, kErrMmaWait); ok = false; break; }
+          if (!mbar_wait_warp(&full_bar[s], ph)) { ok = false; break; }
           const uint32_t a_hi = smem_u32(smem + s * L::kStage);
           const uint32_t b_hi = a_hi + L::kATile;                 // B_lo follows B_hi directly
           const uint32_t a_lo = b_hi + 2 * L::kBTile;
+          if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < BK / 8; ++k) {
-            const uint64_t da_hi = desc(kAMn, a_hi, k), db_hi = desc(kBMn, b_hi, k);
-            umma_tf32(d, da_hi, db_hi, idesc_wide, (i | k) != 0);   // hi*hi | hi*lo
-            if (NPLANES == 2) {
-              umma_tf32(d, desc(kAMn, a_lo, k), db_hi, idesc_half, 1);             // + lo*hi
+            for (int k = 0; k < BK / 8; ++k) {
+              const uint64_t da_hi = desc(kAMn, a_hi, k), db_hi = desc(kBMn, b_hi, k);
+              umma_tf32<PAIR>(d, da_hi, db_hi, idesc_wide, (i | k) != 0);   // hi*hi | hi*lo
+              if (NPLANES == 2) umma_tf32<PAIR>(d + kNarrow, desc(kAMn, a_lo, k), db_hi, idesc_half, 1);   // + lo*hi
             }
+            umma_commit<PAIR>(&empty_bar[s]);  // slot reusable once these UMMAs have read it
           }
-          umma_commit(&empty_bar[s]);  // slot reusable once these UMMAs have read it
+          __syncwarp();
+          if (++s == (uint32_t)L::kStages) { s = 0; ph ^= 1u; }
         }
-        if (ok) umma_commit(&acc_full[buf]);
+        if (ok && elect_one()) umma_commit<PAIR>(&acc_full[buf]);
+        __syncwarp();
       }
+      if (!ok && lane == 0) atomicExch(err_flag, kErrMmaWait);
     }
   } else {
     // ---------------- epilogue: warp w owns TMEM lanes [32*(w%4), +32)
@@ -268,9 +297,10 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
     const bool emit_issuer = warp == 2 && lane == 0;
     uint32_t local = 0, emitted = 0;
     bool ok = true;
-    for (long t = blockIdx.x; t < tmap.total && ok; t += gridDim.x) {
+    for (long t = t_first; t < tmap.total && ok; t += t_step) {
       int tile_m, tile_n, z;
       tmap.decode(t, &tile_m, &tile_n, &z);
+      if (PAIR) tile_m = 2 * tile_m + rank;
       const int batch = z / sp.splits, split = z - batch * sp.splits;
       int kb_begin = split * sp.kb_per_split, kb_end = min(sp.kb_total, kb_begin + sp.kb_per_split);
       if (!pol.clip(tile_m, tile_n, BN, &kb_begin, &kb_end)) continue;   // the same verdict in all three roles
@@ -283,9 +313,15 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
         break;
       }
       tc_fence_after_sync();
-      if (BN == 32 && warp >= 6) {   // one column block only: the second warp of a quarter just hands the accumulator back
+      auto hand_back = [&]() {   // to the issuing thread, which a pair has in rank 0
         __syncwarp();
-        if (lane == 0) mbar_arrive(&acc_empty[buf]);
+        if (lane != 0) return;
+        if constexpr (PAIR) mbar_arrive_cluster(cluster_addr(&acc_empty[buf], 0)); else mbar_arrive(&acc_empty[buf]);
+      };
+      // one column block only: the second warp of a quarter just hands the accumulator back, and so do all of a pair's
+      // second CTA beyond the last row tile
+      if ((BN == 32 && warp >= 6) || (PAIR && tile_m * BM >= sp.rows_total)) {
+        hand_back();
         continue;
       }
       const uint32_t acc = tmem_base + buf * (uint32_t)L::kAccCols + ((uint32_t)(q * 32) << 16);
@@ -294,10 +330,12 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
 #pragma unroll 1
       for (int c = kStep == 1 ? 0 : (warp - 2) >> 2; c < kBlocks; c += kStep) {
         uint32_t r[32];
-        tmem_ld_32x32(acc + (uint32_t)(c * 32), r);
+        // the columns of the first and of the second product (a pair: see kNarrow)
+        const int first = PAIR && NPLANES == 2 && c * 32 >= BN / 2 ? BN / 2 + c * 32 : c * 32;
+        tmem_ld_32x32(acc + (uint32_t)first, r);
         if (NPLANES == 2) {
           uint32_t r2[32];
-          tmem_ld_32x32(acc + (uint32_t)(BN + c * 32), r2);
+          tmem_ld_32x32(acc + (uint32_t)(first + (PAIR ? BN / 2 : BN)), r2);
           tmem_ld_wait();
 #pragma unroll
           for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(r2[j]));
@@ -307,8 +345,7 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
         if (c + kStep >= kBlocks) {
           // Everything this warp needs is in registers: hand the accumulator back.
           tc_fence_before_sync();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&acc_empty[buf]);
+          hand_back();
         }
         if (n0 + c * 32 >= sp.n_total) continue;   // padding columns of a ragged last tile
         if constexpr (!Policy::kCanEmit) {
@@ -384,10 +421,12 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
   }
 
   tc_fence_before_sync();
-  __syncthreads();
+  // (a pair: neither CTA may leave while the other's UMMAs read its memory or arrive on its barriers)
+  __syncwarp();
+  if constexpr (PAIR) cluster_sync(); else __syncthreads();
   if (warp == 1) {
     tc_fence_after_sync();
-    tmem_dealloc(tmem_base, L::kTmemCols);
+    tmem_dealloc<PAIR>(tmem_base, L::kTmemCols);
   }
 }
 
@@ -432,6 +471,33 @@ inline void plan_split(const nrs_ctx* ctx, long tiles, long out_elems, int kb_to
   *splits = (kb_total + per - 1) / per;
 }
 
+// The tile of a launch: its columns, and whether CTAs work in pairs.  kPlans holds the measured clocks per K-slice (3xTF32,
+// TF32), and per tile about what the accumulator's way out adds where nothing hides it.  The tile with the least (rounds
+// of the grid) x (clocks per tile) is taken, a K-split's second pass counted in: wide tiles for large outputs, narrower
+// ones where they fill SMs that would idle or where a ragged column count would pad, pairs where there are enough row
+// tiles.  `limit`: widest tile allowed.
+struct TilePlan { int bn; bool pair; };
+inline TilePlan plan_tile(const nrs_ctx* ctx, long tiles_m, int n, long batches, int kblocks, bool split_planes, int limit = 128) {
+  static const struct { int bn; bool pair; int kb_clk[2], tile_clk; } kPlans[] = {{128, true, {820, 345}, 2600},
+                                                                                  {64, true, {565, 317}, 1700},
+                                                                                  {128, false, {905, 428}, 2600},
+                                                                                  {64, false, {660, 369}, 1700},
+                                                                                  {32, false, {570, 352}, 1300}};
+  TilePlan best{32, false};
+  double best_t = -1.0;
+  for (const auto& c : kPlans) {
+    if (c.bn > limit || (c.bn > 32 && c.bn / 2 >= n)) continue;   // half of the tile or more would be padding
+    const long tiles_n = (n + c.bn - 1) / c.bn;
+    int splits, per;
+    plan_split(ctx, tiles_m * tiles_n * batches, tiles_m * BM * n * batches, kblocks, split_planes, &splits, &per);
+    const long units = (c.pair ? (tiles_m + 1) / 2 : tiles_m) * tiles_n * batches * splits, slots = ctx->sm_count / (c.pair ? 2 : 1);
+    double t = (double)((units + slots - 1) / slots) * ((double)per * c.kb_clk[split_planes ? 0 : 1] + c.tile_clk);
+    if (splits > 1) t += 6000.0 + 4e-4 * (double)splits * tiles_m * BM * n * batches;   // a launch; partial tiles from L2 at 20 TB/s
+    if (best_t < 0.0 || t < best_t) { best_t = t; best = TilePlan{c.bn, c.pair}; }
+  }
+  return best;
+}
+
 // Work units (pixel tiles, image rows) per CTA for a reduction that is split across CTAs, `ctas`
 // CTAs per split and one CTA per SM at a time.  Candidates put the CTA count just under a whole
 // number of waves (a count just over one costs a whole extra round); a CTA's fixed cost
@@ -456,15 +522,15 @@ inline int plan_units_per_cta(int sm_count, int ctas, long units, int min_units,
   return (int)(best_u < 1 ? 1 : best_u);
 }
 
-template <int BN, int NPLANES, class Policy>
+template <int BN, int NPLANES, bool PAIR, class Policy>
 int launch(nrs_ctx* ctx, const CUtensorMap& ta_hi, const CUtensorMap& ta_lo, const CUtensorMap& tb_hi,
            const CUtensorMap& tb_lo, const Policy& pol, int tiles_m, int n_total, int batches, int kb_total,
            const CUtensorMap* out_hi = nullptr, const CUtensorMap* out_lo = nullptr, int* splits_out = nullptr) {
-  using L = SmemLayout<BN, NPLANES, emit_bytes<NPLANES, Policy>()>;
+  using L = SmemLayout<BN, NPLANES, emit_bytes<NPLANES, Policy>(), PAIR>;
   constexpr int kSmem = L::kBytes;
   static_assert(kSmem <= 227 * 1024 && L::kStages >= 2, "shared memory budget");
   static NrsSmemAttr attr;
-  NRS_ENSURE_SMEM(ctx, attr, (tc_kernel<BN, NPLANES, Policy>), kSmem);
+  NRS_ENSURE_SMEM(ctx, attr, (tc_kernel<BN, NPLANES, Policy, PAIR>), kSmem);
   const int tiles_n = (n_total + BN - 1) / BN;
   SplitInfo sp{};
   if (Policy::kMaySplit) {
@@ -488,12 +554,14 @@ int launch(nrs_ctx* ctx, const CUtensorMap& ta_hi, const CUtensorMap& ta_lo, con
   int* err = nullptr;
   int st = nrs_err_flag(ctx, &err);
   if (st != NRS_OK) return st;
-  TileMap tmap{tiles_m, tiles_n, (long)tiles_m * tiles_n * batches * sp.splits};
-  const unsigned grid = (unsigned)(tmap.total < ctx->sm_count ? tmap.total : ctx->sm_count);
+  const int units_m = PAIR ? (tiles_m + 1) / 2 : tiles_m;
+  TileMap tmap{units_m, tiles_n, (long)units_m * tiles_n * batches * sp.splits};
+  const long slots = PAIR ? ctx->sm_count / 2 : ctx->sm_count;
+  const unsigned grid = (unsigned)((tmap.total < slots ? tmap.total : slots) * (PAIR ? 2 : 1));
   // Planes can only be emitted by the direct epilogue; with a K-split the policy's store() writes them.
   const int emit = (Policy::kCanEmit && out_hi && sp.splits == 1) ? (out_lo && NPLANES == 2 ? 2 : 1) : 0;
-  NRS_PDL_LAUNCH((tc_kernel<BN, NPLANES, Policy>), grid, threads<Policy>(), kSmem, ctx->stream, ta_hi, ta_lo, tb_hi, tb_lo,
-                 out_hi ? *out_hi : ta_hi, out_lo ? *out_lo : ta_hi, pol, sp, tmap, emit, err);
+  (void)nrs_pdl_launch_cluster(PAIR ? 2 : 1, tc_kernel<BN, NPLANES, Policy, PAIR>, dim3(grid), dim3(threads<Policy>()), (size_t)kSmem, ctx->stream,
+                               ta_hi, ta_lo, tb_hi, tb_lo, out_hi ? *out_hi : ta_hi, out_lo ? *out_lo : ta_hi, pol, sp, tmap, emit, err);
   NRS_LAUNCHED(ctx);
   if (sp.splits > 1) {
     const size_t per = (size_t)batches * sp.rows_total * n_total;

@@ -70,7 +70,7 @@ tc_wgrad_kernel(const __grid_constant__ CUtensorMap tm_dy_hi, const __grid_const
   uint64_t* accum_bar = empty_bar + STAGES;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accum_bar + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = (int)tc::uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int cbk = blockIdx.x % p.col_blocks;
   const int mg = blockIdx.x / p.col_blocks;
   const int mb = mg / p.n_groups, grp = mg - mb * p.n_groups;
@@ -98,96 +98,111 @@ tc_wgrad_kernel(const __grid_constant__ CUtensorMap tm_dy_hi, const __grid_const
   tc::tc_fence_before_sync();
   __syncthreads();
   tc::tc_fence_after_sync();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = tc::uniform(*tmem_slot);
   if (!p.independent) NRS_PDL_WAIT();   // set-up above may overlap the previous kernel's tail; its results are needed from here
   NRS_PDL_TRIGGER();
 
+  // (Both issuing roles run as whole warps and elect a lane for the instructions themselves: tc::elect_one.)
   if (warp == 0) {
-    if (lane == 0) {
-      // ---------------- TMA producer: one pixel tile per ring slot
-      // One 5-D box per operand plane brings all 32-channel blocks of a pixel tile at once
-      // (the channel-block index is the outermost box dimension), so a tile costs
-      // planes x (1 + taps) TMA instructions instead of one per block.
-      // (a ragged last column block still receives a full box: TMA zero-fills the blocks beyond the tensor)
-      const uint32_t tx = NPLANES * (uint32_t)(p.a_box_blocks + ntaps * (p.col_blocks > 1 ? 8 : p.cblocks)) * blk_bytes;
-      const int i_first = tap0 / p.kw, j_first = tap0 - i_first * p.kw;
-      const int x_blocks = p.col_blocks > 1 ? 8 : p.cblocks;
-      int issued = 0;
-      bool ok = true;
-      for (int it = 0; it < ntiles; ++it, ++issued) {
-        const int s = it % STAGES;
-        const uint32_t ph = (uint32_t)(it / STAGES) & 1u;
-        if (!tc::mbar_wait(&empty_bar[s], ph ^ 1u)) { atomicExch(err_flag, tc::kErrProducerWait); ok = false; break; }
-        const int pt = t_begin + it;
-        const int xt = pt % p.tiles_x, rest = pt / p.tiles_x;
-        const int n0 = (rest / p.tiles_y) * p.Nt, y0 = (rest % p.tiles_y) * p.Ht, x0 = xt * p.Wt;
-        uint8_t* st = smem + (size_t)s * stage_bytes;
-        tc::mbar_expect_tx(&full_bar[s], tx);
-#pragma unroll 1
+    // ---------------- TMA producer: one pixel tile per ring slot
+    // One 5-D box per operand plane brings all 32-channel blocks of a pixel tile at once
+    // (the channel-block index is the outermost box dimension), so a tile costs
+    // planes x (1 + taps) TMA instructions instead of one per block.
+    // (a ragged last column block still receives a full box: TMA zero-fills the blocks beyond the tensor)
+    const uint32_t tx = NPLANES * (uint32_t)(p.a_box_blocks + ntaps * (p.col_blocks > 1 ? 8 : p.cblocks)) * blk_bytes;
+    const int i_first = tap0 / p.kw, j_first = tap0 - i_first * p.kw;
+    const int x_blocks = p.col_blocks > 1 ? 8 : p.cblocks;
+    int xt = t_begin % p.tiles_x, yt = t_begin / p.tiles_x;   // the tile's place, stepped along
+    int nt = yt / p.tiles_y;
+    yt -= nt * p.tiles_y;
+    int issued = 0, s = 0;
+    uint32_t ph = 0;
+    bool ok = true;
+    for (int it = 0; it < ntiles; ++it, ++issued) {
+      if (!tc::mbar_wait_warp(&empty_bar[s], ph ^ 1u)) { ok = false; break; }
+      const int n0 = nt * p.Nt, y0 = yt * p.Ht, x0 = xt * p.Wt;
+      uint8_t* st = smem + (size_t)s * stage_bytes;
+      uint64_t* bar = &full_bar[s];
+      if (tc::elect_one()) {
+        tc::mbar_expect_tx(bar, tx);
+#pragma unroll
         for (int pl = 0; pl < NPLANES; ++pl) {
           const CUtensorMap* tdy = pl == 0 ? &tm_dy_hi : &tm_dy_lo;
           const CUtensorMap* txm = pl == 0 ? &tm_x_hi : &tm_x_lo;
           uint8_t* a_dst = st + pl * (a_bytes + b_bytes);
           uint8_t* b_dst = a_dst + a_bytes;
           if (p.ragged_a) {
-            for (int b = 0; b < p.a_box_blocks; ++b)
-              tc::tma_load_4d(a_dst + b * blk_bytes, tdy, &full_bar[s], (mb * kABlocks + b) * 32, x0, y0, n0);
+#pragma unroll 1
+            for (int b = 0; b < p.a_box_blocks; ++b) tc::tma_load_4d(a_dst + b * blk_bytes, tdy, bar, (mb * kABlocks + b) * 32, x0, y0, n0);
           } else {
-            tc::tma_load_5d(a_dst, tdy, &full_bar[s], 0, x0, y0, n0, mb * kABlocks);
+            tc::tma_load_5d(a_dst, tdy, bar, 0, x0, y0, n0, mb * kABlocks);
           }
           int ti = i_first, tj = j_first;
+#pragma unroll 1
           for (int t = 0; t < ntaps; ++t) {
             const int xx = x0 * p.stride + tj - p.pad, xy = y0 * p.stride + ti - p.pad;
             uint8_t* dst = b_dst + (size_t)t * p.cblocks * blk_bytes;
             if (p.ragged_x) {
-              for (int b = 0; b < x_blocks; ++b) tc::tma_load_4d(dst + b * blk_bytes, txm, &full_bar[s], (cbk * 8 + b) * 32, xx, xy, n0);
+#pragma unroll 1
+              for (int b = 0; b < x_blocks; ++b) tc::tma_load_4d(dst + b * blk_bytes, txm, bar, (cbk * 8 + b) * 32, xx, xy, n0);
             } else {
-              tc::tma_load_5d(dst, txm, &full_bar[s], 0, xx, xy, n0, cbk * 8);
+              tc::tma_load_5d(dst, txm, bar, 0, xx, xy, n0, cbk * 8);
             }
             if (++tj == p.kw) { tj = 0; ++ti; }
           }
         }
       }
-      if (!ok) {
-        for (int it = (issued > STAGES ? issued - STAGES : 0); it < issued; ++it) {
-          const int s = it % STAGES;
-          if (!tc::mbar_wait(&full_bar[s], (uint32_t)(it / STAGES) & 1u)) { atomicExch(err_flag, tc::kErrDrainWait); break; }
+      __syncwarp();
+      if (++s == STAGES) { s = 0; ph ^= 1u; }
+      if (++xt == p.tiles_x) {
+        xt = 0;
+        if (++yt == p.tiles_y) { yt = 0; ++nt; }
+      }
+    }
+    if (!ok) {
+      if (lane == 0) atomicExch(err_flag, tc::kErrProducerWait);
+      for (int it = (issued > STAGES ? issued - STAGES : 0); it < issued; ++it) {
+        const int sj = it % STAGES;
+        if (!tc::mbar_wait_warp(&full_bar[sj], (uint32_t)(it / STAGES) & 1u)) {
+          if (lane == 0) atomicExch(err_flag, tc::kErrDrainWait);
+          break;
         }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      // ---------------- UMMA issuer: both operands MN-major, K-step = 8 pixels = one 1024 B atom
-      const uint32_t idesc = tc::make_idesc_tf32(128, n_cols, true, true);
-      bool ok = true;
-      const int ksteps = p.kp / 8;
-      for (int it = 0; it < ntiles; ++it) {
-        const int s = it % STAGES;
-        const uint32_t ph = (uint32_t)(it / STAGES) & 1u;
-        if (!tc::mbar_wait(&full_bar[s], ph)) { atomicExch(err_flag, tc::kErrMmaWait); ok = false; break; }
-        const uint32_t a_hi = tc::smem_u32(smem + (size_t)s * stage_bytes);
-        const uint32_t b_hi = a_hi + a_bytes;
-        const uint32_t a_lo = b_hi + b_bytes;
-        const uint32_t b_lo = a_lo + a_bytes;
-#pragma unroll 1
+    // ---------------- UMMA issuer: both operands MN-major, K-step = 8 pixels = one 1024 B atom
+    const uint32_t idesc = tc::make_idesc_tf32(128, n_cols, true, true);
+    const uint64_t dc = tc::make_smem_desc_sw128_32b(0, blk_bytes, 512);   // every field but the start address (bytes >> 4)
+    bool ok = true;
+    const int ksteps = p.kp / 8;
+    int s = 0;
+    uint32_t ph = 0;
+    for (int it = 0; it < ntiles; ++it) {
+      if (!tc::mbar_wait_warp(&full_bar[s], ph)) { ok = false; break; }
+      const uint32_t a_hi = tc::smem_u32(smem + (size_t)s * stage_bytes) >> 4;
+      const uint32_t b_hi = a_hi + (a_bytes >> 4);
+      const uint32_t a_lo = b_hi + (b_bytes >> 4);
+      const uint32_t b_lo = a_lo + (a_bytes >> 4);
+      if (tc::elect_one()) {
+#pragma unroll 2
         for (int k = 0; k < ksteps; ++k) {
-          const uint32_t koff = (uint32_t)k * 1024u;
-          const uint64_t da_hi = tc::make_smem_desc_sw128_32b(a_hi + koff, blk_bytes, 512);
-          const uint64_t db_hi = tc::make_smem_desc_sw128_32b(b_hi + koff, blk_bytes, 512);
+          const uint32_t koff = (uint32_t)k * 64u;
           if (NPLANES == 2) {
-            const uint64_t da_lo = tc::make_smem_desc_sw128_32b(a_lo + koff, blk_bytes, 512);
-            const uint64_t db_lo = tc::make_smem_desc_sw128_32b(b_lo + koff, blk_bytes, 512);
-            tc::umma_tf32(tmem_base, da_lo, db_hi, idesc, (it | k) != 0);
-            tc::umma_tf32(tmem_base, da_hi, db_lo, idesc, 1);
-            tc::umma_tf32(tmem_base, da_hi, db_hi, idesc, 1);
+            tc::umma_tf32(tmem_base, dc + (a_lo + koff), dc + (b_hi + koff), idesc, (it | k) != 0);
+            tc::umma_tf32(tmem_base, dc + (a_hi + koff), dc + (b_lo + koff), idesc, 1);
+            tc::umma_tf32(tmem_base, dc + (a_hi + koff), dc + (b_hi + koff), idesc, 1);
           } else {
-            tc::umma_tf32(tmem_base, da_hi, db_hi, idesc, (it | k) != 0);
+            tc::umma_tf32(tmem_base, dc + (a_hi + koff), dc + (b_hi + koff), idesc, (it | k) != 0);
           }
         }
         tc::umma_commit(&empty_bar[s]);
       }
-      if (ok) tc::umma_commit(accum_bar);
+      __syncwarp();
+      if (++s == STAGES) { s = 0; ph ^= 1u; }
     }
+    if (ok && tc::elect_one()) tc::umma_commit(accum_bar);
+    if (!ok && lane == 0) atomicExch(err_flag, tc::kErrMmaWait);
+    __syncwarp();
   } else {
     // ---------------- epilogue: raw partial tile to the workspace
     const int q = warp & 3;
@@ -218,6 +233,7 @@ tc_wgrad_kernel(const __grid_constant__ CUtensorMap tm_dy_hi, const __grid_const
   }
 
   if (p.independent) NRS_PDL_WAIT();   // nothing after this kernel may run ahead of its predecessor
+  __syncwarp();
   tc::tc_fence_before_sync();
   __syncthreads();
   if (warp == 1) {

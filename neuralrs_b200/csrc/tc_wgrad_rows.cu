@@ -112,7 +112,7 @@ tc_wgrad_rows_kernel(const __grid_constant__ CUtensorMap tm_dy_hi, const __grid_
   uint64_t* accum_bar = empty_x + p.SX;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accum_bar + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = (int)tc::uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   // blockIdx.x = (m block, horizontal tap kind, channel chunk).  Unpacked: kind = tap j, x shifted by
   // j - 1.  Packed: kind 0 shifts x by 0 and holds taps j = 1 (plain dy rows) and j = 0 (dy shifted one
   // pixel: sum_p dy[p+1] x[p] = sum_p dy[p] x[p-1]); kind 1 shifts x by +1 and holds j = 2 alone.
@@ -143,104 +143,118 @@ tc_wgrad_rows_kernel(const __grid_constant__ CUtensorMap tm_dy_hi, const __grid_
   tc::tc_fence_before_sync();
   __syncthreads();
   tc::tc_fence_after_sync();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = tc::uniform(*tmem_slot);
   if (!p.independent) NRS_PDL_WAIT();   // set-up above may overlap the previous kernel's tail; its results are needed from here
   NRS_PDL_TRIGGER();
 
+  // (Both issuing roles run as whole warps and elect a lane for the instructions themselves: tc::elect_one.)
   if (warp == 0) {
-    if (lane == 0) {
-      // ---------------- TMA producer.  Step t: x row r0-1+t (if it exists) and dy row r0+t-2 (t >= 2).
-      int sx = 0, sa = 0;
-      uint32_t phx = 0, pha = 0;
-      int xr = r0 - 1, xy = 0, xn = 0;          // x row, and its (row in image, image)
-      if (xr >= 0) { xn = xr / p.H; xy = xr - xn * p.H; } else { xy = -1; }
-      int dn = r0 / p.H, dyy = r0 - dn * p.H;   // dy row of step 2
-      bool ok = true;
-      int t = 0;
-      for (; t < nsteps; ++t) {
-        if (!tc::mbar_wait(&empty_x[sx], phx ^ 1u)) { atomicExch(err_flag, tc::kErrProducerWait); ok = false; break; }
-        const bool has_x = xr >= 0 && xr < p.rows_total;
+    // ---------------- TMA producer.  Step t: x row r0-1+t (if it exists) and dy row r0+t-2 (t >= 2).
+    int sx = 0, sa = 0;
+    uint32_t phx = 0, pha = 0;
+    int xr = r0 - 1, xy = 0, xn = 0;          // x row, and its (row in image, image)
+    if (xr >= 0) { xn = xr / p.H; xy = xr - xn * p.H; } else { xy = -1; }
+    int dn = r0 / p.H, dyy = r0 - dn * p.H;   // dy row of step 2
+    bool ok = true;
+    int t = 0;
+    for (; t < nsteps; ++t) {
+      if (!tc::mbar_wait_warp(&empty_x[sx], phx ^ 1u)) { ok = false; break; }
+      const bool has_x = xr >= 0 && xr < p.rows_total;
+      uint64_t* xbar = &full_x[sx];
+      uint8_t* x_dst = x_base + (size_t)sx * x_slot;
+      if (tc::elect_one()) {
         if (has_x) {
-          tc::mbar_expect_tx(&full_x[sx], NPLANES * x_slot);
-          tc::tma_load_5d(x_base + (size_t)sx * x_slot, &tm_x_hi, &full_x[sx], 0, x_shift, xy, xn, cc * (p.chunk / 32));
-          if (NPLANES == 2)
-            tc::tma_load_5d(x_base + x_ring + (size_t)sx * x_slot, &tm_x_lo, &full_x[sx], 0, x_shift, xy, xn, cc * (p.chunk / 32));
+          tc::mbar_expect_tx(xbar, NPLANES * x_slot);
+          tc::tma_load_5d(x_dst, &tm_x_hi, xbar, 0, x_shift, xy, xn, cc * (p.chunk / 32));
+          if (NPLANES == 2) tc::tma_load_5d(x_dst + x_ring, &tm_x_lo, xbar, 0, x_shift, xy, xn, cc * (p.chunk / 32));
         } else {
-          tc::mbar_arrive(&full_x[sx]);
+          tc::mbar_arrive(xbar);
         }
-        if (t >= 2) {
-          if (!tc::mbar_wait(&empty_a[sa], pha ^ 1u)) { atomicExch(err_flag, tc::kErrProducerWait); ok = false; ++t; break; }
-          tc::mbar_expect_tx(&full_a[sa], NPLANES * (two_taps ? 2u : 1u) * a_box);
-          uint8_t* a_dst = a_base + (size_t)sa * a_slot;
-          tc::tma_load_5d(a_dst, &tm_dy_hi, &full_a[sa], 0, 0, dyy, dn, mb * 4);
-          if (two_taps) tc::tma_load_5d(a_dst + a_box, &tm_dy_hi, &full_a[sa], 0, 1, dyy, dn, mb * 4);
+      }
+      __syncwarp();
+      if (t >= 2) {
+        if (!tc::mbar_wait_warp(&empty_a[sa], pha ^ 1u)) { ok = false; ++t; break; }
+        uint64_t* abar = &full_a[sa];
+        uint8_t* a_dst = a_base + (size_t)sa * a_slot;
+        if (tc::elect_one()) {
+          tc::mbar_expect_tx(abar, NPLANES * (two_taps ? 2u : 1u) * a_box);
+          tc::tma_load_5d(a_dst, &tm_dy_hi, abar, 0, 0, dyy, dn, mb * 4);
+          if (two_taps) tc::tma_load_5d(a_dst + a_box, &tm_dy_hi, abar, 0, 1, dyy, dn, mb * 4);
           if (NPLANES == 2) {
-            tc::tma_load_5d(a_dst + a_plane, &tm_dy_lo, &full_a[sa], 0, 0, dyy, dn, mb * 4);
-            if (two_taps) tc::tma_load_5d(a_dst + a_plane + a_box, &tm_dy_lo, &full_a[sa], 0, 1, dyy, dn, mb * 4);
+            tc::tma_load_5d(a_dst + a_plane, &tm_dy_lo, abar, 0, 0, dyy, dn, mb * 4);
+            if (two_taps) tc::tma_load_5d(a_dst + a_plane + a_box, &tm_dy_lo, abar, 0, 1, dyy, dn, mb * 4);
           }
-          if (++sa == p.SA) { sa = 0; pha ^= 1u; }
-          if (++dyy == p.H) { dyy = 0; ++dn; }
         }
-        if (++sx == p.SX) { sx = 0; phx ^= 1u; }
-        ++xr;
-        if (++xy == p.H) { xy = 0; ++xn; }
+        __syncwarp();
+        if (++sa == p.SA) { sa = 0; pha ^= 1u; }
+        if (++dyy == p.H) { dyy = 0; ++dn; }
       }
-      if (!ok) {
-        // Loads already issued still land in this CTA's shared memory: wait for them (bounded)
-        // before the CTA may retire.  Walk the last ring's worth of steps.
-        for (int u = (t > p.SX ? t - p.SX : 0); u < t; ++u)
-          if (!tc::mbar_wait(&full_x[u % p.SX], (uint32_t)(u / p.SX) & 1u)) { atomicExch(err_flag, tc::kErrDrainWait); break; }
-        for (int u = (t - 2 > p.SA ? t - 2 - p.SA : 0); u < t - 2; ++u)
-          if (!tc::mbar_wait(&full_a[u % p.SA], (uint32_t)(u / p.SA) & 1u)) { atomicExch(err_flag, tc::kErrDrainWait); break; }
-      }
+      if (++sx == p.SX) { sx = 0; phx ^= 1u; }
+      ++xr;
+      if (++xy == p.H) { xy = 0; ++xn; }
+    }
+    if (!ok) {
+      if (lane == 0) atomicExch(err_flag, tc::kErrProducerWait);
+      // Loads already issued still land in this CTA's shared memory: wait for them (bounded)
+      // before the CTA may retire.  Walk the last ring's worth of steps.
+      bool drained = true;
+      for (int u = (t > p.SX ? t - p.SX : 0); u < t && drained; ++u) drained = tc::mbar_wait_warp(&full_x[u % p.SX], (uint32_t)(u / p.SX) & 1u);
+      for (int u = (t - 2 > p.SA ? t - 2 - p.SA : 0); u < t - 2 && drained; ++u)
+        drained = tc::mbar_wait_warp(&full_a[u % p.SA], (uint32_t)(u / p.SA) & 1u);
+      if (!drained && lane == 0) atomicExch(err_flag, tc::kErrDrainWait);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      // ---------------- UMMA issuer
-      bool ok = true;
-      uint32_t started = 0;   // bit i: vertical tap i's accumulator columns hold a sum already
-      const uint64_t dc = tc::make_smem_desc_sw128_32b(0, blk, 512);
-      const uint32_t a_base16 = tc::smem_u32(a_base) >> 4, x_base16 = tc::smem_u32(x_base) >> 4;
-      const uint32_t a_slot16 = a_slot >> 4, a_plane16 = a_plane >> 4, x_slot16 = x_slot >> 4, x_ring16 = x_ring >> 4;
-      // instruction descriptor of a run of `len` taps: N = len * chunk sits in bits [17,23) as N >> 3
-      const uint32_t idesc_n0 = tc::make_idesc_tf32(128, 0, true, true);
-      const uint32_t idesc_per_tap = (uint32_t)(p.chunk >> 3) << 17;
-      int sx = 0, sa = 0;
-      uint32_t phx = 0, pha = 0;
-      int y = r0 % p.H;
-      for (int t = 0; t < nsteps; ++t) {
-        if (!tc::mbar_wait(&full_x[sx], phx)) { atomicExch(err_flag, tc::kErrMmaWait); ok = false; break; }
-        if (t >= 2) {
-          if (!tc::mbar_wait(&full_a[sa], pha)) { atomicExch(err_flag, tc::kErrMmaWait); ok = false; break; }
-          const uint32_t a_hi16 = a_base16 + (uint32_t)sa * a_slot16;
-          const uint32_t a_lo16 = a_hi16 + a_plane16;
-          int sx0 = sx - 2;                     // slot of the x row brought in at step t-2
-          if (sx0 < 0) sx0 += p.SX;
-          // vertical tap i reads the x row brought in at step t-2+i
-          int i = y == 0 ? 1 : 0;
-          const int i_end = y == p.H - 1 ? 2 : 3;
-          while (i < i_end) {
-            int s0 = sx0 + i;
-            if (s0 >= p.SX) s0 -= p.SX;
-            int len = 1;
-            while (len < p.max_run && i + len < i_end && s0 + len < p.SX &&
-                   ((started >> (i + len)) & 1u) == ((started >> i) & 1u))
-              ++len;
-            const uint32_t b_hi16 = x_base16 + (uint32_t)s0 * x_slot16;
-            issue_row<NPLANES, KS>(tmem_base + (uint32_t)(i * p.chunk), dc, a_hi16, a_lo16, b_hi16, b_hi16 + x_ring16,
-                                   idesc_n0 + (uint32_t)len * idesc_per_tap, (started >> i) & 1u);
-            started |= ((1u << len) - 1u) << i;
-            i += len;
-          }
+    // ---------------- UMMA issuer
+    bool ok = true;
+    uint32_t started = 0;   // bit i: vertical tap i's accumulator columns hold a sum already
+    const uint64_t dc = tc::make_smem_desc_sw128_32b(0, blk, 512);
+    const uint32_t a_base16 = tc::smem_u32(a_base) >> 4, x_base16 = tc::smem_u32(x_base) >> 4;
+    const uint32_t a_slot16 = a_slot >> 4, a_plane16 = a_plane >> 4, x_slot16 = x_slot >> 4, x_ring16 = x_ring >> 4;
+    // instruction descriptor of a run of `len` taps: N = len * chunk sits in bits [17,23) as N >> 3
+    const uint32_t idesc_n0 = tc::make_idesc_tf32(128, 0, true, true);
+    const uint32_t idesc_per_tap = (uint32_t)(p.chunk >> 3) << 17;
+    int sx = 0, sa = 0;
+    uint32_t phx = 0, pha = 0;
+    int y = r0 % p.H;
+    for (int t = 0; t < nsteps; ++t) {
+      if (!tc::mbar_wait_warp(&full_x[sx], phx)) { ok = false; break; }
+      if (t >= 2) {
+        if (!tc::mbar_wait_warp(&full_a[sa], pha)) { ok = false; break; }
+        const uint32_t a_hi16 = a_base16 + (uint32_t)sa * a_slot16;
+        const uint32_t a_lo16 = a_hi16 + a_plane16;
+        int sx0 = sx - 2;                     // slot of the x row brought in at step t-2
+        if (sx0 < 0) sx0 += p.SX;
+        // vertical tap i reads the x row brought in at step t-2+i
+        int i = y == 0 ? 1 : 0;
+        const int i_end = y == p.H - 1 ? 2 : 3;
+        while (i < i_end) {
+          int s0 = sx0 + i;
+          if (s0 >= p.SX) s0 -= p.SX;
+          int len = 1;
+          while (len < p.max_run && i + len < i_end && s0 + len < p.SX &&
+                 ((started >> (i + len)) & 1u) == ((started >> i) & 1u))
+            ++len;
+          const uint32_t b_hi16 = x_base16 + (uint32_t)s0 * x_slot16;
+          const uint32_t acc = (started >> i) & 1u, idesc = idesc_n0 + (uint32_t)len * idesc_per_tap;
+          if (tc::elect_one())
+            issue_row<NPLANES, KS>(tmem_base + (uint32_t)(i * p.chunk), dc, a_hi16, a_lo16, b_hi16, b_hi16 + x_ring16, idesc, acc);
+          __syncwarp();
+          started |= ((1u << len) - 1u) << i;
+          i += len;
+        }
+        if (tc::elect_one()) {
           tc::umma_commit(&empty_a[sa]);    // this dy row is done with
           tc::umma_commit(&empty_x[sx0]);   // and so is the x row of step t-2
-          if (++sa == p.SA) { sa = 0; pha ^= 1u; }
-          if (++y == p.H) y = 0;
         }
-        if (++sx == p.SX) { sx = 0; phx ^= 1u; }
+        __syncwarp();
+        if (++sa == p.SA) { sa = 0; pha ^= 1u; }
+        if (++y == p.H) y = 0;
       }
-      if (ok) tc::umma_commit(accum_bar);
+      if (++sx == p.SX) { sx = 0; phx ^= 1u; }
     }
+    if (ok && tc::elect_one()) tc::umma_commit(accum_bar);
+    if (!ok && lane == 0) atomicExch(err_flag, tc::kErrMmaWait);
+    __syncwarp();
   } else {
     // ---------------- epilogue: raw partial tile to the workspace (zeros for taps that never ran)
     const int q = warp & 3;
@@ -274,6 +288,7 @@ tc_wgrad_rows_kernel(const __grid_constant__ CUtensorMap tm_dy_hi, const __grid_
   }
 
   if (p.independent) NRS_PDL_WAIT();   // nothing after this kernel may run ahead of its predecessor
+  __syncwarp();
   tc::tc_fence_before_sync();
   __syncthreads();
   if (warp == 1) {
