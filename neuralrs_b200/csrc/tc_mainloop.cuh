@@ -475,9 +475,11 @@ inline void plan_split(const nrs_ctx* ctx, long tiles, long out_elems, int kb_to
 // TF32), and per tile about what the accumulator's way out adds where nothing hides it.  The tile with the least (rounds
 // of the grid) x (clocks per tile) is taken, a K-split's second pass counted in: wide tiles for large outputs, narrower
 // ones where they fill SMs that would idle or where a ragged column count would pad, pairs where there are enough row
-// tiles.  `limit`: widest tile allowed.
+// tiles.  `reduce_clk`: what the second pass over a K-split costs per output value, on top of its launch (measured: 3.6 us
+// for 51 thousand values of a GEMM, 13.4 us for 819 thousand of a convolution, whose pixels lie strided).  `limit`:
+// widest tile allowed.
 struct TilePlan { int bn; bool pair; };
-inline TilePlan plan_tile(const nrs_ctx* ctx, long tiles_m, int n, long batches, int kblocks, bool split_planes, int limit = 128) {
+inline TilePlan plan_tile(const nrs_ctx* ctx, long tiles_m, int n, long batches, int kblocks, bool split_planes, double reduce_clk, int limit = 128) {
   static const struct { int bn; bool pair; int kb_clk[2], tile_clk; } kPlans[] = {{128, true, {820, 345}, 2600},
                                                                                   {64, true, {565, 317}, 1700},
                                                                                   {128, false, {905, 428}, 2600},
@@ -492,7 +494,7 @@ inline TilePlan plan_tile(const nrs_ctx* ctx, long tiles_m, int n, long batches,
     plan_split(ctx, tiles_m * tiles_n * batches, tiles_m * BM * n * batches, kblocks, split_planes, &splits, &per);
     const long units = (c.pair ? (tiles_m + 1) / 2 : tiles_m) * tiles_n * batches * splits, slots = ctx->sm_count / (c.pair ? 2 : 1);
     double t = (double)((units + slots - 1) / slots) * ((double)per * c.kb_clk[split_planes ? 0 : 1] + c.tile_clk);
-    if (splits > 1) t += 6000.0 + 4e-4 * (double)splits * tiles_m * BM * n * batches;   // a launch; partial tiles from L2 at 20 TB/s
+    if (splits > 1) t += 4000.0 + reduce_clk * (double)tiles_m * BM * n * batches;
     if (best_t < 0.0 || t < best_t) { best_t = t; best = TilePlan{c.bn, c.pair}; }
   }
   return best;
