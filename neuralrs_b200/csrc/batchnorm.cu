@@ -9,7 +9,13 @@
 //   forward   S = sum(x - K), Q = sum((x - K)^2) with the pivot K = the channel's first element, which keeps
 //             Q/N - (S/N)^2 free of the cancellation a raw sum of squares has when |mean| >> std;
 //   backward  S = sum(g) = dbeta, Q = sum(g * xhat) = dgamma.
-// x is read twice in the forward pass (statistics, normalise) and g / xhat twice in the backward pass.
+// x is read twice in the forward pass (statistics, normalise) and g / xhat twice in the backward pass.  The graph keeps
+// no xhat: it saves the means, and the backward kernels take x and recompute (x - mean) * istd, the forward pass's very
+// expression (4 B per element less written).  Where a tensor-core convolution reads the output, or made the input, the
+// normalise and dx kernels also write the NHWC planes that it wants, and the dx kernel the per-tile channel sums that
+// the convolution's bias gradient folds.  Measured (256 images of 64 x 32 x 32, TF32): staging and channel sums as
+// passes of their own took 27 and 26 us a tensor.
+#include "image_tile.cuh"
 #include "nrs_internal.h"
 
 namespace {
@@ -46,7 +52,7 @@ template <bool FWD, bool RELU>
 __global__ void __launch_bounds__(kThreads)
 bn_pair_planes_kernel(const float* __restrict__ a, const float* __restrict__ b, float2* __restrict__ partial, int n,
                       int c, int hw, int splits, const float* __restrict__ gamma, const float* __restrict__ beta,
-                      const float* __restrict__ pivot) {
+                      const float* __restrict__ pivot, const float* __restrict__ mean, const float* __restrict__ istd) {
   NRS_PDL_PROLOGUE();
   __shared__ float2 sm[kThreads / 32];
   const int ch = blockIdx.x, split = blockIdx.y;
@@ -55,6 +61,7 @@ bn_pair_planes_kernel(const float* __restrict__ a, const float* __restrict__ b, 
   const int n0 = split * n_per, n1 = min(n, n0 + n_per);
   const float k = FWD ? (pivot ? pivot[ch] : a[(size_t)ch * hw]) : 0.0f;
   const float ga = RELU ? gamma[ch] : 0.0f, be = RELU ? beta[ch] : 0.0f;
+  const float mu = mean ? mean[ch] : 0.0f, is = mean ? istd[ch] : 1.0f;   // b is x; without them xhat itself
   const bool vec = (hw & 3) == 0 && aligned16(a) && (FWD || aligned16(b));
   // The block's threads walk the split's (image, element) pairs as one flat index, so that planes shorter
   // than a warp's reach (8x8, 4x4 feature maps) still keep every lane loading.
@@ -67,7 +74,10 @@ bn_pair_planes_kernel(const float* __restrict__ a, const float* __restrict__ b, 
     if (vec) {
       float4 va = reinterpret_cast<const float4*>(a + base)[i];
       float4 vb = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (!FWD) vb = reinterpret_cast<const float4*>(b + base)[i];
+      if (!FWD) {
+        vb = reinterpret_cast<const float4*>(b + base)[i];
+        vb = make_float4((vb.x - mu) * is, (vb.y - mu) * is, (vb.z - mu) * is, (vb.w - mu) * is);
+      }
       if (RELU) {
         va.x = fmaf(ga, vb.x, be) > 0.0f ? va.x : 0.0f;
         va.y = fmaf(ga, vb.y, be) > 0.0f ? va.y : 0.0f;
@@ -79,7 +89,7 @@ bn_pair_planes_kernel(const float* __restrict__ a, const float* __restrict__ b, 
       contribute<FWD>(va.z, vb.z, k, s, q);
       contribute<FWD>(va.w, vb.w, k, s1, q1);
     } else {
-      const float vb = FWD ? 0.0f : b[base + i];
+      const float vb = FWD ? 0.0f : (b[base + i] - mu) * is;
       float va = a[base + i];
       if (RELU) va = fmaf(ga, vb, be) > 0.0f ? va : 0.0f;
       contribute<FWD>(va, vb, k, s, q);
@@ -105,7 +115,7 @@ template <bool FWD, bool RELU>
 __global__ void __launch_bounds__(kThreads)
 bn_pair_cols_kernel(const float* __restrict__ a, const float* __restrict__ b, float2* __restrict__ partial, int rows,
                     int cols, int splits, const float* __restrict__ gamma, const float* __restrict__ beta,
-                    const float* __restrict__ pivot) {
+                    const float* __restrict__ pivot, const float* __restrict__ mean, const float* __restrict__ istd) {
   NRS_PDL_PROLOGUE();
   __shared__ float2 sm[kThreads / 32][33];
   const int lane = threadIdx.x & 31, wrp = threadIdx.x >> 5;
@@ -116,9 +126,10 @@ bn_pair_cols_kernel(const float* __restrict__ a, const float* __restrict__ b, fl
   if (col < cols) {
     const float k = FWD ? (pivot ? pivot[col] : a[col]) : 0.0f;
     const float ga = RELU ? gamma[col] : 0.0f, be = RELU ? beta[col] : 0.0f;
+    const float mu = mean ? mean[col] : 0.0f, is = mean ? istd[col] : 1.0f;
     for (int r = r0 + wrp; r < r1; r += kThreads / 32) {
       const size_t i = (size_t)r * cols + col;
-      const float vb = FWD ? 0.0f : b[i];
+      const float vb = FWD ? 0.0f : (b[i] - mu) * is;
       float va = a[i];
       if (RELU) va = fmaf(ga, vb, be) > 0.0f ? va : 0.0f;
       contribute<FWD>(va, vb, k, s, q);
@@ -223,7 +234,8 @@ template <bool VEC, bool RELU>
 __global__ void __launch_bounds__(kThreads)
 bn_dx_kernel(const float* __restrict__ g, const float* __restrict__ xhat, const float* __restrict__ istd,
              const float* __restrict__ gamma, const float* __restrict__ beta, const float2* __restrict__ sums, float* dx,
-             size_t total, int c, int hw, float count, int training, int accumulate, const float* __restrict__ count_dev) {
+             size_t total, int c, int hw, float count, int training, int accumulate, const float* __restrict__ count_dev,
+             const float* __restrict__ mean /* null: xhat is xhat; else it is x */) {
   NRS_PDL_PROLOGUE();
   if (count_dev) count = *count_dev;   // elements per channel over all processes
   const size_t stride = (size_t)gridDim.x * blockDim.x;
@@ -235,6 +247,10 @@ bn_dx_kernel(const float* __restrict__ g, const float* __restrict__ xhat, const 
       float4 vg = reinterpret_cast<const float4*>(g)[i];
       float4 vh = make_float4(0.f, 0.f, 0.f, 0.f);
       if (training || RELU) vh = reinterpret_cast<const float4*>(xhat)[i];
+      if (mean) {
+        const float mu = mean[ch];
+        vh = make_float4((vh.x - mu) * is, (vh.y - mu) * is, (vh.z - mu) * is, (vh.w - mu) * is);
+      }
       if (RELU) {
         const float be = beta[ch];
         vg.x = fmaf(ga, vh.x, be) > 0.0f ? vg.x : 0.0f;
@@ -262,18 +278,102 @@ bn_dx_kernel(const float* __restrict__ g, const float* __restrict__ xhat, const 
     for (size_t i = tid; i < total; i += stride) {
       const int ch = (int)((i / hw) % c);
       const float ga = gamma[ch], is = istd[ch];
-      float gi = g[i];
-      if (RELU) gi = fmaf(ga, xhat[i], beta[ch]) > 0.0f ? gi : 0.0f;
+      float gi = g[i], h = training || RELU ? xhat[i] : 0.0f;
+      if (mean) h = (h - mean[ch]) * is;
+      if (RELU) gi = fmaf(ga, h, beta[ch]) > 0.0f ? gi : 0.0f;
       float r;
       if (training) {
         const float2 sm = sums[ch];
-        r = is * (gi * ga - ga * sm.x / count - xhat[i] * (ga * sm.y / count));
+        r = is * (gi * ga - ga * sm.x / count - h * (ga * sm.y / count));
       } else {
         r = gi * ga * is;
       }
       dx[i] = accumulate ? dx[i] + r : r;
     }
   }
+}
+
+// The normalise pass with the NHWC planes of y (no xhat).
+template <bool SPLIT, bool RELU>
+__global__ void __launch_bounds__(kThreads)
+bn_normalize_planes_kernel(const float* __restrict__ x, const float* __restrict__ mean, const float* __restrict__ istd,
+                           const float* __restrict__ gamma, const float* __restrict__ beta, float* __restrict__ y,
+                           float* __restrict__ hi, float* __restrict__ lo, const img::Grid g) {
+  NRS_PDL_PROLOGUE();
+  __shared__ img::Tile tile;
+  const uint32_t p0 = blockIdx.x * img::kTilePx;
+  const int c0 = blockIdx.y * img::kTileCh, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const img::Pixels px(g, p0);
+  float v[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const int c = c0 + warp + 8 * (i >> 2);
+    v[i] = (c < g.c && px.live[i & 3]) ? x[px.at[i & 3] + (size_t)c * g.hw] : 0.0f;
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int cl = warp + 8 * k, c = c0 + cl;
+    const bool ok = c < g.c;
+    const float m = ok ? mean[c] : 0.0f, is = ok ? istd[c] : 0.0f, ga = ok ? gamma[c] : 0.0f, be = ok ? beta[c] : 0.0f;
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      const float h = (v[4 * k + s] - m) * is;
+      float o = fmaf(ga, h, be);
+      if (RELU) o = fmaxf(o, 0.0f);
+      if (ok && px.live[s]) y[px.at[s] + (size_t)c * g.hw] = o;
+      tile[cl][s * 32 + lane] = o;
+    }
+  }
+  __syncthreads();
+  img::tile_to_planes<SPLIT>(tile, g, p0, c0, hi, lo);
+}
+
+// dx (overwritten) with its NHWC planes, and chan_partial[tile of 128 pixels][c], its sums over the tile.
+template <bool SPLIT, bool RELU>
+__global__ void __launch_bounds__(kThreads)
+bn_dx_planes_kernel(const float* __restrict__ gr, const float* __restrict__ x, const float* __restrict__ mean,
+                    const float* __restrict__ istd, const float* __restrict__ gamma, const float* __restrict__ beta,
+                    const float2* __restrict__ sums, float* __restrict__ dx, float* __restrict__ hi, float* __restrict__ lo,
+                    float* __restrict__ chan_partial, const img::Grid g, float count, int training, const float* __restrict__ count_dev) {
+  NRS_PDL_PROLOGUE();
+  __shared__ img::Tile tile;
+  if (count_dev) count = *count_dev;
+  const uint32_t p0 = blockIdx.x * img::kTilePx;
+  const int c0 = blockIdx.y * img::kTileCh, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const img::Pixels px(g, p0);
+  float vg[16], vx[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const int c = c0 + warp + 8 * (i >> 2);
+    const bool ok = c < g.c && px.live[i & 3];
+    const size_t at = px.at[i & 3] + (size_t)c * g.hw;
+    vg[i] = ok ? gr[at] : 0.0f;
+    vx[i] = ok ? x[at] : 0.0f;
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int cl = warp + 8 * k, c = c0 + cl;
+    const bool ok = c < g.c;
+    const float m = ok ? mean[c] : 0.0f, is = ok ? istd[c] : 0.0f, ga = ok ? gamma[c] : 0.0f, be = ok && RELU ? beta[c] : 0.0f;
+    const float2 sm = ok && training ? sums[c] : make_float2(0.0f, 0.0f);
+    const float m1 = ga * sm.x / count, m2 = ga * sm.y / count;
+    float total = 0.0f;
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      const float h = (vx[4 * k + s] - m) * is;
+      float gi = vg[4 * k + s];
+      if (RELU) gi = fmaf(ga, h, be) > 0.0f ? gi : 0.0f;
+      const bool live = ok && px.live[s];
+      const float r = !live ? 0.0f : training ? is * (gi * ga - m1 - h * m2) : gi * ga * is;
+      if (live) dx[px.at[s] + (size_t)c * g.hw] = r;
+      tile[cl][s * 32 + lane] = r;
+      total += r;
+    }
+    total = wsum(total);
+    if (lane == 0 && ok) chan_partial[(size_t)blockIdx.x * g.c + c] = total;
+  }
+  __syncthreads();
+  img::tile_to_planes<SPLIT>(tile, g, p0, c0, hi, lo);
 }
 
 // Statistics shared by several processes: the splits of this process folded in order into out[ch], the
@@ -311,13 +411,14 @@ int plan_splits(const nrs_ctx* ctx, int n, int c, int hw) {
 
 template <bool FWD, bool RELU>
 int launch_pair(nrs_ctx* ctx, const float* a, const float* b, float2* partial, int n, int c, int hw, int splits,
-                const float* gamma, const float* beta, const float* pivot = nullptr) {
+                const float* gamma, const float* beta, const float* pivot = nullptr, const float* mean = nullptr,
+                const float* istd = nullptr) {
   if (hw == 1) {
     NRS_PDL_LAUNCH((bn_pair_cols_kernel<FWD, RELU>), dim3((c + 31) / 32, splits), kThreads, 0, ctx->stream, a, b, partial, n, c,
-                   splits, gamma, beta, pivot);
+                   splits, gamma, beta, pivot, mean, istd);
   } else {
     NRS_PDL_LAUNCH((bn_pair_planes_kernel<FWD, RELU>), dim3(c, splits), kThreads, 0, ctx->stream, a, b, partial, n, c, hw,
-                   splits, gamma, beta, pivot);
+                   splits, gamma, beta, pivot, mean, istd);
   }
   NRS_LAUNCHED(ctx);
   return NRS_OK;
@@ -340,7 +441,7 @@ namespace {
 
 int bn_forward(nrs_ctx* ctx, const char* who, const float* x, const float* gamma, const float* beta, float* running_mean,
                float* running_var, float* y, float* xhat, float* istd, int n, int c, int hw, float eps, float momentum,
-               int training, bool relu) {
+               int training, bool relu, float* mean_out = nullptr, float* hi = nullptr, float* lo = nullptr) {
   NRS_REQUIRE_CTX(ctx);
   NRS_REQUIRE(ctx, check_dims(n, c, hw), NRS_ERR_SHAPE, "%s: bad shape [%d,%d,%d]", who, n, c, hw);
   NRS_REQUIRE(ctx, x && gamma && beta && running_mean && running_var && y && istd, NRS_ERR_ARG, "%s: null tensor", who);
@@ -353,8 +454,9 @@ int bn_forward(nrs_ctx* ctx, const char* who, const float* x, const float* gamma
   const int st = nrs_workspace(ctx, ((size_t)splits * c * 2 + c + (size_t)c * 2 + 4) * sizeof(float), &ws);
   if (st != NRS_OK) return st;
   float2* partial = (float2*)ws;
-  float* mean = (float*)(partial + (size_t)splits * c);
-  float2* summed = (float2*)(mean + c + (c & 1));   // 8-byte aligned; [c] pairs + the count
+  float* mean_ws = (float*)(partial + (size_t)splits * c);
+  float* mean = mean_out ? mean_out : mean_ws;
+  float2* summed = (float2*)(mean_ws + c + (c & 1));   // 8-byte aligned; [c] pairs + the count
   float* count_slot = (float*)(summed + c);
   if (training) {
     const int sp = launch_pair<true, false>(ctx, x, nullptr, partial, n, c, hw, splits, nullptr, nullptr,
@@ -376,6 +478,17 @@ int bn_forward(nrs_ctx* ctx, const char* who, const float* x, const float* gamma
                    (const float*)nullptr, (const float*)nullptr);
   }
   NRS_LAUNCHED(ctx);
+  if (hi) {
+    const img::Grid grid(n, c, hw);
+#define NRS_BN_NORM(S, R)                                                                                               \
+  NRS_PDL_LAUNCH((bn_normalize_planes_kernel<S, R>), grid.blocks(), kThreads, 0, ctx->stream, x, (const float*)mean, (const float*)istd, \
+                 gamma, beta, y, hi, lo, grid)
+    if (lo) { if (relu) NRS_BN_NORM(true, true); else NRS_BN_NORM(true, false); }
+    else { if (relu) NRS_BN_NORM(false, true); else NRS_BN_NORM(false, false); }
+#undef NRS_BN_NORM
+    NRS_LAUNCHED(ctx);
+    return NRS_OK;
+  }
   const size_t total = (size_t)n * c * hw;
   const bool vec = (hw & 3) == 0 && ((uintptr_t)x & 15) == 0 && ((uintptr_t)y & 15) == 0 && ((uintptr_t)xhat & 15) == 0;
   const unsigned blocks = ew_blocks(ctx, vec ? total / 4 : total);
@@ -391,7 +504,8 @@ int bn_forward(nrs_ctx* ctx, const char* who, const float* x, const float* gamma
 
 int bn_backward(nrs_ctx* ctx, const char* who, const float* g, const float* xhat, const float* istd, const float* gamma,
                 const float* beta, float* dx, float* dgamma, float* dbeta, int n, int c, int hw, int training,
-                int accumulate_dx, int accumulate_params, bool relu) {
+                int accumulate_dx, int accumulate_params, bool relu, const float* mean = nullptr /* xhat is x then */,
+                float* hi = nullptr, float* lo = nullptr, float* chan_partial = nullptr) {
   NRS_REQUIRE_CTX(ctx);
   NRS_REQUIRE(ctx, check_dims(n, c, hw), NRS_ERR_SHAPE, "%s: bad shape [%d,%d,%d]", who, n, c, hw);
   NRS_REQUIRE(ctx, (dgamma == nullptr) == (dbeta == nullptr), NRS_ERR_ARG, "%s: dgamma and dbeta must be given together", who);
@@ -410,8 +524,8 @@ int bn_backward(nrs_ctx* ctx, const char* who, const float* g, const float* xhat
   // process's own sums (they are summed across ranks with all other gradients)
   const bool shared = training && dx && ctx->stat_sync.all_reduce_sum != nullptr;
   if (need_sums) {
-    const int sp = relu ? launch_pair<false, true>(ctx, g, xhat, partial, n, c, hw, splits, gamma, beta)
-                        : launch_pair<false, false>(ctx, g, xhat, partial, n, c, hw, splits, nullptr, nullptr);
+    const int sp = relu ? launch_pair<false, true>(ctx, g, xhat, partial, n, c, hw, splits, gamma, beta, nullptr, mean, istd)
+                        : launch_pair<false, false>(ctx, g, xhat, partial, n, c, hw, splits, nullptr, nullptr, nullptr, mean, istd);
     if (sp != NRS_OK) return sp;
     NRS_PDL_LAUNCH(bn_grad_finish_kernel, nrs_blocks(c, 128), 128, 0, ctx->stream, (const float2*)partial, sums, dgamma, dbeta,
                    c, splits, accumulate_params);
@@ -424,13 +538,24 @@ int bn_backward(nrs_ctx* ctx, const char* who, const float* g, const float* xhat
     const int sr = ctx->stat_sync.all_reduce_sum(ctx->stat_sync.user, (float*)sums, (size_t)c * 2 + 1);
     if (sr != NRS_OK) return sr;
   }
-  const size_t total = (size_t)n * c * hw;
   const float count = (float)((double)n * hw);
+  if (hi) {
+    const img::Grid grid(n, c, hw);
+#define NRS_BN_DX(S, R)                                                                                                  \
+  NRS_PDL_LAUNCH((bn_dx_planes_kernel<S, R>), grid.blocks(), kThreads, 0, ctx->stream, g, xhat, mean, istd, gamma, beta,  \
+                 (const float2*)sums, dx, hi, lo, chan_partial, grid, count, training, shared ? (const float*)count_slot : (const float*)nullptr)
+    if (lo) { if (relu) NRS_BN_DX(true, true); else NRS_BN_DX(true, false); }
+    else { if (relu) NRS_BN_DX(false, true); else NRS_BN_DX(false, false); }
+#undef NRS_BN_DX
+    NRS_LAUNCHED(ctx);
+    return NRS_OK;
+  }
+  const size_t total = (size_t)n * c * hw;
   const bool vec = (hw & 3) == 0 && ((uintptr_t)g & 15) == 0 && ((uintptr_t)xhat & 15) == 0 && ((uintptr_t)dx & 15) == 0;
   const unsigned blocks = ew_blocks(ctx, vec ? total / 4 : total);
 #define NRS_BN_DX(V, R)                                                                                              \
   NRS_PDL_LAUNCH((bn_dx_kernel<V, R>), blocks, kThreads, 0, ctx->stream, g, xhat, istd, gamma, beta, (const float2*)sums, dx, \
-                 total, c, hw, count, training, accumulate_dx, shared ? (const float*)count_slot : (const float*)nullptr)
+                 total, c, hw, count, training, accumulate_dx, shared ? (const float*)count_slot : (const float*)nullptr, mean)
   if (vec) { if (relu) NRS_BN_DX(true, true); else NRS_BN_DX(true, false); }
   else { if (relu) NRS_BN_DX(false, true); else NRS_BN_DX(false, false); }
 #undef NRS_BN_DX
@@ -474,3 +599,19 @@ int nrs_batchnorm_act_bwd(nrs_ctx* ctx, const float* g, const float* xhat, const
   return bn_backward(ctx, "nrs_batchnorm_act_bwd", g, xhat, istd, gamma, beta, dx, dgamma, dbeta, n, c, hw, training,
                      accumulate_dx, accumulate_params, act == NRS_ACT_RELU);
 }
+
+int nrs_batchnorm_fwd_saving_mean(nrs_ctx* ctx, const float* x, const float* gamma, const float* beta, float* running_mean, float* running_var,
+                                  float* y, float* mean, float* istd, int n, int c, int hw, float eps, float momentum, int training, int act,
+                                  float* hi, float* lo) {
+  return bn_forward(ctx, "batchnorm", x, gamma, beta, running_mean, running_var, y, nullptr, istd, n, c, hw, eps, momentum, training,
+                    act == NRS_ACT_RELU, mean, hi, lo);
+}
+
+int nrs_batchnorm_bwd_from_x(nrs_ctx* ctx, const float* g, const float* x, const float* mean, const float* istd, const float* gamma,
+                             const float* beta, float* dx, float* dgamma, float* dbeta, int n, int c, int hw, int training, int accumulate_dx,
+                             int accumulate_params, int act, float* hi, float* lo, float* chan_partial) {
+  return bn_backward(ctx, "batchnorm backward", g, x, istd, gamma, beta, dx, dgamma, dbeta, n, c, hw, training, accumulate_dx, accumulate_params,
+                     act == NRS_ACT_RELU, mean, hi, lo, chan_partial);
+}
+
+int nrs_batchnorm_tiles(int n, int hw) { return (int)(((size_t)n * hw + img::kTilePx - 1) / img::kTilePx); }

@@ -253,7 +253,13 @@ void to_host(const NodeP& n, float* host_out) {
 void set_grad(const NodeP& n, const float* host) {
   require_gpu(n, "set_grad: node");
   Node* r = grad_root(n.get());
-  if (!r->grad) r->grad = dalloc(r->ctx, r->len());
+  (void)grad_target(n);   // what a producer derived from the old gradient is stale
+  if (r->gplanes_hi) {
+    n->ctx->plane_hints.erase(r->grad);
+    nrs_free(n->ctx, r->gplanes_hi);
+    if (r->gplanes_lo) nrs_free(n->ctx, r->gplanes_lo);
+    r->gplanes_hi = r->gplanes_lo = nullptr;
+  }
   check(n->ctx, nrs_h2d(n->ctx, r->grad, host, r->len() * sizeof(float)));
   check(n->ctx, nrs_sync(n->ctx));  // the caller's buffer may go away
   r->grad_valid = true;
@@ -737,7 +743,7 @@ NodeP conv2d_act(const NodeP& x, const NodeP& w, const NodeP& b, size_t stride, 
   // every tensor-core backward pass reads dy planes (the producers of a gradient write them with a pixel stride
   // of the channel count: whole groups of eight only)
   const bool dy_planes = s <= 8 && !(patches && (long)n * oh * ow < kNrsPatchMinPixels);
-  out->wants_grad_planes = act == NRS_ACT_RELU && dy_planes && co % 8 == 0;
+  out->wants_grad_planes = (act == NRS_ACT_RELU || act == NRS_ACT_NONE) && dy_planes && co % 8 == 0;
   out->backward_fn = [self, x, w, b, n, ci, h, wd, co, kh, kw, s, p, act, dy_planes]() {
     nrs_ctx* ctx = self->ctx;
     const float* dy = grad_in(self);
@@ -1009,7 +1015,7 @@ NodeP layernorm_residual(const NodeP& x, const NodeP& residual, const NodeP& gam
 // nodes owned by the caller and updated in place in training mode.
 NodeP batchnorm_nd(const NodeP& x, const NodeP& gamma, const NodeP& beta, const NodeP& running_mean,
                    const NodeP& running_var, float momentum, float eps, bool training, size_t want_dims,
-                   const char* what, int act = NRS_ACT_NONE) {
+                   const char* what, int act = NRS_ACT_NONE, bool emit_planes = false) {
   const std::string w(what);
   require_gpu(x, (w + ": input").c_str());
   require_gpu(gamma, (w + ": gamma").c_str());
@@ -1026,14 +1032,24 @@ NodeP batchnorm_nd(const NodeP& x, const NodeP& gamma, const NodeP& beta, const 
   if ((int)gamma->len() != c || (int)beta->len() != c || (int)running_mean->len() != c || (int)running_var->len() != c)
     fail(NRS_ERR_SHAPE, (w + ": gamma/beta/running statistics length mismatch").c_str());
   NodeP out = make_out(ctx, x->shape, {x, gamma, beta});
-  float* xhat = dalloc(ctx, x->len());
+  float* mean = dalloc(ctx, (size_t)c);
   float* istd = dalloc(ctx, (size_t)c);
-  out->saved.push_back(xhat);
+  out->saved.push_back(mean);
   out->saved.push_back(istd);
-  check(ctx, nrs_batchnorm_act_fwd(ctx, x->data, gamma->data, beta->data, running_mean->data, running_var->data, out->data,
-                                   xhat, istd, n, c, hw, eps, momentum, training ? 1 : 0, act));
+  // the caller knows that a tensor-core convolution reads the output: its planes come out of the same pass
+  const bool planes = x->shape.size() == 4 && c % 8 == 0 && (size_t)n * hw <= 0x7fffffffu && planes_possible(ctx);
+  float *hi = nullptr, *lo = nullptr;
+  if (planes && emit_planes) {
+    hi = dalloc(ctx, out->len());
+    if (ctx->math_mode == NRS_MATH_3XTF32) lo = dalloc(ctx, out->len());
+    out->planes_hi = hi;   // (the node's from here on, whatever happens)
+    out->planes_lo = lo;
+  }
+  check(ctx, nrs_batchnorm_fwd_saving_mean(ctx, x->data, gamma->data, beta->data, running_mean->data, running_var->data, out->data, mean,
+                                           istd, n, c, hw, eps, momentum, training ? 1 : 0, act, hi, lo));
+  if (hi) ctx->plane_hints[out->data] = NrsPlanes{hi, lo, lo ? 1 : 0};
   Node* self = out.get();
-  out->backward_fn = [self, x, gamma, beta, xhat, istd, n, c, hw, training, act]() {
+  out->backward_fn = [self, x, gamma, beta, mean, istd, n, c, hw, training, act, planes]() {
     nrs_ctx* ctx = self->ctx;
     const float* g = grad_in(self);
     float *dg = nullptr, *db = nullptr;
@@ -1051,13 +1067,26 @@ NodeP batchnorm_nd(const NodeP& x, const NodeP& gamma, const NodeP& beta, const 
     }
     float* dx = nullptr;
     int acc_x = 0;
+    float *phi = nullptr, *plo = nullptr, *partial = nullptr;
+    Node* xr = x.get();
     if (x->requires_grad) {
+      // x is the output of a convolution and this is all of its gradient: the convolution's backward pass finds the
+      // planes and the channel sums of it ready
+      const bool emit = planes && xr->wants_grad_planes && !xr->relu_folded && !xr->view_of && !xr->grad_valid && !xr->grad_premasked &&
+                        !xr->gplanes_hi && planes_possible(ctx);
       GradTarget t = grad_target(x);
       dx = t.ptr;
       acc_x = t.accumulate;
+      if (emit) {
+        xr->gplanes_hi = phi = dalloc(ctx, xr->len());
+        if (ctx->math_mode == NRS_MATH_3XTF32) xr->gplanes_lo = plo = dalloc(ctx, xr->len());
+        xr->gchan_rows = nrs_batchnorm_tiles(n, hw);
+        xr->gchan_partial = partial = dalloc(ctx, (size_t)xr->gchan_rows * c);
+        xr->grad_premasked = true;   // there is no mask
+      }
     }
-    check(ctx, nrs_batchnorm_act_bwd(ctx, g, xhat, istd, gamma->data, beta->data, dx, dg, db, n, c, hw, training ? 1 : 0,
-                                     acc_x, acc_p, act));
+    check(ctx, nrs_batchnorm_bwd_from_x(ctx, g, x->data, mean, istd, gamma->data, beta->data, dx, dg, db, n, c, hw, training ? 1 : 0,
+                                        acc_x, acc_p, act, phi, plo, partial));
   };
   return out;
 }
@@ -1075,8 +1104,8 @@ NodeP batchnorm2d(const NodeP& x, const NodeP& gamma, const NodeP& beta, const N
 // batchnorm / batchnorm2d (by the input's rank) followed by `act` (NRS_ACT_NONE or NRS_ACT_RELU) in the same
 // two passes: the conv -> batchnorm2d -> relu unit of examples/cifar_cuda.rs:44-48 without the ReLU's own passes.
 NodeP batchnorm_act(const NodeP& x, const NodeP& gamma, const NodeP& beta, const NodeP& running_mean,
-                    const NodeP& running_var, float momentum, float eps, bool training, int act) {
-  return batchnorm_nd(x, gamma, beta, running_mean, running_var, momentum, eps, training, 0, "cuda bn+act", act);
+                    const NodeP& running_var, float momentum, float eps, bool training, int act, bool emit_planes) {
+  return batchnorm_nd(x, gamma, beta, running_mean, running_var, momentum, eps, training, 0, "cuda bn+act", act, emit_planes);
 }
 
 // dropout (src/cuda/nn/dropout.rs:31-84) and dropout2d (src/cuda/nn/dropout2d.rs:37-end): evaluation returns

@@ -59,7 +59,8 @@ struct Node {
   float* patches_lo = nullptr;
   // Set on the output of a convolution that folded a ReLU into its epilogue.  A max-pool
   // directly above may then hand back a gradient that already carries the ReLU mask
-  // (grad_premasked), together with its NHWC planes (gplanes_*, freed with the node).
+  // (grad_premasked), together with its NHWC planes (gplanes_*, freed with the node).  A batch normalisation above
+  // a convolution without an activation hands back its gradient the same way (there is no mask then).
   bool relu_folded = false, wants_grad_planes = false, grad_premasked = false;
   float* gplanes_hi = nullptr;
   float* gplanes_lo = nullptr;
@@ -156,7 +157,7 @@ NodeP batchnorm2d(const NodeP& x, const NodeP& gamma, const NodeP& beta, const N
                   const NodeP& running_var, float momentum, float eps, bool training);
 // either of the two followed by a fused activation (NRS_ACT_NONE / NRS_ACT_RELU); rank 2 or 4 input
 NodeP batchnorm_act(const NodeP& x, const NodeP& gamma, const NodeP& beta, const NodeP& running_mean,
-                    const NodeP& running_var, float momentum, float eps, bool training, int act);
+                    const NodeP& running_var, float momentum, float eps, bool training, int act, bool emit_planes = false);
 // dropout.rs / dropout2d.rs: evaluation returns `x` itself; `mask` == nullptr draws the mask on the device
 NodeP dropout(const NodeP& x, float p, bool training, const NodeP& mask = nullptr);
 NodeP dropout2d(const NodeP& x, float p, bool training, const NodeP& mask = nullptr);

@@ -287,8 +287,12 @@ NodeP forward(nrs_trainer* t, const NodeP& x, const int32_t* ids_dev, size_t bat
       case NRS_LAYER_FLATTEN: h = nrs::cuda::flatten(h); break;
       case NRS_LAYER_BATCHNORM:
         // a ReLU behind the layer rides in its two passes (relu_next is only set when fusing is on)
-        h = nrs::cuda::batchnorm_act(h, t->params[pi], t->params[pi + 1], t->buffers[bi], t->buffers[bi + 1],
-                                     t->bn_momentum, t->bn_eps, t->training, relu_next ? NRS_ACT_RELU : NRS_ACT_NONE);
+        {
+          const size_t nx = li + (relu_next ? 2 : 1);
+          const bool conv_reads = nx < t->layers.size() && t->layers[nx].kind == NRS_LAYER_CONV && t->layers[nx].d <= 8;
+          h = nrs::cuda::batchnorm_act(h, t->params[pi], t->params[pi + 1], t->buffers[bi], t->buffers[bi + 1], t->bn_momentum, t->bn_eps,
+                                       t->training, relu_next ? NRS_ACT_RELU : NRS_ACT_NONE, conv_reads);
+        }
         pi += 2;
         bi += 2;
         if (relu_next) ++li;

@@ -260,6 +260,17 @@ inline const NrsPlanes* nrs_planes_find(nrs_ctx* ctx, const void* src, bool spli
 // Reads and clears the device error word (the stream must be idle); NRS_ERR_TIMEOUT if a kernel gave up a wait.
 int nrs_check_device_error(nrs_ctx* ctx);
 
+// Batch normalisation for the graph (batchnorm.cu): saves the means instead of xhat, and takes x back for the backward
+// pass.  hi / lo (optional, 4-D tensors with c a multiple of 8): NHWC planes of y, or of dx, which is then overwritten
+// and leaves chan_partial[nrs_batchnorm_tiles(n, hw)][c], its channel sums.
+int nrs_batchnorm_fwd_saving_mean(nrs_ctx* ctx, const float* x, const float* gamma, const float* beta, float* running_mean, float* running_var,
+                                  float* y, float* mean, float* istd, int n, int c, int hw, float eps, float momentum, int training, int act,
+                                  float* hi, float* lo);
+int nrs_batchnorm_bwd_from_x(nrs_ctx* ctx, const float* g, const float* x, const float* mean, const float* istd, const float* gamma,
+                             const float* beta, float* dx, float* dgamma, float* dbeta, int n, int c, int hw, int training, int accumulate_dx,
+                             int accumulate_params, int act, float* hi, float* lo, float* chan_partial);
+int nrs_batchnorm_tiles(int n, int hw);
+
 // Batched weight staging (weight_set.cu).  build: allocates planes for the described weights in the
 // context's current math mode (nothing in FP32 mode) and replaces any earlier set; refresh: one launch
 // that stages them all from the weights' current values; find: the planes of (w, form) when the set is

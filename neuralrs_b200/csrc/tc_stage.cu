@@ -5,6 +5,7 @@
 // TF32: the tensor core truncates its inputs, and truncation's systematic bias
 // compounds through a deep network where rounding's does not.  Transposed sources ([K][rows], e.g. NCHW images seen as
 // [C][H*W]) go through 32x32 shared-memory tiles so both sides stay coalesced.
+#include "image_tile.cuh"
 #include "tc_mainloop.cuh"
 
 namespace {
@@ -77,39 +78,25 @@ stage_transpose_kernel(const float* __restrict__ src, float* __restrict__ hi, fl
   }
 }
 
-// NCHW [n][c][hw] -> NHWC planes [n][hw][ld].  A block takes 32 channels x 128 pixels of an image: 16 independent
-// 128-byte row segments in flight per warp on the way in, full 128-byte lines (32 channels of a pixel, 128-bit
-// stores) on the way out.  HBM-bound: 4 B read and 4 or 8 B written per element.
-constexpr int kStagePx = 128;
+// NCHW [n][c][hw] -> NHWC planes [n][hw][ld].  HBM-bound: 4 B read and 4 or 8 B written per element.
 template <bool SPLIT>
 __global__ void __launch_bounds__(256)
-stage_image_kernel(const float* __restrict__ src, float* __restrict__ hi, float* __restrict__ lo, int c_n, int hw, int ld) {
+stage_image_kernel(const float* __restrict__ src, float* __restrict__ hi, float* __restrict__ lo, const img::Grid g) {
   NRS_PDL_PROLOGUE();
-  __shared__ float tile[32][kStagePx + 1];
-  const int p0 = blockIdx.x * kStagePx, c0 = blockIdx.y * 32;
-  const size_t img = blockIdx.z;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  __shared__ img::Tile tile;
+  const uint32_t p0 = blockIdx.x * img::kTilePx;
+  const int c0 = blockIdx.y * img::kTileCh, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const img::Pixels px(g, p0);
   float v[16];
 #pragma unroll
-  for (int i = 0; i < 16; ++i) {   // warp w: channels w, w+8, ...; four pixel segments each
-    const int c = c0 + warp + 8 * (i >> 2), px = p0 + (i & 3) * 32 + lane;
-    v[i] = (c < c_n && px < hw) ? src[(img * c_n + c) * hw + px] : 0.0f;
+  for (int i = 0; i < 16; ++i) {
+    const int c = c0 + warp + 8 * (i >> 2);
+    v[i] = (c < g.c && px.live[i & 3]) ? src[px.at[i & 3] + (size_t)c * g.hw] : 0.0f;
   }
 #pragma unroll
   for (int i = 0; i < 16; ++i) tile[warp + 8 * (i >> 2)][(i & 3) * 32 + lane] = v[i];
   __syncthreads();
-  const int cq = (threadIdx.x & 7) * 4;
-  if (c0 + cq >= ld) return;
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const int pl = k * 32 + (threadIdx.x >> 3);
-    if (p0 + pl >= hw) break;
-    const float4 f = make_float4(tile[cq][pl], tile[cq + 1][pl], tile[cq + 2][pl], tile[cq + 3][pl]);
-    const float4 h = make_float4(tc::tf32_rn(f.x), tc::tf32_rn(f.y), tc::tf32_rn(f.z), tc::tf32_rn(f.w));
-    const size_t o = (img * hw + p0 + pl) * ld + c0 + cq;
-    *reinterpret_cast<float4*>(hi + o) = h;
-    if (SPLIT) *reinterpret_cast<float4*>(lo + o) = make_float4(f.x - h.x, f.y - h.y, f.z - h.z, f.w - h.w);
-  }
+  img::tile_to_planes<SPLIT>(tile, g, p0, c0, hi, lo);
 }
 
 template <bool SPLIT>
@@ -382,10 +369,10 @@ int nrs_tc_stage_image(nrs_ctx* ctx, const float* src, float* hi, float* lo, int
   if (n <= 0 || c <= 0 || hw <= 0) return NRS_OK;
   const int ld = nrs_plane_ld(c);
   if (hw == 1) return nrs_tc_stage(ctx, src, hi, lo, n, c, ld, 1, 0, 0, false);   // already pixel-major: split only
-  dim3 grid((unsigned)((hw + kStagePx - 1) / kStagePx), (unsigned)((ld + 31) / 32), (unsigned)n);
-  if (grid.y > 65535 || grid.z > 65535) return NRS_ERR_UNSUPPORTED;
-  if (lo) NRS_PDL_LAUNCH((stage_image_kernel<true>), grid, 256, 0, ctx->stream, src, hi, lo, c, hw, ld);
-  else NRS_PDL_LAUNCH((stage_image_kernel<false>), grid, 256, 0, ctx->stream, src, hi, nullptr, c, hw, ld);
+  if ((size_t)n * hw > 0x7fffffffu) return NRS_ERR_UNSUPPORTED;
+  const img::Grid g(n, c, hw);
+  if (lo) NRS_PDL_LAUNCH((stage_image_kernel<true>), g.blocks(), 256, 0, ctx->stream, src, hi, lo, g);
+  else NRS_PDL_LAUNCH((stage_image_kernel<false>), g.blocks(), 256, 0, ctx->stream, src, hi, nullptr, g);
   NRS_LAUNCHED(ctx);
   return NRS_OK;
 }
