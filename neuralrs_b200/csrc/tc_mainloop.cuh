@@ -61,7 +61,9 @@ template <int BN, int NPLANES, int EMIT_BYTES, bool PAIR>
 struct SmemLayout {
   static constexpr int kATile = BM * BK * 4;   // 16 KB
   static constexpr int kBTile = BN / (PAIR ? 2 : 1) * BK * 4;   // this CTA's rows of B
-  static constexpr int kStage = NPLANES * (kATile + kBTile);   // [A_hi][B_hi][B_lo][A_lo]
+  static constexpr int kSlice = NPLANES * (kATile + kBTile);   // [A_hi][B_hi][B_lo][A_lo]
+  static constexpr int kSlices = NPLANES == 1 ? 2 : 1;         // K-slices per ring slot (see above)
+  static constexpr int kStage = kSlices * kSlice;
   static constexpr int kExtra = EMIT_BYTES /*plane staging tile*/ + 1024 /*align*/ + 256 /*barriers*/;
   static constexpr int kRing = 227 * 1024 - kExtra;
   static constexpr int kStages = kRing / kStage >= 8 ? 8 : kRing / kStage;
@@ -189,7 +191,7 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
   if (warp == 0) {
     // ---------------- TMA producer
     // Both CTAs of a pair count their bytes on the barrier of rank 0, which expects the sum.
-    const uint32_t stage_bytes = (uint32_t)(PAIR ? 2 : 1) * NPLANES * (pol.a_slice_bytes() + (uint32_t)L::kBTile);
+    const uint32_t slice_bytes = (uint32_t)(PAIR ? 2 : 1) * NPLANES * (pol.a_slice_bytes() + (uint32_t)L::kBTile);
     uint32_t s = 0, ph = 0, issued = 0;   // ring slot, its use's parity, slices so far: run on across tiles
     bool ok = true;
     for (long t = t_first; t < tmap.total && ok; t += t_step) {
@@ -204,22 +206,31 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
       // Where the K-slices of this tile lie, stepped along instead of recomputed (the divisions of a recomputation per
       // slice and plane made the producer the bottleneck: 58 -> 72 us on a 64-channel convolution).
       typename Policy::Cursor cur = pol.cursor(tile_m, batch, kb_begin);
-      for (int kb = kb_begin; kb < kb_end; ++kb) {
+      for (int kb = kb_begin; kb < kb_end; kb += L::kSlices) {
         if (!mbar_wait_warp(&empty_bar[s], ph ^ 1u)) { ok = false; break; }
+        const bool two = L::kSlices == 2 && kb + 1 < kb_end;
         uint8_t* st = smem + s * L::kStage;
         uint32_t bar;
         if constexpr (PAIR) bar = cluster_addr(&full_bar[s], 0); else bar = smem_u32(&full_bar[s]);
-        if (elect_one()) {
-          if (rank == 0) mbar_expect_tx(&full_bar[s], stage_bytes);
-          pol.template load_a<PAIR>(st, &tm_a_hi, bar, cur);
-          pol.template load_b<BN, PAIR>(st + L::kATile, &tm_b_hi, bar, cur, n0);
+        auto bring = [&](uint8_t* dst) {
+          pol.template load_a<PAIR>(dst, &tm_a_hi, bar, cur);
+          pol.template load_b<BN, PAIR>(dst + L::kATile, &tm_b_hi, bar, cur, n0);
           if (NPLANES == 2) {
-            pol.template load_b<BN, PAIR>(st + L::kATile + L::kBTile, &tm_b_lo, bar, cur, n0);
-            pol.template load_a<PAIR>(st + L::kATile + 2 * L::kBTile, &tm_a_lo, bar, cur);
+            pol.template load_b<BN, PAIR>(dst + L::kATile + L::kBTile, &tm_b_lo, bar, cur, n0);
+            pol.template load_a<PAIR>(dst + L::kATile + 2 * L::kBTile, &tm_a_lo, bar, cur);
           }
+        };
+        const bool leader = elect_one();
+        if (leader) {
+          if (rank == 0) mbar_expect_tx(&full_bar[s], two ? 2 * slice_bytes : slice_bytes);
+          bring(st);
+        }
+        pol.advance(cur);
+        if (two) {
+          if (leader) bring(st + L::kSlice);
+          pol.advance(cur);
         }
         __syncwarp();
-        pol.advance(cur);
         ++issued;
         if (++s == (uint32_t)L::kStages) { s = 0; ph ^= 1u; }
       }
@@ -266,19 +277,24 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
         if (!(PAIR ? mbar_wait_warp_cluster(&acc_empty[buf], (use & 1u) ^ 1u) : mbar_wait_warp(&acc_empty[buf], (use & 1u) ^ 1u))) { ok = false; break; }
         tc_fence_after_sync();
         const uint32_t d = tmem_base + buf * (uint32_t)L::kAccCols;
-        for (int i = 0; i < nkb; ++i) {
+        for (int i = 0; i < nkb; i += L::kSlices) {
           // (No tcgen05 fence here: the mbarrier's complete_tx orders the TMA writes before the
           // UMMAs, and a fence would make the issuing thread wait out the UMMAs in flight.)
           if (!mbar_wait_warp(&full_bar[s], ph)) { ok = false; break; }
-          const uint32_t a_hi = smem_u32(smem + s * L::kStage);
-          const uint32_t b_hi = a_hi + L::kATile;                 // B_lo follows B_hi directly
-          const uint32_t a_lo = b_hi + 2 * L::kBTile;
+          const uint32_t slot = smem_u32(smem + s * L::kStage);
           if (elect_one()) {
 #pragma unroll
-            for (int k = 0; k < BK / 8; ++k) {
-              const uint64_t da_hi = desc(kAMn, a_hi, k), db_hi = desc(kBMn, b_hi, k);
-              umma_tf32<PAIR>(d, da_hi, db_hi, idesc_wide, (i | k) != 0);   // hi*hi | hi*lo
-              if (NPLANES == 2) umma_tf32<PAIR>(d + kNarrow, desc(kAMn, a_lo, k), db_hi, idesc_half, 1);   // + lo*hi
+            for (int sl = 0; sl < L::kSlices; ++sl) {
+              if (sl > 0 && i + sl >= nkb) break;
+              const uint32_t a_hi = slot + sl * L::kSlice;
+              const uint32_t b_hi = a_hi + L::kATile;                 // B_lo follows B_hi directly
+              const uint32_t a_lo = b_hi + 2 * L::kBTile;
+#pragma unroll
+              for (int k = 0; k < BK / 8; ++k) {
+                const uint64_t da_hi = desc(kAMn, a_hi, k), db_hi = desc(kBMn, b_hi, k);
+                umma_tf32<PAIR>(d, da_hi, db_hi, idesc_wide, (i | sl | k) != 0);   // hi*hi | hi*lo
+                if (NPLANES == 2) umma_tf32<PAIR>(d + kNarrow, desc(kAMn, a_lo, k), db_hi, idesc_half, 1);   // + lo*hi
+              }
             }
             umma_commit<PAIR>(&empty_bar[s]);  // slot reusable once these UMMAs have read it
           }
