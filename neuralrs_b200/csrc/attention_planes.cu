@@ -42,14 +42,14 @@ struct HeadPolicy {
   bool vec;            // rows start on 16 bytes
   // Causal products: kTiles: result tiles above the diagonal do not exist.  kUpTo: K-slices beyond the tile's last row
   // are zero.  kFrom: K-slices before the tile's first row are zero.
-  enum { kDense = 0, kTiles = 1, kUpTo = 2, kFrom = 3 };
+  enum { kDense = tc::kRaster, kTiles = tc::kTriangle, kUpTo = tc::kLastFirst, kFrom = tc::kFirstFirst };
   int causal;
   static constexpr bool kCanEmit = false, kMaySplit = false;
   static constexpr bool kAMnMajor = AMN, kBMnMajor = BMN;
-  static constexpr int kEpiWarps = 8;
+  static constexpr int kEpiWarps = 16;
+  int order() const { return causal; }   // the same numbers
 
   __device__ __forceinline__ bool clip(int tile_m, int tile_n, int bn, int* kb_begin, int* kb_end) const {
-    if (causal == kTiles) return tile_n * bn <= tile_m * tc::BM + tc::BM - 1;
     if (causal == kUpTo) *kb_end = min(*kb_end, (tile_m * tc::BM + tc::BM) / tc::BK);
     if (causal == kFrom) *kb_begin = tile_m * tc::BM / tc::BK;
     return *kb_begin < *kb_end;
@@ -81,13 +81,13 @@ struct HeadPolicy {
   }
   __device__ __forceinline__ int row(int, int, int) const { return 0; }
   __device__ __forceinline__ void store(int, int, int, int, float) const {}   // no K-split
-  __device__ __forceinline__ void epilogue(int tile_m, int batch, int r0, int n, float4 (&v)[8]) const {
+  __device__ __forceinline__ void epilogue(int tile_m, int batch, int r0, int n, float4 (&v)[4]) const {
     const int b = batch / heads, m0 = tile_m * tc::BM + r0, nn = N - n;
     const size_t at0 = (size_t)b * bs + (size_t)(batch - b * heads) * hs + (size_t)m0 * ldc + n;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      if (m0 + 4 * i >= M) continue;
-      const size_t at = at0 + (size_t)(4 * i) * ldc;
+    for (int i = 0; i < 4; ++i) {
+      if (m0 + 8 * i >= M) continue;
+      const size_t at = at0 + (size_t)(8 * i) * ldc;
       if (c) tc::store_guarded(c + at, v[i], nn, vec);
       if (hi) {
         const float4 h = make_float4(tc::tf32_rn(v[i].x), tc::tf32_rn(v[i].y), tc::tf32_rn(v[i].z), tc::tf32_rn(v[i].w));

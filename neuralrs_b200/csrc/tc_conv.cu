@@ -134,6 +134,7 @@ struct ConvPolicy {
   static constexpr bool kAMnMajor = false, kBMnMajor = false;
   static constexpr bool kMaySplit = true;
   __device__ __forceinline__ bool clip(int, int, int, int*, int*) const { return true; }
+  int order() const { return tc::kRaster; }
   static constexpr int kEpiWarps = 4;   // 250 registers per thread: no room for more
   __device__ __forceinline__ float* colsum_row(int tile_m, int q) const {
     return colsum_partial ? colsum_partial + ((size_t)tile_m * 4 + q) * n_ch_out : nullptr;

@@ -35,7 +35,10 @@ struct GemmPolicy {
   static constexpr bool kAMnMajor = MN, kBMnMajor = MN;
   static constexpr bool kMaySplit = true;
   __device__ __forceinline__ bool clip(int, int, int, int*, int*) const { return true; }
-  static constexpr int kEpiWarps = 8;   // the epilogue is latency (TMEM, loads, tanh), not registers: two warps per lane quarter
+  // The epilogue is latency (TMEM, loads, GELU at about 66 instructions a value): four warps per lane quarter.  With two,
+  // a 128 x 128 tile with GELU and three outputs took 27 thousand clocks, twice its main loop at K = 512.
+  static constexpr int kEpiWarps = 16;
+  int order() const { return tc::kRaster; }
 
   __device__ __forceinline__ uint32_t a_slice_bytes() const { return tc::BM * tc::BK * 4; }
   struct Cursor { int b_col, row, batch; };
@@ -72,68 +75,68 @@ struct GemmPolicy {
     if (x.lo) x.lo[at] = v - h;
   }
   __device__ __forceinline__ int row(int, int, int) const { return 0; }
-  // Eight row segments of a warp's 32 x 32 block: row r0 + 4*i of the tile, columns n..n+3 (see tc::rows_to_lines).
-  __device__ __forceinline__ void epilogue(int tile_m, int batch, int r0, int n, float4 (&v)[8]) const {
+  // Four row segments of a warp's 32 x 16 block: row r0 + 8*i of the tile, columns n..n+3 (see tc::rows_to_lines).
+  __device__ __forceinline__ void epilogue(int tile_m, int batch, int r0, int n, float4 (&v)[4]) const {
     const int m0 = tile_m * tc::BM + r0, nn = N - n;   // nn: how many of the four columns exist (four or more: all)
-    const size_t at0 = (size_t)batch * batch_stride + (size_t)m0 * N + n, step = (size_t)4 * N;
+    const size_t at0 = (size_t)batch * batch_stride + (size_t)m0 * N + n, step = (size_t)8 * N;
     if (bias) {
       const float4 b = tc::load_guarded(bias + n, nn, vec_ok);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) { v[i].x += b.x; v[i].y += b.y; v[i].z += b.z; v[i].w += b.w; }
+      for (int i = 0; i < 4; ++i) { v[i].x += b.x; v[i].y += b.y; v[i].z += b.z; v[i].w += b.w; }
     }
     if (x.pre) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
-        if (m0 + 4 * i < M) tc::store_guarded(x.pre + at0 + i * step, v[i], nn, vec_ok);
+      for (int i = 0; i < 4; ++i)
+        if (m0 + 8 * i < M) tc::store_guarded(x.pre + at0 + i * step, v[i], nn, vec_ok);
     }
     if (act != NRS_ACT_NONE) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
+      for (int i = 0; i < 4; ++i) {
         v[i].x = nrs_apply_act(v[i].x, act); v[i].y = nrs_apply_act(v[i].y, act);
         v[i].z = nrs_apply_act(v[i].z, act); v[i].w = nrs_apply_act(v[i].w, act);
       }
     }
     if (beta != 0.0f) {
-      float4 o[8];
+      float4 o[4];
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
-        o[i] = m0 + 4 * i < M ? tc::load_guarded(C + at0 + i * step, nn, vec_ok) : make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int i = 0; i < 4; ++i)
+        o[i] = m0 + 8 * i < M ? tc::load_guarded(C + at0 + i * step, nn, vec_ok) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) { v[i].x += beta * o[i].x; v[i].y += beta * o[i].y; v[i].z += beta * o[i].z; v[i].w += beta * o[i].w; }
+      for (int i = 0; i < 4; ++i) { v[i].x += beta * o[i].x; v[i].y += beta * o[i].y; v[i].z += beta * o[i].z; v[i].w += beta * o[i].w; }
     }
     if (!x.skip_c) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
-        if (m0 + 4 * i < M) tc::store_guarded(C + at0 + i * step, v[i], nn, vec_ok);
+      for (int i = 0; i < 4; ++i)
+        if (m0 + 8 * i < M) tc::store_guarded(C + at0 + i * step, v[i], nn, vec_ok);
     }
     if (x.dact != NRS_ACT_NONE) {
-      float4 s[8];
+      float4 s[4];
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
-        s[i] = m0 + 4 * i < M ? tc::load_guarded(x.dact_src + at0 + i * step, nn, vec_ok) : make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int i = 0; i < 4; ++i)
+        s[i] = m0 + 8 * i < M ? tc::load_guarded(x.dact_src + at0 + i * step, nn, vec_ok) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) { v[i].x *= dact(s[i].x); v[i].y *= dact(s[i].y); v[i].z *= dact(s[i].z); v[i].w *= dact(s[i].w); }
+      for (int i = 0; i < 4; ++i) { v[i].x *= dact(s[i].x); v[i].y *= dact(s[i].y); v[i].z *= dact(s[i].z); v[i].w *= dact(s[i].w); }
     }
     if (x.hi) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        if (m0 + 4 * i >= M) continue;
+      for (int i = 0; i < 4; ++i) {
+        if (m0 + 8 * i >= M) continue;
         const float4 h = make_float4(tc::tf32_rn(v[i].x), tc::tf32_rn(v[i].y), tc::tf32_rn(v[i].z), tc::tf32_rn(v[i].w));
         tc::store_guarded(x.hi + at0 + i * step, h, nn, vec_ok);
         if (x.lo) tc::store_guarded(x.lo + at0 + i * step, make_float4(v[i].x - h.x, v[i].y - h.y, v[i].z - h.z, v[i].w - h.w), nn, vec_ok);
       }
     }
-    if (x.colsum) {   // sum over the warp's 32 rows, in a fixed order; lanes 0..7 write four columns each
+    if (x.colsum) {   // sum over the warp's 32 rows, in a fixed order; lanes 0..3 write four columns each
       float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
-        if (m0 + 4 * i < M) { s.x += v[i].x; s.y += v[i].y; s.z += v[i].z; s.w += v[i].w; }
+      for (int i = 0; i < 4; ++i)
+        if (m0 + 8 * i < M) { s.x += v[i].x; s.y += v[i].y; s.z += v[i].z; s.w += v[i].w; }
 #pragma unroll
-      for (int d = 8; d <= 16; d <<= 1) {
+      for (int d = 4; d <= 16; d <<= 1) {
         s.x += __shfl_xor_sync(0xffffffffu, s.x, d); s.y += __shfl_xor_sync(0xffffffffu, s.y, d);
         s.z += __shfl_xor_sync(0xffffffffu, s.z, d); s.w += __shfl_xor_sync(0xffffffffu, s.w, d);
       }
-      if ((threadIdx.x & 31) < 8) tc::store_guarded(x.colsum + ((size_t)tile_m * 4 + (r0 >> 5)) * N + n, s, nn, vec_ok);
+      if ((threadIdx.x & 31) < 4) tc::store_guarded(x.colsum + ((size_t)tile_m * 4 + (r0 >> 5)) * N + n, s, nn, vec_ok);
     }
   }
 };

@@ -3,13 +3,13 @@
 // memory, fed by TMA, consumed by tcgen05.mma kind::tf32.
 //
 // Persistent CTAs (one per SM) walk a list of output tiles (row tile, column tile,
-// batch x K-split).  Six or ten warps, fixed roles:
+// batch x K-split).  Six or eighteen warps, fixed roles:
 //   warp 0     TMA producer: per K-slice, one mbarrier-tracked ring
 //              slot holding the A and B slices (and their residual planes for 3xTF32);
 //              the ring runs ahead across tile boundaries
 //   warp 1     TMEM allocation; issues the UMMAs (M=128, K=8) and commits
 //              ring slots back to the producer, then the accumulator to the epilogue
-//   warps 2..  epilogue (4 or 8 warps, the policy's choice): tcgen05.ld (thread = accumulator row),
+//   warps 2..  epilogue (4 or 16 warps, the policy's choice): tcgen05.ld (thread = accumulator row),
 //              policy-defined store
 // TMEM holds two accumulators, so the epilogue of tile i runs under the main loop of
 // tile i+1.
@@ -46,6 +46,8 @@
 // Every mbarrier wait is bounded: on expiry the kernel records an error code,
 // waits (bounded) for TMA loads it already issued, frees its TMEM and returns.
 #pragma once
+
+#include <algorithm>
 
 #include "igemm_problems.cuh"
 #include "nrs_internal.h"
@@ -86,13 +88,35 @@ struct SplitInfo {
 // Tile list of one launch.  Within a (batch, split) plane tiles are visited in groups of
 // kGroupM row tiles x all column tiles, row tile fastest, so the tiles in flight at any
 // moment cover a compact block of the output and share operand slices through L2.
+// Causal products have lists of their own, walked back and forth (round 0 of the grid from its first CTA, round 1 from
+// its last, ...): with the plain list the tiles a CTA meets are a fixed stride apart, which for four row tiles gave some
+// CTAs nothing but empty tiles and others nothing but the longest.
+enum TileOrder { kRaster = 0, kTriangle = 1 /* only tiles that touch the diagonal or lie below */, kLastFirst = 2, kFirstFirst = 3 /* by row tile,
+                 the one with the most K-slices first, all planes of it before the next */ };
 struct TileMap {
   int tiles_m, tiles_n;
-  long total;          // tiles_m * tiles_n * batches * splits
+  long total;          // tiles_m * tiles_n * batches * splits (kTriangle: the tiles that exist)
+  int order, planes, per_plane;
+  template <int BN>
   __device__ __forceinline__ void decode(long t, int* tile_m, int* tile_n, int* z) const {
-    const int per_z = tiles_m * tiles_n;
-    *z = (int)(t / per_z);
-    const int r = (int)(t - (long)*z * per_z);
+    const uint32_t u = (uint32_t)t;   // (launch() checks the range)
+    if (order >= kLastFirst) {
+      const uint32_t mn = u / (uint32_t)planes;
+      *z = (int)(u - mn * planes);
+      const int m = (int)(mn / (uint32_t)tiles_n);
+      *tile_n = (int)(mn - (uint32_t)m * tiles_n);
+      *tile_m = order == kLastFirst ? tiles_m - 1 - m : m;
+      return;
+    }
+    *z = (int)(u / (uint32_t)per_plane);
+    const int r = (int)(u - (uint32_t)*z * per_plane);
+    if (order == kTriangle) {
+      int m = 0, left = r;
+      for (int cnt; left >= (cnt = min(tiles_n, (m * BM + BM - 1) / BN + 1)); ++m) left -= cnt;
+      *tile_m = m;
+      *tile_n = left;
+      return;
+    }
     const int group = r / (kGroupM * tiles_n);
     const int first = group * kGroupM;
     const int gm = min(kGroupM, tiles_m - first);
@@ -100,12 +124,17 @@ struct TileMap {
     *tile_n = rr / gm;
     *tile_m = first + (rr - *tile_n * gm);
   }
+  // The tile that CTA `me` of `step` takes in the round that starts at `base`; -1: none.
+  __device__ __forceinline__ long at(long base, long me, long step, bool odd) const {
+    const long t = base + (order != kRaster && odd ? step - 1 - me : me);
+    return t < total ? t : -1;
+  }
 };
 
 // Shared memory of the epilogue: the plane-emission staging tile, one [128 rows][128 B] tile per plane, or (row-major
-// results) a 32 x 32 transpose tile per warp.
+// results) a 32 x 16 transpose tile per warp.
 template <int NPLANES, class Policy>
-__host__ __device__ constexpr int emit_bytes() { return Policy::kCanEmit ? NPLANES * BM * 128 : Policy::kEpiWarps * 4096; }
+__host__ __device__ constexpr int emit_bytes() { return Policy::kCanEmit ? NPLANES * BM * 128 : Policy::kEpiWarps * 2048; }
 template <class Policy>
 __host__ __device__ constexpr int threads() { return 64 + 32 * Policy::kEpiWarps; }
 
@@ -122,23 +151,20 @@ __device__ __forceinline__ float4 load_guarded(const float* src, int n, bool vec
   return make_float4(n > 0 ? src[0] : 0.0f, n > 1 ? src[1] : 0.0f, n > 2 ? src[2] : 0.0f, n > 3 ? src[3] : 0.0f);
 }
 
-// A warp's 32 rows x 32 columns, one row per lane, turned into eight float4s per lane that lie along the rows: lane l
-// gets row 4*i + l/8, columns 4*(l%8)..+3 in v[i].  A global access of the warp then covers four full 128-byte lines
-// instead of 16 bytes in each of 32 (which took the store unit 32 cycles an instruction: 2 us per 128 x 128 tile and
-// output).  The tile is 32 rows of 128 bytes with the 16-byte chunks XORed by row % 8: conflict-free both ways.
-__device__ __forceinline__ void rows_to_lines(float* tile, int lane, const uint32_t (&r)[32], float4 (&v)[8]) {
+// A warp's 32 rows x 16 columns, one row per lane, turned into four float4s per lane that lie along the rows: lane l
+// gets row 8*i + l/4, columns 4*(l%4)..+3 in v[i].  A global access of the warp then covers eight 64-byte row segments
+// instead of 16 bytes in each of 32 rows (which took the store unit 32 cycles an instruction: 2 us per 128 x 128 tile and
+// output).  The tile is 16 lines of 128 bytes, two rows a line, its 16-byte chunks XORed by the line: conflict-free both ways.
+__device__ __forceinline__ void rows_to_lines(float* tile, int lane, const uint32_t (&r)[16], float4 (&v)[4]) {
   float4* t4 = reinterpret_cast<float4*>(tile);
+  auto chunk = [](int row, int c) { return row * 4 + (c ^ ((row >> 1) & 3)); };
   __syncwarp();   // the previous block's values have been read
 #pragma unroll
-  for (int g = 0; g < 8; ++g)
-    t4[lane * 8 + (g ^ (lane & 7))] = make_float4(__uint_as_float(r[4 * g]), __uint_as_float(r[4 * g + 1]), __uint_as_float(r[4 * g + 2]),
-                                                  __uint_as_float(r[4 * g + 3]));
+  for (int g = 0; g < 4; ++g)
+    t4[chunk(lane, g)] = make_float4(__uint_as_float(r[4 * g]), __uint_as_float(r[4 * g + 1]), __uint_as_float(r[4 * g + 2]), __uint_as_float(r[4 * g + 3]));
   __syncwarp();
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int row = 4 * i + (lane >> 3);
-    v[i] = t4[row * 8 + ((lane & 7) ^ (row & 7))];
-  }
+  for (int i = 0; i < 4; ++i) v[i] = t4[chunk(8 * i + (lane >> 2), lane & 3)];
 }
 
 template <int BN, int NPLANES, class Policy, bool PAIR>
@@ -194,9 +220,12 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
     const uint32_t slice_bytes = (uint32_t)(PAIR ? 2 : 1) * NPLANES * (pol.a_slice_bytes() + (uint32_t)L::kBTile);
     uint32_t s = 0, ph = 0, issued = 0;   // ring slot, its use's parity, slices so far: run on across tiles
     bool ok = true;
-    for (long t = t_first; t < tmap.total && ok; t += t_step) {
+    bool odd = false;
+    for (long base = 0; base < tmap.total && ok; base += t_step, odd = !odd) {
+      const long t = tmap.at(base, t_first, t_step, odd);
+      if (t < 0) break;
       int tile_m, tile_n, z;
-      tmap.decode(t, &tile_m, &tile_n, &z);
+      tmap.template decode<BN>(t, &tile_m, &tile_n, &z);
       if (PAIR) tile_m = 2 * tile_m + rank;   // beyond the last row tile: TMA fills zeros
       const int batch = z / sp.splits, split = z - batch * sp.splits;
       int kb_begin = split * sp.kb_per_split;
@@ -265,9 +294,12 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
       };
       uint32_t s = 0, ph = 0, local = 0;
       bool ok = true;
-      for (long t = t_first; t < tmap.total && ok; t += t_step) {
+      bool odd = false;
+      for (long base = 0; base < tmap.total && ok; base += t_step, odd = !odd) {
+        const long t = tmap.at(base, t_first, t_step, odd);
+        if (t < 0) break;
         int tile_m, tile_n, z;
-        tmap.decode(t, &tile_m, &tile_n, &z);
+        tmap.template decode<BN>(t, &tile_m, &tile_n, &z);
         const int split = z % sp.splits;
         int kb_begin = split * sp.kb_per_split, kb_end = min(sp.kb_total, kb_begin + sp.kb_per_split);
         if (!pol.clip(tile_m, tile_n, BN, &kb_begin, &kb_end)) continue;
@@ -313,9 +345,12 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
     const bool emit_issuer = warp == 2 && lane == 0;
     uint32_t local = 0, emitted = 0;
     bool ok = true;
-    for (long t = t_first; t < tmap.total && ok; t += t_step) {
+    bool odd = false;
+    for (long base = 0; base < tmap.total && ok; base += t_step, odd = !odd) {
+      const long t = tmap.at(base, t_first, t_step, odd);
+      if (t < 0) break;
       int tile_m, tile_n, z;
-      tmap.decode(t, &tile_m, &tile_n, &z);
+      tmap.template decode<BN>(t, &tile_m, &tile_n, &z);
       if (PAIR) tile_m = 2 * tile_m + rank;
       const int batch = z / sp.splits, split = z - batch * sp.splits;
       int kb_begin = split * sp.kb_per_split, kb_end = min(sp.kb_total, kb_begin + sp.kb_per_split);
@@ -334,27 +369,27 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
         if (lane != 0) return;
         if constexpr (PAIR) mbar_arrive_cluster(cluster_addr(&acc_empty[buf], 0)); else mbar_arrive(&acc_empty[buf]);
       };
-      // one column block only: the second warp of a quarter just hands the accumulator back, and so do all of a pair's
-      // second CTA beyond the last row tile
-      if ((BN == 32 && warp >= 6) || (PAIR && tile_m * BM >= sp.rows_total)) {
+      // The warps of a lane quarter share its column blocks out; those without one just hand the accumulator back, and so
+      // do all of a pair's second CTA beyond the last row tile.
+      constexpr int kW = Policy::kCanEmit ? 32 : 16, kBlocks = BN / kW, kStep = Policy::kEpiWarps / 4;
+      const int c_first = kStep == 1 ? 0 : (warp - 2) >> 2;
+      if (c_first >= kBlocks || (PAIR && tile_m * BM >= sp.rows_total)) {
         hand_back();
         continue;
       }
       const uint32_t acc = tmem_base + buf * (uint32_t)L::kAccCols + ((uint32_t)(q * 32) << 16);
-      // two warps of a lane quarter take alternate 32-column blocks
-      constexpr int kBlocks = BN / 32, kStep = Policy::kEpiWarps / 4;
 #pragma unroll 1
-      for (int c = kStep == 1 ? 0 : (warp - 2) >> 2; c < kBlocks; c += kStep) {
-        uint32_t r[32];
+      for (int c = c_first; c < kBlocks; c += kStep) {
+        uint32_t r[kW];
         // the columns of the first and of the second product (a pair: see kNarrow)
-        const int first = PAIR && NPLANES == 2 && c * 32 >= BN / 2 ? BN / 2 + c * 32 : c * 32;
-        tmem_ld_32x32(acc + (uint32_t)first, r);
+        const int first = PAIR && NPLANES == 2 && c * kW >= BN / 2 ? BN / 2 + c * kW : c * kW;
+        tmem_ld_32(acc + (uint32_t)first, r);
         if (NPLANES == 2) {
-          uint32_t r2[32];
-          tmem_ld_32x32(acc + (uint32_t)(first + (PAIR ? BN / 2 : BN)), r2);
+          uint32_t r2[kW];
+          tmem_ld_32(acc + (uint32_t)(first + (PAIR ? BN / 2 : BN)), r2);
           tmem_ld_wait();
 #pragma unroll
-          for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(r2[j]));
+          for (int j = 0; j < kW; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(r2[j]));
         } else {
           tmem_ld_wait();
         }
@@ -363,15 +398,15 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
           tc_fence_before_sync();
           hand_back();
         }
-        if (n0 + c * 32 >= sp.n_total) continue;   // padding columns of a ragged last tile
+        if (n0 + c * kW >= sp.n_total) continue;   // padding columns of a ragged last tile
         if constexpr (!Policy::kCanEmit) {
-          float4 v[8];
-          rows_to_lines(reinterpret_cast<float*>(emit_tile) + (warp - 2) * 1024, lane, r, v);
-          const int r0 = q * 32 + (lane >> 3), n = n0 + c * 32 + (lane & 7) * 4;
+          float4 v[4];
+          rows_to_lines(reinterpret_cast<float*>(emit_tile) + (warp - 2) * 512, lane, r, v);
+          const int r0 = q * 32 + (lane >> 2), n = n0 + c * kW + (lane & 3) * 4;
           if (sp.splits > 1) {
             float* dst = sp.partial + (((size_t)split * sp.batches + batch) * sp.rows_total + (size_t)tile_m * BM + r0) * sp.n_total + n;
 #pragma unroll
-            for (int i = 0; i < 8; ++i, dst += (size_t)4 * sp.n_total) store_guarded(dst, v[i], sp.n_total - n, sp.n_total % 4 == 0);
+            for (int i = 0; i < 4; ++i, dst += (size_t)8 * sp.n_total) store_guarded(dst, v[i], sp.n_total - n, sp.n_total % 4 == 0);
           } else {
             pol.epilogue(tile_m, batch, r0, n, v);
           }
@@ -573,7 +608,13 @@ int launch(nrs_ctx* ctx, const CUtensorMap& ta_hi, const CUtensorMap& ta_lo, con
   int st = nrs_err_flag(ctx, &err);
   if (st != NRS_OK) return st;
   const int units_m = PAIR ? (tiles_m + 1) / 2 : tiles_m;
-  TileMap tmap{units_m, tiles_n, (long)units_m * tiles_n * batches * sp.splits};
+  TileMap tmap{units_m, tiles_n, 0, pol.order(), batches * sp.splits, units_m * tiles_n};
+  if (tmap.order == kTriangle) {
+    tmap.per_plane = 0;
+    for (int m = 0; m < tiles_m; ++m) tmap.per_plane += std::min(tiles_n, (m * BM + BM - 1) / BN + 1);
+  }
+  tmap.total = (long)tmap.per_plane * tmap.planes;
+  NRS_REQUIRE(ctx, (long)units_m * tiles_n <= 0x7fffffffL && tmap.total <= 0x7fffffffL, NRS_ERR_SHAPE, "tensor-core product: too many tiles");
   const long slots = PAIR ? ctx->sm_count / 2 : ctx->sm_count;
   const unsigned grid = (unsigned)((tmap.total < slots ? tmap.total : slots) * (PAIR ? 2 : 1));
   // Planes can only be emitted by the direct epilogue; with a K-split the policy's store() writes them.
