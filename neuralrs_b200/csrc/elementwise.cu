@@ -108,8 +108,19 @@ colsum_kernel(const float* __restrict__ g, float* __restrict__ out, int rows, in
   const int rows_per = (rows + row_splits - 1) / row_splits;
   const int r0 = split * rows_per, r1 = min(rows, r0 + rows_per);
   float s = 0.0f;
-  if (c < cols)
-    for (int r = r0 + wrp; r < r1; r += 8) s += g[(size_t)r * cols + c];
+  if (c < cols) {
+    const float* p = g + (size_t)(r0 + wrp) * cols + c;
+    const size_t step = (size_t)8 * cols;
+    int r = r0 + wrp;
+    for (; r + 56 < r1; r += 64, p += 8 * step) {   // eight rows in flight: latency is what bounds it
+      float v[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = p[i * step];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) s += v[i];
+    }
+    for (; r < r1; r += 8, p += step) s += *p;
+  }
   sm[wrp][lane] = s;
   __syncthreads();
   if (wrp == 0 && c < cols) {

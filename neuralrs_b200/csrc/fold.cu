@@ -66,29 +66,28 @@ __device__ void fold_columns(const NrsFoldJob& j, unsigned blk, float* sm) {
 
 // dw (+)= sum over splits of partial tiles.  A block is (256 / lanes) outputs (quads of four input channels) x `lanes`
 // split lanes: lane y sums splits y, y + lanes, ... and the lanes are combined in lane order through shared memory: a
-// fixed order of additions without one serial chain of loads per output.  `tile_offset` and `store` are the layouts of
-// the two weight-gradient kernels.
-__device__ void fold_tiles(const NrsFoldJob& j, unsigned blk, float4* lane_sum) {
+// fixed order of additions without one serial chain of loads per output.  Outputs are counted (co, 32-channel block,
+// tap, quad), so that reads of the partials are 128-byte runs along ci and the 8 * taps outputs of a block of channels
+// are one run of dw: with several taps the sums go back through shared memory and leave in dw's order (written from
+// their quads, 4 bytes every 4 * taps, they took twice as long as the reads).
+__device__ void fold_tiles(const NrsFoldJob& j, unsigned blk, float4* sums) {
   const int per_block = 256 / j.lanes;
   const int lane = threadIdx.x / per_block, slot = threadIdx.x - lane * per_block;
-  const int cq = (j.ci + 3) / 4;                  // a thread owns four consecutive input channels (padded in the partials)
-  const size_t total = (size_t)j.co * cq * j.taps;
-  const size_t idx = (size_t)blk * per_block + slot;
-  const bool live = idx < total;
-  // idx enumerates (co, tap, ci/4) so that reads of the partials are coalesced 128-bit loads along ci
-  const int c = (int)(idx % cq) * 4;
-  const int tap = (int)((idx / cq) % j.taps);
-  const int co = (int)(idx / ((size_t)cq * j.taps));
+  const uint32_t cblks = (uint32_t)(j.ci + 31) / 32, run = 8u * j.taps;
+  const uint32_t total = (uint32_t)j.co * cblks * run;   // (below 2^31: nrs_fold_submit)
+  const uint32_t idx = blk * per_block + slot;
+  const uint32_t r = idx / run, u = idx - r * run;
+  const int tap = (int)(u >> 3), co = (int)(r / cblks), c = (int)(r - (uint32_t)co * cblks) * 32 + (int)(u & 7) * 4;
+  const bool live = idx < total && c < j.ci;
   size_t off;
-  int out_tap = tap;
   if (j.kind == NRS_FOLD_WGRAD) {                 // [m block][group][column block][128][group_cols]
     const int mb = co / 128, row = co - mb * 128;
     const int grp = tap / j.taps_per_group, t = tap - grp * j.taps_per_group;
     const int cbk = j.col_blocks > 1 ? c / 256 : 0;
     const size_t col = j.col_blocks > 1 ? (size_t)(c - cbk * 256) : (size_t)t * j.cblocks * 32 + c;
     off = ((((size_t)mb * j.n_groups + grp) * j.col_blocks + cbk) * 128 + row) * j.group_cols + col;
-  } else {                                        // rows kernel: tap = (horizontal j, vertical i), i fastest
-    const int i = tap % 3, jt = tap / 3;
+  } else {                                        // rows kernel: a (horizontal j, vertical i) pair per tap
+    const int i = tap / 3, jt = tap - 3 * i;
     int mb = co / 128, row = co - mb * 128, jk = jt;
     if (j.pack) {   // tap 1 -> kind 0 rows [0,h); tap 0 -> kind 0 rows [h,2h); tap 2 -> kind 1 rows [0,h)
       mb = 0;
@@ -99,7 +98,6 @@ __device__ void fold_tiles(const NrsFoldJob& j, unsigned blk, float4* lane_sum) 
     const int cta = (mb * j.jtypes + jk) * j.n_chunks + cc;
     const size_t cols = (size_t)3 * j.chunk;
     off = ((size_t)cta * 128 + row) * cols + (size_t)i * j.chunk + (c - cc * j.chunk);
-    out_tap = i * 3 + jt;
   }
   float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
   if (live) {
@@ -109,26 +107,50 @@ __device__ void fold_tiles(const NrsFoldJob& j, unsigned blk, float4* lane_sum) 
       s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
     }
   }
-  lane_sum[threadIdx.x] = s;
-  __syncthreads();
-  if (lane != 0 || !live) return;
-  for (int l = 1; l < j.lanes; ++l) {
-    const float4 v = lane_sum[l * per_block + slot];
-    s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+  if (j.lanes > 1) {
+    sums[threadIdx.x] = s;
+    __syncthreads();
+    if (lane == 0)
+      for (int l = 1; l < j.lanes; ++l) {
+        const float4 v = sums[l * per_block + slot];
+        s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+      }
   }
-  // [co][ci][taps]; with out_cols (several matrices side by side) columns c of matrix c / out_cols, each [co][out_cols]
-  const float r[4] = {s.x, s.y, s.z, s.w};
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    if (c + k >= j.ci) continue;
-    float* dst;
-    if (j.out_cols) {
-      const int mat = (c + k) / j.out_cols;
-      dst = j.dst + (size_t)mat * j.co * j.out_cols + (size_t)co * j.out_cols + (c + k - mat * j.out_cols);
-    } else {
-      dst = j.dst + ((size_t)co * j.ci + c + k) * j.taps + out_tap;
+  if (j.taps == 1) {
+    // [co][ci]; with out_cols (several matrices side by side) columns c of matrix c / out_cols, each [co][out_cols]
+    if (lane != 0 || !live) return;
+    if (j.vec) {
+      const int mat = j.out_cols ? c / j.out_cols : 0, ld = j.out_cols ? j.out_cols : j.ci;
+      float4* dst = reinterpret_cast<float4*>(j.dst + (size_t)mat * j.co * ld + (size_t)co * ld + (c - mat * ld));
+      if (j.accumulate) {
+        const float4 o = *dst;
+        s = make_float4(o.x + s.x, o.y + s.y, o.z + s.z, o.w + s.w);
+      }
+      *dst = s;
+      return;
     }
-    put(dst, r[k], j.accumulate);
+    const float e[4] = {s.x, s.y, s.z, s.w};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (c + k >= j.ci) continue;
+      const int mat = j.out_cols ? (c + k) / j.out_cols : 0, ld = j.out_cols ? j.out_cols : j.ci;
+      put(j.dst + (size_t)mat * j.co * ld + (size_t)co * ld + (c + k - mat * ld), e[k], j.accumulate);
+    }
+    return;
+  }
+  __syncthreads();   // (the lanes' sums have been read)
+  if (lane == 0) sums[slot] = s;
+  __syncthreads();
+  const float* f = reinterpret_cast<const float*>(sums);
+  const uint32_t first = blk * per_block, end = min(first + per_block, total);
+  if (first >= total) return;
+  const uint32_t r0 = first / run, r1 = (end - 1) / run + 1;
+  for (uint32_t q = threadIdx.x; q < (r1 - r0) * 4 * run; q += 256) {   // output values of the runs this block has a share in
+    const uint32_t rr = q / (4 * run), p = q - rr * 4 * run;
+    const uint32_t ch = p / (uint32_t)j.taps, t = p - ch * j.taps, id = (r0 + rr) * run + t * 8 + (ch >> 2);
+    const uint32_t o = (r0 + rr) / cblks, cc = (r0 + rr - o * cblks) * 32 + ch;
+    if (id >= first && id < end && cc < (uint32_t)j.ci)
+      put(j.dst + ((size_t)o * j.ci + cc) * j.taps + t, f[(id - first) * 4 + (ch & 3)], j.accumulate);
   }
 }
 
@@ -145,7 +167,7 @@ __global__ void __launch_bounds__(256) fold_kernel(const __grid_constant__ FoldB
 
 unsigned job_blocks(const NrsFoldJob& j) {
   if (j.kind == NRS_FOLD_COLUMNS) return (unsigned)((j.cols + 31) / 32) * (unsigned)j.splits;
-  const size_t total = (size_t)j.co * ((j.ci + 3) / 4) * j.taps;
+  const size_t total = (size_t)j.co * ((j.ci + 31) / 32) * 8 * j.taps;
   return (unsigned)((total + 256 / j.lanes - 1) / (256 / j.lanes));
 }
 
@@ -251,6 +273,11 @@ int nrs_fold_partial(nrs_ctx* ctx, int ws_slot, size_t bytes, float** out) {
 
 int nrs_fold_submit(nrs_ctx* ctx, NrsFoldJob job) {
   NrsFolds& f = ctx->folds;
+  if (job.kind != NRS_FOLD_COLUMNS) {
+    NRS_REQUIRE(ctx, (size_t)job.co * ((job.ci + 31) / 32) * 8 * job.taps < 0x7fffffffu, NRS_ERR_SHAPE, "weight gradient: too large");
+    const int ld = job.out_cols ? job.out_cols : job.ci;
+    job.vec = job.taps == 1 && ld % 4 == 0 && (reinterpret_cast<uintptr_t>(job.dst) & 15) == 0;
+  }
   if (!f.active) return run(ctx, &job, 1);
   const unsigned need = job.kind == NRS_FOLD_COLUMNS && job.splits > 1 ? (unsigned)((job.cols + 31) / 32) : 0;
   if (f.jobs.size() >= (size_t)kMaxJobs || f.tickets_used + need > kNrsFoldTickets) {

@@ -230,6 +230,20 @@ static bool planes_possible(nrs_ctx* ctx) {
 void cache_row_planes(const NodeP& x, size_t rows, size_t cols) { cache_planes_2d(x, rows, cols); }
 bool operand_planes_possible(nrs_ctx* ctx) { return planes_possible(ctx); }
 
+// May a [rows, cols] tensor whose only reader is a product with a [cols, reader_cols] weight exist as planes alone?
+// Both products that read it (forward, weight gradient) have to take planes.
+bool values_as_planes_only(nrs_ctx* ctx, size_t rows, size_t cols, size_t reader_cols) {
+  return reader_cols > 0 && ctx->math_mode == NRS_MATH_3XTF32 && cols % 8 == 0 &&
+         nrs_gemm_on_tensor_cores(ctx, (int)rows, (int)reader_cols, (int)cols) &&
+         nrs_gemm_on_tensor_cores(ctx, (int)cols, (int)reader_cols, (int)rows) && nrs_gemm_tn_reads_planes((int)cols, (int)reader_cols);
+}
+// The math mode was changed between the passes: the values are wanted after all.
+static void need_values(const NodeP& x) {
+  if (!x->planes_only || x->ctx->math_mode == NRS_MATH_3XTF32) return;
+  check(x->ctx, nrs_add(x->ctx, x->planes_hi, x->planes_lo, x->data, x->len()));
+  x->planes_only = false;
+}
+
 namespace cuda {
 
 // ------------------------------------------------------------------ runtime
@@ -330,6 +344,7 @@ NodeP matmul(const NodeP& a, const NodeP& b) {
   out->backward_fn = [self, a, b, m, k, n, tensor_cores]() {
     nrs_ctx* ctx = self->ctx;
     const float* dc = grad_in(self);
+    need_values(a);
     GradPlanes dc_planes(ctx, dc, (size_t)m, (size_t)n, tensor_cores && a->requires_grad && b->requires_grad);
     if (a->requires_grad) {
       const bool emit = a->row_planes_wanted && tensor_cores && k % 8 == 0 && !a->view_of && !a->grad_valid && !a->gplanes_hi;
@@ -339,6 +354,7 @@ NodeP matmul(const NodeP& a, const NodeP& b) {
         NrsGemmExtras e;
         e.hi = dalloc(ctx, a->len());
         if (ctx->math_mode == NRS_MATH_3XTF32) e.lo = dalloc(ctx, a->len());
+        e.skip_c_unsplit = a->internal && e.lo;
         st = nrs_gemm_extras(ctx, 0, 1, m, k, n, dc, b->data, t.ptr, nullptr, NRS_ACT_NONE, 0.0f, &e);
         if (st == NRS_OK) {
           a->gplanes_hi = e.hi;
@@ -1173,6 +1189,7 @@ static void linear_input_grad(nrs_ctx* ctx, const NodeP& x, const NodeP& w, cons
     if (ctx->math_mode == NRS_MATH_3XTF32) e.lo = dalloc(ctx, x->len());
     e.colsum_cap = (m + 127) / 128 * 4;
     e.colsum = dalloc(ctx, (size_t)e.colsum_cap * k);
+    e.skip_c_unsplit = x->internal && e.lo;
     const int st = nrs_gemm_extras(ctx, 0, 1, m, k, n, dz, w->data, t.ptr, nullptr, NRS_ACT_NONE, 0.0f, &e);
     if (st == NRS_OK && e.honoured && e.colsum_rows > 0) {
       x->gplanes_hi = e.hi;
@@ -1192,8 +1209,9 @@ static void linear_input_grad(nrs_ctx* ctx, const NodeP& x, const NodeP& w, cons
 }
 
 // emit_planes: the caller knows that a tensor-core GEMM reads the result (always assumed of a GELU layer, which has
-// no other use in the models of this API): its epilogue writes the result's operand planes.
-NodeP linear_act(const NodeP& x, const NodeP& w, const NodeP& b, int act, bool emit_planes) {
+// no other use in the models of this API): its epilogue writes the result's operand planes.  reader_cols: the caller
+// keeps the result to itself and hands it to one Linear layer of that many outputs.
+NodeP linear_act(const NodeP& x, const NodeP& w, const NodeP& b, int act, bool emit_planes, size_t reader_cols) {
   require_gpu(x, "cuda linear: input");
   require_gpu(w, "cuda linear: weights");
   require_gpu(b, "cuda linear: bias");
@@ -1216,10 +1234,13 @@ NodeP linear_act(const NodeP& x, const NodeP& w, const NodeP& b, int act, bool e
     e.hi = dalloc(ctx, out->len());
     if (ctx->math_mode == NRS_MATH_3XTF32) e.lo = dalloc(ctx, out->len());
   }
+  out->internal = reader_cols > 0;
+  e.skip_c_unsplit = e.lo && act == NRS_ACT_GELU && values_as_planes_only(ctx, (size_t)m, (size_t)n, reader_cols);
   const int st = pre || e.hi ? nrs_gemm_extras(ctx, 0, 0, m, n, k, x->data, w->data, out->data, b->data, act, 0.0f, &e) : NRS_ERR_UNSUPPORTED;
   if (st == NRS_OK && e.hi) {
     out->planes_hi = e.hi;
     out->planes_lo = e.lo;
+    out->planes_only = e.skip_c_unsplit;
     NrsPlanes pl{e.hi, e.lo, e.lo ? 1 : 0};
     pl.rows = m;
     pl.cols = n;
@@ -1242,6 +1263,7 @@ NodeP linear_act(const NodeP& x, const NodeP& w, const NodeP& b, int act, bool e
   out->backward_fn = [self, x, w, b, pre, act, m, k, n, tensor_cores]() {
     nrs_ctx* ctx = self->ctx;
     const bool from_planes = self->gz_valid;
+    need_values(x);
     const float* dz = from_planes ? self->gplanes_hi : grad_in(self);
     if (from_planes) {   // the reader of this layer's output left the planes and column sums of dz
       NrsPlanes pl{self->gplanes_hi, self->gplanes_lo, self->gplanes_lo ? 1 : 0};

@@ -81,6 +81,10 @@ struct Node {
   // consumes it lets its input-gradient kernel write them (gplanes_*, registered under the gradient's address).
   bool row_planes_wanted = false;
 
+  // The result of a step inside a composite layer, which no caller holds: values or a gradient that are read as planes
+  // only need not be written besides.  planes_only: `data` was left out (3xTF32: it is planes_hi + planes_lo exactly).
+  bool internal = false, planes_only = false;
+
   size_t len() const;
   bool on_gpu() const { return data != nullptr; }
   ~Node();
@@ -112,6 +116,7 @@ GradSlot grad_slot(const NodeP& n);   // marks the gradient as written
 const float* grad_view(Node* n);      // a node's own incoming gradient (zeros if nothing wrote it)
 NodeP make_result(nrs_ctx* ctx, const std::vector<size_t>& shape, std::vector<NodeP> parents);
 void cache_row_planes(const NodeP& x, size_t rows, size_t cols);   // TF32 row planes of x's data, kept with the node
+bool values_as_planes_only(nrs_ctx* ctx, size_t rows, size_t cols, size_t reader_cols);   // see Node::planes_only
 bool operand_planes_possible(nrs_ctx* ctx);                        // a TF32 math mode on a device with TMA
 
 namespace cuda {
@@ -164,7 +169,7 @@ NodeP dropout2d(const NodeP& x, float p, bool training, const NodeP& mask = null
 // Fused variants with no counterpart op in the reference: one kernel for
 // x@W + b followed by an activation, and conv + bias + activation.  Backward is
 // the composition of the unfused backward passes.
-NodeP linear_act(const NodeP& x, const NodeP& w, const NodeP& b, int act, bool emit_planes = false);
+NodeP linear_act(const NodeP& x, const NodeP& w, const NodeP& b, int act, bool emit_planes = false, size_t reader_cols = 0);
 // emit_planes: the caller knows a tensor-core convolution reads the result next, so the kernel
 // also writes the result's NHWC operand planes (a hint; ignored where it does not apply).
 NodeP conv2d_act(const NodeP& x, const NodeP& w, const NodeP& b, size_t stride, size_t pad, int act,

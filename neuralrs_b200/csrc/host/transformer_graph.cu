@@ -237,7 +237,9 @@ static NodeP planes_attention(const MultiHeadAttention& m, const NodeP& x, size_
   a.qkv_hi = e.hi; a.qkv_lo = e.lo; a.qkv_ld = (int)(3 * d);
   a.p_hi = saved(square);
   a.p_lo = split ? saved(square) : nullptr;
-  a.out = out->data;
+  out->internal = true;
+  out->planes_only = values_as_planes_only(ctx, tokens, d, d);   // read by the output projection alone
+  a.out = out->planes_only ? nullptr : out->data;
   a.out_hi = block(tokens * d);
   a.out_lo = split ? block(tokens * d) : nullptr;
   out->planes_hi = a.out_hi;        // the output projection reads them (and its weight gradient)
@@ -254,6 +256,11 @@ static NodeP planes_attention(const MultiHeadAttention& m, const NodeP& x, size_
   Node* self = out.get();
   out->backward_fn = [self, x, wq, wk, wv, a, tokens, d, square, split, block]() mutable {
     nrs_ctx* ctx = self->ctx;
+    struct Mode {   // the saved planes are those of the forward pass's mode
+      nrs_ctx* c; const int was;
+      Mode(nrs_ctx* c_, int m) : c(c_), was(c_->math_mode) { c->math_mode = m; }
+      ~Mode() { c->math_mode = was; }
+    } mode{ctx, split ? NRS_MATH_3XTF32 : NRS_MATH_TF32};
     const float* g = grad_view(self);
     // the gradient's row planes: left by the output projection's input-gradient kernel, else staged here
     float *ghi = self->gplanes_hi, *glo = self->gplanes_lo;
@@ -349,7 +356,7 @@ static NodeP block_body(const TransformerBlock& b, const NodeP& x, bool final_no
   NodeP flat = reshape(x1, {batch * seq, d});
   NodeP h, ff;
   if (b.fused_epilogues) {
-    h = linear_act(flat, b.ff1.weights, b.ff1.bias, b.act, true);
+    h = linear_act(flat, b.ff1.weights, b.ff1.bias, b.act, true, b.ff2.weights ? b.ff2.weights->shape.back() : 0);
     ff = linear_act(h, b.ff2.weights, b.ff2.bias, NRS_ACT_NONE);
   } else {
     h = b.ff1.forward(flat);

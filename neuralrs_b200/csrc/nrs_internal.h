@@ -136,6 +136,7 @@ struct NrsFoldJob {
   // weight gradients: the partial tiles' layout (see the kernels)
   int taps_per_group, n_groups, col_blocks, cblocks, group_cols;
   int chunk, n_chunks, jtypes, a_blocks, pack;
+  int vec;                 // 1x1: outputs written 16 bytes at a time
   int out_cols;            // general kernel, 1x1: the columns are several [co][out_cols] matrices side by side (0: one)
   size_t split_stride;     // floats between two splits
 };
@@ -404,6 +405,7 @@ struct NrsGemmExtras {
   int colsum_cap = 0;
   int colsum_rows = 0;         // out: rows of it written (0: none, the caller sums the columns itself)
   bool skip_c = false;         // c is not written (its planes are all that is read)
+  bool skip_c_unsplit = false; // ... only where the result leaves in one pass (a K-split's second pass writes c and makes no column sums)
   bool honoured = false;       // out: the tensor-core kernel ran and did all of the above (but colsum: see colsum_rows)
 };
 int nrs_tc_gemm(nrs_ctx* ctx, int trans_a, int trans_b, int batch, int m, int n, int k,

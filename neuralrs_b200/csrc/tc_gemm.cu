@@ -104,7 +104,7 @@ struct GemmPolicy {
 #pragma unroll
       for (int i = 0; i < 4; ++i) { v[i].x += beta * o[i].x; v[i].y += beta * o[i].y; v[i].z += beta * o[i].z; v[i].w += beta * o[i].w; }
     }
-    if (!x.skip_c) {
+    if (!x.skip_c && !x.skip_c_unsplit) {
 #pragma unroll
       for (int i = 0; i < 4; ++i)
         if (m0 + 8 * i < M) tc::store_guarded(C + at0 + i * step, v[i], nn, vec_ok);
