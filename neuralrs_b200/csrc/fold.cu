@@ -4,19 +4,27 @@
 // Nothing in a backward pass reads these gradients, so inside nrs::backward_graph they are collected and run as ONE
 // launch at its end (nrs_folds_begin / nrs_folds_flush); outside of it each runs as a batch of one.  The job table
 // travels as a kernel parameter.  Every sum has a fixed order, whatever the batch.  Measured on the CIFAR CNN at batch
-// 100: 15 launches, 104 us, become one of 33 us; on the language model (32 x 128 tokens) 21 launches, 125 us, one of 30.
+// 100: 15 launches, 104 us, become one of 38 us; on the language model (32 x 128 tokens) 21 launches, 125 us, one of 40.
 #include "fold.h"
 
 #include <algorithm>
 
+#include "igemm_problems.cuh"
+
 namespace {
 
 constexpr int kMaxJobs = 32;
+// The divisions that place a weight gradient's outputs, as multiplications (with 32-bit divisions the pass was bound by
+// instructions: 740 per warp, most of them there).
+struct FoldDiv {
+  NrsFastDiv run, run4, taps, cblks, group, chunk;
+};
 struct FoldBatch {
   int n;
   NrsFoldJob job[kMaxJobs];
+  FoldDiv div[kMaxJobs];
 };
-static_assert(sizeof(FoldBatch) <= 4000, "the job table is a kernel parameter");
+static_assert(sizeof(FoldBatch) <= 8000, "the job table is a kernel parameter");
 
 __device__ __forceinline__ void put(float* dst, float v, int accumulate) { *dst = accumulate ? *dst + v : v; }
 
@@ -70,31 +78,33 @@ __device__ void fold_columns(const NrsFoldJob& j, unsigned blk, float* sm) {
 // tap, quad), so that reads of the partials are 128-byte runs along ci and the 8 * taps outputs of a block of channels
 // are one run of dw: with several taps the sums go back through shared memory and leave in dw's order (written from
 // their quads, 4 bytes every 4 * taps, they took twice as long as the reads).
-__device__ void fold_tiles(const NrsFoldJob& j, unsigned blk, float4* sums) {
+__device__ void fold_tiles(const NrsFoldJob& j, const FoldDiv& dv, unsigned blk, float4* sums) {
   const int per_block = 256 / j.lanes;
   const int lane = threadIdx.x / per_block, slot = threadIdx.x - lane * per_block;
   const uint32_t cblks = (uint32_t)(j.ci + 31) / 32, run = 8u * j.taps;
   const uint32_t total = (uint32_t)j.co * cblks * run;   // (below 2^31: nrs_fold_submit)
   const uint32_t idx = blk * per_block + slot;
-  const uint32_t r = idx / run, u = idx - r * run;
-  const int tap = (int)(u >> 3), co = (int)(r / cblks), c = (int)(r - (uint32_t)co * cblks) * 32 + (int)(u & 7) * 4;
+  uint32_t r, u, co_u, cb;
+  dv.run.divmod(idx, r, u);
+  dv.cblks.divmod(r, co_u, cb);
+  const int tap = (int)(u >> 3), co = (int)co_u, c = (int)(cb * 32 + (u & 7) * 4);
   const bool live = idx < total && c < j.ci;
   size_t off;
   if (j.kind == NRS_FOLD_WGRAD) {                 // [m block][group][column block][128][group_cols]
-    const int mb = co / 128, row = co - mb * 128;
-    const int grp = tap / j.taps_per_group, t = tap - grp * j.taps_per_group;
-    const int cbk = j.col_blocks > 1 ? c / 256 : 0;
+    const int mb = co >> 7, row = co & 127;
+    const int grp = (int)dv.group.div((uint32_t)tap), t = tap - grp * j.taps_per_group;
+    const int cbk = j.col_blocks > 1 ? c >> 8 : 0;
     const size_t col = j.col_blocks > 1 ? (size_t)(c - cbk * 256) : (size_t)t * j.cblocks * 32 + c;
     off = ((((size_t)mb * j.n_groups + grp) * j.col_blocks + cbk) * 128 + row) * j.group_cols + col;
   } else {                                        // rows kernel: a (horizontal j, vertical i) pair per tap
-    const int i = tap / 3, jt = tap - 3 * i;
-    int mb = co / 128, row = co - mb * 128, jk = jt;
+    const int i = (int)((unsigned)tap / 3u), jt = tap - 3 * i;
+    int mb = co >> 7, row = co & 127, jk = jt;
     if (j.pack) {   // tap 1 -> kind 0 rows [0,h); tap 0 -> kind 0 rows [h,2h); tap 2 -> kind 1 rows [0,h)
       mb = 0;
       jk = jt == 2 ? 1 : 0;
       row = co + (jt == 0 ? 32 * j.a_blocks : 0);
     }
-    const int cc = c / j.chunk;
+    const int cc = (int)dv.chunk.div((uint32_t)c);
     const int cta = (mb * j.jtypes + jk) * j.n_chunks + cc;
     const size_t cols = (size_t)3 * j.chunk;
     off = ((size_t)cta * 128 + row) * cols + (size_t)i * j.chunk + (c - cc * j.chunk);
@@ -144,13 +154,16 @@ __device__ void fold_tiles(const NrsFoldJob& j, unsigned blk, float4* sums) {
   const float* f = reinterpret_cast<const float*>(sums);
   const uint32_t first = blk * per_block, end = min(first + per_block, total);
   if (first >= total) return;
-  const uint32_t r0 = first / run, r1 = (end - 1) / run + 1;
+  const uint32_t r0 = dv.run.div(first), r1 = dv.run.div(end - 1) + 1;
   for (uint32_t q = threadIdx.x; q < (r1 - r0) * 4 * run; q += 256) {   // output values of the runs this block has a share in
-    const uint32_t rr = q / (4 * run), p = q - rr * 4 * run;
-    const uint32_t ch = p / (uint32_t)j.taps, t = p - ch * j.taps, id = (r0 + rr) * run + t * 8 + (ch >> 2);
-    const uint32_t o = (r0 + rr) / cblks, cc = (r0 + rr - o * cblks) * 32 + ch;
-    if (id >= first && id < end && cc < (uint32_t)j.ci)
-      put(j.dst + ((size_t)o * j.ci + cc) * j.taps + t, f[(id - first) * 4 + (ch & 3)], j.accumulate);
+    uint32_t rr, pos, ch, t, o, ob;
+    dv.run4.divmod(q, rr, pos);
+    dv.taps.divmod(pos, ch, t);
+    const uint32_t id = (r0 + rr) * run + t * 8 + (ch >> 2) - first;
+    dv.cblks.divmod(r0 + rr, o, ob);
+    const uint32_t cc = ob * 32 + ch;
+    if (id < end - first && cc < (uint32_t)j.ci)   // (unsigned: below `first` counts as beyond)
+      put(j.dst + ((size_t)o * j.ci + cc) * j.taps + t, f[id * 4 + (ch & 3)], j.accumulate);
   }
 }
 
@@ -162,7 +175,7 @@ __global__ void __launch_bounds__(256) fold_kernel(const __grid_constant__ FoldB
   const NrsFoldJob& j = b.job[i];
   const unsigned blk = blockIdx.x - j.first_block;
   if (j.kind == NRS_FOLD_COLUMNS) fold_columns(j, blk, reinterpret_cast<float*>(sm));
-  else fold_tiles(j, blk, sm);
+  else fold_tiles(j, b.div[i], blk, sm);
 }
 
 unsigned job_blocks(const NrsFoldJob& j) {
@@ -186,6 +199,11 @@ int run(nrs_ctx* ctx, NrsFoldJob* jobs, int n) {
     }
     j.first_block = blocks;
     blocks += job_blocks(j);
+    if (j.kind != NRS_FOLD_COLUMNS) {
+      const bool general = j.kind == NRS_FOLD_WGRAD;
+      b.div[b.n] = FoldDiv{NrsFastDiv(8 * j.taps), NrsFastDiv(32 * j.taps), NrsFastDiv(j.taps), NrsFastDiv((j.ci + 31) / 32),
+                           NrsFastDiv(general ? j.taps_per_group : 1), NrsFastDiv(general ? 1 : j.chunk)};
+    }
     b.job[b.n++] = j;
   }
   if (blocks == 0) return NRS_OK;

@@ -340,7 +340,19 @@ int nrs_tc_conv_wgrad(nrs_ctx* ctx, const float* x, const float* dy, float* dw, 
   // ... unless that leaves most of the GPU idle (a short reduction with a small output: Linear layers)
   while (min_tiles > 4 && (long)(p.n_tiles / min_tiles) * ctas_per_split < ctx->sm_count / 2) min_tiles /= 2;
   if (min_tiles > max_tiles) min_tiles = max_tiles;
-  const int tps = tc::plan_units_per_cta(ctx->sm_count, ctas_per_split, p.n_tiles, min_tiles, max_tiles, 8);
+  int tps = tc::plan_units_per_cta(ctx->sm_count, ctas_per_split, p.n_tiles, min_tiles, max_tiles, 8);
+  // A short reduction with a large output (a Linear layer at a batch of a hundred: 7 tiles, 8 MB) is better walked by
+  // one CTA per output tile, which then is the result: a split's second pass reads splits + 1 times the output at about
+  // 1.1 KB a clock, and a CTA's own time is about 2 clocks per plane product, pixel and 32 columns.
+  const bool can_be_direct = taps == 1 && ci % 32 == 0 && !accumulate && !out_cols && (reinterpret_cast<uintptr_t>(dw) & 15) == 0;
+  if (can_be_direct && tps < p.n_tiles && p.n_tiles <= max_tiles) {
+    const int s = (p.n_tiles + tps - 1) / tps;
+    auto clocks = [&](int tiles, int splits) {
+      const double rounds = (double)((ctas_per_split * splits + ctx->sm_count - 1) / ctx->sm_count);
+      return rounds * tiles * (p.kp + 6) * (split3 ? 3 : 1) * (p.group_cols / 32) * 2.0;
+    };
+    if (clocks(p.n_tiles, 1) < clocks(tps, s) + (s + 1.0) * co * ci * 4 / 1100.0) tps = p.n_tiles;
+  }
   p.tiles_per_split = tps;
   const int splits = (p.n_tiles + tps - 1) / tps;
   if (splits > 65535) return NRS_ERR_UNSUPPORTED;
@@ -351,7 +363,7 @@ int nrs_tc_conv_wgrad(nrs_ctx* ctx, const float* x, const float* dy, float* dw, 
   const size_t partial_floats = (size_t)splits * p.m_blocks * p.n_groups * p.col_blocks * 128 * p.group_cols;
   void *dy_hi = nullptr, *dy_lo = nullptr, *x_hi = nullptr, *x_lo = nullptr;
   // a single split of a 1x1 "convolution" (A^T B) that overwrites its output needs no second pass
-  p.direct = (splits == 1 && taps == 1 && ci % 32 == 0 && !accumulate && !out_cols && (reinterpret_cast<uintptr_t>(dw) & 15) == 0) ? dw : nullptr;
+  p.direct = splits == 1 && can_be_direct ? dw : nullptr;
   int st = p.direct ? NRS_OK : nrs_fold_partial(ctx, NRS_WS_WGRAD_PARTIAL, partial_floats * sizeof(float), &p.partial);
   if (st != NRS_OK) return st;
   bool may_overlap = ctx->independent_next;   // withdrawn below if this call stages an operand itself
