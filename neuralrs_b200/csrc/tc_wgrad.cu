@@ -244,10 +244,12 @@ tc_wgrad_kernel(const __grid_constant__ CUtensorMap tm_dy_hi, const __grid_const
 
 // Pixel tile = one TMA box {32 channels, Wt, Ht, Nt} of kp = Wt*Ht*Nt pixels, a multiple of 8 (a K-step) up to 64.
 // Boxes of whole rows, or of a multiple of 8 pixels of a row; the one that walks the fewest pixels, padding included,
-// is taken, where every tile costs about 6 pixels' worth of ring bookkeeping (measured: 16-pixel tiles with a deeper
-// ring are slower, the single producer thread becomes TMA-issue bound) and a ring of fewer than three slots a few
-// percent.  A box may reach past the last image too (a few 1x1 "images").
-void plan_pixel_box(WgradParams* p, int n, int oh, int ow, size_t bytes_per_pixel) {
+// is taken, where every tile costs half a pixel's worth per TMA load (measured: 3000 x 2048 x 512 in 3xTF32 35.8 us with
+// slots of 16 pixels, 39.2 with two slots of 32; but with the 12 loads of five taps a slot of 16 costs 24.7 us against
+// 18.6), and a ring of fewer than three slots a few percent.  A box may reach past the last image too (a few 1x1 "images").
+void plan_pixel_box(WgradParams* p, int n, int oh, int ow, int planes, size_t bytes_per_pixel) {
+  const int loads = planes * ((p->ragged_a ? kABlocks : 1) + p->taps_per_group * (p->ragged_x ? p->cblocks : 1));
+  const double per_tile = loads > 4 ? 0.5 * loads : 2.0;
   double best = -1.0;
   for (int c = 0; c <= 8; ++c) {
     const int Wt = c == 0 ? ow : 8 * c;
@@ -260,7 +262,7 @@ void plan_pixel_box(WgradParams* p, int n, int oh, int ow, size_t bytes_per_pixe
         const int stages = (int)((200 * 1024) / (bytes_per_pixel * kp));
         if (stages < 2) continue;
         const long tiles = (long)((ow + Wt - 1) / Wt) * ((oh + Ht - 1) / Ht) * ((n + Nt - 1) / Nt);
-        const double cost = (double)tiles * (kp + 6) * (stages < 3 ? 1.06 : 1.0);
+        const double cost = (double)tiles * (kp + per_tile) * (stages < 3 ? 1.06 : 1.0);
         if (best < 0.0 || cost < best) {
           best = cost;
           p->Wt = Wt; p->Ht = Ht; p->Nt = Nt; p->kp = kp;
@@ -318,7 +320,7 @@ int nrs_tc_conv_wgrad(nrs_ctx* ctx, const float* x, const float* dy, float* dw, 
     p.taps_per_group = 1;
     p.group_cols = kMaxN;
   }
-  plan_pixel_box(&p, n, oh, ow, (size_t)planes * (kABlocks + p.group_cols / 32) * 128);
+  plan_pixel_box(&p, n, oh, ow, planes, (size_t)planes * (kABlocks + p.group_cols / 32) * 128);
   if (p.kp == 0) return NRS_ERR_UNSUPPORTED;
   p.tiles_x = (ow + p.Wt - 1) / p.Wt;
   p.tiles_y = (oh + p.Ht - 1) / p.Ht;
