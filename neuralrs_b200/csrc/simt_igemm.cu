@@ -284,6 +284,45 @@ thin_n_rows_kernel(const float* __restrict__ a, const float* __restrict__ bg, fl
   }
 }
 
+// The same product for few rows (a classifier head at a batch of a hundred): a block per row, its threads stride over k,
+// so that a row is two or three loads deep instead of a warp's walk over k behind a copy of all of B.  Warps combine in
+// warp order.  100 x 512 x 10: 12.8 us with eight rows a block, 5.4 here.
+template <bool TB>
+__global__ void __launch_bounds__(256)
+thin_n_row_kernel(const float* __restrict__ a, const float* __restrict__ b, float* c, const float* __restrict__ bias, int n, int k, int act,
+                  float beta) {
+  NRS_PDL_PROLOGUE();
+  __shared__ float part[8][kThinN];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const float* ar = a + (size_t)blockIdx.x * k;
+  float acc[kThinN];
+#pragma unroll
+  for (int j = 0; j < kThinN; ++j) acc[j] = 0.0f;
+#pragma unroll 2
+  for (int kk = threadIdx.x; kk < k; kk += blockDim.x) {
+    const float av = ar[kk];
+#pragma unroll
+    for (int j = 0; j < kThinN; ++j)
+      if (j < n) acc[j] = fmaf(av, TB ? b[(size_t)j * k + kk] : b[(size_t)kk * n + j], acc[j]);
+  }
+#pragma unroll
+  for (int j = 0; j < kThinN; ++j)
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], d);
+#pragma unroll
+  for (int j = 0; j < kThinN; ++j)
+    if (lane == j) part[warp][j] = acc[j];
+  __syncthreads();
+  if (threadIdx.x >= n) return;
+  float v = 0.0f;
+  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) v += part[w][threadIdx.x];
+  if (bias) v += bias[threadIdx.x];
+  v = nrs_apply_act(v, act);
+  float* dst = c + (size_t)blockIdx.x * n + threadIdx.x;
+  if (beta != 0.0f) v += beta * *dst;
+  *dst = v;
+}
+
 // n <= 16, A stored [k][m] (a weight gradient X^T . dY): a block owns 8 output rows; a warp is
 // 4 k-groups x 8 rows (32-byte segments of A[kk][row0..row0+7]), so the block's 8 warps split k 32
 // ways, and the 32 partial sums of an output are added in k-group order through shared memory.
@@ -437,6 +476,10 @@ int thin_gemm(nrs_ctx* ctx, int ta, int tb, int m, int n, int k, const float* a,
     else if (!ta && tb) NRS_PDL_LAUNCH((thin_k_kernel<false, true>), blocks, 256, 0, ctx->stream, a, b, c, bias, m, n, k, act, beta);
     else if (ta && !tb) NRS_PDL_LAUNCH((thin_k_kernel<true, false>), blocks, 256, 0, ctx->stream, a, b, c, bias, m, n, k, act, beta);
     else NRS_PDL_LAUNCH((thin_k_kernel<true, true>), blocks, 256, 0, ctx->stream, a, b, c, bias, m, n, k, act, beta);
+  } else if (!ta && m <= 4 * ctx->sm_count) {   // (beyond, eight rows a block fill the SMs and B is read eight times less)
+    const int threads = k >= 256 ? 256 : (k + 31) / 32 * 32;
+    if (tb) NRS_PDL_LAUNCH((thin_n_row_kernel<true>), (unsigned)m, threads, 0, ctx->stream, a, b, c, bias, n, k, act, beta);
+    else NRS_PDL_LAUNCH((thin_n_row_kernel<false>), (unsigned)m, threads, 0, ctx->stream, a, b, c, bias, n, k, act, beta);
   } else if (!ta) {
     const unsigned blocks = nrs_blocks((size_t)m, 8);
     if (tb) NRS_PDL_LAUNCH((thin_n_rows_kernel<true>), blocks, 256, 0, ctx->stream, a, b, c, bias, m, n, k, act, beta);
