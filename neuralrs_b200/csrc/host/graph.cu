@@ -329,6 +329,8 @@ std::shared_ptr<FlatStore> flatten_params(const std::vector<NodeP>& params) {
 
 // ---------------------------------------------------------------- graph ops
 
+static void linear_input_grad(nrs_ctx* ctx, const NodeP& x, const NodeP& w, const float* dz, int m, int k, int n);
+
 NodeP matmul(const NodeP& a, const NodeP& b) {
   require_gpu(a, "cuda matmul: lhs");
   require_gpu(b, "cuda matmul: rhs");
@@ -346,7 +348,9 @@ NodeP matmul(const NodeP& a, const NodeP& b) {
     const float* dc = grad_in(self);
     need_values(a);
     GradPlanes dc_planes(ctx, dc, (size_t)m, (size_t)n, tensor_cores && a->requires_grad && b->requires_grad);
-    if (a->requires_grad) {
+    if (a->requires_grad && a->fold_act != NRS_ACT_NONE) {
+      linear_input_grad(ctx, a, b, dc, m, k, n);
+    } else if (a->requires_grad) {
       const bool emit = a->row_planes_wanted && tensor_cores && k % 8 == 0 && !a->view_of && !a->grad_valid && !a->gplanes_hi;
       GradTarget t = grad_target(a);  // dA (+)= dC . B^T
       int st = NRS_ERR_UNSUPPORTED;

@@ -39,9 +39,11 @@
 //
 // The tensor core's f32 accumulation is not round-to-nearest; its error grows
 // linearly with the length of one accumulation chain (about 7e-9 relative per K
-// element), so callers keep a chain at or below kMaxChainK by splitting K across
-// tiles, whose partial results are summed in f32 by tc_splitk_reduce_kernel in a
-// fixed order.
+// element), so no chain is longer than kMaxChainK: a tile with more is walked in
+// chunks of K, whose sums the epilogue adds up in f32, in order, in a buffer of the
+// CTA's own that stays in L2 (a second pass over partial tiles took 135 us for a
+// 4096 x 4096 result).  Products with too few tiles to fill the GPU split K across
+// CTAs, and tc_splitk_reduce_kernel sums their partial results in a fixed order.
 //
 // Every mbarrier wait is bounded: on expiry the kernel records an error code,
 // waits (bounded) for TMA loads it already issued, frees its TMEM and returns.
@@ -77,10 +79,11 @@ struct SmemLayout {
 
 struct SplitInfo {
   int splits;          // K-splits per (tile, batch)
-  int kb_per_split;    // K-slices per split
+  int kb_per_split;    // K-slices per split, or per chunk
+  int chunks;          // > 1 (splits == 1 then): K-chunks that a CTA takes one after the other
   int kb_total;        // K-slices in all
   int batches;
-  float* partial;      // [split][batch][tiles_m*128][n_total] when splits > 1
+  float* partial;      // [split][batch][tiles_m*128][n_total] when splits > 1; [CTA][128][BN] when chunks > 1
   int n_total;
   int rows_total;      // tiles_m * 128
 };
@@ -229,7 +232,7 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
       if (PAIR) tile_m = 2 * tile_m + rank;   // beyond the last row tile: TMA fills zeros
       const int batch = z / sp.splits, split = z - batch * sp.splits;
       int kb_begin = split * sp.kb_per_split;
-      int kb_end = min(sp.kb_total, kb_begin + sp.kb_per_split);
+      int kb_end = sp.chunks > 1 ? sp.kb_total : min(sp.kb_total, kb_begin + sp.kb_per_split);
       if (!pol.clip(tile_m, tile_n, BN, &kb_begin, &kb_end)) continue;
       const int n0 = tile_n * BN + (PAIR ? rank * (BN / 2) : 0);
       // Where the K-slices of this tile lie, stepped along instead of recomputed (the divisions of a recomputation per
@@ -301,40 +304,42 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
         int tile_m, tile_n, z;
         tmap.template decode<BN>(t, &tile_m, &tile_n, &z);
         const int split = z % sp.splits;
-        int kb_begin = split * sp.kb_per_split, kb_end = min(sp.kb_total, kb_begin + sp.kb_per_split);
+        int kb_begin = split * sp.kb_per_split, kb_end = sp.chunks > 1 ? sp.kb_total : min(sp.kb_total, kb_begin + sp.kb_per_split);
         if (!pol.clip(tile_m, tile_n, BN, &kb_begin, &kb_end)) continue;
-        const int nkb = kb_end - kb_begin;   // >= 1 by construction
-        const uint32_t buf = local & 1u, use = local >> 1;
-        ++local;
-        if (!(PAIR ? mbar_wait_warp_cluster(&acc_empty[buf], (use & 1u) ^ 1u) : mbar_wait_warp(&acc_empty[buf], (use & 1u) ^ 1u))) { ok = false; break; }
-        tc_fence_after_sync();
-        const uint32_t d = tmem_base + buf * (uint32_t)L::kAccCols;
-        for (int i = 0; i < nkb; i += L::kSlices) {
-          // (No tcgen05 fence here: the mbarrier's complete_tx orders the TMA writes before the
-          // UMMAs, and a fence would make the issuing thread wait out the UMMAs in flight.)
-          if (!mbar_wait_warp(&full_bar[s], ph)) { ok = false; break; }
-          const uint32_t slot = smem_u32(smem + s * L::kStage);
-          if (elect_one()) {
+        for (int k0 = kb_begin; k0 < kb_end && ok; k0 += sp.kb_per_split) {
+          const int nkb = min(sp.kb_per_split, kb_end - k0);   // >= 1 by construction
+          const uint32_t buf = local & 1u, use = local >> 1;
+          ++local;
+          if (!(PAIR ? mbar_wait_warp_cluster(&acc_empty[buf], (use & 1u) ^ 1u) : mbar_wait_warp(&acc_empty[buf], (use & 1u) ^ 1u))) { ok = false; break; }
+          tc_fence_after_sync();
+          const uint32_t d = tmem_base + buf * (uint32_t)L::kAccCols;
+          for (int i = 0; i < nkb; i += L::kSlices) {
+            // (No tcgen05 fence here: the mbarrier's complete_tx orders the TMA writes before the
+            // UMMAs, and a fence would make the issuing thread wait out the UMMAs in flight.)
+            if (!mbar_wait_warp(&full_bar[s], ph)) { ok = false; break; }
+            const uint32_t slot = smem_u32(smem + s * L::kStage);
+            if (elect_one()) {
 #pragma unroll
-            for (int sl = 0; sl < L::kSlices; ++sl) {
-              if (sl > 0 && i + sl >= nkb) break;
-              const uint32_t a_hi = slot + sl * L::kSlice;
-              const uint32_t b_hi = a_hi + L::kATile;                 // B_lo follows B_hi directly
-              const uint32_t a_lo = b_hi + 2 * L::kBTile;
+              for (int sl = 0; sl < L::kSlices; ++sl) {
+                if (sl > 0 && i + sl >= nkb) break;
+                const uint32_t a_hi = slot + sl * L::kSlice;
+                const uint32_t b_hi = a_hi + L::kATile;                 // B_lo follows B_hi directly
+                const uint32_t a_lo = b_hi + 2 * L::kBTile;
 #pragma unroll
-              for (int k = 0; k < BK / 8; ++k) {
-                const uint64_t da_hi = desc(kAMn, a_hi, k), db_hi = desc(kBMn, b_hi, k);
-                umma_tf32<PAIR>(d, da_hi, db_hi, idesc_wide, (i | sl | k) != 0);   // hi*hi | hi*lo
-                if (NPLANES == 2) umma_tf32<PAIR>(d + kNarrow, desc(kAMn, a_lo, k), db_hi, idesc_half, 1);   // + lo*hi
+                for (int k = 0; k < BK / 8; ++k) {
+                  const uint64_t da_hi = desc(kAMn, a_hi, k), db_hi = desc(kBMn, b_hi, k);
+                  umma_tf32<PAIR>(d, da_hi, db_hi, idesc_wide, (i | sl | k) != 0);   // hi*hi | hi*lo
+                  if (NPLANES == 2) umma_tf32<PAIR>(d + kNarrow, desc(kAMn, a_lo, k), db_hi, idesc_half, 1);   // + lo*hi
+                }
               }
+              umma_commit<PAIR>(&empty_bar[s]);  // slot reusable once these UMMAs have read it
             }
-            umma_commit<PAIR>(&empty_bar[s]);  // slot reusable once these UMMAs have read it
+            __syncwarp();
+            if (++s == (uint32_t)L::kStages) { s = 0; ph ^= 1u; }
           }
+          if (ok && elect_one()) umma_commit<PAIR>(&acc_full[buf]);
           __syncwarp();
-          if (++s == (uint32_t)L::kStages) { s = 0; ph ^= 1u; }
         }
-        if (ok && elect_one()) umma_commit<PAIR>(&acc_full[buf]);
-        __syncwarp();
       }
       if (!ok && lane == 0) atomicExch(err_flag, kErrMmaWait);
     }
@@ -353,116 +358,135 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
       tmap.template decode<BN>(t, &tile_m, &tile_n, &z);
       if (PAIR) tile_m = 2 * tile_m + rank;
       const int batch = z / sp.splits, split = z - batch * sp.splits;
-      int kb_begin = split * sp.kb_per_split, kb_end = min(sp.kb_total, kb_begin + sp.kb_per_split);
+      int kb_begin = split * sp.kb_per_split, kb_end = sp.chunks > 1 ? sp.kb_total : min(sp.kb_total, kb_begin + sp.kb_per_split);
       if (!pol.clip(tile_m, tile_n, BN, &kb_begin, &kb_end)) continue;   // the same verdict in all three roles
       const int n0 = tile_n * BN;
-      const uint32_t buf = local & 1u, use = local >> 1;
-      ++local;
       [[maybe_unused]] const auto rw = pol.row(tile_m, batch, row);   // index arithmetic under the main loop
-      if (!mbar_wait(&acc_full[buf], use & 1u)) {
-        if (lane == 0) atomicExch(err_flag, kErrEpilogueWait);
-        break;
-      }
-      tc_fence_after_sync();
-      auto hand_back = [&]() {   // to the issuing thread, which a pair has in rank 0
-        __syncwarp();
-        if (lane != 0) return;
-        if constexpr (PAIR) mbar_arrive_cluster(cluster_addr(&acc_empty[buf], 0)); else mbar_arrive(&acc_empty[buf]);
-      };
-      // The warps of a lane quarter share its column blocks out; those without one just hand the accumulator back, and so
-      // do all of a pair's second CTA beyond the last row tile.
-      constexpr int kW = Policy::kCanEmit ? 32 : 16, kBlocks = BN / kW, kStep = Policy::kEpiWarps / 4;
-      const int c_first = kStep == 1 ? 0 : (warp - 2) >> 2;
-      if (c_first >= kBlocks || (PAIR && tile_m * BM >= sp.rows_total)) {
-        hand_back();
-        continue;
-      }
-      const uint32_t acc = tmem_base + buf * (uint32_t)L::kAccCols + ((uint32_t)(q * 32) << 16);
-#pragma unroll 1
-      for (int c = c_first; c < kBlocks; c += kStep) {
-        uint32_t r[kW];
-        // the columns of the first and of the second product (a pair: see kNarrow)
-        const int first = PAIR && NPLANES == 2 && c * kW >= BN / 2 ? BN / 2 + c * kW : c * kW;
-        tmem_ld_32(acc + (uint32_t)first, r);
-        if (NPLANES == 2) {
-          uint32_t r2[kW];
-          tmem_ld_32(acc + (uint32_t)(first + (PAIR ? BN / 2 : BN)), r2);
-          tmem_ld_wait();
-#pragma unroll
-          for (int j = 0; j < kW; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(r2[j]));
-        } else {
-          tmem_ld_wait();
+      for (int k0 = kb_begin; k0 < kb_end && ok; k0 += sp.kb_per_split) {
+        const uint32_t buf = local & 1u, use = local >> 1;
+        ++local;
+        if (!mbar_wait(&acc_full[buf], use & 1u)) {
+          if (lane == 0) atomicExch(err_flag, kErrEpilogueWait);
+          ok = false;
+          break;
         }
-        if (c + kStep >= kBlocks) {
-          // Everything this warp needs is in registers: hand the accumulator back.
-          tc_fence_before_sync();
+        tc_fence_after_sync();
+        auto hand_back = [&]() {   // to the issuing thread, which a pair has in rank 0
+          __syncwarp();
+          if (lane != 0) return;
+          if constexpr (PAIR) mbar_arrive_cluster(cluster_addr(&acc_empty[buf], 0)); else mbar_arrive(&acc_empty[buf]);
+        };
+        // The warps of a lane quarter share its column blocks out; those without one just hand the accumulator back, and so
+        // do all of a pair's second CTA beyond the last row tile.
+        constexpr int kW = Policy::kCanEmit ? 32 : 16, kBlocks = BN / kW, kStep = Policy::kEpiWarps / 4;
+        const int c_first = kStep == 1 ? 0 : (warp - 2) >> 2;
+        if (c_first >= kBlocks || (PAIR && tile_m * BM >= sp.rows_total)) {
           hand_back();
+          continue;
         }
-        if (n0 + c * kW >= sp.n_total) continue;   // padding columns of a ragged last tile
-        if constexpr (!Policy::kCanEmit) {
-          float4 v[4];
-          rows_to_lines(reinterpret_cast<float*>(emit_tile) + (warp - 2) * 512, lane, r, v);
-          const int r0 = q * 32 + (lane >> 2), n = n0 + c * kW + (lane & 3) * 4;
-          if (sp.splits > 1) {
-            float* dst = sp.partial + (((size_t)split * sp.batches + batch) * sp.rows_total + (size_t)tile_m * BM + r0) * sp.n_total + n;
+        const uint32_t acc = tmem_base + buf * (uint32_t)L::kAccCols + ((uint32_t)(q * 32) << 16);
+#pragma unroll 1
+        for (int c = c_first; c < kBlocks; c += kStep) {
+          uint32_t r[kW];
+          // the columns of the first and of the second product (a pair: see kNarrow)
+          const int first = PAIR && NPLANES == 2 && c * kW >= BN / 2 ? BN / 2 + c * kW : c * kW;
+          tmem_ld_32(acc + (uint32_t)first, r);
+          if (NPLANES == 2) {
+            uint32_t r2[kW];
+            tmem_ld_32(acc + (uint32_t)(first + (PAIR ? BN / 2 : BN)), r2);
+            tmem_ld_wait();
 #pragma unroll
-            for (int i = 0; i < 4; ++i, dst += (size_t)8 * sp.n_total) store_guarded(dst, v[i], sp.n_total - n, sp.n_total % 4 == 0);
+            for (int j = 0; j < kW; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(r2[j]));
           } else {
-            pol.epilogue(tile_m, batch, r0, n, v);
+            tmem_ld_wait();
           }
-        } else if (sp.splits > 1) {
-          float* dst = sp.partial + (((size_t)split * sp.batches + batch) * sp.rows_total + (size_t)tile_m * BM + row) * sp.n_total;
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const int n = n0 + c * 32 + j;
-            if (n < sp.n_total) dst[n] = __uint_as_float(r[j]);
+          if (c + kStep >= kBlocks) {
+            // Everything this warp needs is in registers: hand the accumulator back.
+            tc_fence_before_sync();
+            hand_back();
           }
-        } else {
-          float v[32];
-          pol.epilogue(rw, n0 + c * 32, r, v);
-          if (float* cs = pol.colsum_row(tile_m, q)) {
-            // Sum over this warp's 32 rows, one channel per lane: a 32 x 32 transpose-reduce in 31
-            // shuffles (each stage halves the values a lane holds; fixed order, deterministic).
-            float s[32];
+          if (sp.chunks > 1) {   // rows along the lanes: 512 bytes an access; a thread reads what it wrote itself
+            float4* sum = reinterpret_cast<float4*>(sp.partial) + ((size_t)blockIdx.x * (BN / 4) + c * (kW / 4)) * BM + row;
 #pragma unroll
-            for (int j = 0; j < 32; ++j) s[j] = v[j];
-#pragma unroll
-            for (int d = 16; d >= 1; d >>= 1) {
-              const bool up = (lane & d) != 0;
-#pragma unroll
-              for (int i = 0; i < d; ++i) {
-                const float keep = up ? s[i + d] : s[i];
-                const float send = up ? s[i] : s[i + d];
-                s[i] = keep + __shfl_xor_sync(0xffffffffu, send, d);
+            for (int g = 0; g < kW / 4; ++g) {
+              if (k0 != kb_begin) {
+                const float4 o = sum[g * BM];
+                r[4 * g] = __float_as_uint(o.x + __uint_as_float(r[4 * g]));
+                r[4 * g + 1] = __float_as_uint(o.y + __uint_as_float(r[4 * g + 1]));
+                r[4 * g + 2] = __float_as_uint(o.z + __uint_as_float(r[4 * g + 2]));
+                r[4 * g + 3] = __float_as_uint(o.w + __uint_as_float(r[4 * g + 3]));
               }
+              if (k0 + sp.kb_per_split < kb_end)
+                sum[g * BM] = make_float4(__uint_as_float(r[4 * g]), __uint_as_float(r[4 * g + 1]), __uint_as_float(r[4 * g + 2]), __uint_as_float(r[4 * g + 3]));
             }
-            cs[n0 + c * 32 + lane] = s[0];
+            if (k0 + sp.kb_per_split < kb_end) continue;
           }
-          if (emit) {
-            // The staging tile is free once the previous TMA store has read it; the issuer
-            // arrives on emit_bar[0] only after that.
-            const uint32_t ph = emitted & 1u;
-            ++emitted;
-            if (emit_issuer) bulk_wait_read();
-            mbar_arrive(&emit_bar[0]);
-            if (!mbar_wait(&emit_bar[0], ph)) { atomicExch(err_flag, kErrEpilogueWait); ok = false; break; }
-            uint8_t* row_hi = emit_tile + row * 128;
+          if (n0 + c * kW >= sp.n_total) continue;   // padding columns of a ragged last tile
+          if constexpr (!Policy::kCanEmit) {
+            float4 v[4];
+            rows_to_lines(reinterpret_cast<float*>(emit_tile) + (warp - 2) * 512, lane, r, v);
+            const int r0 = q * 32 + (lane >> 2), n = n0 + c * kW + (lane & 3) * 4;
+            if (sp.splits > 1) {
+              float* dst = sp.partial + (((size_t)split * sp.batches + batch) * sp.rows_total + (size_t)tile_m * BM + r0) * sp.n_total + n;
 #pragma unroll
-            for (int g = 0; g < 8; ++g) {
-              const int chunk = (g ^ (row & 7)) * 16;   // 128-byte swizzle: 16-byte chunk index XOR row % 8
-              const float4 h = make_float4(tf32_rn(v[4 * g]), tf32_rn(v[4 * g + 1]), tf32_rn(v[4 * g + 2]), tf32_rn(v[4 * g + 3]));
-              *reinterpret_cast<float4*>(row_hi + chunk) = h;
-              if (NPLANES == 2 && emit == 2)
-                *reinterpret_cast<float4*>(row_hi + BM * 128 + chunk) =
-                    make_float4(v[4 * g] - h.x, v[4 * g + 1] - h.y, v[4 * g + 2] - h.z, v[4 * g + 3] - h.w);
+              for (int i = 0; i < 4; ++i, dst += (size_t)8 * sp.n_total) store_guarded(dst, v[i], sp.n_total - n, sp.n_total % 4 == 0);
+            } else {
+              pol.epilogue(tile_m, batch, r0, n, v);
             }
-            fence_proxy_async();   // generic-proxy writes -> visible to the TMA engine
-            mbar_arrive(&emit_bar[1]);
-            if (emit_issuer) {
-              if (!mbar_wait(&emit_bar[1], ph)) { atomicExch(err_flag, kErrEpilogueWait); ok = false; break; }
-              tma_store_4d(&tm_out_hi, emit_tile, n0 + c * 32, rw.x0, rw.y0, rw.n0);
-              if (NPLANES == 2 && emit == 2) tma_store_4d(&tm_out_lo, emit_tile + BM * 128, n0 + c * 32, rw.x0, rw.y0, rw.n0);
-              bulk_commit();
+          } else if (sp.splits > 1) {
+            float* dst = sp.partial + (((size_t)split * sp.batches + batch) * sp.rows_total + (size_t)tile_m * BM + row) * sp.n_total;
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+              const int n = n0 + c * 32 + j;
+              if (n < sp.n_total) dst[n] = __uint_as_float(r[j]);
+            }
+          } else {
+            float v[32];
+            pol.epilogue(rw, n0 + c * 32, r, v);
+            if (float* cs = pol.colsum_row(tile_m, q)) {
+              // Sum over this warp's 32 rows, one channel per lane: a 32 x 32 transpose-reduce in 31
+              // shuffles (each stage halves the values a lane holds; fixed order, deterministic).
+              float s[32];
+#pragma unroll
+              for (int j = 0; j < 32; ++j) s[j] = v[j];
+#pragma unroll
+              for (int d = 16; d >= 1; d >>= 1) {
+                const bool up = (lane & d) != 0;
+#pragma unroll
+                for (int i = 0; i < d; ++i) {
+                  const float keep = up ? s[i + d] : s[i];
+                  const float send = up ? s[i] : s[i + d];
+                  s[i] = keep + __shfl_xor_sync(0xffffffffu, send, d);
+                }
+              }
+              cs[n0 + c * 32 + lane] = s[0];
+            }
+            if (emit) {
+              // The staging tile is free once the previous TMA store has read it; the issuer
+              // arrives on emit_bar[0] only after that.
+              const uint32_t ph = emitted & 1u;
+              ++emitted;
+              if (emit_issuer) bulk_wait_read();
+              mbar_arrive(&emit_bar[0]);
+              if (!mbar_wait(&emit_bar[0], ph)) { atomicExch(err_flag, kErrEpilogueWait); ok = false; break; }
+              uint8_t* row_hi = emit_tile + row * 128;
+#pragma unroll
+              for (int g = 0; g < 8; ++g) {
+                const int chunk = (g ^ (row & 7)) * 16;   // 128-byte swizzle: 16-byte chunk index XOR row % 8
+                const float4 h = make_float4(tf32_rn(v[4 * g]), tf32_rn(v[4 * g + 1]), tf32_rn(v[4 * g + 2]), tf32_rn(v[4 * g + 3]));
+                *reinterpret_cast<float4*>(row_hi + chunk) = h;
+                if (NPLANES == 2 && emit == 2)
+                  *reinterpret_cast<float4*>(row_hi + BM * 128 + chunk) =
+                      make_float4(v[4 * g] - h.x, v[4 * g + 1] - h.y, v[4 * g + 2] - h.z, v[4 * g + 3] - h.w);
+              }
+              fence_proxy_async();   // generic-proxy writes -> visible to the TMA engine
+              mbar_arrive(&emit_bar[1]);
+              if (emit_issuer) {
+                if (!mbar_wait(&emit_bar[1], ph)) { atomicExch(err_flag, kErrEpilogueWait); ok = false; break; }
+                tma_store_4d(&tm_out_hi, emit_tile, n0 + c * 32, rw.x0, rw.y0, rw.n0);
+                if (NPLANES == 2 && emit == 2) tma_store_4d(&tm_out_lo, emit_tile + BM * 128, n0 + c * 32, rw.x0, rw.y0, rw.n0);
+                bulk_commit();
+              }
             }
           }
         }
@@ -498,9 +522,9 @@ tc_splitk_reduce_kernel(const Policy pol, const SplitInfo sp) {
   pol.store(row_lin / BM, b, row_lin % BM, n, s);
 }
 
-// Chooses the K-split: enough CTAs to fill the GPU, and no accumulation chain longer
-// than kMaxChainK elements when `limit_chain`.
-inline void plan_split(const nrs_ctx* ctx, long tiles, long out_elems, int kb_total, bool limit_chain, int* splits, int* kb_per_split) {
+// Chooses the K-split: enough CTAs to fill the GPU, and no accumulation chain longer than kMaxChainK elements when
+// `limit_chain` (chunks where the tiles fill the GPU anyway).
+inline void plan_split(const nrs_ctx* ctx, long tiles, long out_elems, int kb_total, bool limit_chain, SplitInfo* sp) {
   int s = 1;
   // (More than half a wave of tiles runs unsplit: the second pass over the partial tiles costs more
   // than the idle SMs.)
@@ -510,16 +534,17 @@ inline void plan_split(const nrs_ctx* ctx, long tiles, long out_elems, int kb_to
     // layer at a batch of a few dozen) that the second pass is nothing: there down to 4
     const int shortest = out_elems <= (1 << 15) ? 4 : 16;
     if (s > kb_total / shortest) s = kb_total / shortest;
+    if (s < 1) s = 1;
   }
-  if (limit_chain) {
-    const int need = (kb_total * BK + kMaxChainK - 1) / kMaxChainK;
-    if (s < need) s = need;
-  }
-  if (s < 1) s = 1;
+  const int need = limit_chain ? (kb_total * BK + kMaxChainK - 1) / kMaxChainK : 1;
+  const bool in_chunks = s == 1 && need > 1;
+  if (s < need) s = need;
   int per = (kb_total + s - 1) / s;
   if (per < 1) per = 1;
-  *kb_per_split = per;
-  *splits = (kb_total + per - 1) / per;
+  s = (kb_total + per - 1) / per;
+  sp->kb_per_split = per;
+  sp->splits = in_chunks ? 1 : s;
+  sp->chunks = in_chunks ? s : 1;
 }
 
 // The tile of a launch: its columns, and whether CTAs work in pairs.  kPlans holds the measured clocks per K-slice (3xTF32,
@@ -541,8 +566,9 @@ inline TilePlan plan_tile(const nrs_ctx* ctx, long tiles_m, int n, long batches,
   for (const auto& c : kPlans) {
     if (c.bn > limit || (c.bn > 32 && c.bn / 2 >= n)) continue;   // half of the tile or more would be padding
     const long tiles_n = (n + c.bn - 1) / c.bn;
-    int splits, per;
-    plan_split(ctx, tiles_m * tiles_n * batches, tiles_m * BM * n * batches, kblocks, split_planes, &splits, &per);
+    SplitInfo sp{};
+    plan_split(ctx, tiles_m * tiles_n * batches, tiles_m * BM * n * batches, kblocks, split_planes, &sp);
+    const int splits = sp.splits, per = sp.kb_per_split * sp.chunks;
     const long units = (c.pair ? (tiles_m + 1) / 2 : tiles_m) * tiles_n * batches * splits, slots = ctx->sm_count / (c.pair ? 2 : 1);
     double t = (double)((units + slots - 1) / slots) * ((double)per * c.kb_clk[split_planes ? 0 : 1] + c.tile_clk);
     if (splits > 1) t += 4000.0 + reduce_clk * (double)tiles_m * BM * n * batches;
@@ -587,9 +613,9 @@ int launch(nrs_ctx* ctx, const CUtensorMap& ta_hi, const CUtensorMap& ta_lo, con
   const int tiles_n = (n_total + BN - 1) / BN;
   SplitInfo sp{};
   if (Policy::kMaySplit) {
-    plan_split(ctx, (long)tiles_m * tiles_n * batches, (long)tiles_m * BM * n_total * batches, kb_total, NPLANES == 2, &sp.splits, &sp.kb_per_split);
+    plan_split(ctx, (long)tiles_m * tiles_n * batches, (long)tiles_m * BM * n_total * batches, kb_total, NPLANES == 2, &sp);
   } else {   // tiles whose K ranges differ
-    sp.splits = 1;
+    sp.splits = sp.chunks = 1;
     sp.kb_per_split = kb_total;
   }
   sp.kb_total = kb_total;
@@ -598,9 +624,10 @@ int launch(nrs_ctx* ctx, const CUtensorMap& ta_hi, const CUtensorMap& ta_lo, con
   sp.rows_total = tiles_m * BM;
   sp.partial = nullptr;
   if (splits_out) *splits_out = sp.splits;
-  if (sp.splits > 1) {
+  if (sp.splits > 1 || sp.chunks > 1) {
     void* ws = nullptr;
-    const int st = nrs_ws_slot(ctx, NRS_WS_PARTIAL, (size_t)sp.splits * batches * sp.rows_total * n_total * sizeof(float), &ws);
+    const size_t floats = sp.splits > 1 ? (size_t)sp.splits * batches * sp.rows_total * n_total : (size_t)ctx->sm_count * BM * BN;
+    const int st = nrs_ws_slot(ctx, NRS_WS_PARTIAL, floats * sizeof(float), &ws);
     if (st != NRS_OK) return st;
     sp.partial = (float*)ws;
   }

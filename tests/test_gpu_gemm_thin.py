@@ -50,3 +50,30 @@ def test_gemm_tn_large_output(gpu_ctx, mode):
             assert rel_l2(dc.get(), i * ref) <= TOL[mode]
     finally:
         gpu_ctx.set_math_mode(_lib.MATH_3XTF32)
+
+
+@pytest.mark.parametrize("m,n,k", [(1300, 1000, 8300), (2500, 130, 4100), (1408, 1024, 12288)])
+def test_gemm_long_reduction_in_chunks(gpu_ctx, oracle64, m, n, k):
+    """Reductions beyond one accumulation chain with enough tiles to fill the GPU; every operand order, added to C."""
+    rng = np.random.default_rng(k)
+    a, b = rng.normal(size=(m, k)).astype(np.float32), rng.normal(size=(k, n)).astype(np.float32)
+    bias, c0 = rng.normal(size=n).astype(np.float32), rng.normal(size=(m, n)).astype(np.float32)
+    rows = np.r_[0:3, 127:130, m - 2:m]
+    ref = oracle64.matmul_fwd(a[rows], b)
+    for ta, tb in ((0, 0), (0, 1), (1, 0)):
+        da, db, dc = Dev(gpu_ctx, a.T if ta else a), Dev(gpu_ctx, b.T if tb else b), Dev(gpu_ctx, c0)
+        call(gpu_ctx, "nrs_gemm", ta, tb, m, n, k, da, db, dc, None, 0, F(1))
+        assert rel_l2(dc.get()[rows], ref + c0[rows]) <= 5e-5
+    call(gpu_ctx, "nrs_gemm", 1, 0, m, n, k, da, db, dc, Dev(gpu_ctx, bias), 1, F(0))
+    assert rel_l2(dc.get()[rows], np.maximum(ref + bias, 0)) <= 5e-5
+
+
+def test_conv_long_reduction_in_chunks(gpu_ctx, oracle64):
+    rng = np.random.default_rng(9)
+    n, ci, h, co = 16, 4100, 10, 330
+    x, w = rng.normal(size=(n, ci, h, h)).astype(np.float32), rng.normal(size=(co, ci, 1, 1)).astype(np.float32)
+    y = Dev(gpu_ctx, shape=(n, co, h, h))
+    call(gpu_ctx, "nrs_conv2d_fwd", Dev(gpu_ctx, x), Dev(gpu_ctx, w), None, y, n, ci, h, h, co, 1, 1, 1, 0, 0)
+    got = y.get()
+    for i in (0, n - 1):
+        assert rel_l2(got[i], oracle64.matmul_fwd(w[:, :, 0, 0], x[i].reshape(ci, h * h))) <= 5e-5
