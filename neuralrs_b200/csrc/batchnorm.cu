@@ -328,7 +328,7 @@ bn_normalize_planes_kernel(const float* __restrict__ x, const float* __restrict_
   img::tile_to_planes<SPLIT>(tile, g, p0, c0, hi, lo);
 }
 
-// dx (overwritten) with its NHWC planes, and chan_partial[tile of 128 pixels][c], its sums over the tile.
+// dx (overwritten; null: planes only) with its NHWC planes, and chan_partial[tile of 128 pixels][c], its sums over the tile.
 template <bool SPLIT, bool RELU>
 __global__ void __launch_bounds__(kThreads)
 bn_dx_planes_kernel(const float* __restrict__ gr, const float* __restrict__ x, const float* __restrict__ mean,
@@ -365,7 +365,7 @@ bn_dx_planes_kernel(const float* __restrict__ gr, const float* __restrict__ x, c
       if (RELU) gi = fmaf(ga, h, be) > 0.0f ? gi : 0.0f;
       const bool live = ok && px.live[s];
       const float r = !live ? 0.0f : training ? is * (gi * ga - m1 - h * m2) : gi * ga * is;
-      if (live) dx[px.at[s] + (size_t)c * g.hw] = r;
+      if (live && dx) dx[px.at[s] + (size_t)c * g.hw] = r;
       tile[cl][s * 32 + lane] = r;
       total += r;
     }
@@ -510,7 +510,7 @@ int bn_backward(nrs_ctx* ctx, const char* who, const float* g, const float* xhat
   NRS_REQUIRE(ctx, check_dims(n, c, hw), NRS_ERR_SHAPE, "%s: bad shape [%d,%d,%d]", who, n, c, hw);
   NRS_REQUIRE(ctx, (dgamma == nullptr) == (dbeta == nullptr), NRS_ERR_ARG, "%s: dgamma and dbeta must be given together", who);
   NRS_REQUIRE(ctx, g && xhat && istd && gamma && (!relu || beta), NRS_ERR_ARG, "%s: null tensor", who);
-  if (!dx && !dgamma) return NRS_OK;
+  if (!dx && !hi && !dgamma) return NRS_OK;
   NrsProfScope prof(ctx, NRS_PROF_BATCHNORM, 12.0 * (double)n * c * hw);   // g, xhat in; dx out
   const bool need_sums = dgamma || training;
   const int splits = need_sums ? plan_splits(ctx, n, c, hw) : 1;
@@ -522,7 +522,7 @@ int bn_backward(nrs_ctx* ctx, const char* who, const float* g, const float* xhat
   float* count_slot = (float*)(sums + c);
   // with shared statistics dx needs the sums over every process's shard; the parameter gradients keep this
   // process's own sums (they are summed across ranks with all other gradients)
-  const bool shared = training && dx && ctx->stat_sync.all_reduce_sum != nullptr;
+  const bool shared = training && (dx || hi) && ctx->stat_sync.all_reduce_sum != nullptr;
   if (need_sums) {
     const int sp = relu ? launch_pair<false, true>(ctx, g, xhat, partial, n, c, hw, splits, gamma, beta, nullptr, mean, istd)
                         : launch_pair<false, false>(ctx, g, xhat, partial, n, c, hw, splits, nullptr, nullptr, nullptr, mean, istd);
@@ -531,7 +531,7 @@ int bn_backward(nrs_ctx* ctx, const char* who, const float* g, const float* xhat
                    c, splits, accumulate_params);
     NRS_LAUNCHED(ctx);
   }
-  if (!dx) return NRS_OK;
+  if (!dx && !hi) return NRS_OK;
   if (shared) {
     NRS_PDL_LAUNCH(bn_set_count_kernel, 1, 32, 0, ctx->stream, count_slot, (float)((double)n * hw));
     NRS_LAUNCHED(ctx);

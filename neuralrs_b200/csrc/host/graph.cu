@@ -144,6 +144,7 @@ static NodeP make_out(nrs_ctx* ctx, const std::vector<size_t>& shape, std::vecto
   out->ctx = ctx;
   out->shape = shape;
   out->data = dalloc(ctx, out->len());
+  out->internal = ctx->internal_graph;
   out->parents = std::move(parents);
   return out;
 }
@@ -633,7 +634,7 @@ static void conv_backward(Node* self, const NodeP& x, const NodeP& w, const Node
         ghi = dalloc(ctx, xr->len());
         if (ctx->math_mode == NRS_MATH_3XTF32) glo = dalloc(ctx, xr->len());
       }
-      ctx->out_extras[t.ptr] = NrsOutExtras{xr->data, ghi, glo};
+      ctx->out_extras[t.ptr] = NrsOutExtras{xr->data, ghi, glo, ghi && xr->internal && xr->grad_planes_suffice};
       // ... and per-tile channel sums of the masked gradient, for the producer's bias gradient.
       const size_t pixels = (size_t)n * h * wd;
       const int cap = (int)(4 * (pixels / 64 + 2));
@@ -764,6 +765,8 @@ NodeP conv2d_act(const NodeP& x, const NodeP& w, const NodeP& b, size_t stride, 
   // of the channel count: whole groups of eight only)
   const bool dy_planes = s <= 8 && !(patches && (long)n * oh * ow < kNrsPatchMinPixels);
   out->wants_grad_planes = (act == NRS_ACT_RELU || act == NRS_ACT_NONE) && dy_planes && co % 8 == 0;
+  // (the tensor-core weight gradient splits at most 65535 ways, 4096 pixels and up each)
+  out->grad_planes_suffice = out->wants_grad_planes && planes_possible(ctx) && (long)n * oh * ow < (1L << 27);
   out->backward_fn = [self, x, w, b, n, ci, h, wd, co, kh, kw, s, p, act, dy_planes]() {
     nrs_ctx* ctx = self->ctx;
     const float* dy = grad_in(self);
@@ -868,8 +871,11 @@ NodeP maxpool2d(const NodeP& x, size_t kernel, size_t stride, bool emit_planes) 
       // self->data (the pooled maximum) is > 0 exactly where the ReLU let the winner through.
       float* partial = k == 2 ? dalloc(ctx, nrs_stage_masked_partial_rows(n, h, w) * (size_t)c) : nullptr;
       int partial_rows = 0;
-      check(ctx, nrs_tc_stage_masked(ctx, 1, g, self->data, (const int32_t*)am, n, c, h, w, k, t.ptr, phi, plo, partial,
+      // even images of 2 x 2 windows: the kernel that makes the channel sums runs
+      const bool values = !(phi && partial && h % 2 == 0 && w % 2 == 0 && xr->internal && xr->grad_planes_suffice);
+      check(ctx, nrs_tc_stage_masked(ctx, 1, g, self->data, (const int32_t*)am, n, c, h, w, k, values ? t.ptr : nullptr, phi, plo, partial,
                                      &partial_rows));
+      if (!values && partial_rows == 0) fail(NRS_ERR_CUDA, "cuda maxpool: channel sums missing");
       if (partial && partial_rows == 0) { nrs_free(ctx, partial); partial = nullptr; }
       xr->gplanes_hi = phi;
       xr->gplanes_lo = plo;
@@ -1103,6 +1109,7 @@ NodeP batchnorm_nd(const NodeP& x, const NodeP& gamma, const NodeP& beta, const 
         xr->gchan_rows = nrs_batchnorm_tiles(n, hw);
         xr->gchan_partial = partial = dalloc(ctx, (size_t)xr->gchan_rows * c);
         xr->grad_premasked = true;   // there is no mask
+        if (xr->internal && xr->grad_planes_suffice) dx = nullptr;
       }
     }
     check(ctx, nrs_batchnorm_bwd_from_x(ctx, g, x->data, mean, istd, gamma->data, beta->data, dx, dg, db, n, c, hw, training ? 1 : 0,
@@ -1238,7 +1245,7 @@ NodeP linear_act(const NodeP& x, const NodeP& w, const NodeP& b, int act, bool e
     e.hi = dalloc(ctx, out->len());
     if (ctx->math_mode == NRS_MATH_3XTF32) e.lo = dalloc(ctx, out->len());
   }
-  out->internal = reader_cols > 0;
+  if (reader_cols > 0) out->internal = true;
   e.skip_c_unsplit = e.lo && act == NRS_ACT_GELU && values_as_planes_only(ctx, (size_t)m, (size_t)n, reader_cols);
   const int st = pre || e.hi ? nrs_gemm_extras(ctx, 0, 0, m, n, k, x->data, w->data, out->data, b->data, act, 0.0f, &e) : NRS_ERR_UNSUPPORTED;
   if (st == NRS_OK && e.hi) {

@@ -62,6 +62,9 @@ struct Node {
   // (grad_premasked), together with its NHWC planes (gplanes_*, freed with the node).  A batch normalisation above
   // a convolution without an activation hands back its gradient the same way (there is no mask then).
   bool relu_folded = false, wants_grad_planes = false, grad_premasked = false;
+  // With the channel sums those planes are all that the convolution's backward pass reads, for certain: on an internal
+  // node the gradient itself is then not written.
+  bool grad_planes_suffice = false;
   float* gplanes_hi = nullptr;
   float* gplanes_lo = nullptr;
   // With a premasked gradient: per-block channel sums of it ([rows][channels]), which the
@@ -81,7 +84,7 @@ struct Node {
   // consumes it lets its input-gradient kernel write them (gplanes_*, registered under the gradient's address).
   bool row_planes_wanted = false;
 
-  // The result of a step inside a composite layer, which no caller holds: values or a gradient that are read as planes
+  // The result of a step inside a composite layer or a native trainer, which no caller holds: values or a gradient that are read as planes
   // only need not be written besides.  planes_only: `data` was left out (3xTF32: it is planes_hi + planes_lo exactly).
   bool internal = false, planes_only = false;
 

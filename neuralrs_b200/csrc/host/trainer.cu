@@ -228,6 +228,11 @@ NodeP linear_layer(nrs_trainer* t, const NodeP& h, const NodeP& w, const NodeP& 
 }
 
 NodeP forward(nrs_trainer* t, const NodeP& x, const int32_t* ids_dev, size_t batch) {
+  struct Internal {   // the nodes of a step are the trainer's own
+    nrs_ctx* c; const bool was;
+    explicit Internal(nrs_ctx* c_) : c(c_), was(c_->internal_graph) { c->internal_graph = true; }
+    ~Internal() { c->internal_graph = was; }
+  } internal(t->ctx);
   NodeP h = x;
   size_t pi = 0, bi = 0;
   for (size_t li = 0; li < t->layers.size(); ++li) {

@@ -69,6 +69,7 @@ struct NrsOutExtras {
   const float* relu_mask_src;   // NCHW tensor of out's shape: out = relu_mask_src > 0 ? out : 0 (or null)
   float* hi;                    // NHWC TF32 planes of the (masked) result, or null
   float* lo;                    // residual plane (3xTF32), or null
+  bool planes_suffice = false;  // the result itself need not be written where its planes and channel sums are
 };
 
 // Request for per-tile channel sums of a convolution kernel's (masked) output, keyed by the output
@@ -153,6 +154,7 @@ struct nrs_ctx {
   cudaStream_t own_stream = nullptr;
   cudaStream_t stream = nullptr;
   int math_mode = NRS_MATH_3XTF32;
+  bool internal_graph = false;   // nodes made now belong to a native trainer: nobody else reads them (see nrs::Node::internal)
   int sm_count = 148;
   uint64_t launches = 0;
   std::string err;

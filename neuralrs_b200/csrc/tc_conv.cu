@@ -53,6 +53,7 @@ struct ConvPolicy {
   float* out_lo;
   // optional: [tiles_m * 4][n_ch_out] sums of the finished values over each epilogue warp's 32 rows
   float* colsum_partial;
+  bool skip_out;   // the finished values leave as planes and channel sums only (a K-split's second pass writes them still)
 
   __device__ __forceinline__ uint32_t a_slice_bytes() const { return slice_bytes; }
   __device__ __forceinline__ void origin(int tile_m, int* x0, int* y0, int* n0) const {
@@ -195,6 +196,7 @@ struct ConvPolicy {
 #pragma unroll
       for (int j = 0; j < 32; ++j) v[j] = mv[j] > 0.0f ? v[j] : 0.0f;
     }
+    if (FULL && skip_out) return;
 #pragma unroll
     for (int j = 0; j < 32; ++j)
       if (FULL || j < nch) dst[(size_t)j * plane] = v[j];
@@ -315,6 +317,7 @@ int conv_common(nrs_ctx* ctx, ConvPlan& p) {
   auto colsum = ctx->colsum_requests.find(p.out);
   if (whole && colsum != ctx->colsum_requests.end() && !p.accumulate && tiles_m * 4 <= colsum->second.cap_rows)
     pol.colsum_partial = colsum->second.partial;
+  pol.skip_out = pol.colsum_partial && pol.out_hi && extras->second.planes_suffice;
 
   // stage the activation: per image [C][H*W] -> [H*W][C] planes
   void *a_hi = nullptr, *a_lo = nullptr;
