@@ -5,6 +5,8 @@
 #include "nrs_internal.h"
 
 #include <cstring>
+#include <mutex>
+#include <vector>
 
 static thread_local std::string g_no_ctx_error;
 
@@ -63,20 +65,51 @@ int nrs_ws_slot(nrs_ctx* ctx, int slot, size_t bytes, void** out) {
   return NRS_OK;
 }
 
+// One page-locked block per context: the device error word, and behind it the slot of small read-backs.  Pinning takes
+// 1 to 3 ms a call whatever the size, so blocks of closed contexts are kept for the next ones (at most kIdlePinned, by
+// any thread; every device may use them).
+namespace {
+constexpr size_t kBounceBytes = 256 * 1024, kErrBytes = 4096;
+constexpr size_t kIdlePinned = 16;
+std::mutex g_pinned_lock;
+std::vector<void*>& idle_pinned() {
+  static auto* v = new std::vector<void*>();   // (not destroyed: contexts may close during static destruction)
+  return *v;
+}
+}  // namespace
+
+static int pinned_block(nrs_ctx* ctx) {
+  if (ctx->pinned) return NRS_OK;
+  void* p = nullptr;
+  {
+    std::lock_guard<std::mutex> g(g_pinned_lock);
+    if (!idle_pinned().empty()) { p = idle_pinned().back(); idle_pinned().pop_back(); }
+  }
+  if (!p) NRS_CUDA(ctx, cudaHostAlloc(&p, kErrBytes + kBounceBytes, cudaHostAllocMapped | cudaHostAllocPortable));
+  *(int*)p = 0;
+  ctx->pinned = p;
+  return NRS_OK;
+}
+
+void nrs_pinned_release(nrs_ctx* ctx) {   // the context's stream is idle
+  if (!ctx->pinned) return;
+  std::lock_guard<std::mutex> g(g_pinned_lock);
+  if (idle_pinned().size() < kIdlePinned) idle_pinned().push_back(ctx->pinned);
+  else cudaFreeHost(ctx->pinned);
+  ctx->pinned = nullptr;
+  ctx->err_host = nullptr;
+  ctx->err_flag = nullptr;
+}
+
 // The word lives in mapped host memory: only a kernel that gives up writes it (across the bus, once), and reading it
 // after a synchronisation is a plain load instead of a copy and a second synchronisation (some 10 us per read-back).
 int nrs_err_flag(nrs_ctx* ctx, int** out) {
   if (!ctx->err_flag) {
-    void* h = nullptr;
-    NRS_CUDA(ctx, cudaHostAlloc(&h, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
-    *(int*)h = 0;
+    const int st = pinned_block(ctx);
+    if (st != NRS_OK) return st;
     void* d = nullptr;
-    const cudaError_t e = cudaHostGetDevicePointer(&d, h, 0);
-    if (e != cudaSuccess) {
-      cudaFreeHost(h);
-      return nrs_fail(ctx, NRS_ERR_CUDA, "error word: cudaHostGetDevicePointer failed: %s", cudaGetErrorString(e));
-    }
-    ctx->err_host = (volatile int*)h;
+    NRS_CUDA(ctx, cudaHostGetDevicePointer(&d, ctx->pinned, 0));
+    ctx->err_host = (volatile int*)ctx->pinned;
     ctx->err_flag = (int*)d;
   }
   *out = ctx->err_flag;
@@ -133,20 +166,18 @@ NrsProfScope::~NrsProfScope() {
 
 // Device -> host: small reads into pageable memory go through a pinned slot of the context's own (one copy, one wait,
 // one memcpy: 64 KB 23 -> 15 us); larger ones, and pinned destinations (nrs_host_alloc), are one asynchronous copy.
-namespace {
-constexpr size_t kBounceBytes = 256 * 1024;
-}
-
 static int nrs_bounce_d2h(nrs_ctx* ctx, void* dst, const void* src, size_t bytes) {
   if (bytes > kBounceBytes) {
     NRS_CUDA(ctx, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
     NRS_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     return NRS_OK;
   }
-  if (!ctx->bounce) NRS_CUDA(ctx, cudaHostAlloc(&ctx->bounce, kBounceBytes, cudaHostAllocPortable));
-  NRS_CUDA(ctx, cudaMemcpyAsync(ctx->bounce, src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+  const int st = pinned_block(ctx);
+  if (st != NRS_OK) return st;
+  void* bounce = (uint8_t*)ctx->pinned + kErrBytes;
+  NRS_CUDA(ctx, cudaMemcpyAsync(bounce, src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
   NRS_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  std::memcpy(dst, ctx->bounce, bytes);
+  std::memcpy(dst, bounce, bytes);
   return NRS_OK;
 }
 
@@ -245,13 +276,13 @@ int nrs_destroy(nrs_ctx* ctx) {
   if (!ctx) return NRS_OK;
   cudaSetDevice(ctx->device);
   cudaStreamSynchronize(ctx->stream);
-  for (auto& kv : ctx->pool.free_blocks) cudaFree(kv.second);
-  for (auto& kv : ctx->pool.live) cudaFree(kv.first);
+  for (auto& kv : ctx->pool.free_blocks) if (kv.first > NrsPool::kSmall) cudaFree(kv.second);
+  for (auto& kv : ctx->pool.live) if (kv.second > NrsPool::kSmall) cudaFree(kv.first);
+  for (void* s : ctx->pool.slabs) cudaFree(s);
   nrs_weight_set_clear(ctx);
   if (ctx->workspace) cudaFree(ctx->workspace);
   for (int i = 0; i < NRS_WS_COUNT; ++i) if (ctx->ws_slot[i]) cudaFree(ctx->ws_slot[i]);
-  if (ctx->err_host) cudaFreeHost((void*)ctx->err_host);
-  if (ctx->bounce) cudaFreeHost(ctx->bounce);
+  nrs_pinned_release(ctx);
   nrs_folds_free(ctx);
   if (ctx->fold_ticket) cudaFree(ctx->fold_ticket);
   for (auto& r : ctx->prof_records) { cudaEventDestroy(r.start); cudaEventDestroy(r.stop); }
@@ -296,20 +327,33 @@ int nrs_alloc(nrs_ctx* ctx, size_t bytes, int zero, void** dptr) {
     p = it->second;
     ctx->pool.free_blocks.erase(it);
   } else {
-    cudaError_t e = cudaMalloc(&p, want);
-    if (e != cudaSuccess) {
-      (void)cudaGetLastError();
-      // Give cached blocks back to the driver and retry once.
-      for (auto& kv : ctx->pool.free_blocks) { cudaFree(kv.second); ctx->pool.bytes_reserved -= kv.first; }
-      ctx->pool.free_blocks.clear();
-      e = cudaMalloc(&p, want);
+    NrsPool& pool = ctx->pool;
+    const bool small = want <= NrsPool::kSmall;
+    if (small && pool.slab_used + want <= NrsPool::kSlab) {
+      p = (uint8_t*)pool.slabs.back() + pool.slab_used;
+      pool.slab_used += want;
+    } else {
+      const size_t ask = small ? NrsPool::kSlab : want;
+      cudaError_t e = cudaMalloc(&p, ask);
       if (e != cudaSuccess) {
         (void)cudaGetLastError();
-        return nrs_fail(ctx, NRS_ERR_ALLOC, "nrs_alloc: cudaMalloc(%zu) failed: %s", want,
-                        cudaGetErrorString(e));
+        // Give cached blocks back to the driver and retry once.
+        for (auto it = pool.free_blocks.upper_bound(NrsPool::kSmall); it != pool.free_blocks.end(); it = pool.free_blocks.erase(it)) {
+          cudaFree(it->second);
+          pool.bytes_reserved -= it->first;
+        }
+        e = cudaMalloc(&p, ask);
+        if (e != cudaSuccess) {
+          (void)cudaGetLastError();
+          return nrs_fail(ctx, NRS_ERR_ALLOC, "nrs_alloc: cudaMalloc(%zu) failed: %s", ask, cudaGetErrorString(e));
+        }
+      }
+      pool.bytes_reserved += ask;
+      if (small) {
+        pool.slabs.push_back(p);
+        pool.slab_used = want;
       }
     }
-    ctx->pool.bytes_reserved += want;
   }
   ctx->pool.live[p] = want;
   if (zero) NRS_CUDA(ctx, cudaMemsetAsync(p, 0, bytes, ctx->stream));

@@ -28,6 +28,8 @@ static_assert(sizeof(FoldBatch) <= 8000, "the job table is a kernel parameter");
 
 __device__ __forceinline__ void put(float* dst, float v, int accumulate) { *dst = accumulate ? *dst + v : v; }
 
+__device__ __forceinline__ float* column_dst(const NrsFoldJob& j, int c) { return j.dst2 && c >= j.cols1 ? j.dst2 + (c - j.cols1) : j.dst + c; }
+
 // dst[c] (+)= sum over rows of src[r*stride + c].  A block takes 32 columns of a row split: its eight warps every eighth
 // row, four rows in flight per thread, combined in warp order; with several splits the last block of a column group to
 // arrive adds the splits in order.
@@ -54,7 +56,7 @@ __device__ void fold_columns(const NrsFoldJob& j, unsigned blk, float* sm) {
     float sum = 0.0f;
 #pragma unroll
     for (int w = 0; w < 8; ++w) sum += sm[w * 32 + lane];
-    if (j.splits == 1) put(j.dst + c, sum, j.accumulate);
+    if (j.splits == 1) put(column_dst(j, c), sum, j.accumulate);
     else j.scratch[(size_t)split * j.cols + c] = sum;
   }
   if (j.splits == 1) return;
@@ -67,7 +69,7 @@ __device__ void fold_columns(const NrsFoldJob& j, unsigned blk, float* sm) {
   if (warp == 0 && c < j.cols) {
     float sum = 0.0f;
     for (int z = 0; z < j.splits; ++z) sum += __ldcg(j.scratch + (size_t)z * j.cols + c);
-    put(j.dst + c, sum, j.accumulate);
+    put(column_dst(j, c), sum, j.accumulate);
   }
   if (threadIdx.x == 0) j.tickets[grp] = 0;
 }
@@ -245,7 +247,7 @@ void nrs_folds_free(nrs_ctx* ctx) {
 
 int nrs_folds_settle(nrs_ctx* ctx, const float* dst) {
   for (const NrsFoldJob& j : ctx->folds.jobs)
-    if (j.dst == dst) return nrs_folds_flush(ctx);
+    if (j.dst == dst || (j.dst2 && j.dst2 == dst)) return nrs_folds_flush(ctx);
   return NRS_OK;
 }
 
@@ -306,15 +308,18 @@ int nrs_fold_submit(nrs_ctx* ctx, NrsFoldJob job) {
     if (st != NRS_OK) return st;
   }
   int st = nrs_folds_settle(ctx, job.dst);   // a second share of the same gradient: the first one goes ahead of it
+  if (st == NRS_OK && job.dst2) st = nrs_folds_settle(ctx, job.dst2);
   if (st != NRS_OK) return st;
   f.tickets_used += need;
   f.jobs.push_back(job);
   return NRS_OK;
 }
 
-int nrs_fold_columns(nrs_ctx* ctx, const float* src, float* dst, int rows, int cols, int stride, int accumulate) {
+static int fold_columns_to(nrs_ctx* ctx, const float* src, float* dst, float* dst2, int cols1, int rows, int cols, int stride, int accumulate) {
   if (cols <= 0) return NRS_OK;
   NrsFoldJob j{};
+  j.dst2 = dst2;
+  j.cols1 = cols1;
   j.kind = NRS_FOLD_COLUMNS;
   j.src = src;
   j.dst = dst;
@@ -333,4 +338,11 @@ int nrs_fold_columns(nrs_ctx* ctx, const float* src, float* dst, int rows, int c
     j.scratch = p;
   }
   return nrs_fold_submit(ctx, j);
+}
+
+int nrs_fold_columns(nrs_ctx* ctx, const float* src, float* dst, int rows, int cols, int stride, int accumulate) {
+  return fold_columns_to(ctx, src, dst, nullptr, cols, rows, cols, stride, accumulate);
+}
+int nrs_fold_column_pair(nrs_ctx* ctx, const float* src, float* dst, float* dst2, int rows, int cols, int stride, int accumulate) {
+  return fold_columns_to(ctx, src, dst, dst2, cols, rows, 2 * cols, stride, accumulate);
 }

@@ -16,3 +16,5 @@ int nrs_fold_partial(nrs_ctx* ctx, int ws_slot, size_t bytes, float** out);
 int nrs_fold_submit(nrs_ctx* ctx, NrsFoldJob job);
 // dst[c] (+)= sum over rows of src[r*stride + c]; src must stay as it is until the fold has run.
 int nrs_fold_columns(nrs_ctx* ctx, const float* src, float* dst, int rows, int cols, int stride, int accumulate);
+// The same for two results side by side: columns [0, cols) to dst, [cols, 2*cols) to dst2.
+int nrs_fold_column_pair(nrs_ctx* ctx, const float* src, float* dst, float* dst2, int rows, int cols, int stride, int accumulate);

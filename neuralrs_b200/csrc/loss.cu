@@ -257,7 +257,10 @@ int run_ce(nrs_ctx* ctx, const char* who, const float* logits, const float* targ
   const float inv_div = 1.0f / (float)divisor;
   // (rows that a register kernel takes: from 32 MB per tensor, beyond what the L2 cache holds of logits and gradient;
   // [4096][1000] 16.5 us there against 19 here, [16384][1000] 55 against 48)
-  if (rowpipe::applies(batch, classes, classes % 4 == 0 && classes <= 1024, 1u << 23, {logits, target, grad})) {
+  // Crossover against the warp-per-row kernels: [16384][1000] 50 us, 46 here; [16384][1001] 128, 102; [3000][1001] 16, 24;
+  // [20000][700] 44, 52 and [40000][777] 218, 233 (lanes idle, two warps to a row).
+  if ((size_t)batch * classes >= (size_t)1 << 23 && rowpipe::fill(classes) >= 0.75 && (classes <= 512 || classes >= 960) &&
+      rowpipe::applies(batch, classes, {logits, target, grad})) {
     rowpipe::Params p{};
     p.in[0] = logits; p.in[1] = target;
     p.n_in = p.n_buf = target ? 2 : 1;

@@ -549,7 +549,11 @@ int layernorm_fwd(nrs_ctx* ctx, const char* who, const float* a, const float* b,
   if (rows == 0) return NRS_OK;
   NRS_REQUIRE(ctx, a && gamma && beta && y, NRS_ERR_ARG, "%s: null tensor", who);
   const int vpl = vec_vpl(f, {a, b, gamma, beta, y, xhat, y_hi, y_lo});
-  if (!(y_hi && vpl) && rowpipe::applies(rows, f, vpl != 0, 1u << 20, {a, b, gamma, beta, y, xhat})) {
+  // Measured crossovers: [16384][1000] 41 us on the register kernel, 35 here; [4096][256] 4.6, 6.6; [20000][700] (a
+  // third of the lanes idle) 39, 40.  Scalar loops: [5000][1502] 30, 25; [16384][1001] 69, 72, with a residual 101, 78.
+  const size_t elems = (size_t)rows * f;
+  const bool pipe = elems >= 6000000 && rowpipe::fill(f) >= 0.75 && (vpl || f >= (b ? 960 : 1400));
+  if (!(y_hi && vpl) && pipe && rowpipe::applies(rows, f, {a, b, gamma, beta, y, xhat})) {
     rowpipe::Params p{};
     p.in[0] = a; p.in[1] = b; p.n_in = b ? 2 : 1; p.n_buf = 2;
     p.out[0] = xhat; p.out_buf[0] = 0;
@@ -575,8 +579,7 @@ int layernorm_fwd(nrs_ctx* ctx, const char* who, const float* a, const float* b,
 
 // partial[part][2][f] -> dgamma, dbeta.
 int fold_params(nrs_ctx* ctx, const float* partial, float* dgamma, float* dbeta, int f, int parts, int accumulate) {
-  const int st = nrs_fold_columns(ctx, partial, dgamma, parts, f, 2 * f, accumulate);
-  return st != NRS_OK ? st : nrs_fold_columns(ctx, partial + f, dbeta, parts, f, 2 * f, accumulate);
+  return nrs_fold_column_pair(ctx, partial, dgamma, dbeta, parts, f, 2 * f, accumulate);
 }
 
 int layernorm_bwd(nrs_ctx* ctx, const char* who, const float* g, const float* xhat, const float* istd, const float* gamma,
@@ -596,7 +599,8 @@ int layernorm_bwd(nrs_ctx* ctx, const char* who, const float* g, const float* xh
   NRS_REQUIRE(ctx, g && xhat && istd && gamma, NRS_ERR_ARG, "%s: null tensor", who);
   if (!dx && !dgamma) return NRS_OK;
   const int vpl = vec_vpl(f, {g, xhat, gamma, dx, dx2, d_hi, d_lo});
-  if (!(d_hi && vpl) && rowpipe::applies(rows, f, vpl != 0, 1u << 20, {g, xhat, gamma, dx, dx2})) {
+  // (register kernel: [16384][1000] 99 us, 44 here, even at 4 M elements; the scalar loops read g and xhat twice)
+  if (!(d_hi && vpl) && (!vpl || (size_t)rows * f >= (size_t)1 << 22) && rowpipe::applies(rows, f, {g, xhat, gamma, dx, dx2})) {
     rowpipe::Params p{};
     p.in[0] = g; p.in[1] = xhat; p.n_in = p.n_buf = 2;
     p.out[0] = dx; p.out_add[0] = acc1;
@@ -721,7 +725,8 @@ int nrs_softmax_fwd(nrs_ctx* ctx, const float* x, float* y, int rows, int width)
   const int vpl = vec_vpl(width, {x, y});
   // (widths the vector kernel takes stay there at every size: bound by its exponentials and divisions, not by HBM, it
   // does better with a full SM of warps: [16384][1000] 24 us against 54)
-  if (!vpl && rowpipe::applies(rows, width, false, 0, {x, y})) {
+  // Scalar loops: [5000][1502] 28 us, 24 here; [16384][1001] 45, 64; [2000][2050] 18, 29.
+  if (!vpl && width >= 1400 && (size_t)rows * width >= 6000000 && rowpipe::applies(rows, width, {x, y})) {
     rowpipe::Params p{};
     p.in[0] = x; p.n_in = p.n_buf = 1;
     p.out[0] = y;
@@ -744,7 +749,9 @@ int nrs_softmax_bwd(nrs_ctx* ctx, const float* y, const float* g, float* dx, int
   if (rows == 0) return NRS_OK;
   NRS_REQUIRE(ctx, y && g && dx, NRS_ERR_ARG, "nrs_softmax_bwd: null tensor");
   const int vpl = vec_vpl(width, {y, g, dx});
-  if (rowpipe::applies(rows, width, vpl != 0, 1u << 20, {y, g, dx})) {
+  // Only against the scalar loops ([16384][1001] 60 us, 36 here; [10086][518], half of the lanes idle, 12, 14): the
+  // register kernel takes 28 us for [16384][1000], 33 here.
+  if (!vpl && rowpipe::fill(width) >= 0.75 && rowpipe::applies(rows, width, {y, g, dx})) {
     rowpipe::Params p{};
     p.in[0] = y; p.in[1] = g; p.n_in = p.n_buf = 2;
     p.out[0] = dx; p.out_add[0] = accumulate;

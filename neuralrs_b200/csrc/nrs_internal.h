@@ -21,6 +21,11 @@ struct NrsPool {
   std::multimap<size_t, void*> free_blocks;   // rounded size -> block
   std::map<void*, size_t> live;               // block -> rounded size
   size_t bytes_reserved = 0;
+  // Blocks up to kSmall bytes are cut from slabs: cudaMalloc takes 0.3 ms whatever the size, and a small model's first
+  // step asks for dozens of sizes.
+  static constexpr size_t kSmall = (size_t)1 << 20, kSlab = (size_t)16 << 20;
+  std::vector<void*> slabs;
+  size_t slab_used = kSlab;                   // of the last one
   static size_t round_up(size_t bytes) {
     const size_t g = bytes <= (1u << 20) ? 512 : (size_t)1 << 16;
     return (bytes + g - 1) / g * g;
@@ -128,6 +133,7 @@ struct NrsFoldJob {
   const float* src;
   float* dst;
   float* scratch;          // columns with several row splits: [splits][cols]
+  float* dst2;             // columns: those from cols1 on go here (null: all to dst)
   unsigned* tickets;
   unsigned first_block;
   int kind, accumulate, splits, lanes;
@@ -137,6 +143,7 @@ struct NrsFoldJob {
   // weight gradients: the partial tiles' layout (see the kernels)
   int taps_per_group, n_groups, col_blocks, cblocks, group_cols;
   int chunk, n_chunks, jtypes, a_blocks, pack;
+  int cols1;
   int vec;                 // 1x1: outputs written 16 bytes at a time
   int out_cols;            // general kernel, 1x1: the columns are several [co][out_cols] matrices side by side (0: one)
   size_t split_stride;     // floats between two splits
@@ -168,7 +175,7 @@ struct nrs_ctx {
   // Device word the tensor-core kernels set when a bounded wait runs out; read at sync points.
   int* err_flag = nullptr;
   volatile int* err_host = nullptr;  // the same word as the host sees it (mapped memory)
-  void* bounce = nullptr;            // pinned slot for small read-backs into pageable memory, made on first use
+  void* pinned = nullptr;            // page-locked: the error word, and a slot for small read-backs; made on first use
   unsigned* fold_ticket = nullptr;   // arrival counter of kernels whose last block folds the blocks' partial sums
   // Planes registered for a source tensor (keyed by its device pointer); the conv kernels
   // use them instead of staging again.  Whoever registers keeps both alive and unregisters.
@@ -225,6 +232,7 @@ int nrs_workspace(nrs_ctx* ctx, size_t bytes, void** out);
 enum { NRS_WS_A_HI = 0, NRS_WS_A_LO = 1, NRS_WS_B_HI = 2, NRS_WS_B_LO = 3, NRS_WS_PARTIAL = 4, NRS_WS_WGRAD_PARTIAL = 5, NRS_WS_FOLD = 6, NRS_WS_COUNT = 8 };
 int nrs_ws_slot(nrs_ctx* ctx, int slot, size_t bytes, void** out);
 int nrs_err_flag(nrs_ctx* ctx, int** out);
+void nrs_pinned_release(nrs_ctx* ctx);
 // Zero-initialised device counters (kNrsFoldTickets of them) for "the last block to arrive folds the partials"
 // reductions; the folding block resets its counter, so consecutive launches on the context's stream can share
 // them.  Slot 0 serves kernels with one counter, slots 1.. kernels with a counter per column block.

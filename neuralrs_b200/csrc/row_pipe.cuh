@@ -208,14 +208,19 @@ row_pipe_kernel(const Params p, const Op op, int* __restrict__ err_flag) {
   op.template finish<NPL, VEC>(tm, cols, state, reinterpret_cast<float*>(smem_raw + 2048), team, teams);
 }
 
-// Whether a tensor set takes this path: 16-byte aligned bases, rows of at most 8192 columns (one slot of two
-// buffers is then 64 KB), and enough elements: `vector_from` where a register kernel takes the width (the operator's
-// own crossover), 128 K where only the scalar loops do (below, their shorter prologue wins: [64][10] 4 us against 20).
-inline bool applies(int rows, int f, bool vector_kernel_exists, size_t vector_from, std::initializer_list<const void*> ptrs) {
+// Share of a row's lanes x elements that hold columns (see launch()).
+inline double fill(int f) {
+  const int unit = 32 * (f <= 256 ? 8 : 16);
+  return (double)f / ((f + unit - 1) / unit * unit);
+}
+// Whether a tensor set can take this path: 16-byte aligned bases, rows of at most 8192 columns (one slot of two
+// buffers is then 64 KB), 128 K elements (below, a shorter prologue wins: [64][10] 4 us against 20).  The operators add
+// their own crossovers against the register kernels (widths of whole float4s) and the scalar loops (other widths).
+inline bool applies(int rows, int f, std::initializer_list<const void*> ptrs) {
   if (f > 8192 || rows < 1) return false;
   for (const void* q : ptrs)
     if (reinterpret_cast<uintptr_t>(q) & 15) return false;
-  return (size_t)rows * f >= (vector_kernel_exists ? vector_from : (size_t)1 << 17);
+  return (size_t)rows * f >= (size_t)1 << 17;
 }
 
 template <int NPL, int VEC, class Op>
