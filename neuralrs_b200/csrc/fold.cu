@@ -190,12 +190,12 @@ int run(nrs_ctx* ctx, NrsFoldJob* jobs, int n) {
   FoldBatch b{};
   unsigned blocks = 0;
   unsigned ticket = 1;   // slot 0 serves kernels with one counter
-  unsigned* tickets = nullptr;
-  int st = nrs_fold_ticket(ctx, &tickets);
-  if (st != NRS_OK) return st;
+  unsigned* tickets = nullptr;   // made when a job asks for some
   for (int i = 0; i < n; ++i) {
     NrsFoldJob& j = jobs[i];
     if (j.kind == NRS_FOLD_COLUMNS && j.splits > 1) {
+      const int st = tickets ? NRS_OK : nrs_fold_ticket(ctx, &tickets);
+      if (st != NRS_OK) return st;
       j.tickets = tickets + ticket;
       ticket += (unsigned)((j.cols + 31) / 32);
     }

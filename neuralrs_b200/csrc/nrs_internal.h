@@ -248,7 +248,9 @@ extern "C" int nrs_layernorm_bwd_planes(nrs_ctx* ctx, const float* g, const floa
 // TF32 planes of a batch of [rows][K] matrices (tc_stage.cu); see tc_mainloop.cuh for the layouts.
 int nrs_tc_stage(nrs_ctx* ctx, const float* src, float* hi, float* lo, int rows, int K, int ldk, int batch,
                  size_t src_bstride, size_t dst_bstride, bool src_k_by_rows);
-int nrs_tc_stage_image(nrs_ctx* ctx, const float* src, float* hi, float* lo, int n, int c, int hw);
+// NHWC planes of an NCHW tensor [n][c][hw], pixel stride nrs_plane_ld(c) floats (zeros between c and there).
+// chan_partial (hw > 1): [nrs_batchnorm_tiles(n, hw)][c] channel sums of the pixels of each tile.
+int nrs_tc_stage_image(nrs_ctx* ctx, const float* src, float* hi, float* lo, int n, int c, int hw, float* chan_partial = nullptr);
 // Counter window of a per-sample draw of `count` elements (count = samples * per-sample) in blocks of four:
 // first block to use and by how many blocks the stream advances.  Falls back to the plain stream (this
 // process's own draws) when no shard is set, the call is not per-sample, or the shard does not start on a

@@ -14,6 +14,7 @@
 // Reference counterparts: matmul_nn/nt/tn + matmul_nt_splitk
 // (src/cuda/graph/matmul.rs:44-261), bmm kernels (src/cuda/graph/bmm.rs:12-56),
 // conv2d im2col/col2out/out2mm/col2im (src/cuda/nn/conv.rs:27-149).
+#include "fold.h"
 #include "igemm_problems.cuh"
 #include "nrs_internal.h"
 #include "tc_common.cuh"
@@ -631,13 +632,30 @@ int nrs_conv2d_bwd(nrs_ctx* ctx, const float* x, const float* w, const float* dy
     nrs_ctx* c; const void* k; bool* on;
     ~Unlend() { if (*on) c->plane_hints.erase(k); }
   } unlend{ctx, dy, &dy_planes_lent};
+  // With the bias gradient wanted too, dy is staged first, and its channel sums come out of that pass.
+  if (db && !dy_had_planes && ctx->math_mode != NRS_MATH_FP32 && tc::tensor_map_encoder() && stride <= 8 && g.oh * g.ow > 1 &&
+      (size_t)n * g.oh * g.ow < ((size_t)1 << 27) && (dx || (dw && !conv_runs_direct(ctx, n, ci, kh, kw, h, wd, stride, pad)))) {
+    const size_t floats = (size_t)n * g.oh * g.ow * nrs_plane_ld(co);
+    const int tiles = nrs_batchnorm_tiles(n, g.oh * g.ow);
+    void *hi = nullptr, *lo = nullptr;
+    float* partial = nullptr;
+    st = nrs_ws_slot(ctx, NRS_WS_A_HI, floats * sizeof(float), &hi);
+    if (st == NRS_OK && split3) st = nrs_ws_slot(ctx, NRS_WS_A_LO, floats * sizeof(float), &lo);
+    if (st == NRS_OK) st = nrs_fold_partial(ctx, -1, (size_t)tiles * co * sizeof(float), &partial);
+    if (st == NRS_OK) st = nrs_tc_stage_image(ctx, dy, (float*)hi, (float*)lo, n, co, g.oh * g.ow, partial);
+    if (st == NRS_OK) st = nrs_fold_columns(ctx, partial, db, tiles, co, co, accumulate);
+    if (st != NRS_OK) return st;
+    db = nullptr;
+    ctx->plane_hints[dy] = NrsPlanes{(float*)hi, (float*)lo, split3 ? 1 : 0};
+    dy_planes_lent = true;
+  }
   if (dx) {
     NrsProfScope prof(ctx, NRS_PROF_CONV_DGRAD, conv_flop);
     st = ctx->math_mode != NRS_MATH_FP32
              ? nrs_tc_conv_dgrad(ctx, w, dy, dx, n, ci, h, wd, co, kh, kw, stride, pad, accumulate)
              : NRS_ERR_UNSUPPORTED;
     if (st != NRS_OK && st != NRS_ERR_UNSUPPORTED) return st;
-    if (st == NRS_OK && dw && !dy_had_planes && ctx->ws_slot[NRS_WS_A_HI] && (!split3 || ctx->ws_slot[NRS_WS_A_LO])) {
+    if (st == NRS_OK && dw && !dy_had_planes && !dy_planes_lent && ctx->ws_slot[NRS_WS_A_HI] && (!split3 || ctx->ws_slot[NRS_WS_A_LO])) {
       ctx->plane_hints[dy] = NrsPlanes{(float*)ctx->ws_slot[NRS_WS_A_HI], split3 ? (float*)ctx->ws_slot[NRS_WS_A_LO] : nullptr, split3 ? 1 : 0};
       dy_planes_lent = true;
     }

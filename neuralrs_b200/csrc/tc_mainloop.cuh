@@ -664,8 +664,6 @@ int launch(nrs_ctx* ctx, const CUtensorMap& ta_hi, const CUtensorMap& ta_lo, con
 // src_k_by_rows: the source is stored [K][rows] (transposed) instead of [rows][K].
 int nrs_tc_stage(nrs_ctx* ctx, const float* src, float* hi, float* lo, int rows, int K, int ldk, int batch,
                  size_t src_bstride, size_t dst_bstride, bool src_k_by_rows);
-// NHWC planes of an NCHW tensor [n][c][hw], pixel stride nrs_plane_ld(c) floats (zeros between c and there).
-int nrs_tc_stage_image(nrs_ctx* ctx, const float* src, float* hi, float* lo, int n, int c, int hw);
 // Masked gradient staging (see stage_masked_kernel): mode 0 = ReLU mask of dy[n,c,h,w] by y;
 // mode 1 = gradient of a k x k / stride-k max-pool (g[n,c,h/k,w/k], argmax) followed by the ReLU
 // mask, taken from the pooled output y[n,c,h/k,w/k].  nchw_out and the planes are each optional
