@@ -43,6 +43,36 @@ __device__ __forceinline__ void contribute(float a, float b, float k, float& s, 
   }
 }
 
+// What the folded sums of a channel become; done by the last block of the channel to arrive (an integer ticket; the
+// splits are added in order whichever block that is), or by a kernel of its own where there are more channels than
+// tickets, columns instead of planes, or sums to be shared across processes first.
+struct BnFinish {
+  unsigned* tickets;   // null: not here
+  // forward: mean, biased variance, running statistics (running = momentum * running + (1 - momentum) * batch value,
+  // batchnorm2d.rs:52-53), 1/sqrt(var + eps)
+  float *mean, *istd, *running_mean, *running_var;
+  float count, eps, momentum;
+  // backward: sums[ch] = (dbeta, dgamma) of this call feeds the dx kernel, and the parameter gradients receive them (+)=
+  float2* sums;
+  float *dgamma, *dbeta;
+  int accumulate;
+};
+__device__ __forceinline__ void finish_stats(int ch, float s, float q, float k, float count, float eps, float momentum, float* mean,
+                                             float* istd, float* running_mean, float* running_var) {
+  const float d = s / count;
+  const float m = k + d;
+  const float v = fmaxf(q / count - d * d, 0.0f);
+  running_mean[ch] = momentum * running_mean[ch] + (1.0f - momentum) * m;
+  running_var[ch] = momentum * running_var[ch] + (1.0f - momentum) * v;
+  mean[ch] = m;
+  istd[ch] = 1.0f / sqrtf(v + eps);
+}
+__device__ __forceinline__ void finish_grads(int ch, float s, float q, float2* sums, float* dgamma, float* dbeta, int accumulate) {
+  sums[ch] = make_float2(s, q);
+  if (dgamma) dgamma[ch] = accumulate ? dgamma[ch] + q : q;
+  if (dbeta) dbeta[ch] = accumulate ? dbeta[ch] + s : s;
+}
+
 // Planes layout (hw >= 2): one block per (channel, sample split), 128-bit loads when the plane allows.
 // partial[split][ch] = (S, Q).
 // RELU (backward only): the layer's output went through a ReLU fused into the normalise pass; the incoming
@@ -52,7 +82,7 @@ template <bool FWD, bool RELU>
 __global__ void __launch_bounds__(kThreads)
 bn_pair_planes_kernel(const float* __restrict__ a, const float* __restrict__ b, float2* __restrict__ partial, int n,
                       int c, int hw, int splits, const float* __restrict__ gamma, const float* __restrict__ beta,
-                      const float* __restrict__ pivot, const float* __restrict__ mean, const float* __restrict__ istd) {
+                      const float* __restrict__ pivot, const float* __restrict__ mean, const float* __restrict__ istd, const BnFinish fin) {
   NRS_PDL_PROLOGUE();
   __shared__ float2 sm[kThreads / 32];
   const int ch = blockIdx.x, split = blockIdx.y;
@@ -106,6 +136,20 @@ bn_pair_planes_kernel(const float* __restrict__ a, const float* __restrict__ b, 
 #pragma unroll
     for (int i = 1; i < kThreads / 32; ++i) { t.x += sm[i].x; t.y += sm[i].y; }
     partial[(size_t)split * c + ch] = t;
+    if (!fin.tickets) return;
+    __threadfence();
+    if (atomicAdd(&fin.tickets[ch], 1u) != (unsigned)splits - 1) return;
+    __threadfence();
+    fin.tickets[ch] = 0;
+    float ts = 0.0f, tq = 0.0f;
+#pragma unroll 4
+    for (int z = 0; z < splits; ++z) {
+      const float2 v = __ldcg(partial + (size_t)z * c + ch);
+      ts += v.x;
+      tq += v.y;
+    }
+    if (FWD) finish_stats(ch, ts, tq, k, fin.count, fin.eps, fin.momentum, fin.mean, fin.istd, fin.running_mean, fin.running_var);
+    else finish_grads(ch, ts, tq, fin.sums, fin.dgamma, fin.dbeta, fin.accumulate);
   }
 }
 
@@ -170,13 +214,7 @@ __global__ void bn_stats_finish_kernel(const float2* __restrict__ partial, const
   }
   const float k = pivot ? pivot[ch] : x[(size_t)ch * hw];
   if (count_dev) count = *count_dev;
-  const float d = s / count;
-  const float m = k + d;
-  const float v = fmaxf(q / count - d * d, 0.0f);
-  running_mean[ch] = momentum * running_mean[ch] + (1.0f - momentum) * m;
-  running_var[ch] = momentum * running_var[ch] + (1.0f - momentum) * v;
-  mean[ch] = m;
-  istd[ch] = 1.0f / sqrtf(v + eps);
+  finish_stats(ch, s, q, k, count, eps, momentum, mean, istd, running_mean, running_var);
 }
 
 // Folds the backward sums; sums[ch] = (dbeta, dgamma) of this call feeds the dx kernel, and the parameter
@@ -192,9 +230,7 @@ __global__ void bn_grad_finish_kernel(const float2* __restrict__ partial, float2
     s += t.x;
     q += t.y;
   }
-  sums[ch] = make_float2(s, q);
-  if (dgamma) dgamma[ch] = accumulate ? dgamma[ch] + q : q;
-  if (dbeta) dbeta[ch] = accumulate ? dbeta[ch] + s : s;
+  finish_grads(ch, s, q, sums, dgamma, dbeta, accumulate);
 }
 
 // y = gamma * xhat + beta, xhat = (x - mean) * istd (bn2d_normalize, batchnorm2d.rs:62-75).
@@ -412,16 +448,24 @@ int plan_splits(const nrs_ctx* ctx, int n, int c, int hw) {
 template <bool FWD, bool RELU>
 int launch_pair(nrs_ctx* ctx, const float* a, const float* b, float2* partial, int n, int c, int hw, int splits,
                 const float* gamma, const float* beta, const float* pivot = nullptr, const float* mean = nullptr,
-                const float* istd = nullptr) {
+                const float* istd = nullptr, const BnFinish& fin = BnFinish{}) {
   if (hw == 1) {
     NRS_PDL_LAUNCH((bn_pair_cols_kernel<FWD, RELU>), dim3((c + 31) / 32, splits), kThreads, 0, ctx->stream, a, b, partial, n, c,
                    splits, gamma, beta, pivot, mean, istd);
   } else {
     NRS_PDL_LAUNCH((bn_pair_planes_kernel<FWD, RELU>), dim3(c, splits), kThreads, 0, ctx->stream, a, b, partial, n, c, hw,
-                   splits, gamma, beta, pivot, mean, istd);
+                   splits, gamma, beta, pivot, mean, istd, fin);
   }
   NRS_LAUNCHED(ctx);
   return NRS_OK;
+}
+// Tickets for a planes-layout reduction that finishes its channels itself; null when it cannot.
+int finish_tickets(nrs_ctx* ctx, int c, int hw, unsigned** out) {
+  *out = nullptr;
+  if (hw == 1 || c + 1 > kNrsFoldTickets) return NRS_OK;
+  const int st = nrs_fold_ticket(ctx, out);
+  if (st == NRS_OK) *out += 1;   // slot 0 belongs to the single-counter users
+  return st;
 }
 
 unsigned ew_blocks(const nrs_ctx* ctx, size_t work_items) {
@@ -458,9 +502,16 @@ int bn_forward(nrs_ctx* ctx, const char* who, const float* x, const float* gamma
   float* mean = mean_out ? mean_out : mean_ws;
   float2* summed = (float2*)(mean_ws + c + (c & 1));   // 8-byte aligned; [c] pairs + the count
   float* count_slot = (float*)(summed + c);
+  BnFinish fin{};
   if (training) {
+    if (!shared) {
+      const int ft = finish_tickets(ctx, c, hw, &fin.tickets);
+      if (ft != NRS_OK) return ft;
+      fin.mean = mean; fin.istd = istd; fin.running_mean = running_mean; fin.running_var = running_var;
+      fin.count = (float)((double)n * hw); fin.eps = eps; fin.momentum = momentum;
+    }
     const int sp = launch_pair<true, false>(ctx, x, nullptr, partial, n, c, hw, splits, nullptr, nullptr,
-                                            shared ? running_mean : nullptr);
+                                            shared ? running_mean : nullptr, nullptr, nullptr, fin);
     if (sp != NRS_OK) return sp;
   }
   if (shared) {
@@ -472,12 +523,13 @@ int bn_forward(nrs_ctx* ctx, const char* who, const float* x, const float* gamma
     NRS_PDL_LAUNCH(bn_stats_finish_kernel, nrs_blocks(c, 128), 128, 0, ctx->stream, (const float2*)summed, x, mean, istd,
                    running_mean, running_var, c, hw, 1, 0.0f, eps, momentum, training, (const float*)running_mean,
                    (const float*)count_slot);
-  } else {
+    NRS_LAUNCHED(ctx);
+  } else if (!fin.tickets) {
     NRS_PDL_LAUNCH(bn_stats_finish_kernel, nrs_blocks(c, 128), 128, 0, ctx->stream, (const float2*)partial, x, mean, istd,
                    running_mean, running_var, c, hw, splits, (float)((double)n * hw), eps, momentum, training,
                    (const float*)nullptr, (const float*)nullptr);
+    NRS_LAUNCHED(ctx);
   }
-  NRS_LAUNCHED(ctx);
   if (hi) {
     const img::Grid grid(n, c, hw);
 #define NRS_BN_NORM(S, R)                                                                                               \
@@ -524,12 +576,18 @@ int bn_backward(nrs_ctx* ctx, const char* who, const float* g, const float* xhat
   // process's own sums (they are summed across ranks with all other gradients)
   const bool shared = training && (dx || hi) && ctx->stat_sync.all_reduce_sum != nullptr;
   if (need_sums) {
-    const int sp = relu ? launch_pair<false, true>(ctx, g, xhat, partial, n, c, hw, splits, gamma, beta, nullptr, mean, istd)
-                        : launch_pair<false, false>(ctx, g, xhat, partial, n, c, hw, splits, nullptr, nullptr, nullptr, mean, istd);
+    BnFinish fin{};
+    const int ft = finish_tickets(ctx, c, hw, &fin.tickets);
+    if (ft != NRS_OK) return ft;
+    fin.sums = sums; fin.dgamma = dgamma; fin.dbeta = dbeta; fin.accumulate = accumulate_params;
+    const int sp = relu ? launch_pair<false, true>(ctx, g, xhat, partial, n, c, hw, splits, gamma, beta, nullptr, mean, istd, fin)
+                        : launch_pair<false, false>(ctx, g, xhat, partial, n, c, hw, splits, nullptr, nullptr, nullptr, mean, istd, fin);
     if (sp != NRS_OK) return sp;
-    NRS_PDL_LAUNCH(bn_grad_finish_kernel, nrs_blocks(c, 128), 128, 0, ctx->stream, (const float2*)partial, sums, dgamma, dbeta,
-                   c, splits, accumulate_params);
-    NRS_LAUNCHED(ctx);
+    if (!fin.tickets) {
+      NRS_PDL_LAUNCH(bn_grad_finish_kernel, nrs_blocks(c, 128), 128, 0, ctx->stream, (const float2*)partial, sums, dgamma, dbeta,
+                     c, splits, accumulate_params);
+      NRS_LAUNCHED(ctx);
+    }
   }
   if (!dx && !hi) return NRS_OK;
   if (shared) {

@@ -352,7 +352,7 @@ int conv_common(nrs_ctx* ctx, ConvPlan& p) {
 
   if (extras != ctx->out_extras.end()) ctx->out_extras.erase(extras);   // honoured from here on
   int splits = 0;
-  const tc::TilePlan tile = tc::plan_tile(ctx, tiles_m, p.n_ch_out, 1, p.ay.taps * p.ax.taps * pol.cblocks, split, 0.025);
+  const tc::TilePlan tile = tc::plan_tile(ctx, tiles_m, p.n_ch_out, 1, p.ay.taps * p.ax.taps * pol.cblocks, split, 0.025, true);
 #define NRS_RUN(BN_, PAIR_)                                                                                              \
   st = split ? run_conv<BN_, 2, PAIR_>(ctx, p, (const float*)a_hi, (const float*)a_lo, (const float*)p.w_hi, (const float*)p.w_lo, pol, (int)tiles_m, &splits) \
              : run_conv<BN_, 1, PAIR_>(ctx, p, (const float*)a_hi, nullptr, (const float*)p.w_hi, nullptr, pol, (int)tiles_m, &splits)

@@ -223,7 +223,7 @@ int run(nrs_ctx* ctx, const Operand& A, const Operand& B, int batch, int b_rows,
 
 // `limit`: widest tile allowed (segmented B: the segment must be whole tiles).
 tc::TilePlan tile_of(const nrs_ctx* ctx, int m, int n, int batch, int k, bool split, int limit = 128) {
-  return tc::plan_tile(ctx, (m + tc::BM - 1) / tc::BM, n, batch, (k + tc::BK - 1) / tc::BK, split, 0.004, limit);
+  return tc::plan_tile(ctx, (m + tc::BM - 1) / tc::BM, n, batch, (k + tc::BK - 1) / tc::BK, split, 0.004, false, limit);
 }
 
 template <bool MN>

@@ -552,10 +552,11 @@ inline void plan_split(const nrs_ctx* ctx, long tiles, long out_elems, int kb_to
 // of the grid) x (clocks per tile) is taken, a K-split's second pass counted in: wide tiles for large outputs, narrower
 // ones where they fill SMs that would idle or where a ragged column count would pad, pairs where there are enough row
 // tiles.  `reduce_clk`: what the second pass over a K-split costs per output value, on top of its launch (measured: 3.6 us
-// for 51 thousand values of a GEMM, 13.4 us for 819 thousand of a convolution, whose pixels lie strided).  `limit`:
-// widest tile allowed.
+// for 51 thousand values of a GEMM, 13.4 us for 819 thousand of a convolution, whose pixels lie strided).  A
+// convolution's 64-column pair is slower than the single tile in TF32 (30.1 us against 27.4 for 64 channels on 100 images
+// of 32 x 32).  `limit`: widest tile allowed.
 struct TilePlan { int bn; bool pair; };
-inline TilePlan plan_tile(const nrs_ctx* ctx, long tiles_m, int n, long batches, int kblocks, bool split_planes, double reduce_clk, int limit = 128) {
+inline TilePlan plan_tile(const nrs_ctx* ctx, long tiles_m, int n, long batches, int kblocks, bool split_planes, double reduce_clk, bool conv, int limit = 128) {
   static const struct { int bn; bool pair; int kb_clk[2], tile_clk; } kPlans[] = {{128, true, {820, 345}, 2600},
                                                                                   {64, true, {565, 317}, 1700},
                                                                                   {128, false, {905, 428}, 2600},
@@ -570,7 +571,8 @@ inline TilePlan plan_tile(const nrs_ctx* ctx, long tiles_m, int n, long batches,
     plan_split(ctx, tiles_m * tiles_n * batches, tiles_m * BM * n * batches, kblocks, split_planes, &sp);
     const int splits = sp.splits, per = sp.kb_per_split * sp.chunks;
     const long units = (c.pair ? (tiles_m + 1) / 2 : tiles_m) * tiles_n * batches * splits, slots = ctx->sm_count / (c.pair ? 2 : 1);
-    double t = (double)((units + slots - 1) / slots) * ((double)per * c.kb_clk[split_planes ? 0 : 1] + c.tile_clk);
+    const int kb_clk = c.pair && c.bn == 64 && conv && !split_planes ? 400 : c.kb_clk[split_planes ? 0 : 1];
+    double t = (double)((units + slots - 1) / slots) * ((double)per * kb_clk + c.tile_clk);
     if (splits > 1) t += 4000.0 + reduce_clk * (double)tiles_m * BM * n * batches;
     if (best_t < 0.0 || t < best_t) { best_t = t; best = TilePlan{c.bn, c.pair}; }
   }
