@@ -22,7 +22,7 @@ namespace {
 
 constexpr int kThreads = 256;
 
-__device__ __forceinline__ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+__host__ __device__ __forceinline__ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 __device__ __forceinline__ float wsum(float v) {
 #pragma unroll
@@ -82,7 +82,7 @@ template <bool FWD, bool RELU>
 __global__ void __launch_bounds__(kThreads)
 bn_pair_planes_kernel(const float* __restrict__ a, const float* __restrict__ b, float2* __restrict__ partial, int n,
                       int c, int hw, int splits, const float* __restrict__ gamma, const float* __restrict__ beta,
-                      const float* __restrict__ pivot, const float* __restrict__ mean, const float* __restrict__ istd, const BnFinish fin) {
+                      const float* __restrict__ pivot, const float* __restrict__ mean, const float* __restrict__ istd, const BnFinish fin, const NrsFastDiv div_per, const int vec /*planes of whole float4s*/) {
   NRS_PDL_PROLOGUE();
   __shared__ float2 sm[kThreads / 32];
   const int ch = blockIdx.x, split = blockIdx.y;
@@ -92,14 +92,14 @@ bn_pair_planes_kernel(const float* __restrict__ a, const float* __restrict__ b, 
   const float k = FWD ? (pivot ? pivot[ch] : a[(size_t)ch * hw]) : 0.0f;
   const float ga = RELU ? gamma[ch] : 0.0f, be = RELU ? beta[ch] : 0.0f;
   const float mu = mean ? mean[ch] : 0.0f, is = mean ? istd[ch] : 1.0f;   // b is x; without them xhat itself
-  const bool vec = (hw & 3) == 0 && aligned16(a) && (FWD || aligned16(b));
   // The block's threads walk the split's (image, element) pairs as one flat index, so that planes shorter
   // than a warp's reach (8x8, 4x4 feature maps) still keep every lane loading.
   float s = 0.0f, q = 0.0f, s1 = 0.0f, q1 = 0.0f;
   const int per = vec ? hw / 4 : hw;                       // items per plane
   const int items = max(n1 - n0, 0) * per;               // n * hw < 2^31 is checked on the host
+#pragma unroll 2
   for (int j = threadIdx.x; j < items; j += kThreads) {
-    const int di = j / per, i = j - di * per;
+    const int di = (int)div_per.div((uint32_t)j), i = j - di * per;
     const size_t base = ((size_t)(n0 + di) * c + ch) * hw;
     if (vec) {
       float4 va = reinterpret_cast<const float4*>(a + base)[i];
@@ -344,7 +344,7 @@ bn_normalize_planes_kernel(const float* __restrict__ x, const float* __restrict_
 #pragma unroll
   for (int i = 0; i < 16; ++i) {
     const int c = c0 + warp + 8 * (i >> 2);
-    v[i] = (c < g.c && px.live[i & 3]) ? x[px.at[i & 3] + (size_t)c * g.hw] : 0.0f;
+    v[i] = (c < g.c && px.live[i & 3]) ? x[px.base + (px.at[i & 3] + (uint32_t)c * g.hw)] : 0.0f;
   }
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
@@ -356,7 +356,7 @@ bn_normalize_planes_kernel(const float* __restrict__ x, const float* __restrict_
       const float h = (v[4 * k + s] - m) * is;
       float o = fmaf(ga, h, be);
       if (RELU) o = fmaxf(o, 0.0f);
-      if (ok && px.live[s]) y[px.at[s] + (size_t)c * g.hw] = o;
+      if (ok && px.live[s]) y[px.base + (px.at[s] + (uint32_t)c * g.hw)] = o;
       tile[cl][s * 32 + lane] = o;
     }
   }
@@ -366,7 +366,7 @@ bn_normalize_planes_kernel(const float* __restrict__ x, const float* __restrict_
 
 // dx (overwritten; null: planes only) with its NHWC planes, and chan_partial[tile of 128 pixels][c], its sums over the tile.
 template <bool SPLIT, bool RELU>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 3)
 bn_dx_planes_kernel(const float* __restrict__ gr, const float* __restrict__ x, const float* __restrict__ mean,
                     const float* __restrict__ istd, const float* __restrict__ gamma, const float* __restrict__ beta,
                     const float2* __restrict__ sums, float* __restrict__ dx, float* __restrict__ hi, float* __restrict__ lo,
@@ -382,7 +382,7 @@ bn_dx_planes_kernel(const float* __restrict__ gr, const float* __restrict__ x, c
   for (int i = 0; i < 16; ++i) {
     const int c = c0 + warp + 8 * (i >> 2);
     const bool ok = c < g.c && px.live[i & 3];
-    const size_t at = px.at[i & 3] + (size_t)c * g.hw;
+    const size_t at = px.base + (px.at[i & 3] + (uint32_t)c * g.hw);
     vg[i] = ok ? gr[at] : 0.0f;
     vx[i] = ok ? x[at] : 0.0f;
   }
@@ -401,7 +401,7 @@ bn_dx_planes_kernel(const float* __restrict__ gr, const float* __restrict__ x, c
       if (RELU) gi = fmaf(ga, h, be) > 0.0f ? gi : 0.0f;
       const bool live = ok && px.live[s];
       const float r = !live ? 0.0f : training ? is * (gi * ga - m1 - h * m2) : gi * ga * is;
-      if (live && dx) dx[px.at[s] + (size_t)c * g.hw] = r;
+      if (live && dx) dx[px.base + (px.at[s] + (uint32_t)c * g.hw)] = r;
       tile[cl][s * 32 + lane] = r;
       total += r;
     }
@@ -453,8 +453,9 @@ int launch_pair(nrs_ctx* ctx, const float* a, const float* b, float2* partial, i
     NRS_PDL_LAUNCH((bn_pair_cols_kernel<FWD, RELU>), dim3((c + 31) / 32, splits), kThreads, 0, ctx->stream, a, b, partial, n, c,
                    splits, gamma, beta, pivot, mean, istd);
   } else {
+    const bool vec = (hw & 3) == 0 && aligned16(a) && (FWD || aligned16(b));
     NRS_PDL_LAUNCH((bn_pair_planes_kernel<FWD, RELU>), dim3(c, splits), kThreads, 0, ctx->stream, a, b, partial, n, c, hw,
-                   splits, gamma, beta, pivot, mean, istd, fin);
+                   splits, gamma, beta, pivot, mean, istd, fin, NrsFastDiv(vec ? hw / 4 : hw), vec ? 1 : 0);
   }
   NRS_LAUNCHED(ctx);
   return NRS_OK;

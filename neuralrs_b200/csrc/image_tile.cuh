@@ -22,18 +22,22 @@ struct Grid {
   dim3 blocks() const { return dim3((pixels + kTilePx - 1) / kTilePx, (unsigned)((ld + kTileCh - 1) / kTileCh)); }
 };
 
-// Where this thread's four pixels (segments) lie in NCHW, channel 0.
+// Where this thread's four pixels (segments) lie in NCHW, channel 0: offsets from the tile's first image, which fit 32
+// bits (a tile touches two images, or 128 pixels of smaller ones).
 struct Pixels {
-  size_t at[4];
+  size_t base;
+  uint32_t at[4];
   bool live[4];
   __device__ __forceinline__ Pixels(const Grid& g, uint32_t p0) {
+    const uint32_t im0 = g.div_hw.div(p0), plane = (uint32_t)g.c * (uint32_t)g.hw;
+    base = (size_t)im0 * plane;
 #pragma unroll
     for (int s = 0; s < 4; ++s) {
       const uint32_t p = p0 + s * 32 + (threadIdx.x & 31);
       uint32_t im, px;
-      g.div_hw.divmod(p < g.pixels ? p : 0, im, px);
+      g.div_hw.divmod(p < g.pixels ? p : p0, im, px);
       live[s] = p < g.pixels;
-      at[s] = (size_t)im * g.c * g.hw + px;
+      at[s] = (im - im0) * plane + px;
     }
   }
 };

@@ -93,7 +93,7 @@ stage_image_kernel(const float* __restrict__ src, float* __restrict__ hi, float*
 #pragma unroll
   for (int i = 0; i < 16; ++i) {
     const int c = c0 + warp + 8 * (i >> 2);
-    v[i] = (c < g.c && px.live[i & 3]) ? src[px.at[i & 3] + (size_t)c * g.hw] : 0.0f;
+    v[i] = (c < g.c && px.live[i & 3]) ? src[px.base + (px.at[i & 3] + (uint32_t)c * g.hw)] : 0.0f;
   }
 #pragma unroll
   for (int i = 0; i < 16; ++i) tile[warp + 8 * (i >> 2)][(i & 3) * 32 + lane] = v[i];
