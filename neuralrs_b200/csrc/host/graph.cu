@@ -1190,7 +1190,7 @@ NodeP dropout2d(const NodeP& x, float p, bool training, const NodeP& mask) {
 // and column sums of the product, which is all that layer's backward pass reads (three passes over the tensor less).
 static void linear_input_grad(nrs_ctx* ctx, const NodeP& x, const NodeP& w, const float* dz, int m, int k, int n) {
   const bool fold = x->fold_act != NRS_ACT_NONE && !x->view_of && !x->grad_valid && !x->gplanes_hi && planes_possible(ctx) &&
-                    nrs_gemm_on_tensor_cores(ctx, m, k, n);
+                    (nrs_gemm_on_tensor_cores(ctx, m, k, n) || (n <= 16 && m <= 4096));
   GradTarget t = grad_target(x);
   if (fold) {
     NrsGemmExtras e;

@@ -102,10 +102,12 @@ struct CeOp {
 // gets (softmax - t) * inv_div.  Scalar path (any width / alignment).
 __global__ void __launch_bounds__(256)
 ce_rows_kernel(const float* __restrict__ logits, const float* __restrict__ target, const int32_t* __restrict__ labels,
-               float* __restrict__ row_loss, float* __restrict__ grad, int batch, int classes, float inv_div) {
+               float* __restrict__ row_loss, float* __restrict__ grad, int batch, int classes, float inv_div, float* block_partial,
+               unsigned* ticket, float* loss_dev) {
   NRS_PDL_PROLOGUE();
   const int lane = threadIdx.x & 31;
   const int warps_per_block = blockDim.x >> 5;
+  float warp_loss = 0.0f;   // this warp's rows, in the order it takes them
   for (int b = blockIdx.x * warps_per_block + (threadIdx.x >> 5); b < batch; b += gridDim.x * warps_per_block) {
     const float* row = logits + (size_t)b * classes;
     const float* trow = target ? target + (size_t)b * classes : nullptr;
@@ -123,11 +125,16 @@ ce_rows_kernel(const float* __restrict__ logits, const float* __restrict__ targe
       loss += -tv * (xv - lse);
       if (grad) grad[(size_t)b * classes + c] = (expf(xv - mx) / se - tv) * inv_div;
     }
-    if (row_loss) {
+    if (row_loss || loss_dev) {
       loss = warp_sum(loss);
-      if (lane == 0) row_loss[b] = loss;
+      if (row_loss && lane == 0) row_loss[b] = loss;
+      warp_loss += loss;
     }
   }
+  if (!loss_dev) return;
+  __shared__ float wsum[32];
+  if (lane == 0) wsum[threadIdx.x >> 5] = warp_loss;
+  fold_batch_loss(wsum, warps_per_block, block_partial, ticket, loss_dev, inv_div);
 }
 
 // The same with the row held in registers: logits (and the one-hot row) are read once with 128-bit
@@ -219,32 +226,6 @@ ce_rows_vec_kernel(const float* __restrict__ logits, const float* __restrict__ t
   fold_batch_loss(wsum, warps_per_block, block_partial, ticket, loss_dev, inv_div);
 }
 
-// loss_dev[0] = (sum_b row_loss[b]) * inv_div, one block, fixed summation tree.
-__global__ void __launch_bounds__(1024)
-ce_mean_kernel(const float* __restrict__ row_loss, float* __restrict__ loss_dev, int batch, float inv_div) {
-  NRS_PDL_PROLOGUE();
-  __shared__ float sm[32];
-  float s = 0.0f;
-  int i = threadIdx.x;
-  const int step = blockDim.x;
-  for (; i + 7 * step < batch; i += 8 * step) {   // eight loads in flight; the additions keep the order of i
-    float v[8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) v[u] = row_loss[i + u * step];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) s += v[u];
-  }
-  for (; i < batch; i += step) s += row_loss[i];
-  s = warp_sum(s);
-  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    float t = threadIdx.x < (blockDim.x >> 5) ? sm[threadIdx.x] : 0.0f;
-    t = warp_sum(t);
-    if (threadIdx.x == 0) loss_dev[0] = t * inv_div;
-  }
-}
-
 int run_ce(nrs_ctx* ctx, const char* who, const float* logits, const float* target, const int32_t* labels, float* loss_dev,
            float* row_loss, float* grad, int batch, int classes, int divisor) {
   NRS_REQUIRE(ctx, batch >= 0 && classes > 0, NRS_ERR_SHAPE, "%s: bad shape [%d,%d]", who, batch, classes);
@@ -284,18 +265,15 @@ int run_ce(nrs_ctx* ctx, const char* who, const float* logits, const float* targ
   if (classes > 512 && blocks > ctx->sm_count * 3) blocks = ctx->sm_count * 3;
   const bool vec = classes % 4 == 0 && classes <= 1024 &&
                    ((reinterpret_cast<uintptr_t>(logits) | reinterpret_cast<uintptr_t>(target) | reinterpret_cast<uintptr_t>(grad)) & 15) == 0;
-  // the vector kernels fold the batch mean themselves (per-block partial sums, last block folds); the scalar
-  // kernel leaves per-row losses to a second launch
-  float* rl = row_loss;
+  // the kernels fold the batch mean themselves (per-block partial sums, last block folds)
   float* partial = nullptr;
   unsigned* ticket = nullptr;
   if (loss_dev) {
     void* ws = nullptr;
-    int st = nrs_workspace(ctx, (size_t)(vec ? blocks : (rl ? 0 : batch)) * sizeof(float) + 16, &ws);
-    if (st == NRS_OK && vec) st = nrs_fold_ticket(ctx, &ticket);
+    int st = nrs_workspace(ctx, (size_t)blocks * sizeof(float) + 16, &ws);
+    if (st == NRS_OK) st = nrs_fold_ticket(ctx, &ticket);
     if (st != NRS_OK) return st;
-    if (vec) partial = (float*)ws;
-    else if (!rl) rl = (float*)ws;
+    partial = (float*)ws;
   }
   if (vec && classes <= 128) {
     NRS_PDL_LAUNCH(ce_rows_vec_kernel<1>, blocks, 256, 0, ctx->stream, logits, target, labels, row_loss, grad, batch, classes, inv_div,
@@ -307,13 +285,10 @@ int run_ce(nrs_ctx* ctx, const char* who, const float* logits, const float* targ
     NRS_PDL_LAUNCH(ce_rows_vec_kernel<8>, blocks, 256, 0, ctx->stream, logits, target, labels, row_loss, grad, batch, classes, inv_div,
                    partial, ticket, loss_dev);
   } else {
-    NRS_PDL_LAUNCH(ce_rows_kernel, blocks, 256, 0, ctx->stream, logits, target, labels, rl, grad, batch, classes, inv_div);
+    NRS_PDL_LAUNCH(ce_rows_kernel, blocks, 256, 0, ctx->stream, logits, target, labels, row_loss, grad, batch, classes, inv_div, partial, ticket,
+                   loss_dev);
   }
   NRS_LAUNCHED(ctx);
-  if (loss_dev && !vec) {
-    NRS_PDL_LAUNCH(ce_mean_kernel, 1, 1024, 0, ctx->stream, rl, loss_dev, batch, inv_div);
-    NRS_LAUNCHED(ctx);
-  }
   return NRS_OK;
 }
 

@@ -15,6 +15,9 @@ NETS = {
                          ("linear", 70, 10)]),
     "odd": ((4, 9, 7), [("conv", 4, 33, 3, 1, 1), ("relu",), ("conv", 33, 65, 4, 1, 2), ("relu",), ("conv", 65, 17, 7, 1, 3), ("relu",), ("flatten",),
                         ("linear", 1360, 131), ("relu",), ("linear", 131, 10)]),
+    # classifier heads over fused activations, more rows than one block takes
+    "head": ((2, 6, 9), [("flatten",), ("linear", 108, 136), ("relu",), ("linear", 136, 10)]),
+    "head_gelu": ((2, 6, 9), [("flatten",), ("linear", 108, 72), ("gelu",), ("linear", 72, 10)]),
 }
 
 
@@ -37,8 +40,9 @@ def gradients(ctx, mode, shape, layers, x, t, params):
 def test_trainer_planes_ragged(gpu_ctx, net, mode, tol):
     shape, layers = NETS[net]
     rng = np.random.default_rng(5)
-    x = rng.standard_normal((24, *shape)).astype(np.float32)
-    t = np.eye(10, dtype=np.float32)[rng.integers(0, 10, 24)]
+    batch = 150 if net.startswith("head") else 24
+    x = rng.standard_normal((batch, *shape)).astype(np.float32)
+    t = np.eye(10, dtype=np.float32)[rng.integers(0, 10, batch)]
     ref_loss, params, ref = gradients(gpu_ctx, _lib.MATH_FP32, shape, layers, x, t, None)
     loss, _, got = gradients(gpu_ctx, mode, shape, layers, x, t, params)
     assert np.isclose(loss, ref_loss, rtol=tol)
