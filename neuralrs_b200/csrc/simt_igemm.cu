@@ -412,7 +412,7 @@ thin_n_cols_kernel(const float* __restrict__ a, const float* __restrict__ b, flo
 // takes 32 columns of a K-split, its 8 warps every eighth row of B (full lines, several in flight), A's rows come from
 // shared memory, and enough splits run to cover the SMs.  The warps are added in order, the splits by the last block of
 // a column group to arrive, in split order (fixed order of additions, no second launch).  [1,3136] x [3136,128]: the
-// 128 x 128 tile took 30 us in two launches, this 6.
+// 128 x 128 tile took 22 us in two launches for one row, this 6.6.
 constexpr int kThinM = 15, kThinMChunk = 512;
 template <int MT>
 __global__ void __launch_bounds__(256)
@@ -428,14 +428,27 @@ thin_m_kernel(const float* __restrict__ a, const float* __restrict__ b, float* c
   float acc[MT];
 #pragma unroll
   for (int i = 0; i < MT; ++i) acc[i] = 0.0f;
+  float w0[8];   // the warp's first eight rows of B are under way before A is staged
+#pragma unroll
+  for (int u = 0; u < 8; ++u) {
+    const int kk = k0 + warp + 8 * u;
+    w0[u] = col < n && kk < k1 ? b[(size_t)kk * n + col] : 0.0f;
+  }
   for (int i = threadIdx.x; i < MT * (k1 - k0); i += blockDim.x) {
-    const int r = i / (k1 - k0), kk = i - r * (k1 - k0);
+    const int r = MT == 1 ? 0 : i / (k1 - k0), kk = i - r * (k1 - k0);
     as[r][kk] = r < m ? a[(size_t)r * k + k0 + kk] : 0.0f;
   }
   __syncthreads();
+#pragma unroll
+  for (int u = 0; u < 8; ++u) {
+    const int kk = warp + 8 * u;
+    if (k0 + kk >= k1) break;
+#pragma unroll
+    for (int i = 0; i < MT; ++i) acc[i] = fmaf(as[i][kk], w0[u], acc[i]);
+  }
   if (col < n) {
 #pragma unroll 8
-    for (int kk = k0 + warp; kk < k1; kk += 8) {
+    for (int kk = k0 + warp + 64; kk < k1; kk += 8) {
       const float w = b[(size_t)kk * n + col];
 #pragma unroll
       for (int i = 0; i < MT; ++i) acc[i] = fmaf(as[i][kk - k0], w, acc[i]);
@@ -467,12 +480,22 @@ thin_m_kernel(const float* __restrict__ a, const float* __restrict__ b, float* c
   __syncthreads();
   if (!last) return;
   __threadfence();
+  // every warp adds every eighth split, and the warps combine in warp order
+  for (int r = 0; r < m; ++r) {
+    float v = 0.0f;
+    if (col < n) {
+#pragma unroll 4
+      for (int z = warp; z < splits; z += 8) v += __ldcg(partial + ((size_t)z * m + r) * n + col);
+    }
+    sums[warp][r][lane] = v;
+  }
+  __syncthreads();
   for (int o = threadIdx.x; o < m * 32; o += blockDim.x) {
-    const int r = o >> 5, cc = blockIdx.x * 32 + (o & 31);
+    const int r = o >> 5, cl = o & 31, cc = blockIdx.x * 32 + cl;
     if (cc >= n) continue;
     float v = 0.0f;
-#pragma unroll 8
-    for (int z = 0; z < splits; ++z) v += __ldcg(partial + ((size_t)z * m + r) * n + cc);
+#pragma unroll
+    for (int w = 0; w < 8; ++w) v += sums[w][r][cl];
     finish(r, cc, v);
   }
   if (threadIdx.x == 0) tickets[blockIdx.x] = 0;

@@ -161,7 +161,7 @@ struct ConvPolicy {
       return;
     }
     // Whole channel blocks take their own instantiation: with per-channel conditions the loads of a block no longer
-    // issue together (measured on the 64-channel data gradient with mask and planes: 58 -> 217 us).
+    // issue together (measured on the 64-channel data gradient with mask and planes: 69 -> 217 us).
     if (n_ch_out - nb >= 32) finish<true>(rw.off, nb, r, v);
     else finish<false>(rw.off, nb, r, v);
   }
