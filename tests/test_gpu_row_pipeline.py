@@ -10,7 +10,8 @@ from .gpu_util import Dev, call
 
 pytestmark = pytest.mark.gpu
 F = C.c_float
-SHAPES = [(3, 17), (9001, 17), (1031, 515), (4100, 256), (1060, 1000), (257, 2050), (130, 4097), (17, 8192), (17, 8193), (70001, 2), (8400, 1000)]
+SHAPES = [(3, 17), (9001, 17), (1031, 515), (4100, 256), (1060, 1000), (257, 2050), (130, 4097), (17, 8192), (17, 8193), (70001, 2), (8400, 1000), (4400, 1406), (8401, 1001),
+          (33601, 250)]
 
 
 @pytest.mark.parametrize("rows,f", SHAPES)
