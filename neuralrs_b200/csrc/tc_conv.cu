@@ -28,11 +28,14 @@
 // Reference counterparts: conv2d_im2col + matmul_nn + conv2d_col2out (forward),
 // conv2d_out2mm + matmul_tn + conv2d_col2im (data gradient) — src/cuda/nn/conv.rs:27-149,
 // 244-312.
+#include <cstring>
+
 #include "tc_mainloop.cuh"
 
 namespace {
 
-struct ConvPolicy {
+template <int EPI>
+struct ConvPolicyOf {
   int Wt, Ht, Nt, tiles_x, tiles_y;   // pixel tile in the space of (u, v), the pixels this launch computes
   int sub_h, sub_w;                   // extents of that space
   int out_h, out_w;                   // the tensor written: pixel (u, v) is (u*out_step + out_y0, v*out_step + out_x0)
@@ -136,7 +139,7 @@ struct ConvPolicy {
   static constexpr bool kMaySplit = true;
   __device__ __forceinline__ bool clip(int, int, int, int*, int*) const { return true; }
   int order() const { return tc::kRaster; }
-  static constexpr int kEpiWarps = 4;   // 250 registers per thread: no room for more
+  static constexpr int kEpiWarps = EPI;   // see emits_on_eight_warps
   __device__ __forceinline__ float* colsum_row(int tile_m, int q) const {
     return colsum_partial ? colsum_partial + ((size_t)tile_m * 4 + q) * n_ch_out : nullptr;
   }
@@ -203,6 +206,14 @@ struct ConvPolicy {
   }
 };
 
+using ConvPolicy = ConvPolicyOf<4>;
+
+// Which launches take two epilogue warps per lane quarter: 64 columns in 3xTF32 with planes to emit, whose epilogue (mask,
+// NCHW store, split and staging: 15 thousand clocks a tile) is longer than the main loop of a 64-channel layer (10).  There
+// 53 -> 47 us forward and 62 -> 58 backward on 100 images of 32 x 32.  Elsewhere the second staging tile costs more ring
+// than the epilogue gains (128 columns without planes 706 -> 726 us a pass, TF32 with planes 1.5 %).
+constexpr bool emits_on_eight_warps(int bn, int nplanes, bool emit) { return bn == 64 && nplanes == 2 && emit; }
+
 // One axis of a (sub-)problem: `len` output pixels at positions u*step + first, `taps` kernel taps tap0,
 // tap0 + tap_step, ..., and the activation coordinate of tap t for pixel u: u * in_step + base + sgn * t.
 struct ConvAxis {
@@ -255,6 +266,15 @@ int run_conv(nrs_ctx* ctx, const ConvPlan& p, const float* a_hi, const float* a_
     if (pol.out_lo) ok = ok && tc::encode_tmap_f32(&to_lo, pol.out_lo, 4, odim, ostr, abox);
   }
   NRS_REQUIRE(ctx, ok, NRS_ERR_CUDA, "tc_conv: cuTensorMapEncodeTiled failed");
+  if constexpr (emits_on_eight_warps(BN, NPLANES, true)) {
+    if (pol.out_hi) {
+      ConvPolicyOf<8> wide;
+      static_assert(sizeof(wide) == sizeof(pol), "the same fields");
+      std::memcpy(&wide, &pol, sizeof(wide));
+      return tc::launch<BN, NPLANES, PAIR, ConvPolicyOf<8>>(ctx, ta_hi, ta_lo, tb_hi, tb_lo, wide, tiles_m, p.n_ch_out, 1,
+                                                            p.ay.taps * p.ax.taps * pol.cblocks, &to_hi, pol.out_lo ? &to_lo : nullptr, splits_out);
+    }
+  }
   return tc::launch<BN, NPLANES, PAIR, ConvPolicy>(ctx, ta_hi, ta_lo, tb_hi, tb_lo, pol, tiles_m, p.n_ch_out, 1,
                                              p.ay.taps * p.ax.taps * pol.cblocks, pol.out_hi ? &to_hi : nullptr,
                                              pol.out_lo ? &to_lo : nullptr, splits_out);

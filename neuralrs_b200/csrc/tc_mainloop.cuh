@@ -3,13 +3,13 @@
 // memory, fed by TMA, consumed by tcgen05.mma kind::tf32.
 //
 // Persistent CTAs (one per SM) walk a list of output tiles (row tile, column tile,
-// batch x K-split).  Six or eighteen warps, fixed roles:
+// batch x K-split).  Six to eighteen warps, fixed roles:
 //   warp 0     TMA producer: per K-slice, one mbarrier-tracked ring
 //              slot holding the A and B slices (and their residual planes for 3xTF32);
 //              the ring runs ahead across tile boundaries
 //   warp 1     TMEM allocation; issues the UMMAs (M=128, K=8) and commits
 //              ring slots back to the producer, then the accumulator to the epilogue
-//   warps 2..  epilogue (4 or 16 warps, the policy's choice): tcgen05.ld (thread = accumulator row),
+//   warps 2..  epilogue (4, 8 or 16 warps, the policy's choice): tcgen05.ld (thread = accumulator row),
 //              policy-defined store
 // TMEM holds two accumulators, so the epilogue of tile i runs under the main loop of
 // tile i+1.
@@ -134,10 +134,10 @@ struct TileMap {
   }
 };
 
-// Shared memory of the epilogue: the plane-emission staging tile, one [128 rows][128 B] tile per plane, or (row-major
+// Shared memory of the epilogue: a plane-emission staging tile per four warps, [128 rows][128 B] per plane, or (row-major
 // results) a 32 x 16 transpose tile per warp.
 template <int NPLANES, class Policy>
-__host__ __device__ constexpr int emit_bytes() { return Policy::kCanEmit ? NPLANES * BM * 128 : Policy::kEpiWarps * 2048; }
+__host__ __device__ constexpr int emit_bytes() { return Policy::kCanEmit ? Policy::kEpiWarps / 4 * NPLANES * BM * 128 : Policy::kEpiWarps * 2048; }
 template <class Policy>
 __host__ __device__ constexpr int threads() { return 64 + 32 * Policy::kEpiWarps; }
 
@@ -181,13 +181,13 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
   using L = SmemLayout<BN, NPLANES, kEmitBytes, PAIR>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  uint8_t* emit_tile = smem + L::kStages * L::kStage;   // [planes][128 rows][128 B], 1024-byte aligned
+  uint8_t* emit_tile = smem + L::kStages * L::kStage;   // [four warps][planes][128 rows][128 B], 1024-byte aligned
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(emit_tile + kEmitBytes);
   uint64_t* empty_bar = full_bar + L::kStages;
   uint64_t* acc_full = empty_bar + L::kStages;   // [2] accumulator ready for the epilogue
   uint64_t* acc_empty = acc_full + 2;            // [2] accumulator drained by the epilogue
-  uint64_t* emit_bar = acc_empty + 2;            // [2] staging tile free / staging tile written
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(emit_bar + 2);
+  uint64_t* emit_bars = acc_empty + 2;           // [four warps][2] staging tile free / staging tile written
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(emit_bars + 4);
 
   const int warp = (int)uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   // A pair walks the tile list together: its CTA of rank r takes row tile 2*i + r of every pair of row tiles i.
@@ -201,7 +201,7 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
     if (emit >= 1) prefetch_tmap(&tm_out_hi);
     if (emit == 2) prefetch_tmap(&tm_out_lo);
     for (int s = 0; s < L::kStages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-    for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], Policy::kEpiWarps * (PAIR ? 2 : 1)); mbar_init(&emit_bar[b], 128); }
+    for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], Policy::kEpiWarps * (PAIR ? 2 : 1)); mbar_init(&emit_bars[b], 128); mbar_init(&emit_bars[2 + b], 128); }
     fence_barrier_init();
   }
   if (warp == 1) {
@@ -347,7 +347,11 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
     // ---------------- epilogue: warp w owns TMEM lanes [32*(w%4), +32)
     const int q = warp & 3;
     const int row = q * 32 + lane;   // row inside the tile
-    const bool emit_issuer = warp == 2 && lane == 0;
+    // (kCanEmit: every four warps take 32-column blocks of their own, with a staging tile and an issuing thread)
+    const int team = (warp - 2) >> 2;
+    const bool emit_issuer = ((warp - 2) & 3) == 0 && lane == 0;
+    uint64_t* emit_bar = emit_bars + (Policy::kCanEmit ? 2 * team : 0);
+    uint8_t* team_tile = emit_tile + (Policy::kCanEmit ? team * NPLANES * BM * 128 : 0);
     uint32_t local = 0, emitted = 0;
     bool ok = true;
     bool odd = false;
@@ -469,7 +473,7 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
               if (emit_issuer) bulk_wait_read();
               mbar_arrive(&emit_bar[0]);
               if (!mbar_wait(&emit_bar[0], ph)) { atomicExch(err_flag, kErrEpilogueWait); ok = false; break; }
-              uint8_t* row_hi = emit_tile + row * 128;
+              uint8_t* row_hi = team_tile + row * 128;
 #pragma unroll
               for (int g = 0; g < 8; ++g) {
                 const int chunk = (g ^ (row & 7)) * 16;   // 128-byte swizzle: 16-byte chunk index XOR row % 8
@@ -483,8 +487,8 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
               mbar_arrive(&emit_bar[1]);
               if (emit_issuer) {
                 if (!mbar_wait(&emit_bar[1], ph)) { atomicExch(err_flag, kErrEpilogueWait); ok = false; break; }
-                tma_store_4d(&tm_out_hi, emit_tile, n0 + c * 32, rw.x0, rw.y0, rw.n0);
-                if (NPLANES == 2 && emit == 2) tma_store_4d(&tm_out_lo, emit_tile + BM * 128, n0 + c * 32, rw.x0, rw.y0, rw.n0);
+                tma_store_4d(&tm_out_hi, team_tile, n0 + c * 32, rw.x0, rw.y0, rw.n0);
+                if (NPLANES == 2 && emit == 2) tma_store_4d(&tm_out_lo, team_tile + BM * 128, n0 + c * 32, rw.x0, rw.y0, rw.n0);
                 bulk_commit();
               }
             }
