@@ -139,7 +139,7 @@ struct ConvPolicyOf {
   static constexpr bool kMaySplit = true;
   __device__ __forceinline__ bool clip(int, int, int, int*, int*) const { return true; }
   int order() const { return tc::kRaster; }
-  static constexpr int kEpiWarps = EPI;   // see emits_on_eight_warps
+  static constexpr int kEpiWarps = EPI;   // see may_take_eight_warps
   __device__ __forceinline__ float* colsum_row(int tile_m, int q) const {
     return colsum_partial ? colsum_partial + ((size_t)tile_m * 4 + q) * n_ch_out : nullptr;
   }
@@ -208,11 +208,12 @@ struct ConvPolicyOf {
 
 using ConvPolicy = ConvPolicyOf<4>;
 
-// Which launches take two epilogue warps per lane quarter: 64 columns in 3xTF32 with planes to emit, whose epilogue (mask,
-// NCHW store, split and staging: 15 thousand clocks a tile) is longer than the main loop of a 64-channel layer (10).  There
-// 53 -> 47 us forward and 62 -> 58 backward on 100 images of 32 x 32.  Elsewhere the second staging tile costs more ring
-// than the epilogue gains (128 columns without planes 706 -> 726 us a pass, TF32 with planes 1.5 %).
-constexpr bool emits_on_eight_warps(int bn, int nplanes, bool emit) { return bn == 64 && nplanes == 2 && emit; }
+// Which launches take two epilogue warps per lane quarter: 64 columns in 3xTF32 with planes to emit, or with bias and
+// activation, whose epilogue (activation or mask, NCHW store, split and staging: 15 thousand clocks a tile) is longer than
+// the main loop of a 64-channel layer (10).  There 53 -> 47 us and 58 -> 51 forward, 62 -> 58 backward on 100 images of
+// 32 x 32.  Elsewhere they lose: plain data gradients (22 -> 26 us for a residue of the 48 -> 80 layer), 128 columns (the
+// second staging tile costs a ring slot: 706 -> 726 us a pass of the 64 -> 128 layer), TF32 (1.5 %).
+constexpr bool may_take_eight_warps(int bn, int nplanes) { return bn == 64 && nplanes == 2; }
 
 // One axis of a (sub-)problem: `len` output pixels at positions u*step + first, `taps` kernel taps tap0,
 // tap0 + tap_step, ..., and the activation coordinate of tap t for pixel u: u * in_step + base + sgn * t.
@@ -266,13 +267,14 @@ int run_conv(nrs_ctx* ctx, const ConvPlan& p, const float* a_hi, const float* a_
     if (pol.out_lo) ok = ok && tc::encode_tmap_f32(&to_lo, pol.out_lo, 4, odim, ostr, abox);
   }
   NRS_REQUIRE(ctx, ok, NRS_ERR_CUDA, "tc_conv: cuTensorMapEncodeTiled failed");
-  if constexpr (emits_on_eight_warps(BN, NPLANES, true)) {
-    if (pol.out_hi) {
+  if constexpr (may_take_eight_warps(BN, NPLANES)) {
+    if (pol.out_hi || (p.bias && p.act != NRS_ACT_NONE)) {
       ConvPolicyOf<8> wide;
       static_assert(sizeof(wide) == sizeof(pol), "the same fields");
       std::memcpy(&wide, &pol, sizeof(wide));
       return tc::launch<BN, NPLANES, PAIR, ConvPolicyOf<8>>(ctx, ta_hi, ta_lo, tb_hi, tb_lo, wide, tiles_m, p.n_ch_out, 1,
-                                                            p.ay.taps * p.ax.taps * pol.cblocks, &to_hi, pol.out_lo ? &to_lo : nullptr, splits_out);
+                                                            p.ay.taps * p.ax.taps * pol.cblocks, pol.out_hi ? &to_hi : nullptr,
+                                                            pol.out_lo ? &to_lo : nullptr, splits_out);
     }
   }
   return tc::launch<BN, NPLANES, PAIR, ConvPolicy>(ctx, ta_hi, ta_lo, tb_hi, tb_lo, pol, tiles_m, p.n_ch_out, 1,
