@@ -101,6 +101,9 @@ int nrs_selftest_bounded_wait(nrs_ctx* ctx, int64_t limit_clocks);
  * ordinal which kernels already had their dynamic shared-memory limit raised, so that contexts on
  * several GPUs of one process each get theirs.  Returns 0 when that bookkeeping behaves. */
 int nrs_selftest_smem_attr_bookkeeping(void);
+/* Host-only self-test (no reference counterpart, needs no GPU): the queue of second-stage reductions of a backward
+ * pass knows every tensor that a queued reduction writes.  Returns 0 when that bookkeeping behaves. */
+int nrs_selftest_fold_bookkeeping(void);
 
 /* Measures the tensor pipe's dense-TF32 rate on this device (no reference counterpart): every SM
  * issues tcgen05.mma.kind::tf32 (128 x 256 x 8) back to back on operands resident in shared memory

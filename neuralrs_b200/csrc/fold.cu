@@ -245,9 +245,18 @@ void nrs_folds_free(nrs_ctx* ctx) {
   ctx->folds.chunks.clear();
 }
 
-int nrs_folds_settle(nrs_ctx* ctx, const float* dst) {
+// Whether a job writes any of the `len` floats at `p`.  (One job may write several tensors: a column pair has two
+// outputs, the weight gradients of Q, K and V lie one behind the other.)
+static bool writes(const NrsFoldJob& j, const float* p, size_t len) {
+  auto meets = [p, len](const float* at, size_t n) { return at < p + len && p < at + n; };
+  if (j.kind != NRS_FOLD_COLUMNS) return meets(j.dst, (size_t)j.co * j.ci * j.taps);
+  if (!j.dst2) return meets(j.dst, (size_t)j.cols);
+  return meets(j.dst, (size_t)j.cols1) || meets(j.dst2, (size_t)(j.cols - j.cols1));
+}
+
+int nrs_folds_settle(nrs_ctx* ctx, const float* dst, size_t len) {
   for (const NrsFoldJob& j : ctx->folds.jobs)
-    if (j.dst == dst || (j.dst2 && j.dst2 == dst)) return nrs_folds_flush(ctx);
+    if (writes(j, dst, len)) return nrs_folds_flush(ctx);
   return NRS_OK;
 }
 
@@ -307,8 +316,10 @@ int nrs_fold_submit(nrs_ctx* ctx, NrsFoldJob job) {
     f.tickets_used = 1;
     if (st != NRS_OK) return st;
   }
-  int st = nrs_folds_settle(ctx, job.dst);   // a second share of the same gradient: the first one goes ahead of it
-  if (st == NRS_OK && job.dst2) st = nrs_folds_settle(ctx, job.dst2);
+  // a second share of the same gradient: the first one goes ahead of it
+  const bool pair = job.kind == NRS_FOLD_COLUMNS && job.dst2;
+  int st = nrs_folds_settle(ctx, job.dst, job.kind != NRS_FOLD_COLUMNS ? (size_t)job.co * job.ci * job.taps : (size_t)(pair ? job.cols1 : job.cols));
+  if (st == NRS_OK && pair) st = nrs_folds_settle(ctx, job.dst2, (size_t)(job.cols - job.cols1));
   if (st != NRS_OK) return st;
   f.tickets_used += need;
   f.jobs.push_back(job);
@@ -345,4 +356,33 @@ int nrs_fold_columns(nrs_ctx* ctx, const float* src, float* dst, int rows, int c
 }
 int nrs_fold_column_pair(nrs_ctx* ctx, const float* src, float* dst, float* dst2, int rows, int cols, int stride, int accumulate) {
   return fold_columns_to(ctx, src, dst, dst2, cols, rows, 2 * cols, stride, accumulate);
+}
+
+// Host bookkeeping of the queue, without a device: how many checks failed (0 = all hold).
+extern "C" int nrs_selftest_fold_bookkeeping(void) {
+  int bad = 0;
+  static float mem[4096];   // addresses only
+  NrsFoldJob qkv{};         // three [8][8] weight gradients one behind the other
+  qkv.kind = NRS_FOLD_WGRAD;
+  qkv.dst = mem + 1024; qkv.co = 8; qkv.ci = 24; qkv.taps = 1; qkv.out_cols = 8;
+  for (int m = 0; m < 3; ++m) bad += writes(qkv, mem + 1024 + m * 64, 64) ? 0 : 1;
+  bad += writes(qkv, mem + 1024 - 64, 64) ? 1 : 0;
+  bad += writes(qkv, mem + 1024 + 192, 64) ? 1 : 0;
+  bad += writes(qkv, mem, 4096) ? 0 : 1;               // a gradient that holds all of it
+  NrsFoldJob conv{};                                    // [4][2][3][3]
+  conv.kind = NRS_FOLD_WGRAD_ROWS;
+  conv.dst = mem; conv.co = 4; conv.ci = 2; conv.taps = 9;
+  bad += writes(conv, mem + 71, 1) ? 0 : 1;
+  bad += writes(conv, mem + 72, 1) ? 1 : 0;
+  NrsFoldJob pair{};
+  pair.kind = NRS_FOLD_COLUMNS;
+  pair.dst = mem; pair.dst2 = mem + 512; pair.cols = 20; pair.cols1 = 10;
+  bad += writes(pair, mem + 9, 4) ? 0 : 1;
+  bad += writes(pair, mem + 10, 502) ? 1 : 0;
+  bad += writes(pair, mem + 521, 1) ? 0 : 1;
+  bad += writes(pair, mem + 522, 1) ? 1 : 0;
+  pair.dst2 = nullptr;                                  // all twenty columns in one place
+  bad += writes(pair, mem + 19, 1) ? 0 : 1;
+  bad += writes(pair, mem + 512, 10) ? 1 : 0;
+  return bad;
 }

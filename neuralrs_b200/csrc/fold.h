@@ -8,8 +8,9 @@ void nrs_folds_begin(nrs_ctx* ctx);
 int nrs_folds_flush(nrs_ctx* ctx);
 void nrs_folds_end(nrs_ctx* ctx);    // leaves the collecting mode; what is still queued is dropped (a failed pass)
 void nrs_folds_free(nrs_ctx* ctx);
-// Runs what is queued if it writes `dst`: called by whoever is about to read or add to a gradient.
-int nrs_folds_settle(nrs_ctx* ctx, const float* dst);
+// Runs what is queued if it writes any of the `len` floats at `dst`: called by whoever is about to read, overwrite or
+// add to a gradient.
+int nrs_folds_settle(nrs_ctx* ctx, const float* dst, size_t len);
 // Memory for a fold's partial sums that lives until the fold has run; outside of the collecting mode the given
 // workspace slot (-1: the context's workspace).
 int nrs_fold_partial(nrs_ctx* ctx, int ws_slot, size_t bytes, float** out);

@@ -100,7 +100,7 @@ struct GradTarget {
 static GradTarget grad_target(const NodeP& n) {
   Node* r = grad_root(n.get());
   if (!r->grad) r->grad = dalloc(r->ctx, r->len());
-  check(r->ctx, nrs_folds_settle(r->ctx, r->grad));   // an earlier share may still wait in the fold queue
+  check(r->ctx, nrs_folds_settle(r->ctx, r->grad, r->len()));   // an earlier share may still wait in the fold queue
   if (r->gz_valid) {   // another share arrives: what was derived from the first one is stale
     r->gz_valid = false;
     nrs_free(r->ctx, r->gplanes_hi);
@@ -126,7 +126,7 @@ static GradTarget grad_target(const NodeP& n) {
 static const float* grad_in(Node* n) {
   Node* r = grad_root(n);
   if (!r->grad) r->grad = dalloc(r->ctx, r->len());
-  check(r->ctx, nrs_folds_settle(r->ctx, r->grad));
+  check(r->ctx, nrs_folds_settle(r->ctx, r->grad, r->len()));
   if (!r->grad_valid) {
     check(r->ctx, nrs_memset_zero(r->ctx, r->grad, r->len() * sizeof(float)));
     r->grad_valid = true;

@@ -48,3 +48,9 @@ def test_shared_memory_attribute_bookkeeping_is_per_device(nrs_lib):
     """A kernel's dynamic shared-memory limit is a per-device setting; the launchers remember it per device
     ordinal (host-only self-test, no GPU needed)."""
     assert nrs_lib.nrs_selftest_smem_attr_bookkeeping() == 0
+
+
+def test_fold_queue_knows_every_tensor_it_writes(nrs_lib):
+    """A gradient that waits in the queue of second-stage reductions is found by any address inside it (host-only
+    self-test): one job may write several parameters' gradients."""
+    assert nrs_lib.nrs_selftest_fold_bookkeeping() == 0
