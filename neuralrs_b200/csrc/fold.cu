@@ -214,30 +214,42 @@ int run(nrs_ctx* ctx, NrsFoldJob* jobs, int n) {
   return NRS_OK;
 }
 
+// Launches what is queued.  Its partial sums stay where they are: place() says when their memory starts over.
+int run_queue(nrs_ctx* ctx) {
+  NrsFolds& f = ctx->folds;
+  if (f.jobs.empty()) return NRS_OK;
+  const int st = run(ctx, f.jobs.data(), (int)f.jobs.size());
+  ctx->independent_next = false;   // whoever writes into that memory next waits for this launch
+  f.jobs.clear();
+  f.tickets_used = 1;
+  return st;
+}
+
+// Memory for partial sums out of the blocks there are, or null.  The blocks start over only when nothing in them is
+// still to be read: no job is queued, and none is being made (its memory is handed out before the kernel that fills it
+// is launched and the job is submitted, and what comes in between may run the queue).
+float* place(NrsFolds& f, size_t bytes) {
+  if (f.jobs.empty() && !f.open) f.chunk = f.used = 0;
+  for (; f.chunk < f.chunks.size(); ++f.chunk, f.used = 0)
+    if (f.used + bytes <= f.chunks[f.chunk].second) {
+      float* p = (float*)((uint8_t*)f.chunks[f.chunk].first + f.used);
+      f.used += bytes;
+      f.open = true;
+      return p;
+    }
+  return nullptr;
+}
+
 }  // namespace
 
 void nrs_folds_begin(nrs_ctx* ctx) { ctx->folds.active = true; }
 
-int nrs_folds_flush(nrs_ctx* ctx) {
-  NrsFolds& f = ctx->folds;
-  int st = NRS_OK;
-  if (!f.jobs.empty()) {
-    st = run(ctx, f.jobs.data(), (int)f.jobs.size());
-    ctx->independent_next = false;   // the blocks start over: who writes them next waits for this launch
-  }
-  f.jobs.clear();
-  f.tickets_used = 1;
-  f.chunk = 0;
-  f.used = 0;
-  return st;
-}
+int nrs_folds_flush(nrs_ctx* ctx) { return run_queue(ctx); }
 
 void nrs_folds_end(nrs_ctx* ctx) {
-  ctx->folds.active = false;
+  ctx->folds.active = ctx->folds.open = false;
   ctx->folds.jobs.clear();
   ctx->folds.tickets_used = 1;
-  ctx->folds.chunk = 0;
-  ctx->folds.used = 0;
 }
 
 void nrs_folds_free(nrs_ctx* ctx) {
@@ -261,8 +273,8 @@ int nrs_folds_settle(nrs_ctx* ctx, const float* dst, size_t len) {
 }
 
 // Partial sums of a job that may wait live in blocks of their own (not pool blocks, which are handed out again as soon
-// as the host releases them, and not a shared slot, which the next layer overwrites).  64 MB at a time, 512 MB at most;
-// beyond that what is queued runs and the blocks start over.
+// as the host releases them, and not a shared slot, which the next layer overwrites).  64 MB at a time; at 512 MB what is
+// queued runs and the blocks start over, or, while a job is being made, there is one block more.
 int nrs_fold_partial(nrs_ctx* ctx, int ws_slot, size_t bytes, float** out) {
   NrsFolds& f = ctx->folds;
   void* p = nullptr;
@@ -273,30 +285,21 @@ int nrs_fold_partial(nrs_ctx* ctx, int ws_slot, size_t bytes, float** out) {
   }
   constexpr size_t kChunk = (size_t)64 << 20, kLimit = (size_t)512 << 20;
   bytes = (bytes + 255) / 256 * 256;
-  for (int pass = 0; pass < 2; ++pass) {
-    for (; f.chunk < f.chunks.size(); ++f.chunk, f.used = 0)
-      if (f.used + bytes <= f.chunks[f.chunk].second) {
-        *out = (float*)((uint8_t*)f.chunks[f.chunk].first + f.used);
-        f.used += bytes;
-        return NRS_OK;
-      }
-    size_t total = 0;
-    for (auto& c : f.chunks) total += c.second;
-    if (pass == 0 && total + bytes > kLimit && !f.chunks.empty()) {
-      const int st = nrs_folds_flush(ctx);   // starts over with the first block
-      if (st != NRS_OK) return st;
-      continue;
-    }
-    const size_t want = std::max(kChunk, bytes);
-    if (cudaMalloc(&p, want) != cudaSuccess) {
-      (void)cudaGetLastError();
-      return nrs_fail(ctx, NRS_ERR_ALLOC, "fold scratch: cudaMalloc(%zu) failed", want);
-    }
-    f.chunks.push_back({p, want});
+  if ((*out = place(f, bytes))) return NRS_OK;
+  size_t total = 0;
+  for (auto& c : f.chunks) total += c.second;
+  if (total + bytes > kLimit && !f.open && !f.jobs.empty()) {
+    const int st = run_queue(ctx);
+    if (st != NRS_OK) return st;
+    if ((*out = place(f, bytes))) return NRS_OK;
   }
-  f.chunk = f.chunks.size() - 1;
-  f.used = bytes;
-  *out = (float*)f.chunks.back().first;
+  const size_t want = std::max(kChunk, bytes);
+  if (cudaMalloc(&p, want) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return nrs_fail(ctx, NRS_ERR_ALLOC, "fold scratch: cudaMalloc(%zu) failed", want);
+  }
+  f.chunks.push_back({p, want});
+  *out = place(f, bytes);
   return NRS_OK;
 }
 
@@ -310,10 +313,7 @@ int nrs_fold_submit(nrs_ctx* ctx, NrsFoldJob job) {
   if (!f.active) return run(ctx, &job, 1);
   const unsigned need = job.kind == NRS_FOLD_COLUMNS && job.splits > 1 ? (unsigned)((job.cols + 31) / 32) : 0;
   if (f.jobs.size() >= (size_t)kMaxJobs || f.tickets_used + need > kNrsFoldTickets) {
-    // (the queue's partials stay where they are until the launch has read them: no reset of the blocks here)
-    const int st = run(ctx, f.jobs.data(), (int)f.jobs.size());
-    f.jobs.clear();
-    f.tickets_used = 1;
+    const int st = run_queue(ctx);
     if (st != NRS_OK) return st;
   }
   // a second share of the same gradient: the first one goes ahead of it
@@ -323,6 +323,7 @@ int nrs_fold_submit(nrs_ctx* ctx, NrsFoldJob job) {
   if (st != NRS_OK) return st;
   f.tickets_used += need;
   f.jobs.push_back(job);
+  f.open = false;
   return NRS_OK;
 }
 
@@ -384,5 +385,23 @@ extern "C" int nrs_selftest_fold_bookkeeping(void) {
   pair.dst2 = nullptr;                                  // all twenty columns in one place
   bad += writes(pair, mem + 19, 1) ? 0 : 1;
   bad += writes(pair, mem + 512, 10) ? 1 : 0;
+
+  // memory handed out stays its job's own until that job has been launched, whatever is launched before it
+  nrs_ctx c;
+  NrsFolds& f = c.folds;
+  f.active = true;
+  f.chunks = {{mem, 8192}, {mem + 2048, 8192}};
+  float* p[6] = {};
+  for (int i = 0; i < 2; ++i) bad += nrs_fold_partial(&c, -1, 1000, &p[i]) == NRS_OK ? 0 : 1;   // two blocks of one job
+  bad += p[0] == mem && p[1] == mem + 256 ? 0 : 1;
+  bad += nrs_fold_submit(&c, pair) == NRS_OK && f.jobs.size() == 1 ? 0 : 1;
+  bad += nrs_fold_partial(&c, -1, 4096, &p[2]) == NRS_OK && p[2] == mem + 512 ? 0 : 1;
+  f.jobs.clear();            // the queue is launched while the second job is being made
+  bad += nrs_fold_partial(&c, -1, 4096, &p[3]) == NRS_OK && p[3] == mem + 2048 ? 0 : 1;
+  bad += nrs_fold_submit(&c, pair) == NRS_OK ? 0 : 1;
+  bad += nrs_fold_partial(&c, -1, 4096, &p[4]) == NRS_OK && p[4] == mem + 3072 ? 0 : 1;
+  bad += nrs_fold_submit(&c, qkv) == NRS_OK && f.jobs.size() == 2 ? 0 : 1;
+  f.jobs.clear();
+  bad += nrs_fold_partial(&c, -1, 16, &p[5]) == NRS_OK && p[5] == mem ? 0 : 1;   // nothing waits: from the start again
   return bad;
 }

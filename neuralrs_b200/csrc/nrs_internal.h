@@ -154,6 +154,7 @@ struct NrsFolds {
   unsigned tickets_used = 1;
   std::vector<std::pair<void*, size_t>> chunks;   // memory for partial sums that wait
   size_t chunk = 0, used = 0;
+  bool open = false;       // some of it has been handed out for a job that is not submitted yet
 };
 
 struct nrs_ctx {
