@@ -211,6 +211,7 @@ int run(nrs_ctx* ctx, NrsFoldJob* jobs, int n) {
   if (blocks == 0) return NRS_OK;
   NRS_PDL_LAUNCH(fold_kernel, blocks, 256, 0, ctx->stream, b);
   NRS_LAUNCHED(ctx);
+  ctx->folds.launched_at = ctx->launches;
   return NRS_OK;
 }
 
@@ -403,5 +404,14 @@ extern "C" int nrs_selftest_fold_bookkeeping(void) {
   bad += nrs_fold_submit(&c, qkv) == NRS_OK && f.jobs.size() == 2 ? 0 : 1;
   f.jobs.clear();
   bad += nrs_fold_partial(&c, -1, 16, &p[5]) == NRS_OK && p[5] == mem ? 0 : 1;   // nothing waits: from the start again
+
+  // a weight gradient never starts under a launch of folds
+  c.launches = 7;
+  { NrsIndependentNext on(&c, true); bad += c.independent_next ? 0 : 1; }
+  f.launched_at = 7;
+  { NrsIndependentNext on(&c, true); bad += c.independent_next ? 1 : 0; }
+  c.launches = 8;            // the data gradient, issued after the folds
+  { NrsIndependentNext on(&c, true); bad += c.independent_next ? 0 : 1; }
+  { NrsIndependentNext off(&c, false); bad += c.independent_next ? 1 : 0; }
   return bad;
 }

@@ -155,6 +155,7 @@ struct NrsFolds {
   std::vector<std::pair<void*, size_t>> chunks;   // memory for partial sums that wait
   size_t chunk = 0, used = 0;
   bool open = false;       // some of it has been handed out for a job that is not submitted yet
+  uint64_t launched_at = ~0ull;   // nrs_ctx::launches right after the last launch of folds
 };
 
 struct nrs_ctx {
@@ -207,10 +208,12 @@ struct nrs_ctx {
 };
 
 // Marks, for the duration of a scope, that the kernel launched last wrote nothing the next tensor-core
-// weight-gradient launch reads (nrs_ctx::independent_next).
+// weight-gradient launch reads (nrs_ctx::independent_next).  Not where folds went out in between (asking for the place
+// of a shared weight's gradient may run the queue): that launch reads memory which the weight gradient's partial sums
+// are written to next.
 struct NrsIndependentNext {
   nrs_ctx* c;
-  NrsIndependentNext(nrs_ctx* ctx, bool on) : c(ctx) { c->independent_next = on; }
+  NrsIndependentNext(nrs_ctx* ctx, bool on) : c(ctx) { c->independent_next = on && c->launches != c->folds.launched_at; }
   ~NrsIndependentNext() { c->independent_next = false; }
   NrsIndependentNext(const NrsIndependentNext&) = delete;
   NrsIndependentNext& operator=(const NrsIndependentNext&) = delete;
