@@ -549,10 +549,15 @@ int layernorm_fwd(nrs_ctx* ctx, const char* who, const float* a, const float* b,
   if (rows == 0) return NRS_OK;
   NRS_REQUIRE(ctx, a && gamma && beta && y, NRS_ERR_ARG, "%s: null tensor", who);
   const int vpl = vec_vpl(f, {a, b, gamma, beta, y, xhat, y_hi, y_lo});
-  // Measured crossovers: [16384][1000] 41 us on the register kernel, 35 here; [4096][256] 4.6, 6.6; [20000][700] (a
-  // third of the lanes idle) 39, 40.  Scalar loops: [5000][1502] 30, 25; [16384][1001] 69, 72, with a residual 101, 78.
+  // Where the row pipeline is the better kernel (us here -> there, tensors that are not in L2).  Float4 rows without a
+  // residual: 16 M elements of 384 columns 40 -> 39, 448 41 -> 36, 512 39 -> 38, 1000 42 -> 36; not 256 (39, 51) or 768
+  // (40, 45; a quarter of the lanes idle).  With a residual (two inputs, two outputs) the register kernel is as good at
+  // every width: 256 47, 54; 512 47, 49; 1000 50, 50, and 114, 124 for 40 M elements.  Scalar loops: 1502 columns 62 -> 51,
+  // 3000 76 -> 43, not 1401 (83, 112; 2.7 live warps); with a residual 1001 100 -> 82, 3000 128 -> 49, not 1281 (98, 130).
   const size_t elems = (size_t)rows * f;
-  const bool pipe = elems >= 6000000 && rowpipe::fill(f) >= 0.75 && (vpl || f >= (b ? 960 : 1400));
+  const double fill = rowpipe::fill(f), live = rowpipe::live_warps(f, 2);
+  const bool pipe = elems >= 6000000 && (vpl ? !b && f >= 384 && (f <= 512 || fill >= 0.8)
+                                             : fill >= 0.75 && (b ? f >= 960 && live >= 3.8 : f >= 1400 && live >= 5.0));
   if (!(y_hi && vpl) && pipe && rowpipe::applies(rows, f, {a, b, gamma, beta, y, xhat})) {
     rowpipe::Params p{};
     p.in[0] = a; p.in[1] = b; p.n_in = b ? 2 : 1; p.n_buf = 2;
@@ -599,8 +604,22 @@ int layernorm_bwd(nrs_ctx* ctx, const char* who, const float* g, const float* xh
   NRS_REQUIRE(ctx, g && xhat && istd && gamma, NRS_ERR_ARG, "%s: null tensor", who);
   if (!dx && !dgamma) return NRS_OK;
   const int vpl = vec_vpl(f, {g, xhat, gamma, dx, dx2, d_hi, d_lo});
-  // (register kernel: [16384][1000] 99 us, 44 here, even at 4 M elements; the scalar loops read g and xhat twice)
-  if (!(d_hi && vpl) && (!vpl || (size_t)rows * f >= (size_t)1 << 22) && rowpipe::applies(rows, f, {g, xhat, gamma, dx, dx2})) {
+  // Where the row pipeline is the better kernel (us here -> there, tensors that are not in L2).  Float4 rows: beyond 256
+  // columns, from 4 M elements up.  dx and parameters of 16 M elements: 260 columns 71 -> 68, 320 69 -> 58, 512 59 -> 42,
+  // 768 98 -> 46, 1000 104 -> 41; but 64 columns 76, 87, 128 48, 67, 256 44, 56 (dx alone 38, 52; parameters alone 30, 36).
+  // Scalar loops, which read g and xhat twice: for dx and parameters from 256 K elements (17 columns 9.8 -> 9.2, 1001
+  // 14 -> 12; 128 K of 385: 8.8, 11.0) or 1024 columns; for parameters alone from 4 M (1001 columns 19 -> 16, 1 M 8.5,
+  // 10.9), 8 M beyond 4000 columns (4 M of 8192: 15, 20); for dx alone with enough columns at work: 16 M elements of 250
+  // columns 63 -> 41, 1002 72 -> 42, 1001 72 -> 56, not 777 (58, 70; 3.1 live warps) or 1281 (64, 83; 2.5), which are taken
+  // only while the rows are few (up to 1.5 M elements; 200 K of 1401 columns: 10.8 -> 5.2).
+  const size_t elems = (size_t)rows * f;
+  const double fill = rowpipe::fill(f), live = rowpipe::live_warps(f, 2);
+  const bool pipe = vpl            ? f > 256 && elems >= (size_t)1 << 22
+                    : dx && dgamma ? f >= 1024 || elems >= (size_t)1 << 18
+                    : dgamma       ? elems >= (size_t)1 << (f <= 4000 ? 22 : 23)
+                                   : (fill >= 0.75 && live >= 5.0) || (fill >= 0.85 && live >= 3.8) || (elems >= (size_t)1 << 23 && live >= 4.5) ||
+                                         (f > 640 && elems < (size_t)3 << 19);
+  if (!(d_hi && vpl) && pipe && rowpipe::applies(rows, f, {g, xhat, gamma, dx, dx2})) {
     rowpipe::Params p{};
     p.in[0] = g; p.in[1] = xhat; p.n_in = p.n_buf = 2;
     p.out[0] = dx; p.out_add[0] = acc1;

@@ -11,9 +11,12 @@
 // warps per SM and no dependence on occupancy.  (The register kernels it replaces at these sizes keep a row per
 // warp in flight: 80 to 160 registers per thread left them latency-bound.)
 //
-// Measured on [16384][1000] (us before -> after; 40, 40, 30, 30 at the measured copy rate): LayerNorm backward with
-// residual and parameters 102 -> 48, LayerNorm forward 52 -> 52, cross-entropy 55 -> 48, softmax backward 34 -> 32.
-// What is left of the gap is work inside a row (reductions, exponentials), not bytes in flight.
+// Measured on [16384][1000] (us, the kernel it replaces -> this one; 40, 30 at the measured copy rate): LayerNorm
+// backward with parameters 104 -> 41, dx alone 96 -> 34, LayerNorm forward 42 -> 36, cross-entropy 52 -> 48.  It is not the
+// better kernel at every width: what decides is how many warps' worth of columns an SM works on (live_warps below) and how
+// much a row costs besides its bytes (a barrier wait, a proxy fence, two team syncs and a store issued by one lane: at
+// 256 columns a row is 1 KB, and LayerNorm backward takes 56 us for 16 M elements against 44 in registers).  The
+// operators state their own lines with both sides measured.
 #pragma once
 
 #include "nrs_internal.h"
@@ -208,10 +211,39 @@ row_pipe_kernel(const Params p, const Op op, int* __restrict__ err_flag) {
   op.template finish<NPL, VEC>(tm, cols, state, reinterpret_cast<float*>(smem_raw + 2048), team, teams);
 }
 
-// Share of a row's lanes x elements that hold columns (see launch()).
+// Elements per lane by width: 8 up to 256 columns, else 16, a row of more than 512 columns being shared by a team of
+// warps (with 32 per lane, one warp per row of 1000 columns, shared memory had room for eight or nine warps and the
+// exponentials of a softmax ran at a third of the rate: 65 us).
+struct Plan {
+  int npl, team_warps, group_rows, teams;   // teams: 0 when three slots of one team do not fit
+  size_t slot;
+};
+constexpr size_t kHead = 2048, kBudget = 220 * 1024 - kHead;
+inline Plan plan(int f, int n_buf) {
+  Plan q{};
+  q.npl = f <= 256 ? 8 : 16;
+  q.team_warps = (f + q.npl * 32 - 1) / (q.npl * 32);
+  // rows per slot: whole 16-byte groups, and at least 1 KB per copy
+  const int unit = f % 4 == 0 ? 1 : f % 2 == 0 ? 2 : 4;
+  q.group_rows = unit;
+  while (q.group_rows * f * 4 < 1024) q.group_rows += unit;
+  q.slot = (size_t)q.group_rows * f * 4 * n_buf;
+  int warps = kThreads / 32;
+  while (warps > q.team_warps && (size_t)(warps / q.team_warps) * 3 * q.slot > kBudget) --warps;
+  q.teams = warps / q.team_warps;
+  if (q.teams > 0 && kBudget / (q.slot * q.teams) < 3) q.teams = 0;
+  return q;
+}
+// Share of a row's lanes x elements that hold columns.
 inline double fill(int f) {
   const int unit = 32 * (f <= 256 ? 8 : 16);
   return (double)f / ((f + unit - 1) / unit * unit);
+}
+// Warps' worth of columns an SM works on: the warps whose slots fit into shared memory (16 at most; groups of four rows
+// of an odd width leave 3 of 1401 columns) times their fill.  With few of them the work inside a row is not hidden.
+inline double live_warps(int f, int n_buf) {
+  const Plan q = plan(f, n_buf);
+  return q.teams * q.team_warps * fill(f);
 }
 // Whether a tensor set can take this path: 16-byte aligned bases, rows of at most 8192 columns (one slot of two
 // buffers is then 64 KB), 128 K elements (below, a shorter prologue wins: [64][10] 4 us against 20).  The operators add
@@ -225,22 +257,17 @@ inline bool applies(int rows, int f, std::initializer_list<const void*> ptrs) {
 
 template <int NPL, int VEC, class Op>
 int launch_one(nrs_ctx* ctx, Params p, const Op& op, int* blocks_out) {
-  constexpr size_t kHead = 2048, kBudget = 220 * 1024 - kHead;
-  p.team_warps = (p.f + NPL * 32 - 1) / (NPL * 32);
-  // rows per slot: whole 16-byte groups, and at least 1 KB per copy
-  const int unit = p.f % 4 == 0 ? 1 : p.f % 2 == 0 ? 2 : 4;
-  p.group_rows = unit;
-  while (p.group_rows * p.f * 4 < 1024) p.group_rows += unit;
-  const size_t slot = (size_t)p.group_rows * p.f * 4 * p.n_buf;
-  int warps = kThreads / 32;
-  while (warps > p.team_warps && (size_t)(warps / p.team_warps) * 3 * slot > kBudget) --warps;
-  int teams = warps / p.team_warps;
+  const Plan q = plan(p.f, p.n_buf);
+  if (q.teams == 0) return NRS_ERR_UNSUPPORTED;
+  p.team_warps = q.team_warps;
+  p.group_rows = q.group_rows;
+  const size_t slot = q.slot;
+  int teams = q.teams;
   // fewer rows than teams: spread them over the SMs
   const long groups = ((long)p.rows + p.group_rows - 1) / p.group_rows;
   while (teams > 1 && (long)(teams - 1) * ctx->sm_count >= groups) --teams;
   p.slots = (int)(kBudget / (slot * teams));
   if (p.slots > 6) p.slots = 6;
-  if (p.slots < 3) return NRS_ERR_UNSUPPORTED;
   long blocks = (groups + teams - 1) / teams;
   if (blocks > ctx->sm_count) blocks = ctx->sm_count;
   size_t smem = kHead + (size_t)teams * p.slots * slot;
@@ -258,10 +285,7 @@ int launch_one(nrs_ctx* ctx, Params p, const Op& op, int* blocks_out) {
   return NRS_OK;
 }
 
-// Elements per lane by width: 8 up to 256 columns, else 16, a row of more than 512 columns being shared by a team of
-// warps (with 32 per lane, one warp per row of 1000 columns, shared memory had room for eight or nine warps and the
-// exponentials of a softmax ran at a third of the rate: 65 us).  Rows whose width is a multiple of four move through
-// registers as float4s.
+// Rows whose width is a multiple of four move through registers as float4s.
 template <class Op>
 int launch(nrs_ctx* ctx, const Params& p, const Op& op, int* blocks_out = nullptr) {
   if (p.f % 4 == 0) return p.f <= 256 ? launch_one<8, 4>(ctx, p, op, blocks_out) : launch_one<16, 4>(ctx, p, op, blocks_out);

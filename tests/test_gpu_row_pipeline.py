@@ -48,3 +48,29 @@ def test_row_pipeline(gpu_ctx, oracle64, rows, f):
         call(gpu_ctx, name, xd, target, loss, o1, rows, f, rows)
         assert abs(loss.get()[0] - ref_loss) <= 1e-5 * max(1.0, abs(ref_loss))
         assert np.linalg.norm(o1.get() - (pr - t) / rows) <= 2e-6 * np.linalg.norm(t) / rows
+
+
+# Both sides of the lines between the pipeline and the kernels it stands beside (rows, columns).
+LINES = [(16500, 256), (16140, 260), (15700, 384), (6100, 1000), (1024, 255), (1029, 255), (200, 1025), (127, 1028), (8400, 501), (1050, 4004),
+         (2100, 4004), (5400, 777), (4300, 1402), (4300, 1403), (149, 1401), (1125, 1401)]
+
+
+@pytest.mark.parametrize("rows,f", LINES)
+def test_layernorm_beside_its_lines(gpu_ctx, oracle64, rows, f):
+    rng = np.random.default_rng(rows * 3 + f)
+    x, g = (rng.normal(size=(rows, f)).astype(np.float32) for _ in range(2))
+    gamma, beta = rng.normal(size=f).astype(np.float32), rng.normal(size=f).astype(np.float32)
+    xd, gd, gm, bt = (Dev(gpu_ctx, v) for v in (x, g, gamma, beta))
+    y, xh, dx = (Dev(gpu_ctx, shape=(rows, f)) for _ in range(3))
+    ist, dg, db = Dev(gpu_ctx, shape=(rows,)), Dev(gpu_ctx, np.ones(f, np.float32)), Dev(gpu_ctx, np.ones(f, np.float32))
+    yr, xhr, isr = oracle64.layernorm_fwd(x, gamma, beta, 1e-5)
+    call(gpu_ctx, "nrs_layernorm_fwd", xd, gm, bt, y, xh, ist, rows, f, F(1e-5))
+    assert np.abs(y.get() - yr).max() <= 2e-4 and np.abs(xh.get() - xhr).max() <= 2e-4 and rel_l2(ist.get(), isr) <= 1e-6
+    dxr, dgr, dbr = oracle64.layernorm_bwd(g, xhr, isr, gamma)
+    call(gpu_ctx, "nrs_layernorm_bwd", gd, xh, ist, gm, dx, None, None, rows, f, 0, 0)
+    assert rel_l2(dx.get(), dxr) <= 2e-5
+    for k in (1, 2):   # parameters alone, added to what is there
+        call(gpu_ctx, "nrs_layernorm_bwd", gd, xh, ist, gm, None, dg, db, rows, f, 0, 1)
+        assert rel_l2(dg.get() - 1.0, k * dgr) <= 2e-5 and rel_l2(db.get() - 1.0, k * dbr) <= 2e-5
+    call(gpu_ctx, "nrs_layernorm_bwd", gd, xh, ist, gm, dx, dg, db, rows, f, 1, 0)
+    assert rel_l2(dx.get(), 2.0 * dxr) <= 2e-5 and rel_l2(dg.get(), dgr) <= 1e-5 and rel_l2(db.get(), dbr) <= 1e-5
