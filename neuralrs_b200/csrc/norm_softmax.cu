@@ -743,9 +743,15 @@ int nrs_softmax_fwd(nrs_ctx* ctx, const float* x, float* y, int rows, int width)
   NRS_REQUIRE(ctx, x && y, NRS_ERR_ARG, "nrs_softmax_fwd: null tensor");
   const int vpl = vec_vpl(width, {x, y});
   // (widths the vector kernel takes stay there at every size: bound by its exponentials and divisions, not by HBM, it
-  // does better with a full SM of warps: [16384][1000] 24 us against 54)
-  // Scalar loops: [5000][1502] 28 us, 24 here; [16384][1001] 45, 64; [2000][2050] 18, 29.
-  if (!vpl && width >= 1400 && (size_t)rows * width >= 6000000 && rowpipe::applies(rows, width, {x, y})) {
+  // does better with a full SM of warps: [16384][1000] 23 us against 54)
+  // Against the scalar loops, with hardly a lane idle and enough columns at work (us there -> here): 8 M elements of 1502
+  // columns 34 -> 26, 3000 39 -> 35; 16 M of 4096 91 -> 46.  Not 1401 (34, 48), 2050 (30, 48; a fifth of the lanes idle)
+  // or 2001 (30, 40; 7.8 live warps), and up to 3400 columns not beyond 24 M elements (40 M of 2000: 118, 128).
+  const size_t elems = (size_t)rows * width;
+  const double live = rowpipe::live_warps(width, 1);
+  const bool pipe = !vpl && width >= 1400 && elems >= 6000000 && rowpipe::fill(width) >= 0.95 &&
+                    ((width >= 3400 && live >= 13.0) || (elems <= (size_t)24 << 20 && live >= 9.5));
+  if (pipe && rowpipe::applies(rows, width, {x, y})) {
     rowpipe::Params p{};
     p.in[0] = x; p.n_in = p.n_buf = 1;
     p.out[0] = y;
@@ -768,8 +774,8 @@ int nrs_softmax_bwd(nrs_ctx* ctx, const float* y, const float* g, float* dx, int
   if (rows == 0) return NRS_OK;
   NRS_REQUIRE(ctx, y && g && dx, NRS_ERR_ARG, "nrs_softmax_bwd: null tensor");
   const int vpl = vec_vpl(width, {y, g, dx});
-  // Only against the scalar loops ([16384][1001] 60 us, 36 here; [10086][518], half of the lanes idle, 12, 14): the
-  // register kernel takes 28 us for [16384][1000], 33 here.
+  // Only against the scalar loops ([16384][1001] 61 us, 37 here; 1 M elements of 50 columns, most lanes idle, 6.2, 8.2):
+  // the register kernel takes 32 us for [16384][1000], and is the better one at every float4 width.
   if (!vpl && rowpipe::fill(width) >= 0.75 && rowpipe::applies(rows, width, {y, g, dx})) {
     rowpipe::Params p{};
     p.in[0] = y; p.in[1] = g; p.n_in = p.n_buf = 2;

@@ -74,3 +74,19 @@ def test_layernorm_beside_its_lines(gpu_ctx, oracle64, rows, f):
         assert rel_l2(dg.get() - 1.0, k * dgr) <= 2e-5 and rel_l2(db.get() - 1.0, k * dbr) <= 2e-5
     call(gpu_ctx, "nrs_layernorm_bwd", gd, xh, ist, gm, dx, dg, db, rows, f, 1, 0)
     assert rel_l2(dx.get(), 2.0 * dxr) <= 2e-5 and rel_l2(dg.get(), dgr) <= 1e-5 and rel_l2(db.get(), dbr) <= 1e-5
+
+
+SOFTMAX_LINES = [(4300, 1401), (4000, 1502), (2950, 2050), (2050, 3000), (17000, 1502), (1500, 4096)]
+
+
+@pytest.mark.parametrize("rows,f", SOFTMAX_LINES)
+def test_softmax_beside_its_lines(gpu_ctx, oracle64, rows, f):
+    rng = np.random.default_rng(rows + 5 * f)
+    x = (4.0 * rng.normal(size=(rows, f))).astype(np.float32)
+    x[1, ::2] = np.finfo(np.float32).min   # a masked row, and one with a single live column
+    x[2, 1:] = -np.inf
+    xd, y = Dev(gpu_ctx, x), Dev(gpu_ctx, shape=(rows, f))
+    call(gpu_ctx, "nrs_softmax_fwd", xd, y, rows, f)
+    got = y.get()
+    assert rel_l2(got, oracle64.softmax_fwd(x)) <= 1e-6
+    assert (got[1, ::2] == 0).all() and got[2, 0] == 1.0 and (got[2, 1:] == 0).all()
