@@ -100,6 +100,10 @@ struct CeOp {
 
 // One warp per row.  row_loss (optional) gets -sum_c t*(x - lse); grad (optional)
 // gets (softmax - t) * inv_div.  Scalar path (any width / alignment).
+// FOLD: the kernel also folds the batch mean, which saves a launch; without, row_loss is left to ce_mean_kernel.  The
+// fold costs the loops 8 of their 40 registers' worth of scheduling and every block a fence and an atomic, so it is for
+// small calls (see run_ce): [64][10] 6.0 us with two launches, 4.0 with one; [16760][1001] with labels 64 and 85.
+template <bool FOLD>
 __global__ void __launch_bounds__(256)
 ce_rows_kernel(const float* __restrict__ logits, const float* __restrict__ target, const int32_t* __restrict__ labels,
                float* __restrict__ row_loss, float* __restrict__ grad, int batch, int classes, float inv_div, float* block_partial,
@@ -125,16 +129,43 @@ ce_rows_kernel(const float* __restrict__ logits, const float* __restrict__ targe
       loss += -tv * (xv - lse);
       if (grad) grad[(size_t)b * classes + c] = (expf(xv - mx) / se - tv) * inv_div;
     }
-    if (row_loss || loss_dev) {
+    if (FOLD || row_loss) {
       loss = warp_sum(loss);
       if (row_loss && lane == 0) row_loss[b] = loss;
-      warp_loss += loss;
+      if (FOLD) warp_loss += loss;
     }
   }
-  if (!loss_dev) return;
-  __shared__ float wsum[32];
-  if (lane == 0) wsum[threadIdx.x >> 5] = warp_loss;
-  fold_batch_loss(wsum, warps_per_block, block_partial, ticket, loss_dev, inv_div);
+  if (FOLD) {
+    __shared__ float wsum[32];
+    if (lane == 0) wsum[threadIdx.x >> 5] = warp_loss;
+    fold_batch_loss(wsum, warps_per_block, block_partial, ticket, loss_dev, inv_div);
+  }
+}
+
+// loss_dev[0] = (sum_b row_loss[b]) * inv_div, one block, fixed summation tree.
+__global__ void __launch_bounds__(1024)
+ce_mean_kernel(const float* __restrict__ row_loss, float* __restrict__ loss_dev, int batch, float inv_div) {
+  NRS_PDL_PROLOGUE();
+  __shared__ float sm[32];
+  float s = 0.0f;
+  int i = threadIdx.x;
+  const int step = blockDim.x;
+  for (; i + 7 * step < batch; i += 8 * step) {   // eight loads in flight; the additions keep the order of i
+    float v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = row_loss[i + u * step];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) s += v[u];
+  }
+  for (; i < batch; i += step) s += row_loss[i];
+  s = warp_sum(s);
+  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    float t = threadIdx.x < (blockDim.x >> 5) ? sm[threadIdx.x] : 0.0f;
+    t = warp_sum(t);
+    if (threadIdx.x == 0) loss_dev[0] = t * inv_div;
+  }
 }
 
 // The same with the row held in registers: logits (and the one-hot row) are read once with 128-bit
@@ -265,15 +296,23 @@ int run_ce(nrs_ctx* ctx, const char* who, const float* logits, const float* targ
   if (classes > 512 && blocks > ctx->sm_count * 3) blocks = ctx->sm_count * 3;
   const bool vec = classes % 4 == 0 && classes <= 1024 &&
                    ((reinterpret_cast<uintptr_t>(logits) | reinterpret_cast<uintptr_t>(target) | reinterpret_cast<uintptr_t>(grad)) & 15) == 0;
-  // the kernels fold the batch mean themselves (per-block partial sums, last block folds)
+  // The vector kernels fold the batch mean themselves (per-block partial sums, last block folds), the scalar one where
+  // a launch weighs more, or where the mean's own launch has very many rows to add.  us with two launches and with one:
+  // 64 x 10 6.0, 4.0; 2048 x 33 6.0, 4.6; 8192 x 33 6.4, 8.5; 512 x 127 5.9, 6.3, with labels (a tensor less to read) 5.9,
+  // 5.0; 512 x 255 7.0, 7.5; with labels 133455 x 33 63, 58 and 9532 x 33 8.6, 9.0; with a one-hot target 508400 x 33 241,
+  // 232 and 133455 x 33 67, 67.
+  const bool small = batch <= 4096 && classes <= (target ? 64 : 128) && (size_t)batch * classes <= (size_t)1 << (target ? 17 : 18);
+  const bool fold = vec || small || batch >= 1 << (target ? 18 : 16);
+  float* rl = row_loss;
   float* partial = nullptr;
   unsigned* ticket = nullptr;
   if (loss_dev) {
     void* ws = nullptr;
-    int st = nrs_workspace(ctx, (size_t)blocks * sizeof(float) + 16, &ws);
-    if (st == NRS_OK) st = nrs_fold_ticket(ctx, &ticket);
+    int st = nrs_workspace(ctx, (size_t)(fold ? blocks : rl ? 0 : batch) * sizeof(float) + 16, &ws);
+    if (st == NRS_OK && fold) st = nrs_fold_ticket(ctx, &ticket);
     if (st != NRS_OK) return st;
-    partial = (float*)ws;
+    if (fold) partial = (float*)ws;
+    else if (!rl) rl = (float*)ws;
   }
   if (vec && classes <= 128) {
     NRS_PDL_LAUNCH(ce_rows_vec_kernel<1>, blocks, 256, 0, ctx->stream, logits, target, labels, row_loss, grad, batch, classes, inv_div,
@@ -285,10 +324,18 @@ int run_ce(nrs_ctx* ctx, const char* who, const float* logits, const float* targ
     NRS_PDL_LAUNCH(ce_rows_vec_kernel<8>, blocks, 256, 0, ctx->stream, logits, target, labels, row_loss, grad, batch, classes, inv_div,
                    partial, ticket, loss_dev);
   } else {
-    NRS_PDL_LAUNCH(ce_rows_kernel, blocks, 256, 0, ctx->stream, logits, target, labels, row_loss, grad, batch, classes, inv_div, partial, ticket,
-                   loss_dev);
+    if (loss_dev && fold)
+      NRS_PDL_LAUNCH(ce_rows_kernel<true>, blocks, 256, 0, ctx->stream, logits, target, labels, rl, grad, batch, classes, inv_div, partial,
+                     ticket, loss_dev);
+    else
+      NRS_PDL_LAUNCH(ce_rows_kernel<false>, blocks, 256, 0, ctx->stream, logits, target, labels, rl, grad, batch, classes, inv_div,
+                     (float*)nullptr, (unsigned*)nullptr, (float*)nullptr);
   }
   NRS_LAUNCHED(ctx);
+  if (loss_dev && !fold) {
+    NRS_PDL_LAUNCH(ce_mean_kernel, 1, 1024, 0, ctx->stream, rl, loss_dev, batch, inv_div);
+    NRS_LAUNCHED(ctx);
+  }
   return NRS_OK;
 }
 

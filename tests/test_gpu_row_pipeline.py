@@ -90,3 +90,28 @@ def test_softmax_beside_its_lines(gpu_ctx, oracle64, rows, f):
     got = y.get()
     assert rel_l2(got, oracle64.softmax_fwd(x)) <= 1e-6
     assert (got[1, ::2] == 0).all() and got[2, 0] == 1.0 and (got[2, 1:] == 0).all()
+
+
+# The scalar kernel with its own mean and with a second launch for it (rows, columns).
+CE_LINES = [(1, 7), (2048, 63), (2100, 63), (4096, 31), (4097, 31), (2048, 127), (300, 1001), (65535, 7), (65536, 7), (262144, 3)]
+
+
+@pytest.mark.parametrize("rows,f", CE_LINES)
+def test_cross_entropy_beside_its_lines(gpu_ctx, oracle64, rows, f):
+    rng = np.random.default_rng(rows + 7 * f)
+    x = (3.0 * rng.normal(size=(rows, f))).astype(np.float32)
+    labels = rng.integers(0, f, rows).astype(np.int32)
+    t = np.zeros((rows, f), np.float32)
+    t[np.arange(rows), labels] = 1.0
+    xd, td, lb = (Dev(gpu_ctx, v) for v in (x, t, labels))
+    g, loss, rl = Dev(gpu_ctx, shape=(rows, f)), Dev(gpu_ctx, shape=(1,)), Dev(gpu_ctx, shape=(rows,))
+    p = oracle64.softmax_fwd(x)
+    each = -np.log(p[np.arange(rows), labels].astype(np.float64))
+    for name, target in (("nrs_ce_fwd_bwd", td), ("nrs_ce_fwd_bwd_indexed", lb)):
+        call(gpu_ctx, name, xd, target, loss, g, rows, f, rows)
+        assert abs(loss.get()[0] - each.mean()) <= 1e-5 * each.mean()
+        assert np.linalg.norm(g.get() - (p - t) / rows) <= 2e-6 * np.linalg.norm(t) / rows
+    call(gpu_ctx, "nrs_ce_fwd", xd, td, None, rl, rows, f, rows)
+    assert rel_l2(rl.get(), each) <= 1e-6
+    call(gpu_ctx, "nrs_ce_fwd", xd, td, loss, rl, rows, f, 2 * rows)
+    assert abs(loss.get()[0] - each.mean() / 2) <= 1e-5 * each.mean() and rel_l2(rl.get(), each) <= 1e-6
