@@ -267,12 +267,22 @@ int run_ce(nrs_ctx* ctx, const char* who, const float* logits, const float* targ
   }
   NRS_REQUIRE(ctx, logits && (target || labels), NRS_ERR_ARG, "%s: null tensor", who);
   const float inv_div = 1.0f / (float)divisor;
-  // (rows that a register kernel takes: from 32 MB per tensor, beyond what the L2 cache holds of logits and gradient;
-  // [4096][1000] 16.5 us there against 19 here, [16384][1000] 55 against 48)
-  // Crossover against the warp-per-row kernels: [16384][1000] 50 us, 46 here; [16384][1001] 128, 102; [3000][1001] 16, 24;
-  // [20000][700] 44, 52 and [40000][777] 218, 233 (lanes idle, two warps to a row).
-  if ((size_t)batch * classes >= (size_t)1 << 23 && rowpipe::fill(classes) >= 0.75 && (classes <= 512 || classes >= 960) &&
-      rowpipe::applies(batch, classes, {logits, target, grad})) {
+  // Where the row pipeline is the better kernel: from 8 M elements up (us here -> there, tensors that are not in L2).
+  // Float4 rows: with a one-hot target [16384][1000] 52 -> 48, 1024 columns 52 -> 45, 512 46 -> 43 (but 64 M elements 146, 155); not 256 (50, 61) or 384 (46, 52); with
+  // labels nowhere (1000: 40, 50; 256: 46, 71).  Scalar loops, with a one-hot target: 16 M elements of 250 columns 107 -> 53,
+  // 385 95 -> 85, 1001 129 -> 107, 3000 136 -> 61, not 1281 (120, 162; 2.5 live warps) or 700 (44, 52 in [20000][700]); with
+  // labels, one tensor less to bring in, only with more columns at work: 250 73 -> 61, 1002 64 -> 50, 4096 97 -> 51, not
+  // 385 (54, 60), 1001 (64, 70), 1281 (59, 73) or 2999 (75, 90).
+  const bool vec = classes % 4 == 0 && classes <= 1024 &&
+                   ((reinterpret_cast<uintptr_t>(logits) | reinterpret_cast<uintptr_t>(target) | reinterpret_cast<uintptr_t>(grad)) & 15) == 0;
+  const double fill = rowpipe::fill(classes), live = rowpipe::live_warps(classes, target ? 2 : 1);
+  const bool wide = classes <= 512 || classes >= 960;
+  const size_t elems = (size_t)batch * classes;
+  const bool pipe = elems >= (size_t)1 << 23 && fill >= 0.75 &&
+                    (vec      ? target && (classes >= 960 || (classes >= 448 && classes <= 512 && elems < (size_t)1 << 25))
+                     : target ? wide && live >= 3.5
+                              : wide && live >= 9.5 && (fill >= 0.85 || classes > 1500));
+  if (pipe && rowpipe::applies(batch, classes, {logits, target, grad})) {
     rowpipe::Params p{};
     p.in[0] = logits; p.in[1] = target;
     p.n_in = p.n_buf = target ? 2 : 1;
@@ -294,8 +304,6 @@ int run_ce(nrs_ctx* ctx, const char* who, const float* logits, const float* targ
   // wide rows: one resident wave (three blocks of 80 registers per SM) of warps that walk several rows each,
   // prefetching the next
   if (classes > 512 && blocks > ctx->sm_count * 3) blocks = ctx->sm_count * 3;
-  const bool vec = classes % 4 == 0 && classes <= 1024 &&
-                   ((reinterpret_cast<uintptr_t>(logits) | reinterpret_cast<uintptr_t>(target) | reinterpret_cast<uintptr_t>(grad)) & 15) == 0;
   // The vector kernels fold the batch mean themselves (per-block partial sums, last block folds), the scalar one where
   // a launch weighs more, or where the mean's own launch has very many rows to add.  us with two launches and with one:
   // 64 x 10 6.0, 4.0; 2048 x 33 6.0, 4.6; 8192 x 33 6.4, 8.5; 512 x 127 5.9, 6.3, with labels (a tensor less to read) 5.9,

@@ -92,8 +92,9 @@ def test_softmax_beside_its_lines(gpu_ctx, oracle64, rows, f):
     assert (got[1, ::2] == 0).all() and got[2, 0] == 1.0 and (got[2, 1:] == 0).all()
 
 
-# The scalar kernel with its own mean and with a second launch for it (rows, columns).
-CE_LINES = [(1, 7), (2048, 63), (2100, 63), (4096, 31), (4097, 31), (2048, 127), (300, 1001), (65535, 7), (65536, 7), (262144, 3)]
+# Both sides of the lines against the pipeline; the scalar kernel with its own mean and with a second launch for it.
+CE_LINES = [(8400, 1000), (16400, 512), (33000, 256), (33000, 255), (21900, 385), (6600, 1281), (5600, 1502), (5600, 1501),
+            (1, 7), (2048, 63), (2100, 63), (4096, 31), (4097, 31), (2048, 127), (300, 1001), (65535, 7), (65536, 7), (262144, 3)]
 
 
 @pytest.mark.parametrize("rows,f", CE_LINES)
