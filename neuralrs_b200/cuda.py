@@ -13,6 +13,7 @@ numpy arrays and handles.  Reference: src/cuda/{runtime,graph,nn,loss,optim}.
 """
 from __future__ import annotations
 
+import collections
 import ctypes as C
 import threading
 
@@ -77,28 +78,58 @@ def _ptr(a: np.ndarray) -> VP:
 class _PinnedPool:
     """Page-locked blocks behind the arrays that read-backs return: a copy from the device lands in them at the bus rate
     (8 MB: 0.17 ms against 0.54 into pageable memory).  A block goes back to the pool when the last array that uses it is
-    gone; the pool keeps at most `limit` bytes of idle blocks, the rest is released.  Safe with several threads."""
+    gone; the pool keeps at most `limit` bytes of idle blocks, the rest is released.  Blocks in use count too: no more
+    than `most` bytes are page-locked at a time, and read-backs beyond that get ordinary memory.  Safe with several
+    threads."""
 
-    def __init__(self, limit: int = 256 << 20):
-        self.limit, self.idle, self.free, self.lock = limit, 0, {}, threading.Lock()
+    def __init__(self, limit: int = 256 << 20, most: int = 1 << 30):
+        self.limit, self.most, self.idle, self.locked = limit, most, 0, 0
+        self.free, self.lock = {}, threading.Lock()
+        self.returned = collections.deque()      # blocks on their way back
 
     def take(self, nbytes: int):
         size = -(-nbytes // 65536) * 65536
         with self.lock:
+            self._sort_in()
             blocks = self.free.get(size)
             if blocks:
                 self.idle -= size
                 return blocks.pop(), size
+            for other, idle in self.free.items():    # room for this size: idle blocks of others go first
+                while idle and self.locked + size > self.most:
+                    self._release(idle.pop(), other)
+                    self.idle -= other
+            if self.locked + size > self.most:
+                return None, 0
+            self.locked += size
         p = VP()
-        return (p.value, size) if _lib.lib().nrs_host_alloc(size, C.byref(p)) == 0 else (None, 0)
+        if _lib.lib().nrs_host_alloc(size, C.byref(p)) == 0:
+            return p.value, size
+        with self.lock:
+            self.locked -= size
+        return None, 0
 
     def give(self, ptr: int, size: int):
-        with self.lock:
+        # (from a finaliser, which may run anywhere in this class's own code too: it must not wait for the lock)
+        self.returned.append((ptr, size))
+        if self.lock.acquire(blocking=False):
+            try:
+                self._sort_in()
+            finally:
+                self.lock.release()
+
+    def _sort_in(self):
+        while self.returned:
+            ptr, size = self.returned.popleft()
             if self.idle + size <= self.limit:
                 self.free.setdefault(size, []).append(ptr)
                 self.idle += size
-                return
+            else:
+                self._release(ptr, size)
+
+    def _release(self, ptr: int, size: int):
         _lib.lib().nrs_host_free(VP(ptr))
+        self.locked -= size
 
 
 _pinned = _PinnedPool()
