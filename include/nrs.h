@@ -104,6 +104,11 @@ int nrs_selftest_smem_attr_bookkeeping(void);
 /* Host-only self-test (no reference counterpart, needs no GPU): the queue of second-stage reductions of a backward
  * pass knows every tensor that a queued reduction writes.  Returns 0 when that bookkeeping behaves. */
 int nrs_selftest_fold_bookkeeping(void);
+/* Self-tests of device memory that runs out (no reference counterpart).  The first is host-only: which slabs of the pool
+ * may go back to the driver.  The second plays a driver that refuses: what the context keeps idle goes back before an
+ * allocation fails, and queued reductions run for the sake of their scratch.  Both return 0 when all is well. */
+int nrs_selftest_pool_bookkeeping(void);
+int nrs_selftest_memory_pressure(nrs_ctx* ctx);
 
 /* Measures the tensor pipe's dense-TF32 rate on this device (no reference counterpart): every SM
  * issues tcgen05.mma.kind::tf32 (128 x 256 x 8) back to back on operands resident in shared memory

@@ -20,6 +20,30 @@ int nrs_fail(nrs_ctx* ctx, int code, const char* fmt, ...) {
   return code;
 }
 
+static void give_back_idle(nrs_ctx* ctx) {   // (cudaFree waits for the kernels in flight)
+  NrsPool& pool = ctx->pool;
+  for (auto it = pool.free_blocks.upper_bound(NrsPool::kSmall); it != pool.free_blocks.end(); it = pool.free_blocks.erase(it)) {
+    cudaFree(it->second);
+    pool.bytes_reserved -= it->first;
+  }
+  for (void* s : pool.take_idle_slabs()) cudaFree(s);
+  if (!ctx->folds.active) nrs_folds_free(ctx);
+}
+
+int nrs_device_alloc(nrs_ctx* ctx, const char* what, size_t bytes, void** out) {
+  *out = nullptr;
+  cudaError_t e = ctx->device_malloc(out, bytes);
+  if (e != cudaSuccess) {
+    (void)cudaGetLastError();
+    give_back_idle(ctx);
+    e = ctx->device_malloc(out, bytes);
+  }
+  if (e == cudaSuccess) return NRS_OK;
+  (void)cudaGetLastError();
+  *out = nullptr;
+  return nrs_fail(ctx, NRS_ERR_ALLOC, "%s: cudaMalloc(%zu) failed: %s", what, bytes, cudaGetErrorString(e));
+}
+
 int nrs_workspace(nrs_ctx* ctx, size_t bytes, void** out) {
   if (bytes > ctx->workspace_bytes) {
     // The old block may still be read by kernels in flight on the stream.
@@ -30,13 +54,8 @@ int nrs_workspace(nrs_ctx* ctx, size_t bytes, void** out) {
       ctx->workspace_bytes = 0;
     }
     const size_t want = (bytes + ((size_t)1 << 20) - 1) >> 20 << 20;
-    cudaError_t e = cudaMalloc(&ctx->workspace, want);
-    if (e != cudaSuccess) {
-      ctx->workspace = nullptr;
-      (void)cudaGetLastError();
-      return nrs_fail(ctx, NRS_ERR_ALLOC, "workspace: cudaMalloc(%zu) failed: %s", want,
-                      cudaGetErrorString(e));
-    }
+    const int st = nrs_device_alloc(ctx, "workspace", want, &ctx->workspace);
+    if (st != NRS_OK) return st;
     ctx->workspace_bytes = want;
   }
   *out = ctx->workspace;
@@ -53,12 +72,8 @@ int nrs_ws_slot(nrs_ctx* ctx, int slot, size_t bytes, void** out) {
       ctx->ws_slot_bytes[slot] = 0;
     }
     const size_t want = (bytes + ((size_t)1 << 20) - 1) >> 20 << 20;
-    cudaError_t e = cudaMalloc(&ctx->ws_slot[slot], want);
-    if (e != cudaSuccess) {
-      ctx->ws_slot[slot] = nullptr;
-      (void)cudaGetLastError();
-      return nrs_fail(ctx, NRS_ERR_ALLOC, "workspace slot %d: cudaMalloc(%zu) failed: %s", slot, want, cudaGetErrorString(e));
-    }
+    const int st = nrs_device_alloc(ctx, "workspace slot", want, &ctx->ws_slot[slot]);
+    if (st != NRS_OK) return st;
     ctx->ws_slot_bytes[slot] = want;
   }
   *out = ctx->ws_slot[slot];
@@ -198,6 +213,65 @@ int nrs_selftest_smem_attr_bookkeeping(void) {
   return bad;
 }
 
+int nrs_selftest_pool_bookkeeping(void) {
+  int bad = 0;
+  NrsPool p;
+  const size_t kb = 1024;
+  uint8_t* base = (uint8_t*)(uintptr_t)((size_t)1 << 40);   // addresses only
+  auto at = [&](int slab, size_t off) { return (void*)(base + (size_t)slab * 2 * NrsPool::kSlab + off); };
+  for (int i = 0; i < 3; ++i) p.slabs.push_back(at(i, 0));
+  p.bytes_reserved = 3 * NrsPool::kSlab + 64 * kb * kb;
+  p.slab_used = 4 * kb;
+  p.free_blocks.emplace(kb, at(0, 0));
+  p.live[at(1, 0)] = kb;                                    // the middle slab is in use
+  p.live[at(1, NrsPool::kSlab - kb)] = kb;
+  p.free_blocks.emplace(kb, at(1, kb));
+  p.free_blocks.emplace(2 * kb, at(2, 0));
+  p.free_blocks.emplace(64 * kb * kb, at(7, 0));            // a block of its own
+  bad += p.take_idle_slabs() == std::vector<void*>{at(0, 0), at(2, 0)} ? 0 : 1;
+  bad += p.slabs == std::vector<void*>{at(1, 0)} && p.slab_used == NrsPool::kSlab ? 0 : 1;
+  bad += p.free_blocks.size() == 2 && p.free_blocks.begin()->second == at(1, kb) ? 0 : 1;
+  bad += p.bytes_reserved == NrsPool::kSlab + 64 * kb * kb ? 0 : 1;
+  bad += p.take_idle_slabs().empty() ? 0 : 1;
+  p.live.clear();
+  bad += p.take_idle_slabs().size() == 1 && p.slabs.empty() && p.free_blocks.size() == 1 ? 0 : 1;
+  return bad;
+}
+
+// A driver that is out of memory, played by an allocator that refuses until something has been given back.
+int nrs_selftest_memory_pressure(nrs_ctx* ctx) {
+  NRS_REQUIRE_CTX(ctx);
+  static thread_local int refuse;
+  static thread_local int calls;
+  const auto real = ctx->device_malloc;
+  ctx->device_malloc = [](void** p, size_t n) { ++calls; return refuse-- > 0 ? cudaErrorMemoryAllocation : cudaMalloc(p, n); };
+  int bad = 0;
+  void* p[40] = {};
+  for (int i = 0; i < 40; ++i) bad += nrs_alloc(ctx, (size_t)900 << 10, 0, &p[i]) == NRS_OK ? 0 : 1;   // three slabs
+  for (void* q : p) bad += nrs_free(ctx, q) == NRS_OK ? 0 : 1;
+  const size_t slabs = ctx->pool.slabs.size();
+  refuse = 1;
+  bad += nrs_alloc(ctx, (size_t)40 << 20, 0, &p[0]) == NRS_OK && ctx->pool.slabs.size() + 2 <= slabs ? 0 : 1;
+  bad += nrs_free(ctx, p[0]) == NRS_OK ? 0 : 1;
+  refuse = 1 << 20;                                          // nothing to be had: an error, and the context goes on
+  calls = 0;
+  bad += nrs_alloc(ctx, (size_t)50 << 20, 0, &p[0]) == NRS_ERR_ALLOC && p[0] == nullptr && calls == 2 ? 0 : 1;
+  // fold scratch: a full block while folds are queued means that they run and the block starts over
+  refuse = 0;
+  float *a = nullptr, *b = nullptr, *dst = nullptr;
+  bad += nrs_alloc(ctx, 4096, 1, (void**)&dst) == NRS_OK ? 0 : 1;
+  nrs_folds_begin(ctx);
+  bad += nrs_fold_partial(ctx, -1, (size_t)40 << 20, &a) == NRS_OK ? 0 : 1;
+  bad += nrs_memset_zero(ctx, a, 4096) == NRS_OK && nrs_fold_columns(ctx, a, dst, 4, 256, 256, 0) == NRS_OK ? 0 : 1;
+  refuse = 1 << 20;
+  bad += nrs_fold_partial(ctx, -1, (size_t)40 << 20, &b) == NRS_OK && b == a && ctx->folds.jobs.empty() ? 0 : 1;
+  refuse = 0;
+  nrs_folds_end(ctx);
+  ctx->device_malloc = real;
+  bad += nrs_free(ctx, dst) == NRS_OK && nrs_sync(ctx) == NRS_OK ? 0 : 1;
+  return bad;
+}
+
 int nrs_profile_enable(nrs_ctx* ctx, int on) {
   NRS_REQUIRE_CTX(ctx);
   ctx->profiling = on != 0;
@@ -334,20 +408,8 @@ int nrs_alloc(nrs_ctx* ctx, size_t bytes, int zero, void** dptr) {
       pool.slab_used += want;
     } else {
       const size_t ask = small ? NrsPool::kSlab : want;
-      cudaError_t e = cudaMalloc(&p, ask);
-      if (e != cudaSuccess) {
-        (void)cudaGetLastError();
-        // Give cached blocks back to the driver and retry once.
-        for (auto it = pool.free_blocks.upper_bound(NrsPool::kSmall); it != pool.free_blocks.end(); it = pool.free_blocks.erase(it)) {
-          cudaFree(it->second);
-          pool.bytes_reserved -= it->first;
-        }
-        e = cudaMalloc(&p, ask);
-        if (e != cudaSuccess) {
-          (void)cudaGetLastError();
-          return nrs_fail(ctx, NRS_ERR_ALLOC, "nrs_alloc: cudaMalloc(%zu) failed: %s", ask, cudaGetErrorString(e));
-        }
-      }
+      const int st = nrs_device_alloc(ctx, "nrs_alloc", ask, &p);
+      if (st != NRS_OK) return st;
       pool.bytes_reserved += ask;
       if (small) {
         pool.slabs.push_back(p);

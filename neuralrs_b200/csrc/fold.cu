@@ -262,6 +262,7 @@ void nrs_folds_end(nrs_ctx* ctx) {
 void nrs_folds_free(nrs_ctx* ctx) {
   for (auto& c : ctx->folds.chunks) cudaFree(c.first);
   ctx->folds.chunks.clear();
+  ctx->folds.chunk = ctx->folds.used = 0;
 }
 
 // Whether a job writes any of the `len` floats at `p`.  (One job may write several tensors: a column pair has two
@@ -301,10 +302,14 @@ int nrs_fold_partial(nrs_ctx* ctx, int ws_slot, size_t bytes, float** out) {
     if ((*out = place(f, bytes))) return NRS_OK;
   }
   const size_t want = std::max(kChunk, bytes);
-  if (cudaMalloc(&p, want) != cudaSuccess) {
-    (void)cudaGetLastError();
-    return nrs_fail(ctx, NRS_ERR_ALLOC, "fold scratch: cudaMalloc(%zu) failed", want);
+  int st = nrs_device_alloc(ctx, "fold scratch", want, &p);
+  if (st != NRS_OK && !f.open && !f.jobs.empty()) {   // what is queued runs, and its memory is to be had again
+    st = run_queue(ctx);
+    if (st != NRS_OK) return st;
+    if ((*out = place(f, bytes))) return NRS_OK;
+    st = nrs_device_alloc(ctx, "fold scratch", want, &p);
   }
+  if (st != NRS_OK) return st;
   f.chunks.push_back({p, want});
   *out = place(f, bytes);
   return NRS_OK;

@@ -6,6 +6,7 @@
 #include <cstdarg>
 #include <cstdint>
 #include <cstdio>
+#include <iterator>
 #include <map>
 #include <string>
 #include <utility>
@@ -29,6 +30,22 @@ struct NrsPool {
   static size_t round_up(size_t bytes) {
     const size_t g = bytes <= (1u << 20) ? 512 : (size_t)1 << 16;
     return (bytes + g - 1) / g * g;
+  }
+  // Takes the slabs none of whose blocks is in use out of the pool, for the caller to give back.
+  std::vector<void*> take_idle_slabs() {
+    std::vector<void*> out;
+    for (size_t i = 0; i < slabs.size();) {
+      uint8_t *lo = (uint8_t*)slabs[i], *hi = lo + kSlab;
+      const auto used = live.lower_bound(lo);
+      if (used != live.end() && (uint8_t*)used->first < hi) { ++i; continue; }
+      for (auto it = free_blocks.begin(); it != free_blocks.end() && it->first <= kSmall;)
+        it = (uint8_t*)it->second >= lo && (uint8_t*)it->second < hi ? free_blocks.erase(it) : std::next(it);
+      if (i + 1 == slabs.size()) slab_used = kSlab;   // the one that was being cut
+      slabs.erase(slabs.begin() + i);
+      bytes_reserved -= kSlab;
+      out.push_back(lo);
+    }
+    return out;
   }
 };
 
@@ -201,6 +218,8 @@ struct nrs_ctx {
   // (dropout masks, augmentation) then take the counters those samples have in the GLOBAL batch's stream
   // and the stream advances by the global batch's amount, so N processes draw what one process would.
   int shard_begin = 0, shard_local = 0, shard_global = 0;
+  // cudaMalloc, or what a self-test puts in its place.
+  cudaError_t (*device_malloc)(void** p, size_t bytes) = [](void** p, size_t bytes) { return cudaMalloc(p, bytes); };
   // Optional per-family device timing (nrs_profile_*).
   bool profiling = false;
   std::vector<NrsProfRecord> prof_records;
@@ -230,6 +249,9 @@ struct NrsProfScope {
 };
 
 int nrs_fail(nrs_ctx* ctx, int code, const char* fmt, ...);
+// Device memory from the driver.  Where there is none left, what the context keeps without using it (large blocks and
+// whole slabs of its pool, idle fold scratch) goes back first.  NRS_ERR_ALLOC names `what`.
+int nrs_device_alloc(nrs_ctx* ctx, const char* what, size_t bytes, void** out);
 int nrs_workspace(nrs_ctx* ctx, size_t bytes, void** out);
 // (the weight-gradient kernels keep their split partials in a slot of their own: they may run while the
 // data gradient's K-split is still being folded out of NRS_WS_PARTIAL)

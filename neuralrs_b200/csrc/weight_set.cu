@@ -154,12 +154,8 @@ int nrs_weight_set_build(nrs_ctx* ctx, const NrsWeightDesc* descs, int count) {
   const bool split = ctx->math_mode == NRS_MATH_3XTF32;
   size_t total = 0;
   for (int i = 0; i < count; ++i) total += (plane_floats(descs[i]) + 63) / 64 * 64 * (split ? 2 : 1);
-  cudaError_t e = cudaMalloc(&ws.storage, total * sizeof(float));
-  if (e != cudaSuccess) {
-    (void)cudaGetLastError();
-    ws.storage = nullptr;
-    return nrs_fail(ctx, NRS_ERR_ALLOC, "weight planes: cudaMalloc(%zu) failed: %s", total * sizeof(float), cudaGetErrorString(e));
-  }
+  const int got = nrs_device_alloc(ctx, "weight planes", total * sizeof(float), &ws.storage);
+  if (got != NRS_OK) return got;
   std::vector<WeightJob> jobs;
   float* cursor = (float*)ws.storage;
   for (int i = 0; i < count; ++i) {
@@ -195,7 +191,7 @@ int nrs_weight_set_build(nrs_ctx* ctx, const NrsWeightDesc* descs, int count) {
     ws.job_src.push_back(j.src);
     ws.job_first.push_back(j.first_block);
   }
-  e = cudaMalloc(&ws.jobs_dev, jobs.size() * sizeof(WeightJob));
+  cudaError_t e = cudaMalloc(&ws.jobs_dev, jobs.size() * sizeof(WeightJob));
   if (e == cudaSuccess) e = cudaMemcpyAsync(ws.jobs_dev, jobs.data(), jobs.size() * sizeof(WeightJob), cudaMemcpyHostToDevice, ctx->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);   // `jobs` is a local
   if (e != cudaSuccess) {

@@ -54,3 +54,7 @@ def test_fold_queue_knows_every_tensor_it_writes(nrs_lib):
     """A gradient that waits in the queue of second-stage reductions is found by any address inside it (host-only
     self-test): one job may write several parameters' gradients."""
     assert nrs_lib.nrs_selftest_fold_bookkeeping() == 0
+
+
+def test_pool_gives_back_slabs_that_are_not_in_use(nrs_lib):
+    assert nrs_lib.nrs_selftest_pool_bookkeeping() == 0

@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 
 from neuralrs_b200 import _lib
-from neuralrs_b200.cuda import Node, backward_graph, graph, nn
+from neuralrs_b200.cuda import Context, Node, backward_graph, graph, nn
 from neuralrs_b200.cuda import runtime as gpu
 from oracle import autograd as og
 from .conftest import rel_l2
@@ -67,3 +67,11 @@ def test_more_reductions_than_one_launch_takes(gpu_ctx, oracle64):
     assert gpu_ctx.launch_count() - before > 2 * layers
     for i, (gn, cn) in enumerate(zip([gx] + gp, [cx] + cp)):
         assert rel_l2(gpu.read_grad(gn), cn.grad) <= 2e-4, i   # twenty 3xTF32 products deep, some 1e-5 each
+
+
+def test_idle_memory_goes_back_before_an_allocation_fails():
+    ctx = Context(0)
+    try:
+        assert _lib.lib().nrs_selftest_memory_pressure(ctx.h) == 0
+    finally:
+        ctx.close()
