@@ -229,14 +229,15 @@ int run_queue(nrs_ctx* ctx) {
   ctx->independent_next = false;   // whoever writes into that memory next waits for this launch
   f.jobs.clear();
   f.tickets_used = 1;
+  f.holding = 0;
   return st;
 }
 
 // Memory for partial sums out of the blocks there are, or null.  The blocks start over only when nothing in them is
-// still to be read: no job is queued, and none is being made (its memory is handed out before the kernel that fills it
+// still to be read: no job with sums there is queued, and none is being made (its memory is handed out before the kernel that fills it
 // is launched and the job is submitted, and what comes in between may run the queue).
 float* place(NrsFolds& f, size_t bytes) {
-  if (f.jobs.empty() && !f.open) f.chunk = f.used = 0;
+  if (f.holding == 0 && !f.open) f.chunk = f.used = 0;
   for (; f.chunk < f.chunks.size(); ++f.chunk, f.used = 0)
     if (f.used + bytes <= f.chunks[f.chunk].second) {
       float* p = (float*)((uint8_t*)f.chunks[f.chunk].first + f.used);
@@ -257,6 +258,7 @@ void nrs_folds_end(nrs_ctx* ctx) {
   ctx->folds.active = ctx->folds.open = false;
   ctx->folds.jobs.clear();
   ctx->folds.tickets_used = 1;
+  ctx->folds.holding = 0;
 }
 
 void nrs_folds_free(nrs_ctx* ctx) {
@@ -335,6 +337,7 @@ int nrs_fold_submit(nrs_ctx* ctx, NrsFoldJob job) {
   if (st != NRS_OK) return st;
   f.tickets_used += need;
   f.jobs.push_back(job);
+  f.holding += f.open ? 1 : 0;
   f.open = false;
   return NRS_OK;
 }
@@ -409,11 +412,14 @@ extern "C" int nrs_selftest_fold_bookkeeping(void) {
   bad += nrs_fold_submit(&c, pair) == NRS_OK && f.jobs.size() == 1 ? 0 : 1;
   bad += nrs_fold_partial(&c, -1, 4096, &p[2]) == NRS_OK && p[2] == mem + 512 ? 0 : 1;
   f.jobs.clear();            // the queue is launched while the second job is being made
+  f.holding = 0;
   bad += nrs_fold_partial(&c, -1, 4096, &p[3]) == NRS_OK && p[3] == mem + 2048 ? 0 : 1;
   bad += nrs_fold_submit(&c, pair) == NRS_OK ? 0 : 1;
   bad += nrs_fold_partial(&c, -1, 4096, &p[4]) == NRS_OK && p[4] == mem + 3072 ? 0 : 1;
   bad += nrs_fold_submit(&c, qkv) == NRS_OK && f.jobs.size() == 2 ? 0 : 1;
   f.jobs.clear();
+  f.holding = 0;
+  bad += nrs_fold_submit(&c, pair) == NRS_OK && f.holding == 0 ? 0 : 1;   // sums in memory of its own: nobody's concern
   bad += nrs_fold_partial(&c, -1, 16, &p[5]) == NRS_OK && p[5] == mem ? 0 : 1;   // nothing waits: from the start again
 
   // a weight gradient never starts under a launch of folds

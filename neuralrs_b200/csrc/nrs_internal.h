@@ -172,6 +172,7 @@ struct NrsFolds {
   std::vector<std::pair<void*, size_t>> chunks;   // memory for partial sums that wait
   size_t chunk = 0, used = 0;
   bool open = false;       // some of it has been handed out for a job that is not submitted yet
+  int holding = 0;         // queued jobs with partial sums in it (others read memory of their own)
   uint64_t launched_at = ~0ull;   // nrs_ctx::launches right after the last launch of folds
 };
 
