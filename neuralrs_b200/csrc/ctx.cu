@@ -26,8 +26,8 @@ static void give_back_idle(nrs_ctx* ctx) {   // (cudaFree waits for the kernels 
     cudaFree(it->second);
     pool.bytes_reserved -= it->first;
   }
-  for (void* s : pool.take_idle_slabs()) cudaFree(s);
   if (!ctx->folds.active) nrs_folds_free(ctx);
+  for (void* s : pool.take_idle_slabs()) cudaFree(s);
 }
 
 int nrs_device_alloc(nrs_ctx* ctx, const char* what, size_t bytes, void** out) {
@@ -44,40 +44,41 @@ int nrs_device_alloc(nrs_ctx* ctx, const char* what, size_t bytes, void** out) {
   return nrs_fail(ctx, NRS_ERR_ALLOC, "%s: cudaMalloc(%zu) failed: %s", what, bytes, cudaGetErrorString(e));
 }
 
+// Grow-only blocks of the context's own: small ones out of the pool's slabs.
+static void drop_block(nrs_ctx* ctx, void** p, size_t* held) {   // the stream is idle
+  if (*p && *held <= NrsPool::kSmall) nrs_free(ctx, *p);
+  else if (*p) cudaFree(*p);
+  *p = nullptr;
+  *held = 0;
+}
+static int grow_block(nrs_ctx* ctx, const char* what, size_t bytes, void** p, size_t* held) {
+  if (bytes <= *held) return NRS_OK;
+  if (*p) NRS_CUDA(ctx, cudaStreamSynchronize(ctx->stream));   // kernels in flight may still read the old block
+  drop_block(ctx, p, held);
+  const size_t want = (bytes + ((size_t)1 << 20) - 1) >> 20 << 20;
+  const int st = want <= NrsPool::kSmall ? nrs_alloc(ctx, want, 0, p) : nrs_device_alloc(ctx, what, want, p);
+  if (st == NRS_OK) *held = want;
+  return st;
+}
+
 int nrs_workspace(nrs_ctx* ctx, size_t bytes, void** out) {
-  if (bytes > ctx->workspace_bytes) {
-    // The old block may still be read by kernels in flight on the stream.
-    if (ctx->workspace) {
-      NRS_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-      NRS_CUDA(ctx, cudaFree(ctx->workspace));
-      ctx->workspace = nullptr;
-      ctx->workspace_bytes = 0;
-    }
-    const size_t want = (bytes + ((size_t)1 << 20) - 1) >> 20 << 20;
-    const int st = nrs_device_alloc(ctx, "workspace", want, &ctx->workspace);
-    if (st != NRS_OK) return st;
-    ctx->workspace_bytes = want;
-  }
+  const int st = grow_block(ctx, "workspace", bytes, &ctx->workspace, &ctx->workspace_bytes);
   *out = ctx->workspace;
-  return NRS_OK;
+  return st;
 }
 
 int nrs_ws_slot(nrs_ctx* ctx, int slot, size_t bytes, void** out) {
   if (slot < 0 || slot >= NRS_WS_COUNT) return nrs_fail(ctx, NRS_ERR_ARG, "workspace: bad slot %d", slot);
-  if (bytes > ctx->ws_slot_bytes[slot]) {
-    if (ctx->ws_slot[slot]) {
-      NRS_CUDA(ctx, cudaStreamSynchronize(ctx->stream));  // kernels in flight may still read the old block
-      NRS_CUDA(ctx, cudaFree(ctx->ws_slot[slot]));
-      ctx->ws_slot[slot] = nullptr;
-      ctx->ws_slot_bytes[slot] = 0;
-    }
-    const size_t want = (bytes + ((size_t)1 << 20) - 1) >> 20 << 20;
-    const int st = nrs_device_alloc(ctx, "workspace slot", want, &ctx->ws_slot[slot]);
-    if (st != NRS_OK) return st;
-    ctx->ws_slot_bytes[slot] = want;
-  }
+  const int st = grow_block(ctx, "workspace slot", bytes, &ctx->ws_slot[slot], &ctx->ws_slot_bytes[slot]);
   *out = ctx->ws_slot[slot];
-  return NRS_OK;
+  return st;
+}
+
+int nrs_ws_planes(nrs_ctx* ctx, int slot, size_t bytes, bool split, void** hi, void** lo) {
+  const size_t each = (bytes + 255) / 256 * 256;
+  const int st = nrs_ws_slot(ctx, slot, split ? 2 * each : bytes, hi);
+  *lo = st == NRS_OK && split ? (uint8_t*)*hi + each : nullptr;
+  return st;
 }
 
 // One page-locked block per context: the device error word, and behind it the slot of small read-backs.  Pinning takes
@@ -133,8 +134,8 @@ int nrs_err_flag(nrs_ctx* ctx, int** out) {
 
 int nrs_fold_ticket(nrs_ctx* ctx, unsigned** out) {
   if (!ctx->fold_ticket) {
-    NRS_CUDA(ctx, cudaMalloc(&ctx->fold_ticket, kNrsFoldTickets * sizeof(unsigned)));
-    NRS_CUDA(ctx, cudaMemsetAsync(ctx->fold_ticket, 0, kNrsFoldTickets * sizeof(unsigned), ctx->stream));
+    const int st = nrs_alloc(ctx, kNrsFoldTickets * sizeof(unsigned), 1, (void**)&ctx->fold_ticket);
+    if (st != NRS_OK) return st;
   }
   *out = ctx->fold_ticket;
   return NRS_OK;
@@ -350,15 +351,14 @@ int nrs_destroy(nrs_ctx* ctx) {
   if (!ctx) return NRS_OK;
   cudaSetDevice(ctx->device);
   cudaStreamSynchronize(ctx->stream);
+  drop_block(ctx, &ctx->workspace, &ctx->workspace_bytes);
+  for (int i = 0; i < NRS_WS_COUNT; ++i) drop_block(ctx, &ctx->ws_slot[i], &ctx->ws_slot_bytes[i]);
+  nrs_folds_free(ctx);
+  nrs_weight_set_clear(ctx);
   for (auto& kv : ctx->pool.free_blocks) if (kv.first > NrsPool::kSmall) cudaFree(kv.second);
   for (auto& kv : ctx->pool.live) if (kv.second > NrsPool::kSmall) cudaFree(kv.first);
   for (void* s : ctx->pool.slabs) cudaFree(s);
-  nrs_weight_set_clear(ctx);
-  if (ctx->workspace) cudaFree(ctx->workspace);
-  for (int i = 0; i < NRS_WS_COUNT; ++i) if (ctx->ws_slot[i]) cudaFree(ctx->ws_slot[i]);
   nrs_pinned_release(ctx);
-  nrs_folds_free(ctx);
-  if (ctx->fold_ticket) cudaFree(ctx->fold_ticket);
   for (auto& r : ctx->prof_records) { cudaEventDestroy(r.start); cudaEventDestroy(r.stop); }
   for (auto& e : ctx->prof_free_events) cudaEventDestroy(e);
   if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);

@@ -262,7 +262,9 @@ void nrs_folds_end(nrs_ctx* ctx) {
 }
 
 void nrs_folds_free(nrs_ctx* ctx) {
-  for (auto& c : ctx->folds.chunks) cudaFree(c.first);
+  for (auto& c : ctx->folds.chunks)
+    if (c.second <= NrsPool::kSmall) nrs_free(ctx, c.first);
+    else cudaFree(c.first);
   ctx->folds.chunks.clear();
   ctx->folds.chunk = ctx->folds.used = 0;
 }
@@ -283,8 +285,9 @@ int nrs_folds_settle(nrs_ctx* ctx, const float* dst, size_t len) {
 }
 
 // Partial sums of a job that may wait live in blocks of their own (not pool blocks, which are handed out again as soon
-// as the host releases them, and not a shared slot, which the next layer overwrites).  64 MB at a time; at 512 MB what is
-// queued runs and the blocks start over, or, while a job is being made, there is one block more.
+// as the host releases them, and not a shared slot, which the next layer overwrites).  The first is small and comes out of
+// a slab (a small model needs no more); then 64 MB at a time; at 512 MB what is queued runs and the blocks start over, or,
+// while a job is being made, there is one block more.
 int nrs_fold_partial(nrs_ctx* ctx, int ws_slot, size_t bytes, float** out) {
   NrsFolds& f = ctx->folds;
   void* p = nullptr;
@@ -303,13 +306,14 @@ int nrs_fold_partial(nrs_ctx* ctx, int ws_slot, size_t bytes, float** out) {
     if (st != NRS_OK) return st;
     if ((*out = place(f, bytes))) return NRS_OK;
   }
-  const size_t want = std::max(kChunk, bytes);
-  int st = nrs_device_alloc(ctx, "fold scratch", want, &p);
+  const size_t want = f.chunks.empty() && bytes <= NrsPool::kSmall ? NrsPool::kSmall : std::max(kChunk, bytes);
+  auto more = [&] { return want <= NrsPool::kSmall ? nrs_alloc(ctx, want, 0, &p) : nrs_device_alloc(ctx, "fold scratch", want, &p); };
+  int st = more();
   if (st != NRS_OK && !f.open && !f.jobs.empty()) {   // what is queued runs, and its memory is to be had again
     st = run_queue(ctx);
     if (st != NRS_OK) return st;
     if ((*out = place(f, bytes))) return NRS_OK;
-    st = nrs_device_alloc(ctx, "fold scratch", want, &p);
+    st = more();
   }
   if (st != NRS_OK) return st;
   f.chunks.push_back({p, want});

@@ -22,9 +22,10 @@ struct NrsPool {
   std::multimap<size_t, void*> free_blocks;   // rounded size -> block
   std::map<void*, size_t> live;               // block -> rounded size
   size_t bytes_reserved = 0;
-  // Blocks up to kSmall bytes are cut from slabs: cudaMalloc takes 0.3 ms whatever the size, and a small model's first
-  // step asks for dozens of sizes.
-  static constexpr size_t kSmall = (size_t)1 << 20, kSlab = (size_t)16 << 20;
+  // Blocks up to kSmall bytes, the context's own workspaces of that size among them, are cut from slabs: cudaMalloc takes
+  // 0.3 ms for anything from 2 MB to 256 MB, and a small model's first step asks for dozens of sizes (the first step of
+  // the digit classifier in a new context: 14 calls of cudaMalloc without, 3 with).
+  static constexpr size_t kSmall = (size_t)2 << 20, kSlab = (size_t)32 << 20;
   std::vector<void*> slabs;
   size_t slab_used = kSlab;                   // of the last one
   static size_t round_up(size_t bytes) {
@@ -190,8 +191,8 @@ struct nrs_ctx {
   void* workspace = nullptr;
   size_t workspace_bytes = 0;
   // Named grow-only scratch blocks (operand staging for the tensor-core kernels).
-  void* ws_slot[8] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
-  size_t ws_slot_bytes[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  void* ws_slot[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
+  size_t ws_slot_bytes[5] = {0, 0, 0, 0, 0};
   // Device word the tensor-core kernels set when a bounded wait runs out; read at sync points.
   int* err_flag = nullptr;
   volatile int* err_host = nullptr;  // the same word as the host sees it (mapped memory)
@@ -256,8 +257,11 @@ int nrs_device_alloc(nrs_ctx* ctx, const char* what, size_t bytes, void** out);
 int nrs_workspace(nrs_ctx* ctx, size_t bytes, void** out);
 // (the weight-gradient kernels keep their split partials in a slot of their own: they may run while the
 // data gradient's K-split is still being folded out of NRS_WS_PARTIAL)
-enum { NRS_WS_A_HI = 0, NRS_WS_A_LO = 1, NRS_WS_B_HI = 2, NRS_WS_B_LO = 3, NRS_WS_PARTIAL = 4, NRS_WS_WGRAD_PARTIAL = 5, NRS_WS_FOLD = 6, NRS_WS_COUNT = 8 };
+enum { NRS_WS_A = 0, NRS_WS_B = 1, NRS_WS_PARTIAL = 2, NRS_WS_WGRAD_PARTIAL = 3, NRS_WS_FOLD = 4, NRS_WS_COUNT = 5 };
 int nrs_ws_slot(nrs_ctx* ctx, int slot, size_t bytes, void** out);
+// Room for operand planes of `bytes` each in one slot: the high plane, and with `split` the residual plane behind it (one
+// block to ask the driver for instead of two); *lo is null otherwise.
+int nrs_ws_planes(nrs_ctx* ctx, int slot, size_t bytes, bool split, void** hi, void** lo);
 int nrs_err_flag(nrs_ctx* ctx, int** out);
 void nrs_pinned_release(nrs_ctx* ctx);
 // Zero-initialised device counters (kNrsFoldTickets of them) for "the last block to arrive folds the partials"

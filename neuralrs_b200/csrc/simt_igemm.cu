@@ -717,8 +717,7 @@ int nrs_conv2d_bwd(nrs_ctx* ctx, const float* x, const float* w, const float* dy
     const int tiles = nrs_batchnorm_tiles(n, g.oh * g.ow);
     void *hi = nullptr, *lo = nullptr;
     float* partial = nullptr;
-    st = nrs_ws_slot(ctx, NRS_WS_A_HI, floats * sizeof(float), &hi);
-    if (st == NRS_OK && split3) st = nrs_ws_slot(ctx, NRS_WS_A_LO, floats * sizeof(float), &lo);
+    st = nrs_ws_planes(ctx, NRS_WS_A, floats * sizeof(float), split3, &hi, &lo);
     if (st == NRS_OK) st = nrs_fold_partial(ctx, -1, (size_t)tiles * co * sizeof(float), &partial);
     if (st == NRS_OK) st = nrs_tc_stage_image(ctx, dy, (float*)hi, (float*)lo, n, co, g.oh * g.ow, partial);
     if (st == NRS_OK) st = nrs_fold_columns(ctx, partial, db, tiles, co, co, accumulate);
@@ -733,8 +732,11 @@ int nrs_conv2d_bwd(nrs_ctx* ctx, const float* x, const float* w, const float* dy
              ? nrs_tc_conv_dgrad(ctx, w, dy, dx, n, ci, h, wd, co, kh, kw, stride, pad, accumulate)
              : NRS_ERR_UNSUPPORTED;
     if (st != NRS_OK && st != NRS_ERR_UNSUPPORTED) return st;
-    if (st == NRS_OK && dw && !dy_had_planes && !dy_planes_lent && ctx->ws_slot[NRS_WS_A_HI] && (!split3 || ctx->ws_slot[NRS_WS_A_LO])) {
-      ctx->plane_hints[dy] = NrsPlanes{(float*)ctx->ws_slot[NRS_WS_A_HI], split3 ? (float*)ctx->ws_slot[NRS_WS_A_LO] : nullptr, split3 ? 1 : 0};
+    if (st == NRS_OK && dw && !dy_had_planes && !dy_planes_lent && ctx->ws_slot[NRS_WS_A]) {   // (as large as dy's planes already)
+      void *hi = nullptr, *lo = nullptr;
+      const int got = nrs_ws_planes(ctx, NRS_WS_A, (size_t)n * g.oh * g.ow * nrs_plane_ld(co) * sizeof(float), split3, &hi, &lo);
+      if (got != NRS_OK) return got;
+      ctx->plane_hints[dy] = NrsPlanes{(float*)hi, (float*)lo, split3 ? 1 : 0};
       dy_planes_lent = true;
     }
     if (st == NRS_ERR_UNSUPPORTED) {
@@ -780,8 +782,7 @@ int nrs_planes_drop(nrs_ctx* ctx, const float* t) {
   if (it == ctx->owned_planes.end()) return NRS_OK;
   auto hint = ctx->plane_hints.find(t);
   if (hint != ctx->plane_hints.end() && hint->second.hi == it->second.hi) ctx->plane_hints.erase(hint);
-  nrs_free(ctx, it->second.hi);
-  if (it->second.lo) nrs_free(ctx, it->second.lo);
+  nrs_free(ctx, it->second.hi);   // (one block for both planes)
   ctx->owned_planes.erase(it);
   return NRS_OK;
 }
@@ -797,16 +798,16 @@ int nrs_planes_cache(nrs_ctx* ctx, const float* t, int n, int c, int h, int w) {
   if (ctx->plane_hints.count(t)) return NRS_OK;   // someone else (the node graph) already keeps planes of it
   const bool split = ctx->math_mode == NRS_MATH_3XTF32;
   const size_t hw = (size_t)h * w, floats = (size_t)n * nrs_plane_ld(c) * hw;
-  void *hi = nullptr, *lo = nullptr;
-  st = nrs_alloc(ctx, floats * sizeof(float), 0, &hi);
-  if (st == NRS_OK && split) st = nrs_alloc(ctx, floats * sizeof(float), 0, &lo);
-  if (st == NRS_OK) st = nrs_tc_stage_image(ctx, t, (float*)hi, (float*)lo, n, c, (int)hw);
+  const size_t each = (floats + 63) / 64 * 64;
+  void* block = nullptr;
+  st = nrs_alloc(ctx, (split ? 2 * each : floats) * sizeof(float), 0, &block);
+  float *hi = (float*)block, *lo = split ? hi + each : nullptr;
+  if (st == NRS_OK) st = nrs_tc_stage_image(ctx, t, hi, lo, n, c, (int)hw);
   if (st != NRS_OK) {
-    if (hi) nrs_free(ctx, hi);
-    if (lo) nrs_free(ctx, lo);
+    if (block) nrs_free(ctx, block);
     return st;
   }
-  const NrsPlanes pl{(float*)hi, (float*)lo, split ? 1 : 0};
+  const NrsPlanes pl{hi, lo, split ? 1 : 0};
   ctx->owned_planes[t] = pl;
   ctx->plane_hints[t] = pl;
   return NRS_OK;

@@ -350,8 +350,7 @@ int conv_common(nrs_ctx* ctx, ConvPlan& p) {
     a_lo = ready->lo;
   } else {
     const size_t a_plane = (size_t)p.n_img * p.a_h * p.a_w * nrs_plane_ld(p.a_ch);
-    st = nrs_ws_slot(ctx, NRS_WS_A_HI, a_plane * sizeof(float), &a_hi);
-    if (st == NRS_OK && split) st = nrs_ws_slot(ctx, NRS_WS_A_LO, a_plane * sizeof(float), &a_lo);
+    st = nrs_ws_planes(ctx, NRS_WS_A, a_plane * sizeof(float), split, &a_hi, &a_lo);
     if (st == NRS_OK) st = nrs_tc_stage_image(ctx, p.act_src, (float*)a_hi, (float*)a_lo, p.n_img, p.a_ch, p.a_h * p.a_w);
     if (st != NRS_OK) return st;
   }
@@ -363,8 +362,7 @@ int conv_common(nrs_ctx* ctx, ConvPlan& p) {
   } else {
     void *w_hi = nullptr, *w_lo = nullptr;
     const size_t w_plane = (size_t)p.n_ch_out * p.kh * p.kw * pol.cblocks * 32;
-    st = nrs_ws_slot(ctx, NRS_WS_B_HI, w_plane * sizeof(float), &w_hi);
-    if (st == NRS_OK && split) st = nrs_ws_slot(ctx, NRS_WS_B_LO, w_plane * sizeof(float), &w_lo);
+    st = nrs_ws_planes(ctx, NRS_WS_B, w_plane * sizeof(float), split, &w_hi, &w_lo);
     if (st != NRS_OK) return st;
     st = nrs_tc_stage_conv_weight(ctx, p.w, (float*)w_hi, (float*)w_lo, p.co, p.ci, p.kh, p.kw, p.for_dgrad);
     if (st != NRS_OK) return st;
@@ -434,8 +432,7 @@ int nrs_tc_conv_dgrad(nrs_ctx* ctx, const float* w, const float* dy, float* dx, 
   if (stride > 1 && !nrs_planes_find(ctx, dy, split)) {
     void *hi = nullptr, *lo = nullptr;
     const size_t plane = (size_t)n * p.a_h * p.a_w * nrs_plane_ld(co);
-    int st = nrs_ws_slot(ctx, NRS_WS_A_HI, plane * sizeof(float), &hi);
-    if (st == NRS_OK && split) st = nrs_ws_slot(ctx, NRS_WS_A_LO, plane * sizeof(float), &lo);
+    int st = nrs_ws_planes(ctx, NRS_WS_A, plane * sizeof(float), split, &hi, &lo);
     if (st == NRS_OK) st = nrs_tc_stage_image(ctx, dy, (float*)hi, (float*)lo, n, co, p.a_h * p.a_w);
     if (st != NRS_OK) return st;
     ctx->plane_hints[dy] = NrsPlanes{(float*)hi, (float*)lo, split ? 1 : 0};

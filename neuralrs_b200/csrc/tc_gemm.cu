@@ -152,7 +152,7 @@ struct Operand {
 // Brings one operand into K-major planes.  stored_kmajor: memory is [rows][K]; else [K][rows].  in_place: plain TF32
 // may read a suitable source as it is (the tensor core truncates it); otherwise it is rounded into a plane.
 int prepare_operand(nrs_ctx* ctx, const float* src, int rows, int K, int batch, bool stored_kmajor, bool split,
-                    int ws_hi, int ws_lo, Operand* out, bool is_weight, bool in_place = true) {
+                    int ws, Operand* out, bool is_weight, bool in_place = true) {
   const int ldk = nrs_plane_ld(K);   // TMA zero-fills what a K-block reads beyond K
   if (batch == 1) {
     // a weight staged ahead with the rest of the model's (weight_set.cu) ...
@@ -180,12 +180,8 @@ int prepare_operand(nrs_ctx* ctx, const float* src, int rows, int K, int batch, 
   }
   const size_t plane = (size_t)rows * ldk;
   void *phi = nullptr, *plo = nullptr;
-  int st = nrs_ws_slot(ctx, ws_hi, plane * batch * sizeof(float), &phi);
+  int st = nrs_ws_planes(ctx, ws, plane * batch * sizeof(float), split, &phi, &plo);
   if (st != NRS_OK) return st;
-  if (split) {
-    st = nrs_ws_slot(ctx, ws_lo, plane * batch * sizeof(float), &plo);
-    if (st != NRS_OK) return st;
-  }
   st = nrs_tc_stage(ctx, src, (float*)phi, (float*)plo, rows, K, ldk, batch, (size_t)rows * K, plane, !stored_kmajor);
   if (st != NRS_OK) return st;
   *out = Operand{(const float*)phi, (const float*)plo, ldk, K, plane};
@@ -355,15 +351,15 @@ int nrs_tc_gemm(nrs_ctx* ctx, int trans_a, int trans_b, int batch, int m, int n,
   Operand A, B;
   int st;
   if (trans_a && !trans_b && batch == 1 && m % 32 == 0 && n % 32 == 0) {   // A^T B on the operands' own rows
-    st = prepare_operand(ctx, a, k, m, 1, true, split, NRS_WS_A_HI, NRS_WS_A_LO, &A, false, false);
-    if (st == NRS_OK) st = prepare_operand(ctx, b, k, n, 1, true, split, NRS_WS_B_HI, NRS_WS_B_LO, &B, false, false);
+    st = prepare_operand(ctx, a, k, m, 1, true, split, NRS_WS_A, &A, false, false);
+    if (st == NRS_OK) st = prepare_operand(ctx, b, k, n, 1, true, split, NRS_WS_B, &B, false, false);
     if (st != NRS_OK) return st;
     GemmPolicy<true> pol{c, bias, act, beta, m, n, (size_t)m * n, false, {}, 0, 0};
     return dispatch<true>(ctx, tile_of(ctx, m, n, 1, k, split), split, A, B, 1, n, 1, m, n, k, pol, extras);
   }
-  st = prepare_operand(ctx, a, m, k, batch, /*stored_kmajor=*/!trans_a, split, NRS_WS_A_HI, NRS_WS_A_LO, &A, false);
+  st = prepare_operand(ctx, a, m, k, batch, /*stored_kmajor=*/!trans_a, split, NRS_WS_A, &A, false);
   if (st != NRS_OK) return st;
-  st = prepare_operand(ctx, b, n, k, batch, /*stored_kmajor=*/trans_b != 0, split, NRS_WS_B_HI, NRS_WS_B_LO, &B, true);
+  st = prepare_operand(ctx, b, n, k, batch, /*stored_kmajor=*/trans_b != 0, split, NRS_WS_B, &B, true);
   if (st != NRS_OK) return st;
   // Batched operands read in place need 16-byte aligned batch strides.
   if (batch > 1 && ((A.bstride % 4) || (B.bstride % 4))) return NRS_ERR_UNSUPPORTED;
@@ -383,7 +379,7 @@ int nrs_tc_gemm_weights(nrs_ctx* ctx, int reduce, int count, int m, int n, int k
   if (!reduce && n % 32 != 0) return NRS_ERR_UNSUPPORTED;   // a column tile belongs to one matrix
   if (reduce && k % 32 != 0) return NRS_ERR_UNSUPPORTED;    // and so does a K-slice
   Operand A, B{};
-  int st = prepare_operand(ctx, x, m, reduce ? count * k : k, 1, true, split, NRS_WS_A_HI, NRS_WS_A_LO, &A, false);
+  int st = prepare_operand(ctx, x, m, reduce ? count * k : k, 1, true, split, NRS_WS_A, &A, false);
   if (st != NRS_OK) return st;
   bool found = true;
   for (int i = 0; i < count && found; ++i) {
@@ -398,8 +394,7 @@ int nrs_tc_gemm_weights(nrs_ctx* ctx, int reduce, int count, int m, int n, int k
     const int ld = nrs_plane_ld(k);
     const size_t plane = (size_t)n * ld;
     void *hi = nullptr, *lo = nullptr;
-    st = nrs_ws_slot(ctx, NRS_WS_B_HI, plane * count * sizeof(float), &hi);
-    if (st == NRS_OK && split) st = nrs_ws_slot(ctx, NRS_WS_B_LO, plane * count * sizeof(float), &lo);
+    st = nrs_ws_planes(ctx, NRS_WS_B, plane * count * sizeof(float), split, &hi, &lo);
     for (int i = 0; i < count && st == NRS_OK; ++i)
       st = nrs_tc_stage(ctx, w[i], (float*)hi + i * plane, split ? (float*)lo + i * plane : nullptr, n, k, ld, 1, 0, 0, !reduce);
     if (st != NRS_OK) return st;

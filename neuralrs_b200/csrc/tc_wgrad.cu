@@ -374,8 +374,7 @@ int nrs_tc_conv_wgrad(nrs_ctx* ctx, const float* x, const float* dy, float* dw, 
     dy_lo = ready->lo;
   } else {
     may_overlap = false;
-    st = nrs_ws_slot(ctx, NRS_WS_A_HI, dy_plane * sizeof(float), &dy_hi);
-    if (st == NRS_OK && split3) st = nrs_ws_slot(ctx, NRS_WS_A_LO, dy_plane * sizeof(float), &dy_lo);
+    st = nrs_ws_planes(ctx, NRS_WS_A, dy_plane * sizeof(float), split3, &dy_hi, &dy_lo);
     if (st == NRS_OK) st = nrs_tc_stage_image(ctx, dy, (float*)dy_hi, (float*)dy_lo, n, co, oh * ow);
     if (st != NRS_OK) return st;
   }
@@ -384,8 +383,7 @@ int nrs_tc_conv_wgrad(nrs_ctx* ctx, const float* x, const float* dy, float* dw, 
     x_lo = ready->lo;
   } else {
     may_overlap = false;
-    st = nrs_ws_slot(ctx, NRS_WS_B_HI, x_plane * sizeof(float), &x_hi);
-    if (st == NRS_OK && split3) st = nrs_ws_slot(ctx, NRS_WS_B_LO, x_plane * sizeof(float), &x_lo);
+    st = nrs_ws_planes(ctx, NRS_WS_B, x_plane * sizeof(float), split3, &x_hi, &x_lo);
     if (st == NRS_OK) st = nrs_tc_stage_image(ctx, x, (float*)x_hi, (float*)x_lo, n, ci, h * wd);
     if (st != NRS_OK) return st;
   }
