@@ -262,17 +262,19 @@ static NodeP planes_attention(const MultiHeadAttention& m, const NodeP& x, size_
       ~Mode() { c->math_mode = was; }
     } mode{ctx, split ? NRS_MATH_3XTF32 : NRS_MATH_TF32};
     const float* g = grad_view(self);
-    // the gradient's row planes: left by the output projection's input-gradient kernel, else staged here
+    // the gradient's row planes: left by the output projection's input-gradient kernel, else staged here (also where that
+    // kernel ran in TF32 and left no residual plane, the math mode having been changed since the forward pass)
     float *ghi = self->gplanes_hi, *glo = self->gplanes_lo;
-    if (!ghi) {
-      ghi = block(tokens * d);
-      glo = split ? block(tokens * d) : nullptr;
-      check(ctx, nrs_tc_stage(ctx, g, ghi, glo, (int)tokens, (int)d, (int)d, 1, 0, 0, false));
-    } else {
+    if (ghi) {
       ctx->plane_hints.erase(g);
       self->gplanes_hi = self->gplanes_lo = nullptr;
     }
-    a.dout_hi = ghi; a.dout_lo = glo;
+    if (!ghi || (split && !glo)) {
+      if (!ghi) ghi = block(tokens * d);
+      if (split) glo = block(tokens * d);
+      check(ctx, nrs_tc_stage(ctx, g, ghi, glo, (int)tokens, (int)d, (int)d, 1, 0, 0, false));
+    }
+    a.dout_hi = ghi; a.dout_lo = split ? glo : nullptr;
     a.scores = block(square);
     a.ds_hi = block(square);
     a.ds_lo = split ? block(square) : nullptr;
