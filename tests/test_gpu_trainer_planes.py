@@ -1,11 +1,11 @@
 """A trainer's operand planes at ragged sizes: weights of both forms (taps beyond one tile, channels that are no multiple
 of a tile, linear layers with odd rows), batch-normalised tensors whose planes come out of the normalise and dx kernels,
-images smaller than a tile; gradients against the same trainer in FP32 mode, which reads no
-planes."""
+images smaller than a tile; gradients in every math mode against the f64 oracle."""
 import numpy as np
 import pytest
 
-from neuralrs_b200 import _lib, cuda
+from neuralrs_b200 import _lib, cuda, workloads
+from oracle import models
 from .conftest import rel_l2
 
 pytestmark = pytest.mark.gpu
@@ -35,20 +35,31 @@ def gradients(ctx, mode, shape, layers, x, t, params):
         ctx.set_math_mode(_lib.MATH_3XTF32)
 
 
+# Relative error (2-norm) of a tensor's gradient.  FP32 and 3xTF32: a chain of K elements errs by some 7e-9 K in 3xTF32, K
+# up to 1800 here, and the layers' errors add (4.7e-6 is the most seen).  TF32 operands carry 11 bits, 1.4e-4 rms each, so a
+# product errs by 2e-4 and a network of smooth layers by a few times that.  A ReLU turns a pre-activation that such an error d
+# moves across zero into a whole unit of gradient: with unit variance a share of 0.8 d of them, which is an error of
+# sqrt(0.8 d) = 2e-2 for d = 5e-4 (3.4e-2 is the most seen, under batch normalisation).
+TOL = {_lib.MATH_FP32: 3e-6, _lib.MATH_3XTF32: 2e-5, _lib.MATH_TF32: 6e-2}
+TOL_SMOOTH_TF32 = 1.5e-3
+
+
 @pytest.mark.parametrize("net", list(NETS))
-@pytest.mark.parametrize("mode,tol", [(_lib.MATH_3XTF32, 2e-4), (_lib.MATH_TF32, 2e-2)], ids=["3xtf32", "tf32"])
-def test_trainer_planes_ragged(gpu_ctx, net, mode, tol):
+@pytest.mark.parametrize("mode", list(TOL), ids=["fp32", "3xtf32", "tf32"])
+def test_trainer_planes_ragged(gpu_ctx, oracle64, net, mode):
     shape, layers = NETS[net]
     rng = np.random.default_rng(5)
     batch = 150 if net.startswith("head") else 24
     x = rng.standard_normal((batch, *shape)).astype(np.float32)
     t = np.eye(10, dtype=np.float32)[rng.integers(0, 10, batch)]
-    ref_loss, params, ref = gradients(gpu_ctx, _lib.MATH_FP32, shape, layers, x, t, None)
-    loss, _, got = gradients(gpu_ctx, mode, shape, layers, x, t, params)
-    assert np.isclose(loss, ref_loss, rtol=tol)
+    loss, params, got = gradients(gpu_ctx, mode, shape, layers, x, t, None)
+    shaped = [p.reshape(like.shape) for p, like in zip(params, workloads.he_init(layers, 1))]
+    ref_loss, ref, _ = models.forward_backward(oracle64, layers, shaped, x, t, buffers=workloads.bn_buffers(layers))
+    tol = TOL_SMOOTH_TF32 if mode == _lib.MATH_TF32 and net == "head_gelu" else TOL[mode]
+    assert np.isclose(loss, ref_loss, rtol=min(tol, 5e-4))
     scale = max(np.abs(b).max() for b in ref)
     for i, (a, b) in enumerate(zip(got, ref)):
         if np.abs(b).max() < 1e-5 * scale:   # a bias under a batch normalisation: rounding noise
-            assert np.abs(a).max() < tol * scale, i
+            assert np.abs(a).max() < 1e-6 * scale, i
         else:
-            assert rel_l2(a, b) <= 10 * tol, i
+            assert rel_l2(a, b) <= tol, i
