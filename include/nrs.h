@@ -52,8 +52,16 @@ enum nrs_status {
 
 /* Contraction precision.  3xTF32 (default): each f32 operand is split into a
  * TF32 high part and a TF32 residual and three tensor-core products are summed
- * in f32 (error ~1e-6 relative).  TF32: one product (error ~1e-3).  FP32: the
- * CUDA-core FFMA kernels only. */
+ * in f32.  The tensor core's sums are not rounded to nearest: the relative error
+ * is some 7e-9 per term of a reduction, 1e-6 for a hundred terms, 2e-5 for
+ * thousands.  TF32: one product of operands rounded to 11 bits (error ~1e-3).
+ * FP32: the CUDA-core FFMA kernels only.
+ * The two TF32 modes hold for every convolution of stride 8 and less, strided and
+ * ragged ones included, for products (nrs_gemm, nrs_bmm) of m >= 16, n >= 32 and
+ * k >= 32 (A^T B: m, n >= 32 and k >= 8), and for attention.  What is smaller
+ * runs in f32 in every mode: fewer than 16 rows, n or k up to 16 (up to 64 M
+ * multiplications), a layer of fewer than 8 channels on fewer than 1024 output
+ * pixels.  A caller who needs f32 arithmetic beyond that asks for FP32. */
 enum nrs_math_mode { NRS_MATH_3XTF32 = 0, NRS_MATH_TF32 = 1, NRS_MATH_FP32 = 2 };
 
 /* Activation fused into a contraction's epilogue. */

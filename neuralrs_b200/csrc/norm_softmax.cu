@@ -7,7 +7,8 @@
 // input gradient (optionally into two destinations: the fused residual add) and the parameter
 // gradients from one read of g and xhat: every warp keeps column partials of dgamma / dbeta in
 // registers over the rows it visits, the block folds its warps in warp order through shared memory,
-// and a second small kernel folds the blocks in block order — fixed order, no atomics, bit-reproducible.
+// and the blocks are folded in block order (fold.cu) — fixed order, no atomics, bit-reproducible.
+// Large tensors and odd widths run on the row pipeline where that is the better one (row_pipe.cuh).
 // (The reference runs one thread per row and three kernels.)
 // Reference: ln_forward / ln_reduce / ln_dx (src/cuda/nn/normalization.rs:14-78),
 // softmax_forward / softmax_backward (src/cuda/graph/softmax.rs:12-35); CPU

@@ -441,8 +441,8 @@ int nrs_tc_conv_wgrad(nrs_ctx* ctx, const float* x, const float* dy, float* dw, 
 int nrs_tc_gemm_tn(nrs_ctx* ctx, int m, int n, int k, const float* a, const float* b, float* c, int accumulate) {
   if (m < 32 || n < 32 || k < 8) return NRS_ERR_UNSUPPORTED;
   // Outputs of up to 4 M elements (the Linear layers of the CNN and transformer configurations).  Larger ones
-  // (4096 x 4096 hidden layers) stay on the persistent GEMM kernel: its rastered tiles reuse operands through L2,
-  // and the transposes it needs are small beside such a product.
+  // (4096 x 4096 hidden layers) stay on the persistent GEMM kernel, which reads both operands as stored too
+  // (transposed while they are staged where m or n is no multiple of 32) and whose rastered tiles reuse them through L2.
   if ((long)m * n > (4L << 20)) return NRS_ERR_UNSUPPORTED;
   return nrs_tc_conv_wgrad(ctx, /*x=*/b, /*dy=*/a, /*dw=*/c, /*n=*/k, /*ci=*/n, 1, 1, /*co=*/m, 1, 1, 1, 0, accumulate);
 }
