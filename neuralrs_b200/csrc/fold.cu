@@ -176,8 +176,11 @@ template <int CAP>
 __global__ void __launch_bounds__(256) fold_kernel(const __grid_constant__ FoldBatch<CAP> b) {
   NRS_PDL_PROLOGUE();
   __shared__ float4 sm[256];
-  int i = b.n - 1;
-  while (i > 0 && b.job[i].first_block > blockIdx.x) --i;
+  int i = CAP - 1;
+  if (CAP > 1) {
+    i = b.n - 1;
+    while (i > 0 && b.job[i].first_block > blockIdx.x) --i;
+  }
   const NrsFoldJob& j = b.job[i];
   const unsigned blk = blockIdx.x - j.first_block;
   if (j.kind == NRS_FOLD_COLUMNS) fold_columns(j, blk, reinterpret_cast<float*>(sm));
