@@ -219,8 +219,10 @@ struct Plan {
   size_t slot;
 };
 constexpr size_t kHead = 2048, kBudget = 220 * 1024 - kHead;
+constexpr int kMaxColumns = 8192;   // one slot of two buffers is then 64 KB
 inline Plan plan(int f, int n_buf) {
   Plan q{};
+  if (f > kMaxColumns) return q;
   q.npl = f <= 256 ? 8 : 16;
   q.team_warps = (f + q.npl * 32 - 1) / (q.npl * 32);
   // rows per slot: whole 16-byte groups, and at least 1 KB per copy
@@ -236,20 +238,21 @@ inline Plan plan(int f, int n_buf) {
 }
 // Share of a row's lanes x elements that hold columns.
 inline double fill(int f) {
+  if (f > kMaxColumns) return 0.0;
   const int unit = 32 * (f <= 256 ? 8 : 16);
   return (double)f / ((f + unit - 1) / unit * unit);
 }
 // Warps' worth of columns an SM works on: the warps whose slots fit into shared memory (16 at most; groups of four rows
 // of an odd width leave 3 of 1401 columns) times their fill.  With few of them the work inside a row is not hidden.
 inline double live_warps(int f, int n_buf) {
-  const Plan q = plan(f, n_buf);
+  const Plan q = plan(f, n_buf);   // (no teams beyond kMaxColumns)
   return q.teams * q.team_warps * fill(f);
 }
-// Whether a tensor set can take this path: 16-byte aligned bases, rows of at most 8192 columns (one slot of two
-// buffers is then 64 KB), 128 K elements (below, a shorter prologue wins: [64][10] 4 us against 20).  The operators add
-// their own crossovers against the register kernels (widths of whole float4s) and the scalar loops (other widths).
+// Whether a tensor set can take this path: 16-byte aligned bases, rows of at most kMaxColumns, 128 K elements (below, a
+// shorter prologue wins: [64][10] 4 us against 20).  The operators add their own lines against the register kernels
+// (widths of whole float4s) and the scalar loops (other widths).
 inline bool applies(int rows, int f, std::initializer_list<const void*> ptrs) {
-  if (f > 8192 || rows < 1) return false;
+  if (f > kMaxColumns || rows < 1) return false;
   for (const void* q : ptrs)
     if (reinterpret_cast<uintptr_t>(q) & 15) return false;
   return (size_t)rows * f >= (size_t)1 << 17;
