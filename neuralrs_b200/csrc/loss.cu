@@ -268,11 +268,11 @@ int run_ce(nrs_ctx* ctx, const char* who, const float* logits, const float* targ
   NRS_REQUIRE(ctx, logits && (target || labels), NRS_ERR_ARG, "%s: null tensor", who);
   const float inv_div = 1.0f / (float)divisor;
   // Where the row pipeline is the better kernel: from 8 M elements up (us here -> there, tensors that are not in L2).
-  // Float4 rows: with a one-hot target [16384][1000] 52 -> 48, 1024 columns 52 -> 45, 512 46 -> 43 (but 64 M elements 146, 155); not 256 (50, 61) or 384 (46, 52); with
-  // labels nowhere (1000: 40, 50; 256: 46, 71).  Scalar loops, with a one-hot target: 16 M elements of 250 columns 107 -> 53,
-  // 385 95 -> 85, 1001 129 -> 107, 3000 136 -> 61, not 1281 (120, 162; 2.5 live warps) or 700 (44, 52 in [20000][700]); with
-  // labels, one tensor less to bring in, only with more columns at work: 250 73 -> 61, 1002 64 -> 50, 4096 97 -> 51, not
-  // 385 (54, 60), 1001 (64, 70), 1281 (59, 73) or 2999 (75, 90).
+  // Float4 rows: with a one-hot target [16384][1000] 52 -> 48, 1024 columns 52 -> 45, 512 46 -> 43 (but 64 M elements 146,
+  // 155); not 256 (50, 61) or 384 (46, 52); with labels nowhere (1000: 40, 50; 256: 46, 71).  Scalar loops, with a one-hot
+  // target: 16 M elements of 250 columns 107 -> 53, 385 95 -> 85, 1001 129 -> 107, 3000 136 -> 61, not 1281 (120, 162; 2.5
+  // live warps) or 700 (44, 52 in [20000][700]); with labels, one tensor less to bring in, only with more columns at work:
+  // 250 73 -> 61, 1002 64 -> 50, 4096 97 -> 51, not 385 (54, 60), 1001 (64, 70), 1281 (59, 73) or 2999 (75, 90).
   const bool vec = classes % 4 == 0 && classes <= 1024 &&
                    ((reinterpret_cast<uintptr_t>(logits) | reinterpret_cast<uintptr_t>(target) | reinterpret_cast<uintptr_t>(grad)) & 15) == 0;
   const double fill = rowpipe::fill(classes), live = rowpipe::live_warps(classes, target ? 2 : 1);

@@ -553,9 +553,10 @@ int layernorm_fwd(nrs_ctx* ctx, const char* who, const float* a, const float* b,
   // Where the row pipeline is the better kernel (us here -> there, tensors that are not in L2).  Float4 rows without a
   // residual: 16 M elements of 384 columns 40 -> 39, 448 41 -> 36, 512 39 -> 38, 1000 42 -> 36; not 256 (39, 51) or 768
   // (40, 45; a quarter of the lanes idle).  With a residual (two inputs, two outputs) the register kernel is as good by
-  // itself at every width (256 47, 54; 512 47, 49; 1000 50, 50, and 114, 124 for 40 M elements), but its stores pass the L2
-  // cache by: where that can hold a good part of the result, the operator that reads y next gains 4 us of 16 M elements.  Scalar loops: 1502 columns 62 -> 51,
-  // 3000 76 -> 43, not 1401 (83, 112; 2.7 live warps); with a residual 1001 100 -> 82, 3000 128 -> 49, not 1281 (98, 130).
+  // itself at every width (256 47, 54; 512 47, 49; 1000 50, 50, and 114, 124 for 40 M elements), but its stores pass the
+  // L2 cache by: where that can hold a good part of the result, the operator that reads y next gains 4 us of 16 M
+  // elements.  Scalar loops: 1502 columns 62 -> 51, 3000 76 -> 43, not 1401 (83, 112; 2.7 live warps); with a residual
+  // 1001 100 -> 82, 3000 128 -> 49, not 1281 (98, 130).
   const size_t elems = (size_t)rows * f;
   const double fill = rowpipe::fill(f), live = rowpipe::live_warps(f, 2);
   const bool pipe = elems >= 6000000 && (vpl ? (b ? f >= 960 && elems < (size_t)24 << 20 : f >= 384 && (f <= 512 || fill >= 0.8))
