@@ -101,8 +101,8 @@ struct CeOp {
 // One warp per row.  row_loss (optional) gets -sum_c t*(x - lse); grad (optional)
 // gets (softmax - t) * inv_div.  Scalar path (any width / alignment).
 // FOLD: the kernel also folds the batch mean, which saves a launch; without, row_loss is left to ce_mean_kernel.  The
-// fold costs the loops 8 of their 40 registers' worth of scheduling and every block a fence and an atomic, so it is for
-// small calls (see run_ce): [64][10] 6.0 us with two launches, 4.0 with one; [16760][1001] with labels 64 and 85.
+// fold costs the loops registers (48 against 40) and every block a fence and an atomic, so it is for small calls and a few
+// others (see run_ce): [64][10] 6.0 us with two launches, 4.0 with one; [16760][1001] with labels 64 and 85.
 template <bool FOLD>
 __global__ void __launch_bounds__(256)
 ce_rows_kernel(const float* __restrict__ logits, const float* __restrict__ target, const int32_t* __restrict__ labels,
@@ -272,7 +272,8 @@ int run_ce(nrs_ctx* ctx, const char* who, const float* logits, const float* targ
   // 155); not 256 (50, 61) or 384 (46, 52); with labels nowhere (1000: 40, 50; 256: 46, 71).  Scalar loops, with a one-hot
   // target: 16 M elements of 250 columns 107 -> 53, 385 95 -> 85, 1001 129 -> 107, 3000 136 -> 61, not 1281 (120, 162; 2.5
   // live warps) or 700 (44, 52 in [20000][700]); with labels, one tensor less to bring in, only with more columns at work:
-  // 250 73 -> 61, 1002 64 -> 50, 4096 97 -> 51, not 385 (54, 60), 1001 (64, 70), 1281 (59, 73) or 2999 (75, 90).
+  // 250 73 -> 61, 1002 64 -> 50, 4096 97 -> 51, not 385 (54, 60), 1001 (64, 70), 1281 (59, 73) or 2999 (75, 90).  Rows of 257
+  // to 512 columns with a one-hot target wait for 12 M elements: 8 M of 385 that lie in L2 take 39 and 48.
   const bool vec = classes % 4 == 0 && classes <= 1024 &&
                    ((reinterpret_cast<uintptr_t>(logits) | reinterpret_cast<uintptr_t>(target) | reinterpret_cast<uintptr_t>(grad)) & 15) == 0;
   const double fill = rowpipe::fill(classes), live = rowpipe::live_warps(classes, target ? 2 : 1);
@@ -280,7 +281,7 @@ int run_ce(nrs_ctx* ctx, const char* who, const float* logits, const float* targ
   const size_t elems = (size_t)batch * classes;
   const bool pipe = elems >= (size_t)1 << 23 && fill >= 0.75 &&
                     (vec      ? target && (classes >= 960 || (classes >= 448 && classes <= 512 && elems < (size_t)1 << 25))
-                     : target ? wide && live >= 3.5
+                     : target ? wide && live >= (classes > 512 || elems >= (size_t)12 << 20 ? 3.5 : 4.5)
                               : wide && live >= 9.5 && (fill >= 0.85 || classes > 1500));
   if (pipe && rowpipe::applies(batch, classes, {logits, target, grad})) {
     rowpipe::Params p{};
@@ -308,9 +309,10 @@ int run_ce(nrs_ctx* ctx, const char* who, const float* logits, const float* targ
   // a launch weighs more, or where the mean's own launch has very many rows to add.  us with two launches and with one:
   // 64 x 10 6.0, 4.0; 2048 x 33 6.0, 4.6; 8192 x 33 6.4, 8.5; 512 x 127 5.9, 6.3, with labels (a tensor less to read) 5.9,
   // 5.0; 512 x 255 7.0, 7.5; with labels 133455 x 33 63, 58 and 9532 x 33 8.6, 9.0; with a one-hot target 508400 x 33 241,
-  // 232 and 133455 x 33 67, 67.
+  // 232 and 133455 x 33 67, 67; beyond 1800 columns always (1024 x 4096 86, 82, with labels 33, 30; 2990 x 1401 39, 41).
   const bool small = batch <= 4096 && classes <= (target ? 64 : 128) && (size_t)batch * classes <= (size_t)1 << (target ? 17 : 18);
-  const bool fold = vec || small || batch >= 1 << (target ? 18 : 16);
+  const bool many = batch >= 1 << (target ? 18 : 16) && classes <= 256;
+  const bool fold = vec || small || many || classes >= 1800;
   float* rl = row_loss;
   float* partial = nullptr;
   unsigned* ticket = nullptr;

@@ -551,16 +551,21 @@ int layernorm_fwd(nrs_ctx* ctx, const char* who, const float* a, const float* b,
   NRS_REQUIRE(ctx, a && gamma && beta && y, NRS_ERR_ARG, "%s: null tensor", who);
   const int vpl = vec_vpl(f, {a, b, gamma, beta, y, xhat, y_hi, y_lo});
   // Where the row pipeline is the better kernel (us here -> there, tensors that are not in L2).  Float4 rows without a
-  // residual: 16 M elements of 384 columns 40 -> 39, 448 41 -> 36, 512 39 -> 38, 1000 42 -> 36; not 256 (39, 51) or 768
-  // (40, 45; a quarter of the lanes idle).  With a residual (two inputs, two outputs) the register kernel is as good by
-  // itself at every width (256 47, 54; 512 47, 49; 1000 50, 50, and 114, 124 for 40 M elements), but its stores pass the
-  // L2 cache by: where that can hold a good part of the result, the operator that reads y next gains 4 us of 16 M
-  // elements.  Scalar loops: 1502 columns 62 -> 51, 3000 76 -> 43, not 1401 (83, 112; 2.7 live warps); with a residual
-  // 1001 100 -> 82, 3000 128 -> 49, not 1281 (98, 130).
+  // residual: 16 M elements of 384 columns 40 -> 39, 448 43 -> 36, 512 40 -> 38, 896 42 -> 39, 1000 42 -> 36; not 256 (39,
+  // 51) or 768 (40, 45; a quarter of the lanes idle).  With a residual (two inputs, two outputs) 8 M of 448 28 -> 26, 896 29
+  // -> 26; not 256 (25, 30), and not far beyond L2 (40 M of 1000 114, 124), although up to there the register kernel's
+  // stores, which pass the cache by, cost the operator that reads y next 4 us of 16 M elements.  Scalar loops: 1502 columns
+  // 62 -> 51, 3000 76 -> 43, not 1401 (83, 112; 2.7 live warps); with a residual 1001 100 -> 82, 3000 128 -> 49, not 1281
+  // (98, 130).  Tensors that still lie in L2 suit the other kernels (8 M elements: 384 columns 19, 22; 2050 27, 33): lines
+  // that are close wait for 12 M.
   const size_t elems = (size_t)rows * f;
   const double fill = rowpipe::fill(f), live = rowpipe::live_warps(f, 2);
-  const bool pipe = elems >= 6000000 && (vpl ? (b ? f >= 960 && elems < (size_t)24 << 20 : f >= 384 && (f <= 512 || fill >= 0.8))
-                                             : fill >= 0.75 && (b ? f >= 960 && live >= 3.8 : f >= 1400 && live >= 5.0));
+  const bool beyond_l2 = elems >= (size_t)12 << 20, full_warp = f >= 448 && f <= 512;
+  bool pipe;
+  if (vpl && b) pipe = f >= 832 ? elems < (size_t)24 << 20 : full_warp && !beyond_l2;
+  else if (vpl) pipe = full_warp || f >= 928 || (beyond_l2 && (f >= 832 || (f >= 384 && f <= 512)));
+  else pipe = fill >= 0.75 && (b ? f >= 960 && live >= 3.8 : f >= 1400 && live >= 5.0 && (beyond_l2 || fill >= 0.85));
+  pipe = pipe && elems >= 6000000;
   if (!(y_hi && vpl) && pipe && rowpipe::applies(rows, f, {a, b, gamma, beta, y, xhat})) {
     rowpipe::Params p{};
     p.in[0] = a; p.in[1] = b; p.n_in = b ? 2 : 1; p.n_buf = 2;
@@ -608,20 +613,29 @@ int layernorm_bwd(nrs_ctx* ctx, const char* who, const float* g, const float* xh
   if (!dx && !dgamma) return NRS_OK;
   const int vpl = vec_vpl(f, {g, xhat, gamma, dx, dx2, d_hi, d_lo});
   // Where the row pipeline is the better kernel (us here -> there, tensors that are not in L2).  Float4 rows: beyond 256
-  // columns, from 4 M elements up.  dx and parameters of 16 M elements: 260 columns 71 -> 68, 320 69 -> 58, 512 59 -> 42,
-  // 768 98 -> 46, 1000 104 -> 41; but 64 columns 76, 87, 128 48, 67, 256 44, 56 (dx alone 38, 52; parameters alone 30, 36).
-  // Scalar loops, which read g and xhat twice: for dx and parameters from 256 K elements (17 columns 9.8 -> 9.2, 1001
-  // 14 -> 12; 128 K of 385: 8.8, 11.0) or 1024 columns; for parameters alone from 4 M (1001 columns 19 -> 16, 1 M 8.5,
-  // 10.9), 8 M beyond 4000 columns (4 M of 8192: 15, 20); for dx alone with enough columns at work: 16 M elements of 250
-  // columns 63 -> 41, 1002 72 -> 42, 1001 72 -> 56, not 777 (58, 70; 3.1 live warps) or 1281 (64, 83; 2.5), which are taken
-  // only while the rows are few (up to 1.5 M elements; 200 K of 1401 columns: 10.8 -> 5.2).
-  const size_t elems = (size_t)rows * f;
+  // columns, from 4 M elements up (8 M below 280 columns).  dx and parameters of 16 M elements: 260 columns 71 -> 68, 320
+  // 69 -> 58, 512 59 -> 42, 768 98 -> 46, 1000 104 -> 41; but 64 columns 76, 87, 128 48, 67, 256 44, 56 (dx alone 38, 52;
+  // parameters alone 30, 36).
+  // Scalar loops, which read g and xhat twice.  dx and parameters: from 256 K elements (17 columns 9.8 -> 9.2, 1001 14 ->
+  // 12; 128 K of 385: 8.8, 11.0), with 60 to 256 columns (128 K of 127 9.5 -> 8.1) or 1024 and more (128 K of 1401 15.5 ->
+  // 11.6) always.  Parameters alone, one read of each: from 12 M (16 M of 1001 columns 64 -> 32), where rows are neither
+  // very short nor very long from 8 M (1001: 34 -> 20; 17 62 -> 57, 6000 29 -> 24), up to 256 columns from 4 M (250: 21 ->
+  // 14); 1 M of 1001 8.5, 10.9.  dx alone: any width of 961 columns and more (4 M of 1028 20 -> 15), narrower ones with
+  // few lanes idle (4 M of 450 16 -> 15) or beyond L2 (16 M of 33 164 -> 134, 301 61 -> 51) or for few rows (512 K of 705
+  // 7.2 -> 5.2); not 16 M of 777 (58, 70; 3.1 live warps) or 1281 (64, 83; 2.5).  Tensors that still lie in L2 suit the
+  // loops, which is why lines that are close wait for more elements: dx and parameters of 4 M of 1281 22, 31, parameters of
+  // 8 M of 17 27, 56, dx of 4 M of 385 14, 18.
+  const size_t elems = (size_t)rows * f, m = (size_t)1 << 20;
   const double fill = rowpipe::fill(f), live = rowpipe::live_warps(f, 2);
-  const bool pipe = vpl            ? f > 256 && elems >= (size_t)1 << 22
-                    : dx && dgamma ? f >= 1024 || elems >= (size_t)1 << 18
-                    : dgamma       ? elems >= (size_t)1 << (f <= 4000 ? 22 : 23)
-                                   : (fill >= 0.75 && live >= 5.0) || (fill >= 0.85 && live >= 3.8) || (elems >= (size_t)1 << 23 && live >= 4.5) ||
-                                         (f > 640 && elems < (size_t)3 << 19);
+  const bool beyond_l2 = elems >= 12 * m, large = elems >= 8 * m, small = elems < 3 * m, few = elems < 3 * m / 2;
+  bool pipe;
+  if (vpl) pipe = f > 256 && elems >= (f < 280 ? 8 : 4) * m;
+  else if (dx && dgamma) pipe = (f >= 1024 || elems >= m / 4 || (f >= 60 && f <= 256)) && (live >= 3.0 || f <= 256 || large || small);
+  else if (dgamma) pipe = beyond_l2 || (large && f >= 24 && f <= 3000 && (live >= 3.0 || f <= 256)) ||
+                          (elems >= 4 * m && f >= 100 && f <= 256);
+  else if (f > 960) pipe = live >= 3.0 || small;
+  else pipe = (fill >= 0.85 && (live >= 3.9 || small || beyond_l2)) || (live >= 7.0 && f > 512 && (fill >= 0.75 || small)) ||
+              (beyond_l2 && (f <= 512 || live >= 4.3)) || (large && f <= 40) || (few && f > 256 && fill >= 0.55 && elems >= m / 4);
   if (!(d_hi && vpl) && pipe && rowpipe::applies(rows, f, {g, xhat, gamma, dx, dx2})) {
     rowpipe::Params p{};
     p.in[0] = g; p.in[1] = xhat; p.n_in = p.n_buf = 2;

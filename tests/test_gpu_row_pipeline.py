@@ -51,8 +51,9 @@ def test_row_pipeline(gpu_ctx, oracle64, rows, f):
 
 
 # Both sides of the lines between the pipeline and the kernels it stands beside (rows, columns).
-LINES = [(16500, 256), (16140, 260), (15700, 384), (6100, 1000), (1024, 255), (1029, 255), (200, 1025), (127, 1028), (8400, 501), (1050, 4004),
-         (2100, 4004), (5400, 777), (4300, 1402), (4300, 1403), (149, 1401), (1125, 1401)]
+LINES = [(16500, 256), (33000, 260), (32900, 384), (11000, 400), (6100, 1000), (1024, 255), (1029, 255), (200, 1025), (127, 1028),
+         (16800, 501), (1050, 4004), (2100, 4004), (95000, 90), (140000, 90), (1600, 90), (17000, 250), (210000, 40),
+         (5400, 777), (10900, 777), (17000, 511), (4300, 1402), (4300, 1403), (149, 1401), (1125, 1401)]
 
 
 @pytest.mark.parametrize("rows,f", LINES)
@@ -76,7 +77,7 @@ def test_layernorm_beside_its_lines(gpu_ctx, oracle64, rows, f):
     assert rel_l2(dx.get(), 2.0 * dxr) <= 2e-5 and rel_l2(dg.get(), dgr) <= 1e-5 and rel_l2(db.get(), dbr) <= 1e-5
 
 
-SOFTMAX_LINES = [(4300, 1401), (4000, 1502), (2950, 2050), (2050, 3000), (17000, 1502), (1500, 4096)]
+SOFTMAX_LINES = [(150, 1281), (3300, 1281), (9900, 1281), (4300, 1401), (4000, 1502), (2950, 2050), (2050, 3000), (17000, 1502), (1500, 4096)]
 
 
 @pytest.mark.parametrize("rows,f", SOFTMAX_LINES)
@@ -85,16 +86,22 @@ def test_softmax_beside_its_lines(gpu_ctx, oracle64, rows, f):
     x = (4.0 * rng.normal(size=(rows, f))).astype(np.float32)
     x[1, ::2] = np.finfo(np.float32).min   # a masked row, and one with a single live column
     x[2, 1:] = -np.inf
-    xd, y = Dev(gpu_ctx, x), Dev(gpu_ctx, shape=(rows, f))
+    g = rng.normal(size=(rows, f)).astype(np.float32)
+    xd, gd, y, dx = Dev(gpu_ctx, x), Dev(gpu_ctx, g), Dev(gpu_ctx, shape=(rows, f)), Dev(gpu_ctx, shape=(rows, f))
     call(gpu_ctx, "nrs_softmax_fwd", xd, y, rows, f)
     got = y.get()
     assert rel_l2(got, oracle64.softmax_fwd(x)) <= 1e-6
     assert (got[1, ::2] == 0).all() and got[2, 0] == 1.0 and (got[2, 1:] == 0).all()
+    yg = got.astype(np.float64) * g
+    want = yg - got * yg.sum(1, keepdims=True)
+    for k in (1, 2):
+        call(gpu_ctx, "nrs_softmax_bwd", y, gd, dx, rows, f, k - 1)
+        assert np.linalg.norm(dx.get() - k * want) <= 1e-5 * np.linalg.norm(yg)
 
 
 # Both sides of the lines against the pipeline; the scalar kernel with its own mean and with a second launch for it.
-CE_LINES = [(8400, 1000), (16400, 512), (33000, 256), (33000, 255), (21900, 385), (6600, 1281), (5600, 1502), (5600, 1501),
-            (1, 7), (2048, 63), (2100, 63), (4096, 31), (4097, 31), (2048, 127), (300, 1001), (65535, 7), (65536, 7), (262144, 3)]
+CE_LINES = [(8400, 1000), (16400, 512), (33000, 256), (33000, 255), (21900, 385), (32800, 385), (6600, 1281), (5600, 1502), (5600, 1501),
+            (1, 7), (2048, 63), (2100, 63), (4096, 31), (4097, 31), (2048, 127), (300, 1001), (70, 1801), (65535, 7), (65536, 7), (262144, 3)]
 
 
 @pytest.mark.parametrize("rows,f", CE_LINES)
