@@ -329,14 +329,47 @@ bn_dx_kernel(const float* __restrict__ g, const float* __restrict__ xhat, const 
   }
 }
 
+// Bounds of what the two kernels below write, for the exponent of f16 pairs: one block.
+// Forward: |xhat| <= sqrt(count) under the batch's own statistics, else istd * (|x| + |mean|).
+__global__ void __launch_bounds__(256)
+bn_bound_kernel(const float* __restrict__ gamma, const float* __restrict__ beta, const float* __restrict__ mean, const float* __restrict__ istd,
+                const NrsRange* __restrict__ x, float count, int training, NrsRange* __restrict__ out, int c) {
+  NRS_PDL_PROLOGUE();
+  uint32_t top = 0;
+  for (int i = threadIdx.x; i < c; i += 256) {
+    const float xhat = training ? sqrtf(count) : istd[i] * (x->top + fabsf(mean[i]));
+    top = pr::seen(top, fminf((fabsf(gamma[i]) * xhat + fabsf(beta[i])) * 1.001f, 3.0e38f));
+  }
+  top = __reduce_max_sync(0xffffffffu, top);
+  if ((threadIdx.x & 31) == 0) atomicMax(reinterpret_cast<unsigned*>(&out->bound), top);
+}
+// Backward: istd * (|g gamma| + |m1| + |xhat| |m2|), the means as bn_dx_planes_kernel takes them.
+__global__ void __launch_bounds__(256)
+bn_dx_bound_kernel(const float* __restrict__ gamma, const float* __restrict__ istd, const float2* __restrict__ sums, const NrsRange* __restrict__ g,
+                   float count, int training, const float* __restrict__ count_dev, NrsRange* __restrict__ out, int c) {
+  NRS_PDL_PROLOGUE();
+  if (count_dev) count = *count_dev;
+  uint32_t top = 0;
+  for (int i = threadIdx.x; i < c; i += 256) {
+    const float ga = fabsf(gamma[i]);
+    float b = ga * g->top;
+    if (training) b += ga * fabsf(sums[i].x) / count + sqrtf(count) * ga * fabsf(sums[i].y) / count;
+    top = pr::seen(top, fminf(istd[i] * b * 1.001f, 3.0e38f));
+  }
+  top = __reduce_max_sync(0xffffffffu, top);
+  if ((threadIdx.x & 31) == 0) atomicMax(reinterpret_cast<unsigned*>(&out->bound), top);
+}
+
 // The normalise pass with the NHWC planes of y (no xhat).
 template <bool SPLIT, bool RELU>
 __global__ void __launch_bounds__(kThreads)
 bn_normalize_planes_kernel(const float* __restrict__ x, const float* __restrict__ mean, const float* __restrict__ istd,
                            const float* __restrict__ gamma, const float* __restrict__ beta, float* __restrict__ y,
-                           float* __restrict__ hi, float* __restrict__ lo, const img::Grid g) {
+                           float* __restrict__ hi, float* __restrict__ lo, const img::Grid g, NrsRange* __restrict__ range) {
   NRS_PDL_PROLOGUE();
   __shared__ img::Tile tile;
+  const float scale = SPLIT ? pr::scale_of(range->bound) : 1.0f;
+  uint32_t top = 0;
   const uint32_t p0 = blockIdx.x * img::kTilePx;
   const int c0 = blockIdx.y * img::kTileCh, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const img::Pixels px(g, p0);
@@ -356,12 +389,16 @@ bn_normalize_planes_kernel(const float* __restrict__ x, const float* __restrict_
       const float h = (v[4 * k + s] - m) * is;
       float o = fmaf(ga, h, be);
       if (RELU) o = fmaxf(o, 0.0f);
-      if (ok && px.live[s]) y[px.base + (px.at[s] + (uint32_t)c * g.hw)] = o;
+      if (ok && px.live[s]) {
+        y[px.base + (px.at[s] + (uint32_t)c * g.hw)] = o;
+        if (SPLIT) top = pr::seen(top, o);
+      }
       tile[cl][s * 32 + lane] = o;
     }
   }
   __syncthreads();
-  img::tile_to_planes<SPLIT>(tile, g, p0, c0, hi, lo);
+  img::tile_to_planes<SPLIT>(tile, g, p0, c0, hi, lo, scale);
+  if (SPLIT) pr::report(range, top);
 }
 
 // dx (overwritten; null: planes only) with its NHWC planes, and chan_partial[tile of 128 pixels][c], its sums over the tile.
@@ -370,9 +407,12 @@ __global__ void __launch_bounds__(kThreads, 3)
 bn_dx_planes_kernel(const float* __restrict__ gr, const float* __restrict__ x, const float* __restrict__ mean,
                     const float* __restrict__ istd, const float* __restrict__ gamma, const float* __restrict__ beta,
                     const float2* __restrict__ sums, float* __restrict__ dx, float* __restrict__ hi, float* __restrict__ lo,
-                    float* __restrict__ chan_partial, const img::Grid g, float count, int training, const float* __restrict__ count_dev) {
+                    float* __restrict__ chan_partial, const img::Grid g, float count, int training, const float* __restrict__ count_dev,
+                    NrsRange* __restrict__ range) {
   NRS_PDL_PROLOGUE();
   __shared__ img::Tile tile;
+  const float scale = SPLIT ? pr::scale_of(range->bound) : 1.0f;
+  uint32_t top = 0;
   if (count_dev) count = *count_dev;
   const uint32_t p0 = blockIdx.x * img::kTilePx;
   const int c0 = blockIdx.y * img::kTileCh, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -403,13 +443,15 @@ bn_dx_planes_kernel(const float* __restrict__ gr, const float* __restrict__ x, c
       const float r = !live ? 0.0f : training ? is * (gi * ga - m1 - h * m2) : gi * ga * is;
       if (live && dx) dx[px.base + (px.at[s] + (uint32_t)c * g.hw)] = r;
       tile[cl][s * 32 + lane] = r;
+      if (SPLIT) top = pr::seen(top, r);
       total += r;
     }
     total = wsum(total);
     if (lane == 0 && ok) chan_partial[(size_t)blockIdx.x * g.c + c] = total;
   }
   __syncthreads();
-  img::tile_to_planes<SPLIT>(tile, g, p0, c0, hi, lo);
+  img::tile_to_planes<SPLIT>(tile, g, p0, c0, hi, lo, scale);
+  if (SPLIT) pr::report(range, top);
 }
 
 // Statistics shared by several processes: the splits of this process folded in order into out[ch], the
@@ -533,9 +575,20 @@ int bn_forward(nrs_ctx* ctx, const char* who, const float* x, const float* gamma
   }
   if (hi) {
     const img::Grid grid(n, c, hw);
+    NrsRange *range = nullptr, *range_x = nullptr;
+    if (lo) {
+      int rs = nrs_range_renew(ctx, hi, &range);
+      if (rs == NRS_OK && !training) rs = nrs_range_renew(ctx, &ctx->scratch_range[0], &range_x);
+      if (rs == NRS_OK && !training) rs = nrs_absmax(ctx, x, (size_t)n * c * hw, range_x);
+      if (rs != NRS_OK) return rs;
+      // (shared statistics: the count of all processes is not known here; each holds at most 2^31 values a channel)
+      NRS_PDL_LAUNCH(bn_bound_kernel, 1, 256, 0, ctx->stream, gamma, beta, (const float*)mean, (const float*)istd, (const NrsRange*)range_x,
+                     shared ? 2147483648.0f * 8.0f : (float)((double)n * hw), training, range, c);
+      NRS_LAUNCHED(ctx);
+    }
 #define NRS_BN_NORM(S, R)                                                                                               \
   NRS_PDL_LAUNCH((bn_normalize_planes_kernel<S, R>), grid.blocks(), kThreads, 0, ctx->stream, x, (const float*)mean, (const float*)istd, \
-                 gamma, beta, y, hi, lo, grid)
+                 gamma, beta, y, hi, lo, grid, range)
     if (lo) { if (relu) NRS_BN_NORM(true, true); else NRS_BN_NORM(true, false); }
     else { if (relu) NRS_BN_NORM(false, true); else NRS_BN_NORM(false, false); }
 #undef NRS_BN_NORM
@@ -600,9 +653,19 @@ int bn_backward(nrs_ctx* ctx, const char* who, const float* g, const float* xhat
   const float count = (float)((double)n * hw);
   if (hi) {
     const img::Grid grid(n, c, hw);
+    NrsRange *range = nullptr, *range_g = nullptr;
+    if (lo) {
+      int rs = nrs_range_renew(ctx, hi, &range);
+      if (rs == NRS_OK) rs = nrs_range_renew(ctx, &ctx->scratch_range[0], &range_g);
+      if (rs == NRS_OK) rs = nrs_absmax(ctx, g, (size_t)n * c * hw, range_g);
+      if (rs != NRS_OK) return rs;
+      NRS_PDL_LAUNCH(bn_dx_bound_kernel, 1, 256, 0, ctx->stream, gamma, istd, (const float2*)sums, (const NrsRange*)range_g, count, training,
+                     shared ? (const float*)count_slot : (const float*)nullptr, range, c);
+      NRS_LAUNCHED(ctx);
+    }
 #define NRS_BN_DX(S, R)                                                                                                  \
   NRS_PDL_LAUNCH((bn_dx_planes_kernel<S, R>), grid.blocks(), kThreads, 0, ctx->stream, g, xhat, mean, istd, gamma, beta,  \
-                 (const float2*)sums, dx, hi, lo, chan_partial, grid, count, training, shared ? (const float*)count_slot : (const float*)nullptr)
+                 (const float2*)sums, dx, hi, lo, chan_partial, grid, count, training, shared ? (const float*)count_slot : (const float*)nullptr, range)
     if (lo) { if (relu) NRS_BN_DX(true, true); else NRS_BN_DX(true, false); }
     else { if (relu) NRS_BN_DX(false, true); else NRS_BN_DX(false, false); }
 #undef NRS_BN_DX

@@ -12,6 +12,7 @@
 // (src/cuda/nn/conv.rs:244-320).
 #include "igemm_problems.cuh"
 #include "nrs_internal.h"
+#include "pair.cuh"
 #include "tc_common.cuh"
 
 namespace {
@@ -23,8 +24,10 @@ constexpr int kMaxPatch = 128;
 template <bool SPLIT>
 __global__ void __launch_bounds__(256)
 patch_planes_kernel(const float* __restrict__ x, float* __restrict__ hi, float* __restrict__ lo, const NrsConvGeom g, int kh,
-                    int kw, const NrsFastDiv div_quads, uint32_t total /*pixels * (row length / 4)*/) {
+                    int kw, const NrsFastDiv div_quads, uint32_t total /*pixels * (row length / 4)*/, NrsRange* range) {
   NRS_PDL_PROLOGUE();
+  const float bound = SPLIT ? *(volatile float*)&range->top : 0.0f, scale = SPLIT ? pr::scale_of(bound) : 1.0f;
+  if (SPLIT && blockIdx.x == 0 && threadIdx.x == 0) range->bound = bound;
   __shared__ int off[kMaxPatch];        // offset of patch value k from the patch's origin
   __shared__ short2 tap[kMaxPatch];     // its (row, column) inside the window
   const int K = g.ci * kh * kw;
@@ -54,9 +57,8 @@ patch_planes_kernel(const float* __restrict__ x, float* __restrict__ hi, float* 
         if ((unsigned)(iy0 + t.x) < (unsigned)g.h && (unsigned)(ix0 + t.y) < (unsigned)g.w) v[e] = src[off[k0 + e]];
       }
     }
-    const float4 h = make_float4(tc::tf32_rn(v[0]), tc::tf32_rn(v[1]), tc::tf32_rn(v[2]), tc::tf32_rn(v[3]));
-    *reinterpret_cast<float4*>(hi + p * ld + k0) = h;
-    if (SPLIT) *reinterpret_cast<float4*>(lo + p * ld + k0) = make_float4(v[0] - h.x, v[1] - h.y, v[2] - h.z, v[3] - h.w);
+    if (SPLIT) pr::put4(hi, lo, p * ld + k0, make_float4(v[0], v[1], v[2], v[3]), scale);
+    else *reinterpret_cast<float4*>(hi + p * ld + k0) = make_float4(tc::tf32_rn(v[0]), tc::tf32_rn(v[1]), tc::tf32_rn(v[2]), tc::tf32_rn(v[3]));
   }
 }
 
@@ -79,14 +81,14 @@ struct Patches {
       }
     }
     const NrsConvGeom g(n, ci, h, wd, 1, kh, kw, stride, pad);
-    const size_t floats = (size_t)n * g.oh * g.ow * nrs_plane_ld(ci * kh * kw);
+    const size_t bytes = (size_t)n * g.oh * g.ow * nrs_plane_ld(ci * kh * kw) * (split ? 2 : 4);
     void *phi = nullptr, *plo = nullptr;
-    int st = nrs_alloc(ctx, floats * sizeof(float), 0, &phi);
+    int st = nrs_alloc(ctx, bytes, 0, &phi);
     if (st != NRS_OK) return st;
     owned = true;
     hi = (float*)phi;
     if (split) {
-      st = nrs_alloc(ctx, floats * sizeof(float), 0, &plo);
+      st = nrs_alloc(ctx, bytes, 0, &plo);
       if (st != NRS_OK) return st;
       lo = (float*)plo;
     }
@@ -111,8 +113,14 @@ int nrs_patch_planes(nrs_ctx* ctx, const float* x, float* hi, float* lo, int n, 
   size_t blocks = (total + 255) / 256;
   const size_t cap = (size_t)ctx->sm_count * 16;
   if (blocks > cap) blocks = cap;
-  if (lo) NRS_PDL_LAUNCH((patch_planes_kernel<true>), (unsigned)blocks, 256, 0, ctx->stream, x, hi, lo, g, kh, kw, NrsFastDiv(quads), (uint32_t)total);
-  else NRS_PDL_LAUNCH((patch_planes_kernel<false>), (unsigned)blocks, 256, 0, ctx->stream, x, hi, nullptr, g, kh, kw, NrsFastDiv(quads), (uint32_t)total);
+  NrsRange* range = nullptr;
+  if (lo) {
+    int st = nrs_range_renew(ctx, hi, &range);
+    if (st == NRS_OK) st = nrs_absmax(ctx, x, (size_t)n * ci * h * wd, range);
+    if (st != NRS_OK) return st;
+  }
+  if (lo) NRS_PDL_LAUNCH((patch_planes_kernel<true>), (unsigned)blocks, 256, 0, ctx->stream, x, hi, lo, g, kh, kw, NrsFastDiv(quads), (uint32_t)total, range);
+  else NRS_PDL_LAUNCH((patch_planes_kernel<false>), (unsigned)blocks, 256, 0, ctx->stream, x, hi, nullptr, g, kh, kw, NrsFastDiv(quads), (uint32_t)total, range);
   NRS_LAUNCHED(ctx);
   return NRS_OK;
 }

@@ -74,11 +74,51 @@ int nrs_ws_slot(nrs_ctx* ctx, int slot, size_t bytes, void** out) {
   return st;
 }
 
-int nrs_ws_planes(nrs_ctx* ctx, int slot, size_t bytes, bool split, void** hi, void** lo) {
-  const size_t each = (bytes + 255) / 256 * 256;
-  const int st = nrs_ws_slot(ctx, slot, split ? 2 * each : bytes, hi);
+int nrs_ws_planes(nrs_ctx* ctx, int slot, size_t values, bool split, void** hi, void** lo) {
+  const size_t each = (values * (split ? 2 : 4) + 255) / 256 * 256;
+  const int st = nrs_ws_slot(ctx, slot, split ? 2 * each : each, hi);
   *lo = st == NRS_OK && split ? (uint8_t*)*hi + each : nullptr;
   return st;
+}
+
+static void give_back_range(nrs_ctx* ctx, NrsRange* r) {
+  for (auto& pg : ctx->range_pool.pages)
+    if (r >= pg.mem && r < pg.mem + NrsRangePool::kPerPage) { --pg.live; return; }
+}
+void nrs_range_drop(nrs_ctx* ctx, const void* p) {
+  auto it = ctx->ranges.find(p);
+  if (it == ctx->ranges.end()) return;
+  give_back_range(ctx, it->second);
+  ctx->ranges.erase(it);
+}
+int nrs_range_renew(nrs_ctx* ctx, const void* p, NrsRange** out) {
+  NrsRangePool& pool = ctx->range_pool;
+  *out = nullptr;
+  nrs_range_drop(ctx, p);
+  constexpr size_t kBytes = NrsRangePool::kPerPage * sizeof(NrsRange);
+  if (pool.pages.empty() || pool.pages[pool.current].used == NrsRangePool::kPerPage) {
+    size_t next = 0;
+    while (next < pool.pages.size() && pool.pages[next].live > 0) ++next;
+    if (next == pool.pages.size()) {
+      void* mem = nullptr;
+      const int st = nrs_alloc(ctx, kBytes, 1, &mem);
+      if (st != NRS_OK) return st;
+      pool.pages.push_back(NrsRangePool::Page{(NrsRange*)mem, 0, 0});
+    } else {
+      NRS_CUDA(ctx, cudaMemsetAsync(pool.pages[next].mem, 0, kBytes, ctx->stream));
+      pool.pages[next].used = 0;
+    }
+    pool.current = next;
+  }
+  NrsRangePool::Page& pg = pool.pages[pool.current];
+  *out = pg.mem + pg.used++;
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  NRS_CUDA(ctx, cudaStreamIsCapturing(ctx->stream, &capturing));
+  if (capturing != cudaStreamCaptureStatusNone)   // a replay meets the range as the last one left it
+    NRS_CUDA(ctx, cudaMemsetAsync(*out, 0, sizeof(NrsRange), ctx->stream));
+  ++pg.live;
+  ctx->ranges[p] = *out;
+  return NRS_OK;
 }
 
 // One page-locked block per context: the device error word, and behind it the slot of small read-backs.  Pinning takes
@@ -428,6 +468,7 @@ int nrs_free(nrs_ctx* ctx, void* dptr) {
   if (!dptr) return NRS_OK;
   auto it = ctx->pool.live.find(dptr);
   NRS_REQUIRE(ctx, it != ctx->pool.live.end(), NRS_ERR_ARG, "nrs_free: %p was not allocated by nrs_alloc", dptr);
+  nrs_range_drop(ctx, dptr);
   ctx->pool.free_blocks.emplace(it->second, dptr);
   ctx->pool.live.erase(it);
   return NRS_OK;

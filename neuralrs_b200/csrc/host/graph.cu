@@ -23,6 +23,10 @@ static float* dalloc(nrs_ctx* ctx, size_t floats, bool zero = false) {
   return (float*)p;
 }
 
+// An operand plane of `values` values in the context's mode.
+static float* nrs_dplane(nrs_ctx* ctx, size_t values, bool split) { return dalloc(ctx, split ? (values + 1) / 2 : values); }
+static float* dplane(nrs_ctx* ctx, size_t values) { return nrs_dplane(ctx, values, ctx->math_mode == NRS_MATH_3XTF32); }
+
 size_t Node::len() const {
   size_t n = 1;
   for (size_t d : shape) n *= d;
@@ -169,9 +173,9 @@ static bool stage_planes(nrs_ctx* ctx, const float* src, const std::vector<size_
   if (ctx->plane_hints.count(src)) return false;   // already there (the tensor feeds two convolutions)
   const bool split = ctx->math_mode == NRS_MATH_3XTF32;
   const size_t n = shape[0], c = shape[1], hw = shape[2] * shape[3];
-  const size_t floats = n * hw * nrs_plane_ld((int)c);
-  *hi = dalloc(ctx, floats);
-  if (split) *lo = dalloc(ctx, floats);
+  const size_t values = n * hw * nrs_plane_ld((int)c);
+  *hi = dplane(ctx, values);
+  if (split) *lo = dplane(ctx, values);
   check(ctx, nrs_tc_stage_image(ctx, src, *hi, *lo, (int)n, (int)c, (int)hw));
   ctx->plane_hints[src] = NrsPlanes{*hi, *lo, split ? 1 : 0};
   return true;
@@ -187,8 +191,8 @@ static bool stage_planes_2d(nrs_ctx* ctx, const float* src, size_t rows, size_t 
   if (!tc::tensor_map_encoder() || ctx->plane_hints.count(src)) return false;
   const bool split = ctx->math_mode == NRS_MATH_3XTF32;
   const int ld = nrs_plane_ld((int)cols);
-  *hi = dalloc(ctx, rows * ld);
-  if (split) *lo = dalloc(ctx, rows * ld);
+  *hi = dplane(ctx, rows * ld);
+  if (split) *lo = dplane(ctx, rows * ld);
   check(ctx, nrs_tc_stage(ctx, src, *hi, *lo, (int)rows, (int)cols, ld, 1, 0, 0, false));
   NrsPlanes pl{*hi, *lo, split ? 1 : 0};
   pl.rows = (int)rows;
@@ -241,7 +245,7 @@ bool values_as_planes_only(nrs_ctx* ctx, size_t rows, size_t cols, size_t reader
 // The math mode was changed between the passes: the values are wanted after all.
 static void need_values(const NodeP& x) {
   if (!x->planes_only || x->ctx->math_mode == NRS_MATH_3XTF32) return;
-  check(x->ctx, nrs_add(x->ctx, x->planes_hi, x->planes_lo, x->data, x->len()));
+  check(x->ctx, nrs_pair_unpack(x->ctx, x->planes_hi, x->planes_lo, x->data, x->len()));
   x->planes_only = false;
 }
 
@@ -357,8 +361,8 @@ NodeP matmul(const NodeP& a, const NodeP& b) {
       int st = NRS_ERR_UNSUPPORTED;
       if (emit && !ctx->plane_hints.count(t.ptr)) {
         NrsGemmExtras e;
-        e.hi = dalloc(ctx, a->len());
-        if (ctx->math_mode == NRS_MATH_3XTF32) e.lo = dalloc(ctx, a->len());
+        e.hi = dplane(ctx, a->len());
+        if (ctx->math_mode == NRS_MATH_3XTF32) e.lo = dplane(ctx, a->len());
         e.skip_c_unsplit = a->internal && e.lo;
         st = nrs_gemm_extras(ctx, 0, 1, m, k, n, dc, b->data, t.ptr, nullptr, NRS_ACT_NONE, 0.0f, &e);
         if (st == NRS_OK) {
@@ -631,8 +635,8 @@ static void conv_backward(Node* self, const NodeP& x, const NodeP& w, const Node
     float *ghi = nullptr, *glo = nullptr;
     if (fold) {
       if (xr->wants_grad_planes) {
-        ghi = dalloc(ctx, xr->len());
-        if (ctx->math_mode == NRS_MATH_3XTF32) glo = dalloc(ctx, xr->len());
+        ghi = dplane(ctx, xr->len());
+        if (ctx->math_mode == NRS_MATH_3XTF32) glo = dplane(ctx, xr->len());
       }
       ctx->out_extras[t.ptr] = NrsOutExtras{xr->data, ghi, glo, ghi && xr->internal && xr->grad_planes_suffice};
       // ... and per-tile channel sums of the masked gradient, for the producer's bias gradient.
@@ -715,9 +719,9 @@ NodeP conv2d_act(const NodeP& x, const NodeP& w, const NodeP& b, size_t stride, 
   // input's patch planes; make them once.
   if (patches && w->requires_grad && !x->patches_hi && planes_possible(ctx) && (long)n * oh * ow >= kNrsPatchMinPixels &&
       !ctx->patch_hints.count(x->data)) {
-    const size_t floats = (size_t)n * oh * ow * nrs_plane_ld(ci * kh * kw);
-    float* phi = dalloc(ctx, floats);
-    float* plo = ctx->math_mode == NRS_MATH_3XTF32 ? dalloc(ctx, floats) : nullptr;
+    const size_t values = (size_t)n * oh * ow * nrs_plane_ld(ci * kh * kw);
+    float* phi = dplane(ctx, values);
+    float* plo = ctx->math_mode == NRS_MATH_3XTF32 ? dplane(ctx, values) : nullptr;
     const int st = nrs_patch_planes(ctx, x->data, phi, plo, n, ci, h, wd, kh, kw, (int)stride, (int)pad);
     if (st == NRS_OK) {
       x->patches_hi = phi;
@@ -733,8 +737,8 @@ NodeP conv2d_act(const NodeP& x, const NodeP& w, const NodeP& b, size_t stride, 
   // output's NHWC planes itself (otherwise the consumer stages them in a pass of its own).
   float *ohi = nullptr, *olo = nullptr;
   if (emit_planes && co % 32 == 0 && planes_possible(ctx)) {
-    ohi = dalloc(ctx, out->len());
-    if (ctx->math_mode == NRS_MATH_3XTF32) olo = dalloc(ctx, out->len());
+    ohi = dplane(ctx, out->len());
+    if (ctx->math_mode == NRS_MATH_3XTF32) olo = dplane(ctx, out->len());
     ctx->out_extras[out->data] = NrsOutExtras{nullptr, ohi, olo};
   }
   try {
@@ -786,8 +790,8 @@ NodeP conv2d_act(const NodeP& x, const NodeP& w, const NodeP& b, size_t stride, 
       masked = dalloc(ctx, self->len());
       if (want_planes && co % 8 == 0) {   // mask and stage in one pass
         const bool split = ctx->math_mode == NRS_MATH_3XTF32;
-        dhi = dalloc(ctx, self->len());
-        if (split) dlo = dalloc(ctx, self->len());
+        dhi = dplane(ctx, self->len());
+        if (split) dlo = dplane(ctx, self->len());
         check(ctx, nrs_tc_stage_masked(ctx, 0, dy, self->data, nullptr, n, co, (int)self->shape[2], (int)self->shape[3], 1,
                                        masked, dhi, dlo));
         ctx->plane_hints[masked] = NrsPlanes{dhi, dlo, split ? 1 : 0};
@@ -837,8 +841,8 @@ NodeP maxpool2d(const NodeP& x, size_t kernel, size_t stride, bool emit_planes) 
   bool done = false;
   if (emit_planes && k == 2 && s == 2 && c % 8 == 0 && planes_possible(ctx)) {
     // a tensor-core convolution reads the result next: write its operand planes in the same pass
-    float* phi = dalloc(ctx, out->len());
-    float* plo = ctx->math_mode == NRS_MATH_3XTF32 ? dalloc(ctx, out->len()) : nullptr;
+    float* phi = dplane(ctx, out->len());
+    float* plo = ctx->math_mode == NRS_MATH_3XTF32 ? dplane(ctx, out->len()) : nullptr;
     const int st = nrs_tc_pool2_fwd_planes(ctx, x->data, out->data, (int32_t*)am, phi, plo, n, c, h, w);
     if (st == NRS_OK) {
       out->planes_hi = phi;
@@ -865,8 +869,8 @@ NodeP maxpool2d(const NodeP& x, size_t kernel, size_t stride, bool emit_planes) 
       GradTarget t = grad_target(x);   // overwrite mode by construction
       float *phi = nullptr, *plo = nullptr;
       if (xr->wants_grad_planes && planes_possible(ctx) && !xr->gplanes_hi) {
-        phi = dalloc(ctx, xr->len());
-        if (ctx->math_mode == NRS_MATH_3XTF32) plo = dalloc(ctx, xr->len());
+        phi = dplane(ctx, xr->len());
+        if (ctx->math_mode == NRS_MATH_3XTF32) plo = dplane(ctx, xr->len());
       }
       // self->data (the pooled maximum) is > 0 exactly where the ReLU let the winner through.
       float* partial = k == 2 ? dalloc(ctx, nrs_stage_masked_partial_rows(n, h, w) * (size_t)c) : nullptr;
@@ -926,8 +930,8 @@ static NodeP layernorm_impl(const NodeP& x, const NodeP& residual, const NodeP& 
   const bool planes = emit_planes && planes_possible(ctx) && f % 32 == 0 && rows > 0;
   const bool split = ctx->math_mode == NRS_MATH_3XTF32;
   if (planes && !ctx->plane_hints.count(out->data)) {
-    float* hi = dalloc(ctx, x->len());
-    float* lo = split ? dalloc(ctx, x->len()) : nullptr;
+    float* hi = dplane(ctx, x->len());
+    float* lo = split ? dplane(ctx, x->len()) : nullptr;
     int emitted = 0;
     const int st = nrs_layernorm_fwd_planes(ctx, x->data, residual ? residual->data : nullptr, gamma->data, beta->data, out->data,
                                             xhat, istd, rows, f, eps, hi, lo, &emitted);
@@ -990,8 +994,8 @@ static NodeP layernorm_impl(const NodeP& x, const NodeP& residual, const NodeP& 
     const bool fresh_slot = rb && !rb->gplanes_hi && hint == ctx->plane_hints.end();
     if (planes && da && db && acc_b == 0 && (mine || fresh_slot)) {
       // the addend's gradient is exactly this kernel's result: its planes come out of the same pass
-      float* hi = mine ? rb->gplanes_hi : dalloc(ctx, self->len());
-      float* lo = mine ? rb->gplanes_lo : (split ? dalloc(ctx, self->len()) : nullptr);
+      float* hi = mine ? rb->gplanes_hi : nrs_dplane(ctx, self->len(), split);
+      float* lo = mine ? rb->gplanes_lo : (split ? nrs_dplane(ctx, self->len(), true) : nullptr);
       int emitted = 0;
       const int st = nrs_layernorm_bwd_planes(ctx, g, xhat, istd, gamma->data, da, db, dg, dbt, rows, f, acc_a, acc_b, acc_p, hi, lo,
                                               &emitted);
@@ -1066,8 +1070,8 @@ NodeP batchnorm_nd(const NodeP& x, const NodeP& gamma, const NodeP& beta, const 
   const bool planes = x->shape.size() == 4 && c % 8 == 0 && (size_t)n * hw <= 0x7fffffffu && planes_possible(ctx);
   float *hi = nullptr, *lo = nullptr;
   if (planes && emit_planes) {
-    hi = dalloc(ctx, out->len());
-    if (ctx->math_mode == NRS_MATH_3XTF32) lo = dalloc(ctx, out->len());
+    hi = dplane(ctx, out->len());
+    if (ctx->math_mode == NRS_MATH_3XTF32) lo = dplane(ctx, out->len());
     out->planes_hi = hi;   // (the node's from here on, whatever happens)
     out->planes_lo = lo;
   }
@@ -1104,8 +1108,8 @@ NodeP batchnorm_nd(const NodeP& x, const NodeP& gamma, const NodeP& beta, const 
       dx = t.ptr;
       acc_x = t.accumulate;
       if (emit) {
-        xr->gplanes_hi = phi = dalloc(ctx, xr->len());
-        if (ctx->math_mode == NRS_MATH_3XTF32) xr->gplanes_lo = plo = dalloc(ctx, xr->len());
+        xr->gplanes_hi = phi = dplane(ctx, xr->len());
+        if (ctx->math_mode == NRS_MATH_3XTF32) xr->gplanes_lo = plo = dplane(ctx, xr->len());
         xr->gchan_rows = nrs_batchnorm_tiles(n, hw);
         xr->gchan_partial = partial = dalloc(ctx, (size_t)xr->gchan_rows * c);
         xr->grad_premasked = true;   // there is no mask
@@ -1196,8 +1200,8 @@ static void linear_input_grad(nrs_ctx* ctx, const NodeP& x, const NodeP& w, cons
     NrsGemmExtras e;
     e.dact = x->fold_act;
     e.dact_src = x->fold_src;
-    e.hi = dalloc(ctx, x->len());
-    if (ctx->math_mode == NRS_MATH_3XTF32) e.lo = dalloc(ctx, x->len());
+    e.hi = dplane(ctx, x->len());
+    if (ctx->math_mode == NRS_MATH_3XTF32) e.lo = dplane(ctx, x->len());
     e.colsum_cap = (m + 127) / 128 * 4;
     e.colsum = dalloc(ctx, (size_t)e.colsum_cap * k);
     e.skip_c_unsplit = x->internal && e.lo;
@@ -1242,8 +1246,8 @@ NodeP linear_act(const NodeP& x, const NodeP& w, const NodeP& b, int act, bool e
   NrsGemmExtras e;
   e.pre = pre;
   if (tensor_cores && w->requires_grad && n % 8 == 0 && (emit_planes || act == NRS_ACT_GELU) && !ctx->plane_hints.count(out->data)) {
-    e.hi = dalloc(ctx, out->len());
-    if (ctx->math_mode == NRS_MATH_3XTF32) e.lo = dalloc(ctx, out->len());
+    e.hi = dplane(ctx, out->len());
+    if (ctx->math_mode == NRS_MATH_3XTF32) e.lo = dplane(ctx, out->len());
   }
   if (reader_cols > 0) out->internal = true;
   e.skip_c_unsplit = e.lo && act == NRS_ACT_GELU && values_as_planes_only(ctx, (size_t)m, (size_t)n, reader_cols);

@@ -85,7 +85,7 @@ struct Node {
   bool row_planes_wanted = false;
 
   // The result of a step inside a composite layer or a native trainer, which no caller holds: values or a gradient that are read as planes
-  // only need not be written besides.  planes_only: `data` was left out (3xTF32: it is planes_hi + planes_lo exactly).
+  // only need not be written besides.  planes_only: `data` was left out (3xTF32: the f16 pairs hold it to 2^-23).
   bool internal = false, planes_only = false;
 
   size_t len() const;

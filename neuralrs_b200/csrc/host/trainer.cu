@@ -316,11 +316,11 @@ void stage_weights(nrs_trainer* t) {
   NrsWeightSet& ws = ctx->weight_set;
   if (ws.owner != t || ws.mode != ctx->math_mode) {
     std::vector<NrsWeightDesc> d;
-    auto linear = [&](const NodeP& w) {   // W[in,out]: transposed for x@W, as stored for dz@W^T
+    auto linear = [&](const NodeP& w, int group = 0) {   // W[in,out]: transposed for x@W, as stored for dz@W^T
       const int in = (int)w->shape[0], out = (int)w->shape[1];
       if (in < 32 || out < 32) return;    // thin products run on the FFMA kernels
-      d.push_back(NrsWeightDesc{w->data, NRS_WF_LINEAR_T, out, in, 0, 0, 0});
-      d.push_back(NrsWeightDesc{w->data, NRS_WF_LINEAR_ROWS, in, out, 0, 0, 0});
+      d.push_back(NrsWeightDesc{w->data, NRS_WF_LINEAR_T, out, in, 0, 0, 0, group});
+      d.push_back(NrsWeightDesc{w->data, NRS_WF_LINEAR_ROWS, in, out, 0, 0, 0, group});
     };
     size_t pi = 0;
     bool first_contraction = true;
@@ -347,7 +347,7 @@ void stage_weights(nrs_trainer* t) {
         case NRS_LAYER_LAYERNORM: pi += 2; break;
         case NRS_LAYER_EMBEDDING: pi += 1; break;
         case NRS_LAYER_TRANSFORMER_BLOCK:
-          for (int k : {0, 1, 2, 3, 8, 10}) linear(t->params[pi + k]);
+          for (int k : {0, 1, 2, 3, 8, 10}) linear(t->params[pi + k], k < 3 ? (int)pi + 1 : 0);   // (Q, K and V are one product)
           first_contraction = false;
           pi += 12;
           break;

@@ -219,29 +219,30 @@ static NodeP planes_attention(const MultiHeadAttention& m, const NodeP& x, size_
     check(ctx, nrs_alloc(ctx, floats * sizeof(float), 0, &p));
     return (float*)p;
   };
-  auto saved = [&](size_t floats) {
-    float* p = block(floats);
+  auto plane = [block, split](size_t values) { return block(split ? (values + 1) / 2 : values); };
+  auto saved_plane = [&](size_t values) {
+    float* p = plane(values);
     out->saved.push_back(p);
     return p;
   };
   cache_row_planes(x, tokens, d);   // read again by the weight gradients
   NrsGemmExtras e;
   e.skip_c = true;
-  e.hi = saved(tokens * 3 * d);
-  e.lo = split ? saved(tokens * 3 * d) : nullptr;
+  e.hi = saved_plane(tokens * 3 * d);
+  e.lo = split ? saved_plane(tokens * 3 * d) : nullptr;
   const float* w[3] = {wq->data, wk->data, wv->data};
   check(ctx, nrs_tc_gemm_weights(ctx, 0, 3, (int)tokens, (int)d, (int)d, x->data, w, nullptr, 0.0f, &e));
   const size_t square = batch * heads * seq * (size_t)nrs_plane_ld((int)seq);
   NrsMhaPlanes a{};
   a.batch = (int)batch; a.seq = (int)seq; a.heads = (int)heads; a.d_head = (int)d_head; a.causal = m.causal ? 1 : 0;
   a.qkv_hi = e.hi; a.qkv_lo = e.lo; a.qkv_ld = (int)(3 * d);
-  a.p_hi = saved(square);
-  a.p_lo = split ? saved(square) : nullptr;
+  a.p_hi = saved_plane(square);
+  a.p_lo = split ? saved_plane(square) : nullptr;
   out->internal = true;
   out->planes_only = values_as_planes_only(ctx, tokens, d, d);   // read by the output projection alone
   a.out = out->planes_only ? nullptr : out->data;
-  a.out_hi = block(tokens * d);
-  a.out_lo = split ? block(tokens * d) : nullptr;
+  a.out_hi = plane(tokens * d);
+  a.out_lo = split ? plane(tokens * d) : nullptr;
   out->planes_hi = a.out_hi;        // the output projection reads them (and its weight gradient)
   out->planes_lo = a.out_lo;
   NrsPlanes pl{a.out_hi, a.out_lo, split ? 1 : 0};
@@ -254,7 +255,7 @@ static NodeP planes_attention(const MultiHeadAttention& m, const NodeP& x, size_
   check(ctx, st);
   out->row_planes_wanted = true;
   Node* self = out.get();
-  out->backward_fn = [self, x, wq, wk, wv, a, tokens, d, square, split, block]() mutable {
+  out->backward_fn = [self, x, wq, wk, wv, a, tokens, d, square, split, block, plane]() mutable {
     nrs_ctx* ctx = self->ctx;
     struct Mode {   // the saved planes are those of the forward pass's mode
       nrs_ctx* c; const int was;
@@ -263,23 +264,29 @@ static NodeP planes_attention(const MultiHeadAttention& m, const NodeP& x, size_
     } mode{ctx, split ? NRS_MATH_3XTF32 : NRS_MATH_TF32};
     const float* g = grad_view(self);
     // the gradient's row planes: left by the output projection's input-gradient kernel, else staged here (also where that
-    // kernel ran in TF32 and left no residual plane, the math mode having been changed since the forward pass)
+    // kernel ran in another mode than the forward pass: the f32 values that f16 pairs stand for may not have been written)
     float *ghi = self->gplanes_hi, *glo = self->gplanes_lo;
     if (ghi) {
       ctx->plane_hints.erase(g);
       self->gplanes_hi = self->gplanes_lo = nullptr;
     }
-    if (!ghi || (split && !glo)) {
-      if (!ghi) ghi = block(tokens * d);
-      if (split) glo = block(tokens * d);
+    if (ghi && split != (glo != nullptr)) {
+      if (glo) check(ctx, nrs_pair_unpack(ctx, ghi, glo, const_cast<float*>(g), tokens * d));
+      nrs_free(ctx, ghi);
+      if (glo) nrs_free(ctx, glo);
+      ghi = glo = nullptr;
+    }
+    if (!ghi) {
+      ghi = plane(tokens * d);
+      if (split) glo = plane(tokens * d);
       check(ctx, nrs_tc_stage(ctx, g, ghi, glo, (int)tokens, (int)d, (int)d, 1, 0, 0, false));
     }
     a.dout_hi = ghi; a.dout_lo = split ? glo : nullptr;
     a.scores = block(square);
-    a.ds_hi = block(square);
-    a.ds_lo = split ? block(square) : nullptr;
-    a.dqkv_hi = block(tokens * 3 * d);
-    a.dqkv_lo = split ? block(tokens * 3 * d) : nullptr;
+    a.ds_hi = plane(square);
+    a.ds_lo = split ? plane(square) : nullptr;
+    a.dqkv_hi = plane(tokens * 3 * d);
+    a.dqkv_lo = split ? plane(tokens * 3 * d) : nullptr;
     struct Release {
       nrs_ctx* c; std::vector<float*> p; const float* key;
       ~Release() {

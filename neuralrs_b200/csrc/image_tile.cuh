@@ -1,11 +1,12 @@
 // A block's tile of an NCHW image batch: 32 channels x 128 pixels, the pixels counted through the batch (images smaller
 // than 128 pixels share a tile).  Read in 128-byte row segments, 16 independent loads per thread (warp w: channels w,
-// w + 8, w + 16, w + 24, four segments each), written as NHWC TF32 planes in full 128-byte lines (32 channels of a
+// w + 8, w + 16, w + 24, four segments each), written as NHWC operand planes in full 128-byte lines (32 channels of a
 // pixel, 128-bit stores).
 #pragma once
 
 #include "igemm_problems.cuh"
 #include "nrs_internal.h"
+#include "pair.cuh"
 #include "tc_common.cuh"
 
 namespace img {
@@ -43,7 +44,8 @@ struct Pixels {
 };
 
 template <bool SPLIT>
-__device__ __forceinline__ void tile_to_planes(const Tile& tile, const Grid& g, uint32_t p0, int c0, float* __restrict__ hi, float* __restrict__ lo) {
+__device__ __forceinline__ void tile_to_planes(const Tile& tile, const Grid& g, uint32_t p0, int c0, float* __restrict__ hi, float* __restrict__ lo,
+                                               float scale = 1.0f) {
   const int cq = (threadIdx.x & 7) * 4;
   if (c0 + cq >= g.ld) return;
 #pragma unroll
@@ -51,10 +53,9 @@ __device__ __forceinline__ void tile_to_planes(const Tile& tile, const Grid& g, 
     const int pl = k * 32 + (threadIdx.x >> 3);
     if (p0 + pl >= g.pixels) break;
     const float4 f = make_float4(tile[cq][pl], tile[cq + 1][pl], tile[cq + 2][pl], tile[cq + 3][pl]);
-    const float4 h = make_float4(tc::tf32_rn(f.x), tc::tf32_rn(f.y), tc::tf32_rn(f.z), tc::tf32_rn(f.w));
     const size_t o = (size_t)(p0 + pl) * g.ld + c0 + cq;
-    *reinterpret_cast<float4*>(hi + o) = h;
-    if (SPLIT) *reinterpret_cast<float4*>(lo + o) = make_float4(f.x - h.x, f.y - h.y, f.z - h.z, f.w - h.w);
+    if (SPLIT) pr::put4(hi, lo, o, f, scale);
+    else *reinterpret_cast<float4*>(hi + o) = make_float4(tc::tf32_rn(f.x), tc::tf32_rn(f.y), tc::tf32_rn(f.z), tc::tf32_rn(f.w));
   }
 }
 

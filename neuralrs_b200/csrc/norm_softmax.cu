@@ -15,6 +15,7 @@
 // semantics src/nn/normalization.rs:38-103, src/autograd/graph/softmax.rs:23-60.
 #include "fold.h"
 #include "nrs_internal.h"
+#include "pair.cuh"
 #include "row_pipe.cuh"
 #include "tc_common.cuh"
 
@@ -170,10 +171,19 @@ struct SoftmaxBwdOp {
 
 // The TF32 operand planes of a value that the next tensor-core GEMM will read (rows x f, the tensor's own
 // layout): written by the producing kernel so that no separate staging pass reads the tensor again.
-__device__ __forceinline__ void put_planes(float* hi, float* lo, size_t at, float4 v) {
-  const float4 h = make_float4(tc::tf32_rn(v.x), tc::tf32_rn(v.y), tc::tf32_rn(v.z), tc::tf32_rn(v.w));
-  *reinterpret_cast<float4*>(hi + at) = h;
-  if (lo) *reinterpret_cast<float4*>(lo + at) = make_float4(v.x - h.x, v.y - h.y, v.z - h.z, v.w - h.w);
+__device__ __forceinline__ void put_planes(float* hi, float* lo, size_t at, float4 v, float scale, uint32_t& top) {
+  if (lo) {
+    top = pr::seen4(top, v);
+    pr::put4(hi, lo, at, v, scale);
+  } else {
+    *reinterpret_cast<float4*>(hi + at) = make_float4(tc::tf32_rn(v.x), tc::tf32_rn(v.y), tc::tf32_rn(v.z), tc::tf32_rn(v.w));
+  }
+}
+// f16 pairs: the scale of a result of `bound`, which one thread of the grid leaves as its range.
+__device__ __forceinline__ float open_pairs(NrsRange* range, float bound) {
+  bound = fminf(bound * 1.001f, 3.0e38f);
+  if (blockIdx.x == 0 && threadIdx.x == 0) range->bound = bound;
+  return pr::scale_of(bound);
 }
 
 __device__ __forceinline__ float wsum(float v) {
@@ -204,11 +214,23 @@ __global__ void __launch_bounds__(kRowThreads)
 ln_fwd_vec_kernel(const float* __restrict__ a, const float* __restrict__ b, const float* __restrict__ gamma,
                   const float* __restrict__ beta, float* __restrict__ y, float* __restrict__ xhat,
                   float* __restrict__ istd_out, int rows, int f, float eps, float* __restrict__ y_hi,
-                  float* __restrict__ y_lo) {
+                  float* __restrict__ y_lo, NrsRange* __restrict__ range) {
   NRS_PDL_PROLOGUE();
   const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
   const int f4 = f >> 2;
   const float inv_f = 1.0f / (float)f;
+  [[maybe_unused]] float scale = 1.0f;
+  [[maybe_unused]] uint32_t top = 0;
+  if (EMIT && y_lo) {   // |xhat| <= sqrt(f)
+    uint32_t mg = 0, mb = 0;
+    for (int c = lane; c < f4; c += 32) {
+      mg = pr::seen4(mg, ld4(gamma + 4 * c));
+      mb = pr::seen4(mb, ld4(beta + 4 * c));
+    }
+    mg = __reduce_max_sync(0xffffffffu, mg);
+    mb = __reduce_max_sync(0xffffffffu, mb);
+    scale = open_pairs(range, sqrtf((float)f) * __uint_as_float(mg) + __uint_as_float(mb));
+  }
   for (int r = blockIdx.x * wpb + (threadIdx.x >> 5); r < rows; r += gridDim.x * wpb) {
     const size_t base = (size_t)r * f;
     float4 v[VPL];
@@ -247,10 +269,11 @@ ln_fwd_vec_kernel(const float* __restrict__ a, const float* __restrict__ b, cons
         if (xhat) st4_stream(xhat + base + 4 * c, xn);
         const float4 out = make_float4(gm.x * xn.x + bt.x, gm.y * xn.y + bt.y, gm.z * xn.z + bt.z, gm.w * xn.w + bt.w);
         st4_stream(y + base + 4 * c, out);
-        if (EMIT) put_planes(y_hi, y_lo, base + 4 * c, out);
+        if (EMIT) put_planes(y_hi, y_lo, base + 4 * c, out, scale, top);
       }
     }
   }
+  if (EMIT && y_lo) pr::report(range, top);
 }
 
 __global__ void __launch_bounds__(kRowThreads)
@@ -286,7 +309,8 @@ template <int VPL, bool EMIT>
 __global__ void __launch_bounds__(kRowThreads)
 ln_bwd_vec_kernel(const float* __restrict__ g, const float* __restrict__ xhat, const float* __restrict__ istd,
                   const float* __restrict__ gamma, float* dx, float* dx2, float* __restrict__ partial, int rows, int f,
-                  int acc1, int acc2, float* __restrict__ d_hi, float* __restrict__ d_lo) {
+                  int acc1, int acc2, float* __restrict__ d_hi, float* __restrict__ d_lo, const NrsRange* __restrict__ range_g,
+                  const NrsRange* __restrict__ range_istd, NrsRange* __restrict__ range) {
   NRS_PDL_PROLOGUE();
   extern __shared__ float ln_smem[];          // [warps][2][f] when partial != nullptr
   const int lane = threadIdx.x & 31, wrp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
@@ -298,6 +322,15 @@ ln_bwd_vec_kernel(const float* __restrict__ g, const float* __restrict__ xhat, c
     const int c = lane + 32 * k;
     gm[k] = c < f4 ? ld4(gamma + 4 * c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     pg[k] = pb[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  }
+  [[maybe_unused]] float scale = 1.0f;
+  [[maybe_unused]] uint32_t top = 0;
+  if (EMIT && d_lo) {   // both means are at most the largest |g * gamma| (times |xhat| <= sqrt(f))
+    uint32_t mg = 0;
+#pragma unroll
+    for (int k = 0; k < VPL; ++k) mg = pr::seen4(mg, gm[k]);
+    mg = __reduce_max_sync(0xffffffffu, mg);
+    scale = open_pairs(range, (2.0f + sqrtf((float)f)) * __uint_as_float(mg) * range_g->top * range_istd->top);
   }
   for (int r = blockIdx.x * wpb + wrp; r < rows; r += gridDim.x * wpb) {
     const size_t base = (size_t)r * f;
@@ -330,7 +363,7 @@ ln_bwd_vec_kernel(const float* __restrict__ g, const float* __restrict__ xhat, c
           float4 o;
           o.x = is * (gv[k].x - s1 - xh[k].x * s2); o.y = is * (gv[k].y - s1 - xh[k].y * s2);
           o.z = is * (gv[k].z - s1 - xh[k].z * s2); o.w = is * (gv[k].w - s1 - xh[k].w * s2);
-          if (EMIT) put_planes(d_hi, d_lo, base + 4 * c, o);   // planes of the gradient itself (before any accumulation)
+          if (EMIT) put_planes(d_hi, d_lo, base + 4 * c, o, scale, top);   // planes of the gradient itself (before any accumulation)
           float4 w = o;
           if (acc1) { const float4 old = ld4(dx + base + 4 * c); w.x += old.x; w.y += old.y; w.z += old.z; w.w += old.w; }
           st4(dx + base + 4 * c, w);
@@ -342,6 +375,7 @@ ln_bwd_vec_kernel(const float* __restrict__ g, const float* __restrict__ xhat, c
       }
     }
   }
+  if (EMIT && d_lo) pr::report(range, top);
   if (partial) {
     float* mine = ln_smem + (size_t)wrp * 2 * f;
 #pragma unroll
@@ -576,12 +610,17 @@ int layernorm_fwd(nrs_ctx* ctx, const char* who, const float* a, const float* b,
     if (st != NRS_ERR_UNSUPPORTED) return st;
   }
   if (vpl) {
+    NrsRange* range = nullptr;
+    if (y_hi && y_lo) {
+      const int st = nrs_range_renew(ctx, y_hi, &range);
+      if (st != NRS_OK) return st;
+    }
     if (y_hi)
       NRS_DISPATCH_VPL(vpl, NRS_PDL_LAUNCH((ln_fwd_vec_kernel<V, true>), row_grid(ctx, rows), kRowThreads, 0, ctx->stream, a, b, gamma,
-                                           beta, y, xhat, istd, rows, f, eps, y_hi, y_lo));
+                                           beta, y, xhat, istd, rows, f, eps, y_hi, y_lo, range));
     else
       NRS_DISPATCH_VPL(vpl, NRS_PDL_LAUNCH((ln_fwd_vec_kernel<V, false>), row_grid(ctx, rows), kRowThreads, 0, ctx->stream, a, b, gamma,
-                                           beta, y, xhat, istd, rows, f, eps, y_hi, y_lo));
+                                           beta, y, xhat, istd, rows, f, eps, y_hi, y_lo, range));
     if (emitted && y_hi) *emitted = 1;
   } else {
     NRS_PDL_LAUNCH(ln_fwd_kernel, row_grid(ctx, rows), kRowThreads, 0, ctx->stream, a, b, gamma, beta, y, xhat, istd, rows, f, eps);
@@ -666,12 +705,21 @@ int layernorm_bwd(nrs_ctx* ctx, const char* who, const float* g, const float* xh
       if (st != NRS_OK) return st;
     }
     const size_t smem = dgamma ? (size_t)warps * 2 * f * sizeof(float) : 0;
+    NrsRange *range = nullptr, *range_g = nullptr, *range_istd = nullptr;
+    if (dx && d_hi && d_lo) {
+      int st = nrs_range_renew(ctx, d_hi, &range);
+      if (st == NRS_OK) st = nrs_range_renew(ctx, &ctx->scratch_range[0], &range_g);
+      if (st == NRS_OK) st = nrs_range_renew(ctx, &ctx->scratch_range[1], &range_istd);
+      if (st == NRS_OK) st = nrs_absmax2(ctx, g, elems, range_g, istd, (size_t)rows, range_istd);
+      if (st != NRS_OK) return st;
+    }
     if (dx && d_hi)
       NRS_DISPATCH_VPL(vpl, NRS_PDL_LAUNCH((ln_bwd_vec_kernel<V, true>), blocks, warps * 32, smem, ctx->stream, g, xhat, istd, gamma, dx,
-                                           dx2, partial, rows, f, acc1, acc2, d_hi, d_lo));
+                                           dx2, partial, rows, f, acc1, acc2, d_hi, d_lo, (const NrsRange*)range_g, (const NrsRange*)range_istd, range));
     else
       NRS_DISPATCH_VPL(vpl, NRS_PDL_LAUNCH((ln_bwd_vec_kernel<V, false>), blocks, warps * 32, smem, ctx->stream, g, xhat, istd, gamma, dx,
-                                           dx2, partial, rows, f, acc1, acc2, (float*)nullptr, (float*)nullptr));
+                                           dx2, partial, rows, f, acc1, acc2, (float*)nullptr, (float*)nullptr, (const NrsRange*)nullptr,
+                                           (const NrsRange*)nullptr, (NrsRange*)nullptr));
     if (emitted && dx && d_hi) *emitted = 1;
     NRS_LAUNCHED(ctx);
     return dgamma ? fold_params(ctx, partial, dgamma, dbeta, f, blocks, accumulate_params) : NRS_OK;

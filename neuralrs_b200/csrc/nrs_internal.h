@@ -9,6 +9,7 @@
 #include <iterator>
 #include <map>
 #include <string>
+#include <unordered_map>
 #include <utility>
 #include <vector>
 
@@ -50,12 +51,32 @@ struct NrsPool {
   }
 };
 
+// What is known on the device about the magnitudes of a tensor whose values exist as f16 pairs (pair.cuh): `bound`, which
+// no finite value exceeds and which the pairs' exponent comes from, and `top`, the largest finite magnitude that was
+// written (where its writer only has a bound: that), which bounds of results are made of.
+struct NrsRange {
+  float bound, top;
+  float pad[6];   // a sector each
+};
+// Ranges are cut from pages that are zeroed as a whole, on the context's stream, once all ranges of a page are back.
+struct NrsRangePool {
+  static constexpr int kPerPage = 256;
+  struct Page { NrsRange* mem; int used, live; };
+  std::vector<Page> pages;
+  size_t current = 0;
+};
+
 struct NrsProfRecord {
   int kind;
   double work;
   cudaEvent_t start, stop;
 };
 
+// The address of value `at` of a plane.
+inline float* nrs_plane_at(const float* plane, size_t at, bool split) { return (float*)((uint8_t*)plane + at * (split ? 2 : 4)); }
+// Operand planes: TF32 mode: the values rounded to TF32, in f32 storage (hi).  3xTF32: f16 pairs (pair.cuh), hi and lo in
+// f16 storage each; the tensor's NrsRange is found by the address of hi (nrs_range_of).  The pointers are typed float* in
+// both cases.
 // NHWC planes of an NCHW activation, staged ahead of time by a caller that knows
 // the tensor will feed several tensor-core convolutions (forward and weight gradient,
 // or data and weight gradient).  lo is null unless `split` (3xTF32).
@@ -90,8 +111,9 @@ constexpr inline int nrs_plane_ld(int channels) { return (channels + 7) & ~7; }
 // an entry still present after the call means the caller has to do the work itself.
 struct NrsOutExtras {
   const float* relu_mask_src;   // NCHW tensor of out's shape: out = relu_mask_src > 0 ? out : 0 (or null)
-  float* hi;                    // NHWC TF32 planes of the (masked) result, or null
-  float* lo;                    // residual plane (3xTF32), or null
+  float* hi;                    // NHWC operand planes of the (masked) result, or null
+  float* lo;                    // (3xTF32)
+  bool measure = false;         // 3xTF32, no planes: leave the result's range with its address (nrs_range_of)
   bool planes_suffice = false;  // the result itself need not be written where its planes and channel sums are
 };
 
@@ -115,10 +137,12 @@ struct NrsWeightDesc {
   int form;
   int rows, K;        // linear forms: the DESTINATION's row count and reduction length
   int co, ci, taps;   // convolution forms
+  int group = 0;      // not 0: consecutive weights of one group share a range (they meet in one product)
 };
 struct NrsWeightPlanes {
   float* hi;
   float* lo;          // null unless 3xTF32
+  const NrsRange* range;
   int rows, K, co, ci, taps;
 };
 struct NrsWeightSet {
@@ -134,6 +158,9 @@ struct NrsWeightSet {
   // per job, in launch order: the weight it reads and its first block (the last entry of job_first is `blocks`)
   std::vector<const float*> job_src;
   std::vector<unsigned> job_first;
+  std::vector<unsigned> job_scan;   // the same of the launch that measures ranges (3xTF32)
+  std::vector<int> job_group;       // first job of its group
+  NrsRange* ranges = nullptr;
   int refreshed_jobs = 0;   // jobs restaged range by range since the last full refresh / reset (refresh_range)
 };
 
@@ -201,7 +228,10 @@ struct nrs_ctx {
   // Planes registered for a source tensor (keyed by its device pointer); the conv kernels
   // use them instead of staging again.  Whoever registers keeps both alive and unregisters.
   std::map<const void*, NrsPlanes> plane_hints;
-  std::map<const void*, NrsPlanes> owned_planes;   // nrs_planes_cache: planes the context itself allocated
+  std::map<const void*, NrsPlanes> owned_planes;
+  std::unordered_map<const void*, NrsRange*> ranges;   // of f16 pair planes (by the address of hi) and of f32 tensors (by their address)
+  NrsRangePool range_pool;
+  char scratch_range[2];   // addresses that own the ranges of measurements inside a call   // nrs_planes_cache: planes the context itself allocated
   std::map<const void*, NrsOutExtras> out_extras;
   std::map<const void*, NrsColsumRequest> colsum_requests;
   // Patch planes (see conv_patch.cu) of a tensor with few channels, keyed by its device pointer: the host graph
@@ -259,9 +289,22 @@ int nrs_workspace(nrs_ctx* ctx, size_t bytes, void** out);
 // data gradient's K-split is still being folded out of NRS_WS_PARTIAL)
 enum { NRS_WS_A = 0, NRS_WS_B = 1, NRS_WS_PARTIAL = 2, NRS_WS_WGRAD_PARTIAL = 3, NRS_WS_FOLD = 4, NRS_WS_COUNT = 5 };
 int nrs_ws_slot(nrs_ctx* ctx, int slot, size_t bytes, void** out);
-// Room for operand planes of `bytes` each in one slot: the high plane, and with `split` the residual plane behind it (one
-// block to ask the driver for instead of two); *lo is null otherwise.
-int nrs_ws_planes(nrs_ctx* ctx, int slot, size_t bytes, bool split, void** hi, void** lo);
+// Room for operand planes of `values` values in one slot (with `split` both of a pair in one block); *lo is null without.
+int nrs_ws_planes(nrs_ctx* ctx, int slot, size_t values, bool split, void** hi, void** lo);
+// A new range, all zero, for what is written to `p` next; it belongs to the address until that is renewed, dropped or
+// freed (nrs_free).
+int nrs_range_renew(nrs_ctx* ctx, const void* p, NrsRange** out);
+void nrs_range_drop(nrs_ctx* ctx, const void* p);
+inline NrsRange* nrs_range_of(const nrs_ctx* ctx, const void* p) {
+  auto it = ctx->ranges.find(p);
+  return it == ctx->ranges.end() ? nullptr : it->second;
+}
+// Largest finite magnitude of `count` values at `src` into r->top and r->bound (tc_stage.cu).
+int nrs_absmax(nrs_ctx* ctx, const float* src, size_t count, NrsRange* r);
+// The same of two tensors in one launch.
+int nrs_absmax2(nrs_ctx* ctx, const float* a, size_t na, NrsRange* ra, const float* b, size_t nb, NrsRange* rb);
+// dst = the values of n consecutive f16 pairs.
+int nrs_pair_unpack(nrs_ctx* ctx, const float* hi, const float* lo, float* dst, size_t n);
 int nrs_err_flag(nrs_ctx* ctx, int** out);
 void nrs_pinned_release(nrs_ctx* ctx);
 // Zero-initialised device counters (kNrsFoldTickets of them) for "the last block to arrive folds the partials"
@@ -276,9 +319,10 @@ extern "C" int nrs_layernorm_fwd_planes(nrs_ctx* ctx, const float* a, const floa
 extern "C" int nrs_layernorm_bwd_planes(nrs_ctx* ctx, const float* g, const float* xhat, const float* istd, const float* gamma,
                                         float* da, float* db, float* dgamma, float* dbeta, int rows, int f, int accumulate_da,
                                         int accumulate_db, int accumulate_params, float* d_hi, float* d_lo, int* emitted);
-// TF32 planes of a batch of [rows][K] matrices (tc_stage.cu); see tc_mainloop.cuh for the layouts.
+// Operand planes of a batch of [rows][K] matrices (tc_stage.cu); see tc_mainloop.cuh for the layouts.  3xTF32: the range
+// of `hi` is renewed and measured first, unless the caller has one that covers the source's values.
 int nrs_tc_stage(nrs_ctx* ctx, const float* src, float* hi, float* lo, int rows, int K, int ldk, int batch,
-                 size_t src_bstride, size_t dst_bstride, bool src_k_by_rows);
+                 size_t src_bstride, size_t dst_bstride, bool src_k_by_rows, NrsRange* measured = nullptr);
 // NHWC planes of an NCHW tensor [n][c][hw], pixel stride nrs_plane_ld(c) floats (zeros between c and there).
 // chan_partial (hw > 1): [nrs_batchnorm_tiles(n, hw)][c] channel sums of the pixels of each tile.
 int nrs_tc_stage_image(nrs_ctx* ctx, const float* src, float* hi, float* lo, int n, int c, int hw, float* chan_partial = nullptr);
@@ -442,8 +486,10 @@ struct NrsGemmExtras {
   // the value without the factor; planes and column sums are of the value with it.
   int dact = NRS_ACT_NONE;
   const float* dact_src = nullptr;
-  float* hi = nullptr;         // TF32 planes [m][n] for the GEMM that reads the result next (n a multiple of 8)
+  float* hi = nullptr;         // operand planes [m][n] for the GEMM that reads the result next (n a multiple of 8)
   float* lo = nullptr;
+  NrsRange* range = nullptr;   // out, 3xTF32: of the planes (or, asked for with `measure`, of c); belongs to hi (c)
+  bool measure = false;        // the largest magnitude of c is wanted where no planes are
   float* colsum = nullptr;     // [colsum_cap][n] partial column sums
   int colsum_cap = 0;
   int colsum_rows = 0;         // out: rows of it written (0: none, the caller sums the columns itself)

@@ -1,0 +1,88 @@
+// Operands of the 3xTF32 mode: an f32 value as a pair of f16 values,
+//
+//   x = (hi + lo / 2048) / 2^e,     hi = f16(x * 2^e),  lo = f16((x * 2^e - hi) * 2048),
+//
+// with one exponent e per tensor, taken from a bound of its largest magnitude (NrsRange::bound): bound * 2^e lies in
+// [2^14, 2^15).  Both roundings are to nearest, so the pair carries x to 2^-23 of itself (a TF32 value and its residual as
+// the tensor core reads it, truncated: 2^-22) down to 2^-29 of the bound, and to 2^-51 of the bound below that.  A product
+// is hi.hi + (hi.lo + lo.hi) / 2048, on kind::f16 at twice the rate of kind::tf32 and with half the bytes per value; the
+// two parts are summed in accumulators of their own, and the epilogue brings them together and takes the exponents out.
+// Infinities and NaNs make hi the same and lo NaN, as a TF32 value and its residual did.
+#pragma once
+
+#include <cuda_fp16.h>
+
+#include "nrs_internal.h"
+
+namespace pr {
+
+constexpr float kLoScale = 2048.0f, kLoUnscale = 1.0f / 2048.0f;
+
+// The exponent for a tensor bounded by `bound` (finite, not negative).
+__device__ __forceinline__ int scale_exp(float bound) { return min(126, 141 - (int)(__float_as_uint(bound) >> 23)); }
+__device__ __forceinline__ float pow2(int e) { return __uint_as_float((uint32_t)(e + 127) << 23); }   // -126 <= e <= 127
+__device__ __forceinline__ float scale_of(float bound) { return pow2(scale_exp(bound)); }
+// The factor that takes two operands' exponents out of their product, in two halves (by itself it may leave f32's range).
+struct Unscale {
+  float a, b;
+  __device__ __forceinline__ Unscale(float bound_a, float bound_b) {
+    const int e = -(scale_exp(bound_a) + scale_exp(bound_b));
+    a = pow2(e / 2);
+    b = pow2(e - e / 2);
+  }
+  __device__ __forceinline__ float operator()(float hh, float cross) const { return fmaf(cross, kLoUnscale, hh) * a * b; }
+};
+
+__device__ __forceinline__ void split(float v, float scale, __half* hi, __half* lo) {
+  const float x = v * scale;
+  *hi = __float2half_rn(x);
+  *lo = __float2half_rn((x - __half2float(*hi)) * kLoScale);
+}
+__device__ __forceinline__ void split2(float x, float y, __half2* hi, __half2* lo) {   // already scaled
+  *hi = __floats2half2_rn(x, y);
+  const float2 f = __half22float2(*hi);
+  *lo = __floats2half2_rn((x - f.x) * kLoScale, (y - f.y) * kLoScale);
+}
+__device__ __forceinline__ uint32_t bits(__half2 h) { return *reinterpret_cast<const uint32_t*>(&h); }
+__device__ __forceinline__ void split4(float4 v, float scale, uint2* hi, uint2* lo) {
+  __half2 h0, h1, l0, l1;
+  split2(v.x * scale, v.y * scale, &h0, &l0);
+  split2(v.z * scale, v.w * scale, &h1, &l1);
+  *hi = make_uint2(bits(h0), bits(h1));
+  *lo = make_uint2(bits(l0), bits(l1));
+}
+__device__ __forceinline__ void put(void* hi, void* lo, size_t at, float v, float scale) {
+  split(v, scale, reinterpret_cast<__half*>(hi) + at, reinterpret_cast<__half*>(lo) + at);
+}
+// Four values to an index that is a multiple of 4.
+__device__ __forceinline__ void put4(void* hi, void* lo, size_t at, float4 v, float scale) {
+  uint2 h, l;
+  split4(v, scale, &h, &l);
+  *reinterpret_cast<uint2*>(reinterpret_cast<__half*>(hi) + at) = h;
+  *reinterpret_cast<uint2*>(reinterpret_cast<__half*>(lo) + at) = l;
+}
+__device__ __forceinline__ float4 get4(const void* hi, const void* lo, size_t at, float unscale) {
+  const uint2 h = *reinterpret_cast<const uint2*>(reinterpret_cast<const __half*>(hi) + at);
+  const uint2 l = *reinterpret_cast<const uint2*>(reinterpret_cast<const __half*>(lo) + at);
+  auto two = [](uint32_t u) { return __half22float2(*reinterpret_cast<const __half2*>(&u)); };
+  const float2 h0 = two(h.x), h1 = two(h.y), l0 = two(l.x), l1 = two(l.y);
+  return make_float4(fmaf(l0.x, kLoUnscale, h0.x) * unscale, fmaf(l0.y, kLoUnscale, h0.y) * unscale, fmaf(l1.x, kLoUnscale, h1.x) * unscale,
+                     fmaf(l1.y, kLoUnscale, h1.y) * unscale);
+}
+
+// Largest finite magnitude seen, as the bits of a float (which order like the magnitudes).
+__device__ __forceinline__ uint32_t seen(uint32_t top, float v) {
+  const uint32_t u = __float_as_uint(v) & 0x7fffffffu;
+  return u < 0x7f800000u && u > top ? u : top;
+}
+__device__ __forceinline__ uint32_t seen4(uint32_t top, float4 v) { return seen(seen(seen(seen(top, v.x), v.y), v.z), v.w); }
+// A whole warp's, into the tensor's range.
+__device__ __forceinline__ void report(NrsRange* r, uint32_t top) {
+  top = __reduce_max_sync(0xffffffffu, top);
+  if ((threadIdx.x & 31) == 0 && top > __float_as_uint(*(volatile float*)&r->top)) atomicMax(reinterpret_cast<unsigned*>(&r->top), top);
+}
+// Bound of a sum of `k` products of values up to a and b, plus a value up to c: with room for the sum's own rounding,
+// and finite.
+__device__ __forceinline__ float product_bound(float k, float a, float b, float c) { return fminf((k * a * b + c) * 1.001f, 3.0e38f); }
+
+}  // namespace pr

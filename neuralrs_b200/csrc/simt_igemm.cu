@@ -17,6 +17,7 @@
 #include "fold.h"
 #include "igemm_problems.cuh"
 #include "nrs_internal.h"
+#include "pair.cuh"
 #include "tc_common.cuh"
 
 namespace {
@@ -245,10 +246,18 @@ thin_k_kernel(const float* __restrict__ a, const float* __restrict__ b, float* c
 constexpr int kFoldRows = 64;
 __global__ void __launch_bounds__(256)
 thin_fold_kernel(const float* __restrict__ dz, const float* __restrict__ w, float* __restrict__ c, const float* __restrict__ src, int relu,
-                 float* __restrict__ hi, float* __restrict__ lo, float* __restrict__ colsum, int m, int k, int n) {
+                 float* __restrict__ hi, float* __restrict__ lo, float* __restrict__ colsum, int m, int k, int n,
+                 const NrsRange* __restrict__ range_dz, const NrsRange* __restrict__ range_w, NrsRange* __restrict__ range) {
   NRS_PDL_PROLOGUE();
   __shared__ float part[8][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float scale = 1.0f;
+  uint32_t top = 0;
+  if (lo) {
+    const float bound = pr::product_bound((float)n, range_dz->top, range_w->top, 0.0f) * (relu ? 1.0f : 1.25f);
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) range->bound = bound;
+    scale = pr::scale_of(bound);
+  }
   const int col = blockIdx.x * 32 + lane, r0 = blockIdx.y * kFoldRows, r1 = min(m, r0 + kFoldRows);
   const bool live = col < k;
   float wv[kThinN];
@@ -265,10 +274,17 @@ thin_fold_kernel(const float* __restrict__ dz, const float* __restrict__ w, floa
     const size_t at = (size_t)r * k + col;
     if (c) c[at] = acc;
     const float s = src[at], v = acc * (relu ? (s > 0.0f ? 1.0f : 0.0f) : nrs_gelu_d(s));
-    const float h = tc::tf32_rn(v);
-    hi[at] = h;
-    if (lo) lo[at] = v - h;
+    if (lo) {
+      top = pr::seen(top, v);
+      pr::put(hi, lo, at, v, scale);
+    } else {
+      hi[at] = tc::tf32_rn(v);
+    }
     sum += v;
+  }
+  if (lo) {
+    __syncwarp();
+    pr::report(range, top);
   }
   part[warp][lane] = sum;
   __syncthreads();
@@ -595,9 +611,17 @@ int nrs_gemm_extras(nrs_ctx* ctx, int trans_a, int trans_b, int m, int n, int k,
       k <= kThinN && n % 8 == 0 && m <= 4096 && !bias && act == NRS_ACT_NONE && beta == 0.0f && !extras->pre) {
     const int row_blocks = (m + kFoldRows - 1) / kFoldRows;
     if (row_blocks <= extras->colsum_cap) {
+      NrsRange *range_a = nullptr, *range_b = nullptr;
+      if (extras->lo) {
+        int st = nrs_range_renew(ctx, extras->hi, &extras->range);
+        if (st == NRS_OK) st = nrs_range_renew(ctx, &ctx->scratch_range[0], &range_a);
+        if (st == NRS_OK) st = nrs_range_renew(ctx, &ctx->scratch_range[1], &range_b);
+        if (st == NRS_OK) st = nrs_absmax2(ctx, a, (size_t)m * k, range_a, b, (size_t)n * k, range_b);
+        if (st != NRS_OK) return st;
+      }
       NRS_PDL_LAUNCH(thin_fold_kernel, dim3((unsigned)((n + 31) / 32), (unsigned)row_blocks), 256, 0, ctx->stream, a, b,
                      extras->skip_c || extras->skip_c_unsplit ? nullptr : c, extras->dact_src, extras->dact == NRS_ACT_RELU ? 1 : 0, extras->hi,
-                     extras->lo, extras->colsum, m, n, k);
+                     extras->lo, extras->colsum, m, n, k, (const NrsRange*)range_a, (const NrsRange*)range_b, extras->range);
       NRS_LAUNCHED(ctx);
       extras->honoured = true;
       extras->colsum_rows = row_blocks;
@@ -713,11 +737,11 @@ int nrs_conv2d_bwd(nrs_ctx* ctx, const float* x, const float* w, const float* dy
   // With the bias gradient wanted too, dy is staged first, and its channel sums come out of that pass.
   if (db && !dy_had_planes && ctx->math_mode != NRS_MATH_FP32 && tc::tensor_map_encoder() && stride <= 8 && g.oh * g.ow > 1 &&
       (size_t)n * g.oh * g.ow < ((size_t)1 << 27) && (dx || (dw && !conv_runs_direct(ctx, n, ci, kh, kw, h, wd, stride, pad)))) {
-    const size_t floats = (size_t)n * g.oh * g.ow * nrs_plane_ld(co);
+    const size_t values = (size_t)n * g.oh * g.ow * nrs_plane_ld(co);
     const int tiles = nrs_batchnorm_tiles(n, g.oh * g.ow);
     void *hi = nullptr, *lo = nullptr;
     float* partial = nullptr;
-    st = nrs_ws_planes(ctx, NRS_WS_A, floats * sizeof(float), split3, &hi, &lo);
+    st = nrs_ws_planes(ctx, NRS_WS_A, values, split3, &hi, &lo);
     if (st == NRS_OK) st = nrs_fold_partial(ctx, -1, (size_t)tiles * co * sizeof(float), &partial);
     if (st == NRS_OK) st = nrs_tc_stage_image(ctx, dy, (float*)hi, (float*)lo, n, co, g.oh * g.ow, partial);
     if (st == NRS_OK) st = nrs_fold_columns(ctx, partial, db, tiles, co, co, accumulate);
@@ -734,7 +758,7 @@ int nrs_conv2d_bwd(nrs_ctx* ctx, const float* x, const float* w, const float* dy
     if (st != NRS_OK && st != NRS_ERR_UNSUPPORTED) return st;
     if (st == NRS_OK && dw && !dy_had_planes && !dy_planes_lent && ctx->ws_slot[NRS_WS_A]) {   // (as large as dy's planes already)
       void *hi = nullptr, *lo = nullptr;
-      const int got = nrs_ws_planes(ctx, NRS_WS_A, (size_t)n * g.oh * g.ow * nrs_plane_ld(co) * sizeof(float), split3, &hi, &lo);
+      const int got = nrs_ws_planes(ctx, NRS_WS_A, (size_t)n * g.oh * g.ow * nrs_plane_ld(co), split3, &hi, &lo);
       if (got != NRS_OK) return got;
       ctx->plane_hints[dy] = NrsPlanes{(float*)hi, (float*)lo, split3 ? 1 : 0};
       dy_planes_lent = true;
@@ -797,11 +821,10 @@ int nrs_planes_cache(nrs_ctx* ctx, const float* t, int n, int c, int h, int w) {
   if (c < 8) return NRS_OK;                        // such layers read patches (nrs_conv_uses_patches)
   if (ctx->plane_hints.count(t)) return NRS_OK;   // someone else (the node graph) already keeps planes of it
   const bool split = ctx->math_mode == NRS_MATH_3XTF32;
-  const size_t hw = (size_t)h * w, floats = (size_t)n * nrs_plane_ld(c) * hw;
-  const size_t each = (floats + 63) / 64 * 64;
+  const size_t hw = (size_t)h * w, each = ((size_t)n * nrs_plane_ld(c) * hw + 127) / 128 * 128;
   void* block = nullptr;
-  st = nrs_alloc(ctx, (split ? 2 * each : floats) * sizeof(float), 0, &block);
-  float *hi = (float*)block, *lo = split ? hi + each : nullptr;
+  st = nrs_alloc(ctx, each * sizeof(float), 0, &block);
+  float *hi = (float*)block, *lo = split ? nrs_plane_at(hi, each, true) : nullptr;
   if (st == NRS_OK) st = nrs_tc_stage_image(ctx, t, hi, lo, n, c, (int)hw);
   if (st != NRS_OK) {
     if (block) nrs_free(ctx, block);

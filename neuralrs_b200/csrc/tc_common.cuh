@@ -154,8 +154,10 @@ __device__ __forceinline__ uint32_t cluster_rank() {
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// (Default semantics: what is handed over is tensor memory, ordered by the tcgen05 fences.  `.release.cluster` made the arriving
+// warp wait for all its global stores: 2 to 3 thousand clocks a tile.)
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
 }
 // The wait of a whole warp on a barrier that threads of other CTAs of the cluster arrive on.
 __device__ __forceinline__ bool mbar_wait_warp_cluster(uint64_t* bar, uint32_t parity) {
@@ -235,6 +237,24 @@ __device__ __forceinline__ void umma_tf32(uint32_t tmem_d, uint64_t desc_a, uint
         ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
         : "memory");
 }
+// The same with f16 operands: one UMMA of shape M x N x 16, at twice the rate of the above.
+template <bool PAIR = false>
+__device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+  if constexpr (PAIR)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
 // Arrive on an mbarrier once every UMMA issued so far by this thread has finished.  PAIR: on the barrier at this offset in
 // both CTAs.
 template <bool PAIR = false>
@@ -284,6 +304,11 @@ __host__ __device__ constexpr uint32_t make_idesc_tf32(int m, int n, bool a_mn_m
          ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
+// kind::f16 with f16 operands (formats 0), otherwise the same.
+__host__ __device__ constexpr uint32_t make_idesc_f16(int m, int n, bool a_mn_major, bool b_mn_major) {
+  return (1u << 4) | ((a_mn_major ? 1u : 0u) << 15) | ((b_mn_major ? 1u : 0u) << 16) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
+}
+
 // Shared-memory matrix descriptor, 128-byte swizzle.
 // bits [0,14) start address >> 4; [16,30) leading byte offset >> 4; [32,46) stride byte
 // offset >> 4; [46,48) version (1 on sm_100); [61,64) layout (2 = SWIZZLE_128B).
@@ -305,6 +330,15 @@ __device__ __forceinline__ uint64_t make_smem_desc_sw128(uint32_t smem_addr, uin
 __device__ __forceinline__ uint64_t make_smem_desc_sw128_32b(uint32_t smem_addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
   return (uint64_t)((smem_addr >> 4) & 0x3FFFu) | ((uint64_t)((lbo_bytes >> 4) & 0x3FFFu) << 16) |
          ((uint64_t)((sbo_bytes >> 4) & 0x3FFFu) << 32) | (1ull << 46) | (1ull << 61);
+}
+
+// 64-byte swizzle (layout type 4), the layout of the f16 operands: 32 values (64 B) a row, the 16-byte chunk index bits
+// [4,6) XORed with the row bits [7,9), groups of 8 rows 512 B apart (SBO).
+//  K-major: rows of M or N; 16 elements along K = +32 B on the start.
+//  MN-major: rows of K; a UMMA's 16 are two groups; 32-element blocks along MN sit LBO apart.
+__device__ __forceinline__ uint64_t make_smem_desc_sw64(uint32_t smem_addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
+  return (uint64_t)((smem_addr >> 4) & 0x3FFFu) | ((uint64_t)((lbo_bytes >> 4) & 0x3FFFu) << 16) |
+         ((uint64_t)((sbo_bytes >> 4) & 0x3FFFu) << 32) | (1ull << 46) | (4ull << 61);
 }
 
 // Round-to-nearest TF32 of an f32 (low 13 mantissa bits cleared in the result).
@@ -337,23 +371,24 @@ inline PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
   return fn;
 }
 
-// f32 tensor of `rank` dims (dim[0] innermost, contiguous), strides in BYTES for dims 1..rank-1
-// (multiples of 16), box extents per dim (box[0]*4 must be 128 for the 128-byte swizzle).  `step` (optional):
-// every step[i]-th element is taken along dim i >= 1 (a strided convolution's pixels); box[i] counts the elements
-// that land in shared memory, and box[i] * step[i] may not exceed 256.
-inline bool encode_tmap_f32(CUtensorMap* out, const void* base, int rank, const uint64_t* dim, const uint64_t* stride_bytes,
-                            const uint32_t* box, bool atom32 = false, const uint32_t* step = nullptr) {
+// Operand tensor of `rank` dims (dim[0] innermost, contiguous) of f32 or (half) f16 values, strides in VALUES for dims
+// 1..rank-1 (multiples of 16 bytes), box extents per dim (box[0]: 128 bytes in the 128-byte swizzle, or 32 values of f16
+// in the 64-byte one; atom32: see make_smem_desc_sw128_32b).  `step` (optional): every step[i]-th element
+// is taken along dim i >= 1 (a strided convolution's pixels); box[i] counts the elements that land in shared memory, and
+// box[i] * step[i] may not exceed 256.
+inline bool encode_tmap(CUtensorMap* out, const void* base, bool half, int rank, const uint64_t* dim, const uint64_t* stride,
+                        const uint32_t* box, bool atom32 = false, const uint32_t* step = nullptr) {
   auto enc = tensor_map_encoder();
   if (!enc) return false;
   cuuint64_t gdim[5];
   cuuint64_t gstr[4];
   cuuint32_t bx[5], es[5];
   for (int i = 0; i < rank; ++i) { gdim[i] = dim[i]; es[i] = step ? step[i] : 1; bx[i] = box[i] * es[i]; }
-  for (int i = 0; i + 1 < rank; ++i) gstr[i] = stride_bytes[i];
-  const CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, (cuuint32_t)rank, const_cast<void*>(base), gdim, gstr, bx, es,
-                         CU_TENSOR_MAP_INTERLEAVE_NONE, atom32 ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B,
-                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  for (int i = 0; i + 1 < rank; ++i) gstr[i] = stride[i] * (half ? 2 : 4);
+  const CUresult r = enc(out, half ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, (cuuint32_t)rank, const_cast<void*>(base),
+                         gdim, gstr, bx, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                         half && box[0] == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : atom32 && !half ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B,
+                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS;
 }
 

@@ -41,14 +41,15 @@ struct ConvPolicyOf {
   int out_h, out_w;                   // the tensor written: pixel (u, v) is (u*out_step + out_y0, v*out_step + out_x0)
   int out_step, out_y0, out_x0;
   int n_img, n_ch_out;
-  int cblocks, tap_cols;              // 32-channel blocks per tap; taps per kernel row that take part
+  int cblocks, tap_cols;              // channel blocks (of KW) per tap; taps per kernel row that take part
   int in_step;                        // pixels of the activation per step of (u, v)
   int sgn, base_y, base_x;
   int w_tap0, w_tap_row, w_tap_col;   // weight tap of (0, 0), and its steps along both tap axes
   float* out;
   const float* bias;
   int act, accumulate;
-  uint32_t slice_bytes;
+  uint32_t slice_rows;                // pixels of a tile's box
+  float k_total;                      // terms of a sum, for the result's bound
   // optional: ReLU mask taken from an NCHW tensor of the output's shape, and NHWC TF32 planes of
   // the result for the next tensor-core kernel
   const float* mask_src;
@@ -58,7 +59,14 @@ struct ConvPolicyOf {
   float* colsum_partial;
   bool skip_out;   // the finished values leave as planes and channel sums only (a K-split's second pass writes them still)
 
-  __device__ __forceinline__ uint32_t a_slice_bytes() const { return slice_bytes; }
+  __device__ __forceinline__ uint32_t a_slice_rows() const { return slice_rows; }
+  // No finished value exceeds this (a whole warp asks).
+  __device__ __forceinline__ float out_bound(float top_a, float top_b, int lane) const {
+    uint32_t b = 0;
+    if (bias)
+      for (int n = lane; n < n_ch_out; n += 32) b = pr::seen(b, bias[n]);
+    return pr::product_bound(k_total, top_a, top_b, __uint_as_float(__reduce_max_sync(0xffffffffu, b)));
+  }
   __device__ __forceinline__ void origin(int tile_m, int* x0, int* y0, int* n0) const {
     const int tx = tile_m % tiles_x, t = tile_m / tiles_x;
     *x0 = tx * Wt;
@@ -67,6 +75,7 @@ struct ConvPolicyOf {
   }
   // Position of a K-slice: tap (i, j), channel block cb; the box origin of tap (i, j) and the weight column.
   struct Cursor { int b_col, cb, i, j, x, y, n, x_first; };
+  template <int KW>
   __device__ __forceinline__ Cursor cursor(int tile_m, int, int kb) const {
     Cursor c;
     const int tap = kb / cblocks;
@@ -78,14 +87,16 @@ struct ConvPolicyOf {
     c.x_first = x0 * in_step + base_x;
     c.x = c.x_first + sgn * c.j;
     c.y = y0 * in_step + base_y + sgn * c.i;
-    c.b_col = weight_column(c);
+    c.b_col = weight_column<KW>(c);
     return c;
   }
+  template <int KW>
   __device__ __forceinline__ int weight_column(const Cursor& c) const {
-    return ((w_tap0 + c.i * w_tap_row + c.j * w_tap_col) * cblocks + c.cb) * 32;
+    return ((w_tap0 + c.i * w_tap_row + c.j * w_tap_col) * cblocks + c.cb) * KW;
   }
+  template <int KW>
   __device__ __forceinline__ void advance(Cursor& c) const {
-    c.b_col += 32;
+    c.b_col += KW;
     if (++c.cb < cblocks) return;
     c.cb = 0;
     c.x += sgn;
@@ -95,15 +106,15 @@ struct ConvPolicyOf {
       c.y += sgn;
       ++c.i;
     }
-    c.b_col = weight_column(c);
+    c.b_col = weight_column<KW>(c);
   }
-  template <int BN, bool PAIR>
+  template <int BN, bool PAIR, int KW, int ROW_BYTES>
   __device__ __forceinline__ void load_b(void* dst, const CUtensorMap* tm, uint32_t bar, const Cursor& c, int n0) const {
     tc::tma_load_3d_to<PAIR>(dst, tm, bar, c.b_col, n0, 0);
   }
-  template <bool PAIR>
+  template <bool PAIR, int KW, int ROW_BYTES>
   __device__ __forceinline__ void load_a(void* dst, const CUtensorMap* tm, uint32_t bar, const Cursor& c) const {
-    tc::tma_load_4d_to<PAIR>(dst, tm, bar, c.cb * 32, c.x, c.y, c.n);
+    tc::tma_load_4d_to<PAIR>(dst, tm, bar, c.cb * KW, c.x, c.y, c.n);
   }
   // NCHW offset of channel 0 of the pixel behind accumulator row `row`, and the pixel's linear index.
   __device__ __forceinline__ bool locate(int tile_m, int row, size_t* nchw_off, size_t* pixel) const {
@@ -119,7 +130,8 @@ struct ConvPolicyOf {
     *pixel = ((size_t)n * out_h + y) * out_w + x;
     return true;
   }
-  __device__ __forceinline__ void store(int tile_m, int, int row, int ch, float v) const {
+  template <bool SPLIT>
+  __device__ __forceinline__ void store(int tile_m, int, int row, int ch, float v, float out_scale, uint32_t& top) const {
     size_t off, pixel;
     if (ch >= n_ch_out || !locate(tile_m, row, &off, &pixel)) return;
     off += (size_t)ch * out_h * out_w;
@@ -128,11 +140,10 @@ struct ConvPolicyOf {
     if (accumulate) v += out[off];
     if (mask_src && !(mask_src[off] > 0.0f)) v = 0.0f;
     out[off] = v;
-    if (out_hi) {
-      const float hv = tc::tf32_rn(v);
-      out_hi[pixel * n_ch_out + ch] = hv;
-      if (out_lo) out_lo[pixel * n_ch_out + ch] = v - hv;
-    }
+    if (SPLIT) top = pr::seen(top, v);
+    if (!out_hi) return;
+    if (SPLIT) pr::put(out_hi, out_lo, pixel * n_ch_out + ch, v, out_scale);
+    else out_hi[pixel * n_ch_out + ch] = tc::tf32_rn(v);
   }
   static constexpr bool kCanEmit = true;
   static constexpr bool kAMnMajor = false, kBMnMajor = false;
@@ -208,12 +219,10 @@ struct ConvPolicyOf {
 
 using ConvPolicy = ConvPolicyOf<4>;
 
-// Which launches take two epilogue warps per lane quarter: 64 columns in 3xTF32 with planes to emit, or with bias and
-// activation, whose epilogue (activation or mask, NCHW store, split and staging: 15 thousand clocks a tile) is longer than
-// the main loop of a 64-channel layer (10).  There 53 -> 47 us and 58 -> 51 forward, 62 -> 58 backward on 100 images of
-// 32 x 32.  Elsewhere they lose: plain data gradients (22 -> 26 us for a residue of the 48 -> 80 layer), 128 columns (the
-// second staging tile costs a ring slot: 706 -> 726 us a pass of the 64 -> 128 layer), TF32 (1.5 %).
-constexpr bool may_take_eight_warps(int bn, int nplanes) { return bn == 64 && nplanes == 2; }
+// 3xTF32 launches of 64 columns and more take two epilogue warps per lane quarter: with the products at the f16 rate the
+// epilogue (activation or mask, NCHW store, split and staging) is the longer part of most tiles.  TF32 keeps one (two: 1.5 %
+// slower).
+constexpr bool takes_eight_warps(int bn, int nplanes) { return bn >= 64 && nplanes == 2; }
 
 // One axis of a (sub-)problem: `len` output pixels at positions u*step + first, `taps` kernel taps tap0,
 // tap0 + tap_step, ..., and the activation coordinate of tap t for pixel u: u * in_step + base + sgn * t.
@@ -231,7 +240,8 @@ struct ConvPlan {
   // weights and which re-layout
   const float* w;
   int co, ci, kh, kw, for_dgrad;
-  void *w_hi, *w_lo;   // its planes once staged (the residues of a strided data gradient share them)
+  const float *w_hi, *w_lo;   // its planes once staged (the residues of a strided data gradient share them)
+  const NrsRange* w_range;
   // output NCHW [n_img][n_ch_out][out_h][out_w]
   float* out;
   int n_ch_out, out_h, out_w;
@@ -241,45 +251,45 @@ struct ConvPlan {
   int act, accumulate;
 };
 
-template <int BN, int NPLANES, bool PAIR>
-int run_conv(nrs_ctx* ctx, const ConvPlan& p, const float* a_hi, const float* a_lo, const float* w_hi, const float* w_lo,
-             const ConvPolicy& pol, int tiles_m, int* splits_out) {
+template <int BN, int NPLANES, bool PAIR, int KW>
+int run_conv(nrs_ctx* ctx, const ConvPlan& p, const float* a_hi, const float* a_lo, const ConvPolicy& pol, const tc::Ranges& rg, int tiles_m,
+             int* splits_out) {
+  constexpr bool kHalf = NPLANES == 2;
   const int a_ld = nrs_plane_ld(p.a_ch);
-  const int kdim = p.kh * p.kw * pol.cblocks * 32;
+  const int kdim = p.kh * p.kw * pol.cblocks * KW;
   CUtensorMap ta_hi, ta_lo, tb_hi, tb_lo;
   const uint64_t adim[4] = {(uint64_t)p.a_ch, (uint64_t)p.a_w, (uint64_t)p.a_h, (uint64_t)p.n_img};
-  const uint64_t astr[3] = {(uint64_t)a_ld * 4, (uint64_t)p.a_w * a_ld * 4, (uint64_t)p.a_h * p.a_w * a_ld * 4};
-  const uint32_t abox[4] = {32, (uint32_t)pol.Wt, (uint32_t)pol.Ht, (uint32_t)pol.Nt};
+  const uint64_t astr[3] = {(uint64_t)a_ld, (uint64_t)p.a_w * a_ld, (uint64_t)p.a_h * p.a_w * a_ld};
+  const uint32_t abox[4] = {(uint32_t)KW, (uint32_t)pol.Wt, (uint32_t)pol.Ht, (uint32_t)pol.Nt};
   const uint32_t astep[4] = {1, (uint32_t)pol.in_step, (uint32_t)pol.in_step, 1};
   const uint64_t bdim[3] = {(uint64_t)kdim, (uint64_t)p.n_ch_out, 1};
-  const uint64_t bstr[2] = {(uint64_t)kdim * 4, (uint64_t)kdim * p.n_ch_out * 4};
-  const uint32_t bbox[3] = {32, (uint32_t)(PAIR ? BN / 2 : BN), 1};
-  bool ok = tc::encode_tmap_f32(&ta_hi, a_hi, 4, adim, astr, abox, false, astep) && tc::encode_tmap_f32(&tb_hi, w_hi, 3, bdim, bstr, bbox);
-  if (NPLANES == 2)
-    ok = ok && tc::encode_tmap_f32(&ta_lo, a_lo, 4, adim, astr, abox, false, astep) && tc::encode_tmap_f32(&tb_lo, w_lo, 3, bdim, bstr, bbox);
+  const uint64_t bstr[2] = {(uint64_t)kdim, (uint64_t)kdim * p.n_ch_out};
+  const uint32_t bbox[3] = {(uint32_t)KW, (uint32_t)(PAIR ? BN / 2 : BN), 1};
+  bool ok = tc::encode_tmap(&ta_hi, a_hi, kHalf, 4, adim, astr, abox, false, astep) && tc::encode_tmap(&tb_hi, p.w_hi, kHalf, 3, bdim, bstr, bbox);
+  if (kHalf) ok = ok && tc::encode_tmap(&ta_lo, a_lo, true, 4, adim, astr, abox, false, astep) && tc::encode_tmap(&tb_lo, p.w_lo, true, 3, bdim, bstr, bbox);
   else { ta_lo = ta_hi; tb_lo = tb_hi; }
   // Output planes (optional): the same box geometry as an activation load, in output space.
   CUtensorMap to_hi, to_lo;
   if (pol.out_hi) {
     const uint64_t odim[4] = {(uint64_t)p.n_ch_out, (uint64_t)p.out_w, (uint64_t)p.out_h, (uint64_t)p.n_img};
-    const uint64_t ostr[3] = {(uint64_t)p.n_ch_out * 4, (uint64_t)p.out_w * p.n_ch_out * 4, (uint64_t)p.out_h * p.out_w * p.n_ch_out * 4};
-    ok = ok && tc::encode_tmap_f32(&to_hi, pol.out_hi, 4, odim, ostr, abox);
-    if (pol.out_lo) ok = ok && tc::encode_tmap_f32(&to_lo, pol.out_lo, 4, odim, ostr, abox);
+    const uint32_t obox[4] = {32, abox[1], abox[2], abox[3]};
+    const uint64_t ostr[3] = {(uint64_t)p.n_ch_out, (uint64_t)p.out_w * p.n_ch_out, (uint64_t)p.out_h * p.out_w * p.n_ch_out};
+    ok = ok && tc::encode_tmap(&to_hi, pol.out_hi, kHalf, 4, odim, ostr, obox);
+    if (pol.out_lo) ok = ok && tc::encode_tmap(&to_lo, pol.out_lo, kHalf, 4, odim, ostr, obox);
   }
   NRS_REQUIRE(ctx, ok, NRS_ERR_CUDA, "tc_conv: cuTensorMapEncodeTiled failed");
-  if constexpr (may_take_eight_warps(BN, NPLANES)) {
-    if (pol.out_hi || (p.bias && p.act != NRS_ACT_NONE)) {
-      ConvPolicyOf<8> wide;
-      static_assert(sizeof(wide) == sizeof(pol), "the same fields");
-      std::memcpy(&wide, &pol, sizeof(wide));
-      return tc::launch<BN, NPLANES, PAIR, ConvPolicyOf<8>>(ctx, ta_hi, ta_lo, tb_hi, tb_lo, wide, tiles_m, p.n_ch_out, 1,
-                                                            p.ay.taps * p.ax.taps * pol.cblocks, pol.out_hi ? &to_hi : nullptr,
+  if constexpr (takes_eight_warps(BN, NPLANES)) {
+    ConvPolicyOf<8> wide;
+    static_assert(sizeof(wide) == sizeof(pol), "the same fields");
+    std::memcpy(&wide, &pol, sizeof(wide));
+    return tc::launch<BN, NPLANES, PAIR, KW, ConvPolicyOf<8>>(ctx, ta_hi, ta_lo, tb_hi, tb_lo, wide, tiles_m, p.n_ch_out, 1,
+                                                            p.ay.taps * p.ax.taps * pol.cblocks, rg, pol.out_hi ? &to_hi : nullptr,
                                                             pol.out_lo ? &to_lo : nullptr, splits_out);
-    }
+  } else {
+    return tc::launch<BN, NPLANES, PAIR, KW, ConvPolicy>(ctx, ta_hi, ta_lo, tb_hi, tb_lo, pol, tiles_m, p.n_ch_out, 1,
+                                                         p.ay.taps * p.ax.taps * pol.cblocks, rg, pol.out_hi ? &to_hi : nullptr,
+                                                         pol.out_lo ? &to_lo : nullptr, splits_out);
   }
-  return tc::launch<BN, NPLANES, PAIR, ConvPolicy>(ctx, ta_hi, ta_lo, tb_hi, tb_lo, pol, tiles_m, p.n_ch_out, 1,
-                                             p.ay.taps * p.ax.taps * pol.cblocks, pol.out_hi ? &to_hi : nullptr,
-                                             pol.out_lo ? &to_lo : nullptr, splits_out);
 }
 
 // Pixel tile: the Wt x Ht x Nt box of at most 128 pixels (a box side times the activation step may not exceed
@@ -317,23 +327,32 @@ int conv_common(nrs_ctx* ctx, ConvPlan& p) {
   pol.sub_h = p.ay.len; pol.sub_w = p.ax.len;
   pol.out_h = p.out_h; pol.out_w = p.out_w; pol.n_img = p.n_img; pol.n_ch_out = p.n_ch_out;
   pol.out_step = p.ay.step; pol.out_y0 = p.ay.first; pol.out_x0 = p.ax.first;
-  pol.cblocks = (p.a_ch + 31) / 32; pol.tap_cols = p.ax.taps;
+  const int blocks32 = (p.a_ch + 31) / 32;
+  const bool wide = split && blocks32 % 2 == 0;   // K-slices of 64 channels: TMA brings rows of 64 bytes at half the rate
+  pol.cblocks = wide ? blocks32 / 2 : blocks32; pol.tap_cols = p.ax.taps;
   pol.in_step = p.ay.in_step;
   pol.sgn = p.sgn; pol.base_y = p.ay.base; pol.base_x = p.ax.base;
   pol.w_tap0 = p.ay.tap0 * p.kw + p.ax.tap0; pol.w_tap_row = p.ay.tap_step * p.kw; pol.w_tap_col = p.ax.tap_step;
   pol.out = p.out; pol.bias = p.bias; pol.act = p.act; pol.accumulate = p.accumulate;
-  pol.slice_bytes = (uint32_t)(pol.Wt * pol.Ht * pol.Nt) * 128u;
+  pol.slice_rows = (uint32_t)(pol.Wt * pol.Ht * pol.Nt);
+  pol.k_total = (float)p.a_ch * p.ay.taps * p.ax.taps;
   // Requests of the caller are honoured where this launch writes every pixel of the output (planes: whole
   // 32-channel blocks); the caller finds the others still registered and does the work itself.
   const bool whole = pol.out_step == 1 && p.n_ch_out % 32 == 0;
+  NrsRange* out_range = nullptr;
   auto extras = whole ? ctx->out_extras.find(p.out) : ctx->out_extras.end();
   if (extras != ctx->out_extras.end()) {
     const NrsOutExtras& e = extras->second;
     if ((e.relu_mask_src && p.accumulate) ||   // the mask would hit the old content too
-        (e.lo && !split)) {
+        ((e.hi || e.measure) && split && p.accumulate) ||   // no bound of the old content
+        (e.hi && (e.lo != nullptr) != split)) {
       extras = ctx->out_extras.end();
     } else {
       pol.mask_src = e.relu_mask_src; pol.out_hi = e.hi; pol.out_lo = e.lo;
+      if (split && (e.hi || e.measure)) {
+        const int got = nrs_range_renew(ctx, e.hi ? (const void*)e.hi : (const void*)p.out, &out_range);
+        if (got != NRS_OK) return got;
+      }
     }
   }
   auto colsum = ctx->colsum_requests.find(p.out);
@@ -350,7 +369,7 @@ int conv_common(nrs_ctx* ctx, ConvPlan& p) {
     a_lo = ready->lo;
   } else {
     const size_t a_plane = (size_t)p.n_img * p.a_h * p.a_w * nrs_plane_ld(p.a_ch);
-    st = nrs_ws_planes(ctx, NRS_WS_A, a_plane * sizeof(float), split, &a_hi, &a_lo);
+    st = nrs_ws_planes(ctx, NRS_WS_A, a_plane, split, &a_hi, &a_lo);
     if (st == NRS_OK) st = nrs_tc_stage_image(ctx, p.act_src, (float*)a_hi, (float*)a_lo, p.n_img, p.a_ch, p.a_h * p.a_w);
     if (st != NRS_OK) return st;
   }
@@ -359,23 +378,27 @@ int conv_common(nrs_ctx* ctx, ConvPlan& p) {
   } else if (wp && wp->co == p.co && wp->ci == p.ci && wp->taps == p.kh * p.kw) {   // staged ahead with the rest of the model's weights
     p.w_hi = wp->hi;
     p.w_lo = wp->lo;
+    p.w_range = wp->range;
   } else {
     void *w_hi = nullptr, *w_lo = nullptr;
-    const size_t w_plane = (size_t)p.n_ch_out * p.kh * p.kw * pol.cblocks * 32;
-    st = nrs_ws_planes(ctx, NRS_WS_B, w_plane * sizeof(float), split, &w_hi, &w_lo);
+    const size_t w_plane = (size_t)p.n_ch_out * p.kh * p.kw * blocks32 * 32;
+    st = nrs_ws_planes(ctx, NRS_WS_B, w_plane, split, &w_hi, &w_lo);
     if (st != NRS_OK) return st;
     st = nrs_tc_stage_conv_weight(ctx, p.w, (float*)w_hi, (float*)w_lo, p.co, p.ci, p.kh, p.kw, p.for_dgrad);
     if (st != NRS_OK) return st;
-    p.w_hi = w_hi;
-    p.w_lo = w_lo;
+    p.w_hi = (const float*)w_hi;
+    p.w_lo = (const float*)w_lo;
+    p.w_range = nrs_range_of(ctx, w_hi);
   }
+  const tc::Ranges rg{nrs_range_of(ctx, a_hi), p.w_range, out_range};
 
   if (extras != ctx->out_extras.end()) ctx->out_extras.erase(extras);   // honoured from here on
   int splits = 0;
-  const tc::TilePlan tile = tc::plan_tile(ctx, tiles_m, p.n_ch_out, 1, p.ay.taps * p.ax.taps * pol.cblocks, split, 0.025, true);
+  const tc::TilePlan tile = tc::plan_tile(ctx, tiles_m, p.n_ch_out, 1, p.ay.taps * p.ax.taps * blocks32, split, 0.025, true);
 #define NRS_RUN(BN_, PAIR_)                                                                                              \
-  st = split ? run_conv<BN_, 2, PAIR_>(ctx, p, (const float*)a_hi, (const float*)a_lo, (const float*)p.w_hi, (const float*)p.w_lo, pol, (int)tiles_m, &splits) \
-             : run_conv<BN_, 1, PAIR_>(ctx, p, (const float*)a_hi, nullptr, (const float*)p.w_hi, nullptr, pol, (int)tiles_m, &splits)
+  st = !split ? run_conv<BN_, 1, PAIR_, 32>(ctx, p, (const float*)a_hi, nullptr, pol, rg, (int)tiles_m, &splits)                \
+       : wide ? run_conv<BN_, 2, PAIR_, 64>(ctx, p, (const float*)a_hi, (const float*)a_lo, pol, rg, (int)tiles_m, &splits)      \
+              : run_conv<BN_, 2, PAIR_, 32>(ctx, p, (const float*)a_hi, (const float*)a_lo, pol, rg, (int)tiles_m, &splits)
   if (tile.pair) { if (tile.bn == 128) NRS_RUN(128, true); else NRS_RUN(64, true); }
   else if (tile.bn == 128) NRS_RUN(128, false);
   else if (tile.bn == 64) NRS_RUN(64, false);
@@ -432,7 +455,7 @@ int nrs_tc_conv_dgrad(nrs_ctx* ctx, const float* w, const float* dy, float* dx, 
   if (stride > 1 && !nrs_planes_find(ctx, dy, split)) {
     void *hi = nullptr, *lo = nullptr;
     const size_t plane = (size_t)n * p.a_h * p.a_w * nrs_plane_ld(co);
-    int st = nrs_ws_planes(ctx, NRS_WS_A, plane * sizeof(float), split, &hi, &lo);
+    int st = nrs_ws_planes(ctx, NRS_WS_A, plane, split, &hi, &lo);
     if (st == NRS_OK) st = nrs_tc_stage_image(ctx, dy, (float*)hi, (float*)lo, n, co, p.a_h * p.a_w);
     if (st != NRS_OK) return st;
     ctx->plane_hints[dy] = NrsPlanes{(float*)hi, (float*)lo, split ? 1 : 0};

@@ -28,6 +28,7 @@ struct GemmPolicy {
   size_t batch_stride;
   bool vec_ok;                 // rows of every output and epilogue input start on 16 bytes
   NrsGemmExtras x;
+  float k_total;               // length of the reduction, for the result's bound
   // Several B matrices side by side ([Wq|Wk|Wv]): columns n0 of matrix n0 / seg_n, or reduction indices k of matrix
   // k / seg_k; 0 = one matrix.  The matrices are the batches of B's tensor map.
   int seg_n, seg_k;
@@ -40,26 +41,37 @@ struct GemmPolicy {
   static constexpr int kEpiWarps = 16;
   int order() const { return tc::kRaster; }
 
-  __device__ __forceinline__ uint32_t a_slice_bytes() const { return tc::BM * tc::BK * 4; }
+  __device__ __forceinline__ uint32_t a_slice_rows() const { return tc::BM; }   // of A, that a load brings
   struct Cursor { int b_col, row, batch; };
-  __device__ __forceinline__ Cursor cursor(int tile_m, int batch, int kb) const { return Cursor{kb * tc::BK, tile_m * tc::BM, batch}; }
-  __device__ __forceinline__ void advance(Cursor& c) const { c.b_col += tc::BK; }
-  template <bool PAIR>
+  template <int KW>
+  __device__ __forceinline__ Cursor cursor(int tile_m, int batch, int kb) const { return Cursor{kb * KW, tile_m * tc::BM, batch}; }
+  template <int KW>
+  __device__ __forceinline__ void advance(Cursor& c) const { c.b_col += KW; }
+  template <bool PAIR, int KW, int ROW_BYTES>
   __device__ __forceinline__ void load_a(void* dst, const CUtensorMap* tm, uint32_t bar, const Cursor& c) const {
-    if (MN) tc::tma_load_3d_to<PAIR>(dst, tm, bar, 0, c.b_col, c.row / 32);
+    if (MN) tc::tma_load_3d_to<PAIR>(dst, tm, bar, 0, c.b_col, c.row / KW);
     else tc::tma_load_3d_to<PAIR>(dst, tm, bar, c.b_col, c.row, c.batch);
   }
-  template <int BN, bool PAIR>
+  template <int BN, bool PAIR, int KW, int ROW_BYTES>
   __device__ __forceinline__ void load_b(void* dst, const CUtensorMap* tm, uint32_t bar, const Cursor& c, int n0) const {
-    if (MN) { tc::tma_load_3d_to<PAIR>(dst, tm, bar, 0, c.b_col, n0 / 32); return; }
+    if (MN) { tc::tma_load_3d_to<PAIR>(dst, tm, bar, 0, c.b_col, n0 / KW); return; }
     int b0 = c.b_col, b1 = n0, b2 = c.batch;
     if (seg_n) { b2 = n0 / seg_n; b1 = n0 - b2 * seg_n; }
     if (seg_k) { b2 = c.b_col / seg_k; b0 = c.b_col - b2 * seg_k; }
     tc::tma_load_3d_to<PAIR>(dst, tm, bar, b0, b1, b2);
   }
   __device__ __forceinline__ float dact(float src) const { return x.dact == NRS_ACT_RELU ? (src > 0.0f ? 1.0f : 0.0f) : nrs_gelu_d(src); }
+  // No finished value exceeds this (a whole warp asks).
+  __device__ __forceinline__ float out_bound(float top_a, float top_b, int lane) const {
+    uint32_t b = 0;
+    if (bias)
+      for (int n = lane; n < N; n += 32) b = pr::seen(b, bias[n]);
+    const float bound = pr::product_bound(k_total, top_a, top_b, __uint_as_float(__reduce_max_sync(0xffffffffu, b)));
+    return x.dact == NRS_ACT_GELU ? fminf(1.25f * bound, 3.0e38f) : bound;   // (GELU's derivative stays below 1.13, the activations within |v|)
+  }
   // One element, from the pass that sums a K-split.
-  __device__ __forceinline__ void store(int tile_m, int batch, int row, int n, float v) const {
+  template <bool SPLIT>
+  __device__ __forceinline__ void store(int tile_m, int batch, int row, int n, float v, float out_scale, uint32_t& top) const {
     const int m = tile_m * tc::BM + row;
     if (m >= M || n >= N) return;
     const size_t at = (size_t)batch * batch_stride + (size_t)m * N + n;
@@ -68,15 +80,20 @@ struct GemmPolicy {
     v = nrs_apply_act(v, act);
     if (beta != 0.0f) v += beta * C[at];
     if (!x.skip_c) C[at] = v;
+    if (SPLIT && !x.hi) top = pr::seen(top, v);
     if (!x.hi) return;
     if (x.dact != NRS_ACT_NONE) v *= dact(x.dact_src[at]);
-    const float h = tc::tf32_rn(v);
-    x.hi[at] = h;
-    if (x.lo) x.lo[at] = v - h;
+    if (SPLIT) {
+      top = pr::seen(top, v);
+      pr::put(x.hi, x.lo, at, v, out_scale);
+    } else {
+      x.hi[at] = tc::tf32_rn(v);
+    }
   }
   __device__ __forceinline__ int row(int, int, int) const { return 0; }
   // Four row segments of a warp's 32 x 16 block: row r0 + 8*i of the tile, columns n..n+3 (see tc::rows_to_lines).
-  __device__ __forceinline__ void epilogue(int tile_m, int batch, int r0, int n, float4 (&v)[4]) const {
+  template <bool SPLIT>
+  __device__ __forceinline__ void epilogue(int tile_m, int batch, int r0, int n, float4 (&v)[4], float out_scale, uint32_t& top) const {
     const int m0 = tile_m * tc::BM + r0, nn = N - n;   // nn: how many of the four columns exist (four or more: all)
     const size_t at0 = (size_t)batch * batch_stride + (size_t)m0 * N + n, step = (size_t)8 * N;
     if (bias) {
@@ -117,13 +134,21 @@ struct GemmPolicy {
 #pragma unroll
       for (int i = 0; i < 4; ++i) { v[i].x *= dact(s[i].x); v[i].y *= dact(s[i].y); v[i].z *= dact(s[i].z); v[i].w *= dact(s[i].w); }
     }
+    if (SPLIT && x.range) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (m0 + 8 * i < M) top = pr::seen4(top, v[i]);
+    }
     if (x.hi) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         if (m0 + 8 * i >= M) continue;
-        const float4 h = make_float4(tc::tf32_rn(v[i].x), tc::tf32_rn(v[i].y), tc::tf32_rn(v[i].z), tc::tf32_rn(v[i].w));
-        tc::store_guarded(x.hi + at0 + i * step, h, nn, vec_ok);
-        if (x.lo) tc::store_guarded(x.lo + at0 + i * step, make_float4(v[i].x - h.x, v[i].y - h.y, v[i].z - h.z, v[i].w - h.w), nn, vec_ok);
+        if (SPLIT) {   // (n is a multiple of 8, so all four columns exist or none)
+          if (nn >= 4) pr::put4(x.hi, x.lo, at0 + i * step, v[i], out_scale);
+        } else {
+          const float4 h = make_float4(tc::tf32_rn(v[i].x), tc::tf32_rn(v[i].y), tc::tf32_rn(v[i].z), tc::tf32_rn(v[i].w));
+          tc::store_guarded(x.hi + at0 + i * step, h, nn, vec_ok);
+        }
       }
     }
     if (x.colsum) {   // sum over the warp's 32 rows, in a fixed order; lanes 0..3 write four columns each
@@ -146,7 +171,8 @@ struct Operand {
   const float* lo;
   int ld;          // leading dimension in floats
   int kdim;        // K extent given to the tensor map (TMA zero-fills beyond it)
-  size_t bstride;  // floats between batches
+  size_t bstride;  // values between batches
+  const NrsRange* range;   // 3xTF32
 };
 
 // Brings one operand into K-major planes.  stored_kmajor: memory is [rows][K]; else [K][rows].  in_place: plain TF32
@@ -160,7 +186,7 @@ int prepare_operand(nrs_ctx* ctx, const float* src, int rows, int K, int batch, 
       const NrsWeightPlanes* wp = nrs_weight_planes_find(ctx, src, stored_kmajor ? NRS_WF_LINEAR_ROWS : NRS_WF_LINEAR_T);
       if (wp && wp->rows == rows && wp->K == K) {
         const int ldw = (K + 31) / 32 * 32;
-        *out = Operand{wp->hi, wp->lo, ldw, ldw, (size_t)rows * ldw};
+        *out = Operand{wp->hi, wp->lo, ldw, ldw, (size_t)rows * ldw, wp->range};
         return NRS_OK;
       }
     }
@@ -168,53 +194,53 @@ int prepare_operand(nrs_ctx* ctx, const float* src, int rows, int K, int batch, 
     if (stored_kmajor) {
       const NrsPlanes* ready = nrs_planes_find(ctx, src, split);
       if (ready && ready->rows == rows && ready->cols == K) {
-        *out = Operand{ready->hi, ready->lo, ldk, K, (size_t)rows * ldk};
+        *out = Operand{ready->hi, ready->lo, ldk, K, (size_t)rows * ldk, nrs_range_of(ctx, ready->hi)};
         return NRS_OK;
       }
     }
   }
   const bool direct = in_place && !split && stored_kmajor && (K % 4 == 0) && ((reinterpret_cast<uintptr_t>(src) & 15) == 0);
   if (direct) {
-    *out = Operand{src, nullptr, K, K, (size_t)rows * K};
+    *out = Operand{src, nullptr, K, K, (size_t)rows * K, nullptr};
     return NRS_OK;
   }
   const size_t plane = (size_t)rows * ldk;
   void *phi = nullptr, *plo = nullptr;
-  int st = nrs_ws_planes(ctx, ws, plane * batch * sizeof(float), split, &phi, &plo);
+  int st = nrs_ws_planes(ctx, ws, plane * batch, split, &phi, &plo);
   if (st != NRS_OK) return st;
   st = nrs_tc_stage(ctx, src, (float*)phi, (float*)plo, rows, K, ldk, batch, (size_t)rows * K, plane, !stored_kmajor);
   if (st != NRS_OK) return st;
-  *out = Operand{(const float*)phi, (const float*)plo, ldk, K, plane};
+  *out = Operand{(const float*)phi, (const float*)plo, ldk, K, plane, nrs_range_of(ctx, phi)};
   return NRS_OK;
 }
 
-bool make_operand_map(CUtensorMap* tm, const float* base, const Operand& op, int rows, int batch, int box_rows) {
+bool make_operand_map(CUtensorMap* tm, const float* base, const Operand& op, int rows, int batch, int box_rows, int kw) {
   const uint64_t dim[3] = {(uint64_t)op.kdim, (uint64_t)rows, (uint64_t)batch};
-  const uint64_t str[2] = {(uint64_t)op.ld * 4, (uint64_t)op.bstride * 4};
-  const uint32_t box[3] = {(uint32_t)tc::BK, (uint32_t)box_rows, 1};
-  return tc::encode_tmap_f32(tm, base, 3, dim, str, box);
+  const uint64_t str[2] = {(uint64_t)op.ld, (uint64_t)op.bstride};
+  const uint32_t box[3] = {(uint32_t)kw, (uint32_t)box_rows, 1};
+  return tc::encode_tmap(tm, base, op.lo != nullptr, 3, dim, str, box);
 }
-// An operand stored [k][rows]: [row block][k][32 rows], one box = a K-slice of box_rows / 32 blocks.
-bool make_mn_operand_map(CUtensorMap* tm, const float* base, const Operand& op, int rows, int k, int box_rows) {
-  const uint64_t dim[3] = {32, (uint64_t)k, (uint64_t)(rows / 32)};
-  const uint64_t str[2] = {(uint64_t)op.ld * 4, 128};
-  const uint32_t box[3] = {32, (uint32_t)tc::BK, (uint32_t)(box_rows / 32)};
-  return tc::encode_tmap_f32(tm, base, 3, dim, str, box, true);
+// An operand stored [k][rows]: [row block][k][kw rows], one box = a K-slice of box_rows / kw blocks.
+bool make_mn_operand_map(CUtensorMap* tm, const float* base, const Operand& op, int rows, int k, int box_rows, int kw) {
+  const uint64_t dim[3] = {(uint64_t)kw, (uint64_t)k, (uint64_t)(rows / kw)};
+  const uint64_t str[2] = {(uint64_t)op.ld, (uint64_t)kw};
+  const uint32_t box[3] = {(uint32_t)kw, (uint32_t)kw, (uint32_t)(box_rows / kw)};
+  return tc::encode_tmap(tm, base, op.lo != nullptr, 3, dim, str, box, true);
 }
 
-template <int BN, int NPLANES, bool PAIR, bool MN>
+template <int BN, int NPLANES, bool PAIR, bool MN, int KW>
 int run(nrs_ctx* ctx, const Operand& A, const Operand& B, int batch, int b_rows, int b_batch, int m, int n, int k,
         const GemmPolicy<MN>& pol, int* splits) {
   constexpr int kBRows = PAIR ? BN / 2 : BN;   // rows of B that one CTA brings
   CUtensorMap ta_hi, ta_lo, tb_hi, tb_lo;
-  auto map_a = [&](CUtensorMap* t, const float* p) { return MN ? make_mn_operand_map(t, p, A, m, k, tc::BM) : make_operand_map(t, p, A, m, batch, tc::BM); };
-  auto map_b = [&](CUtensorMap* t, const float* p) { return MN ? make_mn_operand_map(t, p, B, n, k, kBRows) : make_operand_map(t, p, B, b_rows, b_batch, kBRows); };
+  auto map_a = [&](CUtensorMap* t, const float* p) { return MN ? make_mn_operand_map(t, p, A, m, k, tc::BM, KW) : make_operand_map(t, p, A, m, batch, tc::BM, KW); };
+  auto map_b = [&](CUtensorMap* t, const float* p) { return MN ? make_mn_operand_map(t, p, B, n, k, kBRows, KW) : make_operand_map(t, p, B, b_rows, b_batch, kBRows, KW); };
   bool ok = map_a(&ta_hi, A.hi) && map_b(&tb_hi, B.hi);
   if (NPLANES == 2) ok = ok && map_a(&ta_lo, A.lo) && map_b(&tb_lo, B.lo);
   else { ta_lo = ta_hi; tb_lo = tb_hi; }
   NRS_REQUIRE(ctx, ok, NRS_ERR_CUDA, "tc_gemm: cuTensorMapEncodeTiled failed (m=%d n=%d k=%d)", m, n, k);
-  return tc::launch<BN, NPLANES, PAIR, GemmPolicy<MN>>(ctx, ta_hi, ta_lo, tb_hi, tb_lo, pol, (m + tc::BM - 1) / tc::BM, n, batch,
-                                                 (k + tc::BK - 1) / tc::BK, nullptr, nullptr, splits);
+  return tc::launch<BN, NPLANES, PAIR, KW, GemmPolicy<MN>>(ctx, ta_hi, ta_lo, tb_hi, tb_lo, pol, (m + tc::BM - 1) / tc::BM, n, batch,
+                                                 (k + KW - 1) / KW, tc::Ranges{A.range, B.range, pol.x.range}, nullptr, nullptr, splits);
 }
 
 // `limit`: widest tile allowed (segmented B: the segment must be whole tiles).
@@ -226,15 +252,27 @@ template <bool MN>
 int dispatch(nrs_ctx* ctx, tc::TilePlan tile, bool split, const Operand& A, const Operand& B, int batch, int b_rows, int b_batch, int m, int n,
              int k, GemmPolicy<MN>& pol, NrsGemmExtras* extras) {
   auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+  pol.k_total = (float)k;
   pol.vec_ok = n % 4 == 0 && ((size_t)m * n) % 4 == 0 && aligned(pol.C) && aligned(pol.bias);
   if (extras) {
     pol.x = *extras;
     pol.vec_ok = pol.vec_ok && aligned(extras->pre) && aligned(extras->dact_src);
+    pol.x.range = nullptr;
+    if (split && (extras->hi || extras->measure)) {
+      NRS_REQUIRE(ctx, !extras->hi || pol.beta == 0.0f, NRS_ERR_ARG, "tc_gemm: no planes of an accumulated result");
+      const int st = nrs_range_renew(ctx, extras->hi ? extras->hi : pol.C, &extras->range);
+      if (st != NRS_OK) return st;
+      pol.x.range = extras->range;
+    }
     if (extras->colsum && (m + tc::BM - 1) / tc::BM * 4 > extras->colsum_cap) pol.x.colsum = nullptr;
   }
   int st, splits = 1;
-#define NRS_RUN_GEMM(BN_, PAIR_) (split ? run<BN_, 2, PAIR_, MN>(ctx, A, B, batch, b_rows, b_batch, m, n, k, pol, &splits) \
-                                        : run<BN_, 1, PAIR_, MN>(ctx, A, B, batch, b_rows, b_batch, m, n, k, pol, &splits))
+  // f16 pairs: K-slices of 64, whose rows are 128 bytes, wherever they fit: TMA brings rows of 64 bytes at half the rate.
+  // (MN-major blocks of 64 columns have to be whole, in a CTA's share of B too; a K-slice belongs to one matrix of B.)
+  const bool wide = split && (MN ? m % 64 == 0 && n % 64 == 0 && tile.bn >= (tile.pair ? 128 : 64) : (k % 64 == 0 || k >= 256) && pol.seg_k % 64 == 0);
+#define NRS_RUN_GEMM(BN_, PAIR_) (!split ? run<BN_, 1, PAIR_, MN, 32>(ctx, A, B, batch, b_rows, b_batch, m, n, k, pol, &splits)       \
+                                  : wide ? run<BN_, 2, PAIR_, MN, MN && BN_ < (PAIR_ ? 128 : 64) ? 32 : 64>(ctx, A, B, batch, b_rows, b_batch, m, n, k, pol, &splits) \
+                                         : run<BN_, 2, PAIR_, MN, 32>(ctx, A, B, batch, b_rows, b_batch, m, n, k, pol, &splits))
   if (tile.pair) st = tile.bn == 128 ? NRS_RUN_GEMM(128, true) : NRS_RUN_GEMM(64, true);
   else if (tile.bn == 128) st = NRS_RUN_GEMM(128, false);
   else if (tile.bn == 64) st = NRS_RUN_GEMM(64, false);
@@ -354,7 +392,7 @@ int nrs_tc_gemm(nrs_ctx* ctx, int trans_a, int trans_b, int batch, int m, int n,
     st = prepare_operand(ctx, a, k, m, 1, true, split, NRS_WS_A, &A, false, false);
     if (st == NRS_OK) st = prepare_operand(ctx, b, k, n, 1, true, split, NRS_WS_B, &B, false, false);
     if (st != NRS_OK) return st;
-    GemmPolicy<true> pol{c, bias, act, beta, m, n, (size_t)m * n, false, {}, 0, 0};
+    GemmPolicy<true> pol{c, bias, act, beta, m, n, (size_t)m * n, false, {}, 0.0f, 0, 0};
     return dispatch<true>(ctx, tile_of(ctx, m, n, 1, k, split), split, A, B, 1, n, 1, m, n, k, pol, extras);
   }
   st = prepare_operand(ctx, a, m, k, batch, /*stored_kmajor=*/!trans_a, split, NRS_WS_A, &A, false);
@@ -362,8 +400,8 @@ int nrs_tc_gemm(nrs_ctx* ctx, int trans_a, int trans_b, int batch, int m, int n,
   st = prepare_operand(ctx, b, n, k, batch, /*stored_kmajor=*/trans_b != 0, split, NRS_WS_B, &B, true);
   if (st != NRS_OK) return st;
   // Batched operands read in place need 16-byte aligned batch strides.
-  if (batch > 1 && ((A.bstride % 4) || (B.bstride % 4))) return NRS_ERR_UNSUPPORTED;
-  GemmPolicy<false> pol{c, bias, act, beta, m, n, (size_t)m * n, false, {}, 0, 0};
+  if (batch > 1 && ((A.bstride % (split ? 8 : 4)) || (B.bstride % (split ? 8 : 4)))) return NRS_ERR_UNSUPPORTED;
+  GemmPolicy<false> pol{c, bias, act, beta, m, n, (size_t)m * n, false, {}, 0.0f, 0, 0};
   return dispatch<false>(ctx, tile_of(ctx, m, n, batch, k, split), split, A, B, batch, n, batch, m, n, k, pol, extras);
 }
 
@@ -386,22 +424,27 @@ int nrs_tc_gemm_weights(nrs_ctx* ctx, int reduce, int count, int m, int n, int k
     const NrsWeightPlanes* wp = nrs_weight_planes_find(ctx, w[i], form);
     found = wp && wp->rows == n && wp->K == k;
     if (!found) break;
-    if (i == 0) { B.hi = wp->hi; B.lo = wp->lo; B.ld = (k + 31) / 32 * 32; B.kdim = B.ld; }
-    else if (i == 1) { found = wp->hi > B.hi; B.bstride = (size_t)(wp->hi - B.hi); }
-    found = found && wp->hi == B.hi + (size_t)i * B.bstride && (!split || wp->lo == B.lo + (size_t)i * B.bstride);
+    if (i == 0) { B.hi = wp->hi; B.lo = wp->lo; B.ld = (k + 31) / 32 * 32; B.kdim = B.ld; B.range = wp->range; }
+    else if (i == 1) { found = wp->hi > B.hi; B.bstride = (size_t)((const uint8_t*)wp->hi - (const uint8_t*)B.hi) / (split ? 2 : 4); }
+    found = found && wp->hi == nrs_plane_at(B.hi, i * B.bstride, split) && wp->range == B.range &&
+            (!split || wp->lo == nrs_plane_at(B.lo, i * B.bstride, true));
   }
   if (!found) {
     const int ld = nrs_plane_ld(k);
     const size_t plane = (size_t)n * ld;
     void *hi = nullptr, *lo = nullptr;
-    st = nrs_ws_planes(ctx, NRS_WS_B, plane * count * sizeof(float), split, &hi, &lo);
+    NrsRange* range = nullptr;
+    st = nrs_ws_planes(ctx, NRS_WS_B, plane * count, split, &hi, &lo);
+    if (split && st == NRS_OK) st = nrs_range_renew(ctx, hi, &range);   // one for all of them
+    for (int i = 0; split && i < count && st == NRS_OK; ++i) st = nrs_absmax(ctx, w[i], (size_t)n * k, range);
     for (int i = 0; i < count && st == NRS_OK; ++i)
-      st = nrs_tc_stage(ctx, w[i], (float*)hi + i * plane, split ? (float*)lo + i * plane : nullptr, n, k, ld, 1, 0, 0, !reduce);
+      st = nrs_tc_stage(ctx, w[i], nrs_plane_at((float*)hi, i * plane, split), split ? nrs_plane_at((float*)lo, i * plane, true) : nullptr, n, k, ld, 1,
+                        0, 0, !reduce, range);
     if (st != NRS_OK) return st;
-    B = Operand{(const float*)hi, (const float*)lo, ld, k, plane};
+    B = Operand{(const float*)hi, (const float*)lo, ld, k, plane, range};
   }
   const int cols = reduce ? n : count * n, kk = reduce ? count * k : k;
-  GemmPolicy<false> pol{c, nullptr, NRS_ACT_NONE, beta, m, cols, (size_t)m * cols, false, {}, reduce ? 0 : n, reduce ? k : 0};
+  GemmPolicy<false> pol{c, nullptr, NRS_ACT_NONE, beta, m, cols, (size_t)m * cols, false, {}, 0.0f, reduce ? 0 : n, reduce ? k : 0};
   const int limit = reduce ? 128 : n % 128 == 0 ? 128 : n % 64 == 0 ? 64 : 32;
   NrsProfScope prof(ctx, NRS_PROF_GEMM, 2.0 * m * cols * kk);
   return dispatch<false>(ctx, tile_of(ctx, m, cols, 1, kk, split, limit), split, A, B, 1, n, count, m, cols, kk, pol, extras);

@@ -1,13 +1,13 @@
 // Shared tcgen05 main loop: D[128 x BN] (TMEM, f32) = sum over K-slices of
-// A[128 x 32] . B[BN x 32]^T, both operands K-major in 128-byte-swizzled shared
-// memory, fed by TMA, consumed by tcgen05.mma kind::tf32.
+// A[128 x KW] . B[BN x KW]^T, operands K-major (or MN-major) in swizzled shared
+// memory, fed by TMA, consumed by tcgen05.mma kind::tf32 (TF32 mode) or kind::f16 (3xTF32).
 //
 // Persistent CTAs (one per SM) walk a list of output tiles (row tile, column tile,
 // batch x K-split).  Six to eighteen warps, fixed roles:
 //   warp 0     TMA producer: per K-slice, one mbarrier-tracked ring
 //              slot holding the A and B slices (and their residual planes for 3xTF32);
 //              the ring runs ahead across tile boundaries
-//   warp 1     TMEM allocation; issues the UMMAs (M=128, K=8) and commits
+//   warp 1     TMEM allocation; issues the UMMAs (M=128, K=8 or 16) and commits
 //              ring slots back to the producer, then the accumulator to the epilogue
 //   warps 2..  epilogue (4, 8 or 16 warps, the policy's choice): tcgen05.ld (thread = accumulator row),
 //              policy-defined store
@@ -17,25 +17,26 @@
 // NHWC window for convolution), which K-slices of a tile count and whether the tile
 // exists at all (clip: triangular products), and what the epilogue does with a row of results.
 // A policy with kCanEmit may also hand the finished values back: the epilogue warps then
-// write them as TF32 high / residual planes ([row][32 columns], 128-byte swizzle) into a
+// write them as operand planes ([row][32 columns], swizzled) into a
 // staging tile and one thread sends each tile to global memory with a TMA store — the
 // operand planes of the next tensor-core kernel, written in full lines without a pass of
 // their own.
 //
-// 3xTF32 (NPLANES == 2): the residual plane of B sits directly behind its high plane in
-// the ring slot, so one UMMA of width 2*BN computes A_hi.[B_hi ; B_lo] (hi*hi in columns
-// [0,BN), hi*lo in [BN,2BN)) and a second of width BN adds A_lo.B_hi onto the first half;
-// the epilogue sums the halves.  Against three UMMAs of width BN this reads a quarter
-// less shared memory per K-step, which is what bounds the narrow (BN = 64) tiles.
+// 3xTF32 (NPLANES == 2): operands are f16 pairs (pair.cuh), multiplied by kind::f16 at twice the rate of kind::tf32.  The
+// low halves carry a factor 2^11, so hi*hi and the sum of hi*lo and lo*hi have accumulators of their own (columns [0,BN) and
+// [BN,2BN)); the epilogue adds them and takes the operands' exponents out.  In shared memory B_lo sits directly behind B_hi,
+// so one UMMA of width 2*BN computes A_hi.[B_hi ; B_lo] and a second of width BN adds A_lo.B_hi onto the second half; a pair
+// of CTAs, each holding half of B_hi and of B_lo, takes three UMMAs of width BN.  A K-slice is 64 values wide where the
+// operands allow (rows of 128 bytes; TMA brings rows of 64 at a lower rate: 138 -> 119 us on the data gradient below).
+// Against three kind::tf32 products of a TF32 value and its f32 residual: 16384 x 4096 x 4096 in 787 clocks per 64 values of
+// K (1640), of which the UMMAs alone are 768; x[256,64,32,32] -> 128 channels, 3x3: forward 172 -> 110 us, data gradient
+// 170 -> 119 us.
 //
-// What bounds a tile: with 128 columns in 3xTF32 the tensor pipe (768 clocks of UMMA per K-slice), with fewer the reads of
-// A from shared memory and the way of the operand planes through L2 (48 KB per K-slice of a 128 x 64 tile).  With PAIR the
+// What bounds a tile: with 128 columns the tensor pipe, with 64 the way of A through L2 (40 KB per 64 values of K at about
+// 60 bytes a clock) and the 46 clocks that a UMMA takes at least; short reductions the epilogue.  With PAIR the
 // two CTAs of a cluster work on two row tiles of one column tile: each brings its own A rows and half of the B rows, and
 // one warp issues UMMAs of 256 rows that read B from both (cta_group::2), which halves B's share of that traffic.  The
-// ring, the accumulators and the epilogue stay per CTA.  Clocks per K-slice (3xTF32 GEMM; TF32): single 128 columns
-// 905; 428, 64 columns 660; 369, pairs 820; 345 and 565; 317.  (With one thread per role, see elect_one: 960; 630 and 863;
-// 620, bound by the issuing thread, so that narrower tiles and pairs gained nothing.)  A 64-channel 3x3 layer on 100
-// images of 32 x 32: 59 -> 43 us.
+// ring, the accumulators and the epilogue stay per CTA.
 //
 // The tensor core's f32 accumulation is not round-to-nearest; its error grows
 // linearly with the length of one accumulation chain (about 7e-9 relative per K
@@ -53,20 +54,24 @@
 
 #include "igemm_problems.cuh"
 #include "nrs_internal.h"
+#include "pair.cuh"
 #include "tc_common.cuh"
 
 namespace tc {
 
-constexpr int BM = 128, BK = 32;   // BK f32 = 128 bytes = one swizzle row
+constexpr int BM = 128, BK = 32;   // 32 values: 128 bytes of f32, 64 of f16: one swizzle row
 constexpr int kMaxChainK = 4096;   // longest single accumulation chain in 3xTF32 mode
 constexpr int kGroupM = 16;        // row tiles per raster group (see TileMap)
 
-template <int BN, int NPLANES, int EMIT_BYTES, bool PAIR>
+// KW: values of K in a K-slice, and in a row of it (MN-major operands: columns of a block): 32, or 64 of f16.
+template <int BN, int NPLANES, int EMIT_BYTES, bool PAIR, int KW>
 struct SmemLayout {
-  static constexpr int kATile = BM * BK * 4;   // 16 KB
-  static constexpr int kBTile = BN / (PAIR ? 2 : 1) * BK * 4;   // this CTA's rows of B
+  static_assert(KW == 32 || (KW == 64 && NPLANES == 2), "a row is at most 128 bytes");
+  static constexpr int kRowBytes = KW * (NPLANES == 2 ? 2 : 4);
+  static constexpr int kATile = BM * kRowBytes;                // per plane
+  static constexpr int kBTile = BN / (PAIR ? 2 : 1) * kRowBytes;   // this CTA's rows of B
   static constexpr int kSlice = NPLANES * (kATile + kBTile);   // [A_hi][B_hi][B_lo][A_lo]
-  static constexpr int kSlices = NPLANES == 1 ? 2 : 1;         // K-slices per ring slot (see above)
+  static constexpr int kSlices = KW == 64 ? 1 : 2;             // K-slices per ring slot
   static constexpr int kStage = kSlices * kSlice;
   static constexpr int kExtra = EMIT_BYTES /*plane staging tile*/ + 1024 /*align*/ + 256 /*barriers*/;
   static constexpr int kRing = 227 * 1024 - kExtra;
@@ -75,6 +80,13 @@ struct SmemLayout {
   static constexpr int kAccCols = NPLANES * BN;                 // one accumulator
   static constexpr int kTmemCols = 2 * kAccCols < 32 ? 32 : 2 * kAccCols;   // two of them
   static_assert((kTmemCols & (kTmemCols - 1)) == 0 && kTmemCols <= 512, "TMEM allocation must be a power of two <= 512");
+};
+
+// 3xTF32: ranges of both operands, and of the result where its planes or its largest magnitude are wanted (else null).
+struct Ranges {
+  const NrsRange* a;
+  const NrsRange* b;
+  NrsRange* out;
 };
 
 struct SplitInfo {
@@ -134,10 +146,10 @@ struct TileMap {
   }
 };
 
-// Shared memory of the epilogue: a plane-emission staging tile per four warps, [128 rows][128 B] per plane, or (row-major
-// results) a 32 x 16 transpose tile per warp.
+// Shared memory of the epilogue: a plane-emission staging tile per four warps, [128 rows][128 B] (pairs: [128 rows][64 B] of
+// hi, then of lo), or (row-major results) a 32 x 16 transpose tile per warp.
 template <int NPLANES, class Policy>
-__host__ __device__ constexpr int emit_bytes() { return Policy::kCanEmit ? Policy::kEpiWarps / 4 * NPLANES * BM * 128 : Policy::kEpiWarps * 2048; }
+__host__ __device__ constexpr int emit_bytes() { return Policy::kCanEmit ? Policy::kEpiWarps / 4 * BM * 128 : Policy::kEpiWarps * 2048; }
 template <class Policy>
 __host__ __device__ constexpr int threads() { return 64 + 32 * Policy::kEpiWarps; }
 
@@ -170,15 +182,15 @@ __device__ __forceinline__ void rows_to_lines(float* tile, int lane, const uint3
   for (int i = 0; i < 4; ++i) v[i] = t4[chunk(8 * i + (lane >> 2), lane & 3)];
 }
 
-template <int BN, int NPLANES, class Policy, bool PAIR>
+template <int BN, int NPLANES, class Policy, bool PAIR, int KW>
 __global__ void __launch_bounds__(threads<Policy>(), 1)
 tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ CUtensorMap tm_a_lo,
           const __grid_constant__ CUtensorMap tm_b_hi, const __grid_constant__ CUtensorMap tm_b_lo,
           const __grid_constant__ CUtensorMap tm_out_hi, const __grid_constant__ CUtensorMap tm_out_lo,
           const Policy pol, const SplitInfo sp, const TileMap tmap, const int emit /*planes to emit: 0, 1 or 2*/,
-          int* __restrict__ err_flag) {
+          const Ranges rg, int* __restrict__ err_flag) {
   constexpr int kEmitBytes = emit_bytes<NPLANES, Policy>();
-  using L = SmemLayout<BN, NPLANES, kEmitBytes, PAIR>;
+  using L = SmemLayout<BN, NPLANES, kEmitBytes, PAIR, KW>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint8_t* emit_tile = smem + L::kStages * L::kStage;   // [four warps][planes][128 rows][128 B], 1024-byte aligned
@@ -220,7 +232,7 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
   if (warp == 0) {
     // ---------------- TMA producer
     // Both CTAs of a pair count their bytes on the barrier of rank 0, which expects the sum.
-    const uint32_t slice_bytes = (uint32_t)(PAIR ? 2 : 1) * NPLANES * (pol.a_slice_bytes() + (uint32_t)L::kBTile);
+    const uint32_t slice_bytes = (uint32_t)(PAIR ? 2 : 1) * NPLANES * (pol.a_slice_rows() * (uint32_t)L::kRowBytes + (uint32_t)L::kBTile);
     uint32_t s = 0, ph = 0, issued = 0;   // ring slot, its use's parity, slices so far: run on across tiles
     bool ok = true;
     bool odd = false;
@@ -237,7 +249,7 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
       const int n0 = tile_n * BN + (PAIR ? rank * (BN / 2) : 0);
       // Where the K-slices of this tile lie, stepped along instead of recomputed (the divisions of a recomputation per
       // slice and plane made the producer the bottleneck: 58 -> 72 us on a 64-channel convolution).
-      typename Policy::Cursor cur = pol.cursor(tile_m, batch, kb_begin);
+      typename Policy::Cursor cur = pol.template cursor<KW>(tile_m, batch, kb_begin);
       for (int kb = kb_begin; kb < kb_end; kb += L::kSlices) {
         if (!mbar_wait_warp(&empty_bar[s], ph ^ 1u)) { ok = false; break; }
         const bool two = L::kSlices == 2 && kb + 1 < kb_end;
@@ -245,11 +257,11 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
         uint32_t bar;
         if constexpr (PAIR) bar = cluster_addr(&full_bar[s], 0); else bar = smem_u32(&full_bar[s]);
         auto bring = [&](uint8_t* dst) {
-          pol.template load_a<PAIR>(dst, &tm_a_hi, bar, cur);
-          pol.template load_b<BN, PAIR>(dst + L::kATile, &tm_b_hi, bar, cur, n0);
+          pol.template load_a<PAIR, KW, L::kRowBytes>(dst, &tm_a_hi, bar, cur);
+          pol.template load_b<BN, PAIR, KW, L::kRowBytes>(dst + L::kATile, &tm_b_hi, bar, cur, n0);
           if (NPLANES == 2) {
-            pol.template load_b<BN, PAIR>(dst + L::kATile + L::kBTile, &tm_b_lo, bar, cur, n0);
-            pol.template load_a<PAIR>(dst + L::kATile + 2 * L::kBTile, &tm_a_lo, bar, cur);
+            pol.template load_b<BN, PAIR, KW, L::kRowBytes>(dst + L::kATile + L::kBTile, &tm_b_lo, bar, cur, n0);
+            pol.template load_a<PAIR, KW, L::kRowBytes>(dst + L::kATile + 2 * L::kBTile, &tm_a_lo, bar, cur);
           }
         };
         const bool leader = elect_one();
@@ -257,10 +269,10 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
           if (rank == 0) mbar_expect_tx(&full_bar[s], two ? 2 * slice_bytes : slice_bytes);
           bring(st);
         }
-        pol.advance(cur);
+        pol.template advance<KW>(cur);
         if (two) {
           if (leader) bring(st + L::kSlice);
-          pol.advance(cur);
+          pol.template advance<KW>(cur);
         }
         __syncwarp();
         ++issued;
@@ -285,14 +297,13 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
       // ---------------- UMMA issuer
       constexpr bool kAMn = Policy::kAMnMajor, kBMn = Policy::kBMnMajor;
       constexpr int kRows = PAIR ? 2 * BM : BM;
-      constexpr uint32_t idesc_wide = make_idesc_tf32(kRows, NPLANES * BN, kAMn, kBMn);
-      constexpr uint32_t idesc_half = make_idesc_tf32(kRows, BN, kAMn, kBMn);
-      // A pair's wide product reads [B_hi half ; B_lo half] from each CTA, so its columns are hh0 hl0 hh1 hl1 (h: half of
-      // the tile's columns, 0 and 1).  The narrow one (lh0 lh1) is added to hl0 hh1, one half further on.
-      constexpr uint32_t kNarrow = PAIR ? BN / 2 : 0;
-      // K-major: 8 elements of K are 32 bytes inside the swizzle row.  MN-major: 32-column blocks of [32 k][128 B], so
-      // a K-step is 1024 bytes and blocks are 4096 apart (the blocks of B_lo follow those of B_hi).
+      constexpr uint32_t idesc_wide = NPLANES == 2 ? make_idesc_f16(kRows, 2 * BN, kAMn, kBMn) : make_idesc_tf32(kRows, BN, kAMn, kBMn);
+      constexpr uint32_t idesc_half = make_idesc_f16(kRows, BN, kAMn, kBMn);
+      // K-major: a UMMA's K (8 values of f32, 16 of f16) is 32 bytes inside the swizzle row.  MN-major: 32-column blocks of
+      // [32 k][row], so a K-step is 1024 bytes and blocks are a whole slice apart (the blocks of B_lo follow those of B_hi).
       auto desc = [](bool mn, uint32_t addr, int k) {
+        if (KW == 64) return mn ? make_smem_desc_sw128(addr + (uint32_t)k * 2048u, KW * 128, 1024) : make_smem_desc_sw128(addr + (uint32_t)k * 32u, 16, 1024);
+        if (NPLANES == 2) return mn ? make_smem_desc_sw64(addr + (uint32_t)k * 1024u, BK * 64, 512) : make_smem_desc_sw64(addr + (uint32_t)k * 32u, 16, 512);
         return mn ? make_smem_desc_sw128_32b(addr + (uint32_t)k * 1024u, BK * 128, 512) : make_smem_desc_sw128(addr + (uint32_t)k * 32u, 16, 1024);
       };
       uint32_t s = 0, ph = 0, local = 0;
@@ -326,10 +337,20 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
                 const uint32_t b_hi = a_hi + L::kATile;                 // B_lo follows B_hi directly
                 const uint32_t a_lo = b_hi + 2 * L::kBTile;
 #pragma unroll
-                for (int k = 0; k < BK / 8; ++k) {
+                for (int k = 0; k < (NPLANES == 2 ? KW / 16 : BK / 8); ++k) {
                   const uint64_t da_hi = desc(kAMn, a_hi, k), db_hi = desc(kBMn, b_hi, k);
-                  umma_tf32<PAIR>(d, da_hi, db_hi, idesc_wide, (i | sl | k) != 0);   // hi*hi | hi*lo
-                  if (NPLANES == 2) umma_tf32<PAIR>(d + kNarrow, desc(kAMn, a_lo, k), db_hi, idesc_half, 1);   // + lo*hi
+                  const uint32_t more = (i | sl | k) != 0;
+                  if constexpr (NPLANES == 1) {
+                    umma_tf32<PAIR>(d, da_hi, db_hi, idesc_wide, more);
+                  } else {
+                    if constexpr (PAIR) {   // (each CTA holds its half of B_hi and of B_lo: no one product over both)
+                      umma_f16<PAIR>(d, da_hi, db_hi, idesc_half, more);
+                      umma_f16<PAIR>(d + BN, da_hi, desc(kBMn, b_hi + L::kBTile, k), idesc_half, more);
+                    } else {
+                      umma_f16<PAIR>(d, da_hi, db_hi, idesc_wide, more);   // hi*hi | hi*lo
+                    }
+                    umma_f16<PAIR>(d + BN, desc(kAMn, a_lo, k), db_hi, idesc_half, 1);   // + lo*hi
+                  }
                 }
               }
               umma_commit<PAIR>(&empty_bar[s]);  // slot reusable once these UMMAs have read it
@@ -351,7 +372,19 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
     const int team = (warp - 2) >> 2;
     const bool emit_issuer = ((warp - 2) & 3) == 0 && lane == 0;
     uint64_t* emit_bar = emit_bars + (Policy::kCanEmit ? 2 * team : 0);
-    uint8_t* team_tile = emit_tile + (Policy::kCanEmit ? team * NPLANES * BM * 128 : 0);
+    uint8_t* team_tile = emit_tile + (Policy::kCanEmit ? team * BM * 128 : 0);
+    [[maybe_unused]] float us_a = 1.0f, us_b = 1.0f, out_scale = 1.0f;
+    [[maybe_unused]] uint32_t top = 0;
+    if constexpr (NPLANES == 2) {
+      const pr::Unscale us(rg.a->bound, rg.b->bound);
+      us_a = us.a;
+      us_b = us.b;
+      if (rg.out) {
+        const float bound = pol.out_bound(rg.a->top, rg.b->top, lane);
+        out_scale = pr::scale_of(bound);
+        if (blockIdx.x == 0 && warp == 2 && lane == 0) rg.out->bound = bound;   // (a K-split's second pass and the readers)
+      }
+    }
     uint32_t local = 0, emitted = 0;
     bool ok = true;
     bool odd = false;
@@ -392,15 +425,13 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
 #pragma unroll 1
         for (int c = c_first; c < kBlocks; c += kStep) {
           uint32_t r[kW];
-          // the columns of the first and of the second product (a pair: see kNarrow)
-          const int first = PAIR && NPLANES == 2 && c * kW >= BN / 2 ? BN / 2 + c * kW : c * kW;
-          tmem_ld_32(acc + (uint32_t)first, r);
+          tmem_ld_32(acc + (uint32_t)(c * kW), r);
           if (NPLANES == 2) {
             uint32_t r2[kW];
-            tmem_ld_32(acc + (uint32_t)(first + (PAIR ? BN / 2 : BN)), r2);
+            tmem_ld_32(acc + (uint32_t)(BN + c * kW), r2);
             tmem_ld_wait();
 #pragma unroll
-            for (int j = 0; j < kW; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(r2[j]));
+            for (int j = 0; j < kW; ++j) r[j] = __float_as_uint(fmaf(__uint_as_float(r2[j]), pr::kLoUnscale, __uint_as_float(r[j])) * us_a * us_b);
           } else {
             tmem_ld_wait();
           }
@@ -435,7 +466,7 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
 #pragma unroll
               for (int i = 0; i < 4; ++i, dst += (size_t)8 * sp.n_total) store_guarded(dst, v[i], sp.n_total - n, sp.n_total % 4 == 0);
             } else {
-              pol.epilogue(tile_m, batch, r0, n, v);
+              pol.template epilogue<NPLANES == 2>(tile_m, batch, r0, n, v, out_scale, top);
             }
           } else if (sp.splits > 1) {
             float* dst = sp.partial + (((size_t)split * sp.batches + batch) * sp.rows_total + (size_t)tile_m * BM + row) * sp.n_total;
@@ -447,6 +478,10 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
           } else {
             float v[32];
             pol.epilogue(rw, n0 + c * 32, r, v);
+            if (NPLANES == 2 && rg.out) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) top = pr::seen(top, v[j]);
+            }
             if (float* cs = pol.colsum_row(tile_m, q)) {
               // Sum over this warp's 32 rows, one channel per lane: a 32 x 32 transpose-reduce in 31
               // shuffles (each stage halves the values a lane holds; fixed order, deterministic).
@@ -473,28 +508,41 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
               if (emit_issuer) bulk_wait_read();
               mbar_arrive(&emit_bar[0]);
               if (!mbar_wait(&emit_bar[0], ph)) { atomicExch(err_flag, kErrEpilogueWait); ok = false; break; }
-              uint8_t* row_hi = team_tile + row * 128;
+              if constexpr (NPLANES == 2) {
+                uint8_t* row_hi = team_tile + row * 64;
 #pragma unroll
-              for (int g = 0; g < 8; ++g) {
-                const int chunk = (g ^ (row & 7)) * 16;   // 128-byte swizzle: 16-byte chunk index XOR row % 8
-                const float4 h = make_float4(tf32_rn(v[4 * g]), tf32_rn(v[4 * g + 1]), tf32_rn(v[4 * g + 2]), tf32_rn(v[4 * g + 3]));
-                *reinterpret_cast<float4*>(row_hi + chunk) = h;
-                if (NPLANES == 2 && emit == 2)
-                  *reinterpret_cast<float4*>(row_hi + BM * 128 + chunk) =
-                      make_float4(v[4 * g] - h.x, v[4 * g + 1] - h.y, v[4 * g + 2] - h.z, v[4 * g + 3] - h.w);
+                for (int g = 0; g < 4; ++g) {   // eight values
+                  const int chunk = (g ^ ((row >> 1) & 3)) * 16;   // 64-byte swizzle
+                  uint2 h0, l0, h1, l1;
+                  pr::split4(make_float4(v[8 * g], v[8 * g + 1], v[8 * g + 2], v[8 * g + 3]), out_scale, &h0, &l0);
+                  pr::split4(make_float4(v[8 * g + 4], v[8 * g + 5], v[8 * g + 6], v[8 * g + 7]), out_scale, &h1, &l1);
+                  *reinterpret_cast<uint4*>(row_hi + chunk) = make_uint4(h0.x, h0.y, h1.x, h1.y);
+                  *reinterpret_cast<uint4*>(row_hi + BM * 64 + chunk) = make_uint4(l0.x, l0.y, l1.x, l1.y);
+                }
+              } else {
+                uint8_t* row_hi = team_tile + row * 128;
+#pragma unroll
+                for (int g = 0; g < 8; ++g) {
+                  const int chunk = (g ^ (row & 7)) * 16;   // 128-byte swizzle: 16-byte chunk index XOR row % 8
+                  *reinterpret_cast<float4*>(row_hi + chunk) = make_float4(tf32_rn(v[4 * g]), tf32_rn(v[4 * g + 1]), tf32_rn(v[4 * g + 2]), tf32_rn(v[4 * g + 3]));
+                }
               }
               fence_proxy_async();   // generic-proxy writes -> visible to the TMA engine
               mbar_arrive(&emit_bar[1]);
               if (emit_issuer) {
                 if (!mbar_wait(&emit_bar[1], ph)) { atomicExch(err_flag, kErrEpilogueWait); ok = false; break; }
                 tma_store_4d(&tm_out_hi, team_tile, n0 + c * 32, rw.x0, rw.y0, rw.n0);
-                if (NPLANES == 2 && emit == 2) tma_store_4d(&tm_out_lo, team_tile + BM * 128, n0 + c * 32, rw.x0, rw.y0, rw.n0);
+                if (NPLANES == 2) tma_store_4d(&tm_out_lo, team_tile + BM * 64, n0 + c * 32, rw.x0, rw.y0, rw.n0);
                 bulk_commit();
               }
             }
           }
         }
       }
+    }
+    if constexpr (NPLANES == 2) {
+      __syncwarp();
+      if (rg.out && sp.splits == 1) pr::report(rg.out, top);
     }
     if (emit_issuer) bulk_wait_all();   // shared memory must outlive the stores that read it
   }
@@ -510,41 +558,49 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
 }
 
 // out(row, n) = policy.store(sum over splits of partial), fixed summation order.
-template <class Policy>
+template <bool SPLIT, class Policy>
 __global__ void __launch_bounds__(256)
-tc_splitk_reduce_kernel(const Policy pol, const SplitInfo sp) {
+tc_splitk_reduce_kernel(const Policy pol, const SplitInfo sp, NrsRange* __restrict__ out_range) {
   NRS_PDL_PROLOGUE();
   const size_t per = (size_t)sp.batches * sp.rows_total * sp.n_total;
   const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= per) return;
-  float s = 0.0f;
-  for (int z = 0; z < sp.splits; ++z) s += sp.partial[(size_t)z * per + idx];
-  const int n = (int)(idx % sp.n_total);
-  const size_t t = idx / sp.n_total;
-  const int row_lin = (int)(t % sp.rows_total);
-  const int b = (int)(t / sp.rows_total);
-  pol.store(row_lin / BM, b, row_lin % BM, n, s);
+  uint32_t top = 0;
+  if (idx < per) {
+    float s = 0.0f;
+    for (int z = 0; z < sp.splits; ++z) s += sp.partial[(size_t)z * per + idx];
+    const int n = (int)(idx % sp.n_total);
+    const size_t t = idx / sp.n_total;
+    const int row_lin = (int)(t % sp.rows_total);
+    const int b = (int)(t / sp.rows_total);
+    const float out_scale = SPLIT && out_range ? pr::scale_of(out_range->bound) : 1.0f;
+    pol.template store<SPLIT>(row_lin / BM, b, row_lin % BM, n, s, out_scale, top);
+  }
+  if (SPLIT && out_range) {
+    __syncwarp();
+    pr::report(out_range, top);
+  }
 }
 
 // Chooses the K-split: enough CTAs to fill the GPU, and no accumulation chain longer than kMaxChainK elements when
 // `limit_chain` (chunks where the tiles fill the GPU anyway).
-inline void plan_split(const nrs_ctx* ctx, long tiles, long out_elems, int kb_total, bool limit_chain, SplitInfo* sp) {
+inline void plan_split(const nrs_ctx* ctx, long tiles, long out_elems, int kb_total, int kw, bool limit_chain, SplitInfo* sp) {
   int s = 1;
   // (More than half a wave of tiles runs unsplit: the second pass over the partial tiles costs more
   // than the idle SMs.)
-  if (2 * tiles <= ctx->sm_count && kb_total >= 32) {
+  if (2 * tiles <= ctx->sm_count && kb_total * kw >= 1024) {
     s = (int)(ctx->sm_count / tiles);
     // a split shorter than 16 K-blocks is all prologue and second pass, except where the output is so small (a Linear
     // layer at a batch of a few dozen) that the second pass is nothing: there down to 4
-    const int shortest = out_elems <= (1 << 15) ? 4 : 16;
+    const int shortest = (out_elems <= (1 << 15) ? 4 : 16) * BK / kw;
     if (s > kb_total / shortest) s = kb_total / shortest;
     if (s < 1) s = 1;
   }
-  const int need = limit_chain ? (kb_total * BK + kMaxChainK - 1) / kMaxChainK : 1;
+  const int need = limit_chain ? (int)(((long)kb_total * kw + kMaxChainK - 1) / kMaxChainK) : 1;
   const bool in_chunks = s == 1 && need > 1;
   if (s < need) s = need;
   int per = (kb_total + s - 1) / s;
   if (per < 1) per = 1;
+  if (in_chunks) per += per & 1;   // (a ring slot's two K-slices belong to one chunk)
   s = (kb_total + per - 1) / per;
   sp->kb_per_split = per;
   sp->splits = in_chunks ? 1 : s;
@@ -572,7 +628,7 @@ inline TilePlan plan_tile(const nrs_ctx* ctx, long tiles_m, int n, long batches,
     if (c.bn > limit || (c.bn > 32 && c.bn / 2 >= n)) continue;   // half of the tile or more would be padding
     const long tiles_n = (n + c.bn - 1) / c.bn;
     SplitInfo sp{};
-    plan_split(ctx, tiles_m * tiles_n * batches, tiles_m * BM * n * batches, kblocks, split_planes, &sp);
+    plan_split(ctx, tiles_m * tiles_n * batches, tiles_m * BM * n * batches, kblocks, BK, split_planes, &sp);
     const int splits = sp.splits, per = sp.kb_per_split * sp.chunks;
     const long units = (c.pair ? (tiles_m + 1) / 2 : tiles_m) * tiles_n * batches * splits, slots = ctx->sm_count / (c.pair ? 2 : 1);
     const int kb_clk = c.pair && c.bn == 64 && conv && !split_planes ? 400 : c.kb_clk[split_planes ? 0 : 1];
@@ -607,19 +663,19 @@ inline int plan_units_per_cta(int sm_count, int ctas, long units, int min_units,
   return (int)(best_u < 1 ? 1 : best_u);
 }
 
-template <int BN, int NPLANES, bool PAIR, class Policy>
+template <int BN, int NPLANES, bool PAIR, int KW, class Policy>
 int launch(nrs_ctx* ctx, const CUtensorMap& ta_hi, const CUtensorMap& ta_lo, const CUtensorMap& tb_hi,
            const CUtensorMap& tb_lo, const Policy& pol, int tiles_m, int n_total, int batches, int kb_total,
-           const CUtensorMap* out_hi = nullptr, const CUtensorMap* out_lo = nullptr, int* splits_out = nullptr) {
-  using L = SmemLayout<BN, NPLANES, emit_bytes<NPLANES, Policy>(), PAIR>;
+           const Ranges& rg, const CUtensorMap* out_hi = nullptr, const CUtensorMap* out_lo = nullptr, int* splits_out = nullptr) {
+  using L = SmemLayout<BN, NPLANES, emit_bytes<NPLANES, Policy>(), PAIR, KW>;
   constexpr int kSmem = L::kBytes;
   static_assert(kSmem <= 227 * 1024 && L::kStages >= 2, "shared memory budget");
   static NrsSmemAttr attr;
-  NRS_ENSURE_SMEM(ctx, attr, (tc_kernel<BN, NPLANES, Policy, PAIR>), kSmem);
+  NRS_ENSURE_SMEM(ctx, attr, (tc_kernel<BN, NPLANES, Policy, PAIR, KW>), kSmem);
   const int tiles_n = (n_total + BN - 1) / BN;
   SplitInfo sp{};
   if (Policy::kMaySplit) {
-    plan_split(ctx, (long)tiles_m * tiles_n * batches, (long)tiles_m * BM * n_total * batches, kb_total, NPLANES == 2, &sp);
+    plan_split(ctx, (long)tiles_m * tiles_n * batches, (long)tiles_m * BM * n_total * batches, kb_total, KW, NPLANES == 2, &sp);
   } else {   // tiles whose K ranges differ
     sp.splits = sp.chunks = 1;
     sp.kb_per_split = kb_total;
@@ -652,12 +708,12 @@ int launch(nrs_ctx* ctx, const CUtensorMap& ta_hi, const CUtensorMap& ta_lo, con
   const unsigned grid = (unsigned)((tmap.total < slots ? tmap.total : slots) * (PAIR ? 2 : 1));
   // Planes can only be emitted by the direct epilogue; with a K-split the policy's store() writes them.
   const int emit = (Policy::kCanEmit && out_hi && sp.splits == 1) ? (out_lo && NPLANES == 2 ? 2 : 1) : 0;
-  (void)nrs_pdl_launch_cluster(PAIR ? 2 : 1, tc_kernel<BN, NPLANES, Policy, PAIR>, dim3(grid), dim3(threads<Policy>()), (size_t)kSmem, ctx->stream,
-                               ta_hi, ta_lo, tb_hi, tb_lo, out_hi ? *out_hi : ta_hi, out_lo ? *out_lo : ta_hi, pol, sp, tmap, emit, err);
+  (void)nrs_pdl_launch_cluster(PAIR ? 2 : 1, tc_kernel<BN, NPLANES, Policy, PAIR, KW>, dim3(grid), dim3(threads<Policy>()), (size_t)kSmem, ctx->stream,
+                               ta_hi, ta_lo, tb_hi, tb_lo, out_hi ? *out_hi : ta_hi, out_lo ? *out_lo : ta_hi, pol, sp, tmap, emit, rg, err);
   NRS_LAUNCHED(ctx);
   if (sp.splits > 1) {
     const size_t per = (size_t)batches * sp.rows_total * n_total;
-    NRS_PDL_LAUNCH((tc_splitk_reduce_kernel<Policy>), nrs_blocks(per, 256), 256, 0, ctx->stream, pol, sp);
+    NRS_PDL_LAUNCH((tc_splitk_reduce_kernel<NPLANES == 2, Policy>), nrs_blocks(per, 256), 256, 0, ctx->stream, pol, sp, rg.out);
     NRS_LAUNCHED(ctx);
   }
   return NRS_OK;
@@ -668,8 +724,6 @@ int launch(nrs_ctx* ctx, const CUtensorMap& ta_hi, const CUtensorMap& ta_lo, con
 // Operand staging (tc_stage.cu).  Planes are [batch][rows][ldk] f32 with ldk a multiple of
 // 8 and zeros beyond K; `lo == nullptr` means no split (hi = the values themselves).
 // src_k_by_rows: the source is stored [K][rows] (transposed) instead of [rows][K].
-int nrs_tc_stage(nrs_ctx* ctx, const float* src, float* hi, float* lo, int rows, int K, int ldk, int batch,
-                 size_t src_bstride, size_t dst_bstride, bool src_k_by_rows);
 // Masked gradient staging (see stage_masked_kernel): mode 0 = ReLU mask of dy[n,c,h,w] by y;
 // mode 1 = gradient of a k x k / stride-k max-pool (g[n,c,h/k,w/k], argmax) followed by the ReLU
 // mask, taken from the pooled output y[n,c,h/k,w/k].  nchw_out and the planes are each optional
@@ -678,11 +732,11 @@ int nrs_tc_stage(nrs_ctx* ctx, const float* src, float* hi, float* lo, int rows,
 // were written (0: this path does not produce them and the caller sums the NCHW gradient).
 int nrs_tc_stage_masked(nrs_ctx* ctx, int mode, const float* g, const float* y, const int32_t* argmax, int n, int c,
                         int h, int w, int k, float* nchw_out, float* hi, float* lo, float* chan_partial = nullptr,
-                        int* chan_partial_rows = nullptr);
+                        int* chan_partial_rows = nullptr, const NrsRange* g_range = nullptr);
 // 2x2 / stride-2 max-pool forward that also writes the NHWC planes of the pooled output
 // (NRS_ERR_UNSUPPORTED for odd image sizes).
 int nrs_tc_pool2_fwd_planes(nrs_ctx* ctx, const float* x, float* y, int32_t* argmax, float* hi, float* lo, int n, int c,
-                            int h, int w);
+                            int h, int w, const NrsRange* x_range = nullptr);
 inline size_t nrs_stage_masked_partial_rows(int n, int h, int w) { return ((size_t)n * (h / 2) * (w / 2) + 31) / 32; }
 // Conv weights w[co][ci][kh][kw] -> K-major planes; the channels of a tap are padded with zeros to a multiple of 32.
 //  for_dgrad == 0: out[co][(i*kw + j)*ceil32(ci) + ci]   (forward B operand)

@@ -10,15 +10,65 @@
 
 namespace {
 
+// Largest finite magnitude of n values into r->top.  A read of the tensor, from HBM where it exceeds L2.
+struct Measured { const float* src; size_t n; NrsRange* r; };
+__global__ void __launch_bounds__(256)
+absmax_kernel(const Measured m0, const Measured m1 /*blockIdx.y == 1*/) {
+  NRS_PDL_PROLOGUE();
+  __shared__ uint32_t part[8];
+  const Measured& m = blockIdx.y == 0 ? m0 : m1;
+  const float* __restrict__ src = m.src;
+  const size_t n = m.n;
+  const size_t head = min(n, (size_t)(((16 - (reinterpret_cast<uintptr_t>(src) & 15)) & 15) / 4)), quads = (n - head) / 4;
+  const float4* body = reinterpret_cast<const float4*>(src + head);
+  const size_t step = (size_t)gridDim.x * blockDim.x, first = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  uint32_t top = 0;
+  size_t i = first;
+  for (; i + 3 * step < quads; i += 4 * step) {
+    float4 v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) v[u] = body[i + u * step];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) top = pr::seen4(top, v[u]);
+  }
+  for (; i < quads; i += step) top = pr::seen4(top, body[i]);
+  if (first < head) top = pr::seen(top, src[first]);
+  if (head + 4 * quads + first < n) top = pr::seen(top, src[head + 4 * quads + first]);   // (at most 3, in the first block)
+  top = __reduce_max_sync(0xffffffffu, top);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = top;
+  __syncthreads();
+  if (threadIdx.x >= 32) return;
+  pr::report(m.r, threadIdx.x < 8 ? part[threadIdx.x] : 0u);
+}
+
+__global__ void __launch_bounds__(256)
+pair_unpack_kernel(const float* __restrict__ hi, const float* __restrict__ lo, const NrsRange* __restrict__ range, float* __restrict__ dst, size_t n) {
+  NRS_PDL_PROLOGUE();
+  const float unscale = pr::pow2(-pr::scale_exp(range->bound));
+  const size_t step = (size_t)gridDim.x * blockDim.x;
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += step)
+    dst[i] = fmaf(__half2float(reinterpret_cast<const __half*>(lo)[i]), pr::kLoUnscale, __half2float(reinterpret_cast<const __half*>(hi)[i])) * unscale;
+}
+
+// The scale of planes whose values `*top` bounds; one thread of the grid leaves it as their range.
+__device__ __forceinline__ float open_range(const float* top, NrsRange* range) {
+  const float bound = *reinterpret_cast<const volatile float*>(top);
+  if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) {
+    range->bound = bound;
+    if (top != &range->top) range->top = bound;
+  }
+  return pr::scale_of(bound);
+}
+
 template <bool SPLIT>
 __global__ void __launch_bounds__(256)
 stage_rows_kernel(const float* __restrict__ src, float* __restrict__ hi, float* __restrict__ lo, int rows, int K,
-                  int ldk, size_t src_bstride, size_t dst_bstride) {
+                  int ldk, size_t src_bstride, size_t dst_bstride, NrsRange* range) {
   NRS_PDL_PROLOGUE();
+  const float scale = SPLIT ? open_range(&range->top, range) : 1.0f;
   const int b = blockIdx.y;
   src += b * src_bstride;
-  hi += b * dst_bstride;
-  if (SPLIT) lo += b * dst_bstride;
+  const size_t dst = b * dst_bstride;
   const int q = ldk / 4;
   const size_t total4 = (size_t)rows * q;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
@@ -35,27 +85,21 @@ stage_rows_kernel(const float* __restrict__ src, float* __restrict__ hi, float* 
       if (k + 2 < K) v.z = src[r * K + k + 2];
       if (k + 3 < K) v.w = src[r * K + k + 3];
     }
-    if (SPLIT) {
-      const float4 h = make_float4(tc::tf32_rn(v.x), tc::tf32_rn(v.y), tc::tf32_rn(v.z), tc::tf32_rn(v.w));
-      *reinterpret_cast<float4*>(lo + r * ldk + k) = make_float4(v.x - h.x, v.y - h.y, v.z - h.z, v.w - h.w);
-      *reinterpret_cast<float4*>(hi + r * ldk + k) = h;
-    } else {
-      *reinterpret_cast<float4*>(hi + r * ldk + k) =
-          make_float4(tc::tf32_rn(v.x), tc::tf32_rn(v.y), tc::tf32_rn(v.z), tc::tf32_rn(v.w));
-    }
+    if (SPLIT) pr::put4(hi, lo, dst + r * ldk + k, v, scale);
+    else *reinterpret_cast<float4*>(hi + dst + r * ldk + k) = make_float4(tc::tf32_rn(v.x), tc::tf32_rn(v.y), tc::tf32_rn(v.z), tc::tf32_rn(v.w));
   }
 }
 
 template <bool SPLIT>
 __global__ void __launch_bounds__(256)
 stage_transpose_kernel(const float* __restrict__ src, float* __restrict__ hi, float* __restrict__ lo, int rows, int K,
-                       int ldk, size_t src_bstride, size_t dst_bstride) {
+                       int ldk, size_t src_bstride, size_t dst_bstride, NrsRange* range) {
   NRS_PDL_PROLOGUE();
   __shared__ float tile[32][33];
+  const float scale = SPLIT ? open_range(&range->top, range) : 1.0f;
   const int b = blockIdx.z;
   src += b * src_bstride;
-  hi += b * dst_bstride;
-  if (SPLIT) lo += b * dst_bstride;
+  const size_t dst = b * dst_bstride;
   const int r0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   for (int i = ty; i < 32; i += 8) {
@@ -63,18 +107,20 @@ stage_transpose_kernel(const float* __restrict__ src, float* __restrict__ hi, fl
     tile[i][tx] = (k < K && r < rows) ? src[(size_t)k * rows + r] : 0.0f;
   }
   __syncthreads();
+  if (SPLIT) {   // two values a thread (ldk is even): 64 bytes of a row per half warp
+    for (int i = threadIdx.x >> 4; i < 32; i += 16) {
+      const int r = r0 + i, c = 2 * (threadIdx.x & 15), k = k0 + c;
+      if (r >= rows || k >= ldk) continue;
+      __half2 h, l;
+      pr::split2(tile[c][i] * scale, tile[c + 1][i] * scale, &h, &l);
+      *reinterpret_cast<__half2*>(reinterpret_cast<__half*>(hi) + dst + (size_t)r * ldk + k) = h;
+      *reinterpret_cast<__half2*>(reinterpret_cast<__half*>(lo) + dst + (size_t)r * ldk + k) = l;
+    }
+    return;
+  }
   for (int i = ty; i < 32; i += 8) {
     const int r = r0 + i, k = k0 + tx;
-    if (r < rows && k < ldk) {
-      const float v = tile[tx][i];
-      if (SPLIT) {
-        const float h = tc::tf32_rn(v);
-        hi[(size_t)r * ldk + k] = h;
-        lo[(size_t)r * ldk + k] = v - h;
-      } else {
-        hi[(size_t)r * ldk + k] = tc::tf32_rn(v);
-      }
-    }
+    if (r < rows && k < ldk) hi[dst + (size_t)r * ldk + k] = tc::tf32_rn(tile[tx][i]);
   }
 }
 
@@ -83,9 +129,11 @@ stage_transpose_kernel(const float* __restrict__ src, float* __restrict__ hi, fl
 // 29 us for 256 images of 128 x 32 x 32).
 template <bool SPLIT, bool SUMS>
 __global__ void __launch_bounds__(256)
-stage_image_kernel(const float* __restrict__ src, float* __restrict__ hi, float* __restrict__ lo, float* __restrict__ chan_partial, const img::Grid g) {
+stage_image_kernel(const float* __restrict__ src, float* __restrict__ hi, float* __restrict__ lo, float* __restrict__ chan_partial, const img::Grid g,
+                   NrsRange* range) {
   NRS_PDL_PROLOGUE();
   __shared__ img::Tile tile;
+  const float scale = SPLIT ? open_range(&range->top, range) : 1.0f;
   const uint32_t p0 = blockIdx.x * img::kTilePx;
   const int c0 = blockIdx.y * img::kTileCh, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const img::Pixels px(g, p0);
@@ -108,14 +156,15 @@ stage_image_kernel(const float* __restrict__ src, float* __restrict__ hi, float*
     }
   }
   __syncthreads();
-  img::tile_to_planes<SPLIT>(tile, g, p0, c0, hi, lo);
+  img::tile_to_planes<SPLIT>(tile, g, p0, c0, hi, lo, scale);
 }
 
 template <bool SPLIT>
 __global__ void __launch_bounds__(256)
 stage_conv_weight_kernel(const float* __restrict__ w, float* __restrict__ hi, float* __restrict__ lo, int co_n, int ci_n,
-                         int kh, int kw, int for_dgrad) {
+                         int kh, int kw, int for_dgrad, NrsRange* range) {
   NRS_PDL_PROLOGUE();
+  const float scale = SPLIT ? open_range(&range->top, range) : 1.0f;
   const int taps = kh * kw, rows = for_dgrad ? ci_n : co_n, inner = for_dgrad ? co_n : ci_n, ld = (inner + 31) / 32 * 32;
   const size_t total = (size_t)rows * ld * taps;
   const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -126,13 +175,8 @@ stage_conv_weight_kernel(const float* __restrict__ w, float* __restrict__ hi, fl
   const int row = (int)(idx / ((size_t)ld * taps));
   const int co = for_dgrad ? k : row, ci = for_dgrad ? row : k;
   const float v = k < inner ? w[((size_t)co * ci_n + ci) * taps + t] : 0.0f;
-  if (SPLIT) {
-    const float h = tc::tf32_rn(v);
-    hi[idx] = h;
-    lo[idx] = v - h;
-  } else {
-    hi[idx] = tc::tf32_rn(v);
-  }
+  if (SPLIT) pr::put(hi, lo, idx, v, scale);
+  else hi[idx] = tc::tf32_rn(v);
 }
 
 // Gradient staging fused with the masks that precede a convolution's backward pass.
@@ -146,8 +190,9 @@ template <bool SPLIT, int MODE>
 __global__ void __launch_bounds__(256)
 stage_masked_kernel(const float* __restrict__ g, const float* __restrict__ y, const int32_t* __restrict__ argmax,
                     float* __restrict__ nchw_out, float* __restrict__ hi, float* __restrict__ lo, int c_n, int h,
-                    int w, int k, int oh, int ow) {
+                    int w, int k, int oh, int ow, const float* g_top, NrsRange* range) {
   NRS_PDL_PROLOGUE();
+  const float scale = SPLIT ? open_range(g_top, range) : 1.0f;
   __shared__ float tile[32][33];
   const int img = blockIdx.z, hw = h * w;
   const int p0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
@@ -178,9 +223,8 @@ stage_masked_kernel(const float* __restrict__ g, const float* __restrict__ y, co
     if (px < hw && c < c_n) {
       const float v = tile[tx][i];
       const size_t o = ((size_t)img * hw + px) * c_n + c;
-      const float hv = tc::tf32_rn(v);
-      hi[o] = hv;
-      if (SPLIT) lo[o] = v - hv;
+      if (SPLIT) pr::put(hi, lo, o, v, scale);
+      else hi[o] = tc::tf32_rn(v);
     }
   }
 }
@@ -196,8 +240,9 @@ __global__ void __launch_bounds__(256)
 pool2_bwd_planes_kernel(const float* __restrict__ g, const float* __restrict__ pooled, const int32_t* __restrict__ argmax,
                         float* __restrict__ nchw_out, float* __restrict__ hi, float* __restrict__ lo,
                         float* __restrict__ chan_partial /*[gridDim.x][c_n] per-block channel sums, or null*/, int n_img,
-                        int c_n, int h, int w) {
+                        int c_n, int h, int w, const float* g_top, NrsRange* range) {
   NRS_PDL_PROLOGUE();
+  const float scale = SPLIT ? open_range(g_top, range) : 1.0f;
   __shared__ float tile[32][129];   // [channel][q*32 + position], q = 2*dy + dx inside the window
   __shared__ long long pix_base[32]; // linear index of each position's top-left pixel, -1 beyond the end
   const int oh = h >> 1, ow = w >> 1, ohw = oh * ow, hw = h * w;
@@ -241,6 +286,22 @@ pool2_bwd_planes_kernel(const float* __restrict__ g, const float* __restrict__ p
   }
   if (!hi) return;
   __syncthreads();
+  if (SPLIT) {   // a thread: two channels (c_n is a multiple of 8), a half warp a pixel's 32
+    const int cl = 2 * (threadIdx.x & 15);
+    if (c0 + cl >= c_n) return;
+#pragma unroll 4
+    for (int k = threadIdx.x >> 4; k < 128; k += 16) {
+      const int q = k >> 5, pl = k & 31;
+      const long long base = pix_base[pl];
+      if (base < 0) continue;
+      const size_t o = ((size_t)base + (size_t)(q >> 1) * w + (q & 1)) * c_n + c0 + cl;
+      __half2 hv, lv;
+      pr::split2(tile[cl][k] * scale, tile[cl + 1][k] * scale, &hv, &lv);
+      *reinterpret_cast<__half2*>(reinterpret_cast<__half*>(hi) + o) = hv;
+      *reinterpret_cast<__half2*>(reinterpret_cast<__half*>(lo) + o) = lv;
+    }
+    return;
+  }
   // warp ty writes pixels k = ty, ty+8, ...: lane = channel
   const int c = c0 + tx;
   if (c >= c_n) return;
@@ -250,10 +311,7 @@ pool2_bwd_planes_kernel(const float* __restrict__ g, const float* __restrict__ p
     const long long base = pix_base[pl];
     if (base < 0) continue;
     const size_t pixel = (size_t)base + (size_t)(q >> 1) * w + (q & 1);
-    const float v = tile[tx][k];
-    const float hv = tc::tf32_rn(v);
-    hi[pixel * c_n + c] = hv;
-    if (SPLIT) lo[pixel * c_n + c] = v - hv;
+    hi[pixel * c_n + c] = tc::tf32_rn(tile[tx][k]);
   }
 }
 
@@ -265,9 +323,10 @@ pool2_bwd_planes_kernel(const float* __restrict__ g, const float* __restrict__ p
 template <bool SPLIT>
 __global__ void __launch_bounds__(256)
 pool2_fwd_planes_kernel(const float* __restrict__ x, float* __restrict__ y, int32_t* __restrict__ argmax,
-                        float* __restrict__ hi, float* __restrict__ lo, int n_img, int c_n, int h, int w) {
+                        float* __restrict__ hi, float* __restrict__ lo, int n_img, int c_n, int h, int w, const float* x_top, NrsRange* range) {
   NRS_PDL_PROLOGUE();
   __shared__ float tile[32][33];
+  const float scale = SPLIT ? open_range(x_top, range) : 1.0f;
   const int oh = h >> 1, ow = w >> 1, ohw = oh * ow, hw = h * w;
   const long total_pos = (long)n_img * ohw;
   const long gp0 = (long)blockIdx.x * 32;
@@ -300,78 +359,138 @@ pool2_fwd_planes_kernel(const float* __restrict__ x, float* __restrict__ y, int3
     }
   }
   __syncthreads();
+  if (SPLIT) {   // a thread: two channels (c_n is a multiple of 8), a half warp a pixel's 32
+    const int cl = 2 * (threadIdx.x & 15);
+    if (c0 + cl >= c_n) return;
+#pragma unroll
+    for (int k = threadIdx.x >> 4; k < 32; k += 16) {
+      if (gp0 + k >= total_pos) continue;
+      const size_t o = (size_t)(gp0 + k) * c_n + c0 + cl;
+      __half2 hv, lv;
+      pr::split2(tile[cl][k] * scale, tile[cl + 1][k] * scale, &hv, &lv);
+      *reinterpret_cast<__half2*>(reinterpret_cast<__half*>(hi) + o) = hv;
+      *reinterpret_cast<__half2*>(reinterpret_cast<__half*>(lo) + o) = lv;
+    }
+    return;
+  }
   const int c = c0 + tx;   // lane = channel: one full 128-byte line per warp store
   if (c >= c_n) return;
 #pragma unroll
   for (int k = ty; k < 32; k += 8) {
     const long gp = gp0 + k;
     if (gp >= total_pos) continue;
-    const float v = tile[tx][k];
-    const float hv = tc::tf32_rn(v);
-    hi[(size_t)gp * c_n + c] = hv;
-    if (SPLIT) lo[(size_t)gp * c_n + c] = v - hv;
+    hi[(size_t)gp * c_n + c] = tc::tf32_rn(tile[tx][k]);
   }
 }
 
 }  // namespace
 
+static unsigned absmax_blocks(const nrs_ctx* ctx, size_t count) {
+  const size_t blocks = (count / 4 + 255) / 256 + 1, cap = (size_t)ctx->sm_count * 8;
+  return (unsigned)(blocks < cap ? blocks : cap);
+}
+int nrs_absmax(nrs_ctx* ctx, const float* src, size_t count, NrsRange* r) {
+  if (count == 0) return NRS_OK;
+  const Measured m{src, count, r};
+  NRS_PDL_LAUNCH(absmax_kernel, absmax_blocks(ctx, count), 256, 0, ctx->stream, m, m);
+  NRS_LAUNCHED(ctx);
+  return NRS_OK;
+}
+int nrs_absmax2(nrs_ctx* ctx, const float* a, size_t na, NrsRange* ra, const float* b, size_t nb, NrsRange* rb) {
+  NRS_PDL_LAUNCH(absmax_kernel, dim3(absmax_blocks(ctx, na > nb ? na : nb), 2), 256, 0, ctx->stream, Measured{a, na, ra}, Measured{b, nb, rb});
+  NRS_LAUNCHED(ctx);
+  return NRS_OK;
+}
+int nrs_pair_unpack(nrs_ctx* ctx, const float* hi, const float* lo, float* dst, size_t n) {
+  const NrsRange* range = nrs_range_of(ctx, hi);
+  NRS_REQUIRE(ctx, range != nullptr, NRS_ERR_ARG, "f16 pairs without a range");
+  if (n == 0) return NRS_OK;
+  NRS_PDL_LAUNCH(pair_unpack_kernel, absmax_blocks(ctx, n), 256, 0, ctx->stream, hi, lo, range, dst, n);
+  NRS_LAUNCHED(ctx);
+  return NRS_OK;
+}
+
+// A fresh range for `hi`; *top is what its values are bounded by: the source's own where `known` has it, else measured.
+static int open_planes(nrs_ctx* ctx, const float* hi, const float* src, size_t count, const NrsRange* known, NrsRange** range, const float** top) {
+  int st = nrs_range_renew(ctx, hi, range);
+  if (st == NRS_OK && !known) st = nrs_absmax(ctx, src, count, *range);
+  *top = known ? &known->top : &(*range)->top;
+  return st;
+}
+
 int nrs_tc_pool2_fwd_planes(nrs_ctx* ctx, const float* x, float* y, int32_t* argmax, float* hi, float* lo, int n, int c,
-                            int h, int w) {
+                            int h, int w, const NrsRange* x_range) {
   if (n <= 0 || c <= 0) return NRS_OK;
   if (h % 2 != 0 || w % 2 != 0 || !hi || (reinterpret_cast<uintptr_t>(x) & 7) != 0) return NRS_ERR_UNSUPPORTED;
   const long blocks = ((long)n * (h / 2) * (w / 2) + 31) / 32;
   if (blocks > 2147483647L || (c + 31) / 32 > 65535) return NRS_ERR_UNSUPPORTED;
   dim3 grid((unsigned)blocks, (unsigned)((c + 31) / 32));
-  if (lo) NRS_PDL_LAUNCH((pool2_fwd_planes_kernel<true>), grid, 256, 0, ctx->stream, x, y, argmax, hi, lo, n, c, h, w);
-  else NRS_PDL_LAUNCH((pool2_fwd_planes_kernel<false>), grid, 256, 0, ctx->stream, x, y, argmax, hi, nullptr, n, c, h, w);
+  if (lo) {
+    NrsRange* range = nullptr;
+    const float* top = nullptr;
+    const int st = open_planes(ctx, hi, x, (size_t)n * c * h * w, x_range, &range, &top);
+    if (st != NRS_OK) return st;
+    NRS_PDL_LAUNCH((pool2_fwd_planes_kernel<true>), grid, 256, 0, ctx->stream, x, y, argmax, hi, lo, n, c, h, w, top, range);
+  } else {
+    NRS_PDL_LAUNCH((pool2_fwd_planes_kernel<false>), grid, 256, 0, ctx->stream, x, y, argmax, hi, nullptr, n, c, h, w, nullptr, nullptr);
+  }
   NRS_LAUNCHED(ctx);
   return NRS_OK;
 }
 
 int nrs_tc_stage_masked(nrs_ctx* ctx, int mode, const float* g, const float* y, const int32_t* argmax, int n, int c,
                         int h, int w, int k, float* nchw_out, float* hi, float* lo, float* chan_partial,
-                        int* chan_partial_rows) {
+                        int* chan_partial_rows, const NrsRange* g_range) {
   if (chan_partial_rows) *chan_partial_rows = 0;
   if (n <= 0 || c <= 0) return NRS_OK;
   const int oh = mode == 1 ? h / k : h, ow = mode == 1 ? w / k : w;
   dim3 grid((unsigned)((h * w + 31) / 32), (unsigned)((c + 31) / 32), (unsigned)n);
   if (grid.y > 65535 || grid.z > 65535) return NRS_ERR_UNSUPPORTED;
   const bool split = lo != nullptr;
+  NrsRange* range = nullptr;
+  const float* top = nullptr;
+  if (split) {
+    const int st = open_planes(ctx, hi, g, (size_t)n * c * oh * ow, g_range, &range, &top);
+    if (st != NRS_OK) return st;
+  }
   if (mode == 1 && k == 2 && h % 2 == 0 && w % 2 == 0 && (long)n * (h / 2) * (w / 2) / 32 < 2147483647L) {
     dim3 pgrid((unsigned)(((long)n * (h / 2) * (w / 2) + 31) / 32), (unsigned)((c + 31) / 32));
-    if (split) NRS_PDL_LAUNCH((pool2_bwd_planes_kernel<true>), pgrid, 256, 0, ctx->stream, g, y, argmax, nchw_out, hi, lo, chan_partial, n, c, h, w);
-    else NRS_PDL_LAUNCH((pool2_bwd_planes_kernel<false>), pgrid, 256, 0, ctx->stream, g, y, argmax, nchw_out, hi, lo, chan_partial, n, c, h, w);
+    if (split) NRS_PDL_LAUNCH((pool2_bwd_planes_kernel<true>), pgrid, 256, 0, ctx->stream, g, y, argmax, nchw_out, hi, lo, chan_partial, n, c, h, w, top, range);
+    else NRS_PDL_LAUNCH((pool2_bwd_planes_kernel<false>), pgrid, 256, 0, ctx->stream, g, y, argmax, nchw_out, hi, lo, chan_partial, n, c, h, w, top, range);
     NRS_LAUNCHED(ctx);
     if (chan_partial && chan_partial_rows) *chan_partial_rows = (int)pgrid.x;
     return NRS_OK;
   }
-  if (mode == 0) {
-    if (split) NRS_PDL_LAUNCH((stage_masked_kernel<true, 0>), grid, 256, 0, ctx->stream, g, y, argmax, nchw_out, hi, lo, c, h, w, k, oh, ow);
-    else NRS_PDL_LAUNCH((stage_masked_kernel<false, 0>), grid, 256, 0, ctx->stream, g, y, argmax, nchw_out, hi, lo, c, h, w, k, oh, ow);
-  } else {
-    if (split) NRS_PDL_LAUNCH((stage_masked_kernel<true, 1>), grid, 256, 0, ctx->stream, g, y, argmax, nchw_out, hi, lo, c, h, w, k, oh, ow);
-    else NRS_PDL_LAUNCH((stage_masked_kernel<false, 1>), grid, 256, 0, ctx->stream, g, y, argmax, nchw_out, hi, lo, c, h, w, k, oh, ow);
-  }
+#define NRS_MASKED(S, M) NRS_PDL_LAUNCH((stage_masked_kernel<S, M>), grid, 256, 0, ctx->stream, g, y, argmax, nchw_out, hi, lo, c, h, w, k, oh, ow, top, range)
+  if (mode == 0) { if (split) NRS_MASKED(true, 0); else NRS_MASKED(false, 0); }
+  else { if (split) NRS_MASKED(true, 1); else NRS_MASKED(false, 1); }
+#undef NRS_MASKED
   NRS_LAUNCHED(ctx);
   return NRS_OK;
 }
 
 int nrs_tc_stage(nrs_ctx* ctx, const float* src, float* hi, float* lo, int rows, int K, int ldk, int batch,
-                 size_t src_bstride, size_t dst_bstride, bool src_k_by_rows) {
+                 size_t src_bstride, size_t dst_bstride, bool src_k_by_rows, NrsRange* measured) {
   if (rows <= 0 || K <= 0 || batch <= 0) return NRS_OK;
+  NrsRange* range = measured;
+  if (lo && !range) {
+    const float* top = nullptr;
+    const int st = open_planes(ctx, hi, src, batch == 1 ? (size_t)rows * K : src_bstride * (batch - 1) + (size_t)rows * K, nullptr, &range, &top);
+    if (st != NRS_OK) return st;
+  }
   if (!src_k_by_rows) {
     size_t blocks = ((size_t)rows * (ldk / 4) + 255) / 256;
     const size_t cap = (size_t)ctx->sm_count * 16;
     if (blocks > cap) blocks = cap;
     if (batch > 65535) return NRS_ERR_UNSUPPORTED;
     dim3 grid((unsigned)blocks, (unsigned)batch);
-    if (lo) NRS_PDL_LAUNCH((stage_rows_kernel<true>), grid, 256, 0, ctx->stream, src, hi, lo, rows, K, ldk, src_bstride, dst_bstride);
-    else NRS_PDL_LAUNCH((stage_rows_kernel<false>), grid, 256, 0, ctx->stream, src, hi, nullptr, rows, K, ldk, src_bstride, dst_bstride);
+    if (lo) NRS_PDL_LAUNCH((stage_rows_kernel<true>), grid, 256, 0, ctx->stream, src, hi, lo, rows, K, ldk, src_bstride, dst_bstride, range);
+    else NRS_PDL_LAUNCH((stage_rows_kernel<false>), grid, 256, 0, ctx->stream, src, hi, nullptr, rows, K, ldk, src_bstride, dst_bstride, nullptr);
   } else {
     dim3 grid((unsigned)((rows + 31) / 32), (unsigned)((ldk + 31) / 32), (unsigned)batch);
     if (grid.y > 65535 || grid.z > 65535) return NRS_ERR_UNSUPPORTED;
-    if (lo) NRS_PDL_LAUNCH((stage_transpose_kernel<true>), grid, 256, 0, ctx->stream, src, hi, lo, rows, K, ldk, src_bstride, dst_bstride);
-    else NRS_PDL_LAUNCH((stage_transpose_kernel<false>), grid, 256, 0, ctx->stream, src, hi, nullptr, rows, K, ldk, src_bstride, dst_bstride);
+    if (lo) NRS_PDL_LAUNCH((stage_transpose_kernel<true>), grid, 256, 0, ctx->stream, src, hi, lo, rows, K, ldk, src_bstride, dst_bstride, range);
+    else NRS_PDL_LAUNCH((stage_transpose_kernel<false>), grid, 256, 0, ctx->stream, src, hi, nullptr, rows, K, ldk, src_bstride, dst_bstride, nullptr);
   }
   NRS_LAUNCHED(ctx);
   return NRS_OK;
@@ -383,7 +502,13 @@ int nrs_tc_stage_image(nrs_ctx* ctx, const float* src, float* hi, float* lo, int
   if (hw == 1) return nrs_tc_stage(ctx, src, hi, lo, n, c, ld, 1, 0, 0, false);   // already pixel-major: split only
   if ((size_t)n * hw > 0x7fffffffu) return NRS_ERR_UNSUPPORTED;
   const img::Grid g(n, c, hw);
-#define NRS_STAGE(S, C) NRS_PDL_LAUNCH((stage_image_kernel<S, C>), g.blocks(), 256, 0, ctx->stream, src, hi, lo, chan_partial, g)
+  NrsRange* range = nullptr;
+  const float* top = nullptr;
+  if (lo) {
+    const int st = open_planes(ctx, hi, src, (size_t)n * c * hw, nullptr, &range, &top);
+    if (st != NRS_OK) return st;
+  }
+#define NRS_STAGE(S, C) NRS_PDL_LAUNCH((stage_image_kernel<S, C>), g.blocks(), 256, 0, ctx->stream, src, hi, lo, chan_partial, g, range)
   if (lo) { if (chan_partial) NRS_STAGE(true, true); else NRS_STAGE(true, false); }
   else { if (chan_partial) NRS_STAGE(false, true); else NRS_STAGE(false, false); }
 #undef NRS_STAGE
@@ -395,8 +520,15 @@ int nrs_tc_stage_conv_weight(nrs_ctx* ctx, const float* w, float* hi, float* lo,
                              int for_dgrad) {
   const size_t total = (size_t)(for_dgrad ? ci : co) * (((for_dgrad ? co : ci) + 31) / 32 * 32) * kh * kw;
   if (total == 0) return NRS_OK;
-  if (lo) NRS_PDL_LAUNCH((stage_conv_weight_kernel<true>), nrs_blocks(total, 256), 256, 0, ctx->stream, w, hi, lo, co, ci, kh, kw, for_dgrad);
-  else NRS_PDL_LAUNCH((stage_conv_weight_kernel<false>), nrs_blocks(total, 256), 256, 0, ctx->stream, w, hi, nullptr, co, ci, kh, kw, for_dgrad);
+  if (lo) {
+    NrsRange* range = nullptr;
+    const float* top = nullptr;
+    const int st = open_planes(ctx, hi, w, (size_t)co * ci * kh * kw, nullptr, &range, &top);
+    if (st != NRS_OK) return st;
+    NRS_PDL_LAUNCH((stage_conv_weight_kernel<true>), nrs_blocks(total, 256), 256, 0, ctx->stream, w, hi, lo, co, ci, kh, kw, for_dgrad, range);
+  } else {
+    NRS_PDL_LAUNCH((stage_conv_weight_kernel<false>), nrs_blocks(total, 256), 256, 0, ctx->stream, w, hi, nullptr, co, ci, kh, kw, for_dgrad, nullptr);
+  }
   NRS_LAUNCHED(ctx);
   return NRS_OK;
 }

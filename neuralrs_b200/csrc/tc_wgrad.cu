@@ -34,7 +34,6 @@ namespace {
 
 constexpr int kWgThreads = 192;
 constexpr int kMaxN = 256;        // widest UMMA
-constexpr int kABlocks = 4;       // 4 x 32 output channels = 128 rows
 
 struct WgradParams {
   int Wt, Ht, Nt, tiles_y, tiles_x;  // pixel tile (box) geometry in dy space
@@ -43,14 +42,16 @@ struct WgradParams {
   int tiles_per_split;
   int co, ci, kh, kw, pad, stride;
   int taps_per_group, n_groups;   // taps handled by one CTA
-  int cblocks;                    // ceil(ci / 32)
-  int a_box_blocks;               // 32-channel blocks of dy one box brings (min(4, ceil(co/32)))
+  int wa, wb;                     // channels of a block of dy, of x: 32, or 64 (f16: rows of 128 bytes)
+  int cblocks;                    // ceil(ci / wb)
+  int a_box_blocks;               // blocks of dy one box brings (128 channels at most)
   int ragged_a, ragged_x;         // channel count no multiple of 32: one 4-D box per block instead of one 5-D box for all
   int m_blocks;                   // ceil(co / 128)
   float* partial;                 // [split][m_block][group][col_block][128][group_cols]
   int group_cols;                 // taps_per_group * cblocks * 32 (more than 256 input channels: 256)
   int col_blocks;                 // more than 256 input channels: column blocks of 256, each its own CTA
   int independent;                // reads nothing the kernel launched just before it wrote (NRS_PDL_PROLOGUE)
+  const NrsRange *range_dy, *range_x;   // 3xTF32
   float* direct;                  // 1x1, one split, no accumulation: the tile is the result; written straight to dw[co][ci]
 };
 
@@ -61,9 +62,10 @@ tc_wgrad_kernel(const __grid_constant__ CUtensorMap tm_dy_hi, const __grid_const
                 const WgradParams p, const int n_cols /*UMMA N, multiple of 16*/, int* __restrict__ err_flag) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  const uint32_t blk_bytes = (uint32_t)p.kp * 128u;               // one 32-channel block of one plane
-  const uint32_t a_bytes = kABlocks * blk_bytes;                   // per plane
-  const uint32_t b_bytes = (uint32_t)(p.group_cols / 32) * blk_bytes;
+  const uint32_t value = NPLANES == 2 ? 2u : 4u;
+  const uint32_t a_blk = (uint32_t)(p.kp * p.wa) * value, b_blk = (uint32_t)(p.kp * p.wb) * value;   // one block of one plane
+  const uint32_t a_bytes = (uint32_t)(p.kp * 128) * value;         // per plane
+  const uint32_t b_bytes = (uint32_t)(p.kp * p.group_cols) * value;
   const uint32_t stage_bytes = NPLANES * (a_bytes + b_bytes);
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + STAGES * stage_bytes);
   uint64_t* empty_bar = full_bar + STAGES;
@@ -75,8 +77,8 @@ tc_wgrad_kernel(const __grid_constant__ CUtensorMap tm_dy_hi, const __grid_const
   const int mg = blockIdx.x / p.col_blocks;
   const int mb = mg / p.n_groups, grp = mg - mb * p.n_groups;
   const int split = blockIdx.y;
-  // 32-channel blocks of x this CTA's columns cover (a column block of a wide 1x1 layer may be ragged)
-  const int cblocks = p.col_blocks > 1 ? min(8, p.cblocks - cbk * 8) : p.cblocks;
+  // blocks of x this CTA's columns cover (a column block of a wide layer may be ragged)
+  const int most = kMaxN / p.wb, cblocks = p.col_blocks > 1 ? min(most, p.cblocks - cbk * most) : p.cblocks;
   const int t_begin = split * p.tiles_per_split;
   const int t_end = min(p.n_tiles, t_begin + p.tiles_per_split);
   const int ntiles = t_end - t_begin;
@@ -92,7 +94,7 @@ tc_wgrad_kernel(const __grid_constant__ CUtensorMap tm_dy_hi, const __grid_const
     tc::fence_barrier_init();
   }
   if (warp == 1) {
-    tc::tmem_alloc(tmem_slot, kMaxN);
+    tc::tmem_alloc(tmem_slot, NPLANES * kMaxN);
     tc::tmem_relinquish();
   }
   tc::tc_fence_before_sync();
@@ -109,9 +111,9 @@ tc_wgrad_kernel(const __grid_constant__ CUtensorMap tm_dy_hi, const __grid_const
     // (the channel-block index is the outermost box dimension), so a tile costs
     // planes x (1 + taps) TMA instructions instead of one per block.
     // (a ragged last column block still receives a full box: TMA zero-fills the blocks beyond the tensor)
-    const uint32_t tx = NPLANES * (uint32_t)(p.a_box_blocks + ntaps * (p.col_blocks > 1 ? 8 : p.cblocks)) * blk_bytes;
+    const int x_blocks = p.col_blocks > 1 ? most : p.cblocks;
+    const uint32_t tx = NPLANES * ((uint32_t)p.a_box_blocks * a_blk + (uint32_t)(ntaps * x_blocks) * b_blk);
     const int i_first = tap0 / p.kw, j_first = tap0 - i_first * p.kw;
-    const int x_blocks = p.col_blocks > 1 ? 8 : p.cblocks;
     int xt = t_begin % p.tiles_x, yt = t_begin / p.tiles_x;   // the tile's place, stepped along
     int nt = yt / p.tiles_y;
     yt -= nt * p.tiles_y;
@@ -133,20 +135,20 @@ tc_wgrad_kernel(const __grid_constant__ CUtensorMap tm_dy_hi, const __grid_const
           uint8_t* b_dst = a_dst + a_bytes;
           if (p.ragged_a) {
 #pragma unroll 1
-            for (int b = 0; b < p.a_box_blocks; ++b) tc::tma_load_4d(a_dst + b * blk_bytes, tdy, bar, (mb * kABlocks + b) * 32, x0, y0, n0);
+            for (int b = 0; b < p.a_box_blocks; ++b) tc::tma_load_4d(a_dst + b * a_blk, tdy, bar, mb * 128 + b * p.wa, x0, y0, n0);
           } else {
-            tc::tma_load_5d(a_dst, tdy, bar, 0, x0, y0, n0, mb * kABlocks);
+            tc::tma_load_5d(a_dst, tdy, bar, 0, x0, y0, n0, mb * 128 / p.wa);
           }
           int ti = i_first, tj = j_first;
 #pragma unroll 1
           for (int t = 0; t < ntaps; ++t) {
             const int xx = x0 * p.stride + tj - p.pad, xy = y0 * p.stride + ti - p.pad;
-            uint8_t* dst = b_dst + (size_t)t * p.cblocks * blk_bytes;
+            uint8_t* dst = b_dst + (size_t)t * p.cblocks * b_blk;
             if (p.ragged_x) {
 #pragma unroll 1
-              for (int b = 0; b < x_blocks; ++b) tc::tma_load_4d(dst + b * blk_bytes, txm, bar, (cbk * 8 + b) * 32, xx, xy, n0);
+              for (int b = 0; b < x_blocks; ++b) tc::tma_load_4d(dst + b * b_blk, txm, bar, (cbk * most + b) * p.wb, xx, xy, n0);
             } else {
-              tc::tma_load_5d(dst, txm, bar, 0, xx, xy, n0, cbk * 8);
+              tc::tma_load_5d(dst, txm, bar, 0, xx, xy, n0, cbk * most);
             }
             if (++tj == p.kw) { tj = 0; ++ti; }
           }
@@ -170,11 +172,16 @@ tc_wgrad_kernel(const __grid_constant__ CUtensorMap tm_dy_hi, const __grid_const
       }
     }
   } else if (warp == 1) {
-    // ---------------- UMMA issuer: both operands MN-major, K-step = 8 pixels = one 1024 B atom
-    const uint32_t idesc = tc::make_idesc_tf32(128, n_cols, true, true);
-    const uint64_t dc = tc::make_smem_desc_sw128_32b(0, blk_bytes, 512);   // every field but the start address (bytes >> 4)
+    // ---------------- UMMA issuer: both operands MN-major, K-step = 8 pixels (f16: 16) = 1024 B
+    const uint32_t idesc = NPLANES == 2 ? tc::make_idesc_f16(128, n_cols, true, true) : tc::make_idesc_tf32(128, n_cols, true, true);
+    // every field but the start address (bytes >> 4), and a K-step's bytes >> 4
+    auto desc = [](int w, uint32_t blk) {
+      return NPLANES == 1 ? tc::make_smem_desc_sw128_32b(0, blk, 512) : w == 64 ? tc::make_smem_desc_sw128(0, blk, 1024) : tc::make_smem_desc_sw64(0, blk, 512);
+    };
+    const uint64_t da = desc(p.wa, a_blk), db = desc(p.wb, b_blk);
+    const uint32_t step_a = p.wa == 64 ? 128u : 64u, step_b = p.wb == 64 ? 128u : 64u;
     bool ok = true;
-    const int ksteps = p.kp / 8;
+    const int ksteps = p.kp / (NPLANES == 2 ? 16 : 8);
     int s = 0;
     uint32_t ph = 0;
     for (int it = 0; it < ntiles; ++it) {
@@ -186,13 +193,14 @@ tc_wgrad_kernel(const __grid_constant__ CUtensorMap tm_dy_hi, const __grid_const
       if (tc::elect_one()) {
 #pragma unroll 2
         for (int k = 0; k < ksteps; ++k) {
-          const uint32_t koff = (uint32_t)k * 64u;
+          const uint64_t ah = da + (a_hi + (uint32_t)k * step_a), bh = db + (b_hi + (uint32_t)k * step_b);
+          const uint32_t more = (it | k) != 0;
           if (NPLANES == 2) {
-            tc::umma_tf32(tmem_base, dc + (a_lo + koff), dc + (b_hi + koff), idesc, (it | k) != 0);
-            tc::umma_tf32(tmem_base, dc + (a_hi + koff), dc + (b_lo + koff), idesc, 1);
-            tc::umma_tf32(tmem_base, dc + (a_hi + koff), dc + (b_hi + koff), idesc, 1);
+            tc::umma_f16(tmem_base, ah, bh, idesc, more);
+            tc::umma_f16(tmem_base + kMaxN, ah, db + (b_lo + (uint32_t)k * step_b), idesc, more);
+            tc::umma_f16(tmem_base + kMaxN, da + (a_lo + (uint32_t)k * step_a), bh, idesc, 1);
           } else {
-            tc::umma_tf32(tmem_base, dc + (a_hi + koff), dc + (b_hi + koff), idesc, (it | k) != 0);
+            tc::umma_tf32(tmem_base, ah, bh, idesc, more);
           }
         }
         tc::umma_commit(&empty_bar[s]);
@@ -211,16 +219,26 @@ tc_wgrad_kernel(const __grid_constant__ CUtensorMap tm_dy_hi, const __grid_const
     if (ok) {
       tc::tc_fence_after_sync();
       const int row = q * 32 + lane;
-      const int live_cols = p.col_blocks > 1 ? cblocks * 32 : ntaps * p.cblocks * 32;
+      const int live_cols = (p.col_blocks > 1 ? cblocks : ntaps * p.cblocks) * p.wb;
       float* dst = p.direct ? p.direct + (size_t)(mb * 128 + row) * p.ci + (size_t)cbk * 256
                             : p.partial + (((((size_t)split * p.m_blocks + mb) * p.n_groups + grp) * p.col_blocks + cbk) * 128 + row) *
                                               p.group_cols;
       const bool row_live = mb * 128 + row < p.co;
+      const pr::Unscale unscale(NPLANES == 2 ? p.range_dy->bound : 1.0f, NPLANES == 2 ? p.range_x->bound : 1.0f);
 #pragma unroll 1
       for (int c = 0; c < (live_cols + 31) / 32; ++c) {
         uint32_t r[32];
-        tc::tmem_ld_32x32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(c * 32), r);
-        tc::tmem_ld_wait();
+        const uint32_t at = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(c * 32);
+        tc::tmem_ld_32x32(at, r);
+        if constexpr (NPLANES == 2) {
+          uint32_t x[32];
+          tc::tmem_ld_32x32(at + kMaxN, x);
+          tc::tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(unscale(__uint_as_float(r[j]), __uint_as_float(x[j])));
+        } else {
+          tc::tmem_ld_wait();
+        }
         if (row_live) {
 #pragma unroll
           for (int j = 0; j < 32; j += 4)
@@ -238,7 +256,7 @@ tc_wgrad_kernel(const __grid_constant__ CUtensorMap tm_dy_hi, const __grid_const
   __syncthreads();
   if (warp == 1) {
     tc::tc_fence_after_sync();
-    tc::tmem_dealloc(tmem_base, kMaxN);
+    tc::tmem_dealloc(tmem_base, NPLANES * kMaxN);
   }
 }
 
@@ -248,17 +266,18 @@ tc_wgrad_kernel(const __grid_constant__ CUtensorMap tm_dy_hi, const __grid_const
 // slots of 16 pixels, 39.2 with two slots of 32; but with the 12 loads of five taps a slot of 16 costs 24.7 us against
 // 18.6), and a ring of fewer than three slots a few percent.  A box may reach past the last image too (a few 1x1 "images").
 void plan_pixel_box(WgradParams* p, int n, int oh, int ow, int planes, size_t bytes_per_pixel) {
-  const int loads = planes * ((p->ragged_a ? kABlocks : 1) + p->taps_per_group * (p->ragged_x ? p->cblocks : 1));
+  const int step = planes == 2 ? 16 : 8, most = planes == 2 ? 128 : 64;   // pixels of a K-step; of a box
+  const int loads = planes * ((p->ragged_a ? 128 / p->wa : 1) + p->taps_per_group * (p->ragged_x ? p->cblocks : 1));
   const double per_tile = loads > 4 ? 0.5 * loads : 2.0;
   double best = -1.0;
-  for (int c = 0; c <= 8; ++c) {
+  for (int c = 0; c <= most / 8; ++c) {
     const int Wt = c == 0 ? ow : 8 * c;
-    if (Wt > 64 || Wt * p->stride > 256 || (c > 0 && Wt - ow >= 8)) continue;
-    for (int Ht = 1; Ht <= oh && Wt * Ht <= 64 && Ht * p->stride <= 256; ++Ht) {
+    if (Wt > most || Wt * p->stride > 256 || (c > 0 && Wt - ow >= 8)) continue;
+    for (int Ht = 1; Ht <= (c > 0 && planes == 2 ? oh + 1 : oh) && Wt * Ht <= most && Ht * p->stride <= 256; ++Ht) {
       const bool whole = Ht == oh && Wt >= ow;
-      for (int Nt = 1; Nt <= (whole ? n + 7 : 1) && Wt * Ht * Nt <= 64; ++Nt) {
+      for (int Nt = 1; Nt <= (whole ? n + step - 1 : 1) && Wt * Ht * Nt <= most; ++Nt) {
         const int kp = Wt * Ht * Nt;
-        if (kp % 8 != 0) continue;
+        if (kp % step != 0) continue;
         const int stages = (int)((200 * 1024) / (bytes_per_pixel * kp));
         if (stages < 2) continue;
         const long tiles = (long)((ow + Wt - 1) / Wt) * ((oh + Ht - 1) / Ht) * ((n + Nt - 1) / Nt);
@@ -303,24 +322,30 @@ int nrs_tc_conv_wgrad(nrs_ctx* ctx, const float* x, const float* dy, float* dw, 
 
   WgradParams p{};
   p.co = co; p.ci = ci; p.kh = kh; p.kw = kw; p.pad = pad; p.stride = stride;
-  p.cblocks = (ci + 31) / 32;
-  p.ragged_a = co % 32 != 0;
-  p.ragged_x = ci % 32 != 0;
+  // f16: blocks of 64 channels, unless that pads much more (TMA brings rows of 64 bytes at half the rate of 128)
+  auto padded = [](int c, int w) { return (c + w - 1) / w * w; };
+  p.wa = split3 && co > 32 ? 64 : 32;
+  p.wb = split3 && 20 * padded(ci, 64) <= 23 * padded(ci, 32) ? 64 : 32;
+  p.cblocks = padded(ci, p.wb) / p.wb;
+  p.ragged_a = co % p.wa != 0;
+  p.ragged_x = ci % p.wb != 0;
   p.m_blocks = (co + 127) / 128;
   const int taps = kh * kw;
-  int tpg = p.cblocks * 32 <= kMaxN ? kMaxN / (p.cblocks * 32) : 1;
+  const int tap_cols = p.cblocks * p.wb;
+  int tpg = tap_cols <= kMaxN ? kMaxN / tap_cols : 1;
   if (tpg > taps) tpg = taps;
   p.n_groups = (taps + tpg - 1) / tpg;
   p.taps_per_group = (taps + p.n_groups - 1) / p.n_groups;
-  p.group_cols = p.taps_per_group * p.cblocks * 32;
+  p.group_cols = p.taps_per_group * tap_cols;
   p.col_blocks = 1;
-  if (p.cblocks * 32 > kMaxN) {     // the input channels are cut into column blocks of 256, one CTA each
+  if (tap_cols > kMaxN) {     // the input channels are cut into column blocks of 256, one CTA each
     p.col_blocks = (ci + kMaxN - 1) / kMaxN;
     p.n_groups = taps;
     p.taps_per_group = 1;
     p.group_cols = kMaxN;
   }
-  plan_pixel_box(&p, n, oh, ow, planes, (size_t)planes * (kABlocks + p.group_cols / 32) * 128);
+  const size_t pixel_bytes = (size_t)(128 + p.group_cols) * 4;   // both operands, all planes
+  plan_pixel_box(&p, n, oh, ow, planes, pixel_bytes);
   if (p.kp == 0) return NRS_ERR_UNSUPPORTED;
   p.tiles_x = (ow + p.Wt - 1) / p.Wt;
   p.tiles_y = (oh + p.Ht - 1) / p.Ht;
@@ -329,7 +354,7 @@ int nrs_tc_conv_wgrad(nrs_ctx* ctx, const float* x, const float* dy, float* dw, 
   p.n_tiles = (int)n_tiles;
 
   // ring depth from the shared-memory budget
-  const size_t stage_bytes = (size_t)planes * (kABlocks + p.group_cols / 32) * p.kp * 128;
+  const size_t stage_bytes = pixel_bytes * p.kp;
   int stages = (int)((200 * 1024) / stage_bytes);
   if (stages < 2) return NRS_ERR_UNSUPPORTED;
   if (stages > 6) stages = 6;
@@ -346,7 +371,7 @@ int nrs_tc_conv_wgrad(nrs_ctx* ctx, const float* x, const float* dy, float* dw, 
   // A short reduction with a large output (a Linear layer at a batch of a hundred: 7 tiles, 8 MB) is better walked by
   // one CTA per output tile, which then is the result: a split's second pass reads splits + 1 times the output at about
   // 1.1 KB a clock, and a CTA's own time is about 2 clocks per plane product, pixel and 32 columns.
-  const bool can_be_direct = taps == 1 && ci % 32 == 0 && !accumulate && !out_cols && (reinterpret_cast<uintptr_t>(dw) & 15) == 0;
+  const bool can_be_direct = taps == 1 && ci % p.wb == 0 && !accumulate && !out_cols && (reinterpret_cast<uintptr_t>(dw) & 15) == 0;
   if (can_be_direct && tps < p.n_tiles && p.n_tiles <= max_tiles) {
     const int s = (p.n_tiles + tps - 1) / tps;
     auto clocks = [&](int tiles, int splits) {
@@ -374,7 +399,7 @@ int nrs_tc_conv_wgrad(nrs_ctx* ctx, const float* x, const float* dy, float* dw, 
     dy_lo = ready->lo;
   } else {
     may_overlap = false;
-    st = nrs_ws_planes(ctx, NRS_WS_A, dy_plane * sizeof(float), split3, &dy_hi, &dy_lo);
+    st = nrs_ws_planes(ctx, NRS_WS_A, dy_plane, split3, &dy_hi, &dy_lo);
     if (st == NRS_OK) st = nrs_tc_stage_image(ctx, dy, (float*)dy_hi, (float*)dy_lo, n, co, oh * ow);
     if (st != NRS_OK) return st;
   }
@@ -383,30 +408,32 @@ int nrs_tc_conv_wgrad(nrs_ctx* ctx, const float* x, const float* dy, float* dw, 
     x_lo = ready->lo;
   } else {
     may_overlap = false;
-    st = nrs_ws_planes(ctx, NRS_WS_B, x_plane * sizeof(float), split3, &x_hi, &x_lo);
+    st = nrs_ws_planes(ctx, NRS_WS_B, x_plane, split3, &x_hi, &x_lo);
     if (st == NRS_OK) st = nrs_tc_stage_image(ctx, x, (float*)x_hi, (float*)x_lo, n, ci, h * wd);
     if (st != NRS_OK) return st;
   }
 
-  // Planes viewed as [channel block][n][h][w][32 channels], the block index outermost, so that one box brings all
+  // Planes viewed as [channel block][n][h][w][32 or 64 channels], the block index outermost, so that one box brings all
   // blocks; with a ragged channel count as [n][h][w][channels], one block per box.
   CUtensorMap maps[4];
-  p.a_box_blocks = (co + 31) / 32 < kABlocks ? (co + 31) / 32 : kABlocks;
-  auto encode = [&](CUtensorMap* m, void* base, bool ragged, int c, int ld, int img_h, int img_w, int step, int blocks) {
-    const uint64_t dim[5] = {(uint64_t)(ragged ? c : 32), (uint64_t)img_w, (uint64_t)img_h, (uint64_t)n, (uint64_t)(c / 32)};
-    const uint64_t str[4] = {(uint64_t)ld * 4, (uint64_t)img_w * ld * 4, (uint64_t)img_h * img_w * ld * 4, 128};
-    const uint32_t box[5] = {32, (uint32_t)p.Wt, (uint32_t)p.Ht, (uint32_t)p.Nt, (uint32_t)blocks};
+  p.a_box_blocks = std::min(padded(co, p.wa), 128) / p.wa;
+  auto encode = [&](CUtensorMap* m, void* base, bool ragged, int c, int w, int ld, int img_h, int img_w, int step, int blocks) {
+    const uint64_t dim[5] = {(uint64_t)(ragged ? c : w), (uint64_t)img_w, (uint64_t)img_h, (uint64_t)n, (uint64_t)(c / w)};
+    const uint64_t str[4] = {(uint64_t)ld, (uint64_t)img_w * ld, (uint64_t)img_h * img_w * ld, (uint64_t)w};
+    const uint32_t box[5] = {(uint32_t)w, (uint32_t)p.Wt, (uint32_t)p.Ht, (uint32_t)p.Nt, (uint32_t)blocks};
     const uint32_t es[5] = {1, (uint32_t)step, (uint32_t)step, 1, 1};
-    return tc::encode_tmap_f32(m, base, ragged ? 4 : 5, dim, str, box, true, es);
+    return tc::encode_tmap(m, base, split3, ragged ? 4 : 5, dim, str, box, true, es);
   };
-  const int x_blocks = p.col_blocks > 1 ? 8 : p.cblocks;
-  bool ok = encode(&maps[0], dy_hi, p.ragged_a, co, dy_ld, oh, ow, 1, p.a_box_blocks) &&
-            encode(&maps[2], x_hi, p.ragged_x, ci, x_ld, h, wd, stride, x_blocks);
-  if (split3) ok = ok && encode(&maps[1], dy_lo, p.ragged_a, co, dy_ld, oh, ow, 1, p.a_box_blocks) &&
-                   encode(&maps[3], x_lo, p.ragged_x, ci, x_ld, h, wd, stride, x_blocks);
+  const int x_blocks = p.col_blocks > 1 ? kMaxN / p.wb : p.cblocks;
+  bool ok = encode(&maps[0], dy_hi, p.ragged_a, co, p.wa, dy_ld, oh, ow, 1, p.a_box_blocks) &&
+            encode(&maps[2], x_hi, p.ragged_x, ci, p.wb, x_ld, h, wd, stride, x_blocks);
+  if (split3) ok = ok && encode(&maps[1], dy_lo, p.ragged_a, co, p.wa, dy_ld, oh, ow, 1, p.a_box_blocks) &&
+                   encode(&maps[3], x_lo, p.ragged_x, ci, p.wb, x_ld, h, wd, stride, x_blocks);
   else { maps[1] = maps[0]; maps[3] = maps[2]; }
   NRS_REQUIRE(ctx, ok, NRS_ERR_CUDA, "tc_wgrad: cuTensorMapEncodeTiled failed");
   p.independent = may_overlap ? 1 : 0;
+  p.range_dy = nrs_range_of(ctx, dy_hi);
+  p.range_x = nrs_range_of(ctx, x_hi);
 
 #define NRS_WG(PL)                                                                     \
   switch (stages) {                                                                    \
@@ -426,7 +453,7 @@ int nrs_tc_conv_wgrad(nrs_ctx* ctx, const float* x, const float* dy, float* dw, 
   j.src = p.partial; j.dst = dw;
   j.accumulate = accumulate; j.splits = splits; j.lanes = reduce_lanes(splits);
   j.co = co; j.ci = ci; j.taps = taps;
-  j.taps_per_group = p.taps_per_group; j.n_groups = p.n_groups; j.col_blocks = p.col_blocks; j.cblocks = p.cblocks;
+  j.taps_per_group = p.taps_per_group; j.n_groups = p.n_groups; j.col_blocks = p.col_blocks; j.cblocks = tap_cols / 32;
   j.group_cols = p.group_cols;
   j.out_cols = out_cols;
   j.split_stride = (size_t)p.m_blocks * p.n_groups * p.col_blocks * 128 * p.group_cols;

@@ -46,8 +46,9 @@ struct RowParams {
   int W, H, n_img;                // image geometry (dy and x have the same: pad 1, 3x3)
   int co, ci;
   int chunk, n_chunks;            // input channels per CTA (multiple of 32, <= 128) and how many chunks
-  int a_blocks;                   // 32-channel blocks of dy one box brings (min(4, co/32))
-  int pack;                       // co <= 64: accumulator rows [0,h) and [h,2h), h = 32*a_blocks, hold two
+  int wa, wb;                     // channels of a block of dy, of x: 32, or 64 (f16: rows of 128 bytes)
+  int a_blocks;                   // blocks of dy one box brings (128 channels at most)
+  int pack;                       // co <= 64: accumulator rows [0,h) and [h,2h), h = wa*a_blocks, hold two
                                   // horizontal taps (the second from a copy of the dy row shifted one pixel)
   int jtypes;                     // CTA kinds along the horizontal taps: 3, or 2 when packed
   int m_blocks;                   // ceil(co / 128)
@@ -56,6 +57,8 @@ struct RowParams {
   int SA, SX;                     // ring depths: dy rows, x rows
   int max_run;                    // vertical taps one UMMA may cover (256 / chunk, at most 3)
   float* partial;                 // [split][cta][128][3*chunk]
+  int cross;                      // 3xTF32: accumulator columns between the hi*hi sums and the others
+  const NrsRange *range_dy, *range_x;
   int independent;                // reads nothing the kernel launched just before it wrote (NRS_PDL_PROLOGUE)
 };
 
@@ -69,22 +72,22 @@ __device__ __forceinline__ bool tap_ever_valid(int i, int r0, int r1, int H) {
   return false;
 }
 
-// All UMMAs of one run of vertical taps over one image row (KS K-steps of 8 pixels).  The
+// All UMMAs of one run of vertical taps over one image row (KS K-steps of 8 pixels, of 16 in f16; 1024 B either way).  The
 // descriptors differ from step to step only in their 14-bit start-address field, so they are
 // built once (`dc`: every other field) and advanced by adding (bytes >> 4).
 template <int NPLANES, int KS>
-__device__ __forceinline__ void issue_row(uint32_t d, uint64_t dc, uint32_t a_hi16, uint32_t a_lo16, uint32_t b_hi16,
-                                          uint32_t b_lo16, uint32_t idesc, uint32_t acc_first) {
+__device__ __forceinline__ void issue_row(uint32_t d, uint32_t cross, uint64_t da, uint64_t db, uint32_t step_a, uint32_t step_b, uint32_t a_hi16,
+                                          uint32_t a_lo16, uint32_t b_hi16, uint32_t b_lo16, uint32_t idesc, uint32_t acc_first) {
 #pragma unroll
   for (int k = 0; k < KS; ++k) {
-    const uint32_t ko = (uint32_t)k * 64u;   // 1024 B per K-step
     const uint32_t acc0 = k > 0 ? 1u : acc_first;
+    const uint64_t ah = da + a_hi16 + k * step_a, bh = db + b_hi16 + k * step_b;
     if (NPLANES == 2) {
-      tc::umma_tf32(d, dc + a_lo16 + ko, dc + b_hi16 + ko, idesc, acc0);
-      tc::umma_tf32(d, dc + a_hi16 + ko, dc + b_lo16 + ko, idesc, 1);
-      tc::umma_tf32(d, dc + a_hi16 + ko, dc + b_hi16 + ko, idesc, 1);
+      tc::umma_f16(d, ah, bh, idesc, acc0);
+      tc::umma_f16(d + cross, ah, db + b_lo16 + k * step_b, idesc, acc0);
+      tc::umma_f16(d + cross, da + a_lo16 + k * step_a, bh, idesc, 1);
     } else {
-      tc::umma_tf32(d, dc + a_hi16 + ko, dc + b_hi16 + ko, idesc, acc0);
+      tc::umma_tf32(d, ah, bh, idesc, acc0);
     }
   }
 }
@@ -96,16 +99,17 @@ tc_wgrad_rows_kernel(const __grid_constant__ CUtensorMap tm_dy_hi, const __grid_
                      const RowParams p, int* __restrict__ err_flag) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  constexpr uint32_t blk = (uint32_t)KS * 8u * 128u;         // one 32-channel block of one row (W = 8*KS pixels)
-  const uint32_t a_box = (uint32_t)p.a_blocks * blk;         // one TMA box of dy
+  // one block of one row (KS K-steps of pixels)
+  const uint32_t a_blk = (uint32_t)(KS * 32 * p.wa), b_blk = (uint32_t)(KS * 32 * p.wb);
+  const uint32_t a_box = (uint32_t)p.a_blocks * a_blk;         // one TMA box of dy
   const uint32_t a_plane = (p.pack ? 2u : 1u) * a_box;       // dy row, one plane (packed: plain + shifted copy)
   const uint32_t a_slot = NPLANES * a_plane;
-  const uint32_t x_slot = (uint32_t)(p.chunk / 32) * blk;    // x row, one plane
+  const uint32_t x_slot = (uint32_t)(p.chunk / p.wb) * b_blk;   // x row, one plane
   const uint32_t x_ring = (uint32_t)p.SX * x_slot;
   uint8_t* a_base = smem;                                    // [slot][plane][block][pixel][128 B]
   uint8_t* x_base = smem + (size_t)p.SA * a_slot;            // [plane][slot][block][pixel][128 B]
-  // The UMMA reads 4 blocks of dy whatever a_blocks is: keep that inside the allocation.
-  uint64_t* full_a = reinterpret_cast<uint64_t*>(x_base + (size_t)NPLANES * x_ring + 4 * blk);
+  // The UMMA reads 128 channels of dy whatever a_blocks is: keep that inside the allocation.
+  uint64_t* full_a = reinterpret_cast<uint64_t*>(x_base + (size_t)NPLANES * x_ring + 128 / p.wa * a_blk);
   uint64_t* empty_a = full_a + p.SA;
   uint64_t* full_x = empty_a + p.SA;
   uint64_t* empty_x = full_x + p.SX;
@@ -125,7 +129,7 @@ tc_wgrad_rows_kernel(const __grid_constant__ CUtensorMap tm_dy_hi, const __grid_
   const int r0 = split * p.rows_per_split;
   const int r1 = min(p.rows_total, r0 + p.rows_per_split);
   const int nsteps = (r1 - r0) + 2;                          // two leading steps bring x rows only
-  const uint32_t tmem_cols = kTaps * p.chunk <= 128 ? 128u : (kTaps * p.chunk <= 256 ? 256u : 512u);
+  const uint32_t tmem_cols = (NPLANES == 2 ? 2u : 1u) * (kTaps * p.chunk <= 128 ? 128u : (kTaps * p.chunk <= 256 ? 256u : 512u));
 
   if (warp == 0 && lane == 0) {
     tc::prefetch_tmap(&tm_dy_hi);
@@ -165,8 +169,8 @@ tc_wgrad_rows_kernel(const __grid_constant__ CUtensorMap tm_dy_hi, const __grid_
       if (tc::elect_one()) {
         if (has_x) {
           tc::mbar_expect_tx(xbar, NPLANES * x_slot);
-          tc::tma_load_5d(x_dst, &tm_x_hi, xbar, 0, x_shift, xy, xn, cc * (p.chunk / 32));
-          if (NPLANES == 2) tc::tma_load_5d(x_dst + x_ring, &tm_x_lo, xbar, 0, x_shift, xy, xn, cc * (p.chunk / 32));
+          tc::tma_load_5d(x_dst, &tm_x_hi, xbar, 0, x_shift, xy, xn, cc * (p.chunk / p.wb));
+          if (NPLANES == 2) tc::tma_load_5d(x_dst + x_ring, &tm_x_lo, xbar, 0, x_shift, xy, xn, cc * (p.chunk / p.wb));
         } else {
           tc::mbar_arrive(xbar);
         }
@@ -178,11 +182,11 @@ tc_wgrad_rows_kernel(const __grid_constant__ CUtensorMap tm_dy_hi, const __grid_
         uint8_t* a_dst = a_base + (size_t)sa * a_slot;
         if (tc::elect_one()) {
           tc::mbar_expect_tx(abar, NPLANES * (two_taps ? 2u : 1u) * a_box);
-          tc::tma_load_5d(a_dst, &tm_dy_hi, abar, 0, 0, dyy, dn, mb * 4);
-          if (two_taps) tc::tma_load_5d(a_dst + a_box, &tm_dy_hi, abar, 0, 1, dyy, dn, mb * 4);
+          tc::tma_load_5d(a_dst, &tm_dy_hi, abar, 0, 0, dyy, dn, mb * 128 / p.wa);
+          if (two_taps) tc::tma_load_5d(a_dst + a_box, &tm_dy_hi, abar, 0, 1, dyy, dn, mb * 128 / p.wa);
           if (NPLANES == 2) {
-            tc::tma_load_5d(a_dst + a_plane, &tm_dy_lo, abar, 0, 0, dyy, dn, mb * 4);
-            if (two_taps) tc::tma_load_5d(a_dst + a_plane + a_box, &tm_dy_lo, abar, 0, 1, dyy, dn, mb * 4);
+            tc::tma_load_5d(a_dst + a_plane, &tm_dy_lo, abar, 0, 0, dyy, dn, mb * 128 / p.wa);
+            if (two_taps) tc::tma_load_5d(a_dst + a_plane + a_box, &tm_dy_lo, abar, 0, 1, dyy, dn, mb * 128 / p.wa);
           }
         }
         __syncwarp();
@@ -207,11 +211,15 @@ tc_wgrad_rows_kernel(const __grid_constant__ CUtensorMap tm_dy_hi, const __grid_
     // ---------------- UMMA issuer
     bool ok = true;
     uint32_t started = 0;   // bit i: vertical tap i's accumulator columns hold a sum already
-    const uint64_t dc = tc::make_smem_desc_sw128_32b(0, blk, 512);
+    auto desc = [](int w, uint32_t blk) {
+      return NPLANES == 1 ? tc::make_smem_desc_sw128_32b(0, blk, 512) : w == 64 ? tc::make_smem_desc_sw128(0, blk, 1024) : tc::make_smem_desc_sw64(0, blk, 512);
+    };
+    const uint64_t da = desc(p.wa, a_blk), db = desc(p.wb, b_blk);
+    const uint32_t step_a = p.wa == 64 ? 128u : 64u, step_b = p.wb == 64 ? 128u : 64u;
     const uint32_t a_base16 = tc::smem_u32(a_base) >> 4, x_base16 = tc::smem_u32(x_base) >> 4;
     const uint32_t a_slot16 = a_slot >> 4, a_plane16 = a_plane >> 4, x_slot16 = x_slot >> 4, x_ring16 = x_ring >> 4;
     // instruction descriptor of a run of `len` taps: N = len * chunk sits in bits [17,23) as N >> 3
-    const uint32_t idesc_n0 = tc::make_idesc_tf32(128, 0, true, true);
+    const uint32_t idesc_n0 = NPLANES == 2 ? tc::make_idesc_f16(128, 0, true, true) : tc::make_idesc_tf32(128, 0, true, true);
     const uint32_t idesc_per_tap = (uint32_t)(p.chunk >> 3) << 17;
     int sx = 0, sa = 0;
     uint32_t phx = 0, pha = 0;
@@ -237,7 +245,7 @@ tc_wgrad_rows_kernel(const __grid_constant__ CUtensorMap tm_dy_hi, const __grid_
           const uint32_t b_hi16 = x_base16 + (uint32_t)s0 * x_slot16;
           const uint32_t acc = (started >> i) & 1u, idesc = idesc_n0 + (uint32_t)len * idesc_per_tap;
           if (tc::elect_one())
-            issue_row<NPLANES, KS>(tmem_base + (uint32_t)(i * p.chunk), dc, a_hi16, a_lo16, b_hi16, b_hi16 + x_ring16, idesc, acc);
+            issue_row<NPLANES, KS>(tmem_base + (uint32_t)(i * p.chunk), (uint32_t)p.cross, da, db, step_a, step_b, a_hi16, a_lo16, b_hi16, b_hi16 + x_ring16, idesc, acc);
           __syncwarp();
           started |= ((1u << len) - 1u) << i;
           i += len;
@@ -266,15 +274,25 @@ tc_wgrad_rows_kernel(const __grid_constant__ CUtensorMap tm_dy_hi, const __grid_
       const int cols = kTaps * p.chunk;
       float* dst = p.partial + (((size_t)split * gridDim.x + blockIdx.x) * 128 + row) * cols;
       // packed: rows [0,h) are tap j = 1 or 2, rows [h,2h) tap j = 0 (kind 0 only)
-      const int half = 32 * p.a_blocks;
+      const int half = p.wa * p.a_blocks;
       const bool row_live = p.pack ? (row < half || (two_taps && row < 2 * half)) : (mb * 128 + row < p.co);
       uint32_t valid = 0;
       for (int i = 0; i < kTaps; ++i) valid |= tap_ever_valid(i, r0, r1, p.H) ? (1u << i) : 0u;
+      const pr::Unscale unscale(NPLANES == 2 ? p.range_dy->bound : 1.0f, NPLANES == 2 ? p.range_x->bound : 1.0f);
 #pragma unroll 1
       for (int c = 0; c < cols / 32; ++c) {
         uint32_t r[32];
-        tc::tmem_ld_32x32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(c * 32), r);
-        tc::tmem_ld_wait();
+        const uint32_t at = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(c * 32);
+        tc::tmem_ld_32x32(at, r);
+        if constexpr (NPLANES == 2) {
+          uint32_t x[32];
+          tc::tmem_ld_32x32(at + (uint32_t)p.cross, x);
+          tc::tmem_ld_wait();
+#pragma unroll
+          for (int e = 0; e < 32; ++e) r[e] = __float_as_uint(unscale(__uint_as_float(r[e]), __uint_as_float(x[e])));
+        } else {
+          tc::tmem_ld_wait();
+        }
         const bool live = (valid >> ((c * 32) / p.chunk)) & 1u;
         if (row_live) {
 #pragma unroll
@@ -327,9 +345,13 @@ int nrs_tc_conv_wgrad_rows(nrs_ctx* ctx, const float* x, const float* dy, float*
 
   RowParams p{};
   p.W = wd; p.H = h; p.n_img = n; p.co = co; p.ci = ci;
-  p.chunk = ci % 128 == 0 ? 128 : (ci <= 128 ? ci : (ci % 96 == 0 ? 96 : (ci % 64 == 0 ? 64 : 32)));
+  // (f16 pairs: two accumulators of 3 * chunk columns each in 512)
+  p.chunk = split3 ? (ci % 64 == 0 ? 64 : 32) : ci % 128 == 0 ? 128 : (ci <= 128 ? ci : (ci % 96 == 0 ? 96 : (ci % 64 == 0 ? 64 : 32)));
+  p.cross = kTaps * p.chunk <= 128 ? 128 : 256;
   p.n_chunks = ci / p.chunk;
-  p.a_blocks = co / 32 < 4 ? co / 32 : 4;
+  p.wa = split3 && co % 64 == 0 ? 64 : 32;
+  p.wb = split3 && ci % 64 == 0 ? 64 : 32;
+  p.a_blocks = (co < 128 ? co : 128) / p.wa;
   p.pack = co <= 64 ? 1 : 0;
   p.jtypes = p.pack ? 2 : 3;
   p.m_blocks = (co + 127) / 128;
@@ -337,15 +359,14 @@ int nrs_tc_conv_wgrad_rows(nrs_ctx* ctx, const float* x, const float* dy, float*
   p.max_run = 256 / p.chunk < kTaps ? 256 / p.chunk : kTaps;
 
   // ring depths: a dy row lives one step, an x row three; d rows of prefetch on top of that
-  const size_t blk = (size_t)wd * 128;
-  const size_t a_slot = (size_t)planes * (p.pack ? 2 : 1) * p.a_blocks * blk, x_slot = (size_t)planes * (p.chunk / 32) * blk;
+  const size_t a_slot = (size_t)(p.pack ? 2 : 1) * p.a_blocks * p.wa * wd * 4, x_slot = (size_t)p.chunk * wd * 4;   // all planes
   const long budget = 200 * 1024;
   long d = (budget - 3 * (long)x_slot - (long)a_slot) / (long)(x_slot + a_slot);
   if (d > 8) d = 8;
   if (d < 1) return NRS_ERR_UNSUPPORTED;
   p.SA = 1 + (int)d;
   p.SX = 3 + (int)d;
-  const size_t smem_bytes = p.SA * a_slot + p.SX * x_slot + 4 * blk + (size_t)(2 * (p.SA + p.SX) + 1) * 8 + 16 + 1024;
+  const size_t smem_bytes = p.SA * a_slot + p.SX * x_slot + (size_t)128 * wd * 4 / planes + (size_t)(2 * (p.SA + p.SX) + 1) * 8 + 16 + 1024;
   if (smem_bytes > 227 * 1024) return NRS_ERR_UNSUPPORTED;
 
   // row split: fill the GPU, bound the accumulation chain in 3xTF32 mode, amortise the partial tile
@@ -371,7 +392,7 @@ int nrs_tc_conv_wgrad_rows(nrs_ctx* ctx, const float* x, const float* dy, float*
     dy_lo = ready->lo;
   } else {
     may_overlap = false;
-    st = nrs_ws_planes(ctx, NRS_WS_A, dy_plane * sizeof(float), split3, &dy_hi, &dy_lo);
+    st = nrs_ws_planes(ctx, NRS_WS_A, dy_plane, split3, &dy_hi, &dy_lo);
     if (st == NRS_OK) st = nrs_tc_stage(ctx, dy, (float*)dy_hi, (float*)dy_lo, h * wd, co, co, n, dy_img, dy_img, true);
     if (st != NRS_OK) return st;
   }
@@ -380,29 +401,31 @@ int nrs_tc_conv_wgrad_rows(nrs_ctx* ctx, const float* x, const float* dy, float*
     x_lo = ready->lo;
   } else {
     may_overlap = false;
-    st = nrs_ws_planes(ctx, NRS_WS_B, x_plane * sizeof(float), split3, &x_hi, &x_lo);
+    st = nrs_ws_planes(ctx, NRS_WS_B, x_plane, split3, &x_hi, &x_lo);
     if (st == NRS_OK) st = nrs_tc_stage(ctx, x, (float*)x_hi, (float*)x_lo, h * wd, ci, ci, n, x_img, x_img, true);
     if (st != NRS_OK) return st;
   }
 
   // planes viewed as [channel block][n][h][w][32 channels]; a box is one image row of some blocks
   CUtensorMap maps[4];
-  const uint64_t ddim[5] = {32, (uint64_t)wd, (uint64_t)h, (uint64_t)n, (uint64_t)(co / 32)};
-  const uint64_t dstr[4] = {(uint64_t)co * 4, (uint64_t)wd * co * 4, (uint64_t)h * wd * co * 4, 128};
-  const uint64_t xdim[5] = {32, (uint64_t)wd, (uint64_t)h, (uint64_t)n, (uint64_t)(ci / 32)};
-  const uint64_t xstr[4] = {(uint64_t)ci * 4, (uint64_t)wd * ci * 4, (uint64_t)h * wd * ci * 4, 128};
-  const uint32_t dbox[5] = {32, (uint32_t)wd, 1, 1, (uint32_t)p.a_blocks};
-  const uint32_t xbox[5] = {32, (uint32_t)wd, 1, 1, (uint32_t)(p.chunk / 32)};
-  bool ok = tc::encode_tmap_f32(&maps[0], dy_hi, 5, ddim, dstr, dbox, true) && tc::encode_tmap_f32(&maps[2], x_hi, 5, xdim, xstr, xbox, true);
-  if (split3) ok = ok && tc::encode_tmap_f32(&maps[1], dy_lo, 5, ddim, dstr, dbox, true) && tc::encode_tmap_f32(&maps[3], x_lo, 5, xdim, xstr, xbox, true);
+  const uint64_t ddim[5] = {(uint64_t)p.wa, (uint64_t)wd, (uint64_t)h, (uint64_t)n, (uint64_t)(co / p.wa)};
+  const uint64_t dstr[4] = {(uint64_t)co, (uint64_t)wd * co, (uint64_t)h * wd * co, (uint64_t)p.wa};
+  const uint64_t xdim[5] = {(uint64_t)p.wb, (uint64_t)wd, (uint64_t)h, (uint64_t)n, (uint64_t)(ci / p.wb)};
+  const uint64_t xstr[4] = {(uint64_t)ci, (uint64_t)wd * ci, (uint64_t)h * wd * ci, (uint64_t)p.wb};
+  const uint32_t dbox[5] = {(uint32_t)p.wa, (uint32_t)wd, 1, 1, (uint32_t)p.a_blocks};
+  const uint32_t xbox[5] = {(uint32_t)p.wb, (uint32_t)wd, 1, 1, (uint32_t)(p.chunk / p.wb)};
+  bool ok = tc::encode_tmap(&maps[0], dy_hi, split3, 5, ddim, dstr, dbox, true) && tc::encode_tmap(&maps[2], x_hi, split3, 5, xdim, xstr, xbox, true);
+  if (split3) ok = ok && tc::encode_tmap(&maps[1], dy_lo, true, 5, ddim, dstr, dbox, true) && tc::encode_tmap(&maps[3], x_lo, true, 5, xdim, xstr, xbox, true);
   else { maps[1] = maps[0]; maps[3] = maps[2]; }
   NRS_REQUIRE(ctx, ok, NRS_ERR_CUDA, "tc_wgrad_rows: cuTensorMapEncodeTiled failed");
   p.independent = may_overlap ? 1 : 0;
+  p.range_dy = nrs_range_of(ctx, dy_hi);
+  p.range_x = nrs_range_of(ctx, x_hi);
 
-  switch (wd / 8) {
-    case 2: st = split3 ? launch_rows<2, 2>(ctx, maps, p, ctas, splits, smem_bytes) : launch_rows<1, 2>(ctx, maps, p, ctas, splits, smem_bytes); break;
-    case 4: st = split3 ? launch_rows<2, 4>(ctx, maps, p, ctas, splits, smem_bytes) : launch_rows<1, 4>(ctx, maps, p, ctas, splits, smem_bytes); break;
-    default: st = split3 ? launch_rows<2, 8>(ctx, maps, p, ctas, splits, smem_bytes) : launch_rows<1, 8>(ctx, maps, p, ctas, splits, smem_bytes); break;
+  switch (wd / 16) {
+    case 1: st = split3 ? launch_rows<2, 1>(ctx, maps, p, ctas, splits, smem_bytes) : launch_rows<1, 2>(ctx, maps, p, ctas, splits, smem_bytes); break;
+    case 2: st = split3 ? launch_rows<2, 2>(ctx, maps, p, ctas, splits, smem_bytes) : launch_rows<1, 4>(ctx, maps, p, ctas, splits, smem_bytes); break;
+    default: st = split3 ? launch_rows<2, 4>(ctx, maps, p, ctas, splits, smem_bytes) : launch_rows<1, 8>(ctx, maps, p, ctas, splits, smem_bytes); break;
   }
   if (st != NRS_OK) return st;
   // dw[co][ci][i][j] (+)= sum over splits of the partial accumulators
@@ -411,7 +434,7 @@ int nrs_tc_conv_wgrad_rows(nrs_ctx* ctx, const float* x, const float* dy, float*
   jb.src = p.partial; jb.dst = dw;
   jb.accumulate = accumulate; jb.splits = splits; jb.lanes = reduce_lanes(splits);
   jb.co = co; jb.ci = ci; jb.taps = 9;
-  jb.chunk = p.chunk; jb.n_chunks = p.n_chunks; jb.jtypes = p.jtypes; jb.a_blocks = p.a_blocks; jb.pack = p.pack;
+  jb.chunk = p.chunk; jb.n_chunks = p.n_chunks; jb.jtypes = p.jtypes; jb.a_blocks = p.a_blocks * p.wa / 32; jb.pack = p.pack;
   jb.split_stride = (size_t)ctas * 128 * kTaps * p.chunk;
   return nrs_fold_submit(ctx, jb);
 }

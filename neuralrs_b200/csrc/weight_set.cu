@@ -1,7 +1,7 @@
 // Batched staging of a model's weights for the tensor-core kernels.
 //
-// Every contraction reads its weight operand as K-major TF32 planes (a high plane rounded to nearest
-// and, for 3xTF32, an f32 residual plane), re-laid out per use: convolution forward and data gradient
+// Every contraction reads its weight operand as K-major planes (values rounded to TF32 or, for 3xTF32,
+// f16 pairs), re-laid out per use: convolution forward and data gradient
 // want two different tap-major layouts, x@W wants W transposed, dz@W^T wants W as stored.  Staged per
 // call that is one small launch per layer and pass; a training loop knows all its weights in advance,
 // so they are staged here in ONE launch per step from a job table resident on the device, and the
@@ -20,6 +20,9 @@ struct WeightJob {
   int rows, cols;        // as stored, [rows][cols]; a convolution's [co][ci][taps]
   int taps;
   unsigned first_block;  // this job's first block in the launch
+  // 3xTF32: the range its planes share with those of its group, and the blocks that measure it
+  NrsRange* range;
+  unsigned first_scan, group_scans;
 };
 
 constexpr int kTile = 64;          // linear: 64 x 64 values per block
@@ -34,32 +37,78 @@ inline unsigned job_blocks(const WeightJob& j) {
   return (unsigned)ceil_div(j.rows, kTile) * ceil_div(j.cols, kTile);
 }
 
-__device__ __forceinline__ void put(float* hi, float* lo, size_t i, float v) {
-  const float h = tc::tf32_rn(v);
-  hi[i] = h;
-  if (lo) lo[i] = v - h;
+template <bool SPLIT>
+__device__ __forceinline__ void put(float* hi, float* lo, size_t i, float v, float scale) {
+  if (SPLIT) pr::put(hi, lo, i, v, scale);
+  else hi[i] = tc::tf32_rn(v);
 }
-__device__ __forceinline__ void put4(float* hi, float* lo, size_t i, float4 v) {
-  const float4 h = make_float4(tc::tf32_rn(v.x), tc::tf32_rn(v.y), tc::tf32_rn(v.z), tc::tf32_rn(v.w));
-  *reinterpret_cast<float4*>(hi + i) = h;
-  if (lo) *reinterpret_cast<float4*>(lo + i) = make_float4(v.x - h.x, v.y - h.y, v.z - h.z, v.w - h.w);
+template <bool SPLIT>
+__device__ __forceinline__ void put4(float* hi, float* lo, size_t i, float4 v, float scale) {
+  if (SPLIT) pr::put4(hi, lo, i, v, scale);
+  else *reinterpret_cast<float4*>(hi + i) = make_float4(tc::tf32_rn(v.x), tc::tf32_rn(v.y), tc::tf32_rn(v.z), tc::tf32_rn(v.w));
 }
 
-// HBM / L2-bound: 4 B read and 8 B (TF32: 4) written per value and form.  A block takes a tile that both forms want in
+__device__ __forceinline__ int job_of(const WeightJob* jobs, int n_jobs, unsigned bid, unsigned WeightJob::*first) {
+  int lo = 0, hi = n_jobs - 1;   // the last one whose first block <= bid
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (jobs[mid].*first <= bid) lo = mid; else hi = mid - 1;
+  }
+  return lo;
+}
+
+constexpr int kScan = 8192;   // values per block
+inline unsigned job_scans(const WeightJob& j) { return (unsigned)(((size_t)j.rows * j.cols * j.taps + kScan - 1) / kScan); }
+
+// The largest magnitude of every weight (group), for its planes' exponent.  L2-bound: the optimizer has just written them.
+// A group's last block to arrive turns what all of them left in the range's scratch words into the range, and clears those.
+__global__ void __launch_bounds__(256)
+weight_scan_kernel(const WeightJob* __restrict__ jobs, int n_jobs, unsigned scan_offset) {
+  NRS_PDL_PROLOGUE();
+  __shared__ uint32_t part[8];
+  const unsigned bid = blockIdx.x + scan_offset;
+  const WeightJob j = jobs[job_of(jobs, n_jobs, bid, &WeightJob::first_scan)];
+  const size_t count = (size_t)j.rows * j.cols * j.taps, begin = (size_t)(bid - j.first_scan) * kScan;
+  const int n = (int)min((size_t)kScan, count - begin);
+  const float* src = j.src + begin;
+  uint32_t top = 0;
+  if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+#pragma unroll
+    for (int u = 0; u < kScan / 1024; ++u) {
+      const int i = 4 * (int)threadIdx.x + 1024 * u;
+      if (i + 3 < n) top = pr::seen4(top, *reinterpret_cast<const float4*>(src + i));
+      else
+        for (int e = i; e < n; ++e) top = pr::seen(top, src[e]);
+    }
+  } else {
+    for (int i = threadIdx.x; i < n; i += 256) top = pr::seen(top, src[i]);
+  }
+  top = __reduce_max_sync(0xffffffffu, top);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = top;
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  for (int w = 1; w < 8; ++w) top = max(top, part[w]);
+  unsigned* scratch = reinterpret_cast<unsigned*>(j.range->pad);   // largest so far; blocks that have arrived
+  atomicMax(&scratch[0], top);
+  __threadfence();
+  if (atomicAdd(&scratch[1], 1u) + 1u != j.group_scans) return;
+  __threadfence();
+  const float bound = __uint_as_float(atomicExch(&scratch[0], 0u));
+  scratch[1] = 0;
+  j.range->bound = j.range->top = bound;
+}
+
+// HBM / L2-bound: 4 B read and 4 B written per value and form.  A block takes a tile that both forms want in
 // runs of whole sectors and turns it in shared memory.
+template <bool SPLIT>
 __global__ void __launch_bounds__(256)
 weight_stage_batch_kernel(const WeightJob* __restrict__ jobs, int n_jobs, unsigned block_offset) {
   NRS_PDL_PROLOGUE();
   constexpr int kPitch = kConvCi * kConvTaps + 1;
   __shared__ float tile[kConvCo * kPitch > kTile * (kTile + 1) ? kConvCo * kPitch : kTile * (kTile + 1)];
-  // the job this block belongs to: the last one whose first_block <= its index in the full launch
   const unsigned bid = blockIdx.x + block_offset;
-  int lo_j = 0, hi_j = n_jobs - 1;
-  while (lo_j < hi_j) {
-    const int mid = (lo_j + hi_j + 1) >> 1;
-    if (jobs[mid].first_block <= bid) lo_j = mid; else hi_j = mid - 1;
-  }
-  const WeightJob j = jobs[lo_j];
+  const WeightJob j = jobs[job_of(jobs, n_jobs, bid, &WeightJob::first_block)];
+  const float scale = SPLIT ? pr::scale_of(j.range->bound) : 1.0f;
   const int blk = (int)(bid - j.first_block);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (!j.conv) {
@@ -75,7 +124,7 @@ weight_stage_batch_kernel(const WeightJob* __restrict__ jobs, int n_jobs, unsign
         const float* s = j.src + (size_t)r * j.cols + c;
         if (j.vec && c < j.cols) v = *reinterpret_cast<const float4*>(s);
         else if (!j.vec) v = make_float4(c < j.cols ? s[0] : 0.f, c + 1 < j.cols ? s[1] : 0.f, c + 2 < j.cols ? s[2] : 0.f, c + 3 < j.cols ? s[3] : 0.f);
-        if (j.b_hi && c < ld_b) put4(j.b_hi, j.b_lo, (size_t)r * ld_b + c, v);
+        if (j.b_hi && c < ld_b) put4<SPLIT>(j.b_hi, j.b_lo, (size_t)r * ld_b + c, v, scale);
       }
       float* t = tile + rr * (kTile + 1) + cq;
       t[0] = v.x; t[1] = v.y; t[2] = v.z; t[3] = v.w;
@@ -88,7 +137,7 @@ weight_stage_batch_kernel(const WeightJob* __restrict__ jobs, int n_jobs, unsign
       const int rr = kq + 32 * (i & 1), cc = warp * 4 + (lane >> 3) + 32 * (i >> 1);
       if (c0 + cc >= j.cols || r0 + rr >= ld_a) continue;
       const float* t = tile + rr * (kTile + 1) + cc;
-      put4(j.a_hi, j.a_lo, (size_t)(c0 + cc) * ld_a + r0 + rr, make_float4(t[0], t[kTile + 1], t[2 * (kTile + 1)], t[3 * (kTile + 1)]));
+      put4<SPLIT>(j.a_hi, j.a_lo, (size_t)(c0 + cc) * ld_a + r0 + rr, make_float4(t[0], t[kTile + 1], t[2 * (kTile + 1)], t[3 * (kTile + 1)]), scale);
     }
     return;
   }
@@ -119,7 +168,7 @@ weight_stage_batch_kernel(const WeightJob* __restrict__ jobs, int n_jobs, unsign
     for (int o = warp; o < nco; o += 8)
 #pragma unroll
       for (int t = 0; t < kConvTaps; ++t)
-        if (t < nt) put(j.a_hi, j.a_lo, ((size_t)(co0 + o) * j.taps + t0 + t) * ld + ci0 + lane, tile[o * kPitch + lane * nt + t]);
+        if (t < nt) put<SPLIT>(j.a_hi, j.a_lo, ((size_t)(co0 + o) * j.taps + t0 + t) * ld + ci0 + lane, tile[o * kPitch + lane * nt + t], scale);
   }
   if (j.b_hi) {
     const int ld = ceil32(j.rows), o = lane & 15;
@@ -127,12 +176,12 @@ weight_stage_batch_kernel(const WeightJob* __restrict__ jobs, int n_jobs, unsign
 #pragma unroll
       for (int t2 = 0; t2 < kConvTaps; t2 += 2) {   // the two halves of a warp take neighbouring taps
         const int t = t2 + (lane >> 4);
-        if (t < nt) put(j.b_hi, j.b_lo, ((size_t)(ci0 + i) * j.taps + t0 + t) * ld + co0 + o, tile[o * kPitch + i * nt + t]);
+        if (t < nt) put<SPLIT>(j.b_hi, j.b_lo, ((size_t)(ci0 + i) * j.taps + t0 + t) * ld + co0 + o, tile[o * kPitch + i * nt + t], scale);
       }
   }
 }
 
-size_t plane_floats(const NrsWeightDesc& d) {
+size_t plane_values(const NrsWeightDesc& d) {
   if (d.form == NRS_WF_LINEAR_ROWS || d.form == NRS_WF_LINEAR_T) return (size_t)d.rows * ceil32(d.K);
   return d.form == NRS_WF_CONV_FWD ? (size_t)d.co * ceil32(d.ci) * d.taps : (size_t)d.ci * ceil32(d.co) * d.taps;
 }
@@ -144,6 +193,7 @@ void nrs_weight_set_clear(nrs_ctx* ctx) {
   if (ws.storage || ws.jobs_dev) cudaStreamSynchronize(ctx->stream);
   if (ws.storage) cudaFree(ws.storage);
   if (ws.jobs_dev) cudaFree(ws.jobs_dev);
+  if (ws.ranges) nrs_free(ctx, ws.ranges);
   ws = NrsWeightSet();
 }
 
@@ -153,18 +203,20 @@ int nrs_weight_set_build(nrs_ctx* ctx, const NrsWeightDesc* descs, int count) {
   NrsWeightSet& ws = ctx->weight_set;
   const bool split = ctx->math_mode == NRS_MATH_3XTF32;
   size_t total = 0;
-  for (int i = 0; i < count; ++i) total += (plane_floats(descs[i]) + 63) / 64 * 64 * (split ? 2 : 1);
-  const int got = nrs_device_alloc(ctx, "weight planes", total * sizeof(float), &ws.storage);
+  for (int i = 0; i < count; ++i) total += (plane_values(descs[i]) + 63) / 64 * 64 * sizeof(float);
+  int got = nrs_device_alloc(ctx, "weight planes", total, &ws.storage);
+  if (got == NRS_OK && split) got = nrs_alloc(ctx, count * sizeof(NrsRange), 1, (void**)&ws.ranges);   // (one per job at most)
   if (got != NRS_OK) return got;
   std::vector<WeightJob> jobs;
-  float* cursor = (float*)ws.storage;
+  std::vector<int> groups;   // per job
+  uint8_t* cursor = (uint8_t*)ws.storage;
   for (int i = 0; i < count; ++i) {
     const NrsWeightDesc& d = descs[i];
-    const size_t n = (plane_floats(d) + 63) / 64 * 64;
-    float* hi = cursor;
-    cursor += n;
-    float* lo = split ? cursor : nullptr;
-    if (split) cursor += n;
+    const size_t n = (plane_values(d) + 63) / 64 * 64;
+    float* hi = (float*)cursor;
+    cursor += n * (split ? 2 : 4);
+    float* lo = split ? (float*)cursor : nullptr;
+    if (split) cursor += n * 2;
     const bool conv = d.form == NRS_WF_CONV_FWD || d.form == NRS_WF_CONV_DGRAD, a = d.form == NRS_WF_CONV_FWD || d.form == NRS_WF_LINEAR_T;
     const int rows = conv ? d.co : a ? d.K : d.rows, cols = conv ? d.ci : a ? d.rows : d.K, taps = conv ? d.taps : 1;
     // the other form of a weight already met joins its job
@@ -177,17 +229,28 @@ int nrs_weight_set_build(nrs_ctx* ctx, const NrsWeightDesc* descs, int count) {
       j.conv = conv;
       j.vec = cols % 4 == 0 && (reinterpret_cast<uintptr_t>(d.w) & 15) == 0;
       j.rows = rows; j.cols = cols; j.taps = taps;
+      j.range = ws.ranges;
+      if (split && !jobs.empty()) j.range = jobs.back().range + (d.group != 0 && d.group == groups.back() ? 0 : 1);
+      groups.push_back(d.group);
       jobs.push_back(j);
       job = &jobs.back();
     }
     (a ? job->a_hi : job->b_hi) = hi;
     (a ? job->a_lo : job->b_lo) = lo;
-    ws.planes[std::make_pair((const void*)d.w, d.form)] = NrsWeightPlanes{hi, lo, d.rows, d.K, d.co, d.ci, d.taps};
+    ws.planes[std::make_pair((const void*)d.w, d.form)] = NrsWeightPlanes{hi, lo, job->range, d.rows, d.K, d.co, d.ci, d.taps};
   }
-  unsigned block = 0;
+  unsigned block = 0, scan = 0;
+  for (size_t i = 0, e; i < jobs.size(); i = e) {
+    unsigned total_scans = 0;
+    for (e = i; e < jobs.size() && (e == i || (split && jobs[e].range == jobs[i].range)); ++e) total_scans += job_scans(jobs[e]);
+    for (size_t k = i; k < e; ++k) { jobs[k].group_scans = total_scans; ws.job_group.push_back((int)i); }
+  }
   for (WeightJob& j : jobs) {
     j.first_block = block;
+    j.first_scan = scan;
     block += job_blocks(j);
+    scan += job_scans(j);
+    ws.job_scan.push_back(j.first_scan);
     ws.job_src.push_back(j.src);
     ws.job_first.push_back(j.first_block);
   }
@@ -202,16 +265,35 @@ int nrs_weight_set_build(nrs_ctx* ctx, const NrsWeightDesc* descs, int count) {
   ws.n_jobs = (int)jobs.size();
   ws.blocks = block;
   ws.job_first.push_back(block);
+  ws.job_scan.push_back(scan);
+  ws.job_group.push_back((int)jobs.size());
   ws.split = split;
   ws.fresh = false;
+  return NRS_OK;
+}
+
+// Jobs [first, last), whole groups.
+static int refresh_jobs(nrs_ctx* ctx, int first, int last) {
+  NrsWeightSet& ws = ctx->weight_set;
+  const unsigned block = ws.job_first[first], blocks = ws.job_first[last] - block, scan = ws.job_scan[first], scans = ws.job_scan[last] - scan;
+  if (blocks == 0) return NRS_OK;
+  const WeightJob* jobs = (const WeightJob*)ws.jobs_dev;
+  if (ws.split) {
+    NRS_PDL_LAUNCH(weight_scan_kernel, scans, 256, 0, ctx->stream, jobs, ws.n_jobs, scan);
+    NRS_LAUNCHED(ctx);
+    NRS_PDL_LAUNCH((weight_stage_batch_kernel<true>), blocks, 256, 0, ctx->stream, jobs, ws.n_jobs, block);
+  } else {
+    NRS_PDL_LAUNCH((weight_stage_batch_kernel<false>), blocks, 256, 0, ctx->stream, jobs, ws.n_jobs, block);
+  }
+  NRS_LAUNCHED(ctx);
   return NRS_OK;
 }
 
 int nrs_weight_set_refresh(nrs_ctx* ctx) {
   NrsWeightSet& ws = ctx->weight_set;
   if (ws.n_jobs == 0) return NRS_OK;
-  NRS_PDL_LAUNCH(weight_stage_batch_kernel, ws.blocks, 256, 0, ctx->stream, (const WeightJob*)ws.jobs_dev, ws.n_jobs, 0u);
-  NRS_LAUNCHED(ctx);
+  const int st = refresh_jobs(ctx, 0, ws.n_jobs);
+  if (st != NRS_OK) return st;
   ws.fresh = true;
   ws.refreshed_jobs = 0;
   return NRS_OK;
@@ -220,17 +302,16 @@ int nrs_weight_set_refresh(nrs_ctx* ctx) {
 int nrs_weight_set_refresh_range(nrs_ctx* ctx, const float* lo, const float* hi) {
   NrsWeightSet& ws = ctx->weight_set;
   // one launch per run of consecutive jobs whose weight lies in the range (jobs follow the layer order, so
-  // a bucket of adjacent parameters is one run)
+  // a bucket of adjacent parameters is one run); what shares its range with one of them is restaged too
   int j = 0;
   while (j < ws.n_jobs) {
     if (ws.job_src[j] < lo || ws.job_src[j] >= hi) { ++j; continue; }
     int e = j;
     while (e < ws.n_jobs && ws.job_src[e] >= lo && ws.job_src[e] < hi) ++e;
-    const unsigned first = ws.job_first[j], count = ws.job_first[e] - first;
-    if (count > 0) {
-      NRS_PDL_LAUNCH(weight_stage_batch_kernel, count, 256, 0, ctx->stream, (const WeightJob*)ws.jobs_dev, ws.n_jobs, first);
-      NRS_LAUNCHED(ctx);
-    }
+    int first = ws.job_group[j], last = e;
+    while (last < ws.n_jobs && ws.job_group[last] == ws.job_group[e - 1]) ++last;
+    const int st = refresh_jobs(ctx, first, last);
+    if (st != NRS_OK) return st;
     ws.refreshed_jobs += e - j;
     j = e;
   }
