@@ -611,7 +611,7 @@ int bn_forward(nrs_ctx* ctx, const char* who, const float* x, const float* gamma
 int bn_backward(nrs_ctx* ctx, const char* who, const float* g, const float* xhat, const float* istd, const float* gamma,
                 const float* beta, float* dx, float* dgamma, float* dbeta, int n, int c, int hw, int training,
                 int accumulate_dx, int accumulate_params, bool relu, const float* mean = nullptr /* xhat is x then */,
-                float* hi = nullptr, float* lo = nullptr, float* chan_partial = nullptr) {
+                float* hi = nullptr, float* lo = nullptr, float* chan_partial = nullptr, const NrsRange* known_g = nullptr) {
   NRS_REQUIRE_CTX(ctx);
   NRS_REQUIRE(ctx, check_dims(n, c, hw), NRS_ERR_SHAPE, "%s: bad shape [%d,%d,%d]", who, n, c, hw);
   NRS_REQUIRE(ctx, (dgamma == nullptr) == (dbeta == nullptr), NRS_ERR_ARG, "%s: dgamma and dbeta must be given together", who);
@@ -656,10 +656,10 @@ int bn_backward(nrs_ctx* ctx, const char* who, const float* g, const float* xhat
     NrsRange *range = nullptr, *range_g = nullptr;
     if (lo) {
       int rs = nrs_range_renew(ctx, hi, &range);
-      if (rs == NRS_OK) rs = nrs_range_renew(ctx, &ctx->scratch_range[0], &range_g);
-      if (rs == NRS_OK) rs = nrs_absmax(ctx, g, (size_t)n * c * hw, range_g);
+      if (rs == NRS_OK && !known_g) rs = nrs_range_renew(ctx, &ctx->scratch_range[0], &range_g);
+      if (rs == NRS_OK && !known_g) rs = nrs_absmax(ctx, g, (size_t)n * c * hw, range_g);
       if (rs != NRS_OK) return rs;
-      NRS_PDL_LAUNCH(bn_dx_bound_kernel, 1, 256, 0, ctx->stream, gamma, istd, (const float2*)sums, (const NrsRange*)range_g, count, training,
+      NRS_PDL_LAUNCH(bn_dx_bound_kernel, 1, 256, 0, ctx->stream, gamma, istd, (const float2*)sums, known_g ? known_g : (const NrsRange*)range_g, count, training,
                      shared ? (const float*)count_slot : (const float*)nullptr, range, c);
       NRS_LAUNCHED(ctx);
     }
@@ -731,9 +731,9 @@ int nrs_batchnorm_fwd_saving_mean(nrs_ctx* ctx, const float* x, const float* gam
 
 int nrs_batchnorm_bwd_from_x(nrs_ctx* ctx, const float* g, const float* x, const float* mean, const float* istd, const float* gamma,
                              const float* beta, float* dx, float* dgamma, float* dbeta, int n, int c, int hw, int training, int accumulate_dx,
-                             int accumulate_params, int act, float* hi, float* lo, float* chan_partial) {
+                             int accumulate_params, int act, float* hi, float* lo, float* chan_partial, const NrsRange* range_g) {
   return bn_backward(ctx, "batchnorm backward", g, x, istd, gamma, beta, dx, dgamma, dbeta, n, c, hw, training, accumulate_dx, accumulate_params,
-                     act == NRS_ACT_RELU, mean, hi, lo, chan_partial);
+                     act == NRS_ACT_RELU, mean, hi, lo, chan_partial, range_g);
 }
 
 int nrs_batchnorm_tiles(int n, int hw) { return (int)(((size_t)n * hw + img::kTilePx - 1) / img::kTilePx); }

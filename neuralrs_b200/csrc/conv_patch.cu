@@ -24,10 +24,9 @@ constexpr int kMaxPatch = 128;
 template <bool SPLIT>
 __global__ void __launch_bounds__(256)
 patch_planes_kernel(const float* __restrict__ x, float* __restrict__ hi, float* __restrict__ lo, const NrsConvGeom g, int kh,
-                    int kw, const NrsFastDiv div_quads, uint32_t total /*pixels * (row length / 4)*/, NrsRange* range) {
+                    int kw, const NrsFastDiv div_quads, uint32_t total /*pixels * (row length / 4)*/, int scan_n, NrsRange* range) {
   NRS_PDL_PROLOGUE();
-  const float bound = SPLIT ? *(volatile float*)&range->top : 0.0f, scale = SPLIT ? pr::scale_of(bound) : 1.0f;
-  if (SPLIT && blockIdx.x == 0 && threadIdx.x == 0) range->bound = bound;
+  const float scale = SPLIT ? pr::open_range(scan_n > 0 ? nullptr : &range->top, x, scan_n, range) : 1.0f;
   __shared__ int off[kMaxPatch];        // offset of patch value k from the patch's origin
   __shared__ short2 tap[kMaxPatch];     // its (row, column) inside the window
   const int K = g.ci * kh * kw;
@@ -114,13 +113,16 @@ int nrs_patch_planes(nrs_ctx* ctx, const float* x, float* hi, float* lo, int n, 
   const size_t cap = (size_t)ctx->sm_count * 16;
   if (blocks > cap) blocks = cap;
   NrsRange* range = nullptr;
+  int scan_n = 0;
   if (lo) {
     int st = nrs_range_renew(ctx, hi, &range);
-    if (st == NRS_OK) st = nrs_absmax(ctx, x, (size_t)n * ci * h * wd, range);
+    const size_t count = (size_t)n * ci * h * wd;
+    if (count <= (size_t)pr::kScanAlone) scan_n = (int)count;
+    else if (st == NRS_OK) st = nrs_absmax(ctx, x, count, range);
     if (st != NRS_OK) return st;
   }
-  if (lo) NRS_PDL_LAUNCH((patch_planes_kernel<true>), (unsigned)blocks, 256, 0, ctx->stream, x, hi, lo, g, kh, kw, NrsFastDiv(quads), (uint32_t)total, range);
-  else NRS_PDL_LAUNCH((patch_planes_kernel<false>), (unsigned)blocks, 256, 0, ctx->stream, x, hi, nullptr, g, kh, kw, NrsFastDiv(quads), (uint32_t)total, range);
+  if (lo) NRS_PDL_LAUNCH((patch_planes_kernel<true>), (unsigned)blocks, 256, 0, ctx->stream, x, hi, lo, g, kh, kw, NrsFastDiv(quads), (uint32_t)total, scan_n, range);
+  else NRS_PDL_LAUNCH((patch_planes_kernel<false>), (unsigned)blocks, 256, 0, ctx->stream, x, hi, nullptr, g, kh, kw, NrsFastDiv(quads), (uint32_t)total, scan_n, range);
   NRS_LAUNCHED(ctx);
   return NRS_OK;
 }

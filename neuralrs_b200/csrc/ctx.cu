@@ -81,20 +81,25 @@ int nrs_ws_planes(nrs_ctx* ctx, int slot, size_t values, bool split, void** hi, 
   return st;
 }
 
-static void give_back_range(nrs_ctx* ctx, NrsRange* r) {
+void nrs_range_free(nrs_ctx* ctx, NrsRange* r) {
   for (auto& pg : ctx->range_pool.pages)
     if (r >= pg.mem && r < pg.mem + NrsRangePool::kPerPage) { --pg.live; return; }
 }
 void nrs_range_drop(nrs_ctx* ctx, const void* p) {
   auto it = ctx->ranges.find(p);
   if (it == ctx->ranges.end()) return;
-  give_back_range(ctx, it->second);
+  nrs_range_free(ctx, it->second);
   ctx->ranges.erase(it);
 }
 int nrs_range_renew(nrs_ctx* ctx, const void* p, NrsRange** out) {
+  nrs_range_drop(ctx, p);
+  const int st = nrs_range_new(ctx, out);
+  if (st == NRS_OK) ctx->ranges[p] = *out;
+  return st;
+}
+int nrs_range_new(nrs_ctx* ctx, NrsRange** out) {
   NrsRangePool& pool = ctx->range_pool;
   *out = nullptr;
-  nrs_range_drop(ctx, p);
   constexpr size_t kBytes = NrsRangePool::kPerPage * sizeof(NrsRange);
   if (pool.pages.empty() || pool.pages[pool.current].used == NrsRangePool::kPerPage) {
     size_t next = 0;
@@ -117,7 +122,6 @@ int nrs_range_renew(nrs_ctx* ctx, const void* p, NrsRange** out) {
   if (capturing != cudaStreamCaptureStatusNone)   // a replay meets the range as the last one left it
     NRS_CUDA(ctx, cudaMemsetAsync(*out, 0, sizeof(NrsRange), ctx->stream));
   ++pg.live;
-  ctx->ranges[p] = *out;
   return NRS_OK;
 }
 

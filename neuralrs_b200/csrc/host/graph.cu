@@ -27,6 +27,15 @@ static float* dalloc(nrs_ctx* ctx, size_t floats, bool zero = false) {
 static float* nrs_dplane(nrs_ctx* ctx, size_t values, bool split) { return dalloc(ctx, split ? (values + 1) / 2 : values); }
 static float* dplane(nrs_ctx* ctx, size_t values) { return nrs_dplane(ctx, values, ctx->math_mode == NRS_MATH_3XTF32); }
 
+TopRef::~TopRef() { nrs_range_free(ctx, range); }
+TopP new_top(nrs_ctx* ctx) {
+  if (ctx->math_mode != NRS_MATH_3XTF32) return nullptr;
+  NrsRange* r = nullptr;
+  check(ctx, nrs_range_new(ctx, &r));
+  return std::make_shared<TopRef>(ctx, r);
+}
+static const NrsRange* range_in(const TopP& t) { return t ? t->range : nullptr; }
+
 size_t Node::len() const {
   size_t n = 1;
   for (size_t d : shape) n *= d;
@@ -67,6 +76,7 @@ FlatStore::~FlatStore() {
 void invalidate_operand_caches(Node* n) {
   nrs_ctx* ctx = n->ctx;
   if (!ctx) return;
+  n->top.reset();
   if (n->planes_hi) {
     ctx->plane_hints.erase(n->data);
     nrs_free(ctx, n->planes_hi);
@@ -103,6 +113,7 @@ struct GradTarget {
 // Where a backward pass writes the gradient of `n`, and whether it must add.
 static GradTarget grad_target(const NodeP& n) {
   Node* r = grad_root(n.get());
+  r->gtop.reset();
   if (!r->grad) r->grad = dalloc(r->ctx, r->len());
   check(r->ctx, nrs_folds_settle(r->ctx, r->grad, r->len()));   // an earlier share may still wait in the fold queue
   if (r->gz_valid) {   // another share arrives: what was derived from the first one is stale
@@ -153,6 +164,12 @@ static NodeP make_out(nrs_ctx* ctx, const std::vector<size_t>& shape, std::vecto
   return out;
 }
 
+void set_grad_top(const NodeP& n, TopP top) { grad_root(n.get())->gtop = std::move(top); }
+const NrsRange* grad_top(const Node* n) {
+  while (n->view_of) n = n->view_of.get();
+  return range_in(n->gtop);
+}
+
 // Public faces of the helpers above, for operator files outside this one.
 GradSlot grad_slot(const NodeP& n) {
   GradTarget t = grad_target(n);
@@ -166,7 +183,7 @@ NodeP make_result(nrs_ctx* ctx, const std::vector<size_t>& shape, std::vector<No
 // Stages NHWC planes of an NCHW tensor [n,c,h,w] at `src` into fresh pool blocks and registers
 // them with the context under `src`.  Returns false (nothing allocated) when the tensor-core
 // convolutions would not take this tensor (FP32 mode).
-static bool stage_planes(nrs_ctx* ctx, const float* src, const std::vector<size_t>& shape, float** hi, float** lo) {
+static bool stage_planes(nrs_ctx* ctx, const float* src, const std::vector<size_t>& shape, float** hi, float** lo, const NrsRange* known) {
   *hi = *lo = nullptr;
   if (ctx->math_mode == NRS_MATH_FP32 || shape.size() != 4 || shape[0] == 0) return false;
   if (!tc::tensor_map_encoder()) return false;
@@ -176,7 +193,7 @@ static bool stage_planes(nrs_ctx* ctx, const float* src, const std::vector<size_
   const size_t values = n * hw * nrs_plane_ld((int)c);
   *hi = dplane(ctx, values);
   if (split) *lo = dplane(ctx, values);
-  check(ctx, nrs_tc_stage_image(ctx, src, *hi, *lo, (int)n, (int)c, (int)hw));
+  check(ctx, nrs_tc_stage_image(ctx, src, *hi, *lo, (int)n, (int)c, (int)hw, nullptr, known));
   ctx->plane_hints[src] = NrsPlanes{*hi, *lo, split ? 1 : 0};
   return true;
 }
@@ -185,7 +202,7 @@ static bool stage_planes(nrs_ctx* ctx, const float* src, const std::vector<size_
 // padded to 32 bytes), so the same planes serve it as the A operand of x@W and, read along the rows, as
 // an operand of the weight gradient x^T dz.  Stages them into fresh pool blocks and registers them with
 // the context under `src`; false (nothing allocated) when a tensor-core GEMM would not read them.
-static bool stage_planes_2d(nrs_ctx* ctx, const float* src, size_t rows, size_t cols, float** hi, float** lo) {
+static bool stage_planes_2d(nrs_ctx* ctx, const float* src, size_t rows, size_t cols, float** hi, float** lo, const NrsRange* known) {
   *hi = *lo = nullptr;
   if (ctx->math_mode == NRS_MATH_FP32 || rows == 0 || rows > 2147483647u || cols > 2147483647u) return false;
   if (!tc::tensor_map_encoder() || ctx->plane_hints.count(src)) return false;
@@ -193,7 +210,7 @@ static bool stage_planes_2d(nrs_ctx* ctx, const float* src, size_t rows, size_t 
   const int ld = nrs_plane_ld((int)cols);
   *hi = dplane(ctx, rows * ld);
   if (split) *lo = dplane(ctx, rows * ld);
-  check(ctx, nrs_tc_stage(ctx, src, *hi, *lo, (int)rows, (int)cols, ld, 1, 0, 0, false));
+  check(ctx, nrs_tc_stage(ctx, src, *hi, *lo, (int)rows, (int)cols, ld, 1, 0, 0, false, nullptr, known));
   NrsPlanes pl{*hi, *lo, split ? 1 : 0};
   pl.rows = (int)rows;
   pl.cols = (int)cols;
@@ -207,8 +224,8 @@ struct GradPlanes {
   nrs_ctx* ctx;
   const float* key = nullptr;
   float *hi = nullptr, *lo = nullptr;
-  GradPlanes(nrs_ctx* c, const float* dz, size_t rows, size_t cols, bool wanted) : ctx(c) {
-    if (wanted && stage_planes_2d(c, dz, rows, cols, &hi, &lo)) key = dz;
+  GradPlanes(nrs_ctx* c, const float* dz, size_t rows, size_t cols, bool wanted, const NrsRange* known) : ctx(c) {
+    if (wanted && stage_planes_2d(c, dz, rows, cols, &hi, &lo, known)) key = dz;
   }
   ~GradPlanes() {
     if (!key) return;
@@ -222,7 +239,7 @@ struct GradPlanes {
 static void cache_planes_2d(const NodeP& x, size_t rows, size_t cols) {
   if (x->planes_hi) return;
   float *hi = nullptr, *lo = nullptr;
-  if (stage_planes_2d(x->ctx, x->data, rows, cols, &hi, &lo)) {
+  if (stage_planes_2d(x->ctx, x->data, rows, cols, &hi, &lo, range_in(x->top))) {
     x->planes_hi = hi;
     x->planes_lo = lo;
   }
@@ -336,6 +353,23 @@ std::shared_ptr<FlatStore> flatten_params(const std::vector<NodeP>& params) {
 
 static void linear_input_grad(nrs_ctx* ctx, const NodeP& x, const NodeP& w, const float* dz, int m, int k, int n);
 
+// Gradient of x (+)= dz . w^T; on the tensor cores with its largest magnitude for whoever makes planes of it.
+static void input_grad_product(nrs_ctx* ctx, const NodeP& x, const float* dz, const float* w, const GradTarget& t, int m, int k, int n) {
+  if (nrs_gemm_on_tensor_cores(ctx, m, k, n)) {
+    if (TopP top = new_top(ctx)) {
+      NrsGemmExtras e;
+      e.range = top->range;
+      const int st = nrs_gemm_extras(ctx, 0, 1, m, k, n, dz, w, t.ptr, nullptr, NRS_ACT_NONE, t.accumulate ? 1.0f : 0.0f, &e);
+      if (st == NRS_OK) set_grad_top(x, std::move(top));
+      if (st != NRS_ERR_UNSUPPORTED) {
+        check(ctx, st);
+        return;
+      }
+    }
+  }
+  check(ctx, nrs_gemm(ctx, 0, 1, m, k, n, dz, w, t.ptr, nullptr, NRS_ACT_NONE, t.accumulate ? 1.0f : 0.0f));
+}
+
 NodeP matmul(const NodeP& a, const NodeP& b) {
   require_gpu(a, "cuda matmul: lhs");
   require_gpu(b, "cuda matmul: rhs");
@@ -352,7 +386,7 @@ NodeP matmul(const NodeP& a, const NodeP& b) {
     nrs_ctx* ctx = self->ctx;
     const float* dc = grad_in(self);
     need_values(a);
-    GradPlanes dc_planes(ctx, dc, (size_t)m, (size_t)n, tensor_cores && a->requires_grad && b->requires_grad);
+    GradPlanes dc_planes(ctx, dc, (size_t)m, (size_t)n, tensor_cores && a->requires_grad && b->requires_grad, grad_top(self));
     if (a->requires_grad && a->fold_act != NRS_ACT_NONE) {
       linear_input_grad(ctx, a, b, dc, m, k, n);
     } else if (a->requires_grad) {
@@ -377,9 +411,8 @@ NodeP matmul(const NodeP& a, const NodeP& b) {
           if (e.lo) nrs_free(ctx, e.lo);
         }
       }
-      if (st == NRS_ERR_UNSUPPORTED)
-        st = nrs_gemm(ctx, 0, 1, m, k, n, dc, b->data, t.ptr, nullptr, NRS_ACT_NONE, t.accumulate ? 1.0f : 0.0f);
-      check(ctx, st);
+      if (st == NRS_ERR_UNSUPPORTED) input_grad_product(ctx, a, dc, b->data, t, m, k, n);
+      else check(ctx, st);
     }
     if (b->requires_grad) {
       GradTarget t = grad_target(b);  // dB (+)= A^T . dC: reads nothing dA wrote, so it may start under dA's tail
@@ -433,12 +466,15 @@ NodeP relu(const NodeP& x) {
   NodeP out = make_out(ctx, x->shape, {x});
   const size_t len = x->len();
   check(ctx, nrs_relu_fwd(ctx, x->data, out->data, len));
+  out->top = x->top;
   Node* self = out.get();
   out->backward_fn = [self, x, len]() {
     if (!x->requires_grad) return;
     const float* g = grad_in(self);
+    const TopP top = grad_root(self)->gtop;
     GradTarget t = grad_target(x);
     check(self->ctx, nrs_relu_bwd(self->ctx, x->data, g, t.ptr, len, t.accumulate));
+    if (!t.accumulate) set_grad_top(x, top);
   };
   return out;
 }
@@ -449,6 +485,7 @@ NodeP gelu(const NodeP& x) {
   NodeP out = make_out(ctx, x->shape, {x});
   const size_t len = x->len();
   check(ctx, nrs_gelu_fwd(ctx, x->data, out->data, len));
+  out->top = x->top;   // |gelu(x)| <= |x|
   Node* self = out.get();
   out->backward_fn = [self, x, len]() {
     if (!x->requires_grad) return;
@@ -473,6 +510,7 @@ NodeP reshape(const NodeP& x, const std::vector<size_t>& shape) {
   out->data = x->data;
   out->owns_data = false;
   out->view_of = x;
+  out->top = x->top;
   out->parents = {x};
   out->requires_grad = x->requires_grad;
   return out;
@@ -638,11 +676,16 @@ static void conv_backward(Node* self, const NodeP& x, const NodeP& w, const Node
         ghi = dplane(ctx, xr->len());
         if (ctx->math_mode == NRS_MATH_3XTF32) glo = dplane(ctx, xr->len());
       }
-      ctx->out_extras[t.ptr] = NrsOutExtras{xr->data, ghi, glo, ghi && xr->internal && xr->grad_planes_suffice};
+      ctx->out_extras[t.ptr] = NrsOutExtras{xr->data, ghi, glo, nullptr, ghi && xr->internal && xr->grad_planes_suffice};
       // ... and per-tile channel sums of the masked gradient, for the producer's bias gradient.
       const size_t pixels = (size_t)n * h * wd;
       const int cap = (int)(4 * (pixels / 64 + 2));
       ctx->colsum_requests[t.ptr] = NrsColsumRequest{dalloc(ctx, (size_t)cap * ci), cap, 0};
+    }
+    TopP top = ghi ? nullptr : new_top(ctx);
+    if (top) {
+      NrsOutExtras& e = ctx->out_extras[t.ptr];   // (value-initialised unless set above)
+      e.measure = top->range;
     }
     try {
       check(ctx, nrs_conv2d_bwd(ctx, x->data, w->data, dy, t.ptr, nullptr, nullptr, n, ci, h, wd, co, kh, kw, stride,
@@ -652,13 +695,15 @@ static void conv_backward(Node* self, const NodeP& x, const NodeP& w, const Node
       if (fold) {
         auto it = ctx->colsum_requests.find(t.ptr);
         if (it != ctx->colsum_requests.end()) { nrs_free(ctx, it->second.partial); ctx->colsum_requests.erase(it); }
-        ctx->out_extras.erase(t.ptr);
         if (ghi) nrs_free(ctx, ghi);
         if (glo) nrs_free(ctx, glo);
       }
+      ctx->out_extras.erase(t.ptr);
       throw;
     }
-    if (fold) {
+    if (!fold) {
+      if (!ctx->out_extras.erase(t.ptr) && top) set_grad_top(x, top);   // honoured
+    } else {
       NrsColsumRequest sums = ctx->colsum_requests[t.ptr];
       ctx->colsum_requests.erase(t.ptr);
       if (ctx->out_extras.erase(t.ptr)) {   // not honoured (the kernel that ran does not fold)
@@ -669,6 +714,7 @@ static void conv_backward(Node* self, const NodeP& x, const NodeP& w, const Node
         xr->gplanes_hi = ghi;
         xr->gplanes_lo = glo;
         xr->grad_premasked = true;
+        if (top) set_grad_top(x, top);
       }
       if (sums.rows > 0) {
         xr->gchan_partial = sums.partial;
@@ -713,7 +759,7 @@ NodeP conv2d_act(const NodeP& x, const NodeP& w, const NodeP& b, size_t stride, 
   const bool patches = nrs_conv_uses_patches(ci, kh, kw);
   if (!patches && !x->planes_hi && w->requires_grad && planes_possible(ctx)) {
     float *phi = nullptr, *plo = nullptr;
-    if (stage_planes(ctx, x->data, x->shape, &phi, &plo)) { x->planes_hi = phi; x->planes_lo = plo; }
+    if (stage_planes(ctx, x->data, x->shape, &phi, &plo, range_in(x->top))) { x->planes_hi = phi; x->planes_lo = plo; }
   }
   // Few input channels in a TF32 mode: forward and weight gradient both run on the tensor cores over the
   // input's patch planes; make them once.
@@ -741,17 +787,24 @@ NodeP conv2d_act(const NodeP& x, const NodeP& w, const NodeP& b, size_t stride, 
     if (ctx->math_mode == NRS_MATH_3XTF32) olo = dplane(ctx, out->len());
     ctx->out_extras[out->data] = NrsOutExtras{nullptr, ohi, olo};
   }
+  TopP top = ohi ? nullptr : new_top(ctx);
+  if (top) {
+    NrsOutExtras e{};
+    e.measure = top->range;
+    ctx->out_extras[out->data] = e;
+  }
   try {
     check(ctx, nrs_conv2d_fwd(ctx, x->data, w->data, b->data, out->data, n, ci, h, wd, co, kh, kw, (int)stride,
                               (int)pad, act));
   } catch (...) {
+    ctx->out_extras.erase(out->data);
     if (ohi) {
-      ctx->out_extras.erase(out->data);
       nrs_free(ctx, ohi);
       if (olo) nrs_free(ctx, olo);
     }
     throw;
   }
+  if (top && !ctx->out_extras.erase(out->data)) out->top = top;   // honoured
   if (ohi) {
     if (ctx->out_extras.erase(out->data)) {   // not honoured
       nrs_free(ctx, ohi);
@@ -793,17 +846,17 @@ NodeP conv2d_act(const NodeP& x, const NodeP& w, const NodeP& b, size_t stride, 
         dhi = dplane(ctx, self->len());
         if (split) dlo = dplane(ctx, self->len());
         check(ctx, nrs_tc_stage_masked(ctx, 0, dy, self->data, nullptr, n, co, (int)self->shape[2], (int)self->shape[3], 1,
-                                       masked, dhi, dlo));
+                                       masked, dhi, dlo, nullptr, nullptr, grad_top(self)));
         ctx->plane_hints[masked] = NrsPlanes{dhi, dlo, split ? 1 : 0};
         staged = true;
       } else {
         check(ctx, nrs_relu_bwd(ctx, self->data, dy, masked, self->len(), 0));
-        if (want_planes) staged = stage_planes(ctx, masked, self->shape, &dhi, &dlo);
+        if (want_planes) staged = stage_planes(ctx, masked, self->shape, &dhi, &dlo, grad_top(self));
       }
       dy = masked;
     } else if (want_planes) {
       // dy feeds both the data and the weight gradient: stage its planes once.
-      staged = stage_planes(ctx, dy, self->shape, &dhi, &dlo);
+      staged = stage_planes(ctx, dy, self->shape, &dhi, &dlo, grad_top(self));
     }
     auto cleanup = [&] {
       if (staged) ctx->plane_hints.erase(dy);
@@ -843,7 +896,7 @@ NodeP maxpool2d(const NodeP& x, size_t kernel, size_t stride, bool emit_planes) 
     // a tensor-core convolution reads the result next: write its operand planes in the same pass
     float* phi = dplane(ctx, out->len());
     float* plo = ctx->math_mode == NRS_MATH_3XTF32 ? dplane(ctx, out->len()) : nullptr;
-    const int st = nrs_tc_pool2_fwd_planes(ctx, x->data, out->data, (int32_t*)am, phi, plo, n, c, h, w);
+    const int st = nrs_tc_pool2_fwd_planes(ctx, x->data, out->data, (int32_t*)am, phi, plo, n, c, h, w, range_in(x->top));
     if (st == NRS_OK) {
       out->planes_hi = phi;
       out->planes_lo = plo;
@@ -856,11 +909,13 @@ NodeP maxpool2d(const NodeP& x, size_t kernel, size_t stride, bool emit_planes) 
     }
   }
   if (!done) check(ctx, nrs_maxpool_fwd(ctx, x->data, out->data, (int32_t*)am, n, c, h, w, k, s));
+  out->top = x->top;
   Node* self = out.get();
   out->backward_fn = [self, x, am, n, c, h, w, k, s]() {
     if (!x->requires_grad) return;
     nrs_ctx* ctx = self->ctx;
     const float* g = grad_in(self);
+    const TopP top = grad_root(self)->gtop;
     // Pool over the output of a convolution with a folded ReLU: one pass computes that
     // convolution's masked gradient (and its NHWC planes when its tensor-core backward wants
     // them) instead of pool-backward, ReLU-backward and staging as three passes.
@@ -878,7 +933,8 @@ NodeP maxpool2d(const NodeP& x, size_t kernel, size_t stride, bool emit_planes) 
       // even images of 2 x 2 windows: the kernel that makes the channel sums runs
       const bool values = !(phi && partial && h % 2 == 0 && w % 2 == 0 && xr->internal && xr->grad_planes_suffice);
       check(ctx, nrs_tc_stage_masked(ctx, 1, g, self->data, (const int32_t*)am, n, c, h, w, k, values ? t.ptr : nullptr, phi, plo, partial,
-                                     &partial_rows));
+                                     &partial_rows, range_in(top)));
+      set_grad_top(x, top);   // every value of g goes to one place at most
       if (!values && partial_rows == 0) fail(NRS_ERR_CUDA, "cuda maxpool: channel sums missing");
       if (partial && partial_rows == 0) { nrs_free(ctx, partial); partial = nullptr; }
       xr->gplanes_hi = phi;
@@ -890,6 +946,7 @@ NodeP maxpool2d(const NodeP& x, size_t kernel, size_t stride, bool emit_planes) 
     }
     GradTarget t = grad_target(x);
     check(ctx, nrs_maxpool_bwd(ctx, g, (const int32_t*)am, t.ptr, n, c, h, w, k, s, t.accumulate));
+    if (!t.accumulate && s >= k) set_grad_top(x, top);
   };
   return out;
 }
@@ -928,13 +985,15 @@ static NodeP layernorm_impl(const NodeP& x, const NodeP& residual, const NodeP& 
   out->saved.push_back(xhat);
   out->saved.push_back(istd);
   const bool planes = emit_planes && planes_possible(ctx) && f % 32 == 0 && rows > 0;
+  TopP istd_top = planes ? new_top(ctx) : nullptr;
   const bool split = ctx->math_mode == NRS_MATH_3XTF32;
   if (planes && !ctx->plane_hints.count(out->data)) {
     float* hi = dplane(ctx, x->len());
     float* lo = split ? dplane(ctx, x->len()) : nullptr;
     int emitted = 0;
     const int st = nrs_layernorm_fwd_planes(ctx, x->data, residual ? residual->data : nullptr, gamma->data, beta->data, out->data,
-                                            xhat, istd, rows, f, eps, hi, lo, &emitted);
+                                            xhat, istd, rows, f, eps, hi, lo, &emitted, istd_top ? istd_top->range : nullptr);
+    if (!emitted) istd_top.reset();
     if (st == NRS_OK && emitted) {
       out->planes_hi = hi;
       out->planes_lo = lo;
@@ -948,14 +1007,17 @@ static NodeP layernorm_impl(const NodeP& x, const NodeP& residual, const NodeP& 
     }
     check(ctx, st);
   } else if (residual) {
+    istd_top.reset();
     check(ctx, nrs_layernorm_residual_fwd(ctx, x->data, residual->data, gamma->data, beta->data, out->data, xhat, istd, rows, f, eps));
   } else {
+    istd_top.reset();
     check(ctx, nrs_layernorm_fwd(ctx, x->data, gamma->data, beta->data, out->data, xhat, istd, rows, f, eps));
   }
   Node* self = out.get();
-  out->backward_fn = [self, x, residual, gamma, beta, xhat, istd, rows, f, planes, split]() {
+  out->backward_fn = [self, x, residual, gamma, beta, xhat, istd, rows, f, planes, split, istd_top]() {
     nrs_ctx* ctx = self->ctx;
     const float* g = grad_in(self);
+    const TopP g_top = grad_root(self)->gtop;
     float *da = nullptr, *db = nullptr, *dg = nullptr, *dbt = nullptr;
     int acc_a = 0, acc_b = 0, acc_p = 0;
     if (x->requires_grad) {
@@ -998,7 +1060,7 @@ static NodeP layernorm_impl(const NodeP& x, const NodeP& residual, const NodeP& 
       float* lo = mine ? rb->gplanes_lo : (split ? nrs_dplane(ctx, self->len(), true) : nullptr);
       int emitted = 0;
       const int st = nrs_layernorm_bwd_planes(ctx, g, xhat, istd, gamma->data, da, db, dg, dbt, rows, f, acc_a, acc_b, acc_p, hi, lo,
-                                              &emitted);
+                                              &emitted, range_in(g_top), range_in(istd_top));
       if (st == NRS_OK && emitted) {
         if (!mine) {
           rb->gplanes_hi = hi;
@@ -1082,6 +1144,7 @@ NodeP batchnorm_nd(const NodeP& x, const NodeP& gamma, const NodeP& beta, const 
   out->backward_fn = [self, x, gamma, beta, mean, istd, n, c, hw, training, act, planes]() {
     nrs_ctx* ctx = self->ctx;
     const float* g = grad_in(self);
+    const TopP g_top = grad_root(self)->gtop;
     float *dg = nullptr, *db = nullptr;
     int acc_p = 0;
     if (gamma->requires_grad || beta->requires_grad) {
@@ -1117,7 +1180,7 @@ NodeP batchnorm_nd(const NodeP& x, const NodeP& gamma, const NodeP& beta, const 
       }
     }
     check(ctx, nrs_batchnorm_bwd_from_x(ctx, g, x->data, mean, istd, gamma->data, beta->data, dx, dg, db, n, c, hw, training ? 1 : 0,
-                                        acc_x, acc_p, act, phi, plo, partial));
+                                        acc_x, acc_p, act, phi, plo, partial, range_in(g_top)));
   };
   return out;
 }
@@ -1220,7 +1283,7 @@ static void linear_input_grad(nrs_ctx* ctx, const NodeP& x, const NodeP& w, cons
     if (st == NRS_OK) return;   // the gradient itself is there
     if (st != NRS_ERR_UNSUPPORTED) check(ctx, st);
   }
-  check(ctx, nrs_gemm(ctx, 0, 1, m, k, n, dz, w->data, t.ptr, nullptr, NRS_ACT_NONE, t.accumulate ? 1.0f : 0.0f));
+  input_grad_product(ctx, x, dz, w->data, t, m, k, n);
 }
 
 // emit_planes: the caller knows that a tensor-core GEMM reads the result (always assumed of a GELU layer, which has
@@ -1298,7 +1361,8 @@ NodeP linear_act(const NodeP& x, const NodeP& w, const NodeP& b, int act, bool e
       dz = tmp;
     }
     // dz feeds both dW = x^T dz and dX = dz W^T: its planes are made once
-    GradPlanes dz_planes(ctx, dz, (size_t)m, (size_t)n, !from_planes && tensor_cores && w->requires_grad && x->requires_grad);
+    GradPlanes dz_planes(ctx, dz, (size_t)m, (size_t)n, !from_planes && tensor_cores && w->requires_grad && x->requires_grad,
+                         act == NRS_ACT_GELU || from_planes ? nullptr : grad_top(self));   // (a ReLU's mask keeps the bound)
     if (b->requires_grad) {
       GradTarget t = grad_target(b);
       if (from_planes) check(ctx, nrs_fold_columns(ctx, self->gchan_partial, t.ptr, self->gchan_rows, n, n, t.accumulate));
@@ -1347,6 +1411,7 @@ void cross_entropy_backward(const NodeP& pred, const NodeP& target) {
   batch_classes(pred, &batch, &classes);
   Node* r = grad_root(pred.get());
   if (!r->grad) r->grad = dalloc(ctx, r->len());
+  r->gtop.reset();
   check(ctx, nrs_ce_bwd(ctx, pred->data, target->data, r->grad, batch, classes, batch));
   r->grad_valid = true;  // overwritten, as the reference does
 }
@@ -1360,6 +1425,7 @@ void cross_entropy_fused(const NodeP& pred, const NodeP& target, float* loss_dev
   batch_classes(pred, &batch, &classes);
   Node* r = grad_root(pred.get());
   if (!r->grad) r->grad = dalloc(ctx, r->len());
+  r->gtop.reset();
   check(ctx, nrs_ce_fwd_bwd(ctx, pred->data, target->data, loss_dev, r->grad, batch, classes, divisor));
   r->grad_valid = true;
 }
@@ -1371,6 +1437,7 @@ void cross_entropy_fused_indexed(const NodeP& pred, const int32_t* labels_dev, f
   nrs_ctx* ctx = pred->ctx;
   Node* r = grad_root(pred.get());
   if (!r->grad) r->grad = dalloc(ctx, r->len());
+  r->gtop.reset();
   check(ctx, nrs_ce_fwd_bwd_indexed(ctx, pred->data, labels_dev, loss_dev, r->grad, (int)pred->shape[0], (int)pred->shape[1], divisor));
   r->grad_valid = true;
 }

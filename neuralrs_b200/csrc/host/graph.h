@@ -19,6 +19,8 @@
 
 #include "nrs.h"
 
+struct NrsRange;
+
 namespace nrs {
 
 struct Error : std::runtime_error {
@@ -30,6 +32,18 @@ struct Error : std::runtime_error {
 void check(nrs_ctx* ctx, int status);
 
 struct FlatStore;
+
+// A tensor's largest magnitude, or a bound of it, on the device (NrsRange::top): what f16 pairs of it need to be made without
+// a pass that measures.  Shared by the tensors it bounds.
+struct TopRef {
+  nrs_ctx* ctx;
+  NrsRange* range;
+  TopRef(nrs_ctx* c, NrsRange* r) : ctx(c), range(r) {}
+  TopRef(const TopRef&) = delete;
+  TopRef& operator=(const TopRef&) = delete;
+  ~TopRef();
+};
+using TopP = std::shared_ptr<TopRef>;
 
 // Node of the define-by-run graph (src/autograd/node.rs:38-53).
 struct Node {
@@ -88,6 +102,10 @@ struct Node {
   // only need not be written besides.  planes_only: `data` was left out (3xTF32: the f16 pairs hold it to 2^-23).
   bool internal = false, planes_only = false;
 
+  // 3xTF32: bounds of `data` and of `grad` where their writer left one (null: unknown).  Whoever writes the tensor otherwise
+  // drops them: to_cuda, grad_target.
+  TopP top, gtop;
+
   size_t len() const;
   bool on_gpu() const { return data != nullptr; }
   ~Node();
@@ -116,6 +134,9 @@ struct GradSlot {
   int accumulate;  // 0: overwrite (first writer), 1: add
 };
 GradSlot grad_slot(const NodeP& n);   // marks the gradient as written
+TopP new_top(nrs_ctx* ctx);           // an empty one for a kernel to fill; null outside of 3xTF32
+void set_grad_top(const NodeP& n, TopP top);   // after grad_slot, by a writer that left the bound of what the gradient now is
+const NrsRange* grad_top(const Node* n);
 const float* grad_view(Node* n);      // a node's own incoming gradient (zeros if nothing wrote it)
 NodeP make_result(nrs_ctx* ctx, const std::vector<size_t>& shape, std::vector<NodeP> parents);
 void cache_row_planes(const NodeP& x, size_t rows, size_t cols);   // TF32 row planes of x's data, kept with the node

@@ -303,7 +303,11 @@ static NodeP planes_attention(const MultiHeadAttention& m, const NodeP& x, size_
     if (x->requires_grad) {
       GradSlot t = grad_slot(x);
       const float* w[3] = {wq->data, wk->data, wv->data};
-      check(ctx, nrs_tc_gemm_weights(ctx, 1, 3, (int)tokens, (int)d, (int)d, a.dqkv_hi, w, t.ptr, t.accumulate ? 1.0f : 0.0f, nullptr));
+      NrsGemmExtras e;
+      TopP top = new_top(ctx);   // (the layer below makes planes of the sum)
+      if (top) e.range = top->range;
+      check(ctx, nrs_tc_gemm_weights(ctx, 1, 3, (int)tokens, (int)d, (int)d, a.dqkv_hi, w, t.ptr, t.accumulate ? 1.0f : 0.0f, &e));
+      set_grad_top(x, std::move(top));
     }
     GradSlot s[3] = {grad_slot(wq), grad_slot(wk), grad_slot(wv)};
     const size_t dd = d * d;

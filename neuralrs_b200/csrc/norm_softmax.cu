@@ -214,13 +214,13 @@ __global__ void __launch_bounds__(kRowThreads)
 ln_fwd_vec_kernel(const float* __restrict__ a, const float* __restrict__ b, const float* __restrict__ gamma,
                   const float* __restrict__ beta, float* __restrict__ y, float* __restrict__ xhat,
                   float* __restrict__ istd_out, int rows, int f, float eps, float* __restrict__ y_hi,
-                  float* __restrict__ y_lo, NrsRange* __restrict__ range) {
+                  float* __restrict__ y_lo, NrsRange* __restrict__ range, NrsRange* __restrict__ istd_range) {
   NRS_PDL_PROLOGUE();
   const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
   const int f4 = f >> 2;
   const float inv_f = 1.0f / (float)f;
   [[maybe_unused]] float scale = 1.0f;
-  [[maybe_unused]] uint32_t top = 0;
+  [[maybe_unused]] uint32_t top = 0, top_istd = 0;
   if (EMIT && y_lo) {   // |xhat| <= sqrt(f)
     uint32_t mg = 0, mb = 0;
     for (int c = lane; c < f4; c += 32) {
@@ -258,6 +258,7 @@ ln_fwd_vec_kernel(const float* __restrict__ a, const float* __restrict__ b, cons
       }
     const float istd = 1.0f / sqrtf(wsum(vs) * inv_f + eps);
     if (lane == 0 && istd_out) istd_out[r] = istd;
+    if (EMIT) top_istd = pr::seen(top_istd, istd);
 #pragma unroll
     for (int k = 0; k < VPL; ++k) {
       const int c = lane + 32 * k;
@@ -273,7 +274,10 @@ ln_fwd_vec_kernel(const float* __restrict__ a, const float* __restrict__ b, cons
       }
     }
   }
-  if (EMIT && y_lo) pr::report(range, top);
+  if (EMIT && y_lo) {
+    pr::report(range, top);
+    if (istd_range) pr::report(istd_range, top_istd);
+  }
 }
 
 __global__ void __launch_bounds__(kRowThreads)
@@ -578,7 +582,7 @@ int vec_vpl(int width, std::initializer_list<const void*> ptrs) {
 
 int layernorm_fwd(nrs_ctx* ctx, const char* who, const float* a, const float* b, const float* gamma, const float* beta,
                   float* y, float* xhat, float* istd, int rows, int f, float eps, float* y_hi = nullptr, float* y_lo = nullptr,
-                  int* emitted = nullptr) {
+                  int* emitted = nullptr, NrsRange* istd_range = nullptr) {
   if (emitted) *emitted = 0;
   NRS_REQUIRE(ctx, rows >= 0 && f > 0, NRS_ERR_SHAPE, "%s: bad shape [%d,%d]", who, rows, f);
   if (rows == 0) return NRS_OK;
@@ -617,10 +621,10 @@ int layernorm_fwd(nrs_ctx* ctx, const char* who, const float* a, const float* b,
     }
     if (y_hi)
       NRS_DISPATCH_VPL(vpl, NRS_PDL_LAUNCH((ln_fwd_vec_kernel<V, true>), row_grid(ctx, rows), kRowThreads, 0, ctx->stream, a, b, gamma,
-                                           beta, y, xhat, istd, rows, f, eps, y_hi, y_lo, range));
+                                           beta, y, xhat, istd, rows, f, eps, y_hi, y_lo, range, istd_range));
     else
       NRS_DISPATCH_VPL(vpl, NRS_PDL_LAUNCH((ln_fwd_vec_kernel<V, false>), row_grid(ctx, rows), kRowThreads, 0, ctx->stream, a, b, gamma,
-                                           beta, y, xhat, istd, rows, f, eps, y_hi, y_lo, range));
+                                           beta, y, xhat, istd, rows, f, eps, y_hi, y_lo, range, istd_range));
     if (emitted && y_hi) *emitted = 1;
   } else {
     NRS_PDL_LAUNCH(ln_fwd_kernel, row_grid(ctx, rows), kRowThreads, 0, ctx->stream, a, b, gamma, beta, y, xhat, istd, rows, f, eps);
@@ -636,7 +640,8 @@ int fold_params(nrs_ctx* ctx, const float* partial, float* dgamma, float* dbeta,
 
 int layernorm_bwd(nrs_ctx* ctx, const char* who, const float* g, const float* xhat, const float* istd, const float* gamma,
                   float* dx, float* dx2, float* dgamma, float* dbeta, int rows, int f, int acc1, int acc2, int accumulate_params,
-                  float* d_hi = nullptr, float* d_lo = nullptr, int* emitted = nullptr) {
+                  float* d_hi = nullptr, float* d_lo = nullptr, int* emitted = nullptr, const NrsRange* range_g = nullptr,
+                  const NrsRange* range_istd = nullptr) {
   if (emitted) *emitted = 0;
   NRS_REQUIRE(ctx, rows >= 0 && f > 0, NRS_ERR_SHAPE, "%s: bad shape [%d,%d]", who, rows, f);
   NRS_REQUIRE(ctx, (dgamma == nullptr) == (dbeta == nullptr), NRS_ERR_ARG, "%s: dgamma and dbeta must be given together", who);
@@ -705,17 +710,21 @@ int layernorm_bwd(nrs_ctx* ctx, const char* who, const float* g, const float* xh
       if (st != NRS_OK) return st;
     }
     const size_t smem = dgamma ? (size_t)warps * 2 * f * sizeof(float) : 0;
-    NrsRange *range = nullptr, *range_g = nullptr, *range_istd = nullptr;
+    NrsRange* range = nullptr;
     if (dx && d_hi && d_lo) {
       int st = nrs_range_renew(ctx, d_hi, &range);
-      if (st == NRS_OK) st = nrs_range_renew(ctx, &ctx->scratch_range[0], &range_g);
-      if (st == NRS_OK) st = nrs_range_renew(ctx, &ctx->scratch_range[1], &range_istd);
-      if (st == NRS_OK) st = nrs_absmax2(ctx, g, elems, range_g, istd, (size_t)rows, range_istd);
+      NrsRange *mg = nullptr, *mi = nullptr;
+      if (!range_g && st == NRS_OK) st = nrs_range_renew(ctx, &ctx->scratch_range[0], &mg);
+      if (!range_istd && st == NRS_OK) st = nrs_range_renew(ctx, &ctx->scratch_range[1], &mi);
+      if (st == NRS_OK && mg) st = nrs_absmax(ctx, g, elems, mg);
+      if (st == NRS_OK && mi) st = nrs_absmax(ctx, istd, (size_t)rows, mi);
       if (st != NRS_OK) return st;
+      if (mg) range_g = mg;
+      if (mi) range_istd = mi;
     }
     if (dx && d_hi)
       NRS_DISPATCH_VPL(vpl, NRS_PDL_LAUNCH((ln_bwd_vec_kernel<V, true>), blocks, warps * 32, smem, ctx->stream, g, xhat, istd, gamma, dx,
-                                           dx2, partial, rows, f, acc1, acc2, d_hi, d_lo, (const NrsRange*)range_g, (const NrsRange*)range_istd, range));
+                                           dx2, partial, rows, f, acc1, acc2, d_hi, d_lo, range_g, range_istd, range));
     else
       NRS_DISPATCH_VPL(vpl, NRS_PDL_LAUNCH((ln_bwd_vec_kernel<V, false>), blocks, warps * 32, smem, ctx->stream, g, xhat, istd, gamma, dx,
                                            dx2, partial, rows, f, acc1, acc2, (float*)nullptr, (float*)nullptr, (const NrsRange*)nullptr,
@@ -785,20 +794,22 @@ int nrs_layernorm_residual_bwd(nrs_ctx* ctx, const float* g, const float* xhat, 
 // input gradient backward): *emitted = 1 when the planes were written (vector path), 0 when the caller has
 // to stage them itself.  Internal: the graph's fused transformer block calls them.
 int nrs_layernorm_fwd_planes(nrs_ctx* ctx, const float* a, const float* b, const float* gamma, const float* beta, float* y,
-                             float* xhat, float* istd, int rows, int f, float eps, float* y_hi, float* y_lo, int* emitted) {
+                             float* xhat, float* istd, int rows, int f, float eps, float* y_hi, float* y_lo, int* emitted,
+                             NrsRange* istd_range) {
   NRS_REQUIRE_CTX(ctx);
-  return layernorm_fwd(ctx, "nrs_layernorm_fwd_planes", a, b, gamma, beta, y, xhat, istd, rows, f, eps, y_hi, y_lo, emitted);
+  return layernorm_fwd(ctx, "nrs_layernorm_fwd_planes", a, b, gamma, beta, y, xhat, istd, rows, f, eps, y_hi, y_lo, emitted, istd_range);
 }
 
 int nrs_layernorm_bwd_planes(nrs_ctx* ctx, const float* g, const float* xhat, const float* istd, const float* gamma, float* da,
                              float* db, float* dgamma, float* dbeta, int rows, int f, int accumulate_da, int accumulate_db,
-                             int accumulate_params, float* d_hi, float* d_lo, int* emitted) {
+                             int accumulate_params, float* d_hi, float* d_lo, int* emitted, const NrsRange* range_g,
+                             const NrsRange* range_istd) {
   NRS_REQUIRE_CTX(ctx);
   float* first = da ? da : db;
   float* second = da ? db : nullptr;
   const int acc_first = da ? accumulate_da : accumulate_db;
   return layernorm_bwd(ctx, "nrs_layernorm_bwd_planes", g, xhat, istd, gamma, first, second, dgamma, dbeta, rows, f, acc_first,
-                       accumulate_db, accumulate_params, d_hi, d_lo, emitted);
+                       accumulate_db, accumulate_params, d_hi, d_lo, emitted, range_g, range_istd);
 }
 
 int nrs_softmax_fwd(nrs_ctx* ctx, const float* x, float* y, int rows, int width) {

@@ -113,7 +113,7 @@ struct NrsOutExtras {
   const float* relu_mask_src;   // NCHW tensor of out's shape: out = relu_mask_src > 0 ? out : 0 (or null)
   float* hi;                    // NHWC operand planes of the (masked) result, or null
   float* lo;                    // (3xTF32)
-  bool measure = false;         // 3xTF32, no planes: leave the result's range with its address (nrs_range_of)
+  NrsRange* measure = nullptr;  // 3xTF32, no planes: largest magnitude of the result goes here
   bool planes_suffice = false;  // the result itself need not be written where its planes and channel sums are
 };
 
@@ -294,6 +294,9 @@ int nrs_ws_planes(nrs_ctx* ctx, int slot, size_t values, bool split, void** hi, 
 // A new range, all zero, for what is written to `p` next; it belongs to the address until that is renewed, dropped or
 // freed (nrs_free).
 int nrs_range_renew(nrs_ctx* ctx, const void* p, NrsRange** out);
+// The same without an address: the caller gives it back.
+int nrs_range_new(nrs_ctx* ctx, NrsRange** out);
+void nrs_range_free(nrs_ctx* ctx, NrsRange* r);
 void nrs_range_drop(nrs_ctx* ctx, const void* p);
 inline NrsRange* nrs_range_of(const nrs_ctx* ctx, const void* p) {
   auto it = ctx->ranges.find(p);
@@ -315,17 +318,20 @@ int nrs_fold_ticket(nrs_ctx* ctx, unsigned** out);
 // LayerNorm with the TF32 planes of its result written by the kernel (norm_softmax.cu).
 extern "C" int nrs_layernorm_fwd_planes(nrs_ctx* ctx, const float* a, const float* b, const float* gamma, const float* beta,
                                         float* y, float* xhat, float* istd, int rows, int f, float eps, float* y_hi, float* y_lo,
-                                        int* emitted);
+                                        int* emitted, NrsRange* istd_range);
 extern "C" int nrs_layernorm_bwd_planes(nrs_ctx* ctx, const float* g, const float* xhat, const float* istd, const float* gamma,
                                         float* da, float* db, float* dgamma, float* dbeta, int rows, int f, int accumulate_da,
-                                        int accumulate_db, int accumulate_params, float* d_hi, float* d_lo, int* emitted);
+                                        int accumulate_db, int accumulate_params, float* d_hi, float* d_lo, int* emitted,
+                                        const NrsRange* range_g, const NrsRange* range_istd);
 // Operand planes of a batch of [rows][K] matrices (tc_stage.cu); see tc_mainloop.cuh for the layouts.  3xTF32: the range
-// of `hi` is renewed and measured first, unless the caller has one that covers the source's values.
+// of `hi` is renewed and measured, in the same launch for small tensors, unless the caller has one: `measured` becomes the
+// planes' own, `known` bounds the source's values (NrsRange::top).
 int nrs_tc_stage(nrs_ctx* ctx, const float* src, float* hi, float* lo, int rows, int K, int ldk, int batch,
-                 size_t src_bstride, size_t dst_bstride, bool src_k_by_rows, NrsRange* measured = nullptr);
+                 size_t src_bstride, size_t dst_bstride, bool src_k_by_rows, NrsRange* measured = nullptr, const NrsRange* known = nullptr);
 // NHWC planes of an NCHW tensor [n][c][hw], pixel stride nrs_plane_ld(c) floats (zeros between c and there).
 // chan_partial (hw > 1): [nrs_batchnorm_tiles(n, hw)][c] channel sums of the pixels of each tile.
-int nrs_tc_stage_image(nrs_ctx* ctx, const float* src, float* hi, float* lo, int n, int c, int hw, float* chan_partial = nullptr);
+int nrs_tc_stage_image(nrs_ctx* ctx, const float* src, float* hi, float* lo, int n, int c, int hw, float* chan_partial = nullptr,
+                       const NrsRange* known = nullptr);
 // Counter window of a per-sample draw of `count` elements (count = samples * per-sample) in blocks of four:
 // first block to use and by how many blocks the stream advances.  Falls back to the plain stream (this
 // process's own draws) when no shard is set, the call is not per-sample, or the shard does not start on a
@@ -356,7 +362,7 @@ int nrs_batchnorm_fwd_saving_mean(nrs_ctx* ctx, const float* x, const float* gam
                                   float* hi, float* lo);
 int nrs_batchnorm_bwd_from_x(nrs_ctx* ctx, const float* g, const float* x, const float* mean, const float* istd, const float* gamma,
                              const float* beta, float* dx, float* dgamma, float* dbeta, int n, int c, int hw, int training, int accumulate_dx,
-                             int accumulate_params, int act, float* hi, float* lo, float* chan_partial);
+                             int accumulate_params, int act, float* hi, float* lo, float* chan_partial, const NrsRange* range_g = nullptr);
 int nrs_batchnorm_tiles(int n, int hw);
 
 // Batched weight staging (weight_set.cu).  build: allocates planes for the described weights in the
@@ -488,8 +494,7 @@ struct NrsGemmExtras {
   const float* dact_src = nullptr;
   float* hi = nullptr;         // operand planes [m][n] for the GEMM that reads the result next (n a multiple of 8)
   float* lo = nullptr;
-  NrsRange* range = nullptr;   // out, 3xTF32: of the planes (or, asked for with `measure`, of c); belongs to hi (c)
-  bool measure = false;        // the largest magnitude of c is wanted where no planes are
+  NrsRange* range = nullptr;   // 3xTF32: of the planes (out; belongs to hi); without planes: where the largest magnitude of c goes
   float* colsum = nullptr;     // [colsum_cap][n] partial column sums
   int colsum_cap = 0;
   int colsum_rows = 0;         // out: rows of it written (0: none, the caller sums the columns itself)

@@ -81,6 +81,36 @@ __device__ __forceinline__ void report(NrsRange* r, uint32_t top) {
   top = __reduce_max_sync(0xffffffffu, top);
   if ((threadIdx.x & 31) == 0 && top > __float_as_uint(*(volatile float*)&r->top)) atomicMax(reinterpret_cast<unsigned*>(&r->top), top);
 }
+// What one block finds in n values (all of its threads ask; at most kScanAlone values, else absmax_kernel measures them).
+constexpr int kScanAlone = 32768;
+__device__ __forceinline__ uint32_t scan(const float* __restrict__ src, int n) {
+  __shared__ uint32_t found[32];
+  uint32_t top = 0;
+  const int head = min(n, (int)(((16 - (reinterpret_cast<uintptr_t>(src) & 15)) & 15) / 4)), quads = (n - head) / 4;
+  const float4* body = reinterpret_cast<const float4*>(src + head);
+#pragma unroll 4
+  for (int i = threadIdx.x; i < quads; i += blockDim.x) top = seen4(top, body[i]);
+  if ((int)threadIdx.x < head) top = seen(top, src[threadIdx.x]);
+  const int rest = head + 4 * quads + (int)threadIdx.x;
+  if (rest < n) top = seen(top, src[rest]);   // at most 3
+  top = __reduce_max_sync(0xffffffffu, top);
+  if ((threadIdx.x & 31) == 0) found[threadIdx.x >> 5] = top;
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  top = __reduce_max_sync(0xffffffffu, lane < (int)(blockDim.x >> 5) ? found[lane] : 0u);
+  __syncthreads();
+  return top;
+}
+// The scale of planes whose values are bounded by *top, or (scan_n > 0) are the scan_n values at `src`; one thread of the
+// grid leaves the bound as their range.
+__device__ __forceinline__ float open_range(const float* top, const float* src, int scan_n, NrsRange* range) {
+  const float bound = scan_n > 0 ? __uint_as_float(scan(src, scan_n)) : *reinterpret_cast<const volatile float*>(top);
+  if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) {
+    range->bound = bound;
+    if (top != &range->top) range->top = bound;
+  }
+  return scale_of(bound);
+}
 // Bound of a sum of `k` products of values up to a and b, plus a value up to c: with room for the sum's own rounding,
 // and finite.
 __device__ __forceinline__ float product_bound(float k, float a, float b, float c) { return fminf((k * a * b + c) * 1.001f, 3.0e38f); }

@@ -247,14 +247,17 @@ constexpr int kFoldRows = 64;
 __global__ void __launch_bounds__(256)
 thin_fold_kernel(const float* __restrict__ dz, const float* __restrict__ w, float* __restrict__ c, const float* __restrict__ src, int relu,
                  float* __restrict__ hi, float* __restrict__ lo, float* __restrict__ colsum, int m, int k, int n,
-                 const NrsRange* __restrict__ range_dz, const NrsRange* __restrict__ range_w, NrsRange* __restrict__ range) {
+                 const NrsRange* __restrict__ range_dz, const NrsRange* __restrict__ range_w /*null: scanned here*/,
+                 NrsRange* __restrict__ range) {
   NRS_PDL_PROLOGUE();
   __shared__ float part[8][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   float scale = 1.0f;
   uint32_t top = 0;
   if (lo) {
-    const float bound = pr::product_bound((float)n, range_dz->top, range_w->top, 0.0f) * (relu ? 1.0f : 1.25f);
+    const float top_dz = range_dz ? range_dz->top : __uint_as_float(pr::scan(dz, m * n));
+    const float top_w = range_w ? range_w->top : __uint_as_float(pr::scan(w, k * n));
+    const float bound = fminf(pr::product_bound((float)n, top_dz, top_w, 0.0f) * (relu ? 1.0f : 1.25f), 3.0e38f);
     if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) range->bound = bound;
     scale = pr::scale_of(bound);
   }
@@ -614,9 +617,11 @@ int nrs_gemm_extras(nrs_ctx* ctx, int trans_a, int trans_b, int m, int n, int k,
       NrsRange *range_a = nullptr, *range_b = nullptr;
       if (extras->lo) {
         int st = nrs_range_renew(ctx, extras->hi, &extras->range);
-        if (st == NRS_OK) st = nrs_range_renew(ctx, &ctx->scratch_range[0], &range_a);
-        if (st == NRS_OK) st = nrs_range_renew(ctx, &ctx->scratch_range[1], &range_b);
-        if (st == NRS_OK) st = nrs_absmax2(ctx, a, (size_t)m * k, range_a, b, (size_t)n * k, range_b);
+        if ((size_t)(m + n) * k > (size_t)pr::kScanAlone) {   // (else every block scans them: 3 us less than a launch)
+          if (st == NRS_OK) st = nrs_range_renew(ctx, &ctx->scratch_range[0], &range_a);
+          if (st == NRS_OK) st = nrs_range_renew(ctx, &ctx->scratch_range[1], &range_b);
+          if (st == NRS_OK) st = nrs_absmax2(ctx, a, (size_t)m * k, range_a, b, (size_t)n * k, range_b);
+        }
         if (st != NRS_OK) return st;
       }
       NRS_PDL_LAUNCH(thin_fold_kernel, dim3((unsigned)((n + 31) / 32), (unsigned)row_blocks), 256, 0, ctx->stream, a, b,

@@ -62,6 +62,7 @@ struct ConvPolicyOf {
   __device__ __forceinline__ uint32_t a_slice_rows() const { return slice_rows; }
   // No finished value exceeds this (a whole warp asks).
   __device__ __forceinline__ float out_bound(float top_a, float top_b, int lane) const {
+    if (!out_hi) return 0.0f;   // only the largest magnitude is asked for
     uint32_t b = 0;
     if (bias)
       for (int n = lane; n < n_ch_out; n += 32) b = pr::seen(b, bias[n]);
@@ -340,17 +341,19 @@ int conv_common(nrs_ctx* ctx, ConvPlan& p) {
   // 32-channel blocks); the caller finds the others still registered and does the work itself.
   const bool whole = pol.out_step == 1 && p.n_ch_out % 32 == 0;
   NrsRange* out_range = nullptr;
-  auto extras = whole ? ctx->out_extras.find(p.out) : ctx->out_extras.end();
+  auto extras = pol.out_step == 1 ? ctx->out_extras.find(p.out) : ctx->out_extras.end();
   if (extras != ctx->out_extras.end()) {
     const NrsOutExtras& e = extras->second;
-    if ((e.relu_mask_src && p.accumulate) ||   // the mask would hit the old content too
+    if (((e.relu_mask_src || e.hi) && !whole) ||
+        (e.relu_mask_src && p.accumulate) ||   // the mask would hit the old content too
         ((e.hi || e.measure) && split && p.accumulate) ||   // no bound of the old content
-        (e.hi && (e.lo != nullptr) != split)) {
+        (e.hi && (e.lo != nullptr) != split) || (e.measure && !split)) {
       extras = ctx->out_extras.end();
     } else {
       pol.mask_src = e.relu_mask_src; pol.out_hi = e.hi; pol.out_lo = e.lo;
-      if (split && (e.hi || e.measure)) {
-        const int got = nrs_range_renew(ctx, e.hi ? (const void*)e.hi : (const void*)p.out, &out_range);
+      out_range = e.measure;
+      if (split && e.hi) {
+        const int got = nrs_range_renew(ctx, e.hi, &out_range);
         if (got != NRS_OK) return got;
       }
     }

@@ -63,6 +63,7 @@ struct GemmPolicy {
   __device__ __forceinline__ float dact(float src) const { return x.dact == NRS_ACT_RELU ? (src > 0.0f ? 1.0f : 0.0f) : nrs_gelu_d(src); }
   // No finished value exceeds this (a whole warp asks).
   __device__ __forceinline__ float out_bound(float top_a, float top_b, int lane) const {
+    if (!x.hi) return 0.0f;   // only the largest magnitude is asked for
     uint32_t b = 0;
     if (bias)
       for (int n = lane; n < N; n += 32) b = pr::seen(b, bias[n]);
@@ -257,10 +258,10 @@ int dispatch(nrs_ctx* ctx, tc::TilePlan tile, bool split, const Operand& A, cons
   if (extras) {
     pol.x = *extras;
     pol.vec_ok = pol.vec_ok && aligned(extras->pre) && aligned(extras->dact_src);
-    pol.x.range = nullptr;
-    if (split && (extras->hi || extras->measure)) {
-      NRS_REQUIRE(ctx, !extras->hi || pol.beta == 0.0f, NRS_ERR_ARG, "tc_gemm: no planes of an accumulated result");
-      const int st = nrs_range_renew(ctx, extras->hi ? extras->hi : pol.C, &extras->range);
+    if (!split) pol.x.range = nullptr;
+    if (split && extras->hi) {
+      NRS_REQUIRE(ctx, pol.beta == 0.0f, NRS_ERR_ARG, "tc_gemm: no planes of an accumulated result");
+      const int st = nrs_range_renew(ctx, extras->hi, &extras->range);
       if (st != NRS_OK) return st;
       pol.x.range = extras->range;
     }

@@ -50,22 +50,22 @@ pair_unpack_kernel(const float* __restrict__ hi, const float* __restrict__ lo, c
     dst[i] = fmaf(__half2float(reinterpret_cast<const __half*>(lo)[i]), pr::kLoUnscale, __half2float(reinterpret_cast<const __half*>(hi)[i])) * unscale;
 }
 
-// The scale of planes whose values `*top` bounds; one thread of the grid leaves it as their range.
-__device__ __forceinline__ float open_range(const float* top, NrsRange* range) {
-  const float bound = *reinterpret_cast<const volatile float*>(top);
-  if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) {
-    range->bound = bound;
-    if (top != &range->top) range->top = bound;
-  }
-  return pr::scale_of(bound);
-}
+// Where the bound of a tensor's planes comes from: *top, or a scan of the `scan_n` values at src by every block.
+struct Bound {
+  const float* top;
+  const float* src;
+  int scan_n;
+  NrsRange* range;
+};
+template <bool SPLIT>
+__device__ __forceinline__ float open_range(const Bound& b) { return SPLIT ? pr::open_range(b.top, b.src, b.scan_n, b.range) : 1.0f; }
 
 template <bool SPLIT>
 __global__ void __launch_bounds__(256)
 stage_rows_kernel(const float* __restrict__ src, float* __restrict__ hi, float* __restrict__ lo, int rows, int K,
-                  int ldk, size_t src_bstride, size_t dst_bstride, NrsRange* range) {
+                  int ldk, size_t src_bstride, size_t dst_bstride, const Bound bound) {
   NRS_PDL_PROLOGUE();
-  const float scale = SPLIT ? open_range(&range->top, range) : 1.0f;
+  const float scale = open_range<SPLIT>(bound);
   const int b = blockIdx.y;
   src += b * src_bstride;
   const size_t dst = b * dst_bstride;
@@ -93,10 +93,10 @@ stage_rows_kernel(const float* __restrict__ src, float* __restrict__ hi, float* 
 template <bool SPLIT>
 __global__ void __launch_bounds__(256)
 stage_transpose_kernel(const float* __restrict__ src, float* __restrict__ hi, float* __restrict__ lo, int rows, int K,
-                       int ldk, size_t src_bstride, size_t dst_bstride, NrsRange* range) {
+                       int ldk, size_t src_bstride, size_t dst_bstride, const Bound bound) {
   NRS_PDL_PROLOGUE();
   __shared__ float tile[32][33];
-  const float scale = SPLIT ? open_range(&range->top, range) : 1.0f;
+  const float scale = open_range<SPLIT>(bound);
   const int b = blockIdx.z;
   src += b * src_bstride;
   const size_t dst = b * dst_bstride;
@@ -130,10 +130,10 @@ stage_transpose_kernel(const float* __restrict__ src, float* __restrict__ hi, fl
 template <bool SPLIT, bool SUMS>
 __global__ void __launch_bounds__(256)
 stage_image_kernel(const float* __restrict__ src, float* __restrict__ hi, float* __restrict__ lo, float* __restrict__ chan_partial, const img::Grid g,
-                   NrsRange* range) {
+                   const Bound bound) {
   NRS_PDL_PROLOGUE();
   __shared__ img::Tile tile;
-  const float scale = SPLIT ? open_range(&range->top, range) : 1.0f;
+  const float scale = open_range<SPLIT>(bound);
   const uint32_t p0 = blockIdx.x * img::kTilePx;
   const int c0 = blockIdx.y * img::kTileCh, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const img::Pixels px(g, p0);
@@ -162,9 +162,9 @@ stage_image_kernel(const float* __restrict__ src, float* __restrict__ hi, float*
 template <bool SPLIT>
 __global__ void __launch_bounds__(256)
 stage_conv_weight_kernel(const float* __restrict__ w, float* __restrict__ hi, float* __restrict__ lo, int co_n, int ci_n,
-                         int kh, int kw, int for_dgrad, NrsRange* range) {
+                         int kh, int kw, int for_dgrad, const Bound bound) {
   NRS_PDL_PROLOGUE();
-  const float scale = SPLIT ? open_range(&range->top, range) : 1.0f;
+  const float scale = open_range<SPLIT>(bound);
   const int taps = kh * kw, rows = for_dgrad ? ci_n : co_n, inner = for_dgrad ? co_n : ci_n, ld = (inner + 31) / 32 * 32;
   const size_t total = (size_t)rows * ld * taps;
   const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -190,9 +190,9 @@ template <bool SPLIT, int MODE>
 __global__ void __launch_bounds__(256)
 stage_masked_kernel(const float* __restrict__ g, const float* __restrict__ y, const int32_t* __restrict__ argmax,
                     float* __restrict__ nchw_out, float* __restrict__ hi, float* __restrict__ lo, int c_n, int h,
-                    int w, int k, int oh, int ow, const float* g_top, NrsRange* range) {
+                    int w, int k, int oh, int ow, const Bound bound) {
   NRS_PDL_PROLOGUE();
-  const float scale = SPLIT ? open_range(g_top, range) : 1.0f;
+  const float scale = open_range<SPLIT>(bound);
   __shared__ float tile[32][33];
   const int img = blockIdx.z, hw = h * w;
   const int p0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
@@ -240,9 +240,9 @@ __global__ void __launch_bounds__(256)
 pool2_bwd_planes_kernel(const float* __restrict__ g, const float* __restrict__ pooled, const int32_t* __restrict__ argmax,
                         float* __restrict__ nchw_out, float* __restrict__ hi, float* __restrict__ lo,
                         float* __restrict__ chan_partial /*[gridDim.x][c_n] per-block channel sums, or null*/, int n_img,
-                        int c_n, int h, int w, const float* g_top, NrsRange* range) {
+                        int c_n, int h, int w, const Bound bound) {
   NRS_PDL_PROLOGUE();
-  const float scale = SPLIT ? open_range(g_top, range) : 1.0f;
+  const float scale = open_range<SPLIT>(bound);
   __shared__ float tile[32][129];   // [channel][q*32 + position], q = 2*dy + dx inside the window
   __shared__ long long pix_base[32]; // linear index of each position's top-left pixel, -1 beyond the end
   const int oh = h >> 1, ow = w >> 1, ohw = oh * ow, hw = h * w;
@@ -323,10 +323,10 @@ pool2_bwd_planes_kernel(const float* __restrict__ g, const float* __restrict__ p
 template <bool SPLIT>
 __global__ void __launch_bounds__(256)
 pool2_fwd_planes_kernel(const float* __restrict__ x, float* __restrict__ y, int32_t* __restrict__ argmax,
-                        float* __restrict__ hi, float* __restrict__ lo, int n_img, int c_n, int h, int w, const float* x_top, NrsRange* range) {
+                        float* __restrict__ hi, float* __restrict__ lo, int n_img, int c_n, int h, int w, const Bound bound) {
   NRS_PDL_PROLOGUE();
   __shared__ float tile[32][33];
-  const float scale = SPLIT ? open_range(x_top, range) : 1.0f;
+  const float scale = open_range<SPLIT>(bound);
   const int oh = h >> 1, ow = w >> 1, ohw = oh * ow, hw = h * w;
   const long total_pos = (long)n_img * ohw;
   const long gp0 = (long)blockIdx.x * 32;
@@ -410,12 +410,18 @@ int nrs_pair_unpack(nrs_ctx* ctx, const float* hi, const float* lo, float* dst, 
   return NRS_OK;
 }
 
-// A fresh range for `hi`; *top is what its values are bounded by: the source's own where `known` has it, else measured.
-static int open_planes(nrs_ctx* ctx, const float* hi, const float* src, size_t count, const NrsRange* known, NrsRange** range, const float** top) {
-  int st = nrs_range_renew(ctx, hi, range);
-  if (st == NRS_OK && !known) st = nrs_absmax(ctx, src, count, *range);
-  *top = known ? &known->top : &(*range)->top;
-  return st;
+// A fresh range for `hi` (or the caller's, measured), and where its bound comes from: the source's own where `known` has
+// it, a scan by the staging kernel's blocks for small sources, else a launch that measures.
+static int open_planes(nrs_ctx* ctx, const float* hi, const float* src, size_t count, const NrsRange* known, Bound* b) {
+  *b = Bound{nullptr, src, 0, nullptr};
+  int st = nrs_range_renew(ctx, hi, &b->range);
+  if (st != NRS_OK) return st;
+  b->top = known ? &known->top : &b->range->top;
+  if (known) return NRS_OK;
+  if (count > (size_t)pr::kScanAlone) return nrs_absmax(ctx, src, count, b->range);
+  b->top = nullptr;
+  b->scan_n = (int)count;
+  return NRS_OK;
 }
 
 int nrs_tc_pool2_fwd_planes(nrs_ctx* ctx, const float* x, float* y, int32_t* argmax, float* hi, float* lo, int n, int c,
@@ -425,14 +431,13 @@ int nrs_tc_pool2_fwd_planes(nrs_ctx* ctx, const float* x, float* y, int32_t* arg
   const long blocks = ((long)n * (h / 2) * (w / 2) + 31) / 32;
   if (blocks > 2147483647L || (c + 31) / 32 > 65535) return NRS_ERR_UNSUPPORTED;
   dim3 grid((unsigned)blocks, (unsigned)((c + 31) / 32));
+  Bound bound{};
   if (lo) {
-    NrsRange* range = nullptr;
-    const float* top = nullptr;
-    const int st = open_planes(ctx, hi, x, (size_t)n * c * h * w, x_range, &range, &top);
+    const int st = open_planes(ctx, hi, x, (size_t)n * c * h * w, x_range, &bound);
     if (st != NRS_OK) return st;
-    NRS_PDL_LAUNCH((pool2_fwd_planes_kernel<true>), grid, 256, 0, ctx->stream, x, y, argmax, hi, lo, n, c, h, w, top, range);
+    NRS_PDL_LAUNCH((pool2_fwd_planes_kernel<true>), grid, 256, 0, ctx->stream, x, y, argmax, hi, lo, n, c, h, w, bound);
   } else {
-    NRS_PDL_LAUNCH((pool2_fwd_planes_kernel<false>), grid, 256, 0, ctx->stream, x, y, argmax, hi, nullptr, n, c, h, w, nullptr, nullptr);
+    NRS_PDL_LAUNCH((pool2_fwd_planes_kernel<false>), grid, 256, 0, ctx->stream, x, y, argmax, hi, nullptr, n, c, h, w, bound);
   }
   NRS_LAUNCHED(ctx);
   return NRS_OK;
@@ -447,21 +452,20 @@ int nrs_tc_stage_masked(nrs_ctx* ctx, int mode, const float* g, const float* y, 
   dim3 grid((unsigned)((h * w + 31) / 32), (unsigned)((c + 31) / 32), (unsigned)n);
   if (grid.y > 65535 || grid.z > 65535) return NRS_ERR_UNSUPPORTED;
   const bool split = lo != nullptr;
-  NrsRange* range = nullptr;
-  const float* top = nullptr;
+  Bound bound{};
   if (split) {
-    const int st = open_planes(ctx, hi, g, (size_t)n * c * oh * ow, g_range, &range, &top);
+    const int st = open_planes(ctx, hi, g, (size_t)n * c * oh * ow, g_range, &bound);
     if (st != NRS_OK) return st;
   }
   if (mode == 1 && k == 2 && h % 2 == 0 && w % 2 == 0 && (long)n * (h / 2) * (w / 2) / 32 < 2147483647L) {
     dim3 pgrid((unsigned)(((long)n * (h / 2) * (w / 2) + 31) / 32), (unsigned)((c + 31) / 32));
-    if (split) NRS_PDL_LAUNCH((pool2_bwd_planes_kernel<true>), pgrid, 256, 0, ctx->stream, g, y, argmax, nchw_out, hi, lo, chan_partial, n, c, h, w, top, range);
-    else NRS_PDL_LAUNCH((pool2_bwd_planes_kernel<false>), pgrid, 256, 0, ctx->stream, g, y, argmax, nchw_out, hi, lo, chan_partial, n, c, h, w, top, range);
+    if (split) NRS_PDL_LAUNCH((pool2_bwd_planes_kernel<true>), pgrid, 256, 0, ctx->stream, g, y, argmax, nchw_out, hi, lo, chan_partial, n, c, h, w, bound);
+    else NRS_PDL_LAUNCH((pool2_bwd_planes_kernel<false>), pgrid, 256, 0, ctx->stream, g, y, argmax, nchw_out, hi, lo, chan_partial, n, c, h, w, bound);
     NRS_LAUNCHED(ctx);
     if (chan_partial && chan_partial_rows) *chan_partial_rows = (int)pgrid.x;
     return NRS_OK;
   }
-#define NRS_MASKED(S, M) NRS_PDL_LAUNCH((stage_masked_kernel<S, M>), grid, 256, 0, ctx->stream, g, y, argmax, nchw_out, hi, lo, c, h, w, k, oh, ow, top, range)
+#define NRS_MASKED(S, M) NRS_PDL_LAUNCH((stage_masked_kernel<S, M>), grid, 256, 0, ctx->stream, g, y, argmax, nchw_out, hi, lo, c, h, w, k, oh, ow, bound)
   if (mode == 0) { if (split) NRS_MASKED(true, 0); else NRS_MASKED(false, 0); }
   else { if (split) NRS_MASKED(true, 1); else NRS_MASKED(false, 1); }
 #undef NRS_MASKED
@@ -470,12 +474,11 @@ int nrs_tc_stage_masked(nrs_ctx* ctx, int mode, const float* g, const float* y, 
 }
 
 int nrs_tc_stage(nrs_ctx* ctx, const float* src, float* hi, float* lo, int rows, int K, int ldk, int batch,
-                 size_t src_bstride, size_t dst_bstride, bool src_k_by_rows, NrsRange* measured) {
+                 size_t src_bstride, size_t dst_bstride, bool src_k_by_rows, NrsRange* measured, const NrsRange* known) {
   if (rows <= 0 || K <= 0 || batch <= 0) return NRS_OK;
-  NrsRange* range = measured;
-  if (lo && !range) {
-    const float* top = nullptr;
-    const int st = open_planes(ctx, hi, src, batch == 1 ? (size_t)rows * K : src_bstride * (batch - 1) + (size_t)rows * K, nullptr, &range, &top);
+  Bound bound{measured ? &measured->top : nullptr, src, 0, measured};
+  if (lo && !measured) {
+    const int st = open_planes(ctx, hi, src, batch == 1 ? (size_t)rows * K : src_bstride * (batch - 1) + (size_t)rows * K, known, &bound);
     if (st != NRS_OK) return st;
   }
   if (!src_k_by_rows) {
@@ -484,31 +487,31 @@ int nrs_tc_stage(nrs_ctx* ctx, const float* src, float* hi, float* lo, int rows,
     if (blocks > cap) blocks = cap;
     if (batch > 65535) return NRS_ERR_UNSUPPORTED;
     dim3 grid((unsigned)blocks, (unsigned)batch);
-    if (lo) NRS_PDL_LAUNCH((stage_rows_kernel<true>), grid, 256, 0, ctx->stream, src, hi, lo, rows, K, ldk, src_bstride, dst_bstride, range);
-    else NRS_PDL_LAUNCH((stage_rows_kernel<false>), grid, 256, 0, ctx->stream, src, hi, nullptr, rows, K, ldk, src_bstride, dst_bstride, nullptr);
+    if (lo) NRS_PDL_LAUNCH((stage_rows_kernel<true>), grid, 256, 0, ctx->stream, src, hi, lo, rows, K, ldk, src_bstride, dst_bstride, bound);
+    else NRS_PDL_LAUNCH((stage_rows_kernel<false>), grid, 256, 0, ctx->stream, src, hi, nullptr, rows, K, ldk, src_bstride, dst_bstride, bound);
   } else {
     dim3 grid((unsigned)((rows + 31) / 32), (unsigned)((ldk + 31) / 32), (unsigned)batch);
     if (grid.y > 65535 || grid.z > 65535) return NRS_ERR_UNSUPPORTED;
-    if (lo) NRS_PDL_LAUNCH((stage_transpose_kernel<true>), grid, 256, 0, ctx->stream, src, hi, lo, rows, K, ldk, src_bstride, dst_bstride, range);
-    else NRS_PDL_LAUNCH((stage_transpose_kernel<false>), grid, 256, 0, ctx->stream, src, hi, nullptr, rows, K, ldk, src_bstride, dst_bstride, nullptr);
+    if (lo) NRS_PDL_LAUNCH((stage_transpose_kernel<true>), grid, 256, 0, ctx->stream, src, hi, lo, rows, K, ldk, src_bstride, dst_bstride, bound);
+    else NRS_PDL_LAUNCH((stage_transpose_kernel<false>), grid, 256, 0, ctx->stream, src, hi, nullptr, rows, K, ldk, src_bstride, dst_bstride, bound);
   }
   NRS_LAUNCHED(ctx);
   return NRS_OK;
 }
 
-int nrs_tc_stage_image(nrs_ctx* ctx, const float* src, float* hi, float* lo, int n, int c, int hw, float* chan_partial) {
+int nrs_tc_stage_image(nrs_ctx* ctx, const float* src, float* hi, float* lo, int n, int c, int hw, float* chan_partial,
+                       const NrsRange* known) {
   if (n <= 0 || c <= 0 || hw <= 0) return NRS_OK;
   const int ld = nrs_plane_ld(c);
-  if (hw == 1) return nrs_tc_stage(ctx, src, hi, lo, n, c, ld, 1, 0, 0, false);   // already pixel-major: split only
+  if (hw == 1) return nrs_tc_stage(ctx, src, hi, lo, n, c, ld, 1, 0, 0, false, nullptr, known);   // already pixel-major: split only
   if ((size_t)n * hw > 0x7fffffffu) return NRS_ERR_UNSUPPORTED;
   const img::Grid g(n, c, hw);
-  NrsRange* range = nullptr;
-  const float* top = nullptr;
+  Bound bound{};
   if (lo) {
-    const int st = open_planes(ctx, hi, src, (size_t)n * c * hw, nullptr, &range, &top);
+    const int st = open_planes(ctx, hi, src, (size_t)n * c * hw, known, &bound);
     if (st != NRS_OK) return st;
   }
-#define NRS_STAGE(S, C) NRS_PDL_LAUNCH((stage_image_kernel<S, C>), g.blocks(), 256, 0, ctx->stream, src, hi, lo, chan_partial, g, range)
+#define NRS_STAGE(S, C) NRS_PDL_LAUNCH((stage_image_kernel<S, C>), g.blocks(), 256, 0, ctx->stream, src, hi, lo, chan_partial, g, bound)
   if (lo) { if (chan_partial) NRS_STAGE(true, true); else NRS_STAGE(true, false); }
   else { if (chan_partial) NRS_STAGE(false, true); else NRS_STAGE(false, false); }
 #undef NRS_STAGE
@@ -520,14 +523,13 @@ int nrs_tc_stage_conv_weight(nrs_ctx* ctx, const float* w, float* hi, float* lo,
                              int for_dgrad) {
   const size_t total = (size_t)(for_dgrad ? ci : co) * (((for_dgrad ? co : ci) + 31) / 32 * 32) * kh * kw;
   if (total == 0) return NRS_OK;
+  Bound bound{};
   if (lo) {
-    NrsRange* range = nullptr;
-    const float* top = nullptr;
-    const int st = open_planes(ctx, hi, w, (size_t)co * ci * kh * kw, nullptr, &range, &top);
+    const int st = open_planes(ctx, hi, w, (size_t)co * ci * kh * kw, nullptr, &bound);
     if (st != NRS_OK) return st;
-    NRS_PDL_LAUNCH((stage_conv_weight_kernel<true>), nrs_blocks(total, 256), 256, 0, ctx->stream, w, hi, lo, co, ci, kh, kw, for_dgrad, range);
+    NRS_PDL_LAUNCH((stage_conv_weight_kernel<true>), nrs_blocks(total, 256), 256, 0, ctx->stream, w, hi, lo, co, ci, kh, kw, for_dgrad, bound);
   } else {
-    NRS_PDL_LAUNCH((stage_conv_weight_kernel<false>), nrs_blocks(total, 256), 256, 0, ctx->stream, w, hi, nullptr, co, ci, kh, kw, for_dgrad, nullptr);
+    NRS_PDL_LAUNCH((stage_conv_weight_kernel<false>), nrs_blocks(total, 256), 256, 0, ctx->stream, w, hi, nullptr, co, ci, kh, kw, for_dgrad, bound);
   }
   NRS_LAUNCHED(ctx);
   return NRS_OK;
