@@ -40,6 +40,7 @@ struct HeadPolicy {
   float *hi, *lo;      // planes of the result, or null; same addressing
   size_t ldc, hs, bs;
   int M, N, heads;
+  NrsFastDiv div_heads;
   bool vec;            // rows start on 16 bytes
   // Causal products: kTiles: result tiles above the diagonal do not exist.  kUpTo: K-slices beyond the tile's last row
   // are zero.  kFrom: K-slices before the tile's first row are zero.
@@ -50,7 +51,7 @@ struct HeadPolicy {
   const NrsRange *r0, *r1, *r2;
   static constexpr bool kCanEmit = false, kMaySplit = false;
   static constexpr bool kAMnMajor = AMN, kBMnMajor = BMN;
-  static constexpr int kEpiWarps = 16;
+  static constexpr int kEpiWarps = 16, kTeamWarps = 4;
   int order() const { return causal; }   // the same numbers
   __device__ __forceinline__ float out_bound(float, float, int) const {
     return fminf(factor * fmaxf(r0 ? r0->top : 0.0f, r1 ? r1->top * r2->top : 0.0f), 3.0e38f);
@@ -65,7 +66,7 @@ struct HeadPolicy {
   struct Cursor { int k, row, h, b; };
   template <int KW>
   __device__ __forceinline__ Cursor cursor(int tile_m, int batch, int kb) const {
-    const int b = batch / heads;
+    const int b = (int)div_heads.div((uint32_t)batch);
     return Cursor{kb * tc::BK, tile_m * tc::BM, batch - b * heads, b};
   }
   template <int KW>
@@ -93,7 +94,7 @@ struct HeadPolicy {
   __device__ __forceinline__ void store(int, int, int, int, float, float, uint32_t&) const {}   // no K-split
   template <bool SPLIT>
   __device__ __forceinline__ void epilogue(int tile_m, int batch, int row0, int n, float4 (&v)[4], float out_scale, uint32_t& top) const {
-    const int b = batch / heads, m0 = tile_m * tc::BM + row0, nn = N - n;
+    const int b = (int)div_heads.div((uint32_t)batch), m0 = tile_m * tc::BM + row0, nn = N - n;
     const size_t at0 = (size_t)b * bs + (size_t)(batch - b * heads) * hs + (size_t)m0 * ldc + n;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -142,7 +143,7 @@ struct Out {
 template <bool AMN, bool BMN>
 int product(nrs_ctx* ctx, const HeadMat& A, const HeadMat& B, const Out& o, int batch, int heads, int m, int n, int k, int causal) {
   auto ok16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
-  HeadPolicy<AMN, BMN> pol{o.c, o.hi, o.lo, o.ld, o.hs, o.bs, m, n, heads, false, causal, o.factor, o.r0, o.r1, o.r2};
+  HeadPolicy<AMN, BMN> pol{o.c, o.hi, o.lo, o.ld, o.hs, o.bs, m, n, heads, NrsFastDiv(heads), false, causal, o.factor, o.r0, o.r1, o.r2};
   pol.vec = o.ld % 4 == 0 && o.hs % 4 == 0 && o.bs % 4 == 0 && ok16(o.c) && ok16(o.hi) && ok16(o.lo);
   const bool split = ctx->math_mode == NRS_MATH_3XTF32;
   NrsProfScope prof(ctx, NRS_PROF_GEMM, 2.0 * batch * heads * m * n * k * (causal ? 0.5 : 1.0));

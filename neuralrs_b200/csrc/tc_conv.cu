@@ -36,6 +36,7 @@ namespace {
 
 template <int EPI>
 struct ConvPolicyOf {
+  NrsFastDiv div_Wt, div_Ht, div_tiles_x, div_tiles_y;
   int Wt, Ht, Nt, tiles_x, tiles_y;   // pixel tile in the space of (u, v), the pixels this launch computes
   int sub_h, sub_w;                   // extents of that space
   int out_h, out_w;                   // the tensor written: pixel (u, v) is (u*out_step + out_y0, v*out_step + out_x0)
@@ -69,10 +70,12 @@ struct ConvPolicyOf {
     return pr::product_bound(k_total, top_a, top_b, __uint_as_float(__reduce_max_sync(0xffffffffu, b)));
   }
   __device__ __forceinline__ void origin(int tile_m, int* x0, int* y0, int* n0) const {
-    const int tx = tile_m % tiles_x, t = tile_m / tiles_x;
-    *x0 = tx * Wt;
-    *y0 = (t % tiles_y) * Ht;
-    *n0 = (t / tiles_y) * Nt;
+    uint32_t t, tx, n, ty;
+    div_tiles_x.divmod((uint32_t)tile_m, t, tx);
+    div_tiles_y.divmod(t, n, ty);
+    *x0 = (int)tx * Wt;
+    *y0 = (int)ty * Ht;
+    *n0 = (int)n * Nt;
   }
   // Position of a K-slice: tap (i, j), channel block cb; the box origin of tap (i, j) and the weight column.
   struct Cursor { int b_col, cb, i, j, x, y, n, x_first; };
@@ -122,8 +125,8 @@ struct ConvPolicyOf {
     if (row >= Wt * Ht * Nt) return false;
     int x0, y0, n0;
     origin(tile_m, &x0, &y0, &n0);
-    const int t = row / Wt;
-    const int nt = t / Ht;
+    const int t = (int)div_Wt.div((uint32_t)row);
+    const int nt = (int)div_Ht.div((uint32_t)t);
     const int v = x0 + row - t * Wt, u = y0 + t - nt * Ht, n = n0 + nt;
     if (n >= n_img || u >= sub_h || v >= sub_w) return false;
     const int y = u * out_step + out_y0, x = v * out_step + out_x0;
@@ -151,7 +154,7 @@ struct ConvPolicyOf {
   static constexpr bool kMaySplit = true;
   __device__ __forceinline__ bool clip(int, int, int, int*, int*) const { return true; }
   int order() const { return tc::kRaster; }
-  static constexpr int kEpiWarps = EPI;   // see may_take_eight_warps
+  static constexpr int kEpiWarps = EPI, kTeamWarps = EPI == 16 ? 8 : 4;   // see takes_sixteen_warps
   __device__ __forceinline__ float* colsum_row(int tile_m, int q) const {
     return colsum_partial ? colsum_partial + ((size_t)tile_m * 4 + q) * n_ch_out : nullptr;
   }
@@ -166,64 +169,65 @@ struct ConvPolicyOf {
     origin(tile_m, &w.x0, &w.y0, &w.n0);
     return w;
   }
-  // One accumulator row, channels [nb, nb+32) as far as they exist: bias, activation, accumulate, mask,
+  // One accumulator row, channels [nb, nb + W) as far as they exist: bias, activation, accumulate, mask,
   // NCHW store; the finished values come back in v (zeros for rows and channels outside the tensor) so the
   // caller can emit them as planes.  Loads are issued in batches ahead of the stores.
-  __device__ __forceinline__ void epilogue(const Row& rw, int nb, const uint32_t (&r)[32], float (&v)[32]) const {
+  template <int W>
+  __device__ __forceinline__ void epilogue(const Row& rw, int nb, const uint32_t (&r)[W], float (&v)[W]) const {
     if (!rw.live) {
 #pragma unroll
-      for (int j = 0; j < 32; ++j) v[j] = 0.0f;
+      for (int j = 0; j < W; ++j) v[j] = 0.0f;
       return;
     }
     // Whole channel blocks take their own instantiation: with per-channel conditions the loads of a block no longer
     // issue together (measured on the 64-channel data gradient with mask and planes: 69 -> 217 us).
-    if (n_ch_out - nb >= 32) finish<true>(rw.off, nb, r, v);
+    if (n_ch_out - nb >= W) finish<true>(rw.off, nb, r, v);
     else finish<false>(rw.off, nb, r, v);
   }
-  template <bool FULL>
-  __device__ __forceinline__ void finish(size_t off, int nb, const uint32_t (&r)[32], float (&v)[32]) const {
+  template <bool FULL, int W>
+  __device__ __forceinline__ void finish(size_t off, int nb, const uint32_t (&r)[W], float (&v)[W]) const {
     const size_t plane = (size_t)out_h * out_w;
     float* dst = out + off + (size_t)nb * plane;
-    const int nch = FULL ? 32 : n_ch_out - nb;   // channels of this block that exist
+    const int nch = FULL ? W : n_ch_out - nb;   // channels of this block that exist
 #pragma unroll
-    for (int j = 0; j < 32; ++j) v[j] = (FULL || j < nch) ? __uint_as_float(r[j]) : 0.0f;
+    for (int j = 0; j < W; ++j) v[j] = (FULL || j < nch) ? __uint_as_float(r[j]) : 0.0f;
     if (bias) {
 #pragma unroll
-      for (int j = 0; j < 32; ++j)
+      for (int j = 0; j < W; ++j)
         if (FULL || j < nch) v[j] += __ldg(bias + nb + j);
     }
     if (act != NRS_ACT_NONE) {
 #pragma unroll
-      for (int j = 0; j < 32; ++j) v[j] = nrs_apply_act(v[j], act);
+      for (int j = 0; j < W; ++j) v[j] = nrs_apply_act(v[j], act);
     }
     if (accumulate) {
-      float o[32];
+      float o[W];
 #pragma unroll
-      for (int j = 0; j < 32; ++j) o[j] = (FULL || j < nch) ? dst[(size_t)j * plane] : 0.0f;
+      for (int j = 0; j < W; ++j) o[j] = (FULL || j < nch) ? dst[(size_t)j * plane] : 0.0f;
 #pragma unroll
-      for (int j = 0; j < 32; ++j) v[j] += o[j];
+      for (int j = 0; j < W; ++j) v[j] += o[j];
     }
     if (FULL && mask_src) {   // a mask is taken for whole channel blocks only
       const float* m = mask_src + off + (size_t)nb * plane;
-      float mv[32];
+      float mv[W];
 #pragma unroll
-      for (int j = 0; j < 32; ++j) mv[j] = __ldg(m + (size_t)j * plane);
+      for (int j = 0; j < W; ++j) mv[j] = __ldg(m + (size_t)j * plane);
 #pragma unroll
-      for (int j = 0; j < 32; ++j) v[j] = mv[j] > 0.0f ? v[j] : 0.0f;
+      for (int j = 0; j < W; ++j) v[j] = mv[j] > 0.0f ? v[j] : 0.0f;
     }
     if (FULL && skip_out) return;
 #pragma unroll
-    for (int j = 0; j < 32; ++j)
+    for (int j = 0; j < W; ++j)
       if (FULL || j < nch) dst[(size_t)j * plane] = v[j];
   }
 };
 
 using ConvPolicy = ConvPolicyOf<4>;
 
-// 3xTF32 launches of 64 columns and more take two epilogue warps per lane quarter: with the products at the f16 rate the
-// epilogue (activation or mask, NCHW store, split and staging) is the longer part of most tiles.  TF32 keeps one (two: 1.5 %
-// slower).
-constexpr bool takes_eight_warps(int bn, int nplanes) { return bn >= 64 && nplanes == 2; }
+// 3xTF32 launches take four epilogue warps per lane quarter, 16 columns at a time: with the products at the f16 rate the
+// epilogue (activation or mask, NCHW store, split and staging) is the longer part of most tiles, and it is latency: one
+// warp with 32 columns took 2 thousand clocks a block and spilled.  TF32 keeps one (two: 1.5 % slower).
+constexpr bool takes_sixteen_warps(int nplanes) { return nplanes == 2; }
 
 // One axis of a (sub-)problem: `len` output pixels at positions u*step + first, `taps` kernel taps tap0,
 // tap0 + tap_step, ..., and the activation coordinate of tap t for pixel u: u * in_step + base + sgn * t.
@@ -279,11 +283,11 @@ int run_conv(nrs_ctx* ctx, const ConvPlan& p, const float* a_hi, const float* a_
     if (pol.out_lo) ok = ok && tc::encode_tmap(&to_lo, pol.out_lo, kHalf, 4, odim, ostr, obox);
   }
   NRS_REQUIRE(ctx, ok, NRS_ERR_CUDA, "tc_conv: cuTensorMapEncodeTiled failed");
-  if constexpr (takes_eight_warps(BN, NPLANES)) {
-    ConvPolicyOf<8> wide;
+  if constexpr (takes_sixteen_warps(NPLANES)) {
+    ConvPolicyOf<16> wide;
     static_assert(sizeof(wide) == sizeof(pol), "the same fields");
     std::memcpy(&wide, &pol, sizeof(wide));
-    return tc::launch<BN, NPLANES, PAIR, KW, ConvPolicyOf<8>>(ctx, ta_hi, ta_lo, tb_hi, tb_lo, wide, tiles_m, p.n_ch_out, 1,
+    return tc::launch<BN, NPLANES, PAIR, KW, ConvPolicyOf<16>>(ctx, ta_hi, ta_lo, tb_hi, tb_lo, wide, tiles_m, p.n_ch_out, 1,
                                                             p.ay.taps * p.ax.taps * pol.cblocks, rg, pol.out_hi ? &to_hi : nullptr,
                                                             pol.out_lo ? &to_lo : nullptr, splits_out);
   } else {
@@ -335,6 +339,8 @@ int conv_common(nrs_ctx* ctx, ConvPlan& p) {
   pol.sgn = p.sgn; pol.base_y = p.ay.base; pol.base_x = p.ax.base;
   pol.w_tap0 = p.ay.tap0 * p.kw + p.ax.tap0; pol.w_tap_row = p.ay.tap_step * p.kw; pol.w_tap_col = p.ax.tap_step;
   pol.out = p.out; pol.bias = p.bias; pol.act = p.act; pol.accumulate = p.accumulate;
+  pol.div_Wt = NrsFastDiv(pol.Wt); pol.div_Ht = NrsFastDiv(pol.Ht);
+  pol.div_tiles_x = NrsFastDiv(pol.tiles_x); pol.div_tiles_y = NrsFastDiv(pol.tiles_y);
   pol.slice_rows = (uint32_t)(pol.Wt * pol.Ht * pol.Nt);
   pol.k_total = (float)p.a_ch * p.ay.taps * p.ax.taps;
   // Requests of the caller are honoured where this launch writes every pixel of the output (planes: whole

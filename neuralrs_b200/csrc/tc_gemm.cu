@@ -38,7 +38,7 @@ struct GemmPolicy {
   __device__ __forceinline__ bool clip(int, int, int, int*, int*) const { return true; }
   // The epilogue is latency (TMEM, loads, GELU at about 66 instructions a value): four warps per lane quarter.  With two,
   // a 128 x 128 tile with GELU and three outputs took 27 thousand clocks, twice its main loop at K = 512.
-  static constexpr int kEpiWarps = 16;
+  static constexpr int kEpiWarps = 16, kTeamWarps = 4;
   int order() const { return tc::kRaster; }
 
   __device__ __forceinline__ uint32_t a_slice_rows() const { return tc::BM; }   // of A, that a load brings

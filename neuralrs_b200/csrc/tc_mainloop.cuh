@@ -95,6 +95,7 @@ struct SplitInfo {
   int chunks;          // > 1 (splits == 1 then): K-chunks that a CTA takes one after the other
   int kb_total;        // K-slices in all
   int batches;
+  NrsFastDiv div_splits;
   float* partial;      // [split][batch][tiles_m*128][n_total] when splits > 1; [CTA][128][BN] when chunks > 1
   int n_total;
   int rows_total;      // tiles_m * 128
@@ -112,19 +113,29 @@ struct TileMap {
   int tiles_m, tiles_n;
   long total;          // tiles_m * tiles_n * batches * splits (kTriangle: the tiles that exist)
   int order, planes, per_plane;
+  NrsFastDiv div_planes, div_plane, div_group, div_tiles_n, div_last;   // (integer divisions took each role 2 thousand clocks a tile)
+  void finish() {
+    div_planes = NrsFastDiv(planes);
+    div_plane = NrsFastDiv(per_plane);
+    div_group = NrsFastDiv(kGroupM * tiles_n);
+    div_tiles_n = NrsFastDiv(tiles_n);
+    div_last = NrsFastDiv(tiles_m % kGroupM ? tiles_m % kGroupM : kGroupM);   // row tiles of the last group
+  }
   template <int BN>
   __device__ __forceinline__ void decode(long t, int* tile_m, int* tile_n, int* z) const {
     const uint32_t u = (uint32_t)t;   // (launch() checks the range)
+    uint32_t a, b;
     if (order >= kLastFirst) {
-      const uint32_t mn = u / (uint32_t)planes;
-      *z = (int)(u - mn * planes);
-      const int m = (int)(mn / (uint32_t)tiles_n);
-      *tile_n = (int)(mn - (uint32_t)m * tiles_n);
-      *tile_m = order == kLastFirst ? tiles_m - 1 - m : m;
+      div_planes.divmod(u, a, b);
+      *z = (int)b;
+      const uint32_t m = div_tiles_n.div(a);
+      *tile_n = (int)(a - m * (uint32_t)tiles_n);
+      *tile_m = order == kLastFirst ? tiles_m - 1 - (int)m : (int)m;
       return;
     }
-    *z = (int)(u / (uint32_t)per_plane);
-    const int r = (int)(u - (uint32_t)*z * per_plane);
+    div_plane.divmod(u, a, b);
+    *z = (int)a;
+    const int r = (int)b;
     if (order == kTriangle) {
       int m = 0, left = r;
       for (int cnt; left >= (cnt = min(tiles_n, (m * BM + BM - 1) / BN + 1)); ++m) left -= cnt;
@@ -132,11 +143,9 @@ struct TileMap {
       *tile_n = left;
       return;
     }
-    const int group = r / (kGroupM * tiles_n);
-    const int first = group * kGroupM;
+    const int group = (int)div_group.div((uint32_t)r), first = group * kGroupM, rr = r - group * kGroupM * tiles_n;
     const int gm = min(kGroupM, tiles_m - first);
-    const int rr = r - group * kGroupM * tiles_n;
-    *tile_n = rr / gm;
+    *tile_n = (int)(gm == kGroupM ? (uint32_t)rr / kGroupM : div_last.div((uint32_t)rr));
     *tile_m = first + (rr - *tile_n * gm);
   }
   // The tile that CTA `me` of `step` takes in the round that starts at `base`; -1: none.
@@ -146,10 +155,10 @@ struct TileMap {
   }
 };
 
-// Shared memory of the epilogue: a plane-emission staging tile per four warps, [128 rows][128 B] (pairs: [128 rows][64 B] of
+// Shared memory of the epilogue: a plane-emission staging tile per team of warps (which take 32 columns together), [128 rows][128 B] (pairs: [128 rows][64 B] of
 // hi, then of lo), or (row-major results) a 32 x 16 transpose tile per warp.
 template <int NPLANES, class Policy>
-__host__ __device__ constexpr int emit_bytes() { return Policy::kCanEmit ? Policy::kEpiWarps / 4 * BM * 128 : Policy::kEpiWarps * 2048; }
+__host__ __device__ constexpr int emit_bytes() { return Policy::kCanEmit ? Policy::kEpiWarps / Policy::kTeamWarps * BM * 128 : Policy::kEpiWarps * 2048; }
 template <class Policy>
 __host__ __device__ constexpr int threads() { return 64 + 32 * Policy::kEpiWarps; }
 
@@ -213,7 +222,7 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
     if (emit >= 1) prefetch_tmap(&tm_out_hi);
     if (emit == 2) prefetch_tmap(&tm_out_lo);
     for (int s = 0; s < L::kStages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-    for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], Policy::kEpiWarps * (PAIR ? 2 : 1)); mbar_init(&emit_bars[b], 128); mbar_init(&emit_bars[2 + b], 128); }
+    for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], Policy::kEpiWarps * (PAIR ? 2 : 1)); for (int t = 0; t < 2; ++t) mbar_init(&emit_bars[2 * t + b], Policy::kTeamWarps * 32); }
     fence_barrier_init();
   }
   if (warp == 1) {
@@ -242,7 +251,7 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
       int tile_m, tile_n, z;
       tmap.template decode<BN>(t, &tile_m, &tile_n, &z);
       if (PAIR) tile_m = 2 * tile_m + rank;   // beyond the last row tile: TMA fills zeros
-      const int batch = z / sp.splits, split = z - batch * sp.splits;
+      const int batch = (int)sp.div_splits.div((uint32_t)z), split = z - batch * sp.splits;
       int kb_begin = split * sp.kb_per_split;
       int kb_end = sp.chunks > 1 ? sp.kb_total : min(sp.kb_total, kb_begin + sp.kb_per_split);
       if (!pol.clip(tile_m, tile_n, BN, &kb_begin, &kb_end)) continue;
@@ -314,7 +323,7 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
         if (t < 0) break;
         int tile_m, tile_n, z;
         tmap.template decode<BN>(t, &tile_m, &tile_n, &z);
-        const int split = z % sp.splits;
+        const int split = z - (int)sp.div_splits.div((uint32_t)z) * sp.splits;
         int kb_begin = split * sp.kb_per_split, kb_end = sp.chunks > 1 ? sp.kb_total : min(sp.kb_total, kb_begin + sp.kb_per_split);
         if (!pol.clip(tile_m, tile_n, BN, &kb_begin, &kb_end)) continue;
         for (int k0 = kb_begin; k0 < kb_end && ok; k0 += sp.kb_per_split) {
@@ -368,9 +377,10 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
     // ---------------- epilogue: warp w owns TMEM lanes [32*(w%4), +32)
     const int q = warp & 3;
     const int row = q * 32 + lane;   // row inside the tile
-    // (kCanEmit: every four warps take 32-column blocks of their own, with a staging tile and an issuing thread)
-    const int team = (warp - 2) >> 2;
-    const bool emit_issuer = ((warp - 2) & 3) == 0 && lane == 0;
+    // (kCanEmit: every team of warps takes 32-column blocks of its own, with a staging tile and an issuing thread; four
+    // warps have a whole block each for their lanes' rows, eight half of one)
+    const int team = (warp - 2) / Policy::kTeamWarps, half = Policy::kTeamWarps == 8 ? ((warp - 2) >> 2) & 1 : 0;
+    const bool emit_issuer = (warp - 2) % Policy::kTeamWarps == 0 && lane == 0;
     uint64_t* emit_bar = emit_bars + (Policy::kCanEmit ? 2 * team : 0);
     uint8_t* team_tile = emit_tile + (Policy::kCanEmit ? team * BM * 128 : 0);
     [[maybe_unused]] float us_a = 1.0f, us_b = 1.0f, out_scale = 1.0f;
@@ -394,7 +404,7 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
       int tile_m, tile_n, z;
       tmap.template decode<BN>(t, &tile_m, &tile_n, &z);
       if (PAIR) tile_m = 2 * tile_m + rank;
-      const int batch = z / sp.splits, split = z - batch * sp.splits;
+      const int batch = (int)sp.div_splits.div((uint32_t)z), split = z - batch * sp.splits;
       int kb_begin = split * sp.kb_per_split, kb_end = sp.chunks > 1 ? sp.kb_total : min(sp.kb_total, kb_begin + sp.kb_per_split);
       if (!pol.clip(tile_m, tile_n, BN, &kb_begin, &kb_end)) continue;   // the same verdict in all three roles
       const int n0 = tile_n * BN;
@@ -415,8 +425,8 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
         };
         // The warps of a lane quarter share its column blocks out; those without one just hand the accumulator back, and so
         // do all of a pair's second CTA beyond the last row tile.
-        constexpr int kW = Policy::kCanEmit ? 32 : 16, kBlocks = BN / kW, kStep = Policy::kEpiWarps / 4;
-        const int c_first = kStep == 1 ? 0 : (warp - 2) >> 2;
+        constexpr int kW = Policy::kCanEmit && Policy::kTeamWarps == 4 ? 32 : 16, kBlocks = BN / kW, kStep = Policy::kEpiWarps / 4;
+        const int c_first = kStep == 1 ? 0 : (warp - 2) >> 2;   // (a team of eight: 2 * team + half)
         if (c_first >= kBlocks || (PAIR && tile_m * BM >= sp.rows_total)) {
           hand_back();
           continue;
@@ -471,25 +481,25 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
           } else if (sp.splits > 1) {
             float* dst = sp.partial + (((size_t)split * sp.batches + batch) * sp.rows_total + (size_t)tile_m * BM + row) * sp.n_total;
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              const int n = n0 + c * 32 + j;
+            for (int j = 0; j < kW; ++j) {
+              const int n = n0 + c * kW + j;
               if (n < sp.n_total) dst[n] = __uint_as_float(r[j]);
             }
           } else {
-            float v[32];
-            pol.epilogue(rw, n0 + c * 32, r, v);
+            float v[kW];
+            pol.epilogue(rw, n0 + c * kW, r, v);
             if (NPLANES == 2 && rg.out) {
 #pragma unroll
-              for (int j = 0; j < 32; ++j) top = pr::seen(top, v[j]);
+              for (int j = 0; j < kW; ++j) top = pr::seen(top, v[j]);
             }
             if (float* cs = pol.colsum_row(tile_m, q)) {
-              // Sum over this warp's 32 rows, one channel per lane: a 32 x 32 transpose-reduce in 31
-              // shuffles (each stage halves the values a lane holds; fixed order, deterministic).
-              float s[32];
+              // Sum over this warp's 32 rows, one channel per lane: a transpose-reduce (each stage halves the values a lane
+              // holds; fixed order, deterministic): 31 shuffles for 32 channels, 16 for 16.
+              float s[kW];
 #pragma unroll
-              for (int j = 0; j < 32; ++j) s[j] = v[j];
+              for (int j = 0; j < kW; ++j) s[j] = v[j];
 #pragma unroll
-              for (int d = 16; d >= 1; d >>= 1) {
+              for (int d = kW / 2; d >= 1; d >>= 1) {
                 const bool up = (lane & d) != 0;
 #pragma unroll
                 for (int i = 0; i < d; ++i) {
@@ -498,7 +508,8 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
                   s[i] = keep + __shfl_xor_sync(0xffffffffu, send, d);
                 }
               }
-              cs[n0 + c * 32 + lane] = s[0];
+              if (kW == 16) s[0] += __shfl_xor_sync(0xffffffffu, s[0], 16);
+              if (lane < kW) cs[n0 + c * kW + lane] = s[0];
             }
             if (emit) {
               // The staging tile is free once the previous TMA store has read it; the issuer
@@ -511,15 +522,15 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
               if constexpr (NPLANES == 2) {
                 uint8_t* row_hi = team_tile + row * 64;
 #pragma unroll
-                for (int g = 0; g < 4; ++g) {   // eight values
-                  const int chunk = (g ^ ((row >> 1) & 3)) * 16;   // 64-byte swizzle
+                for (int g = 0; g < kW / 8; ++g) {   // eight values
+                  const int chunk = ((g + 2 * half) ^ ((row >> 1) & 3)) * 16;   // 64-byte swizzle
                   uint2 h0, l0, h1, l1;
                   pr::split4(make_float4(v[8 * g], v[8 * g + 1], v[8 * g + 2], v[8 * g + 3]), out_scale, &h0, &l0);
                   pr::split4(make_float4(v[8 * g + 4], v[8 * g + 5], v[8 * g + 6], v[8 * g + 7]), out_scale, &h1, &l1);
                   *reinterpret_cast<uint4*>(row_hi + chunk) = make_uint4(h0.x, h0.y, h1.x, h1.y);
                   *reinterpret_cast<uint4*>(row_hi + BM * 64 + chunk) = make_uint4(l0.x, l0.y, l1.x, l1.y);
                 }
-              } else {
+              } else if constexpr (kW == 32) {
                 uint8_t* row_hi = team_tile + row * 128;
 #pragma unroll
                 for (int g = 0; g < 8; ++g) {
@@ -531,8 +542,8 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
               mbar_arrive(&emit_bar[1]);
               if (emit_issuer) {
                 if (!mbar_wait(&emit_bar[1], ph)) { atomicExch(err_flag, kErrEpilogueWait); ok = false; break; }
-                tma_store_4d(&tm_out_hi, team_tile, n0 + c * 32, rw.x0, rw.y0, rw.n0);
-                if (NPLANES == 2) tma_store_4d(&tm_out_lo, team_tile + BM * 64, n0 + c * 32, rw.x0, rw.y0, rw.n0);
+                tma_store_4d(&tm_out_hi, team_tile, n0 + c / (32 / kW) * 32, rw.x0, rw.y0, rw.n0);
+                if (NPLANES == 2) tma_store_4d(&tm_out_lo, team_tile + BM * 64, n0 + c / (32 / kW) * 32, rw.x0, rw.y0, rw.n0);
                 bulk_commit();
               }
             }
@@ -681,6 +692,7 @@ int launch(nrs_ctx* ctx, const CUtensorMap& ta_hi, const CUtensorMap& ta_lo, con
     sp.kb_per_split = kb_total;
   }
   sp.kb_total = kb_total;
+  sp.div_splits = NrsFastDiv(sp.splits);
   sp.batches = batches;
   sp.n_total = n_total;
   sp.rows_total = tiles_m * BM;
@@ -697,11 +709,13 @@ int launch(nrs_ctx* ctx, const CUtensorMap& ta_hi, const CUtensorMap& ta_lo, con
   int st = nrs_err_flag(ctx, &err);
   if (st != NRS_OK) return st;
   const int units_m = PAIR ? (tiles_m + 1) / 2 : tiles_m;
-  TileMap tmap{units_m, tiles_n, 0, pol.order(), batches * sp.splits, units_m * tiles_n};
+  TileMap tmap{};
+  tmap.tiles_m = units_m; tmap.tiles_n = tiles_n; tmap.order = pol.order(); tmap.planes = batches * sp.splits; tmap.per_plane = units_m * tiles_n;
   if (tmap.order == kTriangle) {
     tmap.per_plane = 0;
     for (int m = 0; m < tiles_m; ++m) tmap.per_plane += std::min(tiles_n, (m * BM + BM - 1) / BN + 1);
   }
+  tmap.finish();
   tmap.total = (long)tmap.per_plane * tmap.planes;
   NRS_REQUIRE(ctx, (long)units_m * tiles_n <= 0x7fffffffL && tmap.total <= 0x7fffffffL, NRS_ERR_SHAPE, "tensor-core product: too many tiles");
   const long slots = PAIR ? ctx->sm_count / 2 : ctx->sm_count;
