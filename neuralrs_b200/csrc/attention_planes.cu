@@ -297,10 +297,7 @@ head_dsoftmax_kernel(const float* __restrict__ p_hi, const float* __restrict__ p
       }
     }
   }
-  if (lo) {
-    __syncwarp();
-    pr::report(range, top);
-  }
+  if (lo) pr::report_block(range, top);
 }
 
 int row_blocks(const nrs_ctx* ctx, long rows) {

@@ -398,7 +398,7 @@ bn_normalize_planes_kernel(const float* __restrict__ x, const float* __restrict_
   }
   __syncthreads();
   img::tile_to_planes<SPLIT>(tile, g, p0, c0, hi, lo, scale);
-  if (SPLIT) pr::report(range, top);
+  if (SPLIT) pr::report_block(range, top);
 }
 
 // dx (overwritten; null: planes only) with its NHWC planes, and chan_partial[tile of 128 pixels][c], its sums over the tile.
@@ -451,7 +451,7 @@ bn_dx_planes_kernel(const float* __restrict__ gr, const float* __restrict__ x, c
   }
   __syncthreads();
   img::tile_to_planes<SPLIT>(tile, g, p0, c0, hi, lo, scale);
-  if (SPLIT) pr::report(range, top);
+  if (SPLIT) pr::report_block(range, top);
 }
 
 // Statistics shared by several processes: the splits of this process folded in order into out[ch], the

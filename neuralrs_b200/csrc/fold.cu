@@ -96,8 +96,8 @@ __device__ void fold_tiles(const NrsFoldJob& j, const FoldDiv& dv, unsigned blk,
   if (j.kind == NRS_FOLD_WGRAD) {                 // [m block][group][column block][128][group_cols]
     const int mb = co >> 7, row = co & 127;
     const int grp = (int)dv.group.div((uint32_t)tap), t = tap - grp * j.taps_per_group;
-    const int cbk = j.col_blocks > 1 ? c >> 8 : 0;
-    const size_t col = j.col_blocks > 1 ? (size_t)(c - cbk * 256) : (size_t)t * j.cblocks * 32 + c;
+    const int cbk = j.col_blocks > 1 ? c >> (31 - __clz(j.group_cols)) : 0;   // (column blocks are a power of two wide)
+    const size_t col = j.col_blocks > 1 ? (size_t)(c - cbk * j.group_cols) : (size_t)t * j.cblocks * 32 + c;
     off = ((((size_t)mb * j.n_groups + grp) * j.col_blocks + cbk) * 128 + row) * j.group_cols + col;
   } else {                                        // rows kernel: a (horizontal j, vertical i) pair per tap
     const int i = (int)((unsigned)tap / 3u), jt = tap - 3 * i;

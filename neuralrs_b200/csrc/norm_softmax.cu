@@ -275,8 +275,11 @@ ln_fwd_vec_kernel(const float* __restrict__ a, const float* __restrict__ b, cons
     }
   }
   if (EMIT && y_lo) {
-    pr::report(range, top);
-    if (istd_range) pr::report(istd_range, top_istd);
+    pr::report_block(range, top);
+    if (istd_range) {
+      __syncthreads();
+      pr::report_block(istd_range, top_istd);
+    }
   }
 }
 
@@ -379,7 +382,7 @@ ln_bwd_vec_kernel(const float* __restrict__ g, const float* __restrict__ xhat, c
       }
     }
   }
-  if (EMIT && d_lo) pr::report(range, top);
+  if (EMIT && d_lo) pr::report_block(range, top);
   if (partial) {
     float* mine = ln_smem + (size_t)wrp * 2 * f;
 #pragma unroll

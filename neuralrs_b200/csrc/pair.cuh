@@ -79,7 +79,7 @@ __device__ __forceinline__ uint32_t seen4(uint32_t top, float4 v) { return seen(
 // A whole warp's, into the tensor's range.
 __device__ __forceinline__ void report(NrsRange* r, uint32_t top) {
   top = __reduce_max_sync(0xffffffffu, top);
-  if ((threadIdx.x & 31) == 0 && top > __float_as_uint(*(volatile float*)&r->top)) atomicMax(reinterpret_cast<unsigned*>(&r->top), top);
+  if ((threadIdx.x & 31) == 0) atomicMax(reinterpret_cast<unsigned*>(&r->top), top);   // (no result: nothing waits for it)
 }
 // What one block finds in n values (all of its threads ask; at most kScanAlone values, else absmax_kernel measures them).
 constexpr int kScanAlone = 32768;
@@ -110,6 +110,16 @@ __device__ __forceinline__ float open_range(const float* top, const float* src, 
     if (top != &range->top) range->top = bound;
   }
   return scale_of(bound);
+}
+// The same for a whole block (all of its threads ask).
+__device__ __forceinline__ void report_block(NrsRange* r, uint32_t top) {
+  __shared__ uint32_t all;
+  if (threadIdx.x == 0) all = 0;
+  __syncthreads();
+  top = __reduce_max_sync(0xffffffffu, top);
+  if ((threadIdx.x & 31) == 0) atomicMax(&all, top);
+  __syncthreads();
+  if (threadIdx.x == 0) atomicMax(reinterpret_cast<unsigned*>(&r->top), all);
 }
 // Bound of a sum of `k` products of values up to a and b, plus a value up to c: with room for the sum's own rounding,
 // and finite.

@@ -92,20 +92,35 @@ struct GemmPolicy {
     }
   }
   __device__ __forceinline__ int row(int, int, int) const { return 0; }
-  // Four row segments of a warp's 32 x 16 block: row r0 + 8*i of the tile, columns n..n+3 (see tc::rows_to_lines).
+  // Four row segments of a warp's 32 x 16 block: row r0 + 8*i of the tile, columns n..n+3 (see tc::rows_to_lines).  Blocks
+  // that lie inside C on 16-byte boundaries, nearly all of them, take an instantiation without the checks.
   template <bool SPLIT>
   __device__ __forceinline__ void epilogue(int tile_m, int batch, int r0, int n, float4 (&v)[4], float out_scale, uint32_t& top) const {
+    const int nb = n - (int)(threadIdx.x & 3) * 4;
+    if (vec_ok && (tile_m + 1) * tc::BM <= M && nb + 16 <= N) finish<SPLIT, true>(tile_m, batch, r0, n, v, out_scale, top);
+    else finish<SPLIT, false>(tile_m, batch, r0, n, v, out_scale, top);
+  }
+  template <bool SPLIT, bool INSIDE>
+  __device__ __forceinline__ void finish(int tile_m, int batch, int r0, int n, float4 (&v)[4], float out_scale, uint32_t& top) const {
     const int m0 = tile_m * tc::BM + r0, nn = N - n;   // nn: how many of the four columns exist (four or more: all)
-    const size_t at0 = (size_t)batch * batch_stride + (size_t)m0 * N + n, step = (size_t)8 * N;
+    const size_t at0 = (size_t)batch * batch_stride + (size_t)m0 * N + n;
+    const uint32_t step = 8u * (uint32_t)N;
+    auto row = [&](int i) { return INSIDE || m0 + 8 * i < M; };
+    auto get = [&](const float* p) { return INSIDE ? *reinterpret_cast<const float4*>(p) : tc::load_guarded(p, nn, vec_ok); };
+    auto put = [&](float* p, float4 q) {
+      if (INSIDE) *reinterpret_cast<float4*>(p) = q;
+      else tc::store_guarded(p, q, nn, vec_ok);
+    };
     if (bias) {
-      const float4 b = tc::load_guarded(bias + n, nn, vec_ok);
+      const float4 b = get(bias + n);
 #pragma unroll
       for (int i = 0; i < 4; ++i) { v[i].x += b.x; v[i].y += b.y; v[i].z += b.z; v[i].w += b.w; }
     }
     if (x.pre) {
+      float* p = x.pre + at0;
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-        if (m0 + 8 * i < M) tc::store_guarded(x.pre + at0 + i * step, v[i], nn, vec_ok);
+      for (int i = 0; i < 4; ++i, p += step)
+        if (row(i)) put(p, v[i]);
     }
     if (act != NRS_ACT_NONE) {
 #pragma unroll
@@ -116,39 +131,40 @@ struct GemmPolicy {
     }
     if (beta != 0.0f) {
       float4 o[4];
+      const float* p = C + at0;
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-        o[i] = m0 + 8 * i < M ? tc::load_guarded(C + at0 + i * step, nn, vec_ok) : make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int i = 0; i < 4; ++i, p += step) o[i] = row(i) ? get(p) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
       for (int i = 0; i < 4; ++i) { v[i].x += beta * o[i].x; v[i].y += beta * o[i].y; v[i].z += beta * o[i].z; v[i].w += beta * o[i].w; }
     }
     if (!x.skip_c && !x.skip_c_unsplit) {
+      float* p = C + at0;
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-        if (m0 + 8 * i < M) tc::store_guarded(C + at0 + i * step, v[i], nn, vec_ok);
+      for (int i = 0; i < 4; ++i, p += step)
+        if (row(i)) put(p, v[i]);
     }
     if (x.dact != NRS_ACT_NONE) {
       float4 s[4];
+      const float* p = x.dact_src + at0;
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-        s[i] = m0 + 8 * i < M ? tc::load_guarded(x.dact_src + at0 + i * step, nn, vec_ok) : make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int i = 0; i < 4; ++i, p += step) s[i] = row(i) ? get(p) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
       for (int i = 0; i < 4; ++i) { v[i].x *= dact(s[i].x); v[i].y *= dact(s[i].y); v[i].z *= dact(s[i].z); v[i].w *= dact(s[i].w); }
     }
     if (SPLIT && x.range) {
 #pragma unroll
       for (int i = 0; i < 4; ++i)
-        if (m0 + 8 * i < M) top = pr::seen4(top, v[i]);
+        if (row(i)) top = pr::seen4(top, v[i]);
     }
     if (x.hi) {
+      size_t at = at0;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        if (m0 + 8 * i >= M) continue;
+      for (int i = 0; i < 4; ++i, at += step) {
+        if (!row(i)) continue;
         if (SPLIT) {   // (n is a multiple of 8, so all four columns exist or none)
-          if (nn >= 4) pr::put4(x.hi, x.lo, at0 + i * step, v[i], out_scale);
+          if (INSIDE || nn >= 4) pr::put4(x.hi, x.lo, at, v[i], out_scale);
         } else {
-          const float4 h = make_float4(tc::tf32_rn(v[i].x), tc::tf32_rn(v[i].y), tc::tf32_rn(v[i].z), tc::tf32_rn(v[i].w));
-          tc::store_guarded(x.hi + at0 + i * step, h, nn, vec_ok);
+          put(x.hi + at, make_float4(tc::tf32_rn(v[i].x), tc::tf32_rn(v[i].y), tc::tf32_rn(v[i].z), tc::tf32_rn(v[i].w)));
         }
       }
     }
@@ -156,13 +172,13 @@ struct GemmPolicy {
       float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
       for (int i = 0; i < 4; ++i)
-        if (m0 + 8 * i < M) { s.x += v[i].x; s.y += v[i].y; s.z += v[i].z; s.w += v[i].w; }
+        if (row(i)) { s.x += v[i].x; s.y += v[i].y; s.z += v[i].z; s.w += v[i].w; }
 #pragma unroll
       for (int d = 4; d <= 16; d <<= 1) {
         s.x += __shfl_xor_sync(0xffffffffu, s.x, d); s.y += __shfl_xor_sync(0xffffffffu, s.y, d);
         s.z += __shfl_xor_sync(0xffffffffu, s.z, d); s.w += __shfl_xor_sync(0xffffffffu, s.w, d);
       }
-      if ((threadIdx.x & 31) < 4) tc::store_guarded(x.colsum + ((size_t)tile_m * 4 + (r0 >> 5)) * N + n, s, nn, vec_ok);
+      if ((threadIdx.x & 31) < 4) put(x.colsum + ((size_t)tile_m * 4 + (r0 >> 5)) * N + n, s);
     }
   }
 };

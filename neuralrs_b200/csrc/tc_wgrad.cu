@@ -48,8 +48,8 @@ struct WgradParams {
   int ragged_a, ragged_x;         // channel count no multiple of 32: one 4-D box per block instead of one 5-D box for all
   int m_blocks;                   // ceil(co / 128)
   float* partial;                 // [split][m_block][group][col_block][128][group_cols]
-  int group_cols;                 // taps_per_group * cblocks * 32 (more than 256 input channels: 256)
-  int col_blocks;                 // more than 256 input channels: column blocks of 256, each its own CTA
+  int group_cols;                 // taps_per_group * cblocks * wb; in column blocks: the width of one (64, 128 or 256)
+  int col_blocks;                 // column blocks of the input channels, each its own CTA (more than 256 channels, or 1x1)
   int independent;                // reads nothing the kernel launched just before it wrote (NRS_PDL_PROLOGUE)
   const NrsRange *range_dy, *range_x;   // 3xTF32
   float* direct;                  // 1x1, one split, no accumulation: the tile is the result; written straight to dw[co][ci]
@@ -78,7 +78,7 @@ tc_wgrad_kernel(const __grid_constant__ CUtensorMap tm_dy_hi, const __grid_const
   const int mb = mg / p.n_groups, grp = mg - mb * p.n_groups;
   const int split = blockIdx.y;
   // blocks of x this CTA's columns cover (a column block of a wide layer may be ragged)
-  const int most = kMaxN / p.wb, cblocks = p.col_blocks > 1 ? min(most, p.cblocks - cbk * most) : p.cblocks;
+  const int most = p.group_cols / p.wb, cblocks = p.col_blocks > 1 ? min(most, p.cblocks - cbk * most) : p.cblocks;
   const int t_begin = split * p.tiles_per_split;
   const int t_end = min(p.n_tiles, t_begin + p.tiles_per_split);
   const int ntiles = t_end - t_begin;
@@ -220,7 +220,7 @@ tc_wgrad_kernel(const __grid_constant__ CUtensorMap tm_dy_hi, const __grid_const
       tc::tc_fence_after_sync();
       const int row = q * 32 + lane;
       const int live_cols = (p.col_blocks > 1 ? cblocks : ntaps * p.cblocks) * p.wb;
-      float* dst = p.direct ? p.direct + (size_t)(mb * 128 + row) * p.ci + (size_t)cbk * 256
+      float* dst = p.direct ? p.direct + (size_t)(mb * 128 + row) * p.ci + (size_t)cbk * p.group_cols
                             : p.partial + (((((size_t)split * p.m_blocks + mb) * p.n_groups + grp) * p.col_blocks + cbk) * 128 + row) *
                                               p.group_cols;
       const bool row_live = mb * 128 + row < p.co;
@@ -344,42 +344,76 @@ int nrs_tc_conv_wgrad(nrs_ctx* ctx, const float* x, const float* dy, float* dw, 
     p.taps_per_group = 1;
     p.group_cols = kMaxN;
   }
-  const size_t pixel_bytes = (size_t)(128 + p.group_cols) * 4;   // both operands, all planes
-  plan_pixel_box(&p, n, oh, ow, planes, pixel_bytes);
-  if (p.kp == 0) return NRS_ERR_UNSUPPORTED;
-  p.tiles_x = (ow + p.Wt - 1) / p.Wt;
-  p.tiles_y = (oh + p.Ht - 1) / p.Ht;
-  const long n_tiles = (long)((n + p.Nt - 1) / p.Nt) * p.tiles_y * p.tiles_x;
-  if (n_tiles > 2147483647L) return NRS_ERR_UNSUPPORTED;
-  p.n_tiles = (int)n_tiles;
-
-  // ring depth from the shared-memory budget
-  const size_t stage_bytes = pixel_bytes * p.kp;
-  int stages = (int)((200 * 1024) / stage_bytes);
-  if (stages < 2) return NRS_ERR_UNSUPPORTED;
-  if (stages > 6) stages = 6;
-  const size_t smem_bytes = stages * stage_bytes + 1024 + 256;
-
-  // pixel split: fill the GPU, and bound the accumulation chain in 3xTF32 mode
-  const int ctas_per_split = p.m_blocks * p.n_groups * p.col_blocks;
-  const int max_tiles = split3 ? tc::kMaxChainK / p.kp : 1 << 30;
-  int min_tiles = 512 / p.kp;   // amortise the prologue and the partial-tile store
-  // ... unless that leaves most of the GPU idle (a short reduction with a small output: Linear layers)
-  while (min_tiles > 4 && (long)(p.n_tiles / min_tiles) * ctas_per_split < ctx->sm_count / 2) min_tiles /= 2;
-  if (min_tiles > max_tiles) min_tiles = max_tiles;
-  int tps = tc::plan_units_per_cta(ctx->sm_count, ctas_per_split, p.n_tiles, min_tiles, max_tiles, 8);
-  // A short reduction with a large output (a Linear layer at a batch of a hundred: 7 tiles, 8 MB) is better walked by
-  // one CTA per output tile, which then is the result: a split's second pass reads splits + 1 times the output at about
-  // 1.1 KB a clock, and a CTA's own time is about 2 clocks per plane product, pixel and 32 columns.
   const bool can_be_direct = taps == 1 && ci % p.wb == 0 && !accumulate && !out_cols && (reinterpret_cast<uintptr_t>(dw) & 15) == 0;
-  if (can_be_direct && tps < p.n_tiles && p.n_tiles <= max_tiles) {
-    const int s = (p.n_tiles + tps - 1) / tps;
-    auto clocks = [&](int tiles, int splits) {
-      const double rounds = (double)((ctas_per_split * splits + ctx->sm_count - 1) / ctx->sm_count);
-      return rounds * tiles * (p.kp + 6) * (split3 ? 3 : 1) * (p.group_cols / 32) * 2.0;
-    };
-    if (clocks(p.n_tiles, 1) < clocks(tps, s) + (s + 1.0) * co * ci * 4 / 1100.0) tps = p.n_tiles;
+  // The pixel box of a plan, and the ring its operands allow; false where there is none.
+  size_t pixel_bytes = 0;
+  int stages = 0;
+  auto box = [&](WgradParams* q) {
+    pixel_bytes = (size_t)(128 + q->group_cols) * 4;   // both operands, all planes
+    q->kp = 0;
+    plan_pixel_box(q, n, oh, ow, planes, pixel_bytes);
+    if (q->kp == 0) return false;
+    q->tiles_x = (ow + q->Wt - 1) / q->Wt;
+    q->tiles_y = (oh + q->Ht - 1) / q->Ht;
+    const long n_tiles = (long)((n + q->Nt - 1) / q->Nt) * q->tiles_y * q->tiles_x;
+    if (n_tiles > 2147483647L) return false;
+    q->n_tiles = (int)n_tiles;
+    stages = (int)((200 * 1024) / (pixel_bytes * q->kp));
+    if (stages > 6) stages = 6;
+    return stages >= 2;
+  };
+  int tps = 0;   // pixel tiles per CTA
+  if (taps == 1) {
+    // A^T B: columns per CTA and pixel split together, by what a CTA takes (its UMMAs, 46 clocks at least, or its operands'
+    // way at about 60 bytes a clock; 2500 clocks and the store of its tile besides) and the second pass, which reads
+    // splits + 1 times the output at about 1.1 KB a clock.  No split is longer than an accumulation chain may be.
+    // (dW of 256 x 256 over 4096 rows: with 256 columns eight splits of two CTAs.)
+    const WgradParams base = p;
+    double best = -1.0;
+    for (int cols : {256, 128, 64}) {
+      WgradParams q = base;
+      if (cols < tap_cols || tap_cols > kMaxN) {
+        q.col_blocks = (tap_cols + cols - 1) / cols;
+        q.n_groups = q.taps_per_group = 1;
+        q.group_cols = cols;
+      } else if (cols != 256) {
+        continue;   // one CTA takes all columns as it is
+      }
+      if (!box(&q)) continue;
+      const int max_tiles = split3 ? tc::kMaxChainK / q.kp : 1 << 30, ctas = q.m_blocks * q.col_blocks;
+      const double umma = (split3 ? 3.0 : 2.0) * std::max(q.group_cols / 2, 47), fill = 16.0 * pixel_bytes / 60.0;   // per 16 pixels
+      for (int i = 1, last = 0; i <= 96; ++i) {   // up to 64 splits, then whole waves
+        const long s = i <= 64 ? i : (long)(i - 64) * ctx->sm_count / ctas;
+        if (s < 1 || (i > 64 && s <= 64)) continue;
+        const int per = (int)((q.n_tiles + s - 1) / s);
+        if (per > max_tiles || per == last || s > 65535) continue;
+        last = per;
+        const long splits = (q.n_tiles + per - 1) / per;
+        const double rounds = (double)((ctas * splits + ctx->sm_count - 1) / ctx->sm_count);
+        const double fold = s == 1 && can_be_direct ? 0.0 : (splits + 1.0) * co * ci * 4 / 1100.0;
+        const double cost = rounds * (per * (q.kp / 16.0) * std::max(umma, fill) + 2500.0 + 4.0 * q.group_cols) + fold;
+        if (best < 0.0 || cost < best) {
+          best = cost;
+          tps = per;
+          p = q;
+        }
+      }
+    }
+    // (a reduction that needs more splits by the chain limit alone)
+    if (best < 0.0 && box(&p)) tps = std::max(1, split3 ? tc::kMaxChainK / p.kp : p.n_tiles);
+    if (tps == 0 || !box(&p)) return NRS_ERR_UNSUPPORTED;
+  } else {
+    if (!box(&p)) return NRS_ERR_UNSUPPORTED;
+    // pixel split: fill the GPU, and bound the accumulation chain in 3xTF32 mode
+    const int ctas_per_split = p.m_blocks * p.n_groups * p.col_blocks;
+    const int max_tiles = split3 ? tc::kMaxChainK / p.kp : 1 << 30;
+    int min_tiles = 512 / p.kp;   // amortise the prologue and the partial-tile store
+    // ... unless that leaves most of the GPU idle
+    while (min_tiles > 4 && (long)(p.n_tiles / min_tiles) * ctas_per_split < ctx->sm_count / 2) min_tiles /= 2;
+    if (min_tiles > max_tiles) min_tiles = max_tiles;
+    tps = tc::plan_units_per_cta(ctx->sm_count, ctas_per_split, p.n_tiles, min_tiles, max_tiles, 8);
   }
+  const size_t smem_bytes = stages * pixel_bytes * p.kp + 1024 + 256;
   p.tiles_per_split = tps;
   const int splits = (p.n_tiles + tps - 1) / tps;
   if (splits > 65535) return NRS_ERR_UNSUPPORTED;
@@ -424,7 +458,7 @@ int nrs_tc_conv_wgrad(nrs_ctx* ctx, const float* x, const float* dy, float* dw, 
     const uint32_t es[5] = {1, (uint32_t)step, (uint32_t)step, 1, 1};
     return tc::encode_tmap(m, base, split3, ragged ? 4 : 5, dim, str, box, true, es);
   };
-  const int x_blocks = p.col_blocks > 1 ? kMaxN / p.wb : p.cblocks;
+  const int x_blocks = p.col_blocks > 1 ? p.group_cols / p.wb : p.cblocks;
   bool ok = encode(&maps[0], dy_hi, p.ragged_a, co, p.wa, dy_ld, oh, ow, 1, p.a_box_blocks) &&
             encode(&maps[2], x_hi, p.ragged_x, ci, p.wb, x_ld, h, wd, stride, x_blocks);
   if (split3) ok = ok && encode(&maps[1], dy_lo, p.ragged_a, co, p.wa, dy_ld, oh, ow, 1, p.a_box_blocks) &&
