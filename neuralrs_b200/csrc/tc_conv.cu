@@ -34,9 +34,12 @@
 
 namespace {
 
-template <int EPI>
+template <int EPI, bool SLAB>
 struct ConvPolicyOf {
-  NrsFastDiv div_Wt, div_Ht, div_tiles_x, div_tiles_y;
+  static constexpr bool kSlab = SLAB;
+  // A tile's pixels in the order of its box: (x, y, image), in slabs (x, image, y), so that a row of all its images is one
+  // stretch of the slab and the next vertical tap starts Wt * Nt pixels on.
+  NrsFastDiv div_Wt, div_mid /*Ht; slabs: Nt*/, div_tiles_x, div_tiles_y, div_cblocks;
   int Wt, Ht, Nt, tiles_x, tiles_y;   // pixel tile in the space of (u, v), the pixels this launch computes
   int sub_h, sub_w;                   // extents of that space
   int out_h, out_w;                   // the tensor written: pixel (u, v) is (u*out_step + out_y0, v*out_step + out_x0)
@@ -49,6 +52,7 @@ struct ConvPolicyOf {
   float* out;
   const float* bias;
   int act, accumulate;
+  int taps_y;                         // slabs: vertical taps that one serves
   uint32_t slice_rows;                // pixels of a tile's box
   float k_total;                      // terms of a sum, for the result's bound
   // optional: ReLU mask taken from an NCHW tensor of the output's shape, and NHWC TF32 planes of
@@ -61,6 +65,13 @@ struct ConvPolicyOf {
   bool skip_out;   // the finished values leave as planes and channel sums only (a K-split's second pass writes them still)
 
   __device__ __forceinline__ uint32_t a_slice_rows() const { return slice_rows; }
+  __device__ __forceinline__ uint32_t slab_rows() const { return (uint32_t)(Wt * Nt * (Ht + taps_y - 1)); }
+  __device__ __forceinline__ int slab_taps() const { return taps_y; }
+  __device__ __forceinline__ uint32_t slab_tap_row(int i) const { return (uint32_t)((sgn > 0 ? i : taps_y - 1 - i) * Wt * Nt); }
+  template <class Cur>
+  __device__ __forceinline__ int slab_weight(const Cur& c, int i) const { return (w_tap0 + i * w_tap_row + c.j * w_tap_col) * cblocks + c.cb; }
+  template <int KW, class Cur>
+  __device__ __forceinline__ int slab_column(const Cur& c, int i) const { return slab_weight(c, i) * KW; }
   // No finished value exceeds this (a whole warp asks).
   __device__ __forceinline__ float out_bound(float top_a, float top_b, int lane) const {
     if (!out_hi) return 0.0f;   // only the largest magnitude is asked for
@@ -82,16 +93,16 @@ struct ConvPolicyOf {
   template <int KW>
   __device__ __forceinline__ Cursor cursor(int tile_m, int, int kb) const {
     Cursor c;
-    const int tap = kb / cblocks;
+    const int tap = (int)div_cblocks.div((uint32_t)kb);
     c.cb = kb - tap * cblocks;
-    c.i = tap / tap_cols;
+    c.i = SLAB || tap == 0 ? 0 : tap / tap_cols;
     c.j = tap - c.i * tap_cols;
     int x0, y0;
     origin(tile_m, &x0, &y0, &c.n);
     c.x_first = x0 * in_step + base_x;
     c.x = c.x_first + sgn * c.j;
-    c.y = y0 * in_step + base_y + sgn * c.i;
-    c.b_col = weight_column<KW>(c);
+    c.y = y0 * in_step + base_y + (SLAB ? (sgn > 0 ? 0 : 1 - taps_y) : sgn * c.i);
+    c.b_col = SLAB ? 0 : weight_column<KW>(c);
     return c;
   }
   template <int KW>
@@ -104,6 +115,10 @@ struct ConvPolicyOf {
     if (++c.cb < cblocks) return;
     c.cb = 0;
     c.x += sgn;
+    if (SLAB) {
+      ++c.j;
+      return;
+    }
     if (++c.j == tap_cols) {
       c.j = 0;
       c.x = c.x_first;
@@ -118,7 +133,8 @@ struct ConvPolicyOf {
   }
   template <bool PAIR, int KW, int ROW_BYTES>
   __device__ __forceinline__ void load_a(void* dst, const CUtensorMap* tm, uint32_t bar, const Cursor& c) const {
-    tc::tma_load_4d_to<PAIR>(dst, tm, bar, c.cb * KW, c.x, c.y, c.n);
+    if (SLAB) tc::tma_load_4d_to<PAIR>(dst, tm, bar, c.cb * KW, c.x, c.n, c.y);
+    else tc::tma_load_4d_to<PAIR>(dst, tm, bar, c.cb * KW, c.x, c.y, c.n);
   }
   // NCHW offset of channel 0 of the pixel behind accumulator row `row`, and the pixel's linear index.
   __device__ __forceinline__ bool locate(int tile_m, int row, size_t* nchw_off, size_t* pixel) const {
@@ -126,8 +142,8 @@ struct ConvPolicyOf {
     int x0, y0, n0;
     origin(tile_m, &x0, &y0, &n0);
     const int t = (int)div_Wt.div((uint32_t)row);
-    const int nt = (int)div_Ht.div((uint32_t)t);
-    const int v = x0 + row - t * Wt, u = y0 + t - nt * Ht, n = n0 + nt;
+    const int hi = (int)div_mid.div((uint32_t)t), lo = t - hi * (int)div_mid.d;
+    const int v = x0 + row - t * Wt, u = y0 + (SLAB ? hi : lo), n = n0 + (SLAB ? lo : hi);
     if (n >= n_img || u >= sub_h || v >= sub_w) return false;
     const int y = u * out_step + out_y0, x = v * out_step + out_x0;
     *nchw_off = (size_t)n * n_ch_out * out_h * out_w + (size_t)y * out_w + x;
@@ -222,7 +238,7 @@ struct ConvPolicyOf {
   }
 };
 
-using ConvPolicy = ConvPolicyOf<4>;
+using ConvPolicy = ConvPolicyOf<4, false>;
 
 // 3xTF32 launches take four epilogue warps per lane quarter, 16 columns at a time: with the products at the f16 rate the
 // epilogue (activation or mask, NCHW store, split and staging) is the longer part of most tiles, and it is latency: one
@@ -256,45 +272,44 @@ struct ConvPlan {
   int act, accumulate;
 };
 
-template <int BN, int NPLANES, bool PAIR, int KW>
-int run_conv(nrs_ctx* ctx, const ConvPlan& p, const float* a_hi, const float* a_lo, const ConvPolicy& pol, const tc::Ranges& rg, int tiles_m,
+template <int BN, int NPLANES, bool PAIR, int KW, bool SLAB>
+int run_conv(nrs_ctx* ctx, const ConvPlan& p, const float* a_hi, const float* a_lo, const ConvPolicy& base, const tc::Ranges& rg, int tiles_m,
              int* splits_out) {
   constexpr bool kHalf = NPLANES == 2;
+  using Policy = ConvPolicyOf<takes_sixteen_warps(NPLANES) ? 16 : 4, SLAB>;
+  Policy pol;
+  static_assert(sizeof(pol) == sizeof(base), "the same fields");
+  std::memcpy((void*)&pol, &base, sizeof(pol));
   const int a_ld = nrs_plane_ld(p.a_ch);
   const int kdim = p.kh * p.kw * pol.cblocks * KW;
   CUtensorMap ta_hi, ta_lo, tb_hi, tb_lo;
-  const uint64_t adim[4] = {(uint64_t)p.a_ch, (uint64_t)p.a_w, (uint64_t)p.a_h, (uint64_t)p.n_img};
-  const uint64_t astr[3] = {(uint64_t)a_ld, (uint64_t)p.a_w * a_ld, (uint64_t)p.a_h * p.a_w * a_ld};
-  const uint32_t abox[4] = {(uint32_t)KW, (uint32_t)pol.Wt, (uint32_t)pol.Ht, (uint32_t)pol.Nt};
-  const uint32_t astep[4] = {1, (uint32_t)pol.in_step, (uint32_t)pol.in_step, 1};
+  // An activation-shaped tensor of `c` channels, ld apart, as [n][h][w][c] or (slabs) [h][n][w][c], in boxes of a tile and
+  // `more` rows above it.
+  auto image_map = [&](CUtensorMap* m, const float* at, int c, int ld, int h, int w, int box_c, int more, int step) {
+    const uint64_t row = (uint64_t)w * ld, img = (uint64_t)h * row;
+    const uint64_t dim[4] = {(uint64_t)c, (uint64_t)w, (uint64_t)(SLAB ? p.n_img : h), (uint64_t)(SLAB ? h : p.n_img)};
+    const uint64_t str[3] = {(uint64_t)ld, SLAB ? img : row, SLAB ? row : img};
+    const uint32_t box[4] = {(uint32_t)box_c, (uint32_t)pol.Wt, (uint32_t)(SLAB ? pol.Nt : pol.Ht), (uint32_t)(SLAB ? pol.Ht + more : pol.Nt)};
+    const uint32_t es[4] = {1, (uint32_t)step, (uint32_t)step, 1};
+    return tc::encode_tmap(m, at, kHalf, 4, dim, str, box, false, SLAB ? nullptr : es);
+  };
   const uint64_t bdim[3] = {(uint64_t)kdim, (uint64_t)p.n_ch_out, 1};
   const uint64_t bstr[2] = {(uint64_t)kdim, (uint64_t)kdim * p.n_ch_out};
   const uint32_t bbox[3] = {(uint32_t)KW, (uint32_t)(PAIR ? BN / 2 : BN), 1};
-  bool ok = tc::encode_tmap(&ta_hi, a_hi, kHalf, 4, adim, astr, abox, false, astep) && tc::encode_tmap(&tb_hi, p.w_hi, kHalf, 3, bdim, bstr, bbox);
-  if (kHalf) ok = ok && tc::encode_tmap(&ta_lo, a_lo, true, 4, adim, astr, abox, false, astep) && tc::encode_tmap(&tb_lo, p.w_lo, true, 3, bdim, bstr, bbox);
+  const int more = pol.taps_y - 1;
+  bool ok = image_map(&ta_hi, a_hi, p.a_ch, a_ld, p.a_h, p.a_w, KW, more, pol.in_step) && tc::encode_tmap(&tb_hi, p.w_hi, kHalf, 3, bdim, bstr, bbox);
+  if (kHalf) ok = ok && image_map(&ta_lo, a_lo, p.a_ch, a_ld, p.a_h, p.a_w, KW, more, pol.in_step) && tc::encode_tmap(&tb_lo, p.w_lo, true, 3, bdim, bstr, bbox);
   else { ta_lo = ta_hi; tb_lo = tb_hi; }
   // Output planes (optional): the same box geometry as an activation load, in output space.
   CUtensorMap to_hi, to_lo;
   if (pol.out_hi) {
-    const uint64_t odim[4] = {(uint64_t)p.n_ch_out, (uint64_t)p.out_w, (uint64_t)p.out_h, (uint64_t)p.n_img};
-    const uint32_t obox[4] = {32, abox[1], abox[2], abox[3]};
-    const uint64_t ostr[3] = {(uint64_t)p.n_ch_out, (uint64_t)p.out_w * p.n_ch_out, (uint64_t)p.out_h * p.out_w * p.n_ch_out};
-    ok = ok && tc::encode_tmap(&to_hi, pol.out_hi, kHalf, 4, odim, ostr, obox);
-    if (pol.out_lo) ok = ok && tc::encode_tmap(&to_lo, pol.out_lo, kHalf, 4, odim, ostr, obox);
+    ok = ok && image_map(&to_hi, pol.out_hi, p.n_ch_out, p.n_ch_out, p.out_h, p.out_w, 32, 0, 1);
+    if (pol.out_lo) ok = ok && image_map(&to_lo, pol.out_lo, p.n_ch_out, p.n_ch_out, p.out_h, p.out_w, 32, 0, 1);
   }
   NRS_REQUIRE(ctx, ok, NRS_ERR_CUDA, "tc_conv: cuTensorMapEncodeTiled failed");
-  if constexpr (takes_sixteen_warps(NPLANES)) {
-    ConvPolicyOf<16> wide;
-    static_assert(sizeof(wide) == sizeof(pol), "the same fields");
-    std::memcpy(&wide, &pol, sizeof(wide));
-    return tc::launch<BN, NPLANES, PAIR, KW, ConvPolicyOf<16>>(ctx, ta_hi, ta_lo, tb_hi, tb_lo, wide, tiles_m, p.n_ch_out, 1,
-                                                            p.ay.taps * p.ax.taps * pol.cblocks, rg, pol.out_hi ? &to_hi : nullptr,
-                                                            pol.out_lo ? &to_lo : nullptr, splits_out);
-  } else {
-    return tc::launch<BN, NPLANES, PAIR, KW, ConvPolicy>(ctx, ta_hi, ta_lo, tb_hi, tb_lo, pol, tiles_m, p.n_ch_out, 1,
-                                                         p.ay.taps * p.ax.taps * pol.cblocks, rg, pol.out_hi ? &to_hi : nullptr,
-                                                         pol.out_lo ? &to_lo : nullptr, splits_out);
-  }
+  return tc::launch<BN, NPLANES, PAIR, KW, Policy>(ctx, ta_hi, ta_lo, tb_hi, tb_lo, pol, tiles_m, p.n_ch_out, 1,
+                                                   (SLAB ? 1 : p.ay.taps) * p.ax.taps * pol.cblocks, rg, pol.out_hi ? &to_hi : nullptr,
+                                                   pol.out_lo ? &to_lo : nullptr, splits_out, SLAB ? KW * p.ay.taps : KW);
 }
 
 // Pixel tile: the Wt x Ht x Nt box of at most 128 pixels (a box side times the activation step may not exceed
@@ -322,11 +337,39 @@ void plan_pixel_tile(const ConvPlan& p, ConvPolicy* pol) {
   }
 }
 
+// The same for slabs: rows of 8, 16, 24 or 32 pixels (a slab's taps have to start on whole swizzle patterns, and it has
+// room for tc::kSlabRows pixels).  Taken where that costs at most a tenth more tiles.
+bool plan_slab_tile(const ConvPlan& p, ConvPolicy* pol) {
+  if (p.ax.in_step != 1 || p.ay.in_step != 1 || p.ay.taps < 2) return false;
+  const long plain = (long)pol->tiles_x * pol->tiles_y * ((p.n_img + pol->Nt - 1) / pol->Nt);
+  long best = plain + plain / 10;
+  bool found = false;
+  for (int Wt = 8; Wt <= 32 && Wt < p.ax.len + 8; Wt += 8) {
+    int Ht = tc::BM / Wt;
+    if (Ht > p.ay.len) Ht = p.ay.len;
+    int Nt = 1;
+    if (Ht == p.ay.len && Wt >= p.ax.len) Nt = std::max(1, std::min(p.n_img, tc::BM / (Wt * Ht)));
+    while (Nt > 1 && Wt * Nt * (Ht + p.ay.taps - 1) > tc::kSlabRows) --Nt;
+    while (Ht > 1 && Wt * Nt * (Ht + p.ay.taps - 1) > tc::kSlabRows) --Ht;
+    if (Wt * Nt * (Ht + p.ay.taps - 1) > tc::kSlabRows) continue;
+    const int nx = (p.ax.len + Wt - 1) / Wt, ny = (p.ay.len + Ht - 1) / Ht;
+    const long tiles = (long)nx * ny * ((p.n_img + Nt - 1) / Nt);
+    if (tiles <= best) {   // (among equals the widest rows)
+      best = tiles;
+      pol->Wt = Wt; pol->Ht = Ht; pol->Nt = Nt; pol->tiles_x = nx; pol->tiles_y = ny;
+      found = true;
+    }
+  }
+  return found;
+}
+
 int conv_common(nrs_ctx* ctx, ConvPlan& p) {
   if (p.ax.len < 1 || p.ay.len < 1 || p.ax.taps < 1 || p.ay.taps < 1) return NRS_OK;
   const bool split = ctx->math_mode == NRS_MATH_3XTF32;
   ConvPolicy pol{};
   plan_pixel_tile(p, &pol);
+  const bool slab = plan_slab_tile(p, &pol);
+  pol.taps_y = slab ? p.ay.taps : 1;
   const long tiles_m = (long)((p.n_img + pol.Nt - 1) / pol.Nt) * pol.tiles_y * pol.tiles_x;
   if (tiles_m > 2147483647L) return NRS_ERR_UNSUPPORTED;
   pol.sub_h = p.ay.len; pol.sub_w = p.ax.len;
@@ -339,7 +382,8 @@ int conv_common(nrs_ctx* ctx, ConvPlan& p) {
   pol.sgn = p.sgn; pol.base_y = p.ay.base; pol.base_x = p.ax.base;
   pol.w_tap0 = p.ay.tap0 * p.kw + p.ax.tap0; pol.w_tap_row = p.ay.tap_step * p.kw; pol.w_tap_col = p.ax.tap_step;
   pol.out = p.out; pol.bias = p.bias; pol.act = p.act; pol.accumulate = p.accumulate;
-  pol.div_Wt = NrsFastDiv(pol.Wt); pol.div_Ht = NrsFastDiv(pol.Ht);
+  pol.div_Wt = NrsFastDiv(pol.Wt); pol.div_mid = NrsFastDiv(slab ? pol.Nt : pol.Ht);
+  pol.div_cblocks = NrsFastDiv(pol.cblocks);
   pol.div_tiles_x = NrsFastDiv(pol.tiles_x); pol.div_tiles_y = NrsFastDiv(pol.tiles_y);
   pol.slice_rows = (uint32_t)(pol.Wt * pol.Ht * pol.Nt);
   pol.k_total = (float)p.a_ch * p.ay.taps * p.ax.taps;
@@ -404,15 +448,18 @@ int conv_common(nrs_ctx* ctx, ConvPlan& p) {
   if (extras != ctx->out_extras.end()) ctx->out_extras.erase(extras);   // honoured from here on
   int splits = 0;
   const tc::TilePlan tile = tc::plan_tile(ctx, tiles_m, p.n_ch_out, 1, p.ay.taps * p.ax.taps * blocks32, split, 0.025, true);
-#define NRS_RUN(BN_, PAIR_)                                                                                              \
-  st = !split ? run_conv<BN_, 1, PAIR_, 32>(ctx, p, (const float*)a_hi, nullptr, pol, rg, (int)tiles_m, &splits)                \
-       : wide ? run_conv<BN_, 2, PAIR_, 64>(ctx, p, (const float*)a_hi, (const float*)a_lo, pol, rg, (int)tiles_m, &splits)      \
-              : run_conv<BN_, 2, PAIR_, 32>(ctx, p, (const float*)a_hi, (const float*)a_lo, pol, rg, (int)tiles_m, &splits)
-  if (tile.pair) { if (tile.bn == 128) NRS_RUN(128, true); else NRS_RUN(64, true); }
-  else if (tile.bn == 128) NRS_RUN(128, false);
-  else if (tile.bn == 64) NRS_RUN(64, false);
-  else NRS_RUN(32, false);
+#define NRS_RUN_AS(BN_, PAIR_, SLAB_)                                                                                          \
+  st = !split ? run_conv<BN_, 1, PAIR_, 32, SLAB_>(ctx, p, (const float*)a_hi, nullptr, pol, rg, (int)tiles_m, &splits)          \
+       : wide ? run_conv<BN_, 2, PAIR_, 64, SLAB_>(ctx, p, (const float*)a_hi, (const float*)a_lo, pol, rg, (int)tiles_m, &splits) \
+              : run_conv<BN_, 2, PAIR_, 32, SLAB_>(ctx, p, (const float*)a_hi, (const float*)a_lo, pol, rg, (int)tiles_m, &splits)
+#define NRS_RUN(BN_, PAIR_) { if (slab) NRS_RUN_AS(BN_, PAIR_, true); else NRS_RUN_AS(BN_, PAIR_, false); }
+  if (tile.pair && tile.bn == 128) NRS_RUN(128, true)
+  else if (tile.pair) NRS_RUN(64, true)
+  else if (tile.bn == 128) NRS_RUN(128, false)
+  else if (tile.bn == 64) NRS_RUN(64, false)
+  else NRS_RUN(32, false)
 #undef NRS_RUN
+#undef NRS_RUN_AS
   // channel sums come from the direct epilogue only (a K-split stores through the reduce kernel)
   if (st == NRS_OK && pol.colsum_partial && splits == 1) colsum->second.rows = (int)tiles_m * 4;
   return st;

@@ -32,6 +32,11 @@
 // K (1640), of which the UMMAs alone are 768; x[256,64,32,32] -> 128 channels, 3x3: forward 172 -> 110 us, data gradient
 // 170 -> 119 us.
 //
+// Policy::kSlab (convolutions over a pixel grid): a ring slot of A holds a slab of the activation, some image rows more than
+// the tile has, that serves all vertical taps of a horizontal one: tap i is the same operand some pixels further.  B comes
+// through a ring and a producing warp of its own.  A 3x3 layer thus brings 3 slabs of 1.25 to 1.5 tiles per channel block
+// instead of 9 tiles.
+//
 // What bounds a tile: with 128 columns the tensor pipe, with 64 the way of A through L2 (40 KB per 64 values of K at about
 // 60 bytes a clock) and the 46 clocks that a UMMA takes at least; short reductions the epilogue.  With PAIR the
 // two CTAs of a cluster work on two row tiles of one column tile: each brings its own A rows and half of the B rows, and
@@ -62,9 +67,10 @@ namespace tc {
 constexpr int BM = 128, BK = 32;   // 32 values: 128 bytes of f32, 64 of f16: one swizzle row
 constexpr int kMaxChainK = 4096;   // longest single accumulation chain in 3xTF32 mode
 constexpr int kGroupM = 16;        // row tiles per raster group (see TileMap)
+constexpr int kSlabRows = 192;     // most pixels of a slab of A (see Policy::kSlab)
 
 // KW: values of K in a K-slice, and in a row of it (MN-major operands: columns of a block): 32, or 64 of f16.
-template <int BN, int NPLANES, int EMIT_BYTES, bool PAIR, int KW>
+template <int BN, int NPLANES, int EMIT_BYTES, bool PAIR, int KW, bool SLAB>
 struct SmemLayout {
   static_assert(KW == 32 || (KW == 64 && NPLANES == 2), "a row is at most 128 bytes");
   static constexpr int kRowBytes = KW * (NPLANES == 2 ? 2 : 4);
@@ -73,10 +79,16 @@ struct SmemLayout {
   static constexpr int kSlice = NPLANES * (kATile + kBTile);   // [A_hi][B_hi][B_lo][A_lo]
   static constexpr int kSlices = KW == 64 ? 1 : 2;             // K-slices per ring slot
   static constexpr int kStage = kSlices * kSlice;
-  static constexpr int kExtra = EMIT_BYTES /*plane staging tile*/ + 1024 /*align*/ + 256 /*barriers*/;
+  static constexpr int kExtra = EMIT_BYTES /*plane staging tile*/ + 1024 /*align*/ + 512 /*barriers*/;
   static constexpr int kRing = 227 * 1024 - kExtra;
   static constexpr int kStages = kRing / kStage >= 8 ? 8 : kRing / kStage;
-  static constexpr int kBytes = kStages * kStage + kExtra;
+  // Slabs (Policy::kSlab): a ring of A slabs and a ring of B slices.
+  static constexpr int kSlabPlane = kSlabRows * kRowBytes, kSlab = NPLANES * kSlabPlane, kBSlice = NPLANES * kBTile;
+  static constexpr int kMostA = kSlab > 24 * 1024 ? 3 : 4;
+  static constexpr int kSlabsA = kRing - kMostA * kSlab >= 3 * kBSlice ? kMostA : 2;
+  static constexpr int kSlicesB = (kRing - kSlabsA * kSlab) / kBSlice >= 8 ? 8 : (kRing - kSlabsA * kSlab) / kBSlice;
+  static constexpr int kRingBytes = SLAB ? kSlabsA * kSlab + kSlicesB * kBSlice : kStages * kStage;
+  static constexpr int kBytes = kRingBytes + kExtra;
   static constexpr int kAccCols = NPLANES * BN;                 // one accumulator
   static constexpr int kTmemCols = 2 * kAccCols < 32 ? 32 : 2 * kAccCols;   // two of them
   static_assert((kTmemCols & (kTmemCols - 1)) == 0 && kTmemCols <= 512, "TMEM allocation must be a power of two <= 512");
@@ -160,7 +172,7 @@ struct TileMap {
 template <int NPLANES, class Policy>
 __host__ __device__ constexpr int emit_bytes() { return Policy::kCanEmit ? Policy::kEpiWarps / Policy::kTeamWarps * BM * 128 : Policy::kEpiWarps * 2048; }
 template <class Policy>
-__host__ __device__ constexpr int threads() { return 64 + 32 * Policy::kEpiWarps; }
+__host__ __device__ constexpr int threads() { return 64 + 32 * Policy::kEpiWarps + (Policy::kSlab ? 32 : 0); }
 
 // Four consecutive values of which `n` (or more: all) exist; `vec`: dst is 16-byte aligned when all four do.
 __device__ __forceinline__ void store_guarded(float* dst, float4 v, int n, bool vec) {
@@ -199,13 +211,14 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
           const Policy pol, const SplitInfo sp, const TileMap tmap, const int emit /*planes to emit: 0, 1 or 2*/,
           const Ranges rg, int* __restrict__ err_flag) {
   constexpr int kEmitBytes = emit_bytes<NPLANES, Policy>();
-  using L = SmemLayout<BN, NPLANES, kEmitBytes, PAIR, KW>;
+  using L = SmemLayout<BN, NPLANES, kEmitBytes, PAIR, KW, Policy::kSlab>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  uint8_t* emit_tile = smem + L::kStages * L::kStage;   // [four warps][planes][128 rows][128 B], 1024-byte aligned
+  uint8_t* emit_tile = smem + L::kRingBytes;   // [four warps][planes][128 rows][128 B], 1024-byte aligned
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(emit_tile + kEmitBytes);
-  uint64_t* empty_bar = full_bar + L::kStages;
-  uint64_t* acc_full = empty_bar + L::kStages;   // [2] accumulator ready for the epilogue
+  constexpr int kBars = Policy::kSlab ? L::kSlabsA + L::kSlicesB : L::kStages;   // (slabs of A, then slices of B)
+  uint64_t* empty_bar = full_bar + kBars;
+  uint64_t* acc_full = empty_bar + kBars;   // [2] accumulator ready for the epilogue
   uint64_t* acc_empty = acc_full + 2;            // [2] accumulator drained by the epilogue
   uint64_t* emit_bars = acc_empty + 2;           // [four warps][2] staging tile free / staging tile written
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(emit_bars + 4);
@@ -221,7 +234,7 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
     if (NPLANES == 2) { prefetch_tmap(&tm_a_lo); prefetch_tmap(&tm_b_lo); }
     if (emit >= 1) prefetch_tmap(&tm_out_hi);
     if (emit == 2) prefetch_tmap(&tm_out_lo);
-    for (int s = 0; s < L::kStages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
+    for (int s = 0; s < kBars; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
     for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], Policy::kEpiWarps * (PAIR ? 2 : 1)); for (int t = 0; t < 2; ++t) mbar_init(&emit_bars[2 * t + b], Policy::kTeamWarps * 32); }
     fence_barrier_init();
   }
@@ -238,7 +251,62 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
   NRS_PDL_WAIT();
   NRS_PDL_TRIGGER();   // the next kernel may be scheduled as this grid's SMs free up
 
+  if constexpr (Policy::kSlab) {
+    // ---------------- TMA producers: slabs of A (warp 0) and slices of B (the last warp) through rings of their own
+    if (warp == 0 || warp == 2 + Policy::kEpiWarps) {
+      const bool of_a = warp == 0;
+      const uint32_t bytes = (uint32_t)(PAIR ? 2 : 1) * NPLANES * (of_a ? pol.slab_rows() * (uint32_t)L::kRowBytes : (uint32_t)L::kBTile);
+      const int slots = of_a ? L::kSlabsA : L::kSlicesB, first_bar = of_a ? 0 : L::kSlabsA, per_slab = of_a ? 1 : pol.slab_taps();
+      uint32_t s = 0, ph = 0, issued = 0;
+      bool ok = true;
+      for (long base = 0; base < tmap.total && ok; base += t_step) {
+        const long t = tmap.at(base, t_first, t_step, false);
+        if (t < 0) break;
+        int tile_m, tile_n, z;
+        tmap.template decode<BN>(t, &tile_m, &tile_n, &z);
+        if (PAIR) tile_m = 2 * tile_m + rank;
+        const int batch = (int)sp.div_splits.div((uint32_t)z), split = z - batch * sp.splits;
+        const int kb_begin = split * sp.kb_per_split;
+        const int kb_end = sp.chunks > 1 ? sp.kb_total : min(sp.kb_total, kb_begin + sp.kb_per_split);
+        const int n0 = tile_n * BN + (PAIR ? rank * (BN / 2) : 0);
+        typename Policy::Cursor cur = pol.template cursor<KW>(tile_m, batch, kb_begin);
+        for (int kb = kb_begin; kb < kb_end && ok; ++kb) {
+          for (int i = 0; i < per_slab; ++i) {
+            if (!mbar_wait_warp(&empty_bar[first_bar + s], ph ^ 1u)) { ok = false; break; }
+            uint32_t bar;
+            if constexpr (PAIR) bar = cluster_addr(&full_bar[first_bar + s], 0); else bar = smem_u32(&full_bar[first_bar + s]);
+            if (elect_one()) {
+              if (rank == 0) mbar_expect_tx(&full_bar[first_bar + s], bytes);
+              if (of_a) {
+                uint8_t* dst = smem + s * L::kSlab;
+                pol.template load_a<PAIR, KW, L::kRowBytes>(dst, &tm_a_hi, bar, cur);
+                if (NPLANES == 2) pol.template load_a<PAIR, KW, L::kRowBytes>(dst + L::kSlabPlane, &tm_a_lo, bar, cur);
+              } else {
+                uint8_t* dst = smem + L::kSlabsA * L::kSlab + s * L::kBSlice;
+                const int col = pol.template slab_column<KW>(cur, i);
+                tma_load_3d_to<PAIR>(dst, &tm_b_hi, bar, col, n0, 0);
+                if (NPLANES == 2) tma_load_3d_to<PAIR>(dst + L::kBTile, &tm_b_lo, bar, col, n0, 0);
+              }
+            }
+            __syncwarp();
+            ++issued;
+            if (++s == (uint32_t)slots) { s = 0; ph ^= 1u; }
+          }
+          pol.template advance<KW>(cur);
+        }
+      }
+      if (!ok) {   // (as below)
+        if (lane == 0) atomicExch(err_flag, kErrProducerWait);
+        if (rank == 0) for (uint32_t j = (issued > (uint32_t)slots ? issued - slots : 0); j < issued; ++j)
+          if (!mbar_wait_warp(&full_bar[first_bar + j % slots], (j / slots) & 1u)) {
+            if (lane == 0) atomicExch(err_flag, kErrDrainWait);
+            break;
+          }
+      }
+    }
+  }
   if (warp == 0) {
+    if constexpr (!Policy::kSlab) {
     // ---------------- TMA producer
     // Both CTAs of a pair count their bytes on the barrier of rank 0, which expects the sum.
     const uint32_t slice_bytes = (uint32_t)(PAIR ? 2 : 1) * NPLANES * (pol.a_slice_rows() * (uint32_t)L::kRowBytes + (uint32_t)L::kBTile);
@@ -301,6 +369,7 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
         }
       }
     }
+    }
   } else if (warp == 1) {
     if (rank == 0) {
       // ---------------- UMMA issuer
@@ -315,6 +384,26 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
         if (NPLANES == 2) return mn ? make_smem_desc_sw64(addr + (uint32_t)k * 1024u, BK * 64, 512) : make_smem_desc_sw64(addr + (uint32_t)k * 32u, 16, 512);
         return mn ? make_smem_desc_sw128_32b(addr + (uint32_t)k * 1024u, BK * 128, 512) : make_smem_desc_sw128(addr + (uint32_t)k * 32u, 16, 1024);
       };
+      // The products of one K-slice.
+      auto multiply = [&](uint32_t d, uint32_t a_hi, uint32_t a_lo, uint32_t b_hi, bool first) {
+#pragma unroll
+        for (int k = 0; k < (NPLANES == 2 ? KW / 16 : BK / 8); ++k) {
+          const uint64_t da_hi = desc(kAMn, a_hi, k), db_hi = desc(kBMn, b_hi, k);
+          const uint32_t more = !(first && k == 0);
+          if constexpr (NPLANES == 1) {
+            umma_tf32<PAIR>(d, da_hi, db_hi, idesc_wide, more);
+          } else {
+            if constexpr (PAIR) {   // (each CTA holds its half of B_hi and of B_lo: no one product over both)
+              umma_f16<PAIR>(d, da_hi, db_hi, idesc_half, more);
+              umma_f16<PAIR>(d + BN, da_hi, desc(kBMn, b_hi + L::kBTile, k), idesc_half, more);
+            } else {
+              umma_f16<PAIR>(d, da_hi, db_hi, idesc_wide, more);   // hi*hi | hi*lo
+            }
+            umma_f16<PAIR>(d + BN, desc(kAMn, a_lo, k), db_hi, idesc_half, 1);   // + lo*hi
+          }
+        }
+      };
+      [[maybe_unused]] uint32_t sb = 0, phb = 0;   // slabs: the ring of B
       uint32_t s = 0, ph = 0, local = 0;
       bool ok = true;
       bool odd = false;
@@ -333,39 +422,43 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
           if (!(PAIR ? mbar_wait_warp_cluster(&acc_empty[buf], (use & 1u) ^ 1u) : mbar_wait_warp(&acc_empty[buf], (use & 1u) ^ 1u))) { ok = false; break; }
           tc_fence_after_sync();
           const uint32_t d = tmem_base + buf * (uint32_t)L::kAccCols;
-          for (int i = 0; i < nkb; i += L::kSlices) {
-            // (No tcgen05 fence here: the mbarrier's complete_tx orders the TMA writes before the
-            // UMMAs, and a fence would make the issuing thread wait out the UMMAs in flight.)
-            if (!mbar_wait_warp(&full_bar[s], ph)) { ok = false; break; }
-            const uint32_t slot = smem_u32(smem + s * L::kStage);
-            if (elect_one()) {
-#pragma unroll
-              for (int sl = 0; sl < L::kSlices; ++sl) {
-                if (sl > 0 && i + sl >= nkb) break;
-                const uint32_t a_hi = slot + sl * L::kSlice;
-                const uint32_t b_hi = a_hi + L::kATile;                 // B_lo follows B_hi directly
-                const uint32_t a_lo = b_hi + 2 * L::kBTile;
-#pragma unroll
-                for (int k = 0; k < (NPLANES == 2 ? KW / 16 : BK / 8); ++k) {
-                  const uint64_t da_hi = desc(kAMn, a_hi, k), db_hi = desc(kBMn, b_hi, k);
-                  const uint32_t more = (i | sl | k) != 0;
-                  if constexpr (NPLANES == 1) {
-                    umma_tf32<PAIR>(d, da_hi, db_hi, idesc_wide, more);
-                  } else {
-                    if constexpr (PAIR) {   // (each CTA holds its half of B_hi and of B_lo: no one product over both)
-                      umma_f16<PAIR>(d, da_hi, db_hi, idesc_half, more);
-                      umma_f16<PAIR>(d + BN, da_hi, desc(kBMn, b_hi + L::kBTile, k), idesc_half, more);
-                    } else {
-                      umma_f16<PAIR>(d, da_hi, db_hi, idesc_wide, more);   // hi*hi | hi*lo
-                    }
-                    umma_f16<PAIR>(d + BN, desc(kAMn, a_lo, k), db_hi, idesc_half, 1);   // + lo*hi
-                  }
+          // (No tcgen05 fence after a wait: the mbarrier's complete_tx orders the TMA writes before the
+          // UMMAs, and a fence would make the issuing thread wait out the UMMAs in flight.)
+          if constexpr (Policy::kSlab) {
+            for (int i = 0; i < nkb && ok; ++i) {
+              if (!mbar_wait_warp(&full_bar[s], ph)) { ok = false; break; }
+              const uint32_t slab = smem_u32(smem + s * L::kSlab);
+              for (int tap = 0; tap < pol.slab_taps(); ++tap) {
+                if (!mbar_wait_warp(&full_bar[L::kSlabsA + sb], phb)) { ok = false; break; }
+                const uint32_t b_hi = smem_u32(smem + L::kSlabsA * L::kSlab + sb * L::kBSlice);
+                const uint32_t a_hi = slab + pol.slab_tap_row(tap) * (uint32_t)L::kRowBytes;
+                if (elect_one()) {
+                  multiply(d, a_hi, a_hi + L::kSlabPlane, b_hi, (i | tap) == 0);
+                  umma_commit<PAIR>(&empty_bar[L::kSlabsA + sb]);
                 }
+                __syncwarp();
+                if (++sb == (uint32_t)L::kSlicesB) { sb = 0; phb ^= 1u; }
               }
-              umma_commit<PAIR>(&empty_bar[s]);  // slot reusable once these UMMAs have read it
+              if (ok && elect_one()) umma_commit<PAIR>(&empty_bar[s]);
+              __syncwarp();
+              if (++s == (uint32_t)L::kSlabsA) { s = 0; ph ^= 1u; }
             }
-            __syncwarp();
-            if (++s == (uint32_t)L::kStages) { s = 0; ph ^= 1u; }
+          } else {
+            for (int i = 0; i < nkb; i += L::kSlices) {
+              if (!mbar_wait_warp(&full_bar[s], ph)) { ok = false; break; }
+              const uint32_t slot = smem_u32(smem + s * L::kStage);
+              if (elect_one()) {
+#pragma unroll
+                for (int sl = 0; sl < L::kSlices; ++sl) {
+                  if (sl > 0 && i + sl >= nkb) break;
+                  const uint32_t a_hi = slot + sl * L::kSlice, b_hi = a_hi + L::kATile;   // B_lo follows B_hi directly
+                  multiply(d, a_hi, b_hi + 2 * L::kBTile, b_hi, (i | sl) == 0);
+                }
+                umma_commit<PAIR>(&empty_bar[s]);  // slot reusable once these UMMAs have read it
+              }
+              __syncwarp();
+              if (++s == (uint32_t)L::kStages) { s = 0; ph ^= 1u; }
+            }
           }
           if (ok && elect_one()) umma_commit<PAIR>(&acc_full[buf]);
           __syncwarp();
@@ -373,7 +466,7 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
       }
       if (!ok && lane == 0) atomicExch(err_flag, kErrMmaWait);
     }
-  } else {
+  } else if (!Policy::kSlab || warp < 2 + Policy::kEpiWarps) {
     // ---------------- epilogue: warp w owns TMEM lanes [32*(w%4), +32)
     const int q = warp & 3;
     const int row = q * 32 + lane;   // row inside the tile
@@ -542,8 +635,8 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
               mbar_arrive(&emit_bar[1]);
               if (emit_issuer) {
                 if (!mbar_wait(&emit_bar[1], ph)) { atomicExch(err_flag, kErrEpilogueWait); ok = false; break; }
-                tma_store_4d(&tm_out_hi, team_tile, n0 + c / (32 / kW) * 32, rw.x0, rw.y0, rw.n0);
-                if (NPLANES == 2) tma_store_4d(&tm_out_lo, team_tile + BM * 64, n0 + c / (32 / kW) * 32, rw.x0, rw.y0, rw.n0);
+                tma_store_4d(&tm_out_hi, team_tile, n0 + c / (32 / kW) * 32, rw.x0, Policy::kSlab ? rw.n0 : rw.y0, Policy::kSlab ? rw.y0 : rw.n0);
+                if (NPLANES == 2) tma_store_4d(&tm_out_lo, team_tile + BM * 64, n0 + c / (32 / kW) * 32, rw.x0, Policy::kSlab ? rw.n0 : rw.y0, Policy::kSlab ? rw.y0 : rw.n0);
                 bulk_commit();
               }
             }
@@ -602,7 +695,7 @@ inline void plan_split(const nrs_ctx* ctx, long tiles, long out_elems, int kb_to
     s = (int)(ctx->sm_count / tiles);
     // a split shorter than 16 K-blocks is all prologue and second pass, except where the output is so small (a Linear
     // layer at a batch of a few dozen) that the second pass is nothing: there down to 4
-    const int shortest = (out_elems <= (1 << 15) ? 4 : 16) * BK / kw;
+    const int shortest = std::max(1, (out_elems <= (1 << 15) ? 4 : 16) * BK / kw);
     if (s > kb_total / shortest) s = kb_total / shortest;
     if (s < 1) s = 1;
   }
@@ -677,16 +770,17 @@ inline int plan_units_per_cta(int sm_count, int ctas, long units, int min_units,
 template <int BN, int NPLANES, bool PAIR, int KW, class Policy>
 int launch(nrs_ctx* ctx, const CUtensorMap& ta_hi, const CUtensorMap& ta_lo, const CUtensorMap& tb_hi,
            const CUtensorMap& tb_lo, const Policy& pol, int tiles_m, int n_total, int batches, int kb_total,
-           const Ranges& rg, const CUtensorMap* out_hi = nullptr, const CUtensorMap* out_lo = nullptr, int* splits_out = nullptr) {
-  using L = SmemLayout<BN, NPLANES, emit_bytes<NPLANES, Policy>(), PAIR, KW>;
+           const Ranges& rg, const CUtensorMap* out_hi = nullptr, const CUtensorMap* out_lo = nullptr, int* splits_out = nullptr,
+           int k_per_block = KW /*values of K in one of the kb_total blocks*/) {
+  using L = SmemLayout<BN, NPLANES, emit_bytes<NPLANES, Policy>(), PAIR, KW, Policy::kSlab>;
   constexpr int kSmem = L::kBytes;
-  static_assert(kSmem <= 227 * 1024 && L::kStages >= 2, "shared memory budget");
+  static_assert(kSmem <= 227 * 1024 && L::kStages >= 2 && (!Policy::kSlab || L::kSlicesB >= 3), "shared memory budget");
   static NrsSmemAttr attr;
   NRS_ENSURE_SMEM(ctx, attr, (tc_kernel<BN, NPLANES, Policy, PAIR, KW>), kSmem);
   const int tiles_n = (n_total + BN - 1) / BN;
   SplitInfo sp{};
   if (Policy::kMaySplit) {
-    plan_split(ctx, (long)tiles_m * tiles_n * batches, (long)tiles_m * BM * n_total * batches, kb_total, KW, NPLANES == 2, &sp);
+    plan_split(ctx, (long)tiles_m * tiles_n * batches, (long)tiles_m * BM * n_total * batches, kb_total, k_per_block, NPLANES == 2, &sp);
   } else {   // tiles whose K ranges differ
     sp.splits = sp.chunks = 1;
     sp.kb_per_split = kb_total;
