@@ -91,6 +91,8 @@ struct HeadPolicy {
     }
   }
   __device__ __forceinline__ int row(int, int, int) const { return 0; }
+  template <int W>
+  __device__ __forceinline__ int fetch(int, int, bool) const { return 0; }
   template <bool SPLIT>
   __device__ __forceinline__ void store(int, int, int, int, float, float, uint32_t&) const {}   // no K-split
   template <bool SPLIT>

@@ -24,13 +24,28 @@ __device__ __forceinline__ float pow2(int e) { return __uint_as_float((uint32_t)
 __device__ __forceinline__ float scale_of(float bound) { return pow2(scale_exp(bound)); }
 // The factor that takes two operands' exponents out of their product, in two halves (by itself it may leave f32's range).
 struct Unscale {
-  float a, b;
+  float a, a_lo, b;
+  bool halves;   // nearly never: one factor does
   __device__ __forceinline__ Unscale(float bound_a, float bound_b) {
     const int e = -(scale_exp(bound_a) + scale_exp(bound_b));
-    a = pow2(e / 2);
-    b = pow2(e - e / 2);
+    halves = e < -115 || e > 127;
+    const int first = halves ? e / 2 : e;
+    a = pow2(first);
+    a_lo = a * kLoUnscale;
+    b = pow2(e - first);
   }
-  __device__ __forceinline__ float operator()(float hh, float cross) const { return fmaf(cross, kLoUnscale, hh) * a * b; }
+  __device__ __forceinline__ float operator()(float hh, float cross) const {
+    const float v = fmaf(cross, a_lo, hh * a);
+    return halves ? v * b : v;
+  }
+  template <int N>
+  __device__ __forceinline__ void apply(uint32_t (&hh)[N], const uint32_t (&cross)[N]) const {
+#pragma unroll
+    for (int j = 0; j < N; ++j) hh[j] = __float_as_uint(fmaf(__uint_as_float(cross[j]), a_lo, __uint_as_float(hh[j]) * a));
+    if (!halves) return;
+#pragma unroll
+    for (int j = 0; j < N; ++j) hh[j] = __float_as_uint(__uint_as_float(hh[j]) * b);
+  }
 };
 
 __device__ __forceinline__ void split(float v, float scale, __half* hi, __half* lo) {
@@ -75,7 +90,20 @@ __device__ __forceinline__ uint32_t seen(uint32_t top, float v) {
   const uint32_t u = __float_as_uint(v) & 0x7fffffffu;
   return u < 0x7f800000u && u > top ? u : top;
 }
-__device__ __forceinline__ uint32_t seen4(uint32_t top, float4 v) { return seen(seen(seen(seen(top, v.x), v.y), v.z), v.w); }
+template <int N>
+__device__ __forceinline__ uint32_t seen_all(uint32_t top, const float (&v)[N]) {   // infinities and NaNs looked for once
+  uint32_t m = 0;
+#pragma unroll
+  for (int j = 0; j < N; ++j) m = max(m, __float_as_uint(v[j]) & 0x7fffffffu);
+  if (m < 0x7f800000u) return max(top, m);
+#pragma unroll
+  for (int j = 0; j < N; ++j) top = seen(top, v[j]);
+  return top;
+}
+__device__ __forceinline__ uint32_t seen4(uint32_t top, float4 v) {
+  const float a[4] = {v.x, v.y, v.z, v.w};
+  return seen_all(top, a);
+}
 // A whole warp's, into the tensor's range.
 __device__ __forceinline__ void report(NrsRange* r, uint32_t top) {
   top = __reduce_max_sync(0xffffffffu, top);

@@ -62,6 +62,7 @@ struct ConvPolicyOf {
   float* out_lo;
   // optional: [tiles_m * 4][n_ch_out] sums of the finished values over each epilogue warp's 32 rows
   float* colsum_partial;
+  bool bias_vec;   // bias starts on 16 bytes
   bool skip_out;   // the finished values leave as planes and channel sums only (a K-split's second pass writes them still)
 
   __device__ __forceinline__ uint32_t a_slice_rows() const { return slice_rows; }
@@ -188,8 +189,24 @@ struct ConvPolicyOf {
   // One accumulator row, channels [nb, nb + W) as far as they exist: bias, activation, accumulate, mask,
   // NCHW store; the finished values come back in v (zeros for rows and channels outside the tensor) so the
   // caller can emit them as planes.  Loads are issued in batches ahead of the stores.
+  // The mask of W channels from nb on, of one pixel, a bit each.
   template <int W>
-  __device__ __forceinline__ void epilogue(const Row& rw, int nb, const uint32_t (&r)[W], float (&v)[W]) const {
+  __device__ __forceinline__ uint32_t fetch(const Row& rw, int nb, bool any) const {
+    uint32_t keep = ~0u;
+    if (mask_src && any && rw.live) {   // (whole channel blocks only)
+      const size_t plane = (size_t)out_h * out_w;
+      const float* m = mask_src + rw.off + (size_t)nb * plane;
+      float mv[W];
+#pragma unroll
+      for (int j = 0; j < W; ++j) mv[j] = __ldg(m + (size_t)j * plane);
+      keep = 0;
+#pragma unroll
+      for (int j = 0; j < W; ++j) keep |= mv[j] > 0.0f ? 1u << j : 0u;
+    }
+    return keep;
+  }
+  template <int W>
+  __device__ __forceinline__ void epilogue(const Row& rw, int nb, const uint32_t (&r)[W], uint32_t keep, float (&v)[W]) const {
     if (!rw.live) {
 #pragma unroll
       for (int j = 0; j < W; ++j) v[j] = 0.0f;
@@ -197,17 +214,23 @@ struct ConvPolicyOf {
     }
     // Whole channel blocks take their own instantiation: with per-channel conditions the loads of a block no longer
     // issue together (measured on the 64-channel data gradient with mask and planes: 69 -> 217 us).
-    if (n_ch_out - nb >= W) finish<true>(rw.off, nb, r, v);
-    else finish<false>(rw.off, nb, r, v);
+    if (n_ch_out - nb >= W) finish<true>(rw.off, nb, r, keep, v);
+    else finish<false>(rw.off, nb, r, keep, v);
   }
   template <bool FULL, int W>
-  __device__ __forceinline__ void finish(size_t off, int nb, const uint32_t (&r)[W], float (&v)[W]) const {
+  __device__ __forceinline__ void finish(size_t off, int nb, const uint32_t (&r)[W], uint32_t keep, float (&v)[W]) const {
     const size_t plane = (size_t)out_h * out_w;
     float* dst = out + off + (size_t)nb * plane;
     const int nch = FULL ? W : n_ch_out - nb;   // channels of this block that exist
 #pragma unroll
     for (int j = 0; j < W; ++j) v[j] = (FULL || j < nch) ? __uint_as_float(r[j]) : 0.0f;
-    if (bias) {
+    if (bias && FULL && bias_vec) {
+#pragma unroll
+      for (int j = 0; j < W; j += 4) {
+        const float4 b = __ldg(reinterpret_cast<const float4*>(bias + nb + j));
+        v[j] += b.x; v[j + 1] += b.y; v[j + 2] += b.z; v[j + 3] += b.w;
+      }
+    } else if (bias) {
 #pragma unroll
       for (int j = 0; j < W; ++j)
         if (FULL || j < nch) v[j] += __ldg(bias + nb + j);
@@ -223,13 +246,9 @@ struct ConvPolicyOf {
 #pragma unroll
       for (int j = 0; j < W; ++j) v[j] += o[j];
     }
-    if (FULL && mask_src) {   // a mask is taken for whole channel blocks only
-      const float* m = mask_src + off + (size_t)nb * plane;
-      float mv[W];
+    if (FULL && mask_src) {
 #pragma unroll
-      for (int j = 0; j < W; ++j) mv[j] = __ldg(m + (size_t)j * plane);
-#pragma unroll
-      for (int j = 0; j < W; ++j) v[j] = mv[j] > 0.0f ? v[j] : 0.0f;
+      for (int j = 0; j < W; ++j) v[j] = (keep >> j) & 1u ? v[j] : 0.0f;
     }
     if (FULL && skip_out) return;
 #pragma unroll
@@ -386,6 +405,7 @@ int conv_common(nrs_ctx* ctx, ConvPlan& p) {
   pol.div_cblocks = NrsFastDiv(pol.cblocks);
   pol.div_tiles_x = NrsFastDiv(pol.tiles_x); pol.div_tiles_y = NrsFastDiv(pol.tiles_y);
   pol.slice_rows = (uint32_t)(pol.Wt * pol.Ht * pol.Nt);
+  pol.bias_vec = (reinterpret_cast<uintptr_t>(p.bias) & 15) == 0;
   pol.k_total = (float)p.a_ch * p.ay.taps * p.ax.taps;
   // Requests of the caller are honoured where this launch writes every pixel of the output (planes: whole
   // 32-channel blocks); the caller finds the others still registered and does the work itself.
@@ -447,7 +467,7 @@ int conv_common(nrs_ctx* ctx, ConvPlan& p) {
 
   if (extras != ctx->out_extras.end()) ctx->out_extras.erase(extras);   // honoured from here on
   int splits = 0;
-  const tc::TilePlan tile = tc::plan_tile(ctx, tiles_m, p.n_ch_out, 1, p.ay.taps * p.ax.taps * blocks32, split, 0.025, true);
+  const tc::TilePlan tile = tc::plan_tile(ctx, tiles_m, p.n_ch_out, 1, p.ay.taps * p.ax.taps * blocks32, split, 0.025, true, slab);
 #define NRS_RUN_AS(BN_, PAIR_, SLAB_)                                                                                          \
   st = !split ? run_conv<BN_, 1, PAIR_, 32, SLAB_>(ctx, p, (const float*)a_hi, nullptr, pol, rg, (int)tiles_m, &splits)          \
        : wide ? run_conv<BN_, 2, PAIR_, 64, SLAB_>(ctx, p, (const float*)a_hi, (const float*)a_lo, pol, rg, (int)tiles_m, &splits) \

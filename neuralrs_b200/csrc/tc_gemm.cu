@@ -93,6 +93,8 @@ struct GemmPolicy {
     }
   }
   __device__ __forceinline__ int row(int, int, int) const { return 0; }
+  template <int W>
+  __device__ __forceinline__ int fetch(int, int, bool) const { return 0; }
   // Four row segments of a warp's 32 x 16 block: row r0 + 8*i of the tile, columns n..n+3 (see tc::rows_to_lines).  Blocks
   // that lie inside C on 16-byte boundaries, nearly all of them, take an instantiation without the checks.
   template <bool SPLIT>
@@ -263,7 +265,7 @@ int run(nrs_ctx* ctx, const Operand& A, const Operand& B, int batch, int b_rows,
 
 // `limit`: widest tile allowed (segmented B: the segment must be whole tiles).
 tc::TilePlan tile_of(const nrs_ctx* ctx, int m, int n, int batch, int k, bool split, int limit = 128) {
-  return tc::plan_tile(ctx, (m + tc::BM - 1) / tc::BM, n, batch, (k + tc::BK - 1) / tc::BK, split, 0.004, false, limit);
+  return tc::plan_tile(ctx, (m + tc::BM - 1) / tc::BM, n, batch, (k + tc::BK - 1) / tc::BK, split, 0.004, false, false, limit);
 }
 
 template <bool MN>

@@ -83,8 +83,11 @@ struct SmemLayout {
   static constexpr int kRing = 227 * 1024 - kExtra;
   static constexpr int kStages = kRing / kStage >= 8 ? 8 : kRing / kStage;
   // Slabs (Policy::kSlab): a ring of A slabs and a ring of B slices.
-  static constexpr int kSlabPlane = kSlabRows * kRowBytes, kSlab = NPLANES * kSlabPlane, kBSlice = NPLANES * kBTile;
-  static constexpr int kMostA = kSlab > 24 * 1024 ? 3 : 4;
+  static constexpr int kSlabPlane = kSlabRows * kRowBytes, kSlab = NPLANES * kSlabPlane;
+  // A pair's f16 pairs: a third block in a slice of B, B_hi again (see kTwice in tc_kernel).
+  static constexpr bool kTwice = SLAB && PAIR && NPLANES == 2 && BN >= 64;
+  static constexpr int kBSlice = (kTwice ? 3 : NPLANES) * kBTile;
+  static constexpr int kMostA = kSlab > 24 * 1024 ? (BN == 128 ? 2 : 3) : 4;   // (128 columns: more slices of B instead)
   static constexpr int kSlabsA = kRing - kMostA * kSlab >= 3 * kBSlice ? kMostA : 2;
   static constexpr int kSlicesB = (kRing - kSlabsA * kSlab) / kBSlice >= 8 ? 8 : (kRing - kSlabsA * kSlab) / kBSlice;
   static constexpr int kRingBytes = SLAB ? kSlabsA * kSlab + kSlicesB * kBSlice : kStages * kStage;
@@ -255,7 +258,7 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
     // ---------------- TMA producers: slabs of A (warp 0) and slices of B (the last warp) through rings of their own
     if (warp == 0 || warp == 2 + Policy::kEpiWarps) {
       const bool of_a = warp == 0;
-      const uint32_t bytes = (uint32_t)(PAIR ? 2 : 1) * NPLANES * (of_a ? pol.slab_rows() * (uint32_t)L::kRowBytes : (uint32_t)L::kBTile);
+      const uint32_t bytes = (uint32_t)(PAIR ? 2 : 1) * (of_a ? NPLANES * pol.slab_rows() * (uint32_t)L::kRowBytes : (uint32_t)L::kBSlice);
       const int slots = of_a ? L::kSlabsA : L::kSlicesB, first_bar = of_a ? 0 : L::kSlabsA, per_slab = of_a ? 1 : pol.slab_taps();
       uint32_t s = 0, ph = 0, issued = 0;
       bool ok = true;
@@ -284,8 +287,14 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
               } else {
                 uint8_t* dst = smem + L::kSlabsA * L::kSlab + s * L::kBSlice;
                 const int col = pol.template slab_column<KW>(cur, i);
-                tma_load_3d_to<PAIR>(dst, &tm_b_hi, bar, col, n0, 0);
-                if (NPLANES == 2) tma_load_3d_to<PAIR>(dst + L::kBTile, &tm_b_lo, bar, col, n0, 0);
+                if constexpr (L::kTwice) {   // rank 0: hi lo hi, rank 1: lo hi hi
+                  tma_load_3d_to<PAIR>(dst + rank * L::kBTile, &tm_b_hi, bar, col, n0, 0);
+                  tma_load_3d_to<PAIR>(dst + (1 - rank) * L::kBTile, &tm_b_lo, bar, col, n0, 0);
+                  tma_load_3d_to<PAIR>(dst + 2 * L::kBTile, &tm_b_hi, bar, col, n0, 0);
+                } else {
+                  tma_load_3d_to<PAIR>(dst, &tm_b_hi, bar, col, n0, 0);
+                  if (NPLANES == 2) tma_load_3d_to<PAIR>(dst + L::kBTile, &tm_b_lo, bar, col, n0, 0);
+                }
               }
             }
             __syncwarp();
@@ -393,6 +402,15 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
           if constexpr (NPLANES == 1) {
             umma_tf32<PAIR>(d, da_hi, db_hi, idesc_wide, more);
           } else {
+            if constexpr (L::kTwice) {
+              // A_hi read once instead of twice: shared memory is what bounds these tiles (and a UMMA of 64 columns takes
+              // 46 clocks instead of 32).  With B laid out [hi0 lo0 hi0] in one CTA and [lo1 hi1 hi1] in the other (halves 0
+              // and 1 of the columns), the wide product's columns are hh0 hl0 hl1 hh1, and the narrow one (lh0 lh1, of the
+              // third blocks) lands on hl0 hl1.  1014 -> 909 clocks per slice of a 64 -> 128 layer, 895 -> 830 of 128 -> 128.
+              umma_f16<PAIR>(d, da_hi, db_hi, idesc_wide, more);
+              umma_f16<PAIR>(d + BN / 2, desc(kAMn, a_lo, k), desc(kBMn, b_hi + 2 * L::kBTile, k), idesc_half, 1);
+              continue;
+            }
             if constexpr (PAIR) {   // (each CTA holds its half of B_hi and of B_lo: no one product over both)
               umma_f16<PAIR>(d, da_hi, db_hi, idesc_half, more);
               umma_f16<PAIR>(d + BN, da_hi, desc(kBMn, b_hi + L::kBTile, k), idesc_half, more);
@@ -476,12 +494,10 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
     const bool emit_issuer = (warp - 2) % Policy::kTeamWarps == 0 && lane == 0;
     uint64_t* emit_bar = emit_bars + (Policy::kCanEmit ? 2 * team : 0);
     uint8_t* team_tile = emit_tile + (Policy::kCanEmit ? team * BM * 128 : 0);
-    [[maybe_unused]] float us_a = 1.0f, us_b = 1.0f, out_scale = 1.0f;
+    [[maybe_unused]] float out_scale = 1.0f;
     [[maybe_unused]] uint32_t top = 0;
+    [[maybe_unused]] const pr::Unscale unscale(NPLANES == 2 ? rg.a->bound : 1.0f, NPLANES == 2 ? rg.b->bound : 1.0f);
     if constexpr (NPLANES == 2) {
-      const pr::Unscale us(rg.a->bound, rg.b->bound);
-      us_a = us.a;
-      us_b = us.b;
       if (rg.out) {
         const float bound = pol.out_bound(rg.a->top, rg.b->top, lane);
         out_scale = pr::scale_of(bound);
@@ -502,6 +518,10 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
       if (!pol.clip(tile_m, tile_n, BN, &kb_begin, &kb_end)) continue;   // the same verdict in all three roles
       const int n0 = tile_n * BN;
       [[maybe_unused]] const auto rw = pol.row(tile_m, batch, row);   // index arithmetic under the main loop
+      constexpr int kW = Policy::kCanEmit && Policy::kTeamWarps == 4 ? 32 : 16, kBlocks = BN / kW, kStep = Policy::kEpiWarps / 4;
+      const int c_first = kStep == 1 ? 0 : (warp - 2) >> 2;   // (a team of eight: 2 * team + half)
+      // What the first block reads besides the accumulator is under way before that is full.
+      [[maybe_unused]] auto extra = pol.template fetch<kW>(rw, n0 + c_first * kW, c_first < kBlocks);
       for (int k0 = kb_begin; k0 < kb_end && ok; k0 += sp.kb_per_split) {
         const uint32_t buf = local & 1u, use = local >> 1;
         ++local;
@@ -518,8 +538,6 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
         };
         // The warps of a lane quarter share its column blocks out; those without one just hand the accumulator back, and so
         // do all of a pair's second CTA beyond the last row tile.
-        constexpr int kW = Policy::kCanEmit && Policy::kTeamWarps == 4 ? 32 : 16, kBlocks = BN / kW, kStep = Policy::kEpiWarps / 4;
-        const int c_first = kStep == 1 ? 0 : (warp - 2) >> 2;   // (a team of eight: 2 * team + half)
         if (c_first >= kBlocks || (PAIR && tile_m * BM >= sp.rows_total)) {
           hand_back();
           continue;
@@ -528,13 +546,13 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
 #pragma unroll 1
         for (int c = c_first; c < kBlocks; c += kStep) {
           uint32_t r[kW];
-          tmem_ld_32(acc + (uint32_t)(c * kW), r);
+          const int main_col = L::kTwice && c * kW >= BN / 2 ? BN + c * kW : c * kW;   // (kTwice: hh0 hl0 hl1 hh1)
+          tmem_ld_32(acc + (uint32_t)main_col, r);
           if (NPLANES == 2) {
             uint32_t r2[kW];
-            tmem_ld_32(acc + (uint32_t)(BN + c * kW), r2);
+            tmem_ld_32(acc + (uint32_t)((L::kTwice ? BN / 2 : BN) + c * kW), r2);
             tmem_ld_wait();
-#pragma unroll
-            for (int j = 0; j < kW; ++j) r[j] = __float_as_uint(fmaf(__uint_as_float(r2[j]), pr::kLoUnscale, __uint_as_float(r[j])) * us_a * us_b);
+            unscale.apply(r, r2);
           } else {
             tmem_ld_wait();
           }
@@ -580,11 +598,9 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
             }
           } else {
             float v[kW];
-            pol.epilogue(rw, n0 + c * kW, r, v);
-            if (NPLANES == 2 && rg.out) {
-#pragma unroll
-              for (int j = 0; j < kW; ++j) top = pr::seen(top, v[j]);
-            }
+            if (c != c_first || k0 + sp.kb_per_split < kb_end) extra = pol.template fetch<kW>(rw, n0 + c * kW, true);
+            pol.epilogue(rw, n0 + c * kW, r, extra, v);
+            if (NPLANES == 2 && rg.out) top = pr::seen_all(top, v);
             if (float* cs = pol.colsum_row(tile_m, q)) {
               // Sum over this warp's 32 rows, one channel per lane: a transpose-reduce (each stage halves the values a lane
               // holds; fixed order, deterministic): 31 shuffles for 32 channels, 16 for 16.
@@ -711,21 +727,22 @@ inline void plan_split(const nrs_ctx* ctx, long tiles, long out_elems, int kb_to
   sp->chunks = in_chunks ? s : 1;
 }
 
-// The tile of a launch: its columns, and whether CTAs work in pairs.  kPlans holds the measured clocks per K-slice (3xTF32,
-// TF32), and per tile about what the accumulator's way out adds where nothing hides it.  The tile with the least (rounds
-// of the grid) x (clocks per tile) is taken, a K-split's second pass counted in: wide tiles for large outputs, narrower
-// ones where they fill SMs that would idle or where a ragged column count would pad, pairs where there are enough row
-// tiles.  `reduce_clk`: what the second pass over a K-split costs per output value, on top of its launch (measured: 3.6 us
-// for 51 thousand values of a GEMM, 13.4 us for 819 thousand of a convolution, whose pixels lie strided).  A
-// convolution's 64-column pair is slower than the single tile in TF32 (30.1 us against 27.4 for 64 channels on 100 images
+// The tile of a launch: its columns, and whether CTAs work in pairs.  kPlans holds clocks per 32 values of K (3xTF32; 3xTF32
+// in slabs; TF32), and per tile what the accumulator's way out takes (3xTF32: of each round it is hidden behind the next;
+// TF32: adds to each).  The tile with the least time is taken, a K-split's second pass counted in: wide tiles for large
+// outputs, narrower ones where they fill SMs that would idle or where a ragged column count would pad, pairs where there
+// are enough row tiles.  `reduce_clk`: what the second pass over a K-split costs per output value, on top of its launch
+// (measured: 3.6 us for 51 thousand values of a GEMM, 13.4 us for 819 thousand of a convolution, whose pixels lie strided).
+// A convolution's 64-column pair is slower than the single tile in TF32 (30.1 us against 27.4 for 64 channels on 100 images
 // of 32 x 32).  `limit`: widest tile allowed.
 struct TilePlan { int bn; bool pair; };
-inline TilePlan plan_tile(const nrs_ctx* ctx, long tiles_m, int n, long batches, int kblocks, bool split_planes, double reduce_clk, bool conv, int limit = 128) {
-  static const struct { int bn; bool pair; int kb_clk[2], tile_clk; } kPlans[] = {{128, true, {820, 345}, 2600},
-                                                                                  {64, true, {565, 317}, 1700},
-                                                                                  {128, false, {905, 428}, 2600},
-                                                                                  {64, false, {660, 369}, 1700},
-                                                                                  {32, false, {570, 352}, 1300}};
+inline TilePlan plan_tile(const nrs_ctx* ctx, long tiles_m, int n, long batches, int kblocks, bool split_planes, double reduce_clk, bool conv, bool slab,
+                          int limit = 128) {
+  static const struct { int bn; bool pair; int kb_clk[3], tile_clk[2]; } kPlans[] = {{128, true, {395, 395, 345}, {5500, 2600}},
+                                                                                     {64, true, {315, 235, 317}, {3500, 1700}},
+                                                                                     {128, false, {530, 420, 428}, {5500, 2600}},
+                                                                                     {64, false, {400, 280, 369}, {3500, 1700}},
+                                                                                     {32, false, {330, 210, 352}, {2600, 1300}}};
   TilePlan best{32, false};
   double best_t = -1.0;
   for (const auto& c : kPlans) {
@@ -735,8 +752,13 @@ inline TilePlan plan_tile(const nrs_ctx* ctx, long tiles_m, int n, long batches,
     plan_split(ctx, tiles_m * tiles_n * batches, tiles_m * BM * n * batches, kblocks, BK, split_planes, &sp);
     const int splits = sp.splits, per = sp.kb_per_split * sp.chunks;
     const long units = (c.pair ? (tiles_m + 1) / 2 : tiles_m) * tiles_n * batches * splits, slots = ctx->sm_count / (c.pair ? 2 : 1);
-    const int kb_clk = c.pair && c.bn == 64 && conv && !split_planes ? 400 : c.kb_clk[split_planes ? 0 : 1];
-    double t = (double)((units + slots - 1) / slots) * ((double)per * kb_clk + c.tile_clk);
+    const double rounds = (double)((units + slots - 1) / slots);
+    double t;
+    if (split_planes) {
+      t = rounds * std::max((double)per * c.kb_clk[slab ? 1 : 0], (double)c.tile_clk[0]) + c.tile_clk[0];
+    } else {
+      t = rounds * ((double)per * (c.pair && c.bn == 64 && conv ? 400 : c.kb_clk[2]) + c.tile_clk[1]);
+    }
     if (splits > 1) t += 4000.0 + reduce_clk * (double)tiles_m * BM * n * batches;
     if (best_t < 0.0 || t < best_t) { best_t = t; best = TilePlan{c.bn, c.pair}; }
   }
