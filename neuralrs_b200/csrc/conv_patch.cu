@@ -10,6 +10,7 @@
 //
 // Reference counterparts: conv2d_im2col + matmul_nn + col2out and im2col + matmul_nt_splitk
 // (src/cuda/nn/conv.rs:244-320).
+#include "fold.h"
 #include "igemm_problems.cuh"
 #include "nrs_internal.h"
 #include "pair.cuh"
@@ -95,8 +96,8 @@ struct Patches {
   }
   ~Patches() {
     if (!owned) return;
-    nrs_free(ctx, hi);
-    if (lo) nrs_free(ctx, lo);
+    nrs_free_after_wgrads(ctx, hi);
+    if (lo) nrs_free_after_wgrads(ctx, lo);
   }
 };
 

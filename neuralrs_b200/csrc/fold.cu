@@ -6,6 +6,7 @@
 // travels as a kernel parameter.  Every sum has a fixed order, whatever the batch.  Measured on the CIFAR CNN at batch
 // 100: 15 launches, 104 us, become one of 38 us; on the language model (32 x 128 tokens) 21 launches, 125 us, one of 40.
 #include "fold.h"
+#include "wgrad_queue.h"
 
 #include <algorithm>
 
@@ -255,13 +256,35 @@ float* place(NrsFolds& f, size_t bytes) {
 
 void nrs_folds_begin(nrs_ctx* ctx) { ctx->folds.active = true; }
 
-int nrs_folds_flush(nrs_ctx* ctx) { return run_queue(ctx); }
+int nrs_folds_flush(nrs_ctx* ctx) {
+  NrsFolds& f = ctx->folds;
+  int st = NRS_OK;
+  if (!f.waiting.empty()) {
+    f.waiting.clear();
+    st = nrs_wgrad_rows_run(ctx);
+    if (st == NRS_OK) st = nrs_wgrad_tiles_run(ctx);
+  }
+  if (st == NRS_OK) st = run_queue(ctx);
+  for (void* p : f.kept) nrs_free(ctx, p);
+  f.kept.clear();
+  return st;
+}
+
+void nrs_free_after_wgrads(nrs_ctx* ctx, void* p) {
+  if (ctx->folds.waiting.empty()) nrs_free(ctx, p);
+  else if (p) ctx->folds.kept.push_back(p);
+}
 
 void nrs_folds_end(nrs_ctx* ctx) {
   ctx->folds.active = ctx->folds.open = false;
   ctx->folds.jobs.clear();
   ctx->folds.tickets_used = 1;
   ctx->folds.holding = 0;
+  ctx->folds.waiting.clear();
+  ctx->folds.waiting_rows.reset();
+  ctx->folds.waiting_tiles.reset();
+  for (void* p : ctx->folds.kept) nrs_free(ctx, p);
+  ctx->folds.kept.clear();
 }
 
 void nrs_folds_free(nrs_ctx* ctx) {
@@ -282,6 +305,8 @@ static bool writes(const NrsFoldJob& j, const float* p, size_t len) {
 }
 
 int nrs_folds_settle(nrs_ctx* ctx, const float* dst, size_t len) {
+  for (const auto& w : ctx->folds.waiting)
+    if (w.first < dst + len && dst < w.first + w.second) return nrs_folds_flush(ctx);
   for (const NrsFoldJob& j : ctx->folds.jobs)
     if (writes(j, dst, len)) return nrs_folds_flush(ctx);
   return NRS_OK;

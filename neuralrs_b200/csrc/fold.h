@@ -5,7 +5,9 @@
 
 // While on, submitted folds wait for nrs_folds_flush (a backward pass's end) or nrs_folds_settle.
 void nrs_folds_begin(nrs_ctx* ctx);
-int nrs_folds_flush(nrs_ctx* ctx);
+int nrs_folds_flush(nrs_ctx* ctx);   // (and the weight gradients that wait, before them)
+// nrs_free, or, while weight gradients wait that may read it, once they have run.
+void nrs_free_after_wgrads(nrs_ctx* ctx, void* p);
 void nrs_folds_end(nrs_ctx* ctx);    // leaves the collecting mode; what is still queued is dropped (a failed pass)
 void nrs_folds_free(nrs_ctx* ctx);
 // Runs what is queued if it writes any of the `len` floats at `dst`: called by whoever is about to read, overwrite or

@@ -230,8 +230,8 @@ struct GradPlanes {
   ~GradPlanes() {
     if (!key) return;
     ctx->plane_hints.erase(key);
-    nrs_free(ctx, hi);
-    if (lo) nrs_free(ctx, lo);
+    nrs_free_after_wgrads(ctx, hi);
+    if (lo) nrs_free_after_wgrads(ctx, lo);
   }
 };
 
@@ -860,8 +860,8 @@ NodeP conv2d_act(const NodeP& x, const NodeP& w, const NodeP& b, size_t stride, 
     }
     auto cleanup = [&] {
       if (staged) ctx->plane_hints.erase(dy);
-      if (dhi) nrs_free(ctx, dhi);
-      if (dlo) nrs_free(ctx, dlo);
+      if (dhi) nrs_free_after_wgrads(ctx, dhi);
+      if (dlo) nrs_free_after_wgrads(ctx, dlo);
       if (masked) nrs_free(ctx, masked);
     };
     try {

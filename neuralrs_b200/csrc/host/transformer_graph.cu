@@ -291,7 +291,7 @@ static NodeP planes_attention(const MultiHeadAttention& m, const NodeP& x, size_
       nrs_ctx* c; std::vector<float*> p; const float* key;
       ~Release() {
         if (key) c->plane_hints.erase(key);
-        for (float* q : p) if (q) nrs_free(c, q);
+        for (float* q : p) if (q) nrs_free_after_wgrads(c, q);
       }
     } release{ctx, {ghi, glo, a.scores, a.ds_hi, a.ds_lo, a.dqkv_hi, a.dqkv_lo}, nullptr};
     check(ctx, nrs_mha_planes_bwd(ctx, a));

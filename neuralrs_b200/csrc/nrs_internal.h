@@ -8,6 +8,7 @@
 #include <cstdio>
 #include <iterator>
 #include <map>
+#include <memory>
 #include <string>
 #include <unordered_map>
 #include <utility>
@@ -202,6 +203,11 @@ struct NrsFolds {
   bool open = false;       // some of it has been handed out for a job that is not submitted yet
   int holding = 0;         // queued jobs with partial sums in it (others read memory of their own)
   uint64_t launched_at = ~0ull;   // nrs_ctx::launches right after the last launch of folds
+  // Weight gradients that wait for the pass's end (wgrad_queue.h): where they write, their kernels' own queues, and memory
+  // they read whose owner has let go of it.
+  std::vector<std::pair<const float*, size_t>> waiting;
+  std::shared_ptr<void> waiting_rows, waiting_tiles;
+  std::vector<void*> kept;
 };
 
 struct nrs_ctx {

@@ -66,6 +66,7 @@ namespace tc {
 
 constexpr int BM = 128, BK = 32;   // 32 values: 128 bytes of f32, 64 of f16: one swizzle row
 constexpr int kMaxChainK = 4096;   // longest single accumulation chain in 3xTF32 mode
+constexpr int kMaxChainPairs = 8192;   // the same of weight gradients: at this length f16 pairs err as much as TF32 pairs did at half
 constexpr int kGroupM = 16;        // row tiles per raster group (see TileMap)
 constexpr int kSlabRows = 192;     // most pixels of a slab of A (see Policy::kSlab)
 

@@ -29,6 +29,7 @@
 // 298-320).
 #include "fold.h"
 #include "tc_mainloop.cuh"
+#include "wgrad_queue.h"
 
 namespace {
 
@@ -50,17 +51,36 @@ struct WgradParams {
   float* partial;                 // [split][m_block][group][col_block][128][group_cols]
   int group_cols;                 // taps_per_group * cblocks * wb; in column blocks: the width of one (64, 128 or 256)
   int col_blocks;                 // column blocks of the input channels, each its own CTA (more than 256 channels, or 1x1)
-  int independent;                // reads nothing the kernel launched just before it wrote (NRS_PDL_PROLOGUE)
+  int stages;
+  int ctas;                       // per split
+  unsigned first_block;           // of this gradient's in the launch
   const NrsRange *range_dy, *range_x;   // 3xTF32
   float* direct;                  // 1x1, one split, no accumulation: the tile is the result; written straight to dw[co][ci]
 };
 
-template <int NPLANES, int STAGES>
+// The gradients of one launch.
+struct WgradEntry {
+  CUtensorMap dy_hi, dy_lo, x_hi, x_lo;
+  WgradParams p;
+};
+template <int CAP>
+struct WgradBatch {
+  WgradEntry e[CAP];
+  int n;
+  int independent;                // reads nothing the kernel launched just before it wrote (NRS_PDL_PROLOGUE)
+};
+constexpr int kWgBatch = 16;
+
+template <int NPLANES, int CAP>
 __global__ void __launch_bounds__(kWgThreads, 1)
-tc_wgrad_kernel(const __grid_constant__ CUtensorMap tm_dy_hi, const __grid_constant__ CUtensorMap tm_dy_lo,
-                const __grid_constant__ CUtensorMap tm_x_hi, const __grid_constant__ CUtensorMap tm_x_lo,
-                const WgradParams p, const int n_cols /*UMMA N, multiple of 16*/, int* __restrict__ err_flag) {
+tc_wgrad_kernel(const __grid_constant__ WgradBatch<CAP> batch, int* __restrict__ err_flag) {
   extern __shared__ uint8_t smem_raw[];
+  int entry = 0;
+  while (CAP > 1 && entry + 1 < batch.n && batch.e[entry + 1].p.first_block <= blockIdx.x) ++entry;
+  const WgradEntry& en = batch.e[entry];
+  const WgradParams& p = en.p;
+  const CUtensorMap &tm_dy_hi = en.dy_hi, &tm_dy_lo = en.dy_lo, &tm_x_hi = en.x_hi, &tm_x_lo = en.x_lo;
+  const int STAGES = p.stages, n_cols = p.group_cols /*UMMA N, multiple of 16*/;
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const uint32_t value = NPLANES == 2 ? 2u : 4u;
   const uint32_t a_blk = (uint32_t)(p.kp * p.wa) * value, b_blk = (uint32_t)(p.kp * p.wb) * value;   // one block of one plane
@@ -73,10 +93,10 @@ tc_wgrad_kernel(const __grid_constant__ CUtensorMap tm_dy_hi, const __grid_const
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accum_bar + 1);
 
   const int warp = (int)tc::uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
-  const int cbk = blockIdx.x % p.col_blocks;
-  const int mg = blockIdx.x / p.col_blocks;
+  const int local = (int)(blockIdx.x - p.first_block), split = local / p.ctas, cta = local - split * p.ctas;
+  const int cbk = cta % p.col_blocks;
+  const int mg = cta / p.col_blocks;
   const int mb = mg / p.n_groups, grp = mg - mb * p.n_groups;
-  const int split = blockIdx.y;
   // blocks of x this CTA's columns cover (a column block of a wide layer may be ragged)
   const int most = p.group_cols / p.wb, cblocks = p.col_blocks > 1 ? min(most, p.cblocks - cbk * most) : p.cblocks;
   const int t_begin = split * p.tiles_per_split;
@@ -101,7 +121,7 @@ tc_wgrad_kernel(const __grid_constant__ CUtensorMap tm_dy_hi, const __grid_const
   __syncthreads();
   tc::tc_fence_after_sync();
   const uint32_t tmem_base = tc::uniform(*tmem_slot);
-  if (!p.independent) NRS_PDL_WAIT();   // set-up above may overlap the previous kernel's tail; its results are needed from here
+  if (!batch.independent) NRS_PDL_WAIT();   // set-up above may overlap the previous kernel's tail; its results are needed from here
   NRS_PDL_TRIGGER();
 
   // (Both issuing roles run as whole warps and elect a lane for the instructions themselves: tc::elect_one.)
@@ -250,7 +270,7 @@ tc_wgrad_kernel(const __grid_constant__ CUtensorMap tm_dy_hi, const __grid_const
     }
   }
 
-  if (p.independent) NRS_PDL_WAIT();   // nothing after this kernel may run ahead of its predecessor
+  if (batch.independent) NRS_PDL_WAIT();   // nothing after this kernel may run ahead of its predecessor
   __syncwarp();
   tc::tc_fence_before_sync();
   __syncthreads();
@@ -295,18 +315,66 @@ void plan_pixel_box(WgradParams* p, int n, int oh, int ow, int planes, size_t by
 
 namespace {
 
-template <int NPLANES, int STAGES>
-int launch_wgrad(nrs_ctx* ctx, const CUtensorMap* maps, const WgradParams& p, int splits, size_t smem_bytes) {
+// A weight gradient that may wait.
+struct WgradJob {
+  WgradEntry e;
+  int planes;
+  float* dw;
+  int accumulate, out_cols;
+  bool can_be_direct;
+};
+size_t pixel_bytes_of(const WgradParams& p) { return (size_t)(128 + p.group_cols) * 4; }   // both operands, all planes
+size_t split_floats(const WgradParams& p) { return (size_t)p.ctas * 128 * p.group_cols; }
+long max_tiles(const WgradParams& p, int planes) { return planes == 2 ? std::max(1, tc::kMaxChainPairs / p.kp) : 1 << 30; }
+
+template <int NPLANES, int CAP>
+int launch_wgrad(nrs_ctx* ctx, WgradJob* jobs, int n, bool independent) {
   static NrsSmemAttr attr;
-  NRS_ENSURE_SMEM(ctx, attr, (tc_wgrad_kernel<NPLANES, STAGES>), smem_bytes);
+  WgradBatch<CAP> b{};
+  size_t smem = 0;
+  unsigned blocks = 0;
+  b.n = n;
+  b.independent = independent ? 1 : 0;
+  for (int i = 0; i < n; ++i) {
+    WgradParams& p = jobs[i].e.p;
+    const int splits = (p.n_tiles + p.tiles_per_split - 1) / p.tiles_per_split;
+    // a single split of a 1x1 "convolution" (A^T B) that overwrites its output needs no second pass
+    p.direct = splits == 1 && jobs[i].can_be_direct ? jobs[i].dw : nullptr;
+    const int st = p.direct ? NRS_OK : nrs_fold_partial(ctx, NRS_WS_WGRAD_PARTIAL, splits * split_floats(p) * sizeof(float), &p.partial);
+    if (st != NRS_OK) return st;
+    p.first_block = blocks;
+    blocks += (unsigned)(p.ctas * splits);
+    smem = std::max(smem, p.stages * pixel_bytes_of(p) * p.kp + 1024 + 256);
+    b.e[i] = jobs[i].e;
+  }
+  NRS_ENSURE_SMEM(ctx, attr, (tc_wgrad_kernel<NPLANES, CAP>), smem);
   int* err = nullptr;
-  const int st = nrs_err_flag(ctx, &err);
+  int st = nrs_err_flag(ctx, &err);
   if (st != NRS_OK) return st;
-  dim3 grid((unsigned)(p.m_blocks * p.n_groups * p.col_blocks), (unsigned)splits);
-  NRS_PDL_LAUNCH((tc_wgrad_kernel<NPLANES, STAGES>), grid, kWgThreads, smem_bytes, ctx->stream, maps[0], maps[1], maps[2],
-                 maps[3], p, p.group_cols, err);
+  NRS_PDL_LAUNCH((tc_wgrad_kernel<NPLANES, CAP>), blocks, kWgThreads, smem, ctx->stream, b, err);
   NRS_LAUNCHED(ctx);
-  return NRS_OK;
+  // dw[co][ci][tap] (+)= sum over splits of partial[split][mb][grp][col block][row][t*cblocks*wb + c]
+  for (int i = 0; i < n && st == NRS_OK; ++i) {
+    const WgradParams& p = jobs[i].e.p;
+    if (p.direct) continue;
+    NrsFoldJob j{};
+    j.kind = NRS_FOLD_WGRAD;
+    j.src = p.partial; j.dst = jobs[i].dw;
+    j.accumulate = jobs[i].accumulate;
+    j.splits = (p.n_tiles + p.tiles_per_split - 1) / p.tiles_per_split;
+    j.lanes = reduce_lanes(j.splits);
+    j.co = p.co; j.ci = p.ci; j.taps = p.kh * p.kw;
+    j.taps_per_group = p.taps_per_group; j.n_groups = p.n_groups; j.col_blocks = p.col_blocks; j.cblocks = p.cblocks * p.wb / 32;
+    j.group_cols = p.group_cols;
+    j.out_cols = jobs[i].out_cols;
+    j.split_stride = split_floats(p);
+    st = nrs_fold_submit(ctx, j);
+  }
+  return st;
+}
+template <int CAP>
+int launch_wgrad(nrs_ctx* ctx, WgradJob* jobs, int n, bool independent) {
+  return jobs[0].planes == 2 ? launch_wgrad<2, CAP>(ctx, jobs, n, independent) : launch_wgrad<1, CAP>(ctx, jobs, n, independent);
 }
 
 }  // namespace
@@ -346,10 +414,8 @@ int nrs_tc_conv_wgrad(nrs_ctx* ctx, const float* x, const float* dy, float* dw, 
   }
   const bool can_be_direct = taps == 1 && ci % p.wb == 0 && !accumulate && !out_cols && (reinterpret_cast<uintptr_t>(dw) & 15) == 0;
   // The pixel box of a plan, and the ring its operands allow; false where there is none.
-  size_t pixel_bytes = 0;
-  int stages = 0;
   auto box = [&](WgradParams* q) {
-    pixel_bytes = (size_t)(128 + q->group_cols) * 4;   // both operands, all planes
+    const size_t pixel_bytes = pixel_bytes_of(*q);
     q->kp = 0;
     plan_pixel_box(q, n, oh, ow, planes, pixel_bytes);
     if (q->kp == 0) return false;
@@ -358,12 +424,23 @@ int nrs_tc_conv_wgrad(nrs_ctx* ctx, const float* x, const float* dy, float* dw, 
     const long n_tiles = (long)((n + q->Nt - 1) / q->Nt) * q->tiles_y * q->tiles_x;
     if (n_tiles > 2147483647L) return false;
     q->n_tiles = (int)n_tiles;
-    stages = (int)((200 * 1024) / (pixel_bytes * q->kp));
-    if (stages > 6) stages = 6;
-    return stages >= 2;
+    q->stages = std::min(6, (int)((200 * 1024) / (pixel_bytes * q->kp)));
+    q->ctas = q->m_blocks * q->n_groups * q->col_blocks;
+    return q->stages >= 2;
   };
+  const NrsPlanes *dy_ready = nrs_planes_find(ctx, dy, split3), *x_ready = nrs_planes_find(ctx, x, split3);
+  const bool waits = dy_ready && x_ready && nrs_wgrad_may_wait(ctx, dy_ready->hi, x_ready->hi);
   int tps = 0;   // pixel tiles per CTA
-  if (taps == 1) {
+  if (waits) {   // shared out with the others; wide column blocks, which read the least
+    if (tap_cols > kMaxN) {
+      p.col_blocks = (tap_cols + kMaxN - 1) / kMaxN;
+      p.n_groups = taps;
+      p.taps_per_group = 1;
+      p.group_cols = kMaxN;
+    }
+    if (!box(&p)) return NRS_ERR_UNSUPPORTED;
+    tps = p.n_tiles;
+  } else if (taps == 1) {
     // A^T B: columns per CTA and pixel split together, by what a CTA takes (its UMMAs, 46 clocks at least, or its operands'
     // way at about 60 bytes a clock; 2500 clocks and the store of its tile besides) and the second pass, which reads
     // splits + 1 times the output at about 1.1 KB a clock.  No split is longer than an accumulation chain may be.
@@ -380,13 +457,14 @@ int nrs_tc_conv_wgrad(nrs_ctx* ctx, const float* x, const float* dy, float* dw, 
         continue;   // one CTA takes all columns as it is
       }
       if (!box(&q)) continue;
-      const int max_tiles = split3 ? tc::kMaxChainK / q.kp : 1 << 30, ctas = q.m_blocks * q.col_blocks;
-      const double umma = (split3 ? 3.0 : 2.0) * std::max(q.group_cols / 2, 47), fill = 16.0 * pixel_bytes / 60.0;   // per 16 pixels
+      const int ctas = q.ctas;
+      const long most = max_tiles(q, planes);
+      const double umma = (split3 ? 3.0 : 2.0) * std::max(q.group_cols / 2, 47), fill = 16.0 * pixel_bytes_of(q) / 60.0;   // per 16 pixels
       for (int i = 1, last = 0; i <= 96; ++i) {   // up to 64 splits, then whole waves
         const long s = i <= 64 ? i : (long)(i - 64) * ctx->sm_count / ctas;
         if (s < 1 || (i > 64 && s <= 64)) continue;
         const int per = (int)((q.n_tiles + s - 1) / s);
-        if (per > max_tiles || per == last || s > 65535) continue;
+        if (per > most || per == last) continue;
         last = per;
         const long splits = (q.n_tiles + per - 1) / per;
         const double rounds = (double)((ctas * splits + ctx->sm_count - 1) / ctx->sm_count);
@@ -400,46 +478,39 @@ int nrs_tc_conv_wgrad(nrs_ctx* ctx, const float* x, const float* dy, float* dw, 
       }
     }
     // (a reduction that needs more splits by the chain limit alone)
-    if (best < 0.0 && box(&p)) tps = std::max(1, split3 ? tc::kMaxChainK / p.kp : p.n_tiles);
+    if (best < 0.0 && box(&p)) tps = (int)std::min((long)p.n_tiles, max_tiles(p, planes));
     if (tps == 0 || !box(&p)) return NRS_ERR_UNSUPPORTED;
   } else {
     if (!box(&p)) return NRS_ERR_UNSUPPORTED;
     // pixel split: fill the GPU, and bound the accumulation chain in 3xTF32 mode
-    const int ctas_per_split = p.m_blocks * p.n_groups * p.col_blocks;
-    const int max_tiles = split3 ? tc::kMaxChainK / p.kp : 1 << 30;
+    const int ctas_per_split = p.ctas, most = (int)std::min(max_tiles(p, planes), 1L << 30);
     int min_tiles = 512 / p.kp;   // amortise the prologue and the partial-tile store
     // ... unless that leaves most of the GPU idle
     while (min_tiles > 4 && (long)(p.n_tiles / min_tiles) * ctas_per_split < ctx->sm_count / 2) min_tiles /= 2;
-    if (min_tiles > max_tiles) min_tiles = max_tiles;
-    tps = tc::plan_units_per_cta(ctx->sm_count, ctas_per_split, p.n_tiles, min_tiles, max_tiles, 8);
+    if (min_tiles > most) min_tiles = most;
+    tps = tc::plan_units_per_cta(ctx->sm_count, ctas_per_split, p.n_tiles, min_tiles, most, 8);
   }
-  const size_t smem_bytes = stages * pixel_bytes * p.kp + 1024 + 256;
   p.tiles_per_split = tps;
-  const int splits = (p.n_tiles + tps - 1) / tps;
-  if (splits > 65535) return NRS_ERR_UNSUPPORTED;
+  if ((long)p.ctas * ((p.n_tiles + tps - 1) / tps) > 2147483647L) return NRS_ERR_UNSUPPORTED;
 
-  // workspaces: NHWC planes of dy and x, and the partial tiles
+  // workspaces: NHWC planes of dy and x
   const int dy_ld = nrs_plane_ld(co), x_ld = nrs_plane_ld(ci);
   const size_t dy_plane = (size_t)n * oh * ow * dy_ld, x_plane = (size_t)n * h * wd * x_ld;
-  const size_t partial_floats = (size_t)splits * p.m_blocks * p.n_groups * p.col_blocks * 128 * p.group_cols;
   void *dy_hi = nullptr, *dy_lo = nullptr, *x_hi = nullptr, *x_lo = nullptr;
-  // a single split of a 1x1 "convolution" (A^T B) that overwrites its output needs no second pass
-  p.direct = splits == 1 && can_be_direct ? dw : nullptr;
-  int st = p.direct ? NRS_OK : nrs_fold_partial(ctx, NRS_WS_WGRAD_PARTIAL, partial_floats * sizeof(float), &p.partial);
-  if (st != NRS_OK) return st;
+  int st = NRS_OK;
   bool may_overlap = ctx->independent_next;   // withdrawn below if this call stages an operand itself
-  if (const NrsPlanes* ready = nrs_planes_find(ctx, dy, split3)) {
-    dy_hi = ready->hi;
-    dy_lo = ready->lo;
+  if (dy_ready) {
+    dy_hi = dy_ready->hi;
+    dy_lo = dy_ready->lo;
   } else {
     may_overlap = false;
     st = nrs_ws_planes(ctx, NRS_WS_A, dy_plane, split3, &dy_hi, &dy_lo);
     if (st == NRS_OK) st = nrs_tc_stage_image(ctx, dy, (float*)dy_hi, (float*)dy_lo, n, co, oh * ow);
     if (st != NRS_OK) return st;
   }
-  if (const NrsPlanes* ready = nrs_planes_find(ctx, x, split3)) {
-    x_hi = ready->hi;
-    x_lo = ready->lo;
+  if (x_ready) {
+    x_hi = x_ready->hi;
+    x_lo = x_ready->lo;
   } else {
     may_overlap = false;
     st = nrs_ws_planes(ctx, NRS_WS_B, x_plane, split3, &x_hi, &x_lo);
@@ -449,6 +520,7 @@ int nrs_tc_conv_wgrad(nrs_ctx* ctx, const float* x, const float* dy, float* dw, 
 
   // Planes viewed as [channel block][n][h][w][32 or 64 channels], the block index outermost, so that one box brings all
   // blocks; with a ragged channel count as [n][h][w][channels], one block per box.
+  WgradJob job{};
   CUtensorMap maps[4];
   p.a_box_blocks = std::min(padded(co, p.wa), 128) / p.wa;
   auto encode = [&](CUtensorMap* m, void* base, bool ragged, int c, int w, int ld, int img_h, int img_w, int step, int blocks) {
@@ -465,33 +537,48 @@ int nrs_tc_conv_wgrad(nrs_ctx* ctx, const float* x, const float* dy, float* dw, 
                    encode(&maps[3], x_lo, p.ragged_x, ci, p.wb, x_ld, h, wd, stride, x_blocks);
   else { maps[1] = maps[0]; maps[3] = maps[2]; }
   NRS_REQUIRE(ctx, ok, NRS_ERR_CUDA, "tc_wgrad: cuTensorMapEncodeTiled failed");
-  p.independent = may_overlap ? 1 : 0;
   p.range_dy = nrs_range_of(ctx, dy_hi);
   p.range_x = nrs_range_of(ctx, x_hi);
+  job.e = WgradEntry{maps[0], maps[1], maps[2], maps[3], p};
+  job.planes = planes;
+  job.dw = dw;
+  job.accumulate = accumulate;
+  job.out_cols = out_cols;
+  job.can_be_direct = can_be_direct;
+  if (!waits) return launch_wgrad<1>(ctx, &job, 1, may_overlap);
+  NrsFolds& f = ctx->folds;
+  if (!f.waiting_tiles) f.waiting_tiles = std::make_shared<std::vector<WgradJob>>();
+  static_cast<std::vector<WgradJob>*>(f.waiting_tiles.get())->push_back(job);
+  f.waiting.push_back({dw, (size_t)co * ci * taps});
+  return NRS_OK;
+}
 
-#define NRS_WG(PL)                                                                     \
-  switch (stages) {                                                                    \
-    case 2: st = launch_wgrad<PL, 2>(ctx, maps, p, splits, smem_bytes); break;         \
-    case 3: st = launch_wgrad<PL, 3>(ctx, maps, p, splits, smem_bytes); break;         \
-    case 4: st = launch_wgrad<PL, 4>(ctx, maps, p, splits, smem_bytes); break;         \
-    case 5: st = launch_wgrad<PL, 5>(ctx, maps, p, splits, smem_bytes); break;         \
-    default: st = launch_wgrad<PL, 6>(ctx, maps, p, splits, smem_bytes); break;        \
+int nrs_wgrad_tiles_run(nrs_ctx* ctx) {
+  auto all = std::static_pointer_cast<std::vector<WgradJob>>(ctx->folds.waiting_tiles);
+  ctx->folds.waiting_tiles.reset();
+  if (!all) return NRS_OK;
+  constexpr double kMostPartial = 256.0 * (1 << 20);   // bytes of partial tiles in one launch
+  for (size_t i = 0, e; i < all->size(); i = e) {
+    WgradJob* jobs = all->data() + i;
+    const int planes = jobs[0].planes;
+    std::vector<wgq::Piece> pieces;
+    double least = 0.0;
+    for (e = i; e < all->size() && (int)(e - i) < kWgBatch; ++e) {
+      const WgradParams& p = (*all)[e].e.p;
+      const long most = max_tiles(p, planes);
+      const double bytes = (double)split_floats(p) * sizeof(float), need = bytes * ((p.n_tiles + most - 1) / most);
+      if ((*all)[e].planes != planes || (e > i && least + need > kMostPartial)) break;
+      least += need;
+      const double umma = p.kp / 16.0 * (planes == 2 ? 3.0 : 2.0) * std::max(p.group_cols / 2, 47), fill = p.kp * pixel_bytes_of(p) / 60.0;
+      pieces.push_back({p.ctas, p.n_tiles, std::max(umma, fill), 2500.0 + 4.0 * p.group_cols, most, bytes, 0});
+    }
+    wgq::share_out(pieces, ctx->sm_count);
+    const int n = (int)(e - i);
+    for (int k = 0; k < n; ++k) jobs[k].e.p.tiles_per_split = (int)pieces[k].per;
+    const int st = n == 1 ? launch_wgrad<1>(ctx, jobs, 1, false) : launch_wgrad<kWgBatch>(ctx, jobs, n, false);
+    if (st != NRS_OK) return st;
   }
-  if (split3) { NRS_WG(2) } else { NRS_WG(1) }
-#undef NRS_WG
-  if (st != NRS_OK) return st;
-  if (p.direct) return NRS_OK;
-  // dw[co][ci][tap] (+)= sum over splits of partial[split][mb][grp][col block][row][t*cblocks*32 + c]
-  NrsFoldJob j{};
-  j.kind = NRS_FOLD_WGRAD;
-  j.src = p.partial; j.dst = dw;
-  j.accumulate = accumulate; j.splits = splits; j.lanes = reduce_lanes(splits);
-  j.co = co; j.ci = ci; j.taps = taps;
-  j.taps_per_group = p.taps_per_group; j.n_groups = p.n_groups; j.col_blocks = p.col_blocks; j.cblocks = tap_cols / 32;
-  j.group_cols = p.group_cols;
-  j.out_cols = out_cols;
-  j.split_stride = (size_t)p.m_blocks * p.n_groups * p.col_blocks * 128 * p.group_cols;
-  return nrs_fold_submit(ctx, j);
+  return NRS_OK;
 }
 
 // C[m,n] (+)= A^T B for A stored [k][m] and B stored [k][n] (both row-major) without transposing either:

@@ -28,6 +28,7 @@
 // 298-320) for the shapes it covers; everything else takes tc_wgrad.cu.
 #include "fold.h"
 #include "tc_mainloop.cuh"
+#include "wgrad_queue.h"
 
 namespace {
 
@@ -51,20 +52,36 @@ struct RowParams {
   float* partial;                 // [split][cta][128][3*chunk]
   int cross;                      // 3xTF32: accumulator columns between the hi*hi sums and the others
   const NrsRange *range_dy, *range_x;
+  int ctas;                       // per split
+  unsigned first_block;           // of this gradient's in the launch
+};
+// The gradients of one launch.
+struct RowEntry {
+  CUtensorMap dy_hi, dy_lo, x_hi, x_lo;
+  RowParams p;
+};
+template <int CAP>
+struct RowBatch {
+  RowEntry e[CAP];
+  int n;
   int independent;                // reads nothing the kernel launched just before it wrote (NRS_PDL_PROLOGUE)
 };
+constexpr int kRowBatch = 12;
 
 // Bytes of one plane of a stage's operands.  (A UMMA reads 128 channels of dy whatever there are: the slab of x behind
 // them is at least as long as what that reads beyond.)
 __host__ __device__ inline uint32_t dy_bytes(const RowParams& p, int value) { return (uint32_t)((p.pack ? 2 : 1) * p.a_blocks * p.wa * p.P * value); }
 __host__ __device__ inline uint32_t x_bytes(const RowParams& p, int value) { return (uint32_t)(p.chunk * (p.R + 2) * p.Wt * value); }
 
-template <int NPLANES>
+template <int NPLANES, int CAP>
 __global__ void __launch_bounds__(kRowThreads, 1)
-tc_wgrad_rows_kernel(const __grid_constant__ CUtensorMap tm_dy_hi, const __grid_constant__ CUtensorMap tm_dy_lo,
-                     const __grid_constant__ CUtensorMap tm_x_hi, const __grid_constant__ CUtensorMap tm_x_lo,
-                     const RowParams p, int* __restrict__ err_flag) {
+tc_wgrad_rows_kernel(const __grid_constant__ RowBatch<CAP> batch, int* __restrict__ err_flag) {
   extern __shared__ uint8_t smem_raw[];
+  int entry = 0;
+  while (CAP > 1 && entry + 1 < batch.n && batch.e[entry + 1].p.first_block <= blockIdx.x) ++entry;
+  const RowEntry& en = batch.e[entry];
+  const RowParams& p = en.p;
+  const CUtensorMap &tm_dy_hi = en.dy_hi, &tm_dy_lo = en.dy_lo, &tm_x_hi = en.x_hi, &tm_x_lo = en.x_lo;
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   constexpr int kValue = NPLANES == 2 ? 2 : 4;
   constexpr int kStepPixels = NPLANES == 2 ? 16 : 8;
@@ -78,15 +95,15 @@ tc_wgrad_rows_kernel(const __grid_constant__ CUtensorMap tm_dy_hi, const __grid_
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accum_bar + 1);
 
   const int warp = (int)tc::uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
-  // blockIdx.x = (m block, horizontal tap kind, channel chunk).  Unpacked: kind = tap j, x shifted by
+  // A block is (split, m block, horizontal tap kind, channel chunk).  Unpacked: kind = tap j, x shifted by
   // j - 1.  Packed: kind 0 shifts x by 0 and holds taps j = 1 (plain dy) and j = 0 (dy shifted one
   // pixel: sum_p dy[p+1] x[p] = sum_p dy[p] x[p-1]); kind 1 shifts x by +1 and holds j = 2 alone.
-  const int cc = blockIdx.x % p.n_chunks;
-  const int jk = (blockIdx.x / p.n_chunks) % p.jtypes;
-  const int mb = blockIdx.x / (p.n_chunks * p.jtypes);
+  const int local = (int)(blockIdx.x - p.first_block), split = local / p.ctas, cta = local - split * p.ctas;
+  const int cc = cta % p.n_chunks;
+  const int jk = (cta / p.n_chunks) % p.jtypes;
+  const int mb = cta / (p.n_chunks * p.jtypes);
   const int x_shift = p.pack ? jk : jk - 1;
   const bool two_taps = p.pack && jk == 0;
-  const int split = blockIdx.y;
   const int t0 = split * p.tiles_per_split, steps = min(p.n_tiles - t0, p.tiles_per_split);
   const uint32_t tmem_cols = (NPLANES == 2 ? 2u : 1u) * (kTaps * p.chunk <= 128 ? 128u : (kTaps * p.chunk <= 256 ? 256u : 512u));
 
@@ -106,7 +123,7 @@ tc_wgrad_rows_kernel(const __grid_constant__ CUtensorMap tm_dy_hi, const __grid_
   __syncthreads();
   tc::tc_fence_after_sync();
   const uint32_t tmem_base = tc::uniform(*tmem_slot);
-  if (!p.independent) NRS_PDL_WAIT();   // set-up above may overlap the previous kernel's tail; its results are needed from here
+  if (!batch.independent) NRS_PDL_WAIT();   // set-up above may overlap the previous kernel's tail; its results are needed from here
   NRS_PDL_TRIGGER();
 
   // (Both issuing roles run as whole warps and elect a lane for the instructions themselves: tc::elect_one.)
@@ -201,7 +218,7 @@ tc_wgrad_rows_kernel(const __grid_constant__ CUtensorMap tm_dy_hi, const __grid_
       tc::tc_fence_after_sync();
       const int row = q * 32 + lane;
       const int cols = kTaps * p.chunk;
-      float* dst = p.partial + (((size_t)split * gridDim.x + blockIdx.x) * 128 + row) * cols;
+      float* dst = p.partial + ((size_t)local * 128 + row) * cols;
       // packed: rows [0,h) are tap j = 1 or 2, rows [h,2h) tap j = 0 (kind 0 only)
       const int half = p.wa * p.a_blocks;
       const bool row_live = p.pack ? (row < half || (two_taps && row < 2 * half)) : (mb * 128 + row < p.co);
@@ -234,7 +251,7 @@ tc_wgrad_rows_kernel(const __grid_constant__ CUtensorMap tm_dy_hi, const __grid_
     }
   }
 
-  if (p.independent) NRS_PDL_WAIT();   // nothing after this kernel may run ahead of its predecessor
+  if (batch.independent) NRS_PDL_WAIT();   // nothing after this kernel may run ahead of its predecessor
   __syncwarp();
   tc::tc_fence_before_sync();
   __syncthreads();
@@ -273,17 +290,63 @@ bool plan_row_tile(RowParams* p, int h, int w, int planes) {
   return best >= 0.0;
 }
 
-template <int NPLANES>
-int launch_rows(nrs_ctx* ctx, const CUtensorMap* maps, const RowParams& p, int ctas, int splits, size_t smem_bytes) {
+// A weight gradient that may wait.
+struct RowJob {
+  RowEntry e;
+  int planes;
+  float* dw;
+  int accumulate;
+};
+size_t smem_of(const RowParams& p, int planes) {
+  const int value = planes == 2 ? 2 : 4;
+  return (size_t)p.stages * planes * (dy_bytes(p, value) + x_bytes(p, value)) + (size_t)128 * p.P * value + (size_t)(2 * p.stages + 1) * 8 + 16 + 1024;
+}
+long max_tiles(const RowParams& p, int planes) { return planes == 2 ? tc::kMaxChainPairs / p.P : 1 << 30; }
+size_t split_floats(const RowParams& p) { return (size_t)p.ctas * 128 * kTaps * p.chunk; }
+
+template <int NPLANES, int CAP>
+int launch_rows(nrs_ctx* ctx, RowJob* jobs, int n, bool independent) {
   static NrsSmemAttr attr;
-  NRS_ENSURE_SMEM(ctx, attr, (tc_wgrad_rows_kernel<NPLANES>), smem_bytes);
+  RowBatch<CAP> b{};
+  size_t smem = 0;
+  unsigned blocks = 0;
+  b.n = n;
+  b.independent = independent ? 1 : 0;
+  for (int i = 0; i < n; ++i) {
+    RowParams& p = jobs[i].e.p;
+    const int splits = (p.n_tiles + p.tiles_per_split - 1) / p.tiles_per_split;
+    const int st = nrs_fold_partial(ctx, NRS_WS_WGRAD_PARTIAL, splits * split_floats(p) * sizeof(float), &p.partial);
+    if (st != NRS_OK) return st;
+    p.first_block = blocks;
+    blocks += (unsigned)(p.ctas * splits);
+    smem = std::max(smem, smem_of(p, NPLANES));
+    b.e[i] = jobs[i].e;
+  }
+  NRS_ENSURE_SMEM(ctx, attr, (tc_wgrad_rows_kernel<NPLANES, CAP>), smem);
   int* err = nullptr;
-  const int st = nrs_err_flag(ctx, &err);
+  int st = nrs_err_flag(ctx, &err);
   if (st != NRS_OK) return st;
-  dim3 grid((unsigned)ctas, (unsigned)splits);
-  NRS_PDL_LAUNCH((tc_wgrad_rows_kernel<NPLANES>), grid, kRowThreads, smem_bytes, ctx->stream, maps[0], maps[1], maps[2], maps[3], p, err);
+  NRS_PDL_LAUNCH((tc_wgrad_rows_kernel<NPLANES, CAP>), blocks, kRowThreads, smem, ctx->stream, b, err);
   NRS_LAUNCHED(ctx);
-  return NRS_OK;
+  // dw[co][ci][i][j] (+)= sum over splits of the partial accumulators
+  for (int i = 0; i < n && st == NRS_OK; ++i) {
+    const RowParams& p = jobs[i].e.p;
+    NrsFoldJob jb{};
+    jb.kind = NRS_FOLD_WGRAD_ROWS;
+    jb.src = p.partial; jb.dst = jobs[i].dw;
+    jb.accumulate = jobs[i].accumulate;
+    jb.splits = (p.n_tiles + p.tiles_per_split - 1) / p.tiles_per_split;
+    jb.lanes = reduce_lanes(jb.splits);
+    jb.co = p.co; jb.ci = p.ci; jb.taps = 9;
+    jb.chunk = p.chunk; jb.n_chunks = p.n_chunks; jb.jtypes = p.jtypes; jb.a_blocks = p.a_blocks * p.wa / 32; jb.pack = p.pack;
+    jb.split_stride = split_floats(p);
+    st = nrs_fold_submit(ctx, jb);
+  }
+  return st;
+}
+template <int CAP>
+int launch_rows(nrs_ctx* ctx, RowJob* jobs, int n, bool independent) {
+  return jobs[0].planes == 2 ? launch_rows<2, CAP>(ctx, jobs, n, independent) : launch_rows<1, CAP>(ctx, jobs, n, independent);
 }
 
 }  // namespace
@@ -309,30 +372,25 @@ int nrs_tc_conv_wgrad_rows(nrs_ctx* ctx, const float* x, const float* dy, float*
   p.pack = co <= 64 ? 1 : 0;
   p.jtypes = p.pack ? 2 : 3;
   p.m_blocks = (co + 127) / 128;
+  p.ctas = p.m_blocks * p.jtypes * p.n_chunks;
   if (!plan_row_tile(&p, h, wd, planes)) return NRS_ERR_UNSUPPORTED;
   const long tiles = (long)n * p.tiles_x * p.tiles_y;
   if (tiles > 2000000000L) return NRS_ERR_UNSUPPORTED;
   p.n_tiles = (int)tiles;
-  const int value = split3 ? 2 : 4;
-  const size_t smem_bytes = (size_t)p.stages * planes * (dy_bytes(p, value) + x_bytes(p, value)) + (size_t)128 * p.P * value +
-                            (size_t)(2 * p.stages + 1) * 8 + 16 + 1024;
-  if (smem_bytes > 227 * 1024) return NRS_ERR_UNSUPPORTED;
+  if (smem_of(p, planes) > 227 * 1024) return NRS_ERR_UNSUPPORTED;
 
-  // tile split: fill the GPU, bound the accumulation chain in 3xTF32 mode, amortise the partial tile
-  const int ctas = p.m_blocks * p.jtypes * p.n_chunks;
-  const int max_tiles = split3 ? tc::kMaxChainK / p.P : 1 << 30;
+  // tile split (of a gradient that does not wait): fill the GPU, bound the accumulation chain in 3xTF32 mode, amortise the
+  // partial tile
+  const int most = (int)std::min(max_tiles(p, planes), 1L << 30);
   int min_tiles = (512 + p.P - 1) / p.P;
-  if (min_tiles > max_tiles) min_tiles = max_tiles;
-  p.tiles_per_split = tc::plan_units_per_cta(ctx->sm_count, ctas, p.n_tiles, min_tiles, max_tiles, 2 + 256 / p.P);
-  const int splits = (p.n_tiles + p.tiles_per_split - 1) / p.tiles_per_split;
-  if (splits > 65535) return NRS_ERR_UNSUPPORTED;
+  if (min_tiles > most) min_tiles = most;
+  p.tiles_per_split = tc::plan_units_per_cta(ctx->sm_count, p.ctas, p.n_tiles, min_tiles, most, 2 + 256 / p.P);
+  if ((long)p.ctas * ((p.n_tiles + p.tiles_per_split - 1) / p.tiles_per_split) > 2147483647L) return NRS_ERR_UNSUPPORTED;
 
-  // workspaces: NHWC planes of dy and x (or the caller's registered planes), and the partial tiles
+  // workspaces: NHWC planes of dy and x (or the caller's registered planes)
   const size_t dy_plane = (size_t)n * h * wd * co, x_plane = (size_t)n * h * wd * ci;
-  const size_t partial_floats = (size_t)splits * ctas * 128 * kTaps * p.chunk;
   void *dy_hi = nullptr, *dy_lo = nullptr, *x_hi = nullptr, *x_lo = nullptr;
-  int st = nrs_fold_partial(ctx, NRS_WS_WGRAD_PARTIAL, partial_floats * sizeof(float), &p.partial);
-  if (st != NRS_OK) return st;
+  int st = NRS_OK;
   bool may_overlap = ctx->independent_next;   // withdrawn below if this call stages an operand itself
   const size_t dy_img = (size_t)h * wd * co, x_img = (size_t)h * wd * ci;
   if (const NrsPlanes* ready = nrs_planes_find(ctx, dy, split3)) {
@@ -355,29 +413,59 @@ int nrs_tc_conv_wgrad_rows(nrs_ctx* ctx, const float* x, const float* dy, float*
   }
 
   // planes viewed as [channel block][n][h][w][channels of a block]; a box is some rows of some blocks
-  CUtensorMap maps[4];
+  RowJob job{};
   auto encode = [&](CUtensorMap* m, const void* base, int c, int w, int rows, int blocks) {
     const uint64_t dim[5] = {(uint64_t)w, (uint64_t)wd, (uint64_t)h, (uint64_t)n, (uint64_t)(c / w)};
     const uint64_t str[4] = {(uint64_t)c, (uint64_t)wd * c, (uint64_t)h * wd * c, (uint64_t)w};
     const uint32_t box[5] = {(uint32_t)w, (uint32_t)p.Wt, (uint32_t)rows, 1, (uint32_t)blocks};
     return tc::encode_tmap(m, base, split3, 5, dim, str, box, true);
   };
-  bool ok = encode(&maps[0], dy_hi, co, p.wa, p.R, p.a_blocks) && encode(&maps[2], x_hi, ci, p.wb, p.R + 2, p.chunk / p.wb);
-  if (split3) ok = ok && encode(&maps[1], dy_lo, co, p.wa, p.R, p.a_blocks) && encode(&maps[3], x_lo, ci, p.wb, p.R + 2, p.chunk / p.wb);
-  else { maps[1] = maps[0]; maps[3] = maps[2]; }
+  RowEntry& e = job.e;
+  bool ok = encode(&e.dy_hi, dy_hi, co, p.wa, p.R, p.a_blocks) && encode(&e.x_hi, x_hi, ci, p.wb, p.R + 2, p.chunk / p.wb);
+  if (split3) ok = ok && encode(&e.dy_lo, dy_lo, co, p.wa, p.R, p.a_blocks) && encode(&e.x_lo, x_lo, ci, p.wb, p.R + 2, p.chunk / p.wb);
+  else { e.dy_lo = e.dy_hi; e.x_lo = e.x_hi; }
   NRS_REQUIRE(ctx, ok, NRS_ERR_CUDA, "tc_wgrad_rows: cuTensorMapEncodeTiled failed");
-  p.independent = may_overlap ? 1 : 0;
   p.range_dy = nrs_range_of(ctx, dy_hi);
   p.range_x = nrs_range_of(ctx, x_hi);
-  st = split3 ? launch_rows<2>(ctx, maps, p, ctas, splits, smem_bytes) : launch_rows<1>(ctx, maps, p, ctas, splits, smem_bytes);
-  if (st != NRS_OK) return st;
-  // dw[co][ci][i][j] (+)= sum over splits of the partial accumulators
-  NrsFoldJob jb{};
-  jb.kind = NRS_FOLD_WGRAD_ROWS;
-  jb.src = p.partial; jb.dst = dw;
-  jb.accumulate = accumulate; jb.splits = splits; jb.lanes = reduce_lanes(splits);
-  jb.co = co; jb.ci = ci; jb.taps = 9;
-  jb.chunk = p.chunk; jb.n_chunks = p.n_chunks; jb.jtypes = p.jtypes; jb.a_blocks = p.a_blocks * p.wa / 32; jb.pack = p.pack;
-  jb.split_stride = (size_t)ctas * 128 * kTaps * p.chunk;
-  return nrs_fold_submit(ctx, jb);
+  e.p = p;
+  job.planes = planes;
+  job.dw = dw;
+  job.accumulate = accumulate;
+  if (nrs_wgrad_may_wait(ctx, dy_hi, x_hi)) {
+    NrsFolds& f = ctx->folds;
+    if (!f.waiting_rows) f.waiting_rows = std::make_shared<std::vector<RowJob>>();
+    static_cast<std::vector<RowJob>*>(f.waiting_rows.get())->push_back(job);
+    f.waiting.push_back({dw, (size_t)co * ci * 9});
+    return NRS_OK;
+  }
+  return launch_rows<1>(ctx, &job, 1, may_overlap);
+}
+
+int nrs_wgrad_rows_run(nrs_ctx* ctx) {
+  auto all = std::static_pointer_cast<std::vector<RowJob>>(ctx->folds.waiting_rows);
+  ctx->folds.waiting_rows.reset();
+  if (!all) return NRS_OK;
+  constexpr double kMostPartial = 256.0 * (1 << 20);   // bytes of partial tiles in one launch
+  for (size_t i = 0, e; i < all->size(); i = e) {
+    RowJob* jobs = all->data() + i;
+    const int planes = jobs[0].planes;
+    std::vector<wgq::Piece> pieces;
+    double least = 0.0;
+    for (e = i; e < all->size() && (int)(e - i) < kRowBatch; ++e) {
+      const RowParams& p = (*all)[e].e.p;
+      const long most = max_tiles(p, planes);
+      const double bytes = (double)split_floats(p) * sizeof(float), umma = (planes == 2 ? 3 : 1) * (p.chunk / p.wb) * kTaps * p.wb * 0.5;
+      const double need = bytes * ((p.n_tiles + most - 1) / most);
+      if ((*all)[e].planes != planes || (e > i && least + need > kMostPartial)) break;
+      least += need;
+      const double fill = planes * (dy_bytes(p, planes == 2 ? 2 : 4) + x_bytes(p, planes == 2 ? 2 : 4)) / 60.0;
+      pieces.push_back({p.ctas, p.n_tiles, std::max(p.P / (planes == 2 ? 16.0 : 8.0) * umma, fill) + 110.0, 4000.0, most, bytes, 0});
+    }
+    wgq::share_out(pieces, ctx->sm_count);
+    const int n = (int)(e - i);
+    for (int k = 0; k < n; ++k) jobs[k].e.p.tiles_per_split = (int)pieces[k].per;
+    const int st = n == 1 ? launch_rows<1>(ctx, jobs, 1, false) : launch_rows<kRowBatch>(ctx, jobs, n, false);
+    if (st != NRS_OK) return st;
+  }
+  return NRS_OK;
 }
