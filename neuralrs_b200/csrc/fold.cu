@@ -15,6 +15,9 @@
 namespace {
 
 constexpr int kMaxJobs = 32;
+// Rows of a column fold that one block takes at least: 16 per warp, two rounds of loads.  (1024 rows to a block are
+// thirteen rounds of loads, one behind the other.)
+constexpr int kColumnRows = 128;
 // The divisions that place a weight gradient's outputs, as multiplications (with 32-bit divisions the pass was bound by
 // instructions: 740 per warp, most of them there).
 struct FoldDiv {
@@ -23,6 +26,7 @@ struct FoldDiv {
 template <int CAP>
 struct FoldBatch {
   int n;
+  unsigned first_block[CAP];   // of each job, side by side: the search over them is one or two lines of constant memory
   NrsFoldJob job[CAP];
   FoldDiv div[CAP];
 };
@@ -33,8 +37,8 @@ __device__ __forceinline__ void put(float* dst, float v, int accumulate) { *dst 
 __device__ __forceinline__ float* column_dst(const NrsFoldJob& j, int c) { return j.dst2 && c >= j.cols1 ? j.dst2 + (c - j.cols1) : j.dst + c; }
 
 // dst[c] (+)= sum over rows of src[r*stride + c].  A block takes 32 columns of a row split: its eight warps every eighth
-// row, four rows in flight per thread, combined in warp order; with several splits the last block of a column group to
-// arrive adds the splits in order.
+// row, eight rows in flight per thread, combined in warp order; with several splits the last block of a column group to
+// arrive adds the splits in the same way: warp w splits w, w + 8, ...
 __device__ void fold_columns(const NrsFoldJob& j, unsigned blk, float* sm) {
   __shared__ bool last;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -45,12 +49,14 @@ __device__ void fold_columns(const NrsFoldJob& j, unsigned blk, float* sm) {
   if (c < j.cols) {
     const size_t step = (size_t)8 * j.stride;
     const float* s = j.src + (size_t)(r0 + warp) * j.stride + c;
-    int r = r0 + warp;
-    for (; r + 24 < r1; r += 32, s += 4 * step) {
-      const float v0 = s[0], v1 = s[step], v2 = s[2 * step], v3 = s[3 * step];
-      t += v0; t += v1; t += v2; t += v3;
+    for (int r = r0 + warp; r < r1; r += 64, s += 8 * step) {   // eight loads under way, the last round's too
+      float v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = r + 8 * u < r1 ? s[u * step] : 0.0f;
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (r + 8 * u < r1) t += v[u];
     }
-    for (; r < r1; r += 8, s += step) t += *s;
   }
   sm[warp * 32 + lane] = t;
   __syncthreads();
@@ -68,9 +74,22 @@ __device__ void fold_columns(const NrsFoldJob& j, unsigned blk, float* sm) {
   __syncthreads();
   if (!last) return;
   __threadfence();
+  t = 0.0f;
+  if (c < j.cols)
+    for (int z = warp; z < j.splits; z += 64) {
+      float v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = z + 8 * u < j.splits ? __ldcg(j.scratch + (size_t)(z + 8 * u) * j.cols + c) : 0.0f;
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (z + 8 * u < j.splits) t += v[u];
+    }
+  sm[warp * 32 + lane] = t;
+  __syncthreads();
   if (warp == 0 && c < j.cols) {
     float sum = 0.0f;
-    for (int z = 0; z < j.splits; ++z) sum += __ldcg(j.scratch + (size_t)z * j.cols + c);
+#pragma unroll
+    for (int w = 0; w < 8; ++w) sum += sm[w * 32 + lane];
     put(column_dst(j, c), sum, j.accumulate);
   }
   if (threadIdx.x == 0) j.tickets[grp] = 0;
@@ -115,10 +134,15 @@ __device__ void fold_tiles(const NrsFoldJob& j, const FoldDiv& dv, unsigned blk,
   }
   float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
   if (live) {
-#pragma unroll 4
-    for (int z = lane; z < j.splits; z += j.lanes) {
-      const float4 v = *reinterpret_cast<const float4*>(j.src + (size_t)z * j.split_stride + off);
-      s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+    const float* src = j.src + off;
+    for (int z = lane; z < j.splits; z += 8 * j.lanes) {   // eight loads under way, the last round's too
+      float4 v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (z + u * j.lanes < j.splits) v[u] = *reinterpret_cast<const float4*>(src + (size_t)(z + u * j.lanes) * j.split_stride);
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (z + u * j.lanes < j.splits) { s.x += v[u].x; s.y += v[u].y; s.z += v[u].z; s.w += v[u].w; }
     }
   }
   if (j.lanes > 1) {
@@ -180,7 +204,7 @@ __global__ void __launch_bounds__(256) fold_kernel(const __grid_constant__ FoldB
   int i = CAP - 1;
   if (CAP > 1) {
     i = b.n - 1;
-    while (i > 0 && b.job[i].first_block > blockIdx.x) --i;
+    while (i > 0 && b.first_block[i] > blockIdx.x) --i;
   }
   const NrsFoldJob& j = b.job[i];
   const unsigned blk = blockIdx.x - j.first_block;
@@ -215,6 +239,7 @@ int run_table(nrs_ctx* ctx, NrsFoldJob* jobs, int n) {
       b.div[b.n] = FoldDiv{NrsFastDiv(8 * j.taps), NrsFastDiv(32 * j.taps), NrsFastDiv(j.taps), NrsFastDiv((j.ci + 31) / 32),
                            NrsFastDiv(general ? j.taps_per_group : 1), NrsFastDiv(general ? 1 : j.chunk)};
     }
+    b.first_block[b.n] = j.first_block;
     b.job[b.n++] = j;
   }
   if (blocks == 0) return NRS_OK;
@@ -386,8 +411,8 @@ static int fold_columns_to(nrs_ctx* ctx, const float* src, float* dst, float* ds
   j.accumulate = accumulate;
   const int groups = (cols + 31) / 32;
   j.splits = 1;
-  if (rows >= 1024 && groups + 1 <= kNrsFoldTickets) {   // 256 rows per block and up
-    j.splits = std::min(rows / 256, (2 * ctx->sm_count + groups - 1) / groups);
+  if (rows >= 2 * kColumnRows && groups + 1 <= kNrsFoldTickets) {
+    j.splits = std::min(rows / kColumnRows, (2 * ctx->sm_count + groups - 1) / groups);
     if (j.splits < 1) j.splits = 1;
   }
   if (j.splits > 1) {

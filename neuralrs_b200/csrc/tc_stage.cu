@@ -63,7 +63,7 @@ __device__ __forceinline__ float open_range(const Bound& b) { return SPLIT ? pr:
 template <bool SPLIT>
 __global__ void __launch_bounds__(256)
 stage_rows_kernel(const float* __restrict__ src, float* __restrict__ hi, float* __restrict__ lo, int rows, int K,
-                  int ldk, size_t src_bstride, size_t dst_bstride, const Bound bound) {
+                  int ldk, size_t src_bstride, size_t dst_bstride, const NrsFastDiv div_q, const Bound bound) {
   NRS_PDL_PROLOGUE();
   const float scale = open_range<SPLIT>(bound);
   const int b = blockIdx.y;
@@ -74,7 +74,7 @@ stage_rows_kernel(const float* __restrict__ src, float* __restrict__ hi, float* 
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   const bool vec = (K & 3) == 0 && ((reinterpret_cast<uintptr_t>(src) & 15) == 0);
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total4; i += stride) {
-    const size_t r = i / q;
+    const size_t r = total4 < ((size_t)1 << 31) ? div_q.div((uint32_t)i) : i / q;   // (a 64-bit division is some 80 instructions)
     const int k = (int)(i - r * q) * 4;
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     if (vec) {
@@ -230,157 +230,144 @@ stage_masked_kernel(const float* __restrict__ g, const float* __restrict__ y, co
 }
 
 
-// MODE 1 for 2x2 / stride-2 pooling over even-sized images, organised around the POOLED
-// elements (a quarter of the output): a block takes 32 channels x 32 consecutive pooled
-// positions (counted across images), reads g, the pooled output and argmax once, coalesced,
-// and produces the 2x2 windows: NCHW as float2 row segments, NHWC planes one full 128-byte
-// line (32 channels of a pixel) per warp store, through a shared-memory tile.
+// The tile of the two 2x2 / stride-2 pooling kernels below: 32 channels x 32 consecutive pooled positions, counted across
+// the even-sized images.  A thread reads its four channels' values together, all loads under way before the first is used,
+// and writes four channels of a pixel at once.
+struct PoolGrid {
+  int c, h, w;
+  uint32_t positions;   // pooled, in the batch
+  NrsFastDiv div_ohw, div_ow;
+  PoolGrid(int n, int c_, int h_, int w_)
+      : c(c_), h(h_), w(w_), positions((uint32_t)n * (uint32_t)(h_ / 2) * (uint32_t)(w_ / 2)), div_ohw((h_ / 2) * (w_ / 2)), div_ow(w_ / 2) {}
+  static bool fits(int n, int c_, int h_, int w_) { return (double)n * (h_ / 2) * (w_ / 2) < 2147483648.0 && (double)c_ * h_ * w_ < 2147483648.0; }
+  dim3 blocks() const { return dim3((positions + 31) / 32, (unsigned)((c + 31) / 32)); }
+};
+struct PoolPlace {
+  bool live;
+  uint32_t img, po, corner;   // image, pooled position and top left pixel inside its plane
+  __device__ __forceinline__ PoolPlace(const PoolGrid& g, uint32_t pos) {
+    uint32_t oy, ox;
+    live = pos < g.positions;
+    g.div_ohw.divmod(live ? pos : 0u, img, po);
+    g.div_ow.divmod(po, oy, ox);
+    corner = 2 * oy * (uint32_t)g.w + 2 * ox;
+  }
+};
+
+// The backward pass of 2x2 / stride-2 pooling and the ReLU ahead of it, organised around the POOLED elements (a quarter of
+// the output): g, the pooled output and argmax are read once, coalesced; the 2x2 windows leave as float2 row segments
+// (NCHW) and, through a shared-memory tile, as NHWC planes, four channels a store.  Bound by memory where the tensor is
+// large: 12 B read per pooled element and 16 to 32 written.  Small tensors are bound by instructions and latency: with
+// 64-bit divisions per thread, loads one behind the other and two channels a store, the two launches of a step of the small
+// CNN (batch 64, 3xTF32) took 14.7 us, now 9.0; the three of the CIFAR CNN at batch 100 28.6, now 25.
 template <bool SPLIT>
 __global__ void __launch_bounds__(256)
 pool2_bwd_planes_kernel(const float* __restrict__ g, const float* __restrict__ pooled, const int32_t* __restrict__ argmax,
                         float* __restrict__ nchw_out, float* __restrict__ hi, float* __restrict__ lo,
-                        float* __restrict__ chan_partial /*[gridDim.x][c_n] per-block channel sums, or null*/, int n_img,
-                        int c_n, int h, int w, const Bound bound) {
+                        float* __restrict__ chan_partial /*[gridDim.x][c] per-block channel sums, or null*/, const PoolGrid pg, const Bound bound) {
+  __shared__ float tile[32][129];    // [channel][q*32 + position], q = 2*dy + dx inside the window
+  __shared__ long long pix_base[32]; // linear index of each position's top-left pixel, -1 beyond the end
+  const uint32_t gp0 = blockIdx.x * 32u;
+  const int c0 = blockIdx.y * 32, w = pg.w, hw = pg.h * w, ohw = hw >> 2;
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const PoolPlace at(pg, gp0 + tx);
+  if (ty == 0) pix_base[tx] = at.live ? (long long)at.img * hw + at.corner : -1;
   NRS_PDL_PROLOGUE();
   const float scale = open_range<SPLIT>(bound);
-  __shared__ float tile[32][129];   // [channel][q*32 + position], q = 2*dy + dx inside the window
-  __shared__ long long pix_base[32]; // linear index of each position's top-left pixel, -1 beyond the end
-  const int oh = h >> 1, ow = w >> 1, ohw = oh * ow, hw = h * w;
-  const long total_pos = (long)n_img * ohw;
-  const long gp0 = (long)blockIdx.x * 32;
-  const int c0 = blockIdx.y * 32;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  {
-    const long gp = gp0 + tx;
-    const bool live = gp < total_pos;
-    const int img = live ? (int)(gp / ohw) : 0;
-    const int po = live ? (int)(gp - (long)img * ohw) : 0;
-    const int oy = po / ow, ox = po - oy * ow;
-    if (ty == 0) pix_base[tx] = live ? (long long)img * hw + (long long)(2 * oy) * w + 2 * ox : -1;
+  const size_t chan0 = (size_t)at.img * pg.c + c0 + ty;
+  float gv[4], pv[4];
+  int32_t am[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int cl = ty + 8 * i, c = c0 + cl;
-      float v0 = 0.0f, v1 = 0.0f, v2 = 0.0f, v3 = 0.0f, gv = 0.0f;
-      if (live && c < c_n) {
-        const size_t chan = (size_t)img * c_n + c;
-        const size_t o = chan * ohw + po;
-        gv = pooled[o] > 0.0f ? g[o] : 0.0f;
-        const int local = (int)((size_t)argmax[o] - chan * hw);   // winner inside the channel plane
-        const int wy = local / w, wx = local - wy * w;
-        const int q = ((wy - 2 * oy) << 1) | (wx - 2 * ox);
-        v0 = q == 0 ? gv : 0.0f; v1 = q == 1 ? gv : 0.0f; v2 = q == 2 ? gv : 0.0f; v3 = q == 3 ? gv : 0.0f;
-        if (nchw_out) {
-          float* dst = nchw_out + chan * hw + (size_t)(2 * oy) * w + 2 * ox;
-          *reinterpret_cast<float2*>(dst) = make_float2(v0, v1);
-          *reinterpret_cast<float2*>(dst + w) = make_float2(v2, v3);
-        }
-      }
-      tile[cl][tx] = v0; tile[cl][32 + tx] = v1; tile[cl][64 + tx] = v2; tile[cl][96 + tx] = v3;
-      if (chan_partial) {   // the window's four outputs sum to gv: fixed-order butterfly over the 32 positions
-        float sum = gv;
+  for (int i = 0; i < 4; ++i) {
+    const bool ok = at.live && c0 + ty + 8 * i < pg.c;
+    const size_t o = (chan0 + 8 * i) * ohw + at.po;
+    gv[i] = ok ? g[o] : 0.0f;
+    pv[i] = ok ? pooled[o] : 0.0f;
+    am[i] = ok ? argmax[o] : 0;
+  }
 #pragma unroll
-        for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
-        if (tx == 0 && c < c_n) chan_partial[(size_t)blockIdx.x * c_n + c] = sum;
-      }
+  for (int i = 0; i < 4; ++i) {
+    const int cl = ty + 8 * i;
+    const bool ok = at.live && c0 + cl < pg.c;
+    const size_t plane = (chan0 + 8 * i) * hw + at.corner;
+    const float v = pv[i] > 0.0f ? gv[i] : 0.0f;
+    const int d = (int)((size_t)am[i] - plane);   // the winner from the window's corner: 0, 1, w, w + 1
+    const int q = d >= w ? d - w + 2 : d;
+    const float v0 = ok && q == 0 ? v : 0.0f, v1 = ok && q == 1 ? v : 0.0f, v2 = ok && q == 2 ? v : 0.0f, v3 = ok && q == 3 ? v : 0.0f;
+    if (nchw_out && ok) {
+      float* dst = nchw_out + plane;
+      *reinterpret_cast<float2*>(dst) = make_float2(v0, v1);
+      *reinterpret_cast<float2*>(dst + w) = make_float2(v2, v3);
+    }
+    float* t = &tile[cl][tx];
+    t[0] = v0; t[32] = v1; t[64] = v2; t[96] = v3;
+    if (chan_partial) {   // the window's four outputs sum to v: fixed-order butterfly over the 32 positions
+      float sum = v;
+#pragma unroll
+      for (int s = 16; s > 0; s >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, s);
+      if (tx == 0 && c0 + cl < pg.c) chan_partial[(size_t)blockIdx.x * pg.c + c0 + cl] = sum;
     }
   }
   if (!hi) return;
   __syncthreads();
-  if (SPLIT) {   // a thread: two channels (c_n is a multiple of 8), a half warp a pixel's 32
-    const int cl = 2 * (threadIdx.x & 15);
-    if (c0 + cl >= c_n) return;
-#pragma unroll 4
-    for (int k = threadIdx.x >> 4; k < 128; k += 16) {
-      const int q = k >> 5, pl = k & 31;
-      const long long base = pix_base[pl];
-      if (base < 0) continue;
-      const size_t o = ((size_t)base + (size_t)(q >> 1) * w + (q & 1)) * c_n + c0 + cl;
-      __half2 hv, lv;
-      pr::split2(tile[cl][k] * scale, tile[cl + 1][k] * scale, &hv, &lv);
-      *reinterpret_cast<__half2*>(reinterpret_cast<__half*>(hi) + o) = hv;
-      *reinterpret_cast<__half2*>(reinterpret_cast<__half*>(lo) + o) = lv;
-    }
-    return;
-  }
-  // warp ty writes pixels k = ty, ty+8, ...: lane = channel
-  const int c = c0 + tx;
-  if (c >= c_n) return;
-#pragma unroll 4
-  for (int k = ty; k < 128; k += 8) {
-    const int q = k >> 5, pl = k & 31;
-    const long long base = pix_base[pl];
-    if (base < 0) continue;
-    const size_t pixel = (size_t)base + (size_t)(q >> 1) * w + (q & 1);
-    hi[pixel * c_n + c] = tc::tf32_rn(tile[tx][k]);
+  const int cq = (threadIdx.x & 7) * 4, pl = threadIdx.x >> 3;   // (the channels of a tensor with planes are a multiple of 8)
+  const long long base = pix_base[pl];
+  if (c0 + cq >= pg.c || base < 0) return;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int k = q * 32 + pl;
+    const float4 f = make_float4(tile[cq][k], tile[cq + 1][k], tile[cq + 2][k], tile[cq + 3][k]);
+    const size_t o = ((size_t)base + (size_t)(q >> 1) * w + (q & 1)) * pg.c + c0 + cq;
+    if (SPLIT) pr::put4(hi, lo, o, f, scale);
+    else *reinterpret_cast<float4*>(hi + o) = make_float4(tc::tf32_rn(f.x), tc::tf32_rn(f.y), tc::tf32_rn(f.z), tc::tf32_rn(f.w));
   }
 }
 
-
-// 2x2 / stride-2 max-pool forward over even-sized images that also writes the pooled output's
-// NHWC planes (the next convolution's operand).  Same tiling as pool2_bwd_planes_kernel: 32
-// channels x 32 consecutive pooled positions per block; the first maximum in row-major window
-// order wins and argmax is the flat input index, as in maxpool2x2_fwd_kernel.
+// 2x2 / stride-2 max-pool forward that also writes the pooled output's NHWC planes (the next convolution's operand), in
+// the same tiles; the first maximum in row-major window order wins and argmax is the flat input index, as in
+// maxpool2x2_fwd_kernel.
 template <bool SPLIT>
 __global__ void __launch_bounds__(256)
 pool2_fwd_planes_kernel(const float* __restrict__ x, float* __restrict__ y, int32_t* __restrict__ argmax,
-                        float* __restrict__ hi, float* __restrict__ lo, int n_img, int c_n, int h, int w, const Bound bound) {
-  NRS_PDL_PROLOGUE();
+                        float* __restrict__ hi, float* __restrict__ lo, const PoolGrid pg, const Bound bound) {
   __shared__ float tile[32][33];
-  const float scale = open_range<SPLIT>(bound);
-  const int oh = h >> 1, ow = w >> 1, ohw = oh * ow, hw = h * w;
-  const long total_pos = (long)n_img * ohw;
-  const long gp0 = (long)blockIdx.x * 32;
-  const int c0 = blockIdx.y * 32;
+  const uint32_t gp0 = blockIdx.x * 32u;
+  const int c0 = blockIdx.y * 32, w = pg.w, hw = pg.h * w, ohw = hw >> 2;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  {
-    const long gp = gp0 + tx;
-    const bool live = gp < total_pos;
-    const int img = live ? (int)(gp / ohw) : 0;
-    const int po = live ? (int)(gp - (long)img * ohw) : 0;
-    const int oy = po / ow, ox = po - oy * ow;
+  const PoolPlace at(pg, gp0 + tx);
+  NRS_PDL_PROLOGUE();
+  const float scale = open_range<SPLIT>(bound);
+  const size_t chan0 = (size_t)at.img * pg.c + c0 + ty;
+  float2 r0[4], r1[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int cl = ty + 8 * i, c = c0 + cl;
-      float best = 0.0f;
-      if (live && c < c_n) {
-        const size_t chan = (size_t)img * c_n + c;
-        const size_t first = chan * hw + (size_t)(2 * oy) * w + 2 * ox;
-        const float2 r0 = *reinterpret_cast<const float2*>(x + first);
-        const float2 r1 = *reinterpret_cast<const float2*>(x + first + w);
-        best = r0.x;
-        size_t bi = first;
-        if (r0.y > best) { best = r0.y; bi = first + 1; }
-        if (r1.x > best) { best = r1.x; bi = first + w; }
-        if (r1.y > best) { best = r1.y; bi = first + w + 1; }
-        y[chan * ohw + po] = best;
-        if (argmax) argmax[chan * ohw + po] = (int32_t)bi;
-      }
-      tile[cl][tx] = best;
+  for (int i = 0; i < 4; ++i) {
+    const float* s = x + (chan0 + 8 * i) * hw + at.corner;
+    const bool ok = at.live && c0 + ty + 8 * i < pg.c;
+    r0[i] = ok ? *reinterpret_cast<const float2*>(s) : make_float2(0.0f, 0.0f);
+    r1[i] = ok ? *reinterpret_cast<const float2*>(s + w) : make_float2(0.0f, 0.0f);
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const size_t first = (chan0 + 8 * i) * hw + at.corner;
+    float best = r0[i].x;
+    size_t bi = first;
+    if (r0[i].y > best) { best = r0[i].y; bi = first + 1; }
+    if (r1[i].x > best) { best = r1[i].x; bi = first + w; }
+    if (r1[i].y > best) { best = r1[i].y; bi = first + w + 1; }
+    if (at.live && c0 + ty + 8 * i < pg.c) {
+      const size_t o = (chan0 + 8 * i) * ohw + at.po;
+      y[o] = best;
+      if (argmax) argmax[o] = (int32_t)bi;
     }
+    tile[ty + 8 * i][tx] = best;
   }
   __syncthreads();
-  if (SPLIT) {   // a thread: two channels (c_n is a multiple of 8), a half warp a pixel's 32
-    const int cl = 2 * (threadIdx.x & 15);
-    if (c0 + cl >= c_n) return;
-#pragma unroll
-    for (int k = threadIdx.x >> 4; k < 32; k += 16) {
-      if (gp0 + k >= total_pos) continue;
-      const size_t o = (size_t)(gp0 + k) * c_n + c0 + cl;
-      __half2 hv, lv;
-      pr::split2(tile[cl][k] * scale, tile[cl + 1][k] * scale, &hv, &lv);
-      *reinterpret_cast<__half2*>(reinterpret_cast<__half*>(hi) + o) = hv;
-      *reinterpret_cast<__half2*>(reinterpret_cast<__half*>(lo) + o) = lv;
-    }
-    return;
-  }
-  const int c = c0 + tx;   // lane = channel: one full 128-byte line per warp store
-  if (c >= c_n) return;
-#pragma unroll
-  for (int k = ty; k < 32; k += 8) {
-    const long gp = gp0 + k;
-    if (gp >= total_pos) continue;
-    hi[(size_t)gp * c_n + c] = tc::tf32_rn(tile[tx][k]);
-  }
+  const int cq = (threadIdx.x & 7) * 4, pl = threadIdx.x >> 3;
+  if (c0 + cq >= pg.c || gp0 + pl >= pg.positions) return;
+  const float4 f = make_float4(tile[cq][pl], tile[cq + 1][pl], tile[cq + 2][pl], tile[cq + 3][pl]);
+  const size_t o = (size_t)(gp0 + pl) * pg.c + c0 + cq;
+  if (SPLIT) pr::put4(hi, lo, o, f, scale);
+  else *reinterpret_cast<float4*>(hi + o) = make_float4(tc::tf32_rn(f.x), tc::tf32_rn(f.y), tc::tf32_rn(f.z), tc::tf32_rn(f.w));
 }
 
 }  // namespace
@@ -428,16 +415,16 @@ int nrs_tc_pool2_fwd_planes(nrs_ctx* ctx, const float* x, float* y, int32_t* arg
                             int h, int w, const NrsRange* x_range) {
   if (n <= 0 || c <= 0) return NRS_OK;
   if (h % 2 != 0 || w % 2 != 0 || !hi || (reinterpret_cast<uintptr_t>(x) & 7) != 0) return NRS_ERR_UNSUPPORTED;
-  const long blocks = ((long)n * (h / 2) * (w / 2) + 31) / 32;
-  if (blocks > 2147483647L || (c + 31) / 32 > 65535) return NRS_ERR_UNSUPPORTED;
-  dim3 grid((unsigned)blocks, (unsigned)((c + 31) / 32));
+  if (h == 0 || w == 0 || !PoolGrid::fits(n, c, h, w) || (c + 31) / 32 > 65535) return NRS_ERR_UNSUPPORTED;
+  const PoolGrid pg(n, c, h, w);
+  const dim3 grid = pg.blocks();
   Bound bound{};
   if (lo) {
     const int st = open_planes(ctx, hi, x, (size_t)n * c * h * w, x_range, &bound);
     if (st != NRS_OK) return st;
-    NRS_PDL_LAUNCH((pool2_fwd_planes_kernel<true>), grid, 256, 0, ctx->stream, x, y, argmax, hi, lo, n, c, h, w, bound);
+    NRS_PDL_LAUNCH((pool2_fwd_planes_kernel<true>), grid, 256, 0, ctx->stream, x, y, argmax, hi, lo, pg, bound);
   } else {
-    NRS_PDL_LAUNCH((pool2_fwd_planes_kernel<false>), grid, 256, 0, ctx->stream, x, y, argmax, hi, nullptr, n, c, h, w, bound);
+    NRS_PDL_LAUNCH((pool2_fwd_planes_kernel<false>), grid, 256, 0, ctx->stream, x, y, argmax, hi, nullptr, pg, bound);
   }
   NRS_LAUNCHED(ctx);
   return NRS_OK;
@@ -457,10 +444,11 @@ int nrs_tc_stage_masked(nrs_ctx* ctx, int mode, const float* g, const float* y, 
     const int st = open_planes(ctx, hi, g, (size_t)n * c * oh * ow, g_range, &bound);
     if (st != NRS_OK) return st;
   }
-  if (mode == 1 && k == 2 && h % 2 == 0 && w % 2 == 0 && (long)n * (h / 2) * (w / 2) / 32 < 2147483647L) {
-    dim3 pgrid((unsigned)(((long)n * (h / 2) * (w / 2) + 31) / 32), (unsigned)((c + 31) / 32));
-    if (split) NRS_PDL_LAUNCH((pool2_bwd_planes_kernel<true>), pgrid, 256, 0, ctx->stream, g, y, argmax, nchw_out, hi, lo, chan_partial, n, c, h, w, bound);
-    else NRS_PDL_LAUNCH((pool2_bwd_planes_kernel<false>), pgrid, 256, 0, ctx->stream, g, y, argmax, nchw_out, hi, lo, chan_partial, n, c, h, w, bound);
+  if (mode == 1 && k == 2 && h % 2 == 0 && w % 2 == 0 && h > 0 && w > 0 && PoolGrid::fits(n, c, h, w)) {
+    const PoolGrid pg(n, c, h, w);
+    const dim3 pgrid = pg.blocks();
+    if (split) NRS_PDL_LAUNCH((pool2_bwd_planes_kernel<true>), pgrid, 256, 0, ctx->stream, g, y, argmax, nchw_out, hi, lo, chan_partial, pg, bound);
+    else NRS_PDL_LAUNCH((pool2_bwd_planes_kernel<false>), pgrid, 256, 0, ctx->stream, g, y, argmax, nchw_out, hi, lo, chan_partial, pg, bound);
     NRS_LAUNCHED(ctx);
     if (chan_partial && chan_partial_rows) *chan_partial_rows = (int)pgrid.x;
     return NRS_OK;
@@ -487,8 +475,8 @@ int nrs_tc_stage(nrs_ctx* ctx, const float* src, float* hi, float* lo, int rows,
     if (blocks > cap) blocks = cap;
     if (batch > 65535) return NRS_ERR_UNSUPPORTED;
     dim3 grid((unsigned)blocks, (unsigned)batch);
-    if (lo) NRS_PDL_LAUNCH((stage_rows_kernel<true>), grid, 256, 0, ctx->stream, src, hi, lo, rows, K, ldk, src_bstride, dst_bstride, bound);
-    else NRS_PDL_LAUNCH((stage_rows_kernel<false>), grid, 256, 0, ctx->stream, src, hi, nullptr, rows, K, ldk, src_bstride, dst_bstride, bound);
+    if (lo) NRS_PDL_LAUNCH((stage_rows_kernel<true>), grid, 256, 0, ctx->stream, src, hi, lo, rows, K, ldk, src_bstride, dst_bstride, NrsFastDiv(ldk / 4), bound);
+    else NRS_PDL_LAUNCH((stage_rows_kernel<false>), grid, 256, 0, ctx->stream, src, hi, nullptr, rows, K, ldk, src_bstride, dst_bstride, NrsFastDiv(ldk / 4), bound);
   } else {
     dim3 grid((unsigned)((rows + 31) / 32), (unsigned)((ldk + 31) / 32), (unsigned)batch);
     if (grid.y > 65535 || grid.z > 65535) return NRS_ERR_UNSUPPORTED;

@@ -54,7 +54,9 @@ embed_fwd_kernel(const float* __restrict__ w, const int32_t* __restrict__ idx, c
 // token, the matches are compacted IN TOKEN ORDER (warp ballots + a prefix over the warp counts) into a
 // shared list, and then thread d adds the matching gradient rows in that order — the same order of
 // additions as a serial walk over the tokens, so the result is deterministic and independent of the
-// launch shape, at a cost of tokens/256 scan steps per block instead of `tokens` per thread.
+// launch shape, at a cost of tokens/256 scan steps per block instead of `tokens` per thread.  Latency-bound: the indices of
+// a chunk and the rows of four matches are loaded together (4096 tokens x 256, vocabulary 1000, in a training step: one
+// load at a time 17.5 us, so 14; 3000 x 512 13.9 -> 9.2).
 __global__ void __launch_bounds__(256)
 embed_bwd_kernel(const float* __restrict__ g, const int32_t* __restrict__ idx, float* dw, int tokens, int dim,
                  int accumulate) {
@@ -71,9 +73,17 @@ embed_bwd_kernel(const float* __restrict__ g, const int32_t* __restrict__ idx, f
       const int nt = min(kChunk, tokens - t0);
       __syncthreads();                                    // the previous chunk's list has been consumed
       int n_match = 0;                                    // kept by every thread; the same in all of them
-      for (int sub = 0; sub < nt; sub += 256, ++step) {
-        const int t = t0 + sub + threadIdx.x;
-        const bool hit = (sub + (int)threadIdx.x) < nt && idx[t] == row;
+      bool hits[kChunk / 256];                            // (the chunk's indices are loaded together)
+#pragma unroll
+      for (int u = 0; u < kChunk / 256; ++u) {
+        const int i = 256 * u + (int)threadIdx.x;
+        hits[u] = i < nt && idx[t0 + i] == row;
+      }
+#pragma unroll
+      for (int u = 0; u < kChunk / 256; ++u, ++step) {
+        if (256 * u >= nt) break;
+        const int t = t0 + 256 * u + (int)threadIdx.x;
+        const bool hit = hits[u];
         const unsigned ballot = __ballot_sync(0xffffffffu, hit);
         if (lane == 0) s_warp[step & 1][wrp] = __popc(ballot);
         __syncthreads();   // one barrier per step: the next step writes the other buffer, and a warp can only
@@ -89,11 +99,21 @@ embed_bwd_kernel(const float* __restrict__ g, const int32_t* __restrict__ idx, f
         n_match += total;
       }
       __syncthreads();                                    // the list is complete
-      for (int m = 0; m < n_match; ++m) {
-        const float* src = g + (size_t)s_match[m] * dim + d0 + threadIdx.x;
+      for (int m = 0; m < n_match; m += 4) {              // four matches' rows under way, added in order
+        float v[4][4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
-          if (d0 + (int)threadIdx.x + k * 256 < dim) acc[k] += src[k * 256];
+        for (int u = 0; u < 4; ++u) {
+          if (m + u >= n_match) break;
+          const float* src = g + (size_t)s_match[m + u] * dim + d0 + threadIdx.x;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) v[u][k] = d0 + (int)threadIdx.x + k * 256 < dim ? src[k * 256] : 0.0f;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          if (m + u >= n_match) break;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) acc[k] += v[u][k];
+        }
       }
     }
 #pragma unroll

@@ -48,38 +48,37 @@ __device__ __forceinline__ void put4(float* hi, float* lo, size_t i, float4 v, f
   else *reinterpret_cast<float4*>(hi + i) = make_float4(tc::tf32_rn(v.x), tc::tf32_rn(v.y), tc::tf32_rn(v.z), tc::tf32_rn(v.w));
 }
 
-__device__ __forceinline__ int job_of(const WeightJob* jobs, int n_jobs, unsigned bid, unsigned WeightJob::*first) {
-  int lo = 0, hi = n_jobs - 1;   // the last one whose first block <= bid
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (jobs[mid].*first <= bid) lo = mid; else hi = mid - 1;
-  }
-  return lo;
-}
-
-constexpr int kScan = 8192;   // values per block
+constexpr int kScan = 4096;   // values per block
 inline unsigned job_scans(const WeightJob& j) { return (unsigned)(((size_t)j.rows * j.cols * j.taps + kScan - 1) / kScan); }
+
+// Both kernels last a few microseconds, most of it latency.  What a block works on is therefore one load away
+// (`job_of_block`, made with the table; a binary search over the jobs is four loads, each waiting for the one before), is
+// looked up before the wait for the kernel ahead (the tables never change), and all loads of a thread are under way
+// before the first value is used.  Measured in a training step, scan and staging together: small CNN 16 -> 11 us, language
+// model of 32 x 128 tokens 13 -> 8.
 
 // The largest magnitude of every weight (group), for its planes' exponent.  L2-bound: the optimizer has just written them.
 // A group's last block to arrive turns what all of them left in the range's scratch words into the range, and clears those.
 __global__ void __launch_bounds__(256)
-weight_scan_kernel(const WeightJob* __restrict__ jobs, int n_jobs, unsigned scan_offset) {
-  NRS_PDL_PROLOGUE();
+weight_scan_kernel(const WeightJob* __restrict__ jobs, const int* __restrict__ job_of_block, unsigned scan_offset) {
   __shared__ uint32_t part[8];
   const unsigned bid = blockIdx.x + scan_offset;
-  const WeightJob j = jobs[job_of(jobs, n_jobs, bid, &WeightJob::first_scan)];
+  const WeightJob j = jobs[job_of_block[bid]];
+  NRS_PDL_PROLOGUE();
   const size_t count = (size_t)j.rows * j.cols * j.taps, begin = (size_t)(bid - j.first_scan) * kScan;
   const int n = (int)min((size_t)kScan, count - begin);
   const float* src = j.src + begin;
   uint32_t top = 0;
   if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+    float4 v[kScan / 1024];
 #pragma unroll
     for (int u = 0; u < kScan / 1024; ++u) {
       const int i = 4 * (int)threadIdx.x + 1024 * u;
-      if (i + 3 < n) top = pr::seen4(top, *reinterpret_cast<const float4*>(src + i));
-      else
-        for (int e = i; e < n; ++e) top = pr::seen(top, src[e]);
+      v[u] = i + 3 < n ? *reinterpret_cast<const float4*>(src + i) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
+    if ((n & 3) != 0 && threadIdx.x < (unsigned)(n & 3)) top = pr::seen(top, src[(n & ~3) + (int)threadIdx.x]);
+#pragma unroll
+    for (int u = 0; u < kScan / 1024; ++u) top = pr::seen4(top, v[u]);
   } else {
     for (int i = threadIdx.x; i < n; i += 256) top = pr::seen(top, src[i]);
   }
@@ -102,12 +101,12 @@ weight_scan_kernel(const WeightJob* __restrict__ jobs, int n_jobs, unsigned scan
 // runs of whole sectors and turns it in shared memory.
 template <bool SPLIT>
 __global__ void __launch_bounds__(256)
-weight_stage_batch_kernel(const WeightJob* __restrict__ jobs, int n_jobs, unsigned block_offset) {
-  NRS_PDL_PROLOGUE();
+weight_stage_batch_kernel(const WeightJob* __restrict__ jobs, const int* __restrict__ job_of_block, unsigned block_offset) {
   constexpr int kPitch = kConvCi * kConvTaps + 1;
   __shared__ float tile[kConvCo * kPitch > kTile * (kTile + 1) ? kConvCo * kPitch : kTile * (kTile + 1)];
   const unsigned bid = blockIdx.x + block_offset;
-  const WeightJob j = jobs[job_of(jobs, n_jobs, bid, &WeightJob::first_block)];
+  const WeightJob j = jobs[job_of_block[bid]];
+  NRS_PDL_PROLOGUE();
   const float scale = SPLIT ? pr::scale_of(j.range->bound) : 1.0f;
   const int blk = (int)(bid - j.first_block);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -116,18 +115,22 @@ weight_stage_batch_kernel(const WeightJob* __restrict__ jobs, int n_jobs, unsign
     const int r0 = blk / tiles_c * kTile, c0 = (blk % tiles_c) * kTile;
     const int ld_b = ceil32(j.cols), ld_a = ceil32(j.rows);
     const int cq = (threadIdx.x & 15) * 4, c = c0 + cq;
+    float4 v[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int r = r0 + (threadIdx.x >> 4) + 16 * i;
+      const float* s = j.src + (size_t)r * j.cols + c;
+      v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (r >= j.rows) continue;
+      if (j.vec && c < j.cols) v[i] = *reinterpret_cast<const float4*>(s);
+      else if (!j.vec) v[i] = make_float4(c < j.cols ? s[0] : 0.f, c + 1 < j.cols ? s[1] : 0.f, c + 2 < j.cols ? s[2] : 0.f, c + 3 < j.cols ? s[3] : 0.f);
+    }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int rr = (threadIdx.x >> 4) + 16 * i, r = r0 + rr;
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (r < j.rows) {
-        const float* s = j.src + (size_t)r * j.cols + c;
-        if (j.vec && c < j.cols) v = *reinterpret_cast<const float4*>(s);
-        else if (!j.vec) v = make_float4(c < j.cols ? s[0] : 0.f, c + 1 < j.cols ? s[1] : 0.f, c + 2 < j.cols ? s[2] : 0.f, c + 3 < j.cols ? s[3] : 0.f);
-        if (j.b_hi && c < ld_b) put4<SPLIT>(j.b_hi, j.b_lo, (size_t)r * ld_b + c, v, scale);
-      }
+      if (j.b_hi && r < j.rows && c < ld_b) put4<SPLIT>(j.b_hi, j.b_lo, (size_t)r * ld_b + c, v[i], scale);
       float* t = tile + rr * (kTile + 1) + cq;
-      t[0] = v.x; t[1] = v.y; t[2] = v.z; t[3] = v.w;
+      t[0] = v[i].x; t[1] = v[i].y; t[2] = v[i].z; t[3] = v[i].w;
     }
     if (!j.a_hi) return;
     __syncthreads();
@@ -145,23 +148,29 @@ weight_stage_batch_kernel(const WeightJob* __restrict__ jobs, int n_jobs, unsign
   const int ci0 = blk % tiles_i * kConvCi, co0 = blk / tiles_i % tiles_o * kConvCo, t0 = blk / tiles_i / tiles_o * kConvTaps;
   const int nt = min(kConvTaps, j.taps - t0), nci = min(kConvCi, j.cols - ci0), nco = min(kConvCo, j.rows - co0);
   // tile[co][ci * nt + tap], zeros beyond the channels; nearly always nt == taps, and a row of it is one run of memory
+  float v[kConvCo / 8][kConvTaps];
 #pragma unroll
   for (int oo = 0; oo < kConvCo / 8; ++oo) {
     const int o = warp + 8 * oo;
     const float* s = j.src + ((size_t)(co0 + o) * j.cols + ci0) * j.taps + t0;
-    float* t = tile + o * kPitch;
 #pragma unroll
-    for (int u = 0; u < kConvTaps; ++u) {   // kConvCi values a step, so that all loads of a row are under way together
+    for (int u = 0; u < kConvTaps; ++u) {   // kConvCi values a step
       const int e = lane + 32 * u;
-      if (u >= nt) break;
+      v[oo][u] = 0.0f;
+      if (u >= nt || o >= nco) continue;
       if (nt == j.taps) {
-        t[e] = o < nco && e < nci * nt ? s[e] : 0.0f;
+        if (e < nci * nt) v[oo][u] = s[e];
       } else {
         const int ci = e / nt;
-        t[e] = o < nco && ci < nci ? s[(size_t)ci * j.taps + (e - ci * nt)] : 0.0f;
+        if (ci < nci) v[oo][u] = s[(size_t)ci * j.taps + (e - ci * nt)];
       }
     }
   }
+#pragma unroll
+  for (int oo = 0; oo < kConvCo / 8; ++oo)
+#pragma unroll
+    for (int u = 0; u < kConvTaps; ++u)
+      if (u < nt) tile[(warp + 8 * oo) * kPitch + lane + 32 * u] = v[oo][u];
   __syncthreads();
   if (j.a_hi) {
     const int ld = ceil32(j.cols);
@@ -254,9 +263,18 @@ int nrs_weight_set_build(nrs_ctx* ctx, const NrsWeightDesc* descs, int count) {
     ws.job_src.push_back(j.src);
     ws.job_first.push_back(j.first_block);
   }
-  cudaError_t e = cudaMalloc(&ws.jobs_dev, jobs.size() * sizeof(WeightJob));
-  if (e == cudaSuccess) e = cudaMemcpyAsync(ws.jobs_dev, jobs.data(), jobs.size() * sizeof(WeightJob), cudaMemcpyHostToDevice, ctx->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);   // `jobs` is a local
+  std::vector<int> job_of_block, job_of_scan;
+  for (size_t i = 0; i < jobs.size(); ++i) {
+    job_of_block.insert(job_of_block.end(), job_blocks(jobs[i]), (int)i);
+    job_of_scan.insert(job_of_scan.end(), job_scans(jobs[i]), (int)i);
+  }
+  const size_t jobs_bytes = jobs.size() * sizeof(WeightJob);
+  cudaError_t e = cudaMalloc(&ws.jobs_dev, jobs_bytes + (block + scan) * sizeof(int));
+  if (e == cudaSuccess) e = cudaMemcpyAsync(ws.jobs_dev, jobs.data(), jobs_bytes, cudaMemcpyHostToDevice, ctx->stream);
+  int* maps = (int*)((uint8_t*)ws.jobs_dev + jobs_bytes);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(maps, job_of_block.data(), block * sizeof(int), cudaMemcpyHostToDevice, ctx->stream);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(maps + block, job_of_scan.data(), scan * sizeof(int), cudaMemcpyHostToDevice, ctx->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);   // the sources are locals
   if (e != cudaSuccess) {
     (void)cudaGetLastError();
     nrs_weight_set_clear(ctx);
@@ -278,12 +296,13 @@ static int refresh_jobs(nrs_ctx* ctx, int first, int last) {
   const unsigned block = ws.job_first[first], blocks = ws.job_first[last] - block, scan = ws.job_scan[first], scans = ws.job_scan[last] - scan;
   if (blocks == 0) return NRS_OK;
   const WeightJob* jobs = (const WeightJob*)ws.jobs_dev;
+  const int* job_of_block = (const int*)(jobs + ws.n_jobs);
   if (ws.split) {
-    NRS_PDL_LAUNCH(weight_scan_kernel, scans, 256, 0, ctx->stream, jobs, ws.n_jobs, scan);
+    NRS_PDL_LAUNCH(weight_scan_kernel, scans, 256, 0, ctx->stream, jobs, job_of_block + ws.job_first[ws.n_jobs], scan);
     NRS_LAUNCHED(ctx);
-    NRS_PDL_LAUNCH((weight_stage_batch_kernel<true>), blocks, 256, 0, ctx->stream, jobs, ws.n_jobs, block);
+    NRS_PDL_LAUNCH((weight_stage_batch_kernel<true>), blocks, 256, 0, ctx->stream, jobs, job_of_block, block);
   } else {
-    NRS_PDL_LAUNCH((weight_stage_batch_kernel<false>), blocks, 256, 0, ctx->stream, jobs, ws.n_jobs, block);
+    NRS_PDL_LAUNCH((weight_stage_batch_kernel<false>), blocks, 256, 0, ctx->stream, jobs, job_of_block, block);
   }
   NRS_LAUNCHED(ctx);
   return NRS_OK;
