@@ -26,8 +26,6 @@ template <bool SPLIT>
 __global__ void __launch_bounds__(256)
 patch_planes_kernel(const float* __restrict__ x, float* __restrict__ hi, float* __restrict__ lo, const NrsConvGeom g, int kh,
                     int kw, const NrsFastDiv div_quads, uint32_t total /*pixels * (row length / 4)*/, int scan_n, NrsRange* range) {
-  NRS_PDL_PROLOGUE();
-  const float scale = SPLIT ? pr::open_range(scan_n > 0 ? nullptr : &range->top, x, scan_n, range) : 1.0f;
   __shared__ int off[kMaxPatch];        // offset of patch value k from the patch's origin
   __shared__ short2 tap[kMaxPatch];     // its (row, column) inside the window
   const int K = g.ci * kh * kw;
@@ -37,6 +35,8 @@ patch_planes_kernel(const float* __restrict__ x, float* __restrict__ hi, float* 
     tap[k] = make_short2((short)i, (short)j);
   }
   __syncthreads();
+  NRS_PDL_PROLOGUE();   // (the tables are made ahead of the wait)
+  const float scale = SPLIT ? pr::open_range(scan_n > 0 ? nullptr : &range->top, x, scan_n, range) : 1.0f;
   const int ld = nrs_plane_ld(K);
   const uint32_t stride = gridDim.x * blockDim.x;
   for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += stride) {

@@ -178,7 +178,7 @@ __global__ void colsum_fold_kernel(const float* __restrict__ partial, float* __r
 // fixed order, so the result is run-to-run deterministic.
 __global__ void __launch_bounds__(256)
 chansum_kernel(const float* __restrict__ g, float* __restrict__ out, int n, int c, int plane, int splits,
-               int accumulate, float* __restrict__ partial) {
+               int accumulate, float* partial, unsigned* tickets) {
   NRS_PDL_PROLOGUE();
   __shared__ float sm[8];
   const int ch = blockIdx.x, split = blockIdx.y;
@@ -218,6 +218,23 @@ chansum_kernel(const float* __restrict__ g, float* __restrict__ out, int n, int 
     if (splits > 1) partial[(size_t)split * c + ch] = t;
     else out[ch] = accumulate ? out[ch] + t : t;
   }
+  // The channel's last block to arrive adds the splits (in an order that does not depend on which block that is): a launch
+  // and some 3 us less than a second pass.
+  if (splits == 1 || !tickets || wrp != 0) return;
+  bool last = false;
+  if (lane == 0) {
+    __threadfence();
+    last = atomicAdd(&tickets[ch], 1u) == (unsigned)splits - 1;
+    __threadfence();
+  }
+  if (!__shfl_sync(0xffffffffu, last, 0)) return;
+  float t = 0.0f;
+  for (int z = lane; z < splits; z += 32) t += __ldcg(partial + (size_t)z * c + ch);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  if (lane != 0) return;
+  out[ch] = accumulate ? out[ch] + t : t;
+  tickets[ch] = 0;
 }
 
 // Batched transpose through a padded 32x32 shared tile: coalesced both ways.
@@ -357,9 +374,15 @@ int nrs_channel_sum(nrs_ctx* ctx, const float* g, float* out, int n, int c, int 
     if (st != NRS_OK) return st;
     partial = (float*)ws;
   }
-  NRS_PDL_LAUNCH(chansum_kernel, dim3(c, splits), 256, 0, ctx->stream, g, out, n, c, plane, splits, accumulate, partial);
+  unsigned* tickets = nullptr;
+  if (splits > 1 && c + 1 <= kNrsFoldTickets) {
+    const int st = nrs_fold_ticket(ctx, &tickets);
+    if (st != NRS_OK) return st;
+    tickets += 1;   // slot 0 belongs to the single-counter users
+  }
+  NRS_PDL_LAUNCH(chansum_kernel, dim3(c, splits), 256, 0, ctx->stream, g, out, n, c, plane, splits, accumulate, partial, tickets);
   NRS_LAUNCHED(ctx);
-  if (splits > 1) {
+  if (splits > 1 && !tickets) {
     NRS_PDL_LAUNCH(colsum_fold_kernel, nrs_blocks(c, 256), 256, 0, ctx->stream, partial, out, c, splits, accumulate);
     NRS_LAUNCHED(ctx);
   }

@@ -116,8 +116,16 @@ __device__ __forceinline__ uint32_t scan(const float* __restrict__ src, int n) {
   uint32_t top = 0;
   const int head = min(n, (int)(((16 - (reinterpret_cast<uintptr_t>(src) & 15)) & 15) / 4)), quads = (n - head) / 4;
   const float4* body = reinterpret_cast<const float4*>(src + head);
-#pragma unroll 4
-  for (int i = threadIdx.x; i < quads; i += blockDim.x) top = seen4(top, body[i]);
+  for (int i = threadIdx.x; i < quads; i += 8 * blockDim.x) {   // eight loads under way: latency is all there is here
+    float v[32];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int at = i + u * (int)blockDim.x;
+      const float4 q = at < quads ? body[at] : make_float4(0.f, 0.f, 0.f, 0.f);
+      v[4 * u] = q.x; v[4 * u + 1] = q.y; v[4 * u + 2] = q.z; v[4 * u + 3] = q.w;
+    }
+    top = seen_all(top, v);
+  }
   if ((int)threadIdx.x < head) top = seen(top, src[threadIdx.x]);
   const int rest = head + 4 * quads + (int)threadIdx.x;
   if (rest < n) top = seen(top, src[rest]);   // at most 3

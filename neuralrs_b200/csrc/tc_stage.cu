@@ -131,18 +131,18 @@ template <bool SPLIT, bool SUMS>
 __global__ void __launch_bounds__(256)
 stage_image_kernel(const float* __restrict__ src, float* __restrict__ hi, float* __restrict__ lo, float* __restrict__ chan_partial, const img::Grid g,
                    const Bound bound) {
-  NRS_PDL_PROLOGUE();
   __shared__ img::Tile tile;
-  const float scale = open_range<SPLIT>(bound);
   const uint32_t p0 = blockIdx.x * img::kTilePx;
   const int c0 = blockIdx.y * img::kTileCh, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const img::Pixels px(g, p0);
+  NRS_PDL_PROLOGUE();
   float v[16];
 #pragma unroll
   for (int i = 0; i < 16; ++i) {
     const int c = c0 + warp + 8 * (i >> 2);
     v[i] = (c < g.c && px.live[i & 3]) ? src[px.base + (px.at[i & 3] + (uint32_t)c * g.hw)] : 0.0f;
   }
+  const float scale = open_range<SPLIT>(bound);   // (its loads behind those)
 #pragma unroll
   for (int i = 0; i < 16; ++i) tile[warp + 8 * (i >> 2)][(i & 3) * 32 + lane] = v[i];
   if (SUMS) {
@@ -163,18 +163,26 @@ template <bool SPLIT>
 __global__ void __launch_bounds__(256)
 stage_conv_weight_kernel(const float* __restrict__ w, float* __restrict__ hi, float* __restrict__ lo, int co_n, int ci_n,
                          int kh, int kw, int for_dgrad, const Bound bound) {
-  NRS_PDL_PROLOGUE();
-  const float scale = open_range<SPLIT>(bound);
   const int taps = kh * kw, rows = for_dgrad ? ci_n : co_n, inner = for_dgrad ? co_n : ci_n, ld = (inner + 31) / 32 * 32;
   const size_t total = (size_t)rows * ld * taps;
   const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= total) return;
   // idx enumerates the OUTPUT [row][t*ld + k] so writes are coalesced.
-  const int k = (int)(idx % ld);
-  const int t = (int)((idx / ld) % taps);
-  const int row = (int)(idx / ((size_t)ld * taps));
+  size_t above;   // row * taps + t
+  int row, t;
+  if (total < (size_t)1 << 31) {
+    above = (uint32_t)idx / (uint32_t)ld;
+    row = (int)((uint32_t)above / (uint32_t)taps);
+  } else {
+    above = idx / ld;
+    row = (int)(above / taps);
+  }
+  const int k = (int)(idx - above * ld);
+  t = (int)(above - (size_t)row * taps);
   const int co = for_dgrad ? k : row, ci = for_dgrad ? row : k;
-  const float v = k < inner ? w[((size_t)co * ci_n + ci) * taps + t] : 0.0f;
+  NRS_PDL_PROLOGUE();
+  const float v = idx < total && k < inner ? w[((size_t)co * ci_n + ci) * taps + t] : 0.0f;
+  const float scale = open_range<SPLIT>(bound);   // (its loads behind that one)
+  if (idx >= total) return;
   if (SPLIT) pr::put(hi, lo, idx, v, scale);
   else hi[idx] = tc::tf32_rn(v);
 }
@@ -273,7 +281,6 @@ pool2_bwd_planes_kernel(const float* __restrict__ g, const float* __restrict__ p
   const PoolPlace at(pg, gp0 + tx);
   if (ty == 0) pix_base[tx] = at.live ? (long long)at.img * hw + at.corner : -1;
   NRS_PDL_PROLOGUE();
-  const float scale = open_range<SPLIT>(bound);
   const size_t chan0 = (size_t)at.img * pg.c + c0 + ty;
   float gv[4], pv[4];
   int32_t am[4];
@@ -285,6 +292,7 @@ pool2_bwd_planes_kernel(const float* __restrict__ g, const float* __restrict__ p
     pv[i] = ok ? pooled[o] : 0.0f;
     am[i] = ok ? argmax[o] : 0;
   }
+  const float scale = open_range<SPLIT>(bound);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int cl = ty + 8 * i;
@@ -336,7 +344,6 @@ pool2_fwd_planes_kernel(const float* __restrict__ x, float* __restrict__ y, int3
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const PoolPlace at(pg, gp0 + tx);
   NRS_PDL_PROLOGUE();
-  const float scale = open_range<SPLIT>(bound);
   const size_t chan0 = (size_t)at.img * pg.c + c0 + ty;
   float2 r0[4], r1[4];
 #pragma unroll
@@ -346,6 +353,7 @@ pool2_fwd_planes_kernel(const float* __restrict__ x, float* __restrict__ y, int3
     r0[i] = ok ? *reinterpret_cast<const float2*>(s) : make_float2(0.0f, 0.0f);
     r1[i] = ok ? *reinterpret_cast<const float2*>(s + w) : make_float2(0.0f, 0.0f);
   }
+  const float scale = open_range<SPLIT>(bound);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const size_t first = (chan0 + 8 * i) * hw + at.corner;
