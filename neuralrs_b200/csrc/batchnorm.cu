@@ -97,28 +97,42 @@ bn_pair_planes_kernel(const float* __restrict__ a, const float* __restrict__ b, 
   float s = 0.0f, q = 0.0f, s1 = 0.0f, q1 = 0.0f;
   const int per = vec ? hw / 4 : hw;                       // items per plane
   const int items = max(n1 - n0, 0) * per;               // n * hw < 2^31 is checked on the host
+  if (vec) {
+    constexpr int kDeep = 4;   // float4s of each tensor under way per thread, in the last round too
+    for (int j = threadIdx.x; j < items; j += kDeep * kThreads) {
+      float4 fa[kDeep], fb[kDeep];
+#pragma unroll
+      for (int u = 0; u < kDeep; ++u) {
+        const int at = j + u * kThreads;
+        const int di = (int)div_per.div((uint32_t)at), i = at - di * per;
+        const size_t base = ((size_t)(n0 + di) * c + ch) * hw;
+        if (at < items) {
+          fa[u] = reinterpret_cast<const float4*>(a + base)[i];
+          if (!FWD) fb[u] = reinterpret_cast<const float4*>(b + base)[i];
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < kDeep; ++u) {
+        if (j + u * kThreads >= items) break;
+        float4 va = fa[u], vb = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (!FWD) vb = make_float4((fb[u].x - mu) * is, (fb[u].y - mu) * is, (fb[u].z - mu) * is, (fb[u].w - mu) * is);
+        if (RELU) {
+          va.x = fmaf(ga, vb.x, be) > 0.0f ? va.x : 0.0f;
+          va.y = fmaf(ga, vb.y, be) > 0.0f ? va.y : 0.0f;
+          va.z = fmaf(ga, vb.z, be) > 0.0f ? va.z : 0.0f;
+          va.w = fmaf(ga, vb.w, be) > 0.0f ? va.w : 0.0f;
+        }
+        contribute<FWD>(va.x, vb.x, k, s, q);
+        contribute<FWD>(va.y, vb.y, k, s1, q1);
+        contribute<FWD>(va.z, vb.z, k, s, q);
+        contribute<FWD>(va.w, vb.w, k, s1, q1);
+      }
+    }
+  } else {
 #pragma unroll 2
-  for (int j = threadIdx.x; j < items; j += kThreads) {
-    const int di = (int)div_per.div((uint32_t)j), i = j - di * per;
-    const size_t base = ((size_t)(n0 + di) * c + ch) * hw;
-    if (vec) {
-      float4 va = reinterpret_cast<const float4*>(a + base)[i];
-      float4 vb = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (!FWD) {
-        vb = reinterpret_cast<const float4*>(b + base)[i];
-        vb = make_float4((vb.x - mu) * is, (vb.y - mu) * is, (vb.z - mu) * is, (vb.w - mu) * is);
-      }
-      if (RELU) {
-        va.x = fmaf(ga, vb.x, be) > 0.0f ? va.x : 0.0f;
-        va.y = fmaf(ga, vb.y, be) > 0.0f ? va.y : 0.0f;
-        va.z = fmaf(ga, vb.z, be) > 0.0f ? va.z : 0.0f;
-        va.w = fmaf(ga, vb.w, be) > 0.0f ? va.w : 0.0f;
-      }
-      contribute<FWD>(va.x, vb.x, k, s, q);
-      contribute<FWD>(va.y, vb.y, k, s1, q1);
-      contribute<FWD>(va.z, vb.z, k, s, q);
-      contribute<FWD>(va.w, vb.w, k, s1, q1);
-    } else {
+    for (int j = threadIdx.x; j < items; j += kThreads) {
+      const int di = (int)div_per.div((uint32_t)j), i = j - di * per;
+      const size_t base = ((size_t)(n0 + di) * c + ch) * hw;
       const float vb = FWD ? 0.0f : (b[base + i] - mu) * is;
       float va = a[base + i];
       if (RELU) va = fmaf(ga, vb, be) > 0.0f ? va : 0.0f;

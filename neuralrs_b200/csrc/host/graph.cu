@@ -100,6 +100,8 @@ NodeP node_new(nrs_ctx* ctx, const float* host, const std::vector<size_t>& shape
   return n;
 }
 
+GradSums::~GradSums() { nrs_free(ctx, partial); }
+
 // The node whose gradient buffer `n` uses (reshape/flatten results alias their input).
 static Node* grad_root(Node* n) {
   while (n->view_of) n = n->view_of.get();
@@ -114,6 +116,7 @@ struct GradTarget {
 static GradTarget grad_target(const NodeP& n) {
   Node* r = grad_root(n.get());
   r->gtop.reset();
+  r->gsums.reset();
   if (!r->grad) r->grad = dalloc(r->ctx, r->len());
   check(r->ctx, nrs_folds_settle(r->ctx, r->grad, r->len()));   // an earlier share may still wait in the fold queue
   if (r->gz_valid) {   // another share arrives: what was derived from the first one is stale
@@ -1059,8 +1062,12 @@ static NodeP layernorm_impl(const NodeP& x, const NodeP& residual, const NodeP& 
       float* hi = mine ? rb->gplanes_hi : nrs_dplane(ctx, self->len(), split);
       float* lo = mine ? rb->gplanes_lo : (split ? nrs_dplane(ctx, self->len(), true) : nullptr);
       int emitted = 0;
+      std::shared_ptr<GradSums> sums;
+      if (dg && rb->grad_sums_wanted) sums = std::make_shared<GradSums>(ctx, dalloc(ctx, (size_t)nrs_layernorm_sum_rows(ctx) * f), f);
       const int st = nrs_layernorm_bwd_planes(ctx, g, xhat, istd, gamma->data, da, db, dg, dbt, rows, f, acc_a, acc_b, acc_p, hi, lo,
-                                              &emitted, range_in(g_top), range_in(istd_top));
+                                              &emitted, range_in(g_top), range_in(istd_top), sums ? sums->partial : nullptr,
+                                              sums ? &sums->rows : nullptr);
+      if (st == NRS_OK && sums && sums->rows > 0) rb->gsums = std::move(sums);
       if (st == NRS_OK && emitted) {
         if (!mine) {
           rb->gplanes_hi = hi;
@@ -1334,6 +1341,7 @@ NodeP linear_act(const NodeP& x, const NodeP& w, const NodeP& b, int act, bool e
     check(ctx, st);
   }
   Node* self = out.get();
+  out->grad_sums_wanted = act == NRS_ACT_NONE && b->requires_grad;
   if (act != NRS_ACT_NONE && tensor_cores && n % 8 == 0 && w->requires_grad && b->requires_grad && nrs_gemm_tn_reads_planes(k, n)) {
     out->fold_act = act;
     out->fold_src = act == NRS_ACT_GELU ? pre : out->data;
@@ -1366,6 +1374,8 @@ NodeP linear_act(const NodeP& x, const NodeP& w, const NodeP& b, int act, bool e
     if (b->requires_grad) {
       GradTarget t = grad_target(b);
       if (from_planes) check(ctx, nrs_fold_columns(ctx, self->gchan_partial, t.ptr, self->gchan_rows, n, n, t.accumulate));
+      else if (act == NRS_ACT_NONE && self->gsums && self->gsums->cols == n)   // whoever wrote the gradient summed its columns
+        check(ctx, nrs_fold_columns(ctx, self->gsums->partial, t.ptr, self->gsums->rows, n, n, t.accumulate));
       else check(ctx, nrs_sum_axis0(ctx, dz, t.ptr, m, n, t.accumulate));
     }
     if (x->requires_grad) linear_input_grad(ctx, x, w, dz, m, k, n);

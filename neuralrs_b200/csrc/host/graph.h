@@ -45,6 +45,17 @@ struct TopRef {
 };
 using TopP = std::shared_ptr<TopRef>;
 
+// Partial column sums [rows][cols] of a gradient.
+struct GradSums {
+  nrs_ctx* ctx;
+  float* partial;
+  int rows, cols;
+  GradSums(nrs_ctx* c, float* p, int n) : ctx(c), partial(p), rows(0), cols(n) {}
+  GradSums(const GradSums&) = delete;
+  GradSums& operator=(const GradSums&) = delete;
+  ~GradSums();
+};
+
 // Node of the define-by-run graph (src/autograd/node.rs:38-53).
 struct Node {
   nrs_ctx* ctx = nullptr;
@@ -83,6 +94,10 @@ struct Node {
   float* gplanes_lo = nullptr;
   // With a premasked gradient: per-block channel sums of it ([rows][channels]), which the
   // convolution's bias gradient folds instead of summing the whole NCHW gradient again.
+  // Column sums of the whole gradient, left by the kernel that wrote it where the reader wants them (a linear layer's bias
+  // gradient); dropped with gtop when another share arrives.
+  bool grad_sums_wanted = false;
+  std::shared_ptr<GradSums> gsums;
   float* gchan_partial = nullptr;
   int gchan_rows = 0;
 

@@ -328,7 +328,10 @@ extern "C" int nrs_layernorm_fwd_planes(nrs_ctx* ctx, const float* a, const floa
 extern "C" int nrs_layernorm_bwd_planes(nrs_ctx* ctx, const float* g, const float* xhat, const float* istd, const float* gamma,
                                         float* da, float* db, float* dgamma, float* dbeta, int rows, int f, int accumulate_da,
                                         int accumulate_db, int accumulate_params, float* d_hi, float* d_lo, int* emitted,
-                                        const NrsRange* range_g, const NrsRange* range_istd);
+                                        const NrsRange* range_g, const NrsRange* range_istd,
+                                        float* sums /*[nrs_layernorm_sum_rows][f] partial column sums of the gradient, or null*/,
+                                        int* sums_rows /*how many rows of it were written; 0: none*/);
+static inline int nrs_layernorm_sum_rows(const nrs_ctx* ctx) { return 4 * ctx->sm_count; }
 // Operand planes of a batch of [rows][K] matrices (tc_stage.cu); see tc_mainloop.cuh for the layouts.  3xTF32: the range
 // of `hi` is renewed and measured, in the same launch for small tensors, unless the caller has one: `measured` becomes the
 // planes' own, `known` bounds the source's values (NrsRange::top).
