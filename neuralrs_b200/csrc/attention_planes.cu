@@ -52,6 +52,7 @@ struct HeadPolicy {
   static constexpr bool kCanEmit = false, kMaySplit = false;
   static constexpr bool kAMnMajor = AMN, kBMnMajor = BMN;
   static constexpr int kEpiWarps = 16, kTeamWarps = 4;
+  static constexpr bool kConv = false;
   static constexpr bool kSlab = false;
   int order() const { return causal; }   // the same numbers
   __device__ __forceinline__ float out_bound(float, float, int) const {

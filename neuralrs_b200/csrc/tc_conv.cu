@@ -36,6 +36,7 @@ namespace {
 
 template <int EPI, bool SLAB>
 struct ConvPolicyOf {
+  static constexpr bool kConv = true;
   static constexpr bool kSlab = SLAB;
   // A tile's pixels in the order of its box: (x, y, image), in slabs (x, image, y), so that a row of all its images is one
   // stretch of the slab and the next vertical tap starts Wt * Nt pixels on.

@@ -39,6 +39,7 @@ struct GemmPolicy {
   // The epilogue is latency (TMEM, loads, GELU at about 66 instructions a value): four warps per lane quarter.  With two,
   // a 128 x 128 tile with GELU and three outputs took 27 thousand clocks, twice its main loop at K = 512.
   static constexpr int kEpiWarps = 16, kTeamWarps = 4;
+  static constexpr bool kConv = false;
   static constexpr bool kSlab = false;
   int order() const { return tc::kRaster; }
 

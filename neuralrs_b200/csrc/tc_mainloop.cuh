@@ -66,6 +66,10 @@ namespace tc {
 
 constexpr int BM = 128, BK = 32;   // 32 values: 128 bytes of f32, 64 of f16: one swizzle row
 constexpr int kMaxChainK = 4096;   // longest single accumulation chain in 3xTF32 mode
+// The same of a convolution with few pixels (at most half a wave of 128-column tiles).  With TF32 pairs such a product was
+// split over the CTAs there are, down to chains of 512; f16 pairs err a third as much per value, are fast enough in narrow
+// tiles not to be split, and are to err no more.
+constexpr int kFewChainK = 1536;
 constexpr int kMaxChainPairs = 8192;   // the same of weight gradients: at this length f16 pairs err as much as TF32 pairs did at half
 constexpr int kGroupM = 16;        // row tiles per raster group (see TileMap)
 constexpr int kSlabRows = 192;     // most pixels of a slab of A (see Policy::kSlab)
@@ -702,9 +706,10 @@ tc_splitk_reduce_kernel(const Policy pol, const SplitInfo sp, NrsRange* __restri
   }
 }
 
-// Chooses the K-split: enough CTAs to fill the GPU, and no accumulation chain longer than kMaxChainK elements when
+// Chooses the K-split: enough CTAs to fill the GPU, and no accumulation chain longer than kMaxChainK (kFewChainK) values when
 // `limit_chain` (chunks where the tiles fill the GPU anyway).
-inline void plan_split(const nrs_ctx* ctx, long tiles, long out_elems, int kb_total, int kw, bool limit_chain, SplitInfo* sp) {
+inline void plan_split(const nrs_ctx* ctx, long tiles, long out_elems, int kb_total, int kw, bool limit_chain, bool conv, SplitInfo* sp) {
+  const int longest = conv && 2 * out_elems <= (long)ctx->sm_count * BM * 128 ? kFewChainK : kMaxChainK;
   int s = 1;
   // (More than half a wave of tiles runs unsplit: the second pass over the partial tiles costs more
   // than the idle SMs.)
@@ -716,7 +721,7 @@ inline void plan_split(const nrs_ctx* ctx, long tiles, long out_elems, int kb_to
     if (s > kb_total / shortest) s = kb_total / shortest;
     if (s < 1) s = 1;
   }
-  const int need = limit_chain ? (int)(((long)kb_total * kw + kMaxChainK - 1) / kMaxChainK) : 1;
+  const int need = limit_chain ? (int)(((long)kb_total * kw + longest - 1) / longest) : 1;
   const bool in_chunks = s == 1 && need > 1;
   if (s < need) s = need;
   int per = (kb_total + s - 1) / s;
@@ -750,7 +755,7 @@ inline TilePlan plan_tile(const nrs_ctx* ctx, long tiles_m, int n, long batches,
     if (c.bn > limit || (c.bn > 32 && c.bn / 2 >= n)) continue;   // half of the tile or more would be padding
     const long tiles_n = (n + c.bn - 1) / c.bn;
     SplitInfo sp{};
-    plan_split(ctx, tiles_m * tiles_n * batches, tiles_m * BM * n * batches, kblocks, BK, split_planes, &sp);
+    plan_split(ctx, tiles_m * tiles_n * batches, tiles_m * BM * n * batches, kblocks, BK, split_planes, conv, &sp);
     const int splits = sp.splits, per = sp.kb_per_split * sp.chunks;
     const long units = (c.pair ? (tiles_m + 1) / 2 : tiles_m) * tiles_n * batches * splits, slots = ctx->sm_count / (c.pair ? 2 : 1);
     const double rounds = (double)((units + slots - 1) / slots);
@@ -803,7 +808,7 @@ int launch(nrs_ctx* ctx, const CUtensorMap& ta_hi, const CUtensorMap& ta_lo, con
   const int tiles_n = (n_total + BN - 1) / BN;
   SplitInfo sp{};
   if (Policy::kMaySplit) {
-    plan_split(ctx, (long)tiles_m * tiles_n * batches, (long)tiles_m * BM * n_total * batches, kb_total, k_per_block, NPLANES == 2, &sp);
+    plan_split(ctx, (long)tiles_m * tiles_n * batches, (long)tiles_m * BM * n_total * batches, kb_total, k_per_block, NPLANES == 2, Policy::kConv, &sp);
   } else {   // tiles whose K ranges differ
     sp.splits = sp.chunks = 1;
     sp.kb_per_split = kb_total;
