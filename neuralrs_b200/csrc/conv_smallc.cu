@@ -21,14 +21,14 @@ namespace {
 
 constexpr int kTileLd = 36;   // floats per pixel row of the plane-emission tile (16-byte aligned, spreads banks)
 
-// EMIT: also write the result as NHWC TF32 planes (hi, and lo when non-null) for a tensor-core
+// EMIT: also write the result as NHWC TF32 planes for a tensor-core
 // convolution that reads it next.  Each warp (32 consecutive pixels) passes 32 channels at a
 // time through a shared-memory tile so that every plane store covers four full 128-byte lines.
 template <int CI, int KS, bool EMIT>
 __global__ void __launch_bounds__(256)
 smallc_fwd_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ b,
                   float* __restrict__ y, int n, int h, int wd, int co, int pad, int oh, int ow, int act,
-                  float* __restrict__ hi, float* __restrict__ lo) {
+                  float* __restrict__ hi) {
   constexpr int K = CI * KS * KS;
   constexpr int K4 = (K + 3) / 4 * 4;
   extern __shared__ __align__(16) float smem_f[];
@@ -93,7 +93,6 @@ smallc_fwd_kernel(const float* __restrict__ x, const float* __restrict__ w, cons
             const size_t o = (base + pr) * co + c0 + chunk;
             const float4 hv = make_float4(tc::tf32_rn(v.x), tc::tf32_rn(v.y), tc::tf32_rn(v.z), tc::tf32_rn(v.w));
             *reinterpret_cast<float4*>(hi + o) = hv;
-            if (lo) *reinterpret_cast<float4*>(lo + o) = make_float4(v.x - hv.x, v.y - hv.y, v.z - hv.z, v.w - hv.w);
           }
         }
         __syncwarp();
@@ -188,7 +187,7 @@ smallc_wgrad_reduce_kernel(const float* __restrict__ partial, float* dw, int par
 
 template <int CI, int KS, bool EMIT>
 int run_fwd(nrs_ctx* ctx, const float* x, const float* w, const float* b, float* y, int n, int h, int wd, int co,
-            int pad, int oh, int ow, int act, float* hi, float* lo) {
+            int pad, int oh, int ow, int act, float* hi) {
   constexpr int K4 = (CI * KS * KS + 3) / 4 * 4;
   size_t smem = (((size_t)co * K4 + co + 3) / 4 * 4) * sizeof(float);
   if (EMIT) smem += (size_t)8 * 32 * kTileLd * sizeof(float);
@@ -198,7 +197,7 @@ int run_fwd(nrs_ctx* ctx, const float* x, const float* w, const float* b, float*
   size_t blocks = (total + 255) / 256;
   const size_t cap = (size_t)ctx->sm_count * 8;
   if (blocks > cap) blocks = cap;
-  smallc_fwd_kernel<CI, KS, EMIT><<<(unsigned)blocks, 256, smem, ctx->stream>>>(x, w, b, y, n, h, wd, co, pad, oh, ow, act, hi, lo);
+  smallc_fwd_kernel<CI, KS, EMIT><<<(unsigned)blocks, 256, smem, ctx->stream>>>(x, w, b, y, n, h, wd, co, pad, oh, ow, act, hi);
   NRS_LAUNCHED(ctx);
   return NRS_OK;
 }
@@ -244,20 +243,20 @@ int nrs_smallc_conv_fwd(nrs_ctx* ctx, const float* x, const float* w, const floa
                         int wd, int co, int kh, int kw, int stride, int pad, int act) {
   if (!eligible(ci, kh, kw, stride, co)) return NRS_ERR_UNSUPPORTED;
   const int oh = h + 2 * pad - 2, ow = wd + 2 * pad - 2;
-  // Planes of the result requested by the caller (a tensor-core convolution reads it next)?
-  float *hi = nullptr, *lo = nullptr;
+  // Planes of the result requested by the caller (a tensor-core convolution reads it next)?  TF32's only: f16 pairs want a
+  // bound of the result first, and a request that stays where it is sends the caller to a staging pass.
+  float* hi = nullptr;
   auto extras = ctx->out_extras.find(y);
-  if (extras != ctx->out_extras.end() && !extras->second.relu_mask_src && extras->second.hi && co % 32 == 0) {
+  if (extras != ctx->out_extras.end() && !extras->second.relu_mask_src && extras->second.hi && !extras->second.lo && co % 32 == 0) {
     hi = extras->second.hi;
-    lo = extras->second.lo;
     ctx->out_extras.erase(extras);   // honoured
   }
   if (hi) {
-    if (ci == 1) return run_fwd<1, 3, true>(ctx, x, w, b, y, n, h, wd, co, pad, oh, ow, act, hi, lo);
-    return run_fwd<3, 3, true>(ctx, x, w, b, y, n, h, wd, co, pad, oh, ow, act, hi, lo);
+    if (ci == 1) return run_fwd<1, 3, true>(ctx, x, w, b, y, n, h, wd, co, pad, oh, ow, act, hi);
+    return run_fwd<3, 3, true>(ctx, x, w, b, y, n, h, wd, co, pad, oh, ow, act, hi);
   }
-  if (ci == 1) return run_fwd<1, 3, false>(ctx, x, w, b, y, n, h, wd, co, pad, oh, ow, act, nullptr, nullptr);
-  return run_fwd<3, 3, false>(ctx, x, w, b, y, n, h, wd, co, pad, oh, ow, act, nullptr, nullptr);
+  if (ci == 1) return run_fwd<1, 3, false>(ctx, x, w, b, y, n, h, wd, co, pad, oh, ow, act, nullptr);
+  return run_fwd<3, 3, false>(ctx, x, w, b, y, n, h, wd, co, pad, oh, ow, act, nullptr);
 }
 
 int nrs_smallc_conv_wgrad(nrs_ctx* ctx, const float* x, const float* dy, float* dw, int n, int ci, int h, int wd, int co,
