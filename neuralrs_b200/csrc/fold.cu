@@ -394,7 +394,12 @@ int nrs_fold_submit(nrs_ctx* ctx, NrsFoldJob job) {
   if (st != NRS_OK) return st;
   f.tickets_used += need;
   f.jobs.push_back(job);
-  f.holding += f.open ? 1 : 0;
+  bool held = f.open;   // (one launch may leave the sums of several jobs: `open` speaks for the first of them to be submitted)
+  for (const auto& c : f.chunks) {
+    const uintptr_t lo = (uintptr_t)c.first, src = (uintptr_t)job.src, scratch = (uintptr_t)job.scratch;
+    held = held || (src >= lo && src < lo + c.second) || (scratch >= lo && scratch < lo + c.second);
+  }
+  f.holding += held ? 1 : 0;
   f.open = false;
   return NRS_OK;
 }
@@ -478,6 +483,23 @@ extern "C" int nrs_selftest_fold_bookkeeping(void) {
   f.holding = 0;
   bad += nrs_fold_submit(&c, pair) == NRS_OK && f.holding == 0 ? 0 : 1;   // sums in memory of its own: nobody's concern
   bad += nrs_fold_partial(&c, -1, 16, &p[5]) == NRS_OK && p[5] == mem ? 0 : 1;   // nothing waits: from the start again
+
+  // two jobs' sums from one launch, and the queue is launched when the first of them has been submitted
+  f.jobs.clear();
+  f.holding = 0;
+  f.open = false;
+  NrsFoldJob sums = pair;
+  for (int i = 0; i < 2; ++i) bad += nrs_fold_partial(&c, -1, 4096, &p[i]) == NRS_OK ? 0 : 1;
+  sums.src = p[0];
+  bad += nrs_fold_submit(&c, sums) == NRS_OK ? 0 : 1;
+  f.jobs.clear();
+  f.holding = 0;
+  sums.src = p[1];
+  bad += nrs_fold_submit(&c, sums) == NRS_OK && f.holding == 1 ? 0 : 1;
+  bad += nrs_fold_partial(&c, -1, 16, &p[2]) == NRS_OK && p[2] != p[0] && p[2] != p[1] ? 0 : 1;
+  f.jobs.clear();
+  f.holding = 0;
+  f.open = false;
 
   // a weight gradient never starts under a launch of folds
   c.launches = 7;
