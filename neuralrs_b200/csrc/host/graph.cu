@@ -382,7 +382,8 @@ NodeP matmul(const NodeP& a, const NodeP& b) {
   nrs_ctx* ctx = a->ctx;
   NodeP out = make_out(ctx, {(size_t)m, (size_t)n}, {a, b});
   const bool tensor_cores = nrs_gemm_on_tensor_cores(ctx, m, n, k);
-  if (tensor_cores && b->requires_grad) cache_planes_2d(a, (size_t)m, (size_t)k);   // read again by dB = A^T dC
+  // read again by dB = A^T dC; and whose bound is known is staged without a pass that measures it
+  if (tensor_cores && (b->requires_grad || a->top)) cache_planes_2d(a, (size_t)m, (size_t)k);
   check(ctx, nrs_gemm(ctx, 0, 0, m, n, k, a->data, b->data, out->data, nullptr, NRS_ACT_NONE, 0.0f));
   Node* self = out.get();
   out->backward_fn = [self, a, b, m, k, n, tensor_cores]() {
@@ -760,7 +761,8 @@ NodeP conv2d_act(const NodeP& x, const NodeP& w, const NodeP& b, size_t stride, 
   NodeP out = make_out(ctx, {(size_t)n, (size_t)co, (size_t)oh, (size_t)ow}, {x, w, b});
   // The input's NHWC planes serve this forward pass and, later, the weight gradient.
   const bool patches = nrs_conv_uses_patches(ci, kh, kw);
-  if (!patches && !x->planes_hi && w->requires_grad && planes_possible(ctx)) {
+  // (Without one, too, where the input's bound is known: staged here it needs no pass that measures it.)
+  if (!patches && !x->planes_hi && (w->requires_grad || x->top) && planes_possible(ctx)) {
     float *phi = nullptr, *plo = nullptr;
     if (stage_planes(ctx, x->data, x->shape, &phi, &plo, range_in(x->top))) { x->planes_hi = phi; x->planes_lo = plo; }
   }

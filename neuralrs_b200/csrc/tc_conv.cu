@@ -359,10 +359,10 @@ void plan_pixel_tile(const ConvPlan& p, ConvPolicy* pol) {
 
 // The same for slabs: rows of 8, 16, 24 or 32 pixels (a slab's taps have to start on whole swizzle patterns, and it has
 // room for tc::kSlabRows pixels).  Taken where that costs at most a tenth more tiles.
-bool plan_slab_tile(const ConvPlan& p, ConvPolicy* pol) {
-  if (p.ax.in_step != 1 || p.ay.in_step != 1 || p.ay.taps < 2) return false;
+bool plan_slab_tile(const ConvPlan& p, bool split, ConvPolicy* pol) {
+  if (p.ax.in_step != 1 || p.ay.in_step != 1 || p.ay.taps < 2 || (!split && p.n_ch_out <= 32)) return false;
   const long plain = (long)pol->tiles_x * pol->tiles_y * ((p.n_img + pol->Nt - 1) / pol->Nt);
-  long best = plain + plain / 10;
+  long best = plain + (split ? plain / 10 : 0);
   bool found = false;
   for (int Wt = 8; Wt <= 32 && Wt < p.ax.len + 8; Wt += 8) {
     int Ht = tc::BM / Wt;
@@ -388,7 +388,7 @@ int conv_common(nrs_ctx* ctx, ConvPlan& p) {
   const bool split = ctx->math_mode == NRS_MATH_3XTF32;
   ConvPolicy pol{};
   plan_pixel_tile(p, &pol);
-  const bool slab = plan_slab_tile(p, &pol);
+  const bool slab = plan_slab_tile(p, split, &pol);
   pol.taps_y = slab ? p.ay.taps : 1;
   const long tiles_m = (long)((p.n_img + pol.Nt - 1) / pol.Nt) * pol.tiles_y * pol.tiles_x;
   if (tiles_m > 2147483647L) return NRS_ERR_UNSUPPORTED;

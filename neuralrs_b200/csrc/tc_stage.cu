@@ -159,8 +159,11 @@ stage_image_kernel(const float* __restrict__ src, float* __restrict__ hi, float*
   img::tile_to_planes<SPLIT>(tile, g, p0, c0, hi, lo, scale);
 }
 
+// A weight that every block scans itself is staged by blocks of kWideStage threads: five loads a thread instead of eighteen
+// for 64 x 32 x 3 x 3.
+constexpr int kWideStage = 1024, kWideScan = 4096;
 template <bool SPLIT>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kWideStage)
 stage_conv_weight_kernel(const float* __restrict__ w, float* __restrict__ hi, float* __restrict__ lo, int co_n, int ci_n,
                          int kh, int kw, int for_dgrad, const Bound bound) {
   const int taps = kh * kw, rows = for_dgrad ? ci_n : co_n, inner = for_dgrad ? co_n : ci_n, ld = (inner + 31) / 32 * 32;
@@ -523,7 +526,8 @@ int nrs_tc_stage_conv_weight(nrs_ctx* ctx, const float* w, float* hi, float* lo,
   if (lo) {
     const int st = open_planes(ctx, hi, w, (size_t)co * ci * kh * kw, nullptr, &bound);
     if (st != NRS_OK) return st;
-    NRS_PDL_LAUNCH((stage_conv_weight_kernel<true>), nrs_blocks(total, 256), 256, 0, ctx->stream, w, hi, lo, co, ci, kh, kw, for_dgrad, bound);
+    const int threads = bound.scan_n > kWideScan ? kWideStage : 256;
+    NRS_PDL_LAUNCH((stage_conv_weight_kernel<true>), nrs_blocks(total, threads), threads, 0, ctx->stream, w, hi, lo, co, ci, kh, kw, for_dgrad, bound);
   } else {
     NRS_PDL_LAUNCH((stage_conv_weight_kernel<false>), nrs_blocks(total, 256), 256, 0, ctx->stream, w, hi, nullptr, co, ci, kh, kw, for_dgrad, bound);
   }
