@@ -205,7 +205,9 @@ static bool stage_planes(nrs_ctx* ctx, const float* src, const std::vector<size_
 // padded to 32 bytes), so the same planes serve it as the A operand of x@W and, read along the rows, as
 // an operand of the weight gradient x^T dz.  Stages them into fresh pool blocks and registers them with
 // the context under `src`; false (nothing allocated) when a tensor-core GEMM would not read them.
-static bool stage_planes_2d(nrs_ctx* ctx, const float* src, size_t rows, size_t cols, float** hi, float** lo, const NrsRange* known) {
+// `also`: a weight to measure in the same launch (see WeightTop).
+static bool stage_planes_2d(nrs_ctx* ctx, const float* src, size_t rows, size_t cols, float** hi, float** lo, const NrsRange* known,
+                            const float* also = nullptr, size_t also_count = 0, NrsRange* also_range = nullptr) {
   *hi = *lo = nullptr;
   if (ctx->math_mode == NRS_MATH_FP32 || rows == 0 || rows > 2147483647u || cols > 2147483647u) return false;
   if (!tc::tensor_map_encoder() || ctx->plane_hints.count(src)) return false;
@@ -213,7 +215,7 @@ static bool stage_planes_2d(nrs_ctx* ctx, const float* src, size_t rows, size_t 
   const int ld = nrs_plane_ld((int)cols);
   *hi = dplane(ctx, rows * ld);
   if (split) *lo = dplane(ctx, rows * ld);
-  check(ctx, nrs_tc_stage(ctx, src, *hi, *lo, (int)rows, (int)cols, ld, 1, 0, 0, false, nullptr, known));
+  check(ctx, nrs_tc_stage(ctx, src, *hi, *lo, (int)rows, (int)cols, ld, 1, 0, 0, false, nullptr, known, also, also_count, also_range));
   NrsPlanes pl{*hi, *lo, split ? 1 : 0};
   pl.rows = (int)rows;
   pl.cols = (int)cols;
@@ -221,14 +223,42 @@ static bool stage_planes_2d(nrs_ctx* ctx, const float* src, size_t rows, size_t 
   return true;
 }
 
+// The largest magnitude of a weight that a product is about to stage, measured by the launch that stages the product's other
+// operand; known to the staging until the end of the scope, which is that of the operator.
+struct WeightTop {
+  nrs_ctx* ctx;
+  const NodeP& w;
+  TopP top;
+  bool known = false;
+  WeightTop(nrs_ctx* c, const NodeP& w_, bool wanted) : ctx(c), w(w_) {
+    if (wanted && c->math_mode == NRS_MATH_3XTF32 && w->len() > (size_t)pr::kScanAlone && !c->plane_hints.count(w->data) &&
+        !nrs_weight_planes_find(c, w->data, NRS_WF_LINEAR_T) && !nrs_weight_planes_find(c, w->data, NRS_WF_LINEAR_ROWS))
+      top = new_top(c);
+  }
+  bool stage(const float* src, size_t rows, size_t cols, float** hi, float** lo, const NrsRange* of_src) {
+    const bool staged = top ? stage_planes_2d(ctx, src, rows, cols, hi, lo, of_src, w->data, w->len(), top->range)
+                            : stage_planes_2d(ctx, src, rows, cols, hi, lo, of_src);
+    if (staged && top) {
+      ctx->known_tops[w->data] = top->range;
+      known = true;
+    }
+    return staged;
+  }
+  ~WeightTop() {
+    if (known) ctx->known_tops.erase(w->data);
+  }
+};
+
 // Planes of a backward pass's incoming gradient, staged once for the two products that read it
 // (dX = dz W^T and dW = x^T dz) and dropped when the scope ends.
 struct GradPlanes {
   nrs_ctx* ctx;
   const float* key = nullptr;
   float *hi = nullptr, *lo = nullptr;
-  GradPlanes(nrs_ctx* c, const float* dz, size_t rows, size_t cols, bool wanted, const NrsRange* known) : ctx(c) {
-    if (wanted && stage_planes_2d(c, dz, rows, cols, &hi, &lo, known)) key = dz;
+  WeightTop weight;   // (which the data gradient stages)
+  GradPlanes(nrs_ctx* c, const float* dz, size_t rows, size_t cols, bool wanted, const NrsRange* known, const NodeP& w)
+      : ctx(c), weight(c, w, wanted) {
+    if (wanted && weight.stage(dz, rows, cols, &hi, &lo, known)) key = dz;
   }
   ~GradPlanes() {
     if (!key) return;
@@ -239,10 +269,11 @@ struct GradPlanes {
 };
 
 // The forward operand's planes live with its node (both products that read x find them there).
-static void cache_planes_2d(const NodeP& x, size_t rows, size_t cols) {
+static void cache_planes_2d(const NodeP& x, size_t rows, size_t cols, WeightTop* weight = nullptr) {
   if (x->planes_hi) return;
   float *hi = nullptr, *lo = nullptr;
-  if (stage_planes_2d(x->ctx, x->data, rows, cols, &hi, &lo, range_in(x->top))) {
+  if (weight ? weight->stage(x->data, rows, cols, &hi, &lo, range_in(x->top))
+             : stage_planes_2d(x->ctx, x->data, rows, cols, &hi, &lo, range_in(x->top))) {
     x->planes_hi = hi;
     x->planes_lo = lo;
   }
@@ -383,14 +414,15 @@ NodeP matmul(const NodeP& a, const NodeP& b) {
   NodeP out = make_out(ctx, {(size_t)m, (size_t)n}, {a, b});
   const bool tensor_cores = nrs_gemm_on_tensor_cores(ctx, m, n, k);
   // read again by dB = A^T dC; and whose bound is known is staged without a pass that measures it
-  if (tensor_cores && (b->requires_grad || a->top)) cache_planes_2d(a, (size_t)m, (size_t)k);
+  WeightTop b_top(ctx, b, tensor_cores);
+  if (tensor_cores && (b->requires_grad || a->top)) cache_planes_2d(a, (size_t)m, (size_t)k, &b_top);
   check(ctx, nrs_gemm(ctx, 0, 0, m, n, k, a->data, b->data, out->data, nullptr, NRS_ACT_NONE, 0.0f));
   Node* self = out.get();
   out->backward_fn = [self, a, b, m, k, n, tensor_cores]() {
     nrs_ctx* ctx = self->ctx;
     const float* dc = grad_in(self);
     need_values(a);
-    GradPlanes dc_planes(ctx, dc, (size_t)m, (size_t)n, tensor_cores && a->requires_grad && b->requires_grad, grad_top(self));
+    GradPlanes dc_planes(ctx, dc, (size_t)m, (size_t)n, tensor_cores && a->requires_grad && b->requires_grad, grad_top(self), b);
     if (a->requires_grad && a->fold_act != NRS_ACT_NONE) {
       linear_input_grad(ctx, a, b, dc, m, k, n);
     } else if (a->requires_grad) {
@@ -1309,7 +1341,8 @@ NodeP linear_act(const NodeP& x, const NodeP& w, const NodeP& b, int act, bool e
   const int m = (int)x->shape[0], k = (int)x->shape[1], n = (int)w->shape[1];
   NodeP out = make_out(ctx, {(size_t)m, (size_t)n}, {x, w, b});
   const bool tensor_cores = nrs_gemm_on_tensor_cores(ctx, m, n, k);
-  if (tensor_cores && w->requires_grad) cache_planes_2d(x, (size_t)m, (size_t)k);   // read again by dW = x^T dz
+  WeightTop w_top(ctx, w, tensor_cores);
+  if (tensor_cores && (w->requires_grad || x->top)) cache_planes_2d(x, (size_t)m, (size_t)k, &w_top);   // read again by dW = x^T dz
   float* pre = nullptr;  // GELU's derivative needs the pre-activation
   if (act == NRS_ACT_GELU) {
     pre = dalloc(ctx, out->len());
@@ -1372,7 +1405,7 @@ NodeP linear_act(const NodeP& x, const NodeP& w, const NodeP& b, int act, bool e
     }
     // dz feeds both dW = x^T dz and dX = dz W^T: its planes are made once
     GradPlanes dz_planes(ctx, dz, (size_t)m, (size_t)n, !from_planes && tensor_cores && w->requires_grad && x->requires_grad,
-                         act == NRS_ACT_GELU || from_planes ? nullptr : grad_top(self));   // (a ReLU's mask keeps the bound)
+                         act == NRS_ACT_GELU || from_planes ? nullptr : grad_top(self), w);   // (a ReLU's mask keeps the bound)
     if (b->requires_grad) {
       GradTarget t = grad_target(b);
       if (from_planes) check(ctx, nrs_fold_columns(ctx, self->gchan_partial, t.ptr, self->gchan_rows, n, n, t.accumulate));

@@ -233,6 +233,8 @@ struct nrs_ctx {
   unsigned* fold_ticket = nullptr;   // arrival counter of kernels whose last block folds the blocks' partial sums
   // Planes registered for a source tensor (keyed by its device pointer); the conv kernels
   // use them instead of staging again.  Whoever registers keeps both alive and unregisters.
+  // Bounds of tensors for the duration of a call that stages them (an operator that had them measured in another launch).
+  std::map<const void*, const NrsRange*> known_tops;
   std::map<const void*, NrsPlanes> plane_hints;
   std::map<const void*, NrsPlanes> owned_planes;
   std::unordered_map<const void*, NrsRange*> ranges;   // of f16 pair planes (by the address of hi) and of f32 tensors (by their address)
@@ -336,7 +338,9 @@ static inline int nrs_layernorm_sum_rows(const nrs_ctx* ctx) { return 4 * ctx->s
 // of `hi` is renewed and measured, in the same launch for small tensors, unless the caller has one: `measured` becomes the
 // planes' own, `known` bounds the source's values (NrsRange::top).
 int nrs_tc_stage(nrs_ctx* ctx, const float* src, float* hi, float* lo, int rows, int K, int ldk, int batch,
-                 size_t src_bstride, size_t dst_bstride, bool src_k_by_rows, NrsRange* measured = nullptr, const NrsRange* known = nullptr);
+                 size_t src_bstride, size_t dst_bstride, bool src_k_by_rows, NrsRange* measured = nullptr, const NrsRange* known = nullptr,
+                 const float* also = nullptr /*rows as stored, f16 pairs, one matrix: a tensor to measure in the same launch*/,
+                 size_t also_count = 0, NrsRange* also_range = nullptr);
 // NHWC planes of an NCHW tensor [n][c][hw], pixel stride nrs_plane_ld(c) floats (zeros between c and there).
 // chan_partial (hw > 1): [nrs_batchnorm_tiles(n, hw)][c] channel sums of the pixels of each tile.
 int nrs_tc_stage_image(nrs_ctx* ctx, const float* src, float* hi, float* lo, int n, int c, int hw, float* chan_partial = nullptr,

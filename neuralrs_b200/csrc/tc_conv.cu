@@ -359,10 +359,10 @@ void plan_pixel_tile(const ConvPlan& p, ConvPolicy* pol) {
 
 // The same for slabs: rows of 8, 16, 24 or 32 pixels (a slab's taps have to start on whole swizzle patterns, and it has
 // room for tc::kSlabRows pixels).  Taken where that costs at most a tenth more tiles.
-bool plan_slab_tile(const ConvPlan& p, bool split, ConvPolicy* pol) {
-  if (p.ax.in_step != 1 || p.ay.in_step != 1 || p.ay.taps < 2 || (!split && p.n_ch_out <= 32)) return false;
+bool plan_slab_tile(const ConvPlan& p, ConvPolicy* pol) {
+  if (p.ax.in_step != 1 || p.ay.in_step != 1 || p.ay.taps < 2) return false;
   const long plain = (long)pol->tiles_x * pol->tiles_y * ((p.n_img + pol->Nt - 1) / pol->Nt);
-  long best = plain + (split ? plain / 10 : 0);
+  long best = plain + plain / 10;
   bool found = false;
   for (int Wt = 8; Wt <= 32 && Wt < p.ax.len + 8; Wt += 8) {
     int Ht = tc::BM / Wt;
@@ -388,7 +388,7 @@ int conv_common(nrs_ctx* ctx, ConvPlan& p) {
   const bool split = ctx->math_mode == NRS_MATH_3XTF32;
   ConvPolicy pol{};
   plan_pixel_tile(p, &pol);
-  const bool slab = plan_slab_tile(p, split, &pol);
+  const bool slab = split && plan_slab_tile(p, &pol);   // (TF32: 5 % slower with slabs on most layers, 256 x 200 x 9 x 8 -> 200 205 us, without 186)
   pol.taps_y = slab ? p.ay.taps : 1;
   const long tiles_m = (long)((p.n_img + pol.Nt - 1) / pol.Nt) * pol.tiles_y * pol.tiles_x;
   if (tiles_m > 2147483647L) return NRS_ERR_UNSUPPORTED;
@@ -470,10 +470,14 @@ int conv_common(nrs_ctx* ctx, ConvPlan& p) {
   int splits = 0;
   const tc::TilePlan tile = tc::plan_tile(ctx, tiles_m, p.n_ch_out, 1, p.ay.taps * p.ax.taps * blocks32, split, 0.025, true, slab);
 #define NRS_RUN_AS(BN_, PAIR_, SLAB_)                                                                                          \
-  st = !split ? run_conv<BN_, 1, PAIR_, 32, SLAB_>(ctx, p, (const float*)a_hi, nullptr, pol, rg, (int)tiles_m, &splits)          \
-       : wide ? run_conv<BN_, 2, PAIR_, 64, SLAB_>(ctx, p, (const float*)a_hi, (const float*)a_lo, pol, rg, (int)tiles_m, &splits) \
-              : run_conv<BN_, 2, PAIR_, 32, SLAB_>(ctx, p, (const float*)a_hi, (const float*)a_lo, pol, rg, (int)tiles_m, &splits)
-#define NRS_RUN(BN_, PAIR_) { if (slab) NRS_RUN_AS(BN_, PAIR_, true); else NRS_RUN_AS(BN_, PAIR_, false); }
+  st = wide ? run_conv<BN_, 2, PAIR_, 64, SLAB_>(ctx, p, (const float*)a_hi, (const float*)a_lo, pol, rg, (int)tiles_m, &splits) \
+            : run_conv<BN_, 2, PAIR_, 32, SLAB_>(ctx, p, (const float*)a_hi, (const float*)a_lo, pol, rg, (int)tiles_m, &splits)
+#define NRS_RUN(BN_, PAIR_)                                                                                                    \
+  {                                                                                                                            \
+    if (!split) st = run_conv<BN_, 1, PAIR_, 32, false>(ctx, p, (const float*)a_hi, nullptr, pol, rg, (int)tiles_m, &splits);   \
+    else if (slab) NRS_RUN_AS(BN_, PAIR_, true);                                                                               \
+    else NRS_RUN_AS(BN_, PAIR_, false);                                                                                        \
+  }
   if (tile.pair && tile.bn == 128) NRS_RUN(128, true)
   else if (tile.pair) NRS_RUN(64, true)
   else if (tile.bn == 128) NRS_RUN(128, false)

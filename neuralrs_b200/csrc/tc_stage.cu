@@ -60,18 +60,49 @@ struct Bound {
 template <bool SPLIT>
 __device__ __forceinline__ float open_range(const Bound& b) { return SPLIT ? pr::open_range(b.top, b.src, b.scan_n, b.range) : 1.0f; }
 
+// `also`: a tensor whose largest magnitude the grid's last blocks measure meanwhile (the weight that the staged rows are to
+// be multiplied with: a launch of its own costs a small model's step 3 us).
+struct Also {
+  const float* src;
+  size_t count;
+  NrsRange* range;
+  unsigned blocks;
+};
+__device__ __forceinline__ void measure_also(const Also& a, unsigned first) {
+  uint32_t top = 0;
+  const size_t step = (size_t)a.blocks * blockDim.x, tid = (size_t)(blockIdx.x - first) * blockDim.x + threadIdx.x;
+  const size_t quads = (reinterpret_cast<uintptr_t>(a.src) & 15) == 0 ? a.count / 4 : 0;
+  const float4* body = reinterpret_cast<const float4*>(a.src);
+  for (size_t i = tid; i < quads; i += 4 * step) {
+    float v[16];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const float4 q = i + u * step < quads ? body[i + u * step] : make_float4(0.f, 0.f, 0.f, 0.f);
+      v[4 * u] = q.x; v[4 * u + 1] = q.y; v[4 * u + 2] = q.z; v[4 * u + 3] = q.w;
+    }
+    top = pr::seen_all(top, v);
+  }
+  for (size_t i = 4 * quads + tid; i < a.count; i += step) top = pr::seen(top, a.src[i]);
+  pr::report_block(a.range, top);
+}
+
 template <bool SPLIT>
 __global__ void __launch_bounds__(256)
 stage_rows_kernel(const float* __restrict__ src, float* __restrict__ hi, float* __restrict__ lo, int rows, int K,
-                  int ldk, size_t src_bstride, size_t dst_bstride, const NrsFastDiv div_q, const Bound bound) {
+                  int ldk, size_t src_bstride, size_t dst_bstride, const NrsFastDiv div_q, const Bound bound, const Also also) {
   NRS_PDL_PROLOGUE();
+  const unsigned blocks = gridDim.x - also.blocks;
+  if (SPLIT && blockIdx.x >= blocks) {
+    measure_also(also, blocks);
+    return;
+  }
   const float scale = open_range<SPLIT>(bound);
   const int b = blockIdx.y;
   src += b * src_bstride;
   const size_t dst = b * dst_bstride;
   const int q = ldk / 4;
   const size_t total4 = (size_t)rows * q;
-  const size_t stride = (size_t)gridDim.x * blockDim.x;
+  const size_t stride = (size_t)blocks * blockDim.x;
   const bool vec = (K & 3) == 0 && ((reinterpret_cast<uintptr_t>(src) & 15) == 0);
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total4; i += stride) {
     const size_t r = total4 < ((size_t)1 << 31) ? div_q.div((uint32_t)i) : i / q;   // (a 64-bit division is some 80 instructions)
@@ -412,6 +443,10 @@ int nrs_pair_unpack(nrs_ctx* ctx, const float* hi, const float* lo, float* dst, 
 // it, a scan by the staging kernel's blocks for small sources, else a launch that measures.
 static int open_planes(nrs_ctx* ctx, const float* hi, const float* src, size_t count, const NrsRange* known, Bound* b) {
   *b = Bound{nullptr, src, 0, nullptr};
+  if (!known && !ctx->known_tops.empty()) {
+    auto it = ctx->known_tops.find(src);
+    if (it != ctx->known_tops.end()) known = it->second;
+  }
   int st = nrs_range_renew(ctx, hi, &b->range);
   if (st != NRS_OK) return st;
   b->top = known ? &known->top : &b->range->top;
@@ -473,7 +508,8 @@ int nrs_tc_stage_masked(nrs_ctx* ctx, int mode, const float* g, const float* y, 
 }
 
 int nrs_tc_stage(nrs_ctx* ctx, const float* src, float* hi, float* lo, int rows, int K, int ldk, int batch,
-                 size_t src_bstride, size_t dst_bstride, bool src_k_by_rows, NrsRange* measured, const NrsRange* known) {
+                 size_t src_bstride, size_t dst_bstride, bool src_k_by_rows, NrsRange* measured, const NrsRange* known,
+                 const float* also, size_t also_count, NrsRange* also_range) {
   if (rows <= 0 || K <= 0 || batch <= 0) return NRS_OK;
   Bound bound{measured ? &measured->top : nullptr, src, 0, measured};
   if (lo && !measured) {
@@ -485,9 +521,11 @@ int nrs_tc_stage(nrs_ctx* ctx, const float* src, float* hi, float* lo, int rows,
     const size_t cap = (size_t)ctx->sm_count * 16;
     if (blocks > cap) blocks = cap;
     if (batch > 65535) return NRS_ERR_UNSUPPORTED;
-    dim3 grid((unsigned)blocks, (unsigned)batch);
-    if (lo) NRS_PDL_LAUNCH((stage_rows_kernel<true>), grid, 256, 0, ctx->stream, src, hi, lo, rows, K, ldk, src_bstride, dst_bstride, NrsFastDiv(ldk / 4), bound);
-    else NRS_PDL_LAUNCH((stage_rows_kernel<false>), grid, 256, 0, ctx->stream, src, hi, nullptr, rows, K, ldk, src_bstride, dst_bstride, NrsFastDiv(ldk / 4), bound);
+    Also more{};
+    if (also && lo && batch == 1) more = Also{also, also_count, also_range, absmax_blocks(ctx, also_count)};
+    dim3 grid((unsigned)blocks + more.blocks, (unsigned)batch);
+    if (lo) NRS_PDL_LAUNCH((stage_rows_kernel<true>), grid, 256, 0, ctx->stream, src, hi, lo, rows, K, ldk, src_bstride, dst_bstride, NrsFastDiv(ldk / 4), bound, more);
+    else NRS_PDL_LAUNCH((stage_rows_kernel<false>), grid, 256, 0, ctx->stream, src, hi, nullptr, rows, K, ldk, src_bstride, dst_bstride, NrsFastDiv(ldk / 4), bound, more);
   } else {
     dim3 grid((unsigned)((rows + 31) / 32), (unsigned)((ldk + 31) / 32), (unsigned)batch);
     if (grid.y > 65535 || grid.z > 65535) return NRS_ERR_UNSUPPORTED;

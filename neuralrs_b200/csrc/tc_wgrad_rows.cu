@@ -359,6 +359,9 @@ int nrs_tc_conv_wgrad_rows(nrs_ctx* ctx, const float* x, const float* dy, float*
   if (kh != 3 || kw != 3 || stride != 1 || pad != 1 || ci % 32 != 0 || co % 32 != 0 || n < 1 || h < 1 || wd < 1) return NRS_ERR_UNSUPPORTED;
   const bool split3 = ctx->math_mode == NRS_MATH_3XTF32;
   const int planes = split3 ? 2 : 1;
+  // A TF32 gradient on its own: rows of 16, 32 or 64 pixels (256 x 12 x 12, 256 -> 128 channels: 58 us here, 49 by the general
+  // kernel).  Among others of a backward pass all of them (CIFAR CNN with batch normalisation: a step 1.35 ms, 1.38 without).
+  if (!split3 && wd != 16 && wd != 32 && wd != 64 && !ctx->folds.active) return NRS_ERR_UNSUPPORTED;
 
   RowParams p{};
   p.co = co; p.ci = ci;
