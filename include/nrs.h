@@ -182,7 +182,7 @@ int nrs_conv2d_bwd(nrs_ctx* ctx, const float* x, const float* w, const float* dy
                    int accumulate);
 
 /* Operand caching for callers that drive the convolutions operator by operator.  The tensor-core
- * kernels read an activation as channels-last TF32 planes; nrs_conv2d_fwd / _bwd make them from the
+ * kernels read an activation as channels-last operand planes; nrs_conv2d_fwd / _bwd make them from the
  * NCHW tensor on every call.  A caller that knows a tensor is read more than once (x by the forward
  * pass and by the weight gradient; dy by both gradients) has them made once:
  * nrs_planes_cache(t, [n,c,h,w]) stages the planes of t's CURRENT contents into memory the library

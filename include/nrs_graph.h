@@ -40,7 +40,8 @@ int nrs_node_set_requires_grad(nrs_node* n, int flag);
  * the next nrs_to_cuda uploads it into the node's existing device buffer. */
 int nrs_node_set_data(nrs_node* n, const float* host_data);
 /* Device pointers of a resident node (NULL when absent).  The library caches re-laid-out copies
- * of a tensor that a convolution has read (its tensor-core operand planes); a caller that writes
+ * of a tensor that a convolution has read (its tensor-core operand planes) and the largest magnitude
+ * that the operator which made it has met; a caller that writes
  * new values through nrs_node_data_ptr must call nrs_node_invalidate afterwards, or use a fresh
  * node.  nrs_to_cuda invalidates by itself. */
 float* nrs_node_data_ptr(nrs_node* n);

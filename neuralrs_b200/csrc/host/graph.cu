@@ -1000,7 +1000,7 @@ NodeP flatten(const NodeP& x) {
 // (the add + layernorm pairs of src/cuda/nn/transformer_block.rs:33-34,41-42).  One backward launch
 // produces the input gradient(s) and, through per-block partial sums, dgamma / dbeta.
 // emit_planes: the caller knows that the result feeds tensor-core GEMMs and that the residual addend's only
-// reader is this node (the transformer block): the forward kernel then writes the result's TF32 planes itself,
+// reader is this node (the transformer block): the forward kernel then writes the result's operand planes itself,
 // and the backward kernel those of the addend's gradient, instead of a staging pass per tensor.
 static NodeP layernorm_impl(const NodeP& x, const NodeP& residual, const NodeP& gamma, const NodeP& beta, float eps,
                             bool emit_planes = false) {

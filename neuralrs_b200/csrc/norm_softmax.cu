@@ -208,7 +208,7 @@ __device__ __forceinline__ void st4_stream(float* p, float4 v) { __stcs(reinterp
 
 // ------------------------------------------------------------------ LayerNorm forward
 // x = a (+ b when given: the residual add folded in); y = gamma * xhat + beta.
-// EMIT: also write the TF32 planes of y (a separate instantiation, so that the plain kernel keeps its registers).
+// EMIT: also write the operand planes of y (a separate instantiation, so that the plain kernel keeps its registers).
 template <int VPL, bool EMIT>
 __global__ void __launch_bounds__(kRowThreads)
 ln_fwd_vec_kernel(const float* __restrict__ a, const float* __restrict__ b, const float* __restrict__ gamma,
@@ -817,7 +817,7 @@ int nrs_layernorm_residual_bwd(nrs_ctx* ctx, const float* g, const float* xhat, 
                        accumulate_db, accumulate_params);
 }
 
-// The same two operators with the TF32 planes of their result written by the kernel itself (y forward; the
+// The same two operators with the operand planes of their result written by the kernel itself (y forward; the
 // input gradient backward): *emitted = 1 when the planes were written (vector path), 0 when the caller has
 // to stage them itself.  Internal: the graph's fused transformer block calls them.
 int nrs_layernorm_fwd_planes(nrs_ctx* ctx, const float* a, const float* b, const float* gamma, const float* beta, float* y,

@@ -323,7 +323,7 @@ void nrs_pinned_release(nrs_ctx* ctx);
 // them.  Slot 0 serves kernels with one counter, slots 1.. kernels with a counter per column block.
 constexpr int kNrsFoldTickets = 4096;
 int nrs_fold_ticket(nrs_ctx* ctx, unsigned** out);
-// LayerNorm with the TF32 planes of its result written by the kernel (norm_softmax.cu).
+// LayerNorm with the operand planes of its result written by the kernel (norm_softmax.cu).
 extern "C" int nrs_layernorm_fwd_planes(nrs_ctx* ctx, const float* a, const float* b, const float* gamma, const float* beta,
                                         float* y, float* xhat, float* istd, int rows, int f, float eps, float* y_hi, float* y_lo,
                                         int* emitted, NrsRange* istd_range);

@@ -56,7 +56,7 @@ struct ConvPolicyOf {
   int taps_y;                         // slabs: vertical taps that one serves
   uint32_t slice_rows;                // pixels of a tile's box
   float k_total;                      // terms of a sum, for the result's bound
-  // optional: ReLU mask taken from an NCHW tensor of the output's shape, and NHWC TF32 planes of
+  // optional: ReLU mask taken from an NCHW tensor of the output's shape, and NHWC operand planes of
   // the result for the next tensor-core kernel
   const float* mask_src;
   float* out_hi;

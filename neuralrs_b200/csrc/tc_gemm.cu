@@ -6,7 +6,7 @@
 // (dense K-major row slices, row-major store with bias/activation/accumulate) and
 // operand preparation.  Both operands are consumed K-major: an operand stored
 // the other way round is transposed by the staging pass, which for 3xTF32 also
-// writes the high/residual planes.  Plain TF32 reads untransposed, 16-byte
+// writes f16 pairs.  Plain TF32 reads untransposed, 16-byte
 // aligned operands in place.
 //
 // Reference counterparts: matmul_nn / matmul_nt / matmul_tn, 64x64x16 FFMA tiles

@@ -3,9 +3,9 @@
 // memory, fed by TMA, consumed by tcgen05.mma kind::tf32 (TF32 mode) or kind::f16 (3xTF32).
 //
 // Persistent CTAs (one per SM) walk a list of output tiles (row tile, column tile,
-// batch x K-split).  Six to eighteen warps, fixed roles:
+// batch x K-split).  Six to nineteen warps, fixed roles:
 //   warp 0     TMA producer: per K-slice, one mbarrier-tracked ring
-//              slot holding the A and B slices (and their residual planes for 3xTF32);
+//              slot holding the A and B slices (for 3xTF32 both halves of the pairs);
 //              the ring runs ahead across tile boundaries
 //   warp 1     TMEM allocation; issues the UMMAs (M=128, K=8 or 16) and commits
 //              ring slots back to the producer, then the accumulator to the epilogue

@@ -1,7 +1,6 @@
 // Operand staging for the tensor-core kernels: one memory-bound pass that brings an
 // operand into the K-major form with 16-byte aligned rows that TMA wants and, for 3xTF32,
-// splits it into a TF32 high plane (round-to-nearest) and an f32 residual plane
-// (x - hi, exact).  Without the split the single plane is still rounded to nearest
+// makes f16 pairs of it (pair.cuh).  Without the split the single plane is still rounded to nearest
 // TF32: the tensor core truncates its inputs, and truncation's systematic bias
 // compounds through a deep network where rounding's does not.  Transposed sources ([K][rows], e.g. NCHW images seen as
 // [C][H*W]) go through 32x32 shared-memory tiles so both sides stay coalesced.
@@ -227,7 +226,7 @@ stage_conv_weight_kernel(const float* __restrict__ w, float* __restrict__ hi, fl
 //           y is the POOLED output here: the window's maximum is > 0 exactly where the winner
 //           passed the ReLU, so the full-resolution activation is not read at all)
 // One pass reads the NCHW sources through 32 channel x 32 pixel tiles and writes the
-// masked gradient in NCHW (optional) and as NHWC TF32 planes (optional).
+// masked gradient in NCHW (optional) and as NHWC operand planes (optional).
 template <bool SPLIT, int MODE>
 __global__ void __launch_bounds__(256)
 stage_masked_kernel(const float* __restrict__ g, const float* __restrict__ y, const int32_t* __restrict__ argmax,
