@@ -1377,7 +1377,9 @@ NodeP linear_act(const NodeP& x, const NodeP& w, const NodeP& b, int act, bool e
   }
   Node* self = out.get();
   out->grad_sums_wanted = act == NRS_ACT_NONE && b->requires_grad;
-  if (act != NRS_ACT_NONE && tensor_cores && n % 8 == 0 && w->requires_grad && b->requires_grad && nrs_gemm_tn_reads_planes(k, n)) {
+  // (a weight gradient over 16 rows or fewer runs on the FFMA kernels, which read values, not planes)
+  if (act != NRS_ACT_NONE && tensor_cores && n % 8 == 0 && w->requires_grad && b->requires_grad && m > 16 && nrs_gemm_on_tensor_cores(ctx, k, n, m) &&
+      nrs_gemm_tn_reads_planes(k, n)) {
     out->fold_act = act;
     out->fold_src = act == NRS_ACT_GELU ? pre : out->data;
   }
