@@ -112,6 +112,9 @@ int nrs_selftest_smem_attr_bookkeeping(void);
 /* Host-only self-test (no reference counterpart, needs no GPU): the queue of second-stage reductions of a backward
  * pass knows every tensor that a queued reduction writes.  Returns 0 when that bookkeeping behaves. */
 int nrs_selftest_fold_bookkeeping(void);
+/* Host-only self-test (no reference counterpart, needs no GPU): what a convolution's epilogue reads ahead of the
+ * accumulator belongs to channels that exist, also in a last column tile with few of them.  Returns 0 when so. */
+int nrs_selftest_conv_reads_ahead(void);
 /* Self-tests of device memory that runs out (no reference counterpart).  The first is host-only: which slabs of the pool
  * may go back to the driver.  The second plays a driver that refuses: what the context keeps idle goes back before an
  * allocation fails, and queued reductions run for the sake of their scratch.  Both return 0 when all is well. */

@@ -194,7 +194,7 @@ struct ConvPolicyOf {
   template <int W>
   __device__ __forceinline__ uint32_t fetch(const Row& rw, int nb, bool any) const {
     uint32_t keep = ~0u;
-    if (mask_src && any && rw.live) {   // (whole channel blocks only)
+    if (mask_src && any && rw.live && nb < n_ch_out) {   // (whole channel blocks only)
       const size_t plane = (size_t)out_h * out_w;
       const float* m = mask_src + rw.off + (size_t)nb * plane;
       float mv[W];
@@ -551,4 +551,49 @@ int nrs_tc_conv_dgrad(nrs_ctx* ctx, const float* w, const float* dy, float* dx, 
     }
   if (lent) ctx->plane_hints.erase(dy);
   return st;
+}
+
+namespace {
+
+// Columns [n, n + width) that the epilogue warps read ahead of a layer's accumulators: checks that failed.
+template <int BN, bool SLAB>
+int check_reads_ahead(int n_ch, int* ragged) {
+  using E = tc::EpiBlocks<BN, ConvPolicyOf<16, SLAB>>;
+  int bad = 0;
+  for (int n0 = 0; n0 < n_ch; n0 += BN) {
+    if (n_ch - n0 < BN) ++*ragged;
+    for (int warp = 0; warp < 16; ++warp) {
+      const int c = E::first(warp), n = n0 + c * E::kW;
+      const bool reads = E::reads_first(c, n0, n_ch, 1);
+      bad += reads == (c < E::kBlocks && n < n_ch) && !(reads && n + E::kW > n_ch) ? 0 : 1;
+      bad += E::reads_first(c, n0, n_ch, 2) ? 1 : 0;   // (a K-split's results do not pass through here)
+    }
+  }
+  return bad;
+}
+
+}  // namespace
+
+// Host-only: over layers of whole 32-channel blocks (those whose data gradient may apply a mask) on images of several sizes, the
+// plan that their data gradient takes never has an epilogue warp read a channel that the layer does not have.
+extern "C" int nrs_selftest_conv_reads_ahead(void) {
+  static const struct { int n, hw; } kImages[] = {{1, 32}, {9, 32}, {64, 32}, {64, 16}, {100, 8}, {13, 10}, {256, 4}, {1024, 32}};
+  nrs_ctx ctx;   // (only its SM count is asked for)
+  int bad = 0, ragged = 0;
+  for (const auto& im : kImages)
+    for (int ch = 32; ch <= 512; ch += 32)
+      for (int co : {32, 128, 200}) {
+        ConvPlan p{};
+        p.n_img = im.n; p.a_ch = co;
+        p.ay = p.ax = ConvAxis{im.hw, 1, 0, 3, 0, 1, 1, 1};
+        ConvPolicy pol{};
+        plan_pixel_tile(p, &pol);
+        const bool slab = plan_slab_tile(p, &pol);
+        const long tiles_m = (long)((im.n + pol.Nt - 1) / pol.Nt) * pol.tiles_y * pol.tiles_x;
+        const tc::TilePlan tile = tc::plan_tile(&ctx, tiles_m, ch, 1, 9 * ((co + 31) / 32), true, 0.025, true, slab);
+        if (tile.bn == 128) bad += slab ? check_reads_ahead<128, true>(ch, &ragged) : check_reads_ahead<128, false>(ch, &ragged);
+        else if (tile.bn == 64) bad += slab ? check_reads_ahead<64, true>(ch, &ragged) : check_reads_ahead<64, false>(ch, &ragged);
+        else bad += slab ? check_reads_ahead<32, true>(ch, &ragged) : check_reads_ahead<32, false>(ch, &ragged);
+      }
+  return bad + (ragged > 0 ? 0 : 1);   // (layers with a ragged last column tile are among them)
 }

@@ -211,6 +211,21 @@ __device__ __forceinline__ void rows_to_lines(float* tile, int lane, const uint3
   for (int i = 0; i < 4; ++i) v[i] = t4[chunk(8 * i + (lane >> 2), lane & 3)];
 }
 
+// The column blocks of an epilogue warp: block c of a tile is its columns [c * kW, (c + 1) * kW); a warp takes c_first,
+// c_first + kStep, ...
+template <int BN, class Policy>
+struct EpiBlocks {
+  static constexpr int kW = Policy::kCanEmit && Policy::kTeamWarps == 4 ? 32 : 16, kBlocks = BN / kW, kStep = Policy::kEpiWarps / 4;
+  // (a team of eight: 2 * team + half)
+  __host__ __device__ static constexpr int first(int warp /*from 0, of the epilogue*/) { return kStep == 1 ? 0 : warp >> 2; }
+  // Does the epilogue of the tile whose columns start at n0 read what belongs to the warp's first block?  The tile has that
+  // block, the output has columns in it (a ragged last column tile may not), and the results leave here, not through a
+  // K-split's second pass.
+  __host__ __device__ static constexpr bool reads_first(int c_first, int n0, int n_total, int splits) {
+    return c_first < kBlocks && n0 + c_first * kW < n_total && splits == 1;
+  }
+};
+
 template <int BN, int NPLANES, class Policy, bool PAIR, int KW>
 __global__ void __launch_bounds__(threads<Policy>(), 1)
 tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ CUtensorMap tm_a_lo,
@@ -523,10 +538,11 @@ tc_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ C
       if (!pol.clip(tile_m, tile_n, BN, &kb_begin, &kb_end)) continue;   // the same verdict in all three roles
       const int n0 = tile_n * BN;
       [[maybe_unused]] const auto rw = pol.row(tile_m, batch, row);   // index arithmetic under the main loop
-      constexpr int kW = Policy::kCanEmit && Policy::kTeamWarps == 4 ? 32 : 16, kBlocks = BN / kW, kStep = Policy::kEpiWarps / 4;
-      const int c_first = kStep == 1 ? 0 : (warp - 2) >> 2;   // (a team of eight: 2 * team + half)
+      using E = EpiBlocks<BN, Policy>;
+      constexpr int kW = E::kW, kBlocks = E::kBlocks, kStep = E::kStep;
+      const int c_first = E::first(warp - 2);
       // What the first block reads besides the accumulator is under way before that is full.
-      [[maybe_unused]] auto extra = pol.template fetch<kW>(rw, n0 + c_first * kW, c_first < kBlocks);
+      [[maybe_unused]] auto extra = pol.template fetch<kW>(rw, n0 + c_first * kW, E::reads_first(c_first, n0, sp.n_total, sp.splits));
       for (int k0 = kb_begin; k0 < kb_end && ok; k0 += sp.kb_per_split) {
         const uint32_t buf = local & 1u, use = local >> 1;
         ++local;

@@ -58,3 +58,8 @@ def test_fold_queue_knows_every_tensor_it_writes(nrs_lib):
 
 def test_pool_gives_back_slabs_that_are_not_in_use(nrs_lib):
     assert nrs_lib.nrs_selftest_pool_bookkeeping() == 0
+
+
+def test_convolution_epilogues_read_ahead_only_what_exists(nrs_lib):
+    """Masked data gradients over every count of whole 32-channel blocks: no epilogue warp asks for a channel beyond the last."""
+    assert nrs_lib.nrs_selftest_conv_reads_ahead() == 0

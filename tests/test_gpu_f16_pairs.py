@@ -201,6 +201,25 @@ def test_trainer_convolutions(gpu_ctx, oracle64, net):
         assert rel_l2(a, b) <= 2 * convs * chain_tolerance(648) + chain_tolerance(13 * 24 * 16), i
 
 
+@pytest.mark.parametrize("c,n,hw", [(96, 9, 32), (96, 100, 8), (160, 20, 16), (160, 5, 32)])
+def test_masked_data_gradients_with_a_ragged_column_tile(gpu_ctx, oracle64, c, n, hw):
+    """64-column tiles by pairs of CTAs, 32 live channels in the last one, and the mask of the ReLU below.  Whole inputs and
+    weights and a bias of a half: no pre-activation is near zero, whatever the rounding."""
+    layers = [("conv", 3, c, 3, 1, 1), ("relu",), ("conv", c, 32, 3, 1, 1), ("flatten",), ("linear", 32 * hw * hw, 10)]
+    rng = np.random.default_rng(c + n)
+    x = rng.integers(-3, 4, (n, 3, hw, hw)).astype(np.float32)
+    t = np.eye(10, dtype=np.float32)[rng.integers(0, 10, n)]
+    params = workloads.he_init(layers, 7)
+    params[0][:] = rng.integers(-1, 2, params[0].shape)
+    params[1][:] = 0.5
+    tr = cuda.Trainer(layers, (3, hw, hw), 10, ctx=gpu_ctx)
+    tr.set_params([p.ravel() for p in params])
+    tr.forward_backward(x, t)
+    _, ref, _ = models.forward_backward(oracle64, layers, params, x, t, buffers={})
+    for i, b in enumerate(ref):   # three products in a row each way, then the gradient's own
+        assert rel_l2(tr.get_grad(i), b) <= 6 * chain_tolerance(9 * c) + chain_tolerance(min(8192, n * hw * hw)), i
+
+
 @pytest.mark.parametrize("d,rows", [(64, 12), (256, 700), (512, 90)])
 def test_bias_gradient_from_the_layernorm_above(gpu_ctx, oracle64, d, rows):
     """The column sums that LayerNorm's backward pass leaves for the feed-forward layer below it."""
