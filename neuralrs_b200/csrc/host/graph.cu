@@ -71,12 +71,21 @@ FlatStore::~FlatStore() {
   if (grad) nrs_free(ctx, grad);
 }
 
+// The node whose memory `n` uses, values and gradient (reshape/flatten results alias their input).
+static Node* grad_root(Node* n) {
+  while (n->view_of) n = n->view_of.get();
+  return n;
+}
+// What is known of `n`'s values belongs to their memory: a view asks its root, so whoever rewrites the memory has one place
+// to tell.
+static const TopP& data_top(const NodeP& n) { return grad_root(n.get())->top; }
+
 // Operand planes and patch planes are functions of the tensor's contents: whoever rewrites `data`
 // in place drops them (and the context's hints), so the next convolution stages fresh ones.
 void invalidate_operand_caches(Node* n) {
   nrs_ctx* ctx = n->ctx;
   if (!ctx) return;
-  n->top.reset();
+  grad_root(n)->top.reset();
   if (n->planes_hi) {
     ctx->plane_hints.erase(n->data);
     nrs_free(ctx, n->planes_hi);
@@ -101,12 +110,6 @@ NodeP node_new(nrs_ctx* ctx, const float* host, const std::vector<size_t>& shape
 }
 
 GradSums::~GradSums() { nrs_free(ctx, partial); }
-
-// The node whose gradient buffer `n` uses (reshape/flatten results alias their input).
-static Node* grad_root(Node* n) {
-  while (n->view_of) n = n->view_of.get();
-  return n;
-}
 
 struct GradTarget {
   float* ptr;
@@ -272,8 +275,8 @@ struct GradPlanes {
 static void cache_planes_2d(const NodeP& x, size_t rows, size_t cols, WeightTop* weight = nullptr) {
   if (x->planes_hi) return;
   float *hi = nullptr, *lo = nullptr;
-  if (weight ? weight->stage(x->data, rows, cols, &hi, &lo, range_in(x->top))
-             : stage_planes_2d(x->ctx, x->data, rows, cols, &hi, &lo, range_in(x->top))) {
+  if (weight ? weight->stage(x->data, rows, cols, &hi, &lo, range_in(data_top(x)))
+             : stage_planes_2d(x->ctx, x->data, rows, cols, &hi, &lo, range_in(data_top(x)))) {
     x->planes_hi = hi;
     x->planes_lo = lo;
   }
@@ -415,7 +418,7 @@ NodeP matmul(const NodeP& a, const NodeP& b) {
   const bool tensor_cores = nrs_gemm_on_tensor_cores(ctx, m, n, k);
   // read again by dB = A^T dC; and whose bound is known is staged without a pass that measures it
   WeightTop b_top(ctx, b, tensor_cores);
-  if (tensor_cores && (b->requires_grad || a->top)) cache_planes_2d(a, (size_t)m, (size_t)k, &b_top);
+  if (tensor_cores && (b->requires_grad || data_top(a))) cache_planes_2d(a, (size_t)m, (size_t)k, &b_top);
   check(ctx, nrs_gemm(ctx, 0, 0, m, n, k, a->data, b->data, out->data, nullptr, NRS_ACT_NONE, 0.0f));
   Node* self = out.get();
   out->backward_fn = [self, a, b, m, k, n, tensor_cores]() {
@@ -502,7 +505,7 @@ NodeP relu(const NodeP& x) {
   NodeP out = make_out(ctx, x->shape, {x});
   const size_t len = x->len();
   check(ctx, nrs_relu_fwd(ctx, x->data, out->data, len));
-  out->top = x->top;
+  out->top = data_top(x);
   Node* self = out.get();
   out->backward_fn = [self, x, len]() {
     if (!x->requires_grad) return;
@@ -521,7 +524,7 @@ NodeP gelu(const NodeP& x) {
   NodeP out = make_out(ctx, x->shape, {x});
   const size_t len = x->len();
   check(ctx, nrs_gelu_fwd(ctx, x->data, out->data, len));
-  out->top = x->top;   // |gelu(x)| <= |x|
+  out->top = data_top(x);   // |gelu(x)| <= |x|
   Node* self = out.get();
   out->backward_fn = [self, x, len]() {
     if (!x->requires_grad) return;
@@ -546,7 +549,6 @@ NodeP reshape(const NodeP& x, const std::vector<size_t>& shape) {
   out->data = x->data;
   out->owns_data = false;
   out->view_of = x;
-  out->top = x->top;
   out->parents = {x};
   out->requires_grad = x->requires_grad;
   return out;
@@ -794,9 +796,9 @@ NodeP conv2d_act(const NodeP& x, const NodeP& w, const NodeP& b, size_t stride, 
   // The input's NHWC planes serve this forward pass and, later, the weight gradient.
   const bool patches = nrs_conv_uses_patches(ci, kh, kw);
   // (Without one, too, where the input's bound is known: staged here it needs no pass that measures it.)
-  if (!patches && !x->planes_hi && (w->requires_grad || x->top) && planes_possible(ctx)) {
+  if (!patches && !x->planes_hi && (w->requires_grad || data_top(x)) && planes_possible(ctx)) {
     float *phi = nullptr, *plo = nullptr;
-    if (stage_planes(ctx, x->data, x->shape, &phi, &plo, range_in(x->top))) { x->planes_hi = phi; x->planes_lo = plo; }
+    if (stage_planes(ctx, x->data, x->shape, &phi, &plo, range_in(data_top(x)))) { x->planes_hi = phi; x->planes_lo = plo; }
   }
   // Few input channels in a TF32 mode: forward and weight gradient both run on the tensor cores over the
   // input's patch planes; make them once.
@@ -933,7 +935,7 @@ NodeP maxpool2d(const NodeP& x, size_t kernel, size_t stride, bool emit_planes) 
     // a tensor-core convolution reads the result next: write its operand planes in the same pass
     float* phi = dplane(ctx, out->len());
     float* plo = ctx->math_mode == NRS_MATH_3XTF32 ? dplane(ctx, out->len()) : nullptr;
-    const int st = nrs_tc_pool2_fwd_planes(ctx, x->data, out->data, (int32_t*)am, phi, plo, n, c, h, w, range_in(x->top));
+    const int st = nrs_tc_pool2_fwd_planes(ctx, x->data, out->data, (int32_t*)am, phi, plo, n, c, h, w, range_in(data_top(x)));
     if (st == NRS_OK) {
       out->planes_hi = phi;
       out->planes_lo = plo;
@@ -946,7 +948,7 @@ NodeP maxpool2d(const NodeP& x, size_t kernel, size_t stride, bool emit_planes) 
     }
   }
   if (!done) check(ctx, nrs_maxpool_fwd(ctx, x->data, out->data, (int32_t*)am, n, c, h, w, k, s));
-  out->top = x->top;
+  out->top = data_top(x);
   Node* self = out.get();
   out->backward_fn = [self, x, am, n, c, h, w, k, s]() {
     if (!x->requires_grad) return;
@@ -1342,7 +1344,7 @@ NodeP linear_act(const NodeP& x, const NodeP& w, const NodeP& b, int act, bool e
   NodeP out = make_out(ctx, {(size_t)m, (size_t)n}, {x, w, b});
   const bool tensor_cores = nrs_gemm_on_tensor_cores(ctx, m, n, k);
   WeightTop w_top(ctx, w, tensor_cores);
-  if (tensor_cores && (w->requires_grad || x->top)) cache_planes_2d(x, (size_t)m, (size_t)k, &w_top);   // read again by dW = x^T dz
+  if (tensor_cores && (w->requires_grad || data_top(x))) cache_planes_2d(x, (size_t)m, (size_t)k, &w_top);   // read again by dW = x^T dz
   float* pre = nullptr;  // GELU's derivative needs the pre-activation
   if (act == NRS_ACT_GELU) {
     pre = dalloc(ctx, out->len());

@@ -117,8 +117,8 @@ struct Node {
   // only need not be written besides.  planes_only: `data` was left out (3xTF32: the f16 pairs hold it to 2^-23).
   bool internal = false, planes_only = false;
 
-  // 3xTF32: bounds of `data` and of `grad` where their writer left one (null: unknown).  Whoever writes the tensor otherwise
-  // drops them: to_cuda, grad_target.
+  // 3xTF32: bounds of `data` and of `grad` where their writer left one (null: unknown), with the node that owns the memory
+  // (null on its views).  Whoever writes the tensor otherwise drops them: to_cuda, nrs_node_invalidate, grad_target.
   TopP top, gtop;
 
   size_t len() const;

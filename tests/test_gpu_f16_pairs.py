@@ -220,6 +220,24 @@ def test_masked_data_gradients_with_a_ragged_column_tile(gpu_ctx, oracle64, c, n
         assert rel_l2(tr.get_grad(i), b) <= 6 * chain_tolerance(9 * c) + chain_tolerance(min(8192, n * hw * hw)), i
 
 
+@pytest.mark.parametrize("told", ["root", "view", "sibling"])
+def test_views_of_rewritten_values(gpu_ctx, oracle64, told):
+    """Values a hundred times the bound their operator left, written through the device pointer and announced through any
+    node that shares them: whoever shares them multiplies the new ones."""
+    n, ci, hw, co, out = 32, 32, 4, 32, 64
+    rng = np.random.default_rng(3)
+    x, wt = rng.standard_normal((n, ci, hw, hw)).astype(np.float32), (rng.standard_normal((co, ci, 3, 3)) / 17).astype(np.float32)
+    w = (rng.standard_normal((co * hw * hw, out)) / 23).astype(np.float32)
+    h = nn.conv2d(on_gpu(x), on_gpu(wt), on_gpu(np.zeros(co, np.float32)), 1, 1)
+    views = [nn.flatten(h), graph.reshape(h, [n, co * hw * hw])]
+    new = (100 * rng.standard_normal((n, co * hw * hw))).astype(np.float32)
+    call(gpu_ctx, "nrs_d2d", _lib.VP(h.data_ptr()), Dev(gpu_ctx, new), new.nbytes)
+    {"root": h, "view": views[0], "sibling": views[1]}[told].invalidate()
+    got = gpu.to_host(graph.matmul(views[0], on_gpu(w))).reshape(n, out)
+    err = np.abs(got - new.astype(np.float64) @ w.astype(np.float64))
+    assert (err <= entry_bound(new, w, co * hw * hw)).all(), float(np.abs(got).max())
+
+
 @pytest.mark.parametrize("d,rows", [(64, 12), (256, 700), (512, 90)])
 def test_bias_gradient_from_the_layernorm_above(gpu_ctx, oracle64, d, rows):
     """The column sums that LayerNorm's backward pass leaves for the feed-forward layer below it."""
