@@ -43,6 +43,33 @@ __device__ __forceinline__ void contribute(float a, float b, float k, float& s, 
   }
 }
 
+// 3xTF32, where the planes of the result are written: their exponent comes from a bound of it, which is made of what the
+// reduction ahead of it meets in its own reading of the tensors (a bound from the count, |xhat| <= sqrt(count), is far
+// looser, and does not hold where the variance is lost in the rounding of its sums: a channel that is constant but for its
+// first value).  extremes[split][ch] = forward (largest |x - k|, 0), backward (largest |g|, largest |xhat|); of finite values.
+struct BnBound {
+  NrsRange* out;         // null: no planes, or the bound is not made here
+  const NrsRange* x;     // evaluation, forward: the input's
+  const float *gamma, *beta, *istd;
+  int training;
+};
+// By any thread, once a channel.  (A channel whose statistics are not finite has no finite results to bound.)
+__device__ __forceinline__ void take_bound(NrsRange* out, float b) {
+  atomicMax(reinterpret_cast<unsigned*>(&out->bound), __float_as_uint(fminf(b * 1.001f, 3.0e38f)));
+}
+__device__ __forceinline__ bool finite(float v) { return fabsf(v) < __int_as_float(0x7f800000); }
+__device__ __forceinline__ void bound_output(const BnBound& b, int ch, float far /*of x from k*/, float k, float mean, float istd) {
+  if (!b.out || !finite(mean) || !finite(istd)) return;
+  const float xhat = istd * (b.training ? far + fabsf(k - mean) : b.x->top + fabsf(mean));
+  take_bound(b.out, fabsf(b.gamma[ch]) * xhat + fabsf(b.beta[ch]));
+}
+__device__ __forceinline__ void bound_dx(const BnBound& b, int ch, float g, float xhat, float s, float q, float count) {
+  const float ga = fabsf(b.gamma[ch]), istd = b.istd[ch];
+  const float means = b.training ? ga * fabsf(s) / count + xhat * (ga * fabsf(q) / count) : 0.0f;
+  if (!b.out || !finite(istd) || !finite(s) || !finite(q)) return;
+  take_bound(b.out, istd * (ga * g + means));
+}
+
 // What the folded sums of a channel become; done by the last block of the channel to arrive (an integer ticket; the
 // splits are added in order whichever block that is), or by a kernel of its own where there are more channels than
 // tickets, columns instead of planes, or sums to be shared across processes first.
@@ -56,16 +83,19 @@ struct BnFinish {
   float2* sums;
   float *dgamma, *dbeta;
   int accumulate;
+  BnBound bound;
 };
 __device__ __forceinline__ void finish_stats(int ch, float s, float q, float k, float count, float eps, float momentum, float* mean,
-                                             float* istd, float* running_mean, float* running_var) {
+                                             float* istd, float* running_mean, float* running_var, const BnBound& bound, float far) {
   const float d = s / count;
   const float m = k + d;
   const float v = fmaxf(q / count - d * d, 0.0f);
   running_mean[ch] = momentum * running_mean[ch] + (1.0f - momentum) * m;
   running_var[ch] = momentum * running_var[ch] + (1.0f - momentum) * v;
   mean[ch] = m;
-  istd[ch] = 1.0f / sqrtf(v + eps);
+  const float is = 1.0f / sqrtf(v + eps);
+  istd[ch] = is;
+  bound_output(bound, ch, far, k, m, is);
 }
 __device__ __forceinline__ void finish_grads(int ch, float s, float q, float2* sums, float* dgamma, float* dbeta, int accumulate) {
   sums[ch] = make_float2(s, q);
@@ -74,17 +104,19 @@ __device__ __forceinline__ void finish_grads(int ch, float s, float q, float2* s
 }
 
 // Planes layout (hw >= 2): one block per (channel, sample split), 128-bit loads when the plane allows.
-// partial[split][ch] = (S, Q).
+// partial[split][ch] = (S, Q).  MEASURE: extremes too (see BnBound).
 // RELU (backward only): the layer's output went through a ReLU fused into the normalise pass; the incoming
 // gradient is masked where that output was not positive, the output being recomputed from xhat with the very
 // expression of the forward pass (fmaf(gamma, xhat, beta)), so the mask is the forward one bit for bit.
-template <bool FWD, bool RELU>
+template <bool FWD, bool RELU, bool MEASURE>
 __global__ void __launch_bounds__(kThreads)
-bn_pair_planes_kernel(const float* __restrict__ a, const float* __restrict__ b, float2* __restrict__ partial, int n,
-                      int c, int hw, int splits, const float* __restrict__ gamma, const float* __restrict__ beta,
+bn_pair_planes_kernel(const float* __restrict__ a, const float* __restrict__ b, float2* __restrict__ partial, float2* __restrict__ extremes,
+                      int n, int c, int hw, int splits, const float* __restrict__ gamma, const float* __restrict__ beta,
                       const float* __restrict__ pivot, const float* __restrict__ mean, const float* __restrict__ istd, const BnFinish fin, const NrsFastDiv div_per, const int vec /*planes of whole float4s*/) {
   NRS_PDL_PROLOGUE();
   __shared__ float2 sm[kThreads / 32];
+  [[maybe_unused]] __shared__ uint2 sm_top[kThreads / 32];
+  [[maybe_unused]] uint32_t top_a = 0, top_b = 0;
   const int ch = blockIdx.x, split = blockIdx.y;
   const int lane = threadIdx.x & 31, wrp = threadIdx.x >> 5;
   const int n_per = (n + splits - 1) / splits;
@@ -126,6 +158,10 @@ bn_pair_planes_kernel(const float* __restrict__ a, const float* __restrict__ b, 
         contribute<FWD>(va.y, vb.y, k, s1, q1);
         contribute<FWD>(va.z, vb.z, k, s, q);
         contribute<FWD>(va.w, vb.w, k, s1, q1);
+        if (MEASURE) {
+          top_a = pr::seen4(top_a, FWD ? make_float4(va.x - k, va.y - k, va.z - k, va.w - k) : va);
+          if (!FWD) top_b = pr::seen4(top_b, vb);
+        }
       }
     }
   } else {
@@ -137,6 +173,10 @@ bn_pair_planes_kernel(const float* __restrict__ a, const float* __restrict__ b, 
       float va = a[base + i];
       if (RELU) va = fmaf(ga, vb, be) > 0.0f ? va : 0.0f;
       contribute<FWD>(va, vb, k, s, q);
+      if (MEASURE) {
+        top_a = pr::seen(top_a, FWD ? va - k : va);
+        if (!FWD) top_b = pr::seen(top_b, vb);
+      }
     }
   }
   s += s1;
@@ -144,12 +184,21 @@ bn_pair_planes_kernel(const float* __restrict__ a, const float* __restrict__ b, 
   s = wsum(s);
   q = wsum(q);
   if (lane == 0) sm[wrp] = make_float2(s, q);
+  if (MEASURE) {
+    top_a = __reduce_max_sync(0xffffffffu, top_a);
+    top_b = __reduce_max_sync(0xffffffffu, top_b);
+    if (lane == 0) sm_top[wrp] = make_uint2(top_a, top_b);
+  }
   __syncthreads();
   if (threadIdx.x == 0) {
     float2 t = sm[0];
 #pragma unroll
     for (int i = 1; i < kThreads / 32; ++i) { t.x += sm[i].x; t.y += sm[i].y; }
     partial[(size_t)split * c + ch] = t;
+    if (MEASURE) {
+      for (int i = 1; i < kThreads / 32; ++i) { top_a = max(top_a, sm_top[i].x); top_b = max(top_b, sm_top[i].y); }
+      extremes[(size_t)split * c + ch] = make_float2(__uint_as_float(top_a), __uint_as_float(top_b));
+    }
     if (!fin.tickets) return;
     __threadfence();
     if (atomicAdd(&fin.tickets[ch], 1u) != (unsigned)splits - 1) return;
@@ -162,20 +211,42 @@ bn_pair_planes_kernel(const float* __restrict__ a, const float* __restrict__ b, 
       ts += v.x;
       tq += v.y;
     }
-    if (FWD) finish_stats(ch, ts, tq, k, fin.count, fin.eps, fin.momentum, fin.mean, fin.istd, fin.running_mean, fin.running_var);
-    else finish_grads(ch, ts, tq, fin.sums, fin.dgamma, fin.dbeta, fin.accumulate);
+    [[maybe_unused]] float2 ext = make_float2(0.0f, 0.0f);
+    if (MEASURE) {
+#pragma unroll 4
+      for (int z = 0; z < splits; ++z) {
+        const float2 v = __ldcg(extremes + (size_t)z * c + ch);
+        ext = make_float2(fmaxf(ext.x, v.x), fmaxf(ext.y, v.y));
+      }
+    }
+    if (FWD) {
+      finish_stats(ch, ts, tq, k, fin.count, fin.eps, fin.momentum, fin.mean, fin.istd, fin.running_mean, fin.running_var, fin.bound, ext.x);
+    } else {
+      finish_grads(ch, ts, tq, fin.sums, fin.dgamma, fin.dbeta, fin.accumulate);
+      if (MEASURE && fin.bound.out) bound_dx(fin.bound, ch, ext.x, ext.y, ts, tq, fin.count);
+    }
   }
+}
+__device__ __forceinline__ float2 fold_extremes(const float2* __restrict__ extremes, int ch, int c, int splits) {
+  float2 e = make_float2(0.0f, 0.0f);
+  for (int z = 0; extremes && z < splits; ++z) {
+    const float2 v = extremes[(size_t)z * c + ch];
+    e = make_float2(fmaxf(e.x, v.x), fmaxf(e.y, v.y));
+  }
+  return e;
 }
 
 // Columns layout (hw == 1): a block owns 32 features and a slice of the rows; its 8 warps stride the rows
 // reading 128-byte row segments.
 template <bool FWD, bool RELU>
 __global__ void __launch_bounds__(kThreads)
-bn_pair_cols_kernel(const float* __restrict__ a, const float* __restrict__ b, float2* __restrict__ partial, int rows,
-                    int cols, int splits, const float* __restrict__ gamma, const float* __restrict__ beta,
+bn_pair_cols_kernel(const float* __restrict__ a, const float* __restrict__ b, float2* __restrict__ partial,
+                    float2* __restrict__ extremes /*or null*/, int rows, int cols, int splits, const float* __restrict__ gamma, const float* __restrict__ beta,
                     const float* __restrict__ pivot, const float* __restrict__ mean, const float* __restrict__ istd) {
   NRS_PDL_PROLOGUE();
   __shared__ float2 sm[kThreads / 32][33];
+  __shared__ uint2 sm_top[kThreads / 32][33];
+  uint32_t top_a = 0, top_b = 0;
   const int lane = threadIdx.x & 31, wrp = threadIdx.x >> 5;
   const int col = blockIdx.x * 32 + lane, split = blockIdx.y;
   const int rows_per = (rows + splits - 1) / splits;
@@ -191,15 +262,24 @@ bn_pair_cols_kernel(const float* __restrict__ a, const float* __restrict__ b, fl
       float va = a[i];
       if (RELU) va = fmaf(ga, vb, be) > 0.0f ? va : 0.0f;
       contribute<FWD>(va, vb, k, s, q);
+      if (extremes) {
+        top_a = pr::seen(top_a, FWD ? va - k : va);
+        if (!FWD) top_b = pr::seen(top_b, vb);
+      }
     }
   }
   sm[wrp][lane] = make_float2(s, q);
+  sm_top[wrp][lane] = make_uint2(top_a, top_b);
   __syncthreads();
   if (wrp == 0 && col < cols) {
     float2 t = sm[0][lane];
 #pragma unroll
     for (int i = 1; i < kThreads / 32; ++i) { t.x += sm[i][lane].x; t.y += sm[i][lane].y; }
     partial[(size_t)split * cols + col] = t;
+    if (extremes) {
+      for (int i = 1; i < kThreads / 32; ++i) { top_a = max(top_a, sm_top[i][lane].x); top_b = max(top_b, sm_top[i][lane].y); }
+      extremes[(size_t)split * cols + col] = make_float2(__uint_as_float(top_a), __uint_as_float(top_b));
+    }
   }
 }
 
@@ -211,13 +291,16 @@ bn_pair_cols_kernel(const float* __restrict__ a, const float* __restrict__ b, fl
 __global__ void bn_stats_finish_kernel(const float2* __restrict__ partial, const float* __restrict__ x, float* mean,
                                        float* istd, float* running_mean, float* running_var, int c, int hw,
                                        int splits, float count, float eps, float momentum, int training,
-                                       const float* __restrict__ pivot, const float* __restrict__ count_dev) {
+                                       const float* __restrict__ pivot, const float* __restrict__ count_dev,
+                                       const float2* __restrict__ extremes, int extreme_splits, const BnBound bound) {
   NRS_PDL_PROLOGUE();
   const int ch = blockIdx.x * blockDim.x + threadIdx.x;
   if (ch >= c) return;
   if (!training) {
-    mean[ch] = running_mean[ch];
-    istd[ch] = 1.0f / sqrtf(running_var[ch] + eps);
+    const float m = running_mean[ch], is = 1.0f / sqrtf(running_var[ch] + eps);
+    mean[ch] = m;
+    istd[ch] = is;
+    bound_output(bound, ch, 0.0f, 0.0f, m, is);
     return;
   }
   float s = 0.0f, q = 0.0f;
@@ -228,13 +311,14 @@ __global__ void bn_stats_finish_kernel(const float2* __restrict__ partial, const
   }
   const float k = pivot ? pivot[ch] : x[(size_t)ch * hw];
   if (count_dev) count = *count_dev;
-  finish_stats(ch, s, q, k, count, eps, momentum, mean, istd, running_mean, running_var);
+  finish_stats(ch, s, q, k, count, eps, momentum, mean, istd, running_mean, running_var, bound, fold_extremes(extremes, ch, c, extreme_splits).x);
 }
 
 // Folds the backward sums; sums[ch] = (dbeta, dgamma) of this call feeds the dx kernel, and the parameter
 // gradients receive them (+)=.
 __global__ void bn_grad_finish_kernel(const float2* __restrict__ partial, float2* __restrict__ sums, float* dgamma,
-                                      float* dbeta, int c, int splits, int accumulate) {
+                                      float* dbeta, int c, int splits, int accumulate, const float2* __restrict__ extremes,
+                                      float count, const BnBound bound) {
   NRS_PDL_PROLOGUE();
   const int ch = blockIdx.x * blockDim.x + threadIdx.x;
   if (ch >= c) return;
@@ -245,6 +329,9 @@ __global__ void bn_grad_finish_kernel(const float2* __restrict__ partial, float2
     q += t.y;
   }
   finish_grads(ch, s, q, sums, dgamma, dbeta, accumulate);
+  if (!bound.out) return;
+  const float2 e = fold_extremes(extremes, ch, c, splits);
+  bound_dx(bound, ch, e.x, e.y, s, q, count);
 }
 
 // y = gamma * xhat + beta, xhat = (x - mean) * istd (bn2d_normalize, batchnorm2d.rs:62-75).
@@ -343,35 +430,14 @@ bn_dx_kernel(const float* __restrict__ g, const float* __restrict__ xhat, const 
   }
 }
 
-// Bounds of what the two kernels below write, for the exponent of f16 pairs: one block.
-// Forward: |xhat| <= sqrt(count) under the batch's own statistics, else istd * (|x| + |mean|).
-__global__ void __launch_bounds__(256)
-bn_bound_kernel(const float* __restrict__ gamma, const float* __restrict__ beta, const float* __restrict__ mean, const float* __restrict__ istd,
-                const NrsRange* __restrict__ x, float count, int training, NrsRange* __restrict__ out, int c) {
+// The bound of dx where the sums are those of several processes (elsewhere it is made where the sums are finished).
+__global__ void bn_dx_bound_kernel(const float2* __restrict__ sums, const float2* __restrict__ extremes, int splits,
+                                   const float* __restrict__ count_dev, int c, const BnBound bound) {
   NRS_PDL_PROLOGUE();
-  uint32_t top = 0;
-  for (int i = threadIdx.x; i < c; i += 256) {
-    const float xhat = training ? sqrtf(count) : istd[i] * (x->top + fabsf(mean[i]));
-    top = pr::seen(top, fminf((fabsf(gamma[i]) * xhat + fabsf(beta[i])) * 1.001f, 3.0e38f));
-  }
-  top = __reduce_max_sync(0xffffffffu, top);
-  if ((threadIdx.x & 31) == 0) atomicMax(reinterpret_cast<unsigned*>(&out->bound), top);
-}
-// Backward: istd * (|g gamma| + |m1| + |xhat| |m2|), the means as bn_dx_planes_kernel takes them.
-__global__ void __launch_bounds__(256)
-bn_dx_bound_kernel(const float* __restrict__ gamma, const float* __restrict__ istd, const float2* __restrict__ sums, const NrsRange* __restrict__ g,
-                   float count, int training, const float* __restrict__ count_dev, NrsRange* __restrict__ out, int c) {
-  NRS_PDL_PROLOGUE();
-  if (count_dev) count = *count_dev;
-  uint32_t top = 0;
-  for (int i = threadIdx.x; i < c; i += 256) {
-    const float ga = fabsf(gamma[i]);
-    float b = ga * g->top;
-    if (training) b += ga * fabsf(sums[i].x) / count + sqrtf(count) * ga * fabsf(sums[i].y) / count;
-    top = pr::seen(top, fminf(istd[i] * b * 1.001f, 3.0e38f));
-  }
-  top = __reduce_max_sync(0xffffffffu, top);
-  if ((threadIdx.x & 31) == 0) atomicMax(reinterpret_cast<unsigned*>(&out->bound), top);
+  const int ch = blockIdx.x * blockDim.x + threadIdx.x;
+  if (ch >= c) return;
+  const float2 e = fold_extremes(extremes, ch, c, splits), t = sums[ch];
+  bound_dx(bound, ch, e.x, e.y, t.x, t.y, *count_dev);
 }
 
 // The normalise pass with the NHWC planes of y (no xhat).
@@ -502,16 +568,19 @@ int plan_splits(const nrs_ctx* ctx, int n, int c, int hw) {
 }
 
 template <bool FWD, bool RELU>
-int launch_pair(nrs_ctx* ctx, const float* a, const float* b, float2* partial, int n, int c, int hw, int splits,
+int launch_pair(nrs_ctx* ctx, const float* a, const float* b, float2* partial, float2* extremes, int n, int c, int hw, int splits,
                 const float* gamma, const float* beta, const float* pivot = nullptr, const float* mean = nullptr,
                 const float* istd = nullptr, const BnFinish& fin = BnFinish{}) {
   if (hw == 1) {
-    NRS_PDL_LAUNCH((bn_pair_cols_kernel<FWD, RELU>), dim3((c + 31) / 32, splits), kThreads, 0, ctx->stream, a, b, partial, n, c,
-                   splits, gamma, beta, pivot, mean, istd);
+    NRS_PDL_LAUNCH((bn_pair_cols_kernel<FWD, RELU>), dim3((c + 31) / 32, splits), kThreads, 0, ctx->stream, a, b, partial, extremes,
+                   n, c, splits, gamma, beta, pivot, mean, istd);
   } else {
     const bool vec = (hw & 3) == 0 && aligned16(a) && (FWD || aligned16(b));
-    NRS_PDL_LAUNCH((bn_pair_planes_kernel<FWD, RELU>), dim3(c, splits), kThreads, 0, ctx->stream, a, b, partial, n, c, hw,
-                   splits, gamma, beta, pivot, mean, istd, fin, NrsFastDiv(vec ? hw / 4 : hw), vec ? 1 : 0);
+#define NRS_BN_PAIR(M)                                                                                                         \
+  NRS_PDL_LAUNCH((bn_pair_planes_kernel<FWD, RELU, M>), dim3(c, splits), kThreads, 0, ctx->stream, a, b, partial, extremes, n, c, hw, \
+                 splits, gamma, beta, pivot, mean, istd, fin, NrsFastDiv(vec ? hw / 4 : hw), vec ? 1 : 0)
+    if (extremes) NRS_BN_PAIR(true); else NRS_BN_PAIR(false);
+#undef NRS_BN_PAIR
   }
   NRS_LAUNCHED(ctx);
   return NRS_OK;
@@ -542,7 +611,8 @@ namespace {
 
 int bn_forward(nrs_ctx* ctx, const char* who, const float* x, const float* gamma, const float* beta, float* running_mean,
                float* running_var, float* y, float* xhat, float* istd, int n, int c, int hw, float eps, float momentum,
-               int training, bool relu, float* mean_out = nullptr, float* hi = nullptr, float* lo = nullptr) {
+               int training, bool relu, float* mean_out = nullptr, float* hi = nullptr, float* lo = nullptr,
+               const NrsRange* known_x = nullptr) {
   NRS_REQUIRE_CTX(ctx);
   NRS_REQUIRE(ctx, check_dims(n, c, hw), NRS_ERR_SHAPE, "%s: bad shape [%d,%d,%d]", who, n, c, hw);
   NRS_REQUIRE(ctx, x && gamma && beta && running_mean && running_var && y && istd, NRS_ERR_ARG, "%s: null tensor", who);
@@ -552,14 +622,29 @@ int bn_forward(nrs_ctx* ctx, const char* who, const float* x, const float* gamma
   // summed across ranks together with the element count, then finished as usual
   const bool shared = training && ctx->stat_sync.all_reduce_sum != nullptr;
   void* ws = nullptr;
-  const int st = nrs_workspace(ctx, ((size_t)splits * c * 2 + c + (size_t)c * 2 + 4) * sizeof(float), &ws);
+  const bool pairs = hi && lo;
+  const int st = nrs_workspace(ctx, ((size_t)splits * c * (pairs ? 4 : 2) + c + (size_t)c * 2 + 4) * sizeof(float), &ws);
   if (st != NRS_OK) return st;
   float2* partial = (float2*)ws;
-  float* mean_ws = (float*)(partial + (size_t)splits * c);
+  float2* extremes = pairs ? partial + (size_t)splits * c : nullptr;
+  float* mean_ws = (float*)(partial + (size_t)splits * c * (pairs ? 2 : 1));
   float* mean = mean_out ? mean_out : mean_ws;
   float2* summed = (float2*)(mean_ws + c + (c & 1));   // 8-byte aligned; [c] pairs + the count
   float* count_slot = (float*)(summed + c);
   BnFinish fin{};
+  NrsRange* range = nullptr;
+  if (pairs) {
+    int rs = nrs_range_renew(ctx, hi, &range);
+    if (rs == NRS_OK && !training && !known_x) {
+      NrsRange* measured = nullptr;
+      rs = nrs_range_renew(ctx, &ctx->scratch_range[0], &measured);
+      if (rs == NRS_OK) rs = nrs_absmax(ctx, x, (size_t)n * c * hw, measured);
+      known_x = measured;
+    }
+    if (rs != NRS_OK) return rs;
+  }
+  const BnBound bound{range, known_x, gamma, beta, nullptr, training};
+  fin.bound = bound;
   if (training) {
     if (!shared) {
       const int ft = finish_tickets(ctx, c, hw, &fin.tickets);
@@ -567,7 +652,7 @@ int bn_forward(nrs_ctx* ctx, const char* who, const float* x, const float* gamma
       fin.mean = mean; fin.istd = istd; fin.running_mean = running_mean; fin.running_var = running_var;
       fin.count = (float)((double)n * hw); fin.eps = eps; fin.momentum = momentum;
     }
-    const int sp = launch_pair<true, false>(ctx, x, nullptr, partial, n, c, hw, splits, nullptr, nullptr,
+    const int sp = launch_pair<true, false>(ctx, x, nullptr, partial, extremes, n, c, hw, splits, nullptr, nullptr,
                                             shared ? running_mean : nullptr, nullptr, nullptr, fin);
     if (sp != NRS_OK) return sp;
   }
@@ -579,27 +664,16 @@ int bn_forward(nrs_ctx* ctx, const char* who, const float* x, const float* gamma
     if (sr != NRS_OK) return sr;
     NRS_PDL_LAUNCH(bn_stats_finish_kernel, nrs_blocks(c, 128), 128, 0, ctx->stream, (const float2*)summed, x, mean, istd,
                    running_mean, running_var, c, hw, 1, 0.0f, eps, momentum, training, (const float*)running_mean,
-                   (const float*)count_slot);
+                   (const float*)count_slot, (const float2*)extremes, splits, bound);   // (this process's own extremes: its planes)
     NRS_LAUNCHED(ctx);
   } else if (!fin.tickets) {
     NRS_PDL_LAUNCH(bn_stats_finish_kernel, nrs_blocks(c, 128), 128, 0, ctx->stream, (const float2*)partial, x, mean, istd,
                    running_mean, running_var, c, hw, splits, (float)((double)n * hw), eps, momentum, training,
-                   (const float*)nullptr, (const float*)nullptr);
+                   (const float*)nullptr, (const float*)nullptr, (const float2*)extremes, splits, bound);
     NRS_LAUNCHED(ctx);
   }
   if (hi) {
     const img::Grid grid(n, c, hw);
-    NrsRange *range = nullptr, *range_x = nullptr;
-    if (lo) {
-      int rs = nrs_range_renew(ctx, hi, &range);
-      if (rs == NRS_OK && !training) rs = nrs_range_renew(ctx, &ctx->scratch_range[0], &range_x);
-      if (rs == NRS_OK && !training) rs = nrs_absmax(ctx, x, (size_t)n * c * hw, range_x);
-      if (rs != NRS_OK) return rs;
-      // (shared statistics: the count of all processes is not known here; each holds at most 2^31 values a channel)
-      NRS_PDL_LAUNCH(bn_bound_kernel, 1, 256, 0, ctx->stream, gamma, beta, (const float*)mean, (const float*)istd, (const NrsRange*)range_x,
-                     shared ? 2147483648.0f * 8.0f : (float)((double)n * hw), training, range, c);
-      NRS_LAUNCHED(ctx);
-    }
 #define NRS_BN_NORM(S, R)                                                                                               \
   NRS_PDL_LAUNCH((bn_normalize_planes_kernel<S, R>), grid.blocks(), kThreads, 0, ctx->stream, x, (const float*)mean, (const float*)istd, \
                  gamma, beta, y, hi, lo, grid, range)
@@ -625,35 +699,46 @@ int bn_forward(nrs_ctx* ctx, const char* who, const float* x, const float* gamma
 int bn_backward(nrs_ctx* ctx, const char* who, const float* g, const float* xhat, const float* istd, const float* gamma,
                 const float* beta, float* dx, float* dgamma, float* dbeta, int n, int c, int hw, int training,
                 int accumulate_dx, int accumulate_params, bool relu, const float* mean = nullptr /* xhat is x then */,
-                float* hi = nullptr, float* lo = nullptr, float* chan_partial = nullptr, const NrsRange* known_g = nullptr) {
+                float* hi = nullptr, float* lo = nullptr, float* chan_partial = nullptr) {
   NRS_REQUIRE_CTX(ctx);
   NRS_REQUIRE(ctx, check_dims(n, c, hw), NRS_ERR_SHAPE, "%s: bad shape [%d,%d,%d]", who, n, c, hw);
   NRS_REQUIRE(ctx, (dgamma == nullptr) == (dbeta == nullptr), NRS_ERR_ARG, "%s: dgamma and dbeta must be given together", who);
   NRS_REQUIRE(ctx, g && xhat && istd && gamma && (!relu || beta), NRS_ERR_ARG, "%s: null tensor", who);
   if (!dx && !hi && !dgamma) return NRS_OK;
   NrsProfScope prof(ctx, NRS_PROF_BATCHNORM, 12.0 * (double)n * c * hw);   // g, xhat in; dx out
-  const bool need_sums = dgamma || training;
+  const bool pairs = hi && lo;
+  const bool need_sums = dgamma || training || pairs;   // (pairs: the same reading bounds dx)
   const int splits = need_sums ? plan_splits(ctx, n, c, hw) : 1;
   void* ws = nullptr;
-  const int st = nrs_workspace(ctx, ((size_t)splits * c * 2 + (size_t)c * 2 + 4) * sizeof(float), &ws);
+  const int st = nrs_workspace(ctx, ((size_t)splits * c * (pairs ? 4 : 2) + (size_t)c * 2 + 4) * sizeof(float), &ws);
   if (st != NRS_OK) return st;
   float2* partial = (float2*)ws;
-  float2* sums = partial + (size_t)splits * c;
+  float2* extremes = pairs ? partial + (size_t)splits * c : nullptr;
+  float2* sums = partial + (size_t)splits * c * (pairs ? 2 : 1);
   float* count_slot = (float*)(sums + c);
   // with shared statistics dx needs the sums over every process's shard; the parameter gradients keep this
   // process's own sums (they are summed across ranks with all other gradients)
   const bool shared = training && (dx || hi) && ctx->stat_sync.all_reduce_sum != nullptr;
+  const float count = (float)((double)n * hw);
+  NrsRange* range = nullptr;
+  if (pairs) {
+    const int rs = nrs_range_renew(ctx, hi, &range);
+    if (rs != NRS_OK) return rs;
+  }
+  const BnBound bound{range, nullptr, gamma, nullptr, istd, training};
   if (need_sums) {
     BnFinish fin{};
+    if (!shared) fin.bound = bound;   // (else once the sums are those of all processes)
+    fin.count = count;
     const int ft = finish_tickets(ctx, c, hw, &fin.tickets);
     if (ft != NRS_OK) return ft;
     fin.sums = sums; fin.dgamma = dgamma; fin.dbeta = dbeta; fin.accumulate = accumulate_params;
-    const int sp = relu ? launch_pair<false, true>(ctx, g, xhat, partial, n, c, hw, splits, gamma, beta, nullptr, mean, istd, fin)
-                        : launch_pair<false, false>(ctx, g, xhat, partial, n, c, hw, splits, nullptr, nullptr, nullptr, mean, istd, fin);
+    const int sp = relu ? launch_pair<false, true>(ctx, g, xhat, partial, extremes, n, c, hw, splits, gamma, beta, nullptr, mean, istd, fin)
+                        : launch_pair<false, false>(ctx, g, xhat, partial, extremes, n, c, hw, splits, nullptr, nullptr, nullptr, mean, istd, fin);
     if (sp != NRS_OK) return sp;
     if (!fin.tickets) {
       NRS_PDL_LAUNCH(bn_grad_finish_kernel, nrs_blocks(c, 128), 128, 0, ctx->stream, (const float2*)partial, sums, dgamma, dbeta,
-                     c, splits, accumulate_params);
+                     c, splits, accumulate_params, (const float2*)extremes, count, fin.bound);
       NRS_LAUNCHED(ctx);
     }
   }
@@ -663,20 +748,14 @@ int bn_backward(nrs_ctx* ctx, const char* who, const float* g, const float* xhat
     NRS_LAUNCHED(ctx);
     const int sr = ctx->stat_sync.all_reduce_sum(ctx->stat_sync.user, (float*)sums, (size_t)c * 2 + 1);
     if (sr != NRS_OK) return sr;
-  }
-  const float count = (float)((double)n * hw);
-  if (hi) {
-    const img::Grid grid(n, c, hw);
-    NrsRange *range = nullptr, *range_g = nullptr;
-    if (lo) {
-      int rs = nrs_range_renew(ctx, hi, &range);
-      if (rs == NRS_OK && !known_g) rs = nrs_range_renew(ctx, &ctx->scratch_range[0], &range_g);
-      if (rs == NRS_OK && !known_g) rs = nrs_absmax(ctx, g, (size_t)n * c * hw, range_g);
-      if (rs != NRS_OK) return rs;
-      NRS_PDL_LAUNCH(bn_dx_bound_kernel, 1, 256, 0, ctx->stream, gamma, istd, (const float2*)sums, known_g ? known_g : (const NrsRange*)range_g, count, training,
-                     shared ? (const float*)count_slot : (const float*)nullptr, range, c);
+    if (pairs) {
+      NRS_PDL_LAUNCH(bn_dx_bound_kernel, nrs_blocks(c, 128), 128, 0, ctx->stream, (const float2*)sums, (const float2*)extremes, splits,
+                     (const float*)count_slot, c, bound);
       NRS_LAUNCHED(ctx);
     }
+  }
+  if (hi) {
+    const img::Grid grid(n, c, hw);
 #define NRS_BN_DX(S, R)                                                                                                  \
   NRS_PDL_LAUNCH((bn_dx_planes_kernel<S, R>), grid.blocks(), kThreads, 0, ctx->stream, g, xhat, mean, istd, gamma, beta,  \
                  (const float2*)sums, dx, hi, lo, chan_partial, grid, count, training, shared ? (const float*)count_slot : (const float*)nullptr, range)
@@ -738,16 +817,16 @@ int nrs_batchnorm_act_bwd(nrs_ctx* ctx, const float* g, const float* xhat, const
 
 int nrs_batchnorm_fwd_saving_mean(nrs_ctx* ctx, const float* x, const float* gamma, const float* beta, float* running_mean, float* running_var,
                                   float* y, float* mean, float* istd, int n, int c, int hw, float eps, float momentum, int training, int act,
-                                  float* hi, float* lo) {
+                                  float* hi, float* lo, const NrsRange* range_x) {
   return bn_forward(ctx, "batchnorm", x, gamma, beta, running_mean, running_var, y, nullptr, istd, n, c, hw, eps, momentum, training,
-                    act == NRS_ACT_RELU, mean, hi, lo);
+                    act == NRS_ACT_RELU, mean, hi, lo, range_x);
 }
 
 int nrs_batchnorm_bwd_from_x(nrs_ctx* ctx, const float* g, const float* x, const float* mean, const float* istd, const float* gamma,
                              const float* beta, float* dx, float* dgamma, float* dbeta, int n, int c, int hw, int training, int accumulate_dx,
-                             int accumulate_params, int act, float* hi, float* lo, float* chan_partial, const NrsRange* range_g) {
+                             int accumulate_params, int act, float* hi, float* lo, float* chan_partial) {
   return bn_backward(ctx, "batchnorm backward", g, x, istd, gamma, beta, dx, dgamma, dbeta, n, c, hw, training, accumulate_dx, accumulate_params,
-                     act == NRS_ACT_RELU, mean, hi, lo, chan_partial, range_g);
+                     act == NRS_ACT_RELU, mean, hi, lo, chan_partial);
 }
 
 int nrs_batchnorm_tiles(int n, int hw) { return (int)(((size_t)n * hw + img::kTilePx - 1) / img::kTilePx); }

@@ -1181,13 +1181,12 @@ NodeP batchnorm_nd(const NodeP& x, const NodeP& gamma, const NodeP& beta, const 
     out->planes_lo = lo;
   }
   check(ctx, nrs_batchnorm_fwd_saving_mean(ctx, x->data, gamma->data, beta->data, running_mean->data, running_var->data, out->data, mean,
-                                           istd, n, c, hw, eps, momentum, training ? 1 : 0, act, hi, lo));
+                                           istd, n, c, hw, eps, momentum, training ? 1 : 0, act, hi, lo, range_in(data_top(x))));
   if (hi) ctx->plane_hints[out->data] = NrsPlanes{hi, lo, lo ? 1 : 0};
   Node* self = out.get();
   out->backward_fn = [self, x, gamma, beta, mean, istd, n, c, hw, training, act, planes]() {
     nrs_ctx* ctx = self->ctx;
     const float* g = grad_in(self);
-    const TopP g_top = grad_root(self)->gtop;
     float *dg = nullptr, *db = nullptr;
     int acc_p = 0;
     if (gamma->requires_grad || beta->requires_grad) {
@@ -1223,7 +1222,7 @@ NodeP batchnorm_nd(const NodeP& x, const NodeP& gamma, const NodeP& beta, const 
       }
     }
     check(ctx, nrs_batchnorm_bwd_from_x(ctx, g, x->data, mean, istd, gamma->data, beta->data, dx, dg, db, n, c, hw, training ? 1 : 0,
-                                        acc_x, acc_p, act, phi, plo, partial, range_in(g_top)));
+                                        acc_x, acc_p, act, phi, plo, partial));
   };
   return out;
 }

@@ -372,10 +372,10 @@ int nrs_check_device_error(nrs_ctx* ctx);
 // and leaves chan_partial[nrs_batchnorm_tiles(n, hw)][c], its channel sums.
 int nrs_batchnorm_fwd_saving_mean(nrs_ctx* ctx, const float* x, const float* gamma, const float* beta, float* running_mean, float* running_var,
                                   float* y, float* mean, float* istd, int n, int c, int hw, float eps, float momentum, int training, int act,
-                                  float* hi, float* lo);
+                                  float* hi, float* lo, const NrsRange* range_x = nullptr);
 int nrs_batchnorm_bwd_from_x(nrs_ctx* ctx, const float* g, const float* x, const float* mean, const float* istd, const float* gamma,
                              const float* beta, float* dx, float* dgamma, float* dbeta, int n, int c, int hw, int training, int accumulate_dx,
-                             int accumulate_params, int act, float* hi, float* lo, float* chan_partial, const NrsRange* range_g = nullptr);
+                             int accumulate_params, int act, float* hi, float* lo, float* chan_partial);
 int nrs_batchnorm_tiles(int n, int hw);
 
 // Batched weight staging (weight_set.cu).  build: allocates planes for the described weights in the

@@ -238,6 +238,50 @@ def test_views_of_rewritten_values(gpu_ctx, oracle64, told):
     assert (err <= entry_bound(new, w, co * hw * hw)).all(), float(np.abs(got).max())
 
 
+def test_batchnorm_whose_variance_is_lost(gpu_ctx):
+    """Channels that are constant but for their first value, over 2^21 values: what is left of the variance is the rounding of
+    its sums, and the first value lies up to thousands of times sqrt(count) away.  As planes for the next convolution it stays
+    finite: the layer's statistics are the same in both modes, its products are not."""
+    layers = [("batchnorm", 8), ("conv", 8, 32, 3, 1, 1), ("flatten",), ("linear", 32 * 64 * 64, 10)]
+    rng = np.random.default_rng(4)
+    x = np.zeros((512, 8, 64, 64), np.float32)
+    x[0, :, 0, 0] = [100.1, 37.3, 211.7, 5.9, 1e4, 777.7, 3.3e-3, 63.1]
+    t = np.eye(10, dtype=np.float32)[rng.integers(0, 10, 512)]
+    params = workloads.he_init(layers, 7)
+    got = {}
+    try:
+        for mode in (_lib.MATH_3XTF32, _lib.MATH_FP32):
+            gpu_ctx.set_math_mode(mode)
+            tr = cuda.Trainer(layers, (8, 64, 64), 10, ctx=gpu_ctx)
+            tr.set_params([p.ravel() for p in params])
+            tr.forward_backward(x, t)
+            got[mode] = [tr.get_grad(2), tr.get_grad(4)]   # what the planes are multiplied with, and what they make
+    finally:
+        gpu_ctx.set_math_mode(_lib.MATH_3XTF32)
+    for a, b in zip(*got.values()):   # a chain of 72, then of at most 8192 pixels; in f32 as many roundings again
+        assert np.isfinite(a).all() and rel_l2(a, b) <= 2 * chain_tolerance(72) + 2 * chain_tolerance(8192)
+
+
+def test_batchnorm_channels_over_many_octaves(gpu_ctx, oracle64):
+    """Gradients of channels down to 2^-23 of the largest: as planes, below a batch normalisation, they keep their bits."""
+    n, c, hw = 8, 64, 8
+    layers = [("conv", 16, c, 3, 1, 1), ("batchnorm", c), ("conv", c, 32, 3, 1, 1), ("flatten",), ("linear", 32 * hw * hw, 10)]
+    rng = np.random.default_rng(6)
+    x = rng.standard_normal((n, 16, hw, hw)).astype(np.float32)
+    t = np.eye(10, dtype=np.float32)[rng.integers(0, 10, n)]
+    params = workloads.he_init(layers, 7)
+    params[2] = (2.0 ** -(np.arange(c) % 24)).astype(np.float32).reshape(params[2].shape)
+    tr = cuda.Trainer(layers, (16, hw, hw), 10, ctx=gpu_ctx)
+    tr.set_params([p.ravel() for p in params])
+    tr.forward_backward(x, t)
+    _, ref, _ = models.forward_backward(oracle64, layers, params, x, t, buffers=workloads.bn_buffers(layers))
+    got, want = np.asarray(tr.get_grad(0)).reshape(c, -1), np.asarray(ref[0]).reshape(c, -1)
+    # two products forward and one back, twice for what is taken off again in between, then the gradient's own
+    bound = 2 * (chain_tolerance(144) + 2 * chain_tolerance(9 * c)) + chain_tolerance(n * hw * hw)
+    err = np.linalg.norm(got - want, axis=1) / np.linalg.norm(want, axis=1)
+    assert (err <= bound).all(), float((err / bound).max())
+
+
 @pytest.mark.parametrize("d,rows", [(64, 12), (256, 700), (512, 90)])
 def test_bias_gradient_from_the_layernorm_above(gpu_ctx, oracle64, d, rows):
     """The column sums that LayerNorm's backward pass leaves for the feed-forward layer below it."""
