@@ -287,14 +287,20 @@ static NodeP planes_attention(const MultiHeadAttention& m, const NodeP& x, size_
     a.ds_lo = split ? plane(square) : nullptr;
     a.dqkv_hi = plane(tokens * 3 * d);
     a.dqkv_lo = split ? plane(tokens * 3 * d) : nullptr;
-    struct Release {
-      nrs_ctx* c; std::vector<float*> p; const float* key;
+    struct Release {   // (the weight gradient may wait: it reads dqkv, and nothing else of these)
+      nrs_ctx* c; std::vector<float*> now, later; const float* key;
+      void free_now() {
+        for (float* q : now) if (q) nrs_free(c, q);
+        now.clear();
+      }
       ~Release() {
         if (key) c->plane_hints.erase(key);
-        for (float* q : p) if (q) nrs_free_after_wgrads(c, q);
+        free_now();
+        for (float* q : later) if (q) nrs_free_after_wgrads(c, q);
       }
-    } release{ctx, {ghi, glo, a.scores, a.ds_hi, a.ds_lo, a.dqkv_hi, a.dqkv_lo}, nullptr};
+    } release{ctx, {ghi, glo, a.scores, a.ds_hi, a.ds_lo}, {a.dqkv_hi, a.dqkv_lo}, nullptr};
     check(ctx, nrs_mha_planes_bwd(ctx, a));
+    release.free_now();
     NrsPlanes pl{a.dqkv_hi, a.dqkv_lo, split ? 1 : 0};
     pl.rows = (int)tokens;
     pl.cols = (int)(3 * d);
@@ -318,7 +324,7 @@ static NodeP planes_attention(const MultiHeadAttention& m, const NodeP& x, size_
     check(ctx, nrs_tc_conv_wgrad(ctx, a.dqkv_hi, x->data, dst, (int)tokens, (int)(3 * d), 1, 1, (int)d, 1, 1, 1, 0,
                                  side_by_side ? s[0].accumulate : 0, (int)d));
     if (!side_by_side) {
-      release.p.push_back(dst);
+      release.now.push_back(dst);
       check(ctx, nrs_folds_flush(ctx));
       for (int i = 0; i < 3; ++i)
         check(ctx, s[i].accumulate ? nrs_accumulate(ctx, s[i].ptr, dst + i * dd, dd)

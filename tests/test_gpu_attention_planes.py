@@ -1,11 +1,13 @@
 """Multi-head attention over operand planes: sequences inside, at and across the 128-row tiles and the 1024-column row
 kernels, head sizes with padded column and K tiles, causal and not, separate weights and weights of one flat block,
 gradients overwritten and added to; against the f64 oracle."""
+import ctypes
+
 import numpy as np
 import pytest
 
 from neuralrs_b200 import _lib
-from neuralrs_b200.cuda import Node, backward_graph, nn
+from neuralrs_b200.cuda import Context, Node, backward_graph, nn
 from neuralrs_b200.cuda import runtime as gpu
 from oracle import autograd as og
 from .conftest import rel_l2
@@ -47,3 +49,40 @@ def test_mha_over_planes(gpu_ctx, oracle64, shape, causal, mode):
                 assert rel_l2(gpu.read_grad(gn), total * cn.grad) <= TOL[mode]
     finally:
         gpu_ctx.set_math_mode(_lib.MATH_3XTF32)
+
+
+def test_backward_memory_does_not_grow_with_the_square(gpu_ctx):
+    """The weight gradients of Q, K and V wait for the end of the pass where the three lie side by side; what a layer holds for
+    them until then is the planes of their operands, not its scores."""
+    S, D, H = 2048, 128, 4
+    libcuda = ctypes.CDLL("libcuda.so.1")
+
+    def used(ctx):
+        ctx.sync()
+        free, total = ctypes.c_size_t(), ctypes.c_size_t()
+        assert libcuda.cuMemGetInfo_v2(ctypes.byref(free), ctypes.byref(total)) == 0
+        return total.value - free.value
+
+    def grown(layers):
+        ctx = Context(0)
+        try:
+            rng = np.random.default_rng(layers)
+            new = lambda *shape: Node.new((rng.standard_normal(shape) / np.sqrt(D)).astype(np.float32), list(shape), ctx=ctx)  # noqa: E731
+            w = [new(D, D) for _ in range(4 * layers)]
+            h = x = new(1, S, D)
+            for n in w + [x]:
+                gpu.to_cuda(n)
+            gpu.flatten_params(w)
+            for i in range(layers):
+                h = nn.MultiHeadAttention(*w[4 * i:4 * i + 4], D, H, True).forward_batch(h)
+            gpu.set_grad(h, np.ones((1, S, D), np.float32))
+            before = used(ctx)
+            backward_graph(h)
+            after = used(ctx)
+            assert all(np.isfinite(gpu.read_grad(n)).all() for n in w[:4])
+            return after - before
+        finally:
+            ctx.close()
+
+    per_layer = (grown(9) - grown(3)) / 6
+    assert per_layer <= 20 * S * D * 4, per_layer   # (scores and the planes of dS: 8 * H * S * S bytes, 128 times S * D * 4)
