@@ -117,7 +117,8 @@ int nrs_selftest_fold_bookkeeping(void);
 int nrs_selftest_conv_reads_ahead(void);
 /* Self-tests of device memory that runs out (no reference counterpart).  The first is host-only: which slabs of the pool
  * may go back to the driver.  The second plays a driver that refuses: what the context keeps idle goes back before an
- * allocation fails, and queued reductions run for the sake of their scratch.  Both return 0 when all is well. */
+ * allocation fails, queued reductions run for the sake of their scratch, and weight gradients that wait for the sake of what
+ * they hold.  Both return 0 when all is well. */
 int nrs_selftest_pool_bookkeeping(void);
 int nrs_selftest_memory_pressure(nrs_ctx* ctx);
 

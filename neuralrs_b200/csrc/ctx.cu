@@ -38,6 +38,13 @@ int nrs_device_alloc(nrs_ctx* ctx, const char* what, size_t bytes, void** out) {
     give_back_idle(ctx);
     e = ctx->device_malloc(out, bytes);
   }
+  if (e != cudaSuccess && !ctx->folds.waiting.empty()) {   // weight gradients that wait hold what they read
+    (void)cudaGetLastError();
+    const int st = nrs_folds_relieve(ctx);
+    if (st != NRS_OK) return st;
+    give_back_idle(ctx);
+    e = ctx->device_malloc(out, bytes);
+  }
   if (e == cudaSuccess) return NRS_OK;
   (void)cudaGetLastError();
   *out = nullptr;
@@ -304,15 +311,51 @@ int nrs_selftest_memory_pressure(nrs_ctx* ctx) {
   // fold scratch: a full block while folds are queued means that they run and the block starts over
   refuse = 0;
   float *a = nullptr, *b = nullptr, *dst = nullptr;
-  bad += nrs_alloc(ctx, 4096, 1, (void**)&dst) == NRS_OK ? 0 : 1;
+  bad += nrs_alloc(ctx, 40960, 1, (void**)&dst) == NRS_OK ? 0 : 1;
   nrs_folds_begin(ctx);
   bad += nrs_fold_partial(ctx, -1, (size_t)40 << 20, &a) == NRS_OK ? 0 : 1;
   bad += nrs_memset_zero(ctx, a, 4096) == NRS_OK && nrs_fold_columns(ctx, a, dst, 4, 256, 256, 0) == NRS_OK ? 0 : 1;
   refuse = 1 << 20;
   bad += nrs_fold_partial(ctx, -1, (size_t)40 << 20, &b) == NRS_OK && b == a && ctx->folds.jobs.empty() ? 0 : 1;
   refuse = 0;
+  // weight gradients that wait hold what they read: they run, and it goes back, before an allocation fails, and ahead of the
+  // next one where too much is held
+  const int mode = ctx->math_mode;
+  ctx->math_mode = NRS_MATH_3XTF32;
+  const int n = 8, c = 32, hw = 16;
+  const size_t image = sizeof(float) * n * c * hw * hw, weight = sizeof(float) * c * c * 9;
+  float *x = nullptr, *dy = nullptr, *dw = nullptr;
+  bad += nrs_alloc(ctx, image, 1, (void**)&x) == NRS_OK && nrs_alloc(ctx, image, 1, (void**)&dy) == NRS_OK && nrs_alloc(ctx, weight, 0, (void**)&dw) == NRS_OK ? 0 : 1;
+  bad += nrs_planes_cache(ctx, x, n, c, hw, hw) == NRS_OK && nrs_planes_cache(ctx, dy, n, c, hw, hw) == NRS_OK ? 0 : 1;
+  const NrsFolds& f = ctx->folds;
+  for (int limit = 0; limit < 2; ++limit) {
+    bad += cudaMemsetAsync(dw, 0xff, weight, ctx->stream) == cudaSuccess ? 0 : 1;
+    bad += nrs_conv2d_bwd(ctx, x, dw /*no data gradient reads it*/, dy, nullptr, dw, nullptr, n, c, hw, hw, c, 3, 3, 1, 1, 0) == NRS_OK && f.waiting.size() == 1 ? 0 : 1;
+    void *held = nullptr, *more = nullptr;
+    bad += nrs_alloc(ctx, (size_t)60 << 20, 0, &held) == NRS_OK ? 0 : 1;
+    nrs_free_after_wgrads(ctx, held);
+    bad += f.kept.size() == 1 && f.kept_bytes == (size_t)60 << 20 ? 0 : 1;
+    if (limit) {
+      ctx->folds.kept_bytes = kNrsKeptBytes + 1;
+      bad += nrs_conv2d_bwd(ctx, x, dw, dy, nullptr, dst, nullptr, n, c, hw, hw, c, 3, 3, 1, 1, 0) == NRS_OK && f.waiting.size() == 1 ? 0 : 1;
+    } else {
+      refuse = 2;   // what the context keeps idle is not enough
+      bad += nrs_alloc(ctx, (size_t)70 << 20, 0, &more) == NRS_OK && f.waiting.empty() ? 0 : 1;
+      refuse = 0;
+      bad += nrs_free(ctx, more) == NRS_OK ? 0 : 1;
+    }
+    bad += f.kept.empty() && f.kept_bytes == 0 ? 0 : 1;
+    float got[2] = {1.0f, 1.0f};
+    bad += nrs_d2h(ctx, got, dw, sizeof(got)) == NRS_OK && got[0] == 0.0f && got[1] == 0.0f ? 0 : 1;
+  }
+  bad += nrs_folds_flush(ctx) == NRS_OK && f.waiting.empty() ? 0 : 1;
+  // memory of a job that is being made stays its own while others run for the sake of memory
+  bad += nrs_fold_partial(ctx, -1, 1024, &a) == NRS_OK && nrs_folds_relieve(ctx) == NRS_OK && nrs_fold_partial(ctx, -1, 1024, &b) == NRS_OK && a != b ? 0 : 1;
+  bad += nrs_planes_drop(ctx, x) == NRS_OK && nrs_planes_drop(ctx, dy) == NRS_OK ? 0 : 1;
+  ctx->math_mode = mode;
   nrs_folds_end(ctx);
   ctx->device_malloc = real;
+  for (void* q : {(void*)x, (void*)dy, (void*)dw}) bad += nrs_free(ctx, q) == NRS_OK ? 0 : 1;
   bad += nrs_free(ctx, dst) == NRS_OK && nrs_sync(ctx) == NRS_OK ? 0 : 1;
   return bad;
 }

@@ -264,9 +264,9 @@ int run_queue(nrs_ctx* ctx) {
 
 // Memory for partial sums out of the blocks there are, or null.  The blocks start over only when nothing in them is
 // still to be read: no job with sums there is queued, and none is being made (its memory is handed out before the kernel that fills it
-// is launched and the job is submitted, and what comes in between may run the queue).
+// is launched and the job is submitted, and what comes in between may run the queue, or other jobs for the sake of memory).
 float* place(NrsFolds& f, size_t bytes) {
-  if (f.holding == 0 && !f.open) f.chunk = f.used = 0;
+  if (f.holding == 0 && !f.open && !f.relieving) f.chunk = f.used = 0;
   for (; f.chunk < f.chunks.size(); ++f.chunk, f.used = 0)
     if (f.used + bytes <= f.chunks[f.chunk].second) {
       float* p = (float*)((uint8_t*)f.chunks[f.chunk].first + f.used);
@@ -281,6 +281,12 @@ float* place(NrsFolds& f, size_t bytes) {
 
 void nrs_folds_begin(nrs_ctx* ctx) { ctx->folds.active = true; }
 
+static void drop_kept(nrs_ctx* ctx) {
+  for (void* p : ctx->folds.kept) nrs_free(ctx, p);
+  ctx->folds.kept.clear();
+  ctx->folds.kept_bytes = 0;
+}
+
 int nrs_folds_flush(nrs_ctx* ctx) {
   NrsFolds& f = ctx->folds;
   int st = NRS_OK;
@@ -290,14 +296,30 @@ int nrs_folds_flush(nrs_ctx* ctx) {
     if (st == NRS_OK) st = nrs_wgrad_tiles_run(ctx);
   }
   if (st == NRS_OK) st = run_queue(ctx);
-  for (void* p : f.kept) nrs_free(ctx, p);
-  f.kept.clear();
+  drop_kept(ctx);
+  return st;
+}
+
+int nrs_folds_relieve(nrs_ctx* ctx) {
+  NrsFolds& f = ctx->folds;
+  const bool open = f.open, relieving = f.relieving;
+  f.relieving = true;
+  const int st = nrs_folds_flush(ctx);
+  f.relieving = relieving;
+  f.open = open;                  // whose job is being made still has its memory
+  ctx->independent_next = false;  // the kernel launched last is not the one its caller had in mind
   return st;
 }
 
 void nrs_free_after_wgrads(nrs_ctx* ctx, void* p) {
-  if (ctx->folds.waiting.empty()) nrs_free(ctx, p);
-  else if (p) ctx->folds.kept.push_back(p);
+  NrsFolds& f = ctx->folds;
+  if (f.waiting.empty()) {
+    nrs_free(ctx, p);
+  } else if (p) {
+    f.kept.push_back(p);
+    const auto it = ctx->pool.live.find(p);
+    f.kept_bytes += it == ctx->pool.live.end() ? 0 : it->second;
+  }
 }
 
 void nrs_folds_end(nrs_ctx* ctx) {
@@ -308,8 +330,7 @@ void nrs_folds_end(nrs_ctx* ctx) {
   ctx->folds.waiting.clear();
   ctx->folds.waiting_rows.reset();
   ctx->folds.waiting_tiles.reset();
-  for (void* p : ctx->folds.kept) nrs_free(ctx, p);
-  ctx->folds.kept.clear();
+  drop_kept(ctx);
 }
 
 void nrs_folds_free(nrs_ctx* ctx) {

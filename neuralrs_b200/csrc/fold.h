@@ -8,6 +8,11 @@ void nrs_folds_begin(nrs_ctx* ctx);
 int nrs_folds_flush(nrs_ctx* ctx);   // (and the weight gradients that wait, before them)
 // nrs_free, or, while weight gradients wait that may read it, once they have run.
 void nrs_free_after_wgrads(nrs_ctx* ctx, void* p);
+// Launches the weight gradients that wait and lets go of what was kept for them: ahead of another one where more than
+// kNrsKeptBytes are (nrs_wgrad_may_wait's callers), and where the driver has no memory left (at any point of a pass).
+constexpr size_t kNrsKeptBytes = (size_t)1 << 30;
+int nrs_folds_relieve(nrs_ctx* ctx);
+inline int nrs_folds_limit_kept(nrs_ctx* ctx) { return ctx->folds.kept_bytes > kNrsKeptBytes ? nrs_folds_relieve(ctx) : NRS_OK; }
 void nrs_folds_end(nrs_ctx* ctx);    // leaves the collecting mode; what is still queued is dropped (a failed pass)
 void nrs_folds_free(nrs_ctx* ctx);
 // Runs what is queued if it writes any of the `len` floats at `dst`: called by whoever is about to read, overwrite or

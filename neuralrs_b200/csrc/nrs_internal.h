@@ -208,6 +208,8 @@ struct NrsFolds {
   std::vector<std::pair<const float*, size_t>> waiting;
   std::shared_ptr<void> waiting_rows, waiting_tiles;
   std::vector<void*> kept;
+  size_t kept_bytes = 0;
+  bool relieving = false;  // the waiting gradients run for the sake of memory, maybe while a job is being made
 };
 
 struct nrs_ctx {

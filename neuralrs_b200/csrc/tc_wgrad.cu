@@ -546,6 +546,8 @@ int nrs_tc_conv_wgrad(nrs_ctx* ctx, const float* x, const float* dy, float* dw, 
   job.out_cols = out_cols;
   job.can_be_direct = can_be_direct;
   if (!waits) return launch_wgrad<1>(ctx, &job, 1, may_overlap);
+  st = nrs_folds_limit_kept(ctx);
+  if (st != NRS_OK) return st;
   NrsFolds& f = ctx->folds;
   if (!f.waiting_tiles) f.waiting_tiles = std::make_shared<std::vector<WgradJob>>();
   static_cast<std::vector<WgradJob>*>(f.waiting_tiles.get())->push_back(job);

@@ -435,6 +435,8 @@ int nrs_tc_conv_wgrad_rows(nrs_ctx* ctx, const float* x, const float* dy, float*
   job.dw = dw;
   job.accumulate = accumulate;
   if (nrs_wgrad_may_wait(ctx, dy_hi, x_hi)) {
+    st = nrs_folds_limit_kept(ctx);
+    if (st != NRS_OK) return st;
     NrsFolds& f = ctx->folds;
     if (!f.waiting_rows) f.waiting_rows = std::make_shared<std::vector<RowJob>>();
     static_cast<std::vector<RowJob>*>(f.waiting_rows.get())->push_back(job);
