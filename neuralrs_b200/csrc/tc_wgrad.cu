@@ -319,6 +319,7 @@ namespace {
 struct WgradJob {
   WgradEntry e;
   int planes;
+  long most;   // tiles of an accumulation chain
   float* dw;
   int accumulate, out_cols;
   bool can_be_direct;
@@ -431,6 +432,15 @@ int nrs_tc_conv_wgrad(nrs_ctx* ctx, const float* x, const float* dy, float* dw, 
   const NrsPlanes *dy_ready = nrs_planes_find(ctx, dy, split3), *x_ready = nrs_planes_find(ctx, x, split3);
   const bool waits = dy_ready && x_ready && nrs_wgrad_may_wait(ctx, dy_ready->hi, x_ready->hi);
   int tps = 0;   // pixel tiles per CTA
+  // The split that fills the GPU with this product alone, and bounds the accumulation chain in 3xTF32 mode.
+  auto alone = [&](const WgradParams& q) {
+    const int most = (int)std::min(max_tiles(q, planes), 1L << 30);
+    int min_tiles = 512 / q.kp;   // amortise the prologue and the partial-tile store
+    // ... unless that leaves most of the GPU idle
+    while (min_tiles > 4 && (long)(q.n_tiles / min_tiles) * q.ctas < ctx->sm_count / 2) min_tiles /= 2;
+    if (min_tiles > most) min_tiles = most;
+    return tc::plan_units_per_cta(ctx->sm_count, q.ctas, q.n_tiles, min_tiles, most, 8);
+  };
   if (waits) {   // shared out with the others; wide column blocks, which read the least
     if (tap_cols > kMaxN) {
       p.col_blocks = (tap_cols + kMaxN - 1) / kMaxN;
@@ -482,13 +492,7 @@ int nrs_tc_conv_wgrad(nrs_ctx* ctx, const float* x, const float* dy, float* dw, 
     if (tps == 0 || !box(&p)) return NRS_ERR_UNSUPPORTED;
   } else {
     if (!box(&p)) return NRS_ERR_UNSUPPORTED;
-    // pixel split: fill the GPU, and bound the accumulation chain in 3xTF32 mode
-    const int ctas_per_split = p.ctas, most = (int)std::min(max_tiles(p, planes), 1L << 30);
-    int min_tiles = 512 / p.kp;   // amortise the prologue and the partial-tile store
-    // ... unless that leaves most of the GPU idle
-    while (min_tiles > 4 && (long)(p.n_tiles / min_tiles) * ctas_per_split < ctx->sm_count / 2) min_tiles /= 2;
-    if (min_tiles > most) min_tiles = most;
-    tps = tc::plan_units_per_cta(ctx->sm_count, ctas_per_split, p.n_tiles, min_tiles, most, 8);
+    tps = alone(p);
   }
   p.tiles_per_split = tps;
   if ((long)p.ctas * ((p.n_tiles + tps - 1) / tps) > 2147483647L) return NRS_ERR_UNSUPPORTED;
@@ -541,6 +545,7 @@ int nrs_tc_conv_wgrad(nrs_ctx* ctx, const float* x, const float* dy, float* dw, 
   p.range_x = nrs_range_of(ctx, x_hi);
   job.e = WgradEntry{maps[0], maps[1], maps[2], maps[3], p};
   job.planes = planes;
+  job.most = split3 ? max_tiles(p, planes) : std::max((long)alone(p), (long)tc::kMaxChainK / p.kp);   // (see wgrad_queue.h)
   job.dw = dw;
   job.accumulate = accumulate;
   job.out_cols = out_cols;
@@ -567,7 +572,7 @@ int nrs_wgrad_tiles_run(nrs_ctx* ctx) {
     double least = 0.0;
     for (e = i; e < all->size() && (int)(e - i) < kWgBatch; ++e) {
       const WgradParams& p = (*all)[e].e.p;
-      const long most = max_tiles(p, planes);
+      const long most = (*all)[e].most;
       const double bytes = (double)split_floats(p) * sizeof(float), need = bytes * ((p.n_tiles + most - 1) / most);
       if ((*all)[e].planes != planes || (e > i && least + need > kMostPartial)) break;
       least += need;

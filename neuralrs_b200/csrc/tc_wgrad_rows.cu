@@ -294,6 +294,7 @@ bool plan_row_tile(RowParams* p, int h, int w, int planes) {
 struct RowJob {
   RowEntry e;
   int planes;
+  long most;   // tiles of an accumulation chain
   float* dw;
   int accumulate;
 };
@@ -432,6 +433,7 @@ int nrs_tc_conv_wgrad_rows(nrs_ctx* ctx, const float* x, const float* dy, float*
   p.range_x = nrs_range_of(ctx, x_hi);
   e.p = p;
   job.planes = planes;
+  job.most = split3 ? max_tiles(p, planes) : std::max((long)p.tiles_per_split, (long)tc::kMaxChainK / p.P);   // (see wgrad_queue.h)
   job.dw = dw;
   job.accumulate = accumulate;
   if (nrs_wgrad_may_wait(ctx, dy_hi, x_hi)) {
@@ -458,7 +460,7 @@ int nrs_wgrad_rows_run(nrs_ctx* ctx) {
     double least = 0.0;
     for (e = i; e < all->size() && (int)(e - i) < kRowBatch; ++e) {
       const RowParams& p = (*all)[e].e.p;
-      const long most = max_tiles(p, planes);
+      const long most = (*all)[e].most;
       const double bytes = (double)split_floats(p) * sizeof(float), umma = (planes == 2 ? 3 : 1) * (p.chunk / p.wb) * kTaps * p.wb * 0.5;
       const double need = bytes * ((p.n_tiles + most - 1) / most);
       if ((*all)[e].planes != planes || (e > i && least + need > kMostPartial)) break;

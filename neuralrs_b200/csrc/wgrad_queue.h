@@ -4,7 +4,8 @@
 // pixels among all SMs, pays a launch, a ramp and a partial tile of 98 KB from every SM, and the partial tiles are read again
 // by the folds.  Nothing in a pass reads a parameter's gradient, so the layers' products wait until its end and share one
 // launch: every CTA takes a longer run of pixels of one layer, and there are as many partial tiles as SMs in all instead of
-// per layer.  Collected while folds are (NrsFolds::active), where both operands' planes are there and stay: their owners
+// per layer.  No accumulation chain becomes longer for it than it may be: in 3xTF32 the mode's limit, in TF32, which has none
+// of its own, what the product would have alone, or tc::kMaxChainK values.  Collected while folds are (NrsFolds::active), where both operands' planes are there and stay: their owners
 // release them through nrs_free_after_wgrads.
 #pragma once
 

@@ -340,3 +340,26 @@ def test_embedding_gradient_in_token_order(gpu_ctx, tokens, vocab, dim):
     got = out.get()
     starts = np.arange(0, tokens, 1024)   # (the walk keeps one sum through all of its lists)
     assert len(starts) and np.array_equal(got, ref)
+
+
+def test_collected_chains_in_tf32(gpu_ctx):
+    """Sixteen weight gradients over 2^17 rows in one launch: no accumulation chain becomes longer than 4096 rows for it.  All
+    values are positive and exact in TF32, so what is lost is what the tensor core cuts: at most 2^-23 of the partial sum at each
+    step of 8 rows, half of that over a chain whose sum grows evenly; the chains' sums are added up in f32."""
+    rows, d, n = 1 << 17, 64, 16
+    rng = np.random.default_rng(9)
+    x, seed = ((1.0 + rng.integers(0, 1024, (rows, d)) / 1024.0).astype(np.float32) for _ in range(2))
+    ref = x.astype(np.float64).T @ seed.astype(np.float64)
+    gpu_ctx.set_math_mode(_lib.MATH_TF32)
+    try:
+        gx = on_gpu(x)   # (its gradient is wanted: the planes of the incoming one serve both products, and the second may wait)
+        gw = [on_gpu((0.1 * rng.standard_normal((d, d))).astype(np.float32)) for _ in range(n)]
+        out = graph.matmul(gx, gw[0])
+        for w in gw[1:]:
+            out = graph.add(out, graph.matmul(gx, w))
+        gpu.set_grad(out, seed)
+        backward_graph(out)
+        for w in gw:
+            assert rel_l2(gpu.read_grad(w), ref) <= (4096 / 8 / 2 + rows / 4096 + 8) * 2.0**-23
+    finally:
+        gpu_ctx.set_math_mode(_lib.MATH_3XTF32)
