@@ -108,6 +108,21 @@ int nrs_range_new(nrs_ctx* ctx, NrsRange** out) {
   NrsRangePool& pool = ctx->range_pool;
   *out = nullptr;
   constexpr size_t kBytes = NrsRangePool::kPerPage * sizeof(NrsRange);
+  if (pool.captured_left == 0) {   // (ahead of the first capture: the driver may refuse memory during one)
+    void* mem = nullptr;
+    const int st = nrs_alloc(ctx, NrsRangePool::kCaptured * sizeof(NrsRange), 0, &mem);
+    if (st != NRS_OK) return st;
+    pool.captured = (NrsRange*)mem;
+    pool.captured_left = NrsRangePool::kCaptured;
+  }
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  NRS_CUDA(ctx, cudaStreamIsCapturing(ctx->stream, &capturing));
+  if (capturing != cudaStreamCaptureStatusNone) {
+    *out = pool.captured++;
+    --pool.captured_left;
+    NRS_CUDA(ctx, cudaMemsetAsync(*out, 0, sizeof(NrsRange), ctx->stream));
+    return NRS_OK;
+  }
   if (pool.pages.empty() || pool.pages[pool.current].used == NrsRangePool::kPerPage) {
     size_t next = 0;
     while (next < pool.pages.size() && pool.pages[next].live > 0) ++next;
@@ -124,10 +139,6 @@ int nrs_range_new(nrs_ctx* ctx, NrsRange** out) {
   }
   NrsRangePool::Page& pg = pool.pages[pool.current];
   *out = pg.mem + pg.used++;
-  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-  NRS_CUDA(ctx, cudaStreamIsCapturing(ctx->stream, &capturing));
-  if (capturing != cudaStreamCaptureStatusNone)   // a replay meets the range as the last one left it
-    NRS_CUDA(ctx, cudaMemsetAsync(*out, 0, sizeof(NrsRange), ctx->stream));
   ++pg.live;
   return NRS_OK;
 }

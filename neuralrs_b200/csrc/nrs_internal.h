@@ -59,12 +59,16 @@ struct NrsRange {
   float bound, top;
   float pad[6];   // a sector each
 };
-// Ranges are cut from pages that are zeroed as a whole, on the context's stream, once all ranges of a page are back.
+// Ranges are cut from pages that are zeroed as a whole, on the context's stream, once all ranges of a page are back.  While
+// the stream is being captured they come from memory apart: a graph may be replayed at any time, so its ranges are cleared
+// one by one, by the graph itself, and nobody else ever gets them.
 struct NrsRangePool {
-  static constexpr int kPerPage = 256;
+  static constexpr int kPerPage = 256, kCaptured = 1024;
   struct Page { NrsRange* mem; int used, live; };
   std::vector<Page> pages;
   size_t current = 0;
+  NrsRange* captured = nullptr;
+  int captured_left = 0;
 };
 
 struct NrsProfRecord {

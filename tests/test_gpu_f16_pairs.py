@@ -1,6 +1,8 @@
 """3xTF32 products as f16 pairs (one power-of-two exponent a tensor) and the kernels around them: magnitudes and ranges,
 zeros, infinities, many live ranges; convolutions by slabs at the edges of their tiles; weight gradients in column blocks, by
 slabs and collected to the end of a pass; the small kernels' second stages.  Against f64."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -363,3 +365,47 @@ def test_collected_chains_in_tf32(gpu_ctx):
             assert rel_l2(gpu.read_grad(w), ref) <= (4096 / 8 / 2 + rows / 4096 + 8) * 2.0**-23
     finally:
         gpu_ctx.set_math_mode(_lib.MATH_3XTF32)
+
+
+def test_ranges_of_a_captured_graph(gpu_ctx):
+    """A graph of convolutions, replayed between eager work: its ranges start from nothing each time, and the tensors that were
+    staged after its capture keep theirs."""
+    n, ci, h, co, layers = 2, 32, 6, 32, 150
+    args = (n, ci, h, h, co, 3, 3, 1, 1, 0)
+    rng = np.random.default_rng(12)
+    x = rng.standard_normal((n, ci, h, h)).astype(np.float32)
+    wt = (rng.standard_normal((co, ci, 3, 3)) / 17).astype(np.float32)
+    cu, ctx = ctypes.CDLL("libcuda.so.1"), cuda.Context(0)
+    try:
+        wd, bd = Dev(ctx, wt), Dev(ctx, np.zeros(co, np.float32))
+        xd, ys = Dev(ctx, x), [Dev(ctx, shape=(n, co, h, h)) for _ in range(layers)]
+        eager = Dev(ctx, shape=(n, co, h, h))
+
+        def expect(values):
+            call(ctx, "nrs_h2d", xd, _lib.VP(values.ctypes.data), values.nbytes)
+            call(ctx, "nrs_conv2d_fwd", xd, wd, bd, eager, *args)
+            return eager.get()
+
+        want = {s: expect(np.ascontiguousarray(x * np.float32(s))) for s in (1.0, 1e6, 1e-6)}
+        stream, graph_h, exec_h = ctypes.c_void_p(ctx._l.nrs_get_stream(ctx.h)), ctypes.c_void_p(), ctypes.c_void_p()
+        assert cu.cuStreamBeginCapture_v2(stream, 2) == 0      # relaxed
+        for y in ys:
+            call(ctx, "nrs_conv2d_fwd", xd, wd, bd, y, *args)
+        assert cu.cuStreamEndCapture(stream, ctypes.byref(graph_h)) == 0
+        assert cu.cuGraphInstantiateWithFlags(ctypes.byref(exec_h), graph_h, ctypes.c_ulonglong(0)) == 0
+        scaled = [(2.0**i, Dev(ctx, (x * np.float32(2.0**i)).astype(np.float32))) for i in range(-20, 20)]
+        scaled += [(1.0, Dev(ctx, x)) for _ in range(260)]      # (more than a page of ranges)
+        for _, t in scaled:
+            call(ctx, "nrs_planes_cache", t, n, ci, h, h)
+        for s, ref in list(want.items()) * 2:
+            v = np.ascontiguousarray(x * np.float32(s))
+            call(ctx, "nrs_h2d", xd, _lib.VP(v.ctypes.data), v.nbytes)
+            assert cu.cuGraphLaunch(exec_h, stream) == 0
+            ctx.sync()
+            assert all(np.array_equal(ys[i].get(), ref) for i in (0, 1, layers // 2, layers - 1)), s
+        for f, t in scaled:
+            call(ctx, "nrs_conv2d_fwd", t, wd, bd, eager, *args)
+            assert np.array_equal(eager.get(), want[1.0] * np.float32(f)), f
+        assert cu.cuGraphExecDestroy(exec_h) == 0 and cu.cuGraphDestroy(graph_h) == 0
+    finally:
+        ctx.close()
