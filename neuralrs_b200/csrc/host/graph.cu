@@ -218,7 +218,7 @@ static bool stage_planes_2d(nrs_ctx* ctx, const float* src, size_t rows, size_t 
   const int ld = nrs_plane_ld((int)cols);
   *hi = dplane(ctx, rows * ld);
   if (split) *lo = dplane(ctx, rows * ld);
-  check(ctx, nrs_tc_stage(ctx, src, *hi, *lo, (int)rows, (int)cols, ld, 1, 0, 0, false, nullptr, known, also, also_count, also_range));
+  check(ctx, nrs_tc_stage(ctx, src, *hi, *lo, (int)rows, (int)cols, ld, 1, 0, 0, false, known, also, also_count, also_range));
   NrsPlanes pl{*hi, *lo, split ? 1 : 0};
   pl.rows = (int)rows;
   pl.cols = (int)cols;

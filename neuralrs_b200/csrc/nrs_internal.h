@@ -341,12 +341,15 @@ extern "C" int nrs_layernorm_bwd_planes(nrs_ctx* ctx, const float* g, const floa
                                         int* sums_rows /*how many rows of it were written; 0: none*/);
 static inline int nrs_layernorm_sum_rows(const nrs_ctx* ctx) { return 4 * ctx->sm_count; }
 // Operand planes of a batch of [rows][K] matrices (tc_stage.cu); see tc_mainloop.cuh for the layouts.  3xTF32: the range
-// of `hi` is renewed and measured, in the same launch for small tensors, unless the caller has one: `measured` becomes the
-// planes' own, `known` bounds the source's values (NrsRange::top).
+// of `hi` is renewed and measured, in the same launch for small tensors, unless the caller knows a bound of the source's
+// values (NrsRange::top).
 int nrs_tc_stage(nrs_ctx* ctx, const float* src, float* hi, float* lo, int rows, int K, int ldk, int batch,
-                 size_t src_bstride, size_t dst_bstride, bool src_k_by_rows, NrsRange* measured = nullptr, const NrsRange* known = nullptr,
+                 size_t src_bstride, size_t dst_bstride, bool src_k_by_rows, const NrsRange* known = nullptr,
                  const float* also = nullptr /*rows as stored, f16 pairs, one matrix: a tensor to measure in the same launch*/,
                  size_t also_count = 0, NrsRange* also_range = nullptr);
+// The same of `count` matrices that lie anywhere, with one range for all of them; four to a launch, measured and staged.
+int nrs_tc_stage_each(nrs_ctx* ctx, const float* const* src, int count, float* hi, float* lo, int rows, int K, int ldk, size_t dst_bstride,
+                      bool src_k_by_rows);
 // NHWC planes of an NCHW tensor [n][c][hw], pixel stride nrs_plane_ld(c) floats (zeros between c and there).
 // chan_partial (hw > 1): [nrs_batchnorm_tiles(n, hw)][c] channel sums of the pixels of each tile.
 int nrs_tc_stage_image(nrs_ctx* ctx, const float* src, float* hi, float* lo, int n, int c, int hw, float* chan_partial = nullptr,

@@ -454,15 +454,10 @@ int nrs_tc_gemm_weights(nrs_ctx* ctx, int reduce, int count, int m, int n, int k
     const int ld = nrs_plane_ld(k);
     const size_t plane = (size_t)n * ld;
     void *hi = nullptr, *lo = nullptr;
-    NrsRange* range = nullptr;
     st = nrs_ws_planes(ctx, NRS_WS_B, plane * count, split, &hi, &lo);
-    if (split && st == NRS_OK) st = nrs_range_renew(ctx, hi, &range);   // one for all of them
-    for (int i = 0; split && i < count && st == NRS_OK; ++i) st = nrs_absmax(ctx, w[i], (size_t)n * k, range);
-    for (int i = 0; i < count && st == NRS_OK; ++i)
-      st = nrs_tc_stage(ctx, w[i], nrs_plane_at((float*)hi, i * plane, split), split ? nrs_plane_at((float*)lo, i * plane, true) : nullptr, n, k, ld, 1,
-                        0, 0, !reduce, range);
+    if (st == NRS_OK) st = nrs_tc_stage_each(ctx, w, count, (float*)hi, (float*)lo, n, k, ld, plane, !reduce);
     if (st != NRS_OK) return st;
-    B = Operand{(const float*)hi, (const float*)lo, ld, k, plane, range};
+    B = Operand{(const float*)hi, (const float*)lo, ld, k, plane, nrs_range_of(ctx, hi)};
   }
   const int cols = reduce ? n : count * n, kk = reduce ? count * k : k;
   GemmPolicy<false> pol{c, nullptr, NRS_ACT_NONE, beta, m, cols, (size_t)m * cols, false, {}, 0.0f, reduce ? 0 : n, reduce ? k : 0};

@@ -11,11 +11,13 @@ namespace {
 
 // Largest finite magnitude of n values into r->top.  A read of the tensor, from HBM where it exceeds L2.
 struct Measured { const float* src; size_t n; NrsRange* r; };
+constexpr int kSources = 4;   // tensors of one launch
+struct MeasuredSet { Measured m[kSources]; };
 __global__ void __launch_bounds__(256)
-absmax_kernel(const Measured m0, const Measured m1 /*blockIdx.y == 1*/) {
+absmax_kernel(const __grid_constant__ MeasuredSet set) {
   NRS_PDL_PROLOGUE();
   __shared__ uint32_t part[8];
-  const Measured& m = blockIdx.y == 0 ? m0 : m1;
+  const Measured& m = set.m[blockIdx.y];
   const float* __restrict__ src = m.src;
   const size_t n = m.n;
   const size_t head = min(n, (size_t)(((16 - (reinterpret_cast<uintptr_t>(src) & 15)) & 15) / 4)), quads = (n - head) / 4;
@@ -85,10 +87,19 @@ __device__ __forceinline__ void measure_also(const Also& a, unsigned first) {
   pr::report_block(a.range, top);
 }
 
+// Where the matrices of a batch lie: at equal distances, or (weights that meet in one product) each by itself.
+struct Sources {
+  const float* first;
+  size_t stride;
+  const float* each[kSources];   // null: by the stride
+  Sources(const float* src, size_t bstride) : first(src), stride(bstride), each{} {}
+  __device__ __forceinline__ const float* at(int b) const { return each[0] ? each[b] : first + b * stride; }
+};
+
 template <bool SPLIT>
 __global__ void __launch_bounds__(256)
-stage_rows_kernel(const float* __restrict__ src, float* __restrict__ hi, float* __restrict__ lo, int rows, int K,
-                  int ldk, size_t src_bstride, size_t dst_bstride, const NrsFastDiv div_q, const Bound bound, const Also also) {
+stage_rows_kernel(const __grid_constant__ Sources sources, float* __restrict__ hi, float* __restrict__ lo, int rows, int K,
+                  int ldk, size_t dst_bstride, const NrsFastDiv div_q, const Bound bound, const Also also) {
   NRS_PDL_PROLOGUE();
   const unsigned blocks = gridDim.x - also.blocks;
   if (SPLIT && blockIdx.x >= blocks) {
@@ -97,7 +108,7 @@ stage_rows_kernel(const float* __restrict__ src, float* __restrict__ hi, float* 
   }
   const float scale = open_range<SPLIT>(bound);
   const int b = blockIdx.y;
-  src += b * src_bstride;
+  const float* __restrict__ src = sources.at(b);
   const size_t dst = b * dst_bstride;
   const int q = ldk / 4;
   const size_t total4 = (size_t)rows * q;
@@ -122,13 +133,13 @@ stage_rows_kernel(const float* __restrict__ src, float* __restrict__ hi, float* 
 
 template <bool SPLIT>
 __global__ void __launch_bounds__(256)
-stage_transpose_kernel(const float* __restrict__ src, float* __restrict__ hi, float* __restrict__ lo, int rows, int K,
-                       int ldk, size_t src_bstride, size_t dst_bstride, const Bound bound) {
+stage_transpose_kernel(const __grid_constant__ Sources sources, float* __restrict__ hi, float* __restrict__ lo, int rows, int K,
+                       int ldk, size_t dst_bstride, const Bound bound) {
   NRS_PDL_PROLOGUE();
   __shared__ float tile[32][33];
   const float scale = open_range<SPLIT>(bound);
   const int b = blockIdx.z;
-  src += b * src_bstride;
+  const float* __restrict__ src = sources.at(b);
   const size_t dst = b * dst_bstride;
   const int r0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
@@ -419,13 +430,17 @@ static unsigned absmax_blocks(const nrs_ctx* ctx, size_t count) {
 }
 int nrs_absmax(nrs_ctx* ctx, const float* src, size_t count, NrsRange* r) {
   if (count == 0) return NRS_OK;
-  const Measured m{src, count, r};
-  NRS_PDL_LAUNCH(absmax_kernel, absmax_blocks(ctx, count), 256, 0, ctx->stream, m, m);
+  MeasuredSet set{};
+  set.m[0] = Measured{src, count, r};
+  NRS_PDL_LAUNCH(absmax_kernel, absmax_blocks(ctx, count), 256, 0, ctx->stream, set);
   NRS_LAUNCHED(ctx);
   return NRS_OK;
 }
 int nrs_absmax2(nrs_ctx* ctx, const float* a, size_t na, NrsRange* ra, const float* b, size_t nb, NrsRange* rb) {
-  NRS_PDL_LAUNCH(absmax_kernel, dim3(absmax_blocks(ctx, na > nb ? na : nb), 2), 256, 0, ctx->stream, Measured{a, na, ra}, Measured{b, nb, rb});
+  MeasuredSet set{};
+  set.m[0] = Measured{a, na, ra};
+  set.m[1] = Measured{b, nb, rb};
+  NRS_PDL_LAUNCH(absmax_kernel, dim3(absmax_blocks(ctx, na > nb ? na : nb), 2), 256, 0, ctx->stream, set);
   NRS_LAUNCHED(ctx);
   return NRS_OK;
 }
@@ -506,15 +521,8 @@ int nrs_tc_stage_masked(nrs_ctx* ctx, int mode, const float* g, const float* y, 
   return NRS_OK;
 }
 
-int nrs_tc_stage(nrs_ctx* ctx, const float* src, float* hi, float* lo, int rows, int K, int ldk, int batch,
-                 size_t src_bstride, size_t dst_bstride, bool src_k_by_rows, NrsRange* measured, const NrsRange* known,
-                 const float* also, size_t also_count, NrsRange* also_range) {
-  if (rows <= 0 || K <= 0 || batch <= 0) return NRS_OK;
-  Bound bound{measured ? &measured->top : nullptr, src, 0, measured};
-  if (lo && !measured) {
-    const int st = open_planes(ctx, hi, src, batch == 1 ? (size_t)rows * K : src_bstride * (batch - 1) + (size_t)rows * K, known, &bound);
-    if (st != NRS_OK) return st;
-  }
+static int stage(nrs_ctx* ctx, const Sources& src, float* hi, float* lo, int rows, int K, int ldk, int batch, size_t dst_bstride, bool src_k_by_rows,
+                 const Bound& bound, const float* also, size_t also_count, NrsRange* also_range) {
   if (!src_k_by_rows) {
     size_t blocks = ((size_t)rows * (ldk / 4) + 255) / 256;
     const size_t cap = (size_t)ctx->sm_count * 16;
@@ -523,15 +531,54 @@ int nrs_tc_stage(nrs_ctx* ctx, const float* src, float* hi, float* lo, int rows,
     Also more{};
     if (also && lo && batch == 1) more = Also{also, also_count, also_range, absmax_blocks(ctx, also_count)};
     dim3 grid((unsigned)blocks + more.blocks, (unsigned)batch);
-    if (lo) NRS_PDL_LAUNCH((stage_rows_kernel<true>), grid, 256, 0, ctx->stream, src, hi, lo, rows, K, ldk, src_bstride, dst_bstride, NrsFastDiv(ldk / 4), bound, more);
-    else NRS_PDL_LAUNCH((stage_rows_kernel<false>), grid, 256, 0, ctx->stream, src, hi, nullptr, rows, K, ldk, src_bstride, dst_bstride, NrsFastDiv(ldk / 4), bound, more);
+    if (lo) NRS_PDL_LAUNCH((stage_rows_kernel<true>), grid, 256, 0, ctx->stream, src, hi, lo, rows, K, ldk, dst_bstride, NrsFastDiv(ldk / 4), bound, more);
+    else NRS_PDL_LAUNCH((stage_rows_kernel<false>), grid, 256, 0, ctx->stream, src, hi, nullptr, rows, K, ldk, dst_bstride, NrsFastDiv(ldk / 4), bound, more);
   } else {
     dim3 grid((unsigned)((rows + 31) / 32), (unsigned)((ldk + 31) / 32), (unsigned)batch);
     if (grid.y > 65535 || grid.z > 65535) return NRS_ERR_UNSUPPORTED;
-    if (lo) NRS_PDL_LAUNCH((stage_transpose_kernel<true>), grid, 256, 0, ctx->stream, src, hi, lo, rows, K, ldk, src_bstride, dst_bstride, bound);
-    else NRS_PDL_LAUNCH((stage_transpose_kernel<false>), grid, 256, 0, ctx->stream, src, hi, nullptr, rows, K, ldk, src_bstride, dst_bstride, bound);
+    if (lo) NRS_PDL_LAUNCH((stage_transpose_kernel<true>), grid, 256, 0, ctx->stream, src, hi, lo, rows, K, ldk, dst_bstride, bound);
+    else NRS_PDL_LAUNCH((stage_transpose_kernel<false>), grid, 256, 0, ctx->stream, src, hi, nullptr, rows, K, ldk, dst_bstride, bound);
   }
   NRS_LAUNCHED(ctx);
+  return NRS_OK;
+}
+
+int nrs_tc_stage(nrs_ctx* ctx, const float* src, float* hi, float* lo, int rows, int K, int ldk, int batch,
+                 size_t src_bstride, size_t dst_bstride, bool src_k_by_rows, const NrsRange* known,
+                 const float* also, size_t also_count, NrsRange* also_range) {
+  if (rows <= 0 || K <= 0 || batch <= 0) return NRS_OK;
+  Bound bound{};
+  if (lo) {
+    const int st = open_planes(ctx, hi, src, batch == 1 ? (size_t)rows * K : src_bstride * (batch - 1) + (size_t)rows * K, known, &bound);
+    if (st != NRS_OK) return st;
+  }
+  return stage(ctx, Sources(src, src_bstride), hi, lo, rows, K, ldk, batch, dst_bstride, src_k_by_rows, bound, also, also_count, also_range);
+}
+
+int nrs_tc_stage_each(nrs_ctx* ctx, const float* const* src, int count, float* hi, float* lo, int rows, int K, int ldk, size_t dst_bstride,
+                      bool src_k_by_rows) {
+  if (rows <= 0 || K <= 0 || count <= 0) return NRS_OK;
+  NrsRange* range = nullptr;
+  if (lo) {
+    const int st = nrs_range_renew(ctx, hi, &range);
+    if (st != NRS_OK) return st;
+    for (int i = 0; i < count; i += kSources) {
+      MeasuredSet set{};
+      const int n = std::min(count - i, kSources);
+      for (int k = 0; k < n; ++k) set.m[k] = Measured{src[i + k], (size_t)rows * K, range};
+      NRS_PDL_LAUNCH(absmax_kernel, dim3(absmax_blocks(ctx, (size_t)rows * K), n), 256, 0, ctx->stream, set);
+      NRS_LAUNCHED(ctx);
+    }
+  }
+  const Bound bound{range ? &range->top : nullptr, nullptr, 0, range};
+  for (int i = 0; i < count; i += kSources) {
+    Sources s(nullptr, 0);
+    const int n = std::min(count - i, kSources);
+    for (int k = 0; k < n; ++k) s.each[k] = src[i + k];
+    const int st = stage(ctx, s, nrs_plane_at(hi, i * dst_bstride, lo != nullptr), lo ? nrs_plane_at(lo, i * dst_bstride, true) : nullptr, rows, K, ldk, n,
+                         dst_bstride, src_k_by_rows, bound, nullptr, 0, nullptr);
+    if (st != NRS_OK) return st;
+  }
   return NRS_OK;
 }
 
@@ -539,7 +586,7 @@ int nrs_tc_stage_image(nrs_ctx* ctx, const float* src, float* hi, float* lo, int
                        const NrsRange* known) {
   if (n <= 0 || c <= 0 || hw <= 0) return NRS_OK;
   const int ld = nrs_plane_ld(c);
-  if (hw == 1) return nrs_tc_stage(ctx, src, hi, lo, n, c, ld, 1, 0, 0, false, nullptr, known);   // already pixel-major: split only
+  if (hw == 1) return nrs_tc_stage(ctx, src, hi, lo, n, c, ld, 1, 0, 0, false, known);   // already pixel-major: split only
   if ((size_t)n * hw > 0x7fffffffu) return NRS_ERR_UNSUPPORTED;
   const img::Grid g(n, c, hw);
   Bound bound{};
