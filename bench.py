@@ -469,23 +469,6 @@ def attention_microbench(ctx, stream, iters=20):
             "fwd_tflops": flop / (fwd / 1e3) / 1e12, "bwd_tflops": 2.5 * flop / (bwd / 1e3) / 1e12}
 
 
-# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of the dominant kernel of a family from
-# the `ncu --set full` captures summarised under profiles/: (bytes, per-GPU batch of the capture,
-# kernel).  Traffic of these kernels is proportional to the pixel count, so it is scaled to the
-# per-GPU batch of this run.  (None of the kernels as they are now has been captured.)
-NCU_TRAFFIC = {
-}
-
-
-def ncu_traffic(workload, math, family, per_gpu_batch):
-    hit = NCU_TRAFFIC.get((workload, math, family))
-    if not hit:
-        return {"traffic": None}
-    nbytes, cap_batch, kernel = hit
-    return {"traffic": nbytes * per_gpu_batch / cap_batch, "traffic_unit": "bytes per launch", "traffic_kernel": kernel,
-            "traffic_source": f"ncu --set full capture at per-GPU batch {cap_batch} (profiles/), scaled by the pixel count"}
-
-
 def cpu_baseline_entry(r):
     return {"value": r["value"], "unit": "samples/s", "cores": r["cores"], "kind": "port", "sample": r["sample"]}
 
@@ -661,11 +644,15 @@ def run_ours(args):
 
     for i in range(max(3, args.warmup)):
         dev_step(i)
-    _lib.check(ctx.h, l.nrs_profile_reset(ctx.h))
     # The per-family CUDA-event brackets sit between kernels, where they defeat the chaining of
     # consecutive launches; they are switched on for every fourth timed step only (the first
-    # included), and the family figures are scaled to the bracketed steps.
+    # included), and the family figures are scaled to the bracketed steps.  (Their events are made
+    # in two steps ahead of the timing.)
     bracket_every = 4
+    _lib.check(ctx.h, l.nrs_profile_enable(ctx.h, 1))
+    for i in range(2):
+        dev_step(i)
+    _lib.check(ctx.h, l.nrs_profile_reset(ctx.h))
     bracketed = len(range(0, args.steps, bracket_every)) * N_WINDOWS
 
     def dev_step_bracketed(i):
@@ -731,7 +718,7 @@ def run_ours(args):
         pairs = args.math == "3xtf32"        # three products of f16 pairs at the bf16 rate; TF32 runs at half of it
         tf32_peak = peaks["bf16_sustained"] / (1.0 if pairs else 2.0)
         umma = C.c_double()
-        _lib.check(ctx.h, l.nrs_measure_tf32_umma_peak(ctx.h, C.byref(umma)))
+        _lib.check(ctx.h, (l.nrs_measure_f16_umma_peak if pairs else l.nrs_measure_tf32_umma_peak)(ctx.h, C.byref(umma)))
         contraction_ms = sum(prof[k]["ms"] for k in contractions)
         contraction_work = sum(prof[k]["work"] for k in contractions)
         adam = prof["adamw"]
@@ -770,15 +757,15 @@ def run_ours(args):
             "clocks": clk.summary(),
             "roofline": {"bound": "tensor", "kernel": fam, "achieved": achieved, "peak": tf32_peak, "unit": "TFLOP/s",
                          "frac": achieved / tf32_peak if tf32_peak else None,
-                         **ncu_traffic(args.workload, args.math, fam, batch),
+                         "traffic": None,
                          "peak_source": f"{peaks['source']}: sustained bf16 cuBLAS{'' if pairs else ' / 2'} (f16 pairs run at the bf16 rate, "
                                         f"dense TF32 at half of it); {args.math} issues {issue:.0f}x the algorithmic FLOP counted in `achieved`",
                          "issued_tflops": achieved * issue,
                          "frac_issued_of_peak": achieved * issue / tf32_peak if tf32_peak else None,
-                         "tf32_umma_peak_tflops": umma.value,
+                         "umma_peak_tflops": umma.value,
                          "frac_issued_of_umma_peak": achieved * issue / umma.value if umma.value else None,
-                         "tf32_umma_peak_source": "measured in this run: back-to-back tcgen05.mma.kind::tf32 128x256x8 from "
-                                                  "shared memory on every SM (nrs_measure_tf32_umma_peak)",
+                         "umma_peak_source": "measured in this run: back-to-back tcgen05.mma.kind::%s from shared memory on every SM "
+                                             "(nrs_measure_%s_umma_peak)" % (("f16 128x256x16", "f16") if pairs else ("tf32 128x256x8", "tf32")),
                          "launch_ms_avg": f["ms"] / f["calls"] if f["calls"] else None, "calls": f["calls"],
                          "all_contractions_tflops": (contraction_work / (contraction_ms / 1e3) / 1e12) if contraction_ms else None,
                          "families_ms_per_step": {k: prof[k]["ms"] / bracketed for k in prof},

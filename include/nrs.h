@@ -127,6 +127,8 @@ int nrs_selftest_memory_pressure(nrs_ctx* ctx);
  * for a few milliseconds; the result is what the contraction kernels' tensor-core roofline is
  * quoted against.  Waits for the stream. */
 int nrs_measure_tf32_umma_peak(nrs_ctx* ctx, double* tflops_out);
+/* The same of tcgen05.mma.kind::f16 (128 x 256 x 16), which the products of 3xTF32 are issued as. */
+int nrs_measure_f16_umma_peak(nrs_ctx* ctx, double* tflops_out);
 
 int nrs_profile_enable(nrs_ctx* ctx, int on);
 int nrs_profile_reset(nrs_ctx* ctx);

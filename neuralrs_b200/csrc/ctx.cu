@@ -231,6 +231,7 @@ NrsProfScope::NrsProfScope(nrs_ctx* c, int kind, double work) : ctx(c) {
   if (!c || !c->profiling) return;
   rec.kind = kind;
   rec.work = work;
+  queued = c->folds.queued;
   rec.start = prof_event(c);
   rec.stop = prof_event(c);
   if (!rec.start || !rec.stop) return;
@@ -239,6 +240,11 @@ NrsProfScope::NrsProfScope(nrs_ctx* c, int kind, double work) : ctx(c) {
 
 NrsProfScope::~NrsProfScope() {
   if (!active) return;
+  if (queued != ctx->folds.queued) {
+    ctx->prof_free_events.push_back(rec.start);
+    ctx->prof_free_events.push_back(rec.stop);
+    return;
+  }
   if (cudaEventRecord(rec.stop, ctx->stream) == cudaSuccess) ctx->prof_records.push_back(rec);
 }
 

@@ -210,6 +210,7 @@ struct NrsFolds {
   // Weight gradients that wait for the pass's end (wgrad_queue.h): where they write, their kernels' own queues, and memory
   // they read whose owner has let go of it.
   std::vector<std::pair<const float*, size_t>> waiting;
+  uint64_t queued = 0;     // how many have ever waited
   std::shared_ptr<void> waiting_rows, waiting_tiles;
   std::vector<void*> kept;
   size_t kept_bytes = 0;
@@ -285,10 +286,12 @@ struct NrsIndependentNext {
 };
 
 // Brackets the launches issued during its lifetime with two events when
-// profiling is on; free otherwise.
+// profiling is on; free otherwise.  A product that was queued meanwhile is not counted here but where
+// it is launched.
 struct NrsProfScope {
   nrs_ctx* ctx;
   bool active = false;
+  uint64_t queued = 0;
   NrsProfRecord rec{};
   NrsProfScope(nrs_ctx* c, int kind, double work);
   ~NrsProfScope();

@@ -334,9 +334,10 @@ extern "C" int nrs_selftest_bounded_wait(nrs_ctx* ctx, int64_t limit_clocks) {
 }
 
 namespace {
-// Back-to-back tcgen05.mma.kind::tf32 (M = 128, N = 256, K = 8) on operands that never leave shared
+// Back-to-back tcgen05.mma (M = 128, N = 256, 32 bytes of K: 8 values of kind::tf32, 16 of kind::f16) on operands that never leave shared
 // memory: the tensor pipe's own rate, with no TMA traffic and no epilogue.  One issuing thread per CTA,
 // one CTA per SM; every wait is bounded.
+template <bool HALF>
 __global__ void __launch_bounds__(128, 1) umma_rate_kernel(int iters, int* __restrict__ err_flag) {
   extern __shared__ uint8_t umma_rate_smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(umma_rate_smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -351,12 +352,14 @@ __global__ void __launch_bounds__(128, 1) umma_rate_kernel(int iters, int* __res
   tc::tc_fence_after_sync();
   const uint32_t tmem = tmem_slot;
   if (threadIdx.x == 0) {
-    const uint32_t idesc = tc::make_idesc_tf32(128, 256, false, false);
+    const uint32_t idesc = HALF ? tc::make_idesc_f16(128, 256, false, false) : tc::make_idesc_tf32(128, 256, false, false);
     const uint32_t a = tc::smem_u32(smem), b = a + 16384;     // A: 128 rows x 128 B; B: 256 rows x 128 B
     for (int i = 0; i < iters; ++i) {
-      const uint32_t koff = (uint32_t)(i & 3) * 32u;            // the four K-steps of a 32-element K block
-      tc::umma_tf32(tmem + ((i & 1) ? 256u : 0u), tc::make_smem_desc_sw128(a + koff, 16, 1024),
-                    tc::make_smem_desc_sw128(b + koff, 16, 1024), idesc, 1);
+      const uint32_t koff = (uint32_t)(i & 3) * 32u;            // the four K-steps of a row of 128 bytes
+      const uint32_t d = tmem + ((i & 1) ? 256u : 0u);
+      const uint64_t da = tc::make_smem_desc_sw128(a + koff, 16, 1024), db = tc::make_smem_desc_sw128(b + koff, 16, 1024);
+      if (HALF) tc::umma_f16(d, da, db, idesc, 1);
+      else tc::umma_tf32(d, da, db, idesc, 1);
     }
     tc::umma_commit(&bar);
     if (!tc::mbar_wait(&bar, 0)) atomicExch(err_flag, tc::kErrMmaWait);
@@ -365,25 +368,25 @@ __global__ void __launch_bounds__(128, 1) umma_rate_kernel(int iters, int* __res
   __syncthreads();
   if (threadIdx.x < 32) { tc::tc_fence_after_sync(); tc::tmem_dealloc(tmem, 512); }
 }
-}  // namespace
 
-extern "C" int nrs_measure_tf32_umma_peak(nrs_ctx* ctx, double* tflops_out) {
+template <bool HALF>
+int measure_umma_peak(nrs_ctx* ctx, const char* who, double* tflops_out) {
   NRS_REQUIRE_CTX(ctx);
-  NRS_REQUIRE(ctx, tflops_out != nullptr, NRS_ERR_ARG, "nrs_measure_tf32_umma_peak: null output");
+  NRS_REQUIRE(ctx, tflops_out != nullptr, NRS_ERR_ARG, "%s: null output", who);
   *tflops_out = 0.0;
   int* err = nullptr;
   int st = nrs_err_flag(ctx, &err);
   if (st != NRS_OK) return st;
   constexpr int kSmem = 64 * 1024, kIters = 40000;          // ~2.6 ms at 128 clocks per UMMA
   static NrsSmemAttr attr;
-  NRS_ENSURE_SMEM(ctx, attr, umma_rate_kernel, kSmem);
+  NRS_ENSURE_SMEM(ctx, attr, umma_rate_kernel<HALF>, kSmem);
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   NRS_CUDA(ctx, cudaEventCreate(&e0));
   NRS_CUDA(ctx, cudaEventCreate(&e1));
   float best_ms = 0.0f;
   for (int rep = 0; rep < 4; ++rep) {                        // the first launch warms up
     cudaEventRecord(e0, ctx->stream);
-    umma_rate_kernel<<<ctx->sm_count, 128, kSmem, ctx->stream>>>(kIters, err);
+    umma_rate_kernel<HALF><<<ctx->sm_count, 128, kSmem, ctx->stream>>>(kIters, err);
     ctx->launches++;
     cudaEventRecord(e1, ctx->stream);
     if (cudaEventSynchronize(e1) != cudaSuccess) break;
@@ -396,9 +399,13 @@ extern "C" int nrs_measure_tf32_umma_peak(nrs_ctx* ctx, double* tflops_out) {
   NRS_CUDA(ctx, cudaGetLastError());
   st = nrs_check_device_error(ctx);
   if (st != NRS_OK) return st;
-  if (best_ms > 0.0f) *tflops_out = 2.0 * 128 * 256 * 8 * (double)kIters * ctx->sm_count / (best_ms * 1e-3) / 1e12;
+  if (best_ms > 0.0f) *tflops_out = 2.0 * 128 * 256 * (HALF ? 16 : 8) * (double)kIters * ctx->sm_count / (best_ms * 1e-3) / 1e12;
   return NRS_OK;
 }
+}  // namespace
+
+extern "C" int nrs_measure_tf32_umma_peak(nrs_ctx* ctx, double* tflops_out) { return measure_umma_peak<false>(ctx, "nrs_measure_tf32_umma_peak", tflops_out); }
+extern "C" int nrs_measure_f16_umma_peak(nrs_ctx* ctx, double* tflops_out) { return measure_umma_peak<true>(ctx, "nrs_measure_f16_umma_peak", tflops_out); }
 
 int nrs_tc_gemm(nrs_ctx* ctx, int trans_a, int trans_b, int batch, int m, int n, int k, const float* a, const float* b,
                 float* c, const float* bias, int act, float beta, NrsGemmExtras* extras) {

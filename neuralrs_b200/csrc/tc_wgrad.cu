@@ -320,6 +320,8 @@ struct WgradJob {
   WgradEntry e;
   int planes;
   long most;   // tiles of an accumulation chain
+  double flop;
+  bool linear;
   float* dw;
   int accumulate, out_cols;
   bool can_be_direct;
@@ -546,6 +548,8 @@ int nrs_tc_conv_wgrad(nrs_ctx* ctx, const float* x, const float* dy, float* dw, 
   job.e = WgradEntry{maps[0], maps[1], maps[2], maps[3], p};
   job.planes = planes;
   job.most = split3 ? max_tiles(p, planes) : std::max((long)alone(p), (long)tc::kMaxChainK / p.kp);   // (see wgrad_queue.h)
+  job.flop = 2.0 * n * oh * ow * co * ci * taps;
+  job.linear = oh * ow == 1;
   job.dw = dw;
   job.accumulate = accumulate;
   job.out_cols = out_cols;
@@ -557,6 +561,7 @@ int nrs_tc_conv_wgrad(nrs_ctx* ctx, const float* x, const float* dy, float* dw, 
   if (!f.waiting_tiles) f.waiting_tiles = std::make_shared<std::vector<WgradJob>>();
   static_cast<std::vector<WgradJob>*>(f.waiting_tiles.get())->push_back(job);
   f.waiting.push_back({dw, (size_t)co * ci * taps});
+  ++f.queued;
   return NRS_OK;
 }
 
@@ -569,19 +574,22 @@ int nrs_wgrad_tiles_run(nrs_ctx* ctx) {
     WgradJob* jobs = all->data() + i;
     const int planes = jobs[0].planes;
     std::vector<wgq::Piece> pieces;
-    double least = 0.0;
+    double least = 0.0, flop = 0.0, linear = 0.0;
     for (e = i; e < all->size() && (int)(e - i) < kWgBatch; ++e) {
       const WgradParams& p = (*all)[e].e.p;
       const long most = (*all)[e].most;
       const double bytes = (double)split_floats(p) * sizeof(float), need = bytes * ((p.n_tiles + most - 1) / most);
       if ((*all)[e].planes != planes || (e > i && least + need > kMostPartial)) break;
       least += need;
+      flop += (*all)[e].flop;
+      if ((*all)[e].linear) linear += (*all)[e].flop;
       const double umma = p.kp / 16.0 * (planes == 2 ? 3.0 : 2.0) * std::max(p.group_cols / 2, 47), fill = p.kp * pixel_bytes_of(p) / 60.0;
       pieces.push_back({p.ctas, p.n_tiles, std::max(umma, fill), 2500.0 + 4.0 * p.group_cols, most, bytes, 0});
     }
     wgq::share_out(pieces, ctx->sm_count);
     const int n = (int)(e - i);
     for (int k = 0; k < n; ++k) jobs[k].e.p.tiles_per_split = (int)pieces[k].per;
+    NrsProfScope prof(ctx, 2.0 * linear > flop ? NRS_PROF_GEMM : NRS_PROF_CONV_WGRAD, flop);   // (a launch of both: by the larger part)
     const int st = n == 1 ? launch_wgrad<1>(ctx, jobs, 1, false) : launch_wgrad<kWgBatch>(ctx, jobs, n, false);
     if (st != NRS_OK) return st;
   }

@@ -295,6 +295,7 @@ struct RowJob {
   RowEntry e;
   int planes;
   long most;   // tiles of an accumulation chain
+  double flop;
   float* dw;
   int accumulate;
 };
@@ -434,6 +435,7 @@ int nrs_tc_conv_wgrad_rows(nrs_ctx* ctx, const float* x, const float* dy, float*
   e.p = p;
   job.planes = planes;
   job.most = split3 ? max_tiles(p, planes) : std::max((long)p.tiles_per_split, (long)tc::kMaxChainK / p.P);   // (see wgrad_queue.h)
+  job.flop = 18.0 * n * h * wd * co * ci;
   job.dw = dw;
   job.accumulate = accumulate;
   if (nrs_wgrad_may_wait(ctx, dy_hi, x_hi)) {
@@ -443,6 +445,7 @@ int nrs_tc_conv_wgrad_rows(nrs_ctx* ctx, const float* x, const float* dy, float*
     if (!f.waiting_rows) f.waiting_rows = std::make_shared<std::vector<RowJob>>();
     static_cast<std::vector<RowJob>*>(f.waiting_rows.get())->push_back(job);
     f.waiting.push_back({dw, (size_t)co * ci * 9});
+    ++f.queued;
     return NRS_OK;
   }
   return launch_rows<1>(ctx, &job, 1, may_overlap);
@@ -457,7 +460,7 @@ int nrs_wgrad_rows_run(nrs_ctx* ctx) {
     RowJob* jobs = all->data() + i;
     const int planes = jobs[0].planes;
     std::vector<wgq::Piece> pieces;
-    double least = 0.0;
+    double least = 0.0, flop = 0.0;
     for (e = i; e < all->size() && (int)(e - i) < kRowBatch; ++e) {
       const RowParams& p = (*all)[e].e.p;
       const long most = (*all)[e].most;
@@ -465,12 +468,14 @@ int nrs_wgrad_rows_run(nrs_ctx* ctx) {
       const double need = bytes * ((p.n_tiles + most - 1) / most);
       if ((*all)[e].planes != planes || (e > i && least + need > kMostPartial)) break;
       least += need;
+      flop += (*all)[e].flop;
       const double fill = planes * (dy_bytes(p, planes == 2 ? 2 : 4) + x_bytes(p, planes == 2 ? 2 : 4)) / 60.0;
       pieces.push_back({p.ctas, p.n_tiles, std::max(p.P / (planes == 2 ? 16.0 : 8.0) * umma, fill) + 110.0, 4000.0, most, bytes, 0});
     }
     wgq::share_out(pieces, ctx->sm_count);
     const int n = (int)(e - i);
     for (int k = 0; k < n; ++k) jobs[k].e.p.tiles_per_split = (int)pieces[k].per;
+    NrsProfScope prof(ctx, NRS_PROF_CONV_WGRAD, flop);
     const int st = n == 1 ? launch_rows<1>(ctx, jobs, 1, false) : launch_rows<kRowBatch>(ctx, jobs, n, false);
     if (st != NRS_OK) return st;
   }

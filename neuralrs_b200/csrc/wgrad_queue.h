@@ -16,7 +16,7 @@
 
 // May the weight gradient of these planes wait?
 inline bool nrs_wgrad_may_wait(const nrs_ctx* ctx, const void* dy_hi, const void* x_hi) {
-  if (!ctx->folds.active || ctx->profiling) return false;
+  if (!ctx->folds.active) return false;
   for (const void* s : ctx->ws_slot)
     if (s == dy_hi || s == x_hi) return false;   // scratch that the next layer overwrites
   return true;

@@ -409,3 +409,27 @@ def test_ranges_of_a_captured_graph(gpu_ctx):
         assert cu.cuGraphExecDestroy(exec_h) == 0 and cu.cuGraphDestroy(graph_h) == 0
     finally:
         ctx.close()
+
+
+def test_profiling_brackets_what_a_step_launches(gpu_ctx):
+    """The launches of a step are the same with brackets around them, and a family's work is its layers'."""
+    shape, layers = NETS["deep"]
+    n = 13
+    rng = np.random.default_rng(1)
+    x, t = rng.standard_normal((n, *shape)).astype(np.float32), np.eye(10, dtype=np.float32)[rng.integers(0, 10, n)]
+    tr = cuda.Trainer(layers, shape, 10, ctx=gpu_ctx)
+    tr.set_params([p.ravel() for p in workloads.he_init(layers, 7)])
+    tr.step(x, t)
+    launches, ms, work, calls = [], ctypes.c_double(), ctypes.c_double(), ctypes.c_uint64()
+    try:
+        for on in (0, 1):
+            call(gpu_ctx, "nrs_profile_enable", on)
+            before = gpu_ctx.launch_count()
+            tr.step(x, t)
+            launches.append(gpu_ctx.launch_count() - before)
+        call(gpu_ctx, "nrs_profile_get", 2, ctypes.byref(ms), ctypes.byref(work), ctypes.byref(calls))   # weight gradients of convolutions
+    finally:
+        call(gpu_ctx, "nrs_profile_enable", 0)
+        call(gpu_ctx, "nrs_profile_reset")
+    assert launches[0] == launches[1] and calls.value < 15 and ms.value > 0
+    assert np.isclose(work.value, sum(18.0 * n * 64 * ly[1] * ly[2] for ly in layers if ly[0] == "conv"))
