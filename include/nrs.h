@@ -50,11 +50,18 @@ enum nrs_status {
   NRS_ERR_UNSUPPORTED = 7  /* valid request this build has no kernel for     */
 };
 
-/* Contraction precision.  3xTF32 (default): each f32 operand is split into a
- * TF32 high part and a TF32 residual and three tensor-core products are summed
- * in f32.  The tensor core's sums are not rounded to nearest: the relative error
- * is some 7e-9 per term of a reduction, 1e-6 for a hundred terms, 2e-5 for
- * thousands.  TF32: one product of operands rounded to 11 bits (error ~1e-3).
+/* Contraction precision.  3xTF32 (default): each f32 operand is held as two f16
+ * values, 22 bits together, with one power-of-two exponent per tensor, and three
+ * tensor-core products are summed in f32.  The exponent comes from a bound of
+ * the tensor's largest magnitude: values down to 2^-28 of the bound keep their
+ * 22 bits, smaller ones an absolute error of 2^-50 of it (what lies below that
+ * is zero).  The bound of a tensor that the caller brings is its largest value,
+ * of a result that one layer leaves for the next up to some 2^12 above it (a
+ * product over K terms: K times the operands' largest); all matrices of an
+ * nrs_bmm share one.  The tensor core's sums are not rounded to nearest: the
+ * relative error is some 3e-9 per term of a reduction, 1e-6 for a few hundred
+ * terms, 1e-5 for thousands.  A caller whose rows or channels differ by more
+ * than that range and who needs their bits asks for FP32.  TF32: one product of operands rounded to 11 bits (error ~1e-3).
  * FP32: the CUDA-core FFMA kernels only.
  * The two TF32 modes hold for every convolution of stride 8 and less, strided and
  * ragged ones included, for products (nrs_gemm, nrs_bmm) of m >= 16, n >= 32 and

@@ -1,4 +1,4 @@
-// Multi-head attention over TF32 operand planes: any sequence length up to 4096 and any head size that is a
+// Multi-head attention over operand planes (f16 pairs, or TF32 values): any sequence length up to 4096 and any head size that is a
 // multiple of 8, where the one-CTA-per-head kernels (attention_tc.cu: 128 keys, 32 columns) end.
 //
 //   forward   S = Q K^T                 P = softmax(scale S, causal)      O = P V
@@ -11,9 +11,9 @@
 // lies in memory (K-major, or MN-major where the reduction index is the slow one), a causal product neither computes
 // the tiles above the diagonal nor walks the K-slices that are zero, and P, dS, O and the three gradients leave
 // their kernels as the planes the next product reads.  HBM-bound by the [batch*heads][seq][seq] matrices: 4 B written
-// and read per element for S and dP, 8 B for P and dS, half of it when causal.
+// and read per element of each of S, dP, P and dS (two halves of a pair, or a TF32 value), half of it when causal.
 //
-// Measured on the 512-wide model (6 sequences of 500, 8 heads of 64, causal, 3xTF32), one layer forward + backward:
+// Measured before f16 pairs, on the 512-wide model (6 sequences of 500, 8 heads of 64, causal, 3xTF32), one layer forward + backward:
 // 204 us (products 163, row kernels 41); with the permutations, transposes, scale, mask and softmax kernels that it
 // replaces there, and Q, K, V as three products each way, a step of two layers took 0.92 ms more.  At 32 sequences of
 // 128, 8 heads of 32: 96 us, where the one-CTA-per-head kernels take 107 and need K, V and the gradients unsplit.

@@ -94,12 +94,12 @@ struct Node {
   float* gplanes_lo = nullptr;
   // With a premasked gradient: per-block channel sums of it ([rows][channels]), which the
   // convolution's bias gradient folds instead of summing the whole NCHW gradient again.
+  float* gchan_partial = nullptr;
+  int gchan_rows = 0;
   // Column sums of the whole gradient, left by the kernel that wrote it where the reader wants them (a linear layer's bias
   // gradient); dropped with gtop when another share arrives.
   bool grad_sums_wanted = false;
   std::shared_ptr<GradSums> gsums;
-  float* gchan_partial = nullptr;
-  int gchan_rows = 0;
 
   // Set on the output of a Linear layer with a fused activation whose backward pass can start from planes: the
   // activation and what its derivative is taken from (RELU: the output, GELU: the pre-activation).  The Linear layer

@@ -238,15 +238,15 @@ struct nrs_ctx {
   volatile int* err_host = nullptr;  // the same word as the host sees it (mapped memory)
   void* pinned = nullptr;            // page-locked: the error word, and a slot for small read-backs; made on first use
   unsigned* fold_ticket = nullptr;   // arrival counter of kernels whose last block folds the blocks' partial sums
-  // Planes registered for a source tensor (keyed by its device pointer); the conv kernels
-  // use them instead of staging again.  Whoever registers keeps both alive and unregisters.
   // Bounds of tensors for the duration of a call that stages them (an operator that had them measured in another launch).
   std::map<const void*, const NrsRange*> known_tops;
+  // Planes registered for a source tensor (keyed by its device pointer); the conv kernels
+  // use them instead of staging again.  Whoever registers keeps both alive and unregisters.
   std::map<const void*, NrsPlanes> plane_hints;
-  std::map<const void*, NrsPlanes> owned_planes;
-  std::unordered_map<const void*, NrsRange*> ranges;   // of f16 pair planes (by the address of hi) and of f32 tensors (by their address)
+  std::map<const void*, NrsPlanes> owned_planes;   // nrs_planes_cache: planes the context itself allocated
+  std::unordered_map<const void*, NrsRange*> ranges;   // of f16 pair planes, by the address of hi
   NrsRangePool range_pool;
-  char scratch_range[2];   // addresses that own the ranges of measurements inside a call   // nrs_planes_cache: planes the context itself allocated
+  char scratch_range[2];   // addresses that own the ranges of measurements inside a call
   std::map<const void*, NrsOutExtras> out_extras;
   std::map<const void*, NrsColsumRequest> colsum_requests;
   // Patch planes (see conv_patch.cu) of a tensor with few channels, keyed by its device pointer: the host graph

@@ -6,7 +6,7 @@
 // (up to 256 columns), reduction over output pixels.  Both operands come from
 // the NHWC planes the forward / data-gradient kernels also use, so along the
 // reduction (pixels) they are MN-major: a TMA box {32 channels, Wt, Ht, Nt}
-// lands in shared memory as [pixel][32 channels = 128 B].  For 32-bit operands
+// lands in shared memory as [pixel][32 channels = 128 B] (f16 pairs: 64 channels, or 32 in 64 B).  For 32-bit operands
 // kind::tf32 takes MN-major data only in the 128-byte swizzle with 32-byte atoms
 // (4 pixels x 128 B per swizzle group), which TMA produces with
 // CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B.  A K-step of 8 pixels is two groups (SBO =
@@ -22,8 +22,8 @@
 // sums the partials in a fixed order (deterministic, unlike the reference's
 // atomicAdd split-K, src/cuda/graph/matmul.rs:207-261) and scatters into the
 // [co][ci][kh][kw] layout.  In 3xTF32 mode no CTA accumulates more than
-// tc::kMaxChainK pixels (the tensor core's f32 accumulation error grows with the
-// chain length).
+// tc::kMaxChainPairs pixels (the tensor core's f32 accumulation error grows with the
+// chain length); for TF32 mode see wgrad_queue.h.
 //
 // Replaces conv2d_im2col + conv2d_out2mm + matmul_nt_splitk (src/cuda/nn/conv.rs:
 // 298-320).

@@ -21,7 +21,7 @@
 // this kernel did before, took 1300 clocks per 32-pixel row, more than half of them bookkeeping of the issuing warp:
 // x[256,64,32,32] -> 128 channels in 3xTF32 112 us, here 79 (1270 clocks per 64 pixels, of which the UMMAs are 1152).
 //
-// Tiles are split across CTAs (no accumulation chain longer than tc::kMaxChainK pixels in 3xTF32 mode); partial sums are
+// Tiles are split across CTAs (no accumulation chain longer than tc::kMaxChainPairs pixels in 3xTF32 mode); partial sums are
 // added up in a fixed order by a second kernel, which also scatters into [co][ci][3][3].
 //
 // Replaces conv2d_im2col + conv2d_out2mm + matmul_nt_splitk (src/cuda/nn/conv.rs:
