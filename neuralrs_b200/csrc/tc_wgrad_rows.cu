@@ -262,7 +262,9 @@ tc_wgrad_rows_kernel(const __grid_constant__ RowBatch<CAP> batch, int* __restric
 }
 
 // The tile: the Wt x R rectangle that walks the image in the least time, by what a step costs: its UMMAs or its bytes
-// through L2 (60 a clock), whichever is more, and about 150 clocks besides; rings of two stages lose about a sixth.
+// through L2 (60 a clock), whichever is more, and about 150 clocks besides (118 of them measured, above); rings of two
+// stages lose about a sixth (forced to two: 256 images, 64 -> 128 channels, 32 x 32 73 -> 95 us, 256 -> 128, 12 x 12 55 -> 68,
+// 64 of 64 x 24 x 24 16.2 -> 16.7).
 bool plan_row_tile(RowParams* p, int h, int w, int planes) {
   const int value = planes == 2 ? 2 : 4, step = planes == 2 ? 16 : 8;
   const double step_clk = (planes == 2 ? 3 : 1) * (p->chunk / p->wb) * kTaps * p->wb * 0.5;
@@ -361,8 +363,10 @@ int nrs_tc_conv_wgrad_rows(nrs_ctx* ctx, const float* x, const float* dy, float*
   if (kh != 3 || kw != 3 || stride != 1 || pad != 1 || ci % 32 != 0 || co % 32 != 0 || n < 1 || h < 1 || wd < 1) return NRS_ERR_UNSUPPORTED;
   const bool split3 = ctx->math_mode == NRS_MATH_3XTF32;
   const int planes = split3 ? 2 : 1;
-  // A TF32 gradient on its own: rows of 16, 32 or 64 pixels (256 x 12 x 12, 256 -> 128 channels: 58 us here, 49 by the general
-  // kernel).  Among others of a backward pass all of them (CIFAR CNN with batch normalisation: a step 1.35 ms, 1.38 without).
+  // A TF32 gradient on its own: rows of 16, 32 or 64 pixels, of which a tile wastes nothing.  At other widths the general
+  // kernel is faster or as fast (us here / there: 8 pixels 30 / 23, 12 58 / 39, 14 20 / 17, 24 16 / 14, 28 41 / 34, 40 28 / 30,
+  // 48 78 / 74, 56 61 / 62; 64 to 256 channels).  Among others of a backward pass all of them (CIFAR CNN with batch
+  // normalisation: a step 1.35 ms, 1.38 without).
   if (!split3 && wd != 16 && wd != 32 && wd != 64 && !ctx->folds.active) return NRS_ERR_UNSUPPORTED;
 
   RowParams p{};
