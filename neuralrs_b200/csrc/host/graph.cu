@@ -234,7 +234,7 @@ struct WeightTop {
   TopP top;
   bool known = false;
   WeightTop(nrs_ctx* c, const NodeP& w_, bool wanted) : ctx(c), w(w_) {
-    if (wanted && c->math_mode == NRS_MATH_3XTF32 && w->len() > (size_t)pr::kScanAlone && !c->plane_hints.count(w->data) && !c->known_tops.count(w->data) &&
+    if (wanted && c->math_mode == NRS_MATH_3XTF32 && w->len() > (size_t)pr::kScanAlone && !c->plane_hints.count(w->data) &&
         !nrs_weight_planes_find(c, w->data, NRS_WF_LINEAR_T) && !nrs_weight_planes_find(c, w->data, NRS_WF_LINEAR_ROWS))
       top = new_top(c);
   }

@@ -366,40 +366,9 @@ NodeP MultiHeadAttention::forward_batch(const NodeP& x) const {
   return reshape(matmul(reshape(concat, {batch * seq, d}), w_o), {batch, seq, d});
 }
 
-// 3xTF32, weights that nobody has staged yet: bounds of those that a block's products will stage one by one, measured in one
-// launch and known until the end of its forward pass.  (A launch each: 274 us a step instead of 262 with TF32 pairs at 256
-// tokens of 256.)
-struct WeightsMeasured {
-  nrs_ctx* ctx;
-  std::vector<TopP> tops;
-  std::vector<const float*> keys;
-  WeightsMeasured(nrs_ctx* c, size_t tokens, std::initializer_list<NodeP> weights) : ctx(c) {
-    if (c->math_mode != NRS_MATH_3XTF32 || tokens > 0x7fffffff) return;
-    std::vector<NrsMeasure> m;
-    for (const NodeP& w : weights) {
-      if (!w || !w->on_gpu() || w->shape.size() != 2 || w->len() <= (size_t)kNrsScanAlone || w->shape[0] > 0x7fffffff || w->shape[1] > 0x7fffffff) continue;
-      if (!nrs_gemm_on_tensor_cores(c, (int)tokens, (int)w->shape[1], (int)w->shape[0]) || nrs_weight_planes_find(c, w->data, NRS_WF_LINEAR_T) ||
-          c->plane_hints.count(w->data) || c->known_tops.count(w->data) || m.size() == (size_t)kNrsMeasured)
-        continue;
-      tops.push_back(new_top(c));
-      m.push_back(NrsMeasure{w->data, w->len(), tops.back()->range});
-    }
-    if (m.size() < 2) return;
-    check(c, nrs_absmax_each(c, m.data(), (int)m.size()));
-    for (const NrsMeasure& k : m)
-      if (c->known_tops.emplace(k.src, k.r).second) keys.push_back(k.src);
-  }
-  ~WeightsMeasured() {
-    for (const float* k : keys) ctx->known_tops.erase(k);
-  }
-  WeightsMeasured(const WeightsMeasured&) = delete;
-  WeightsMeasured& operator=(const WeightsMeasured&) = delete;
-};
-
 static NodeP block_body(const TransformerBlock& b, const NodeP& x, bool final_norm) {
   if (!x || x->shape.size() != 3) fail(NRS_ERR_SHAPE, "cuda transformer block: input must be [batch, seq, d_model]");
   const size_t batch = x->shape[0], seq = x->shape[1], d = x->shape[2];
-  WeightsMeasured measured(x->ctx, batch * seq, {b.mha.w_o, b.ff1.weights, b.ff2.weights});
   NodeP attn_out = b.mha.forward_batch(x);
   NodeP x1 = b.fused_epilogues ? layernorm_residual(x, attn_out, b.norm1.gamma, b.norm1.beta, b.norm1.eps, true)
                                : b.norm1.forward(add(x, attn_out));

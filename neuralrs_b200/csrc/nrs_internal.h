@@ -319,14 +319,10 @@ inline NrsRange* nrs_range_of(const nrs_ctx* ctx, const void* p) {
   auto it = ctx->ranges.find(p);
   return it == ctx->ranges.end() ? nullptr : it->second;
 }
-// Tensors of up to this many values are measured by the blocks of the launch that stages them.
-constexpr int kNrsScanAlone = 32768;
 // Largest finite magnitude of `count` values at `src` into r->top and r->bound (tc_stage.cu).
 int nrs_absmax(nrs_ctx* ctx, const float* src, size_t count, NrsRange* r);
-// The same of up to kNrsMeasured tensors in one launch.
-struct NrsMeasure { const float* src; size_t n; NrsRange* r; };
-constexpr int kNrsMeasured = 4;
-int nrs_absmax_each(nrs_ctx* ctx, const NrsMeasure* m, int count);
+// The same of two tensors in one launch.
+int nrs_absmax2(nrs_ctx* ctx, const float* a, size_t na, NrsRange* ra, const float* b, size_t nb, NrsRange* rb);
 // dst = the values of n consecutive f16 pairs.
 int nrs_pair_unpack(nrs_ctx* ctx, const float* hi, const float* lo, float* dst, size_t n);
 int nrs_err_flag(nrs_ctx* ctx, int** out);

@@ -110,7 +110,7 @@ __device__ __forceinline__ void report(NrsRange* r, uint32_t top) {
   if ((threadIdx.x & 31) == 0) atomicMax(reinterpret_cast<unsigned*>(&r->top), top);   // (no result: nothing waits for it)
 }
 // What one block finds in n values (all of its threads ask; at most kScanAlone values, else absmax_kernel measures them).
-constexpr int kScanAlone = kNrsScanAlone;
+constexpr int kScanAlone = 32768;
 __device__ __forceinline__ uint32_t scan(const float* __restrict__ src, int n) {
   __shared__ uint32_t found[32];
   uint32_t top = 0;

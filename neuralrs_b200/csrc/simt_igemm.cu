@@ -620,8 +620,7 @@ int nrs_gemm_extras(nrs_ctx* ctx, int trans_a, int trans_b, int m, int n, int k,
         if ((size_t)(m + n) * k > (size_t)pr::kScanAlone) {   // (else every block scans them: 3 us less than a launch)
           if (st == NRS_OK) st = nrs_range_renew(ctx, &ctx->scratch_range[0], &range_a);
           if (st == NRS_OK) st = nrs_range_renew(ctx, &ctx->scratch_range[1], &range_b);
-          const NrsMeasure both[2] = {{a, (size_t)m * k, range_a}, {b, (size_t)n * k, range_b}};
-          if (st == NRS_OK) st = nrs_absmax_each(ctx, both, 2);
+          if (st == NRS_OK) st = nrs_absmax2(ctx, a, (size_t)m * k, range_a, b, (size_t)n * k, range_b);
         }
         if (st != NRS_OK) return st;
       }

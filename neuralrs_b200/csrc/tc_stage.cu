@@ -10,13 +10,14 @@
 namespace {
 
 // Largest finite magnitude of n values into r->top.  A read of the tensor, from HBM where it exceeds L2.
-constexpr int kSources = kNrsMeasured;   // tensors of one launch
-struct MeasuredSet { NrsMeasure m[kSources]; };
+struct Measured { const float* src; size_t n; NrsRange* r; };
+constexpr int kSources = 4;   // tensors of one launch
+struct MeasuredSet { Measured m[kSources]; };
 __global__ void __launch_bounds__(256)
 absmax_kernel(const __grid_constant__ MeasuredSet set) {
   NRS_PDL_PROLOGUE();
   __shared__ uint32_t part[8];
-  const NrsMeasure& m = set.m[blockIdx.y];
+  const Measured& m = set.m[blockIdx.y];
   const float* __restrict__ src = m.src;
   const size_t n = m.n;
   const size_t head = min(n, (size_t)(((16 - (reinterpret_cast<uintptr_t>(src) & 15)) & 15) / 4)), quads = (n - head) / 4;
@@ -428,19 +429,18 @@ static unsigned absmax_blocks(const nrs_ctx* ctx, size_t count) {
   return (unsigned)(blocks < cap ? blocks : cap);
 }
 int nrs_absmax(nrs_ctx* ctx, const float* src, size_t count, NrsRange* r) {
-  const NrsMeasure m{src, count, r};
-  return nrs_absmax_each(ctx, &m, 1);
-}
-int nrs_absmax_each(nrs_ctx* ctx, const NrsMeasure* m, int count) {
-  NRS_REQUIRE(ctx, count >= 0 && count <= kSources, NRS_ERR_ARG, "too many tensors to measure");
+  if (count == 0) return NRS_OK;
   MeasuredSet set{};
-  size_t longest = 0;
-  for (int i = 0; i < count; ++i) {
-    set.m[i] = m[i];
-    longest = std::max(longest, m[i].n);
-  }
-  if (longest == 0) return NRS_OK;
-  NRS_PDL_LAUNCH(absmax_kernel, dim3(absmax_blocks(ctx, longest), count), 256, 0, ctx->stream, set);
+  set.m[0] = Measured{src, count, r};
+  NRS_PDL_LAUNCH(absmax_kernel, absmax_blocks(ctx, count), 256, 0, ctx->stream, set);
+  NRS_LAUNCHED(ctx);
+  return NRS_OK;
+}
+int nrs_absmax2(nrs_ctx* ctx, const float* a, size_t na, NrsRange* ra, const float* b, size_t nb, NrsRange* rb) {
+  MeasuredSet set{};
+  set.m[0] = Measured{a, na, ra};
+  set.m[1] = Measured{b, nb, rb};
+  NRS_PDL_LAUNCH(absmax_kernel, dim3(absmax_blocks(ctx, na > nb ? na : nb), 2), 256, 0, ctx->stream, set);
   NRS_LAUNCHED(ctx);
   return NRS_OK;
 }
@@ -563,11 +563,11 @@ int nrs_tc_stage_each(nrs_ctx* ctx, const float* const* src, int count, float* h
     const int st = nrs_range_renew(ctx, hi, &range);
     if (st != NRS_OK) return st;
     for (int i = 0; i < count; i += kSources) {
-      NrsMeasure m[kSources];
+      MeasuredSet set{};
       const int n = std::min(count - i, kSources);
-      for (int k = 0; k < n; ++k) m[k] = NrsMeasure{src[i + k], (size_t)rows * K, range};
-      const int got = nrs_absmax_each(ctx, m, n);
-      if (got != NRS_OK) return got;
+      for (int k = 0; k < n; ++k) set.m[k] = Measured{src[i + k], (size_t)rows * K, range};
+      NRS_PDL_LAUNCH(absmax_kernel, dim3(absmax_blocks(ctx, (size_t)rows * K), n), 256, 0, ctx->stream, set);
+      NRS_LAUNCHED(ctx);
     }
   }
   const Bound bound{range ? &range->top : nullptr, nullptr, 0, range};

@@ -89,24 +89,19 @@ def test_backward_memory_does_not_grow_with_the_square(gpu_ctx):
 
 
 def test_weights_of_one_product_are_measured_together(gpu_ctx):
-    """f16 pairs want exponents: of the input, of Q, K and V in one launch, of the other weights; nothing else is launched
+    """f16 pairs want exponents: of the input, of Q, K and V in one launch, of the output projection; nothing else is launched
     more than in TF32."""
     B, S, D, H = 2, 128, 256, 8
     rng = np.random.default_rng(1)
     w, x = [on_gpu((rng.standard_normal((D, D)) / 16).astype(np.float32)) for _ in range(4)], rng.standard_normal((B, S, D)).astype(np.float32)
-    mha = nn.MultiHeadAttention(*w, D, H, True)
-    new = lambda *shape: on_gpu((rng.standard_normal(shape) / 16).astype(np.float32))  # noqa: E731
-    block = nn.TransformerBlock(mha, nn.LayerNorm(new(D), new(D), 1e-5), nn.LayerNorm(new(D), new(D), 1e-5), nn.Linear(new(D, 4 * D), new(4 * D)),
-                                nn.Linear(new(4 * D, D), new(D)), D, 4 * D, _lib.ACT_GELU)   # (its three other weights: one launch, too)
-    for forward in (mha.forward_batch, block.forward):
-        launches = {}
-        try:
-            for mode in TOL:
-                gpu_ctx.set_math_mode(mode)
-                gx = on_gpu(x)
-                before = gpu_ctx.launch_count()
-                forward(gx)
-                launches[mode] = gpu_ctx.launch_count() - before
-        finally:
-            gpu_ctx.set_math_mode(_lib.MATH_3XTF32)
-        assert launches[_lib.MATH_3XTF32] <= launches[_lib.MATH_TF32] + 3, launches
+    mha, launches = nn.MultiHeadAttention(*w, D, H, True), {}
+    try:
+        for mode in TOL:
+            gpu_ctx.set_math_mode(mode)
+            gx = on_gpu(x)
+            before = gpu_ctx.launch_count()
+            mha.forward_batch(gx)
+            launches[mode] = gpu_ctx.launch_count() - before
+    finally:
+        gpu_ctx.set_math_mode(_lib.MATH_3XTF32)
+    assert launches[_lib.MATH_3XTF32] <= launches[_lib.MATH_TF32] + 3, launches
