@@ -264,7 +264,8 @@ def test_batchnorm_whose_variance_is_lost(gpu_ctx):
         assert np.isfinite(a).all() and rel_l2(a, b) <= 2 * chain_tolerance(72) + 2 * chain_tolerance(8192)
 
 
-def test_batchnorm_channels_over_many_octaves(gpu_ctx, oracle64):
+@pytest.mark.parametrize("training", [True, False])
+def test_batchnorm_channels_over_many_octaves(gpu_ctx, oracle64, training):
     """Gradients of channels down to 2^-23 of the largest: as planes, below a batch normalisation, they keep their bits."""
     n, c, hw = 8, 64, 8
     layers = [("conv", 16, c, 3, 1, 1), ("batchnorm", c), ("conv", c, 32, 3, 1, 1), ("flatten",), ("linear", 32 * hw * hw, 10)]
@@ -275,8 +276,9 @@ def test_batchnorm_channels_over_many_octaves(gpu_ctx, oracle64):
     params[2] = (2.0 ** -(np.arange(c) % 24)).astype(np.float32).reshape(params[2].shape)
     tr = cuda.Trainer(layers, (16, hw, hw), 10, ctx=gpu_ctx)
     tr.set_params([p.ravel() for p in params])
+    tr.set_training(training)
     tr.forward_backward(x, t)
-    _, ref, _ = models.forward_backward(oracle64, layers, params, x, t, buffers=workloads.bn_buffers(layers))
+    _, ref, _ = models.forward_backward(oracle64, layers, params, x, t, buffers=workloads.bn_buffers(layers), training=training)
     got, want = np.asarray(tr.get_grad(0)).reshape(c, -1), np.asarray(ref[0]).reshape(c, -1)
     # two products forward and one back, twice for what is taken off again in between, then the gradient's own
     bound = 2 * (chain_tolerance(144) + 2 * chain_tolerance(9 * c)) + chain_tolerance(n * hw * hw)
